@@ -54,9 +54,16 @@ __device__ __forceinline__ uint64_t mx_desc(uint32_t saddr, uint32_t lbo, uint32
 __device__ __forceinline__ void mx_mma(uint32_t tmem_c, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}\n" ::"r"(tmem_c),
-      "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_c),
+      "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+// one lane of a converged warp: issuing under this predicate keeps the operands in uniform registers
+// (a product every 10-12 cycles; under "lane == 0" 48, which bound every tile of fewer than 96 tokens)
+__device__ __forceinline__ bool mx_elect() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ void mx_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mx_s32(bar))
@@ -211,7 +218,7 @@ __global__ void __launch_bounds__(MX_NT, 1) k_tc_mx(const MxArgs A) {
       // full[s]: named barrier 1 + s (workers arrive, this warp waits)
       asm volatile("bar.sync %0, %1;" ::"r"(1 + s), "n"(MX_NT) : "memory");
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if ((tid & 31) == 0) {
+      if (mx_elect()) {
         MX_STAMP(1, kc, 0)
         // (descriptors of stage s, step ks = those of stage 0, step 0 plus the byte offset >> 4 in
         // the address field: shared memory addresses stay below 2^18)
