@@ -8,6 +8,7 @@
 #include <cstring>
 #include <new>
 #include <map>
+#include <memory>
 #include <vector>
 
 #include "decode_mega.cuh"
@@ -378,6 +379,7 @@ struct pm_layer {
   LayerDev dev{};
   std::vector<void *> owned;
   std::vector<uint8_t> expert_set;
+  std::shared_ptr<LayerMaps> maps;  // TMA descriptions of the planes (dev.maps)
   bool router_set = false, shared_set = false;
   uint64_t gen = 0;  // bumped by every call that may change a device pointer or a weight (stacks re-snapshot)
   float *router_w = nullptr, *logit_bias = nullptr, *select_bias = nullptr;
@@ -401,6 +403,38 @@ static int32_t wmat_alloc(pm_layer *ly, WMat &W, int type, int n_exp, int rows, 
       CU(cudaMalloc(&W.plane[p], W.stride[p] * (size_t)n_exp + 256));
       ly->owned.push_back(W.plane[p]);
     }
+  }
+  return PM_OK;
+}
+
+// the planes the tensor-core products read, as [expert][row][bytes] with boxes of box_rows rows x one block
+typedef CUresult (*pm_encode_tiled_t)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                      const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                      CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static int32_t wmat_maps(const WMat &W, int n_exp, int box_rows, WMaps &M) {
+  if (W.type != PM_TYPE_Q4_K && W.type != PM_TYPE_Q6_K) return PM_OK;
+  static pm_encode_tiled_t enc = nullptr;
+  if (!enc) {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    CU(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q));
+    if (q != cudaDriverEntryPointSuccess || !f) return fail(PM_ERR_CUDA, "cuTensorMapEncodeTiled is not there");
+    enc = (pm_encode_tiled_t)f;
+  }
+  const int nb = W.cols / 256, n = W.type == PM_TYPE_Q4_K ? 1 : 2;
+  const int block[2] = {W.type == PM_TYPE_Q4_K ? 144 : 128, 64};
+  // Q6_K: 128- and 64-byte rows swizzled so that the row-per-thread reads of the unpack have no bank conflicts
+  // (a Q4_K row of 144 bytes has none as it is)
+  const CUtensorMapSwizzle sw[2] = {W.type == PM_TYPE_Q4_K ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                                    CU_TENSOR_MAP_SWIZZLE_64B};
+  for (int p = 0; p < n; p++) {
+    const cuuint64_t row = (cuuint64_t)nb * block[p];
+    const cuuint64_t dims[3] = {row, (cuuint64_t)W.rows, (cuuint64_t)n_exp}, strides[2] = {row, (cuuint64_t)W.stride[p]};
+    const cuuint32_t box[3] = {(cuuint32_t)block[p], (cuuint32_t)box_rows, 1}, es[3] = {1, 1, 1};
+    const CUresult r = enc(&M.m[p], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, W.plane[p], dims, strides, box, es,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, sw[p], CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(PM_ERR_CUDA, "cuTensorMapEncodeTiled: %d", (int)r);
   }
   return PM_OK;
 }
@@ -508,6 +542,20 @@ extern "C" int32_t pm_layer_create(pm_ctx *ctx, const pm_layer_desc *desc, pm_la
     chk(wmat_alloc(ly, dv.sgate, desc->type_gate, 1, desc->shared_ff, d));
     chk(wmat_alloc(ly, dv.sup, desc->type_up, 1, desc->shared_ff, d));
     chk(wmat_alloc(ly, dv.sdown, desc->type_down, 1, d, desc->shared_ff));
+  }
+  if (rc != PM_OK) {
+    pm_layer_destroy(ly);
+    return rc;
+  }
+  ly->maps = std::make_shared<LayerMaps>();
+  dv.maps = ly->maps.get();
+  rc = wmat_maps(dv.gate, nl, 64, ly->maps->gate);
+  if (rc == PM_OK) rc = wmat_maps(dv.up, nl, 64, ly->maps->up);
+  if (rc == PM_OK) rc = wmat_maps(dv.down, nl, 128, ly->maps->down);
+  if (rc == PM_OK && desc->shared) {
+    rc = wmat_maps(dv.sgate, 1, 64, ly->maps->sgate);
+    if (rc == PM_OK) rc = wmat_maps(dv.sup, 1, 64, ly->maps->sup);
+    if (rc == PM_OK) rc = wmat_maps(dv.sdown, 1, 128, ly->maps->sdown);
   }
   if (rc != PM_OK) {
     pm_layer_destroy(ly);
@@ -893,12 +941,17 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
   Groups g = plan_groups(S.plan, D.n_exp);
   const bool q8 = D.act_quant == PM_AQ_Q8X_256, f16s = D.act_quant == PM_AQ_Q8_32_F16;
   const bool q32 = D.act_quant == PM_AQ_Q8_32 || f16s;
-  if (q8 && !prequant) { PROF(c, PH_QUANT_X); launch_quant_q8x(L, x, (size_t)T, D.d, S.xq, S.xd, S.xbsum, S.xbm, S.xs); }
-  if (q32 && !prequant) { PROF(c, PH_QUANT_X); launch_quant_q8_32(L, x, (size_t)T, D.d, S.xq, S.xd, f16s); }
-  const bool tc = q8 && c->tc_min_tokens > 0 && T >= c->tc_min_tokens;
+  const bool many = c->tc_min_tokens > 0 && T >= c->tc_min_tokens;
+  const bool tc = q8 && many, tc_gu = tc && D.type_gate == D.type_up;
   // MXFP4 weights with f32 activations: the bf16 tensor-core kernels (tolerance parity, not bits)
-  const bool tcmx = D.act_quant == PM_AQ_F32 && D.type_gate == PM_TYPE_MXFP4 && D.type_up == PM_TYPE_MXFP4 &&
-                    D.type_down == PM_TYPE_MXFP4 && c->tc_min_tokens > 0 && T >= c->tc_min_tokens && S.xhl;
+  const bool tcmx = many && D.act_quant == PM_AQ_F32 && D.type_gate == PM_TYPE_MXFP4 && D.type_up == PM_TYPE_MXFP4 &&
+                    D.type_down == PM_TYPE_MXFP4 && S.xhl;
+  TcTiles tt{};
+  if (tc || tcmx) {
+    PROF(c, PH_PLAN);
+    tt = tc_tiles_of(S.tiles, P, g.max_groups, tcmx ? 1 : std::min(D.n_exp, dv.n_local));
+    launch_tc_tiles(L, dv, false, g, tt);
+  }
   if (tcmx) {
     const size_t nx = (size_t)T * D.d, nh = (size_t)P * D.ff;
     {
@@ -907,7 +960,7 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
     }
     {
       PROF(c, PH_GATEUP);
-      CU(launch_tc_mx(L, dv, false, g, P, S.tiles, S.xhl, S.xhl + nx, w, S.h, c->dev_err, c->wait_ns));
+      CU(launch_tc_mx(L, dv, false, g, P, tt, S.xhl, S.xhl + nx, w, S.h, c->dev_err, c->wait_ns));
     }
     {
       PROF(c, PH_QUANT_H);
@@ -915,28 +968,46 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
     }
     {
       PROF(c, PH_DOWN);
-      CU(launch_tc_mx(L, dv, true, g, P, S.tiles, S.hhl, S.hhl + nh, nullptr, S.eo, c->dev_err, c->wait_ns));
+      CU(launch_tc_mx(L, dv, true, g, P, tt, S.hhl, S.hhl + nh, nullptr, S.eo, c->dev_err, c->wait_ns));
     }
     c->path_count[PM_PATH_TENSOR] += 2;
     CU(cudaGetLastError());
     return PM_OK;
   }
   {
+    PROF(c, PH_QUANT_X);
+    if (tc_gu) {
+      // (many rows: quantise every token once and gather the quantised rows, see k_tc_quant_rows)
+      const bool gather = prequant || (size_t)P * D.d > ((size_t)8 << 20);
+      if (gather && !prequant) launch_quant_q8x(L, x, (size_t)T, D.d, S.xq, S.xd, S.xbsum, S.xbm, S.xs);
+      if (gather) launch_tc_rows(L, g, P, tt, g.pair_token, D.d, S.xq, S.xd, S.xbm, S.xs, S.rec);
+      else launch_tc_quant_rows(L, g, P, tt, g.pair_token, D.d, x, S.rec);
+    } else if (q8 && !prequant) {
+      launch_quant_q8x(L, x, (size_t)T, D.d, S.xq, S.xd, S.xbsum);
+    } else if (q32 && !prequant) {
+      launch_quant_q8_32(L, x, (size_t)T, D.d, S.xq, S.xd, f16s);
+    }
+  }
+  {
     PROF(c, PH_GATEUP);
-    if (tc && D.type_gate == D.type_up) {
-      CU(launch_tc_q4k(L, dv, false, false, g, P, S.tiles, S.rec, g.pair_token, S.xq, S.xd, S.xbm, S.xs, w, S.h, c->dev_err, c->wait_ns, c->tc_fault_block));
+    if (tc_gu) {
+      CU(launch_tc(L, dv, false, false, g, P, tt, S.rec, w, S.h, c->dev_err, c->wait_ns, c->tc_fault_block));
       c->path_count[PM_PATH_TENSOR]++;
     } else {
       launch_gateup(L, dv, false, g, P, x, S.xq, S.xd, S.xbsum, w, S.h);
       c->path_count[PM_PATH_GENERAL]++;
     }
   }
-  if (q8) { PROF(c, PH_QUANT_H); launch_quant_q8x(L, S.h, (size_t)P, D.ff, S.hq, S.hd, S.hbsum, S.hbm, S.hs); }
-  if (q32) { PROF(c, PH_QUANT_H); launch_quant_q8_32(L, S.h, (size_t)P, D.ff, S.hq, S.hd, f16s); }
+  {
+    PROF(c, PH_QUANT_H);
+    if (tc) launch_tc_quant_rows(L, g, P, tt, nullptr, D.ff, S.h, S.rec);
+    else if (q8) launch_quant_q8x(L, S.h, (size_t)P, D.ff, S.hq, S.hd, S.hbsum);
+    else if (q32) launch_quant_q8_32(L, S.h, (size_t)P, D.ff, S.hq, S.hd, f16s);
+  }
   {
     PROF(c, PH_DOWN);
     if (tc) {
-      CU(launch_tc_q4k(L, dv, false, true, g, P, S.tiles, S.rec, nullptr, S.hq, S.hd, S.hbm, S.hs, nullptr, S.eo, c->dev_err, c->wait_ns, c->tc_fault_block));
+      CU(launch_tc(L, dv, false, true, g, P, tt, S.rec, nullptr, S.eo, c->dev_err, c->wait_ns, c->tc_fault_block));
       c->path_count[PM_PATH_TENSOR]++;
     } else {
       launch_down(L, dv, false, g, P, S.h, S.hq, S.hd, S.hbsum, S.eo);
@@ -971,20 +1042,28 @@ static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
   g.max_groups = 1;
   const bool q8 = D.act_quant == PM_AQ_Q8X_256, f16s = D.act_quant == PM_AQ_Q8_32_F16;
   const bool q32 = D.act_quant == PM_AQ_Q8_32 || f16s;
-  // (S.xq holds the tokens' Q8x form already when the routed experts ran first)
-  if (q8) launch_quant_q8x(L, x, (size_t)T, D.d, S.xq, S.xd, S.xbsum, S.xbm, S.xs);
-  if (q32) launch_quant_q8_32(L, x, (size_t)T, D.d, S.xq, S.xd, f16s);
-  const bool use_tc = q8 && c->tc_min_tokens > 0 && T >= c->tc_min_tokens;
-  if (use_tc && D.type_gate == D.type_up)
-    CU(launch_tc_q4k(L, dv, true, false, g, T, S.tiles, S.rec, g.pair_token, S.xq, S.xd, S.xbm, S.xs, nullptr, S.sh, c->dev_err, c->wait_ns, c->tc_fault_block));
-  else
+  const bool use_tc = q8 && c->tc_min_tokens > 0 && T >= c->tc_min_tokens, tc_gu = use_tc && D.type_gate == D.type_up;
+  TcTiles tt{};
+  if (use_tc) {
+    tt = tc_tiles_of(S.tiles, T, 1, 1);
+    launch_tc_tiles(L, dv, true, g, tt);
+  }
+  if (tc_gu) {
+    launch_tc_quant_rows(L, g, T, tt, nullptr, D.d, x, S.rec);
+    CU(launch_tc(L, dv, true, false, g, T, tt, S.rec, nullptr, S.sh, c->dev_err, c->wait_ns, c->tc_fault_block));
+  } else {
+    if (q8) launch_quant_q8x(L, x, (size_t)T, D.d, S.xq, S.xd, S.xbsum);
+    if (q32) launch_quant_q8_32(L, x, (size_t)T, D.d, S.xq, S.xd, f16s);
     launch_gateup(L, dv, true, g, T, x, S.xq, S.xd, S.xbsum, nullptr, S.sh);
-  if (q8) launch_quant_q8x(L, S.sh, (size_t)T, D.shared_ff, S.shq, S.shd, S.shbsum, S.shbm, S.shs);
-  if (q32) launch_quant_q8_32(L, S.sh, (size_t)T, D.shared_ff, S.shq, S.shd, f16s);
-  if (use_tc)
-    CU(launch_tc_q4k(L, dv, true, true, g, T, S.tiles, S.rec, nullptr, S.shq, S.shd, S.shbm, S.shs, nullptr, S.shared_out, c->dev_err, c->wait_ns, c->tc_fault_block));
-  else
+  }
+  if (use_tc) {
+    launch_tc_quant_rows(L, g, T, tt, nullptr, D.shared_ff, S.sh, S.rec);
+    CU(launch_tc(L, dv, true, true, g, T, tt, S.rec, nullptr, S.shared_out, c->dev_err, c->wait_ns, c->tc_fault_block));
+  } else {
+    if (q8) launch_quant_q8x(L, S.sh, (size_t)T, D.shared_ff, S.shq, S.shd, S.shbsum);
+    if (q32) launch_quant_q8_32(L, S.sh, (size_t)T, D.shared_ff, S.shq, S.shd, f16s);
     launch_down(L, dv, true, g, T, S.sh, S.shq, S.shd, S.shbsum, S.shared_out);
+  }
   if (D.shared == PM_SHARED_SIGMOID_GATED) launch_shared_gate_logit(L, dv, x, T, S.shared_logit);
   else S.shared_logit = nullptr;
   CU(cudaGetLastError());

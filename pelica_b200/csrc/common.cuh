@@ -215,3 +215,26 @@ __device__ __forceinline__ int pm_warp_sum_i32(int v) {
   for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(PM_FULL, v, o);
   return v;
 }
+
+// `Q8x::new` / `Q8::new` rounding of eight values x * id (half away from zero, as f32::round, src/ds4_cpu.rs:25): the
+// low bytes of two words. id = 127 / (largest |x| of the block), so |x * id| rounds to at most 127. The common
+// case takes five float operations a value: adding 1.5 * 2^23 rounds to the nearest integer (ties to even) and
+// leaves it in the low byte; a value exactly between two integers - and a block so small that 127 / max is
+// infinite - takes the plain form instead.
+__device__ __forceinline__ void pm_q8_pack8(const float v[8], float id, uint32_t &w0, uint32_t &w1) {
+  const float M = 12582912.0f;
+  uint32_t b[8];
+  bool odd = !(id <= 3.4028234e38f);
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const float f = __fmul_rn(v[j], id), m = __fadd_rn(f, M);
+    odd = odd || fabsf(__fsub_rn(f, __fsub_rn(m, M))) == 0.5f;
+    b[j] = __float_as_uint(m);
+  }
+  if (odd) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) b[j] = (uint32_t)(int)fminf(fmaxf(roundf(__fmul_rn(v[j], id)), -127.0f), 127.0f);
+  }
+  w0 = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+  w1 = __byte_perm(__byte_perm(b[4], b[5], 0x0040), __byte_perm(b[6], b[7], 0x0040), 0x5410);
+}

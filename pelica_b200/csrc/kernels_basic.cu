@@ -285,41 +285,36 @@ void launch_dequant(const Launch &L, int type, size_t n, const uint8_t *p0, cons
 // ===========================================================================
 // activation quantiser: `Q8x::new` (src/ds4_cpu.rs:13-35)
 // ===========================================================================
-// one warp per 256-value block, 8 blocks per CTA; lane L holds values L, L+32, ...
-// so that value group j (32 consecutive values) is exactly register j across the warp
+// one warp per 256-value block, 8 blocks per CTA; lane L holds values 8 L .. 8 L + 7, so that the lanes
+// 4 j .. 4 j + 3 hold value group j (32 consecutive values)
 __global__ void __launch_bounds__(256) k_quant_q8x(const float *__restrict__ x, size_t n_blocks,
                                                   int8_t *q, float *d, int32_t *bsum, uint16_t *bm,
                                                   int32_t *xs) {
-  size_t b = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const size_t b = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (b >= n_blocks) return;
-  int lane = threadIdx.x & 31;
-  float v[8];
-#pragma unroll
-  for (int j = 0; j < 8; j++) v[j] = x[b * 256 + 32 * j + lane];
+  const int lane = threadIdx.x & 31;
+  const float4 *src = (const float4 *)(x + b * 256) + 2 * lane;
+  const float4 p0 = __ldg(src), p1 = __ldg(src + 1);
+  const float v[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
   float a = 0.0f;
 #pragma unroll
   for (int j = 0; j < 8; j++) a = fmaxf(a, fabsf(v[j]));
-  a = pm_warp_max(a);
-  float id = a != 0.0f ? __fdiv_rn(127.0f, a) : 0.0f;
-  int tot = 0;
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    int r = 0;
-    if (a != 0.0f) {
-      float f = roundf(__fmul_rn(v[j], id));  // half away from zero, as f32::round
-      r = (int)fminf(fmaxf(f, -127.0f), 127.0f);
-    }
-    q[b * 256 + 32 * j + lane] = (int8_t)r;
-    int s = __reduce_add_sync(PM_FULL, r);
-    tot += s;
-    if (lane == 0) {
-      bsum[b * 8 + j] = s;
-      if (bm) {  // s = 64 * (s >> 6) + (s & 63), both parts exact in f16
-        bm[b * 16 + j] = __half_as_ushort(__int2half_rn((s >> 6) * 64));
-        bm[b * 16 + 8 + j] = __half_as_ushort(__int2half_rn(s & 63));
-      }
+  a = __uint_as_float(__reduce_max_sync(PM_FULL, __float_as_uint(a)));  // (non-negative floats order like integers)
+  uint32_t w0, w1;
+  pm_q8_pack8(v, a != 0.0f ? __fdiv_rn(127.0f, a) : 0.0f, w0, w1);
+  *((uint2 *)(q + b * 256) + lane) = make_uint2(w0, w1);
+  int s = __dp4a((int)w1, 0x01010101, __dp4a((int)w0, 0x01010101, 0));
+  s += __shfl_xor_sync(PM_FULL, s, 1);
+  s += __shfl_xor_sync(PM_FULL, s, 2);
+  if ((lane & 3) == 0) {
+    const int j = lane >> 2;
+    bsum[b * 8 + j] = s;
+    if (bm) {  // s = 64 * (s >> 6) + (s & 63), both parts exact in f16
+      bm[b * 16 + j] = __half_as_ushort(__int2half_rn((s >> 6) * 64));
+      bm[b * 16 + 8 + j] = __half_as_ushort(__int2half_rn(s & 63));
     }
   }
+  const int tot = __reduce_add_sync(PM_FULL, (lane & 3) == 0 ? s : 0);
   if (lane == 0) {
     d[b] = a != 0.0f ? __fdiv_rn(a, 127.0f) : 0.0f;
     if (xs) xs[b] = tot;

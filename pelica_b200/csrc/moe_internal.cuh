@@ -1,6 +1,8 @@
 // moe_internal.cuh - device-side descriptions shared by the kernels and the C ABI.
 #pragma once
 
+#include <cuda.h>  // CUtensorMap
+
 #include "common.cuh"
 
 // One expert tensor family ([n_local experts][rows][cols]) in its device layout.
@@ -24,6 +26,15 @@ struct WMat {
   size_t stride[4];  // bytes per expert in each plane
 };
 
+// TMA descriptions of a family's planes as [expert][row][bytes of the row], boxes of 64 rows (gate, up) or 128 rows
+// (down) x one 256-value block (Q4_K: plane 0; Q6_K: ql, qh). Host memory of the layer: launchers copy them into parameters.
+struct WMaps {
+  CUtensorMap m[2];
+};
+struct LayerMaps {
+  WMaps gate, up, down, sgate, sup, sdown;
+};
+
 struct LayerDev {
   pm_layer_desc desc;
   int n_local, first_local;
@@ -35,6 +46,7 @@ struct LayerDev {
   WMat sgate, sup, sdown;                        // shared expert (1 "expert")
   const float *shared_gate_inp;                  // [d] or null
   uint32_t *usage;                               // [E]
+  const LayerMaps *maps;                         // host pointer
 };
 
 // pair_pos of a pair whose expert id was refused by the plan (combine reads a zero row)
@@ -135,21 +147,33 @@ void launch_gateup(const Launch &L, const LayerDev &ly, bool shared, Groups g, i
 void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int n_pairs,
                  const float *h, const int8_t *hq, const float *hd, const int32_t *hbsum,
                  float *eo);
-// tensor-core (tcgen05 int8) form of launch_gateup / launch_down for Q4_K x Q8x (prefill_tc.cu)
-// tile_buf: tc_tile_words(n_pairs, g.max_groups) words of scratch for the tile list; rec_buf:
-// tc_rec_bytes(n_pairs, g.max_groups, cols) bytes for the activation rows regrouped by expert in the
-// products' layout; src_row: row of xq / xd / xbm / xs that holds pair p (null: row p itself)
-int tc_max_tiles(int n_pairs, int max_groups);
+// tensor-core (tcgen05 int8) form of launch_gateup / launch_down for Q4_K / Q6_K x Q8x (prefill_tc.cu):
+// the token tiles of a grouping (one list serves both products), the activation rows regrouped by expert
+// in the products' layout (rec: tc_rec_bytes(n_pairs, max_groups, cols) bytes), the products.
+// src_row: row of the activations that holds pair p (null: row p itself)
+struct TcTiles {
+  int *n;              // [1] tiles
+  unsigned int *next;  // [2] item counters of the gate/up and the down launch (each list serves one of each)
+  uint4 *tiles;        // (expert slot or ~0, first pair, pairs, first record row)
+  uint32_t *group_r0;  // [512] first record row of a group
+  int ntok;            // tokens of a full tile (128, or 64 where the groups are small)
+  int max_tiles;
+};
 size_t tc_tile_words(int n_pairs, int max_groups);
+// n_groups: groups that can have pairs (the experts this GPU holds)
+TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups);  // buf: tc_tile_words words, 16-byte aligned
 size_t tc_rec_bytes(int n_pairs, int max_groups, int cols);
-cudaError_t launch_tc_q4k(const Launch &L, const LayerDev &ly, bool shared, bool down, Groups g,
-                          int n_pairs, uint32_t *tile_buf, uint8_t *rec_buf, const uint32_t *src_row,
-                          const int8_t *xq, const float *xd, const uint16_t *xbm, const int32_t *xs,
-                          const float *wts, float *out, int *err, unsigned long long wait_ns, int fault_block);
+void launch_tc_tiles(const Launch &L, const LayerDev &ly, bool shared, Groups g, const TcTiles &t);
+void launch_tc_quant_rows(const Launch &L, Groups g, int n_pairs, const TcTiles &t, const uint32_t *src_row, int cols,
+                          const float *x, uint8_t *rec);
+void launch_tc_rows(const Launch &L, Groups g, int n_pairs, const TcTiles &t, const uint32_t *src_row, int cols,
+                    const int8_t *xq, const float *xd, const uint16_t *xbm, const int32_t *xs, uint8_t *rec);
+cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared, bool down, Groups g, int n_pairs, const TcTiles &t,
+                      const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns, int fault_block);
 // tensor-core (tcgen05 bf16) form for MXFP4 weights and f32 activations given as their bf16
 // (hi, lo) split (prefill_mx.cu); launch_split_bf16 makes the split: hi[n], lo[n] bf16
 void launch_split_bf16(const Launch &L, const float *x, size_t n, void *hi, void *lo);
-cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, Groups g, int n_pairs, uint32_t *tile_buf,
+cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, Groups g, int n_pairs, const TcTiles &t,
                          const void *xhi, const void *xlo, const float *wts, float *out, int *err,
                          unsigned long long wait_ns);
 // expert parallelism (kernels_basic.cu): per-rank pair counts, the wire records of a dispatch,

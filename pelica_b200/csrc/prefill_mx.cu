@@ -154,23 +154,21 @@ struct MxArgs {
   int *err;
   unsigned long long wait_ns;
   const int *n_tiles;
-  const uint32_t *tile_group, *tile_n0;
+  const uint4 *tiles;
 };
 
 __global__ void __launch_bounds__(MX_NT, 1) k_tc_mx(const MxArgs A) {
   extern __shared__ __align__(128) uint8_t smem[];
   if ((int)blockIdx.y >= *A.n_tiles) return;
-  const int a = (int)A.tile_group[blockIdx.y];
+  const uint4 tile = A.tiles[blockIdx.y];
   const LayerDev &ly = A.ly;
   const WMat &W0 = A.down ? ly.down : ly.gate;
   const WMat &W1 = ly.up;
   const int cols = W0.cols, nb = cols / 32, rows = W0.rows;
   const int nkc = (cols + MX_KC - 1) / MX_KC;  // K chunks (the last one may hold a single block)
-  const int e = (int)A.g.expert[a];
-  const int el = e - ly.first_local;
-  const uint32_t off = A.g.offset[a], cnt = A.g.count[a];
-  const int n0 = (int)A.tile_n0[blockIdx.y];
-  const int nvalid = min((int)cnt - n0, MX_NMAX);
+  const int el = (int)tile.x;
+  const uint32_t first = tile.y;  // first pair
+  const int nvalid = (int)tile.z;
   const int npad = (nvalid + 15) & ~15;
   const int tid = threadIdx.x, warp = tid >> 5;
   const bool local = el >= 0 && el < ly.n_local;
@@ -180,7 +178,7 @@ __global__ void __launch_bounds__(MX_NT, 1) k_tc_mx(const MxArgs A) {
     if (A.down)
       for (int i = tid; i < nvalid * MX_M; i += MX_NT) {
         int n = i / MX_M, m = i % MX_M;
-        if (r0 + m < rows) A.out[(size_t)(off + n0 + n) * rows + r0 + m] = 0.0f;
+        if (r0 + m < rows) A.out[(size_t)(first + n) * rows + r0 + m] = 0.0f;
       }
     return;
   }
@@ -248,7 +246,7 @@ __global__ void __launch_bounds__(MX_NT, 1) k_tc_mx(const MxArgs A) {
 #pragma unroll
     for (int i = 0; i < 2; i++) {
       const int t = (tid >> 3) + 64 * i;
-      brow[i] = t < nvalid ? (A.down ? (int)(off + n0 + t) : (int)A.g.pair_token[off + n0 + t]) : -1;
+      brow[i] = t < nvalid ? (A.down ? (int)(first + t) : (int)A.g.pair_token[first + t]) : -1;
     }
     const int bc = tid & 7;
     // (through registers: 16-byte cp.async moves about 21 bytes a cycle per SM, a chunk's 32 KB of
@@ -400,7 +398,7 @@ __global__ void __launch_bounds__(MX_NT, 1) k_tc_mx(const MxArgs A) {
           if (i < ew && n < nvalid && rvalid) {
             float o = total[i];
             if (ly.bias_down) o = __fadd_rn(o, bd);
-            A.out[(size_t)(off + n0 + n) * rows + grow] = o;
+            A.out[(size_t)(first + n) * rows + grow] = o;
           }
         }
       }
@@ -421,7 +419,7 @@ __global__ void __launch_bounds__(MX_NT, 1) k_tc_mx(const MxArgs A) {
             gv = __fadd_rn(gv, ly.bias_gate[(size_t)el * rows + r0 + j]);
             uv = __fadd_rn(uv, ly.bias_up[(size_t)el * rows + r0 + j]);
           }
-          const uint32_t p = off + n0 + n;
+          const uint32_t p = first + n;
           const float w = fold ? A.wts[A.g.pair_src[p]] : 1.0f;
           A.out[(size_t)p * rows + r0 + j] = pm_act(D.act, D.act_limit, D.act_alpha, gv, uv, w, fold);
         }
@@ -433,19 +431,12 @@ __global__ void __launch_bounds__(MX_NT, 1) k_tc_mx(const MxArgs A) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)MX_TMEM_COLS) : "memory");
 }
 
-int tc_max_tiles(int n_pairs, int max_groups);
-void launch_tc_tiles(const Launch &L, Groups g, int *n_tiles, uint32_t *tile_group, uint32_t *tile_n0, int max_tiles);
-
 // Tensor-core form of launch_gateup / launch_down for MXFP4 weights and f32 activations given
 // as their bf16 (hi, lo) split.
-cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, Groups g, int n_pairs, uint32_t *tile_buf,
+cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, Groups g, int n_pairs, const TcTiles &t,
                          const void *xhi, const void *xlo, const float *wts, float *out, int *err,
                          unsigned long long wait_ns) {
   if (n_pairs == 0) return cudaSuccess;
-  const int max_tiles = tc_max_tiles(n_pairs, g.max_groups);
-  int *n_tiles = (int *)tile_buf;
-  uint32_t *tile_group = tile_buf + 4, *tile_n0 = tile_buf + 4 + max_tiles;
-  launch_tc_tiles(L, g, n_tiles, tile_group, tile_n0, max_tiles);
   const WMat &W = down ? ly.down : ly.gate;
   const size_t ex = (size_t)MX_M * (MX_NMAX + 1) * 4;
   const size_t smem = ((size_t)MX_ST * MX_STAGE > ex ? (size_t)MX_ST * MX_STAGE : ex) + 8 * (MX_ST + 1) + 16;
@@ -461,11 +452,10 @@ cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, Groups 
   A.out = out;
   A.err = err;
   A.wait_ns = wait_ns;
-  A.n_tiles = n_tiles;
-  A.tile_group = tile_group;
-  A.tile_n0 = tile_n0;
+  A.n_tiles = t.n;
+  A.tiles = t.tiles;
   const int row_tiles = down ? (W.rows + MX_M - 1) / MX_M : (W.rows + 63) / 64;
-  dim3 grid(row_tiles, max_tiles);
+  dim3 grid(row_tiles, t.max_tiles);
   k_tc_mx<<<grid, MX_NT, smem, L.stream>>>(A);
   if (L.count) ++*L.count;
   return cudaGetLastError();
