@@ -89,7 +89,10 @@ struct pm_ctx {
   bool own_stream = true;
   int *dev_err = nullptr;   // error word of kernels with bounded waits
   unsigned int *route_ticket = nullptr;  // [1] zero between launches: the few-token routing kernel's last-CTA ticket
-  int tc_min_tokens = 32;   // tensor-core expert products from this many tokens (the reference's TC_MIN, src/moe.rs:35); 0 = never
+  // Tensor-core expert products from this many tokens (the reference's TC_MIN, src/moe.rs:35); 0 = never. Until the
+  // caller sets it, the exact integer products take fewer (see int_tc_min): they give the same bits either way.
+  int tc_min_tokens = 32;
+  bool tc_min_set = false;
   int64_t launches = 0;
   int64_t path_count[PM_PATH_N] = {0, 0, 0, 0};  // launches per expert-product path (pelica_moe_diag.h)
   unsigned long long wait_ns = 2000000000ull;    // limit of every bounded device-side wait
@@ -271,6 +274,7 @@ extern "C" int32_t pm_sync(pm_ctx *c) {
 extern "C" int32_t pm_ctx_set_tensor_core_min_tokens(pm_ctx *c, int32_t min_tokens) {
   if (!c || min_tokens < 0) return fail(PM_ERR_INVALID, "pm_ctx_set_tensor_core_min_tokens");
   c->tc_min_tokens = min_tokens;
+  c->tc_min_set = true;
   return PM_OK;
 }
 extern "C" int32_t pm_stack_destroy(pm_stack *s);
@@ -828,6 +832,7 @@ struct Scratch {
   float *eo;
   uint16_t *xhl, *hhl;  // MXFP4 tensor-core path: bf16 (hi, lo) split of x [2][T*d] and of h [2][P*ff]
   uint32_t *tiles;  // tile list of the tensor-core kernels
+  uint32_t *seg;    // per-segment counts of the plan
   uint8_t *rec;     // activation rows regrouped into the int8 tensor-core kernel's records
   // shared expert
   int *one; uint32_t *zero_u, *tcount, *iota;
@@ -835,10 +840,13 @@ struct Scratch {
   float *shared_out, *shared_logit;
 };
 
+// whether the shared expert can run as one more group of the routed experts' tensor-core launches
+static bool shared_merges(const pm_layer_desc &D) { return D.shared && D.shared_ff == D.ff && D.act_quant == PM_AQ_Q8X_256; }
+
 // the largest record buffer any tensor-core launch of a T-token call needs (Q8x activations only)
 static size_t scratch_rec_bytes(const pm_layer_desc &D, int T) {
   if (D.act_quant != PM_AQ_Q8X_256) return 0;
-  const int P = T * D.top_k, E = D.n_exp;
+  const int m = shared_merges(D) ? 1 : 0, P = T * (D.top_k + m), E = D.n_exp + m;
   size_t r = std::max(tc_rec_bytes(P, E, D.d), tc_rec_bytes(P, E, D.ff));
   if (D.shared) r = std::max(r, std::max(tc_rec_bytes(T, 1, D.d), tc_rec_bytes(T, 1, D.shared_ff)));
   return r;
@@ -848,12 +856,14 @@ static size_t scratch_bytes(const pm_layer_desc &D, int T) {
   size_t P = (size_t)T * D.top_k, E = (size_t)D.n_exp, d = (size_t)D.d, ff = (size_t)D.ff;
   size_t b = 0;
   b += al(T * E * 4) + al(P * 4) * 2;                  // logits, ids, w
-  b += al(4) + al(E * 4) * 5 + al(P * 4) * 3;          // plan
+  b += al(4) + al((E + 1) * 4) * 5 + al((P + T) * 4) * 3;  // plan
+  b += al(route_seg_words(T, D.n_exp) * 4);
   b += al(T * d) + al(T * (d / 32 + 1) * 4) + al(T * (d / 256 + 1) * 4) + al(T * (d / 32) * 4) * 2;
-  b += al(P * ff * 4) + al(P * ff) + al(P * (ff / 32 + 1) * 4) + al(P * (ff / 256 + 1) * 4) + al(P * (ff / 32) * 4) * 2;
-  b += al(P * d * 4);
+  const size_t Pm = P + (shared_merges(D) ? T : 0);    // pairs with the shared expert's
+  b += al(Pm * ff * 4) + al(P * ff) + al(P * (ff / 32 + 1) * 4) + al(P * (ff / 256 + 1) * 4) + al(P * (ff / 32) * 4) * 2;
+  b += al(Pm * d * 4);
   if (D.act_quant == PM_AQ_F32 && D.type_gate == PM_TYPE_MXFP4) b += al(T * d * 4) + al(P * ff * 4);
-  b += al(tc_tile_words((int)(P > (size_t)T ? P : (size_t)T), (int)E + 1) * 4);
+  b += al(tc_tile_words((int)P + T, (int)E + 1) * 4);
   b += al(scratch_rec_bytes(D, T));
   if (D.shared) {
     size_t sf = (size_t)D.shared_ff;
@@ -870,12 +880,12 @@ static void scratch_carve(pm_ctx *c, const pm_layer_desc &D, int T, Scratch &S) 
   S.ids = ws_take<uint32_t>(c, P);
   S.w = ws_take<float>(c, P);
   S.plan.n_active = ws_take<int>(c, 1);
-  S.plan.active = ws_take<uint32_t>(c, E);
-  S.plan.offset = ws_take<uint32_t>(c, E);
-  S.plan.count = ws_take<uint32_t>(c, E);
-  S.plan.base = ws_take<uint32_t>(c, E);
-  S.plan.cnt = ws_take<uint32_t>(c, E);
-  S.plan.pair_token = ws_take<uint32_t>(c, P);
+  S.plan.active = ws_take<uint32_t>(c, E + 1);
+  S.plan.offset = ws_take<uint32_t>(c, E + 1);
+  S.plan.count = ws_take<uint32_t>(c, E + 1);
+  S.plan.base = ws_take<uint32_t>(c, E + 1);
+  S.plan.cnt = ws_take<uint32_t>(c, E + 1);
+  S.plan.pair_token = ws_take<uint32_t>(c, P + T);  // (and the shared expert's tokens)
   S.plan.pair_pos = ws_take<uint32_t>(c, P);
   S.plan.pair_src = ws_take<uint32_t>(c, P);
   S.xq = ws_take<int8_t>(c, T * d);
@@ -883,19 +893,21 @@ static void scratch_carve(pm_ctx *c, const pm_layer_desc &D, int T, Scratch &S) 
   S.xbsum = ws_take<int32_t>(c, T * (d / 32));
   S.xbm = ws_take<uint16_t>(c, T * (d / 16));
   S.xs = ws_take<int32_t>(c, T * (d / 256 + 1));
-  S.h = ws_take<float>(c, P * ff);
+  const size_t Pm = P + (shared_merges(D) ? T : 0);
+  S.h = ws_take<float>(c, Pm * ff);
   S.hq = ws_take<int8_t>(c, P * ff);
   S.hd = ws_take<float>(c, P * (ff / 32 + 1));
   S.hbsum = ws_take<int32_t>(c, P * (ff / 32));
   S.hbm = ws_take<uint16_t>(c, P * (ff / 16));
   S.hs = ws_take<int32_t>(c, P * (ff / 256 + 1));
-  S.eo = ws_take<float>(c, P * d);
+  S.eo = ws_take<float>(c, Pm * d);
   S.xhl = S.hhl = nullptr;
   if (D.act_quant == PM_AQ_F32 && D.type_gate == PM_TYPE_MXFP4) {
     S.xhl = ws_take<uint16_t>(c, 2 * T * d);
     S.hhl = ws_take<uint16_t>(c, 2 * P * ff);
   }
-  S.tiles = ws_take<uint32_t>(c, tc_tile_words((int)(P > (size_t)T ? P : (size_t)T), (int)E + 1));
+  S.tiles = ws_take<uint32_t>(c, tc_tile_words((int)P + T, (int)E + 1));
+  S.seg = ws_take<uint32_t>(c, route_seg_words(T, D.n_exp));
   S.rec = ws_take<uint8_t>(c, scratch_rec_bytes(D, T));
   if (D.shared) {
     size_t sf = (size_t)D.shared_ff;
@@ -929,30 +941,58 @@ static Groups plan_groups(const PlanDev &pl, int E) {
   return g;
 }
 
-// routed experts: x (and its Q8x form) -> eo[P][d]
+// which kernels serve the expert products of a T-token call
+struct Path {
+  bool tc, tc_gu;  // int8 tensor-core products (both; gate/up needs one type for the two matrices)
+  bool mx;         // bf16 tensor-core products for MXFP4 weights and f32 activations (tolerance parity, not bits)
+  bool merge;      // the shared expert is one more group of the routed experts' launches
+};
+static Path pick_path(pm_layer *ly, int T, const Scratch &S) {
+  const pm_ctx *c = ly->ctx;
+  const pm_layer_desc &D = ly->dev.desc;
+  Path p;
+  // The integer products give the same bits on either path, so until the caller sets the threshold the faster one
+  // decides: two tokens up (one token, 8 experts x 2048 x 1024: 27 us on both; 8 tokens of a 7168-wide layer: 453 us
+  // on the row kernels, 323 us on the tensor cores), and one where the shared expert joins the launch.
+  const int int_min = c->tc_min_set ? c->tc_min_tokens : (shared_merges(D) ? 1 : 2);
+  p.tc = D.act_quant == PM_AQ_Q8X_256 && c->tc_min_tokens > 0 && T >= int_min;
+  p.tc_gu = p.tc && D.type_gate == D.type_up;
+  p.mx = c->tc_min_tokens > 0 && T >= c->tc_min_tokens && D.act_quant == PM_AQ_F32 && D.type_gate == PM_TYPE_MXFP4 &&
+         D.type_up == PM_TYPE_MXFP4 && D.type_down == PM_TYPE_MXFP4 && S.xhl;
+  p.merge = p.tc_gu && shared_merges(D);
+  return p;
+}
+static TcTiles path_tiles(pm_layer *ly, int T, const Path &p, const Scratch &S, bool merge) {
+  const pm_layer_desc &D = ly->dev.desc;
+  TcTiles t{};
+  if (p.tc || p.mx)
+    t = tc_tiles_of(S.tiles, T * D.top_k, D.n_exp, p.mx ? 1 : std::min(D.n_exp, ly->dev.n_local), merge ? T : 0);
+  return t;
+}
+
+// routed experts: x (and its Q8x form) -> eo[P][d] (and, tt->shared, the shared expert's rows behind them)
 // prequant: S.xq / S.xd / S.xbsum (and their derived forms) already hold the rows' quantised
-// form (rows received from another rank arrive quantised)
-static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, const float *w, bool prequant = false) {
+// form (rows received from another rank arrive quantised); tt: the tile list the plan's kernels made, or null
+static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, const float *w, bool prequant, const TcTiles *made) {
   pm_ctx *c = ly->ctx;
   const LayerDev &dv = ly->dev;
   const pm_layer_desc &D = dv.desc;
   Launch L = c->launch();
-  int P = T * D.top_k;
+  const Path path = pick_path(ly, T, S);
+  const bool tc = path.tc, tc_gu = path.tc_gu;
   Groups g = plan_groups(S.plan, D.n_exp);
+  const int P = T * D.top_k;
   const bool q8 = D.act_quant == PM_AQ_Q8X_256, f16s = D.act_quant == PM_AQ_Q8_32_F16;
   const bool q32 = D.act_quant == PM_AQ_Q8_32 || f16s;
-  const bool many = c->tc_min_tokens > 0 && T >= c->tc_min_tokens;
-  const bool tc = q8 && many, tc_gu = tc && D.type_gate == D.type_up;
-  // MXFP4 weights with f32 activations: the bf16 tensor-core kernels (tolerance parity, not bits)
-  const bool tcmx = many && D.act_quant == PM_AQ_F32 && D.type_gate == PM_TYPE_MXFP4 && D.type_up == PM_TYPE_MXFP4 &&
-                    D.type_down == PM_TYPE_MXFP4 && S.xhl;
   TcTiles tt{};
-  if (tc || tcmx) {
+  if (made) {
+    tt = *made;
+  } else if (tc || path.mx) {
     PROF(c, PH_PLAN);
-    tt = tc_tiles_of(S.tiles, P, g.max_groups, tcmx ? 1 : std::min(D.n_exp, dv.n_local));
-    launch_tc_tiles(L, dv, false, g, tt);
+    tt = path_tiles(ly, T, path, S, false);
+    launch_tc_tiles(L, dv, g, tt);
   }
-  if (tcmx) {
+  if (path.mx) {
     const size_t nx = (size_t)T * D.d, nh = (size_t)P * D.ff;
     {
       PROF(c, PH_QUANT_X);
@@ -974,14 +1014,16 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
     CU(cudaGetLastError());
     return PM_OK;
   }
+  const int Pr = P + (tt.shared ? T : 0);  // rows of the products
+  if (tt.shared) g.max_groups = D.n_exp + 1;
   {
     PROF(c, PH_QUANT_X);
     if (tc_gu) {
       // (many rows: quantise every token once and gather the quantised rows, see k_tc_quant_rows)
       const bool gather = prequant || (size_t)P * D.d > ((size_t)8 << 20);
       if (gather && !prequant) launch_quant_q8x(L, x, (size_t)T, D.d, S.xq, S.xd, S.xbsum, S.xbm, S.xs);
-      if (gather) launch_tc_rows(L, g, P, tt, g.pair_token, D.d, S.xq, S.xd, S.xbm, S.xs, S.rec);
-      else launch_tc_quant_rows(L, g, P, tt, g.pair_token, D.d, x, S.rec);
+      if (gather) launch_tc_rows(L, g, Pr, tt, g.pair_token, D.d, S.xq, S.xd, S.xbm, S.xs, S.rec);
+      else launch_tc_quant_rows(L, g, Pr, tt, g.pair_token, D.d, x, S.rec);
     } else if (q8 && !prequant) {
       launch_quant_q8x(L, x, (size_t)T, D.d, S.xq, S.xd, S.xbsum);
     } else if (q32 && !prequant) {
@@ -991,7 +1033,7 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
   {
     PROF(c, PH_GATEUP);
     if (tc_gu) {
-      CU(launch_tc(L, dv, false, false, g, P, tt, S.rec, w, S.h, c->dev_err, c->wait_ns, c->tc_fault_block));
+      CU(launch_tc(L, dv, false, false, g.pair_src, tt, S.rec, w, S.h, c->dev_err, c->wait_ns, c->tc_fault_block));
       c->path_count[PM_PATH_TENSOR]++;
     } else {
       launch_gateup(L, dv, false, g, P, x, S.xq, S.xd, S.xbsum, w, S.h);
@@ -1000,14 +1042,14 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
   }
   {
     PROF(c, PH_QUANT_H);
-    if (tc) launch_tc_quant_rows(L, g, P, tt, nullptr, D.ff, S.h, S.rec);
+    if (tc) launch_tc_quant_rows(L, g, Pr, tt, nullptr, D.ff, S.h, S.rec);
     else if (q8) launch_quant_q8x(L, S.h, (size_t)P, D.ff, S.hq, S.hd, S.hbsum);
     else if (q32) launch_quant_q8_32(L, S.h, (size_t)P, D.ff, S.hq, S.hd, f16s);
   }
   {
     PROF(c, PH_DOWN);
     if (tc) {
-      CU(launch_tc(L, dv, false, true, g, P, tt, S.rec, nullptr, S.eo, c->dev_err, c->wait_ns, c->tc_fault_block));
+      CU(launch_tc(L, dv, false, true, g.pair_src, tt, S.rec, nullptr, S.eo, c->dev_err, c->wait_ns, c->tc_fault_block));
       c->path_count[PM_PATH_TENSOR]++;
     } else {
       launch_down(L, dv, false, g, P, S.h, S.hq, S.hd, S.hbsum, S.eo);
@@ -1018,7 +1060,14 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
   return PM_OK;
 }
 
-// shared expert over every token -> S.shared_out (and the gate logit)
+static int32_t shared_gate(pm_layer *ly, const float *x, int T, Scratch &S) {
+  if (ly->dev.desc.shared == PM_SHARED_SIGMOID_GATED) launch_shared_gate_logit(ly->ctx->launch(), ly->dev, x, T, S.shared_logit);
+  else S.shared_logit = nullptr;
+  CU(cudaGetLastError());
+  return PM_OK;
+}
+
+// shared expert over every token -> S.shared_out (and the gate logit), in launches of its own
 static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
   pm_ctx *c = ly->ctx;
   const LayerDev &dv = ly->dev;
@@ -1026,12 +1075,11 @@ static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
   if (!D.shared) return PM_OK;
   PROF(c, PH_SHARED);
   Launch L = c->launch();
-  const int one = 1;
-  const uint32_t zero = 0, tc = (uint32_t)T;
-  CU(cudaMemcpyAsync(S.one, &one, 4, cudaMemcpyHostToDevice, c->stream));
-  CU(cudaMemcpyAsync(S.zero_u, &zero, 4, cudaMemcpyHostToDevice, c->stream));
-  CU(cudaMemcpyAsync(S.tcount, &tc, 4, cudaMemcpyHostToDevice, c->stream));
-  launch_iota(L, S.iota, (uint32_t)T);
+  const Path path = pick_path(ly, T, S);
+  const bool use_tc = path.tc, tc_gu = path.tc_gu;
+  TcTiles tt{};
+  if (use_tc) tt = tc_tiles_of(S.tiles, T, 1, 1, 0);
+  launch_shared_groups(L, S.one, S.zero_u, S.tcount, S.iota, T, tt);
   Groups g;
   g.n_groups = S.one;
   g.expert = S.zero_u;
@@ -1042,15 +1090,9 @@ static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
   g.max_groups = 1;
   const bool q8 = D.act_quant == PM_AQ_Q8X_256, f16s = D.act_quant == PM_AQ_Q8_32_F16;
   const bool q32 = D.act_quant == PM_AQ_Q8_32 || f16s;
-  const bool use_tc = q8 && c->tc_min_tokens > 0 && T >= c->tc_min_tokens, tc_gu = use_tc && D.type_gate == D.type_up;
-  TcTiles tt{};
-  if (use_tc) {
-    tt = tc_tiles_of(S.tiles, T, 1, 1);
-    launch_tc_tiles(L, dv, true, g, tt);
-  }
   if (tc_gu) {
     launch_tc_quant_rows(L, g, T, tt, nullptr, D.d, x, S.rec);
-    CU(launch_tc(L, dv, true, false, g, T, tt, S.rec, nullptr, S.sh, c->dev_err, c->wait_ns, c->tc_fault_block));
+    CU(launch_tc(L, dv, true, false, nullptr, tt, S.rec, nullptr, S.sh, c->dev_err, c->wait_ns, c->tc_fault_block));
   } else {
     if (q8) launch_quant_q8x(L, x, (size_t)T, D.d, S.xq, S.xd, S.xbsum);
     if (q32) launch_quant_q8_32(L, x, (size_t)T, D.d, S.xq, S.xd, f16s);
@@ -1058,16 +1100,13 @@ static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
   }
   if (use_tc) {
     launch_tc_quant_rows(L, g, T, tt, nullptr, D.shared_ff, S.sh, S.rec);
-    CU(launch_tc(L, dv, true, true, g, T, tt, S.rec, nullptr, S.shared_out, c->dev_err, c->wait_ns, c->tc_fault_block));
+    CU(launch_tc(L, dv, true, true, nullptr, tt, S.rec, nullptr, S.shared_out, c->dev_err, c->wait_ns, c->tc_fault_block));
   } else {
     if (q8) launch_quant_q8x(L, S.sh, (size_t)T, D.shared_ff, S.shq, S.shd, S.shbsum);
     if (q32) launch_quant_q8_32(L, S.sh, (size_t)T, D.shared_ff, S.shq, S.shd, f16s);
     launch_down(L, dv, true, g, T, S.sh, S.shq, S.shd, S.shbsum, S.shared_out);
   }
-  if (D.shared == PM_SHARED_SIGMOID_GATED) launch_shared_gate_logit(L, dv, x, T, S.shared_logit);
-  else S.shared_logit = nullptr;
-  CU(cudaGetLastError());
-  return PM_OK;
+  return shared_gate(ly, x, T, S);
 }
 
 // the whole layer on device pointers (workspace already reserved and carved)
@@ -1076,19 +1115,26 @@ static int32_t dev_forward(pm_layer *ly, const float *x, int T, float *y, bool a
   pm_ctx *c = ly->ctx;
   const LayerDev &dv = ly->dev;
   Launch L = c->launch();
-  if (T < PM_SMALL_ROUTE_TOKENS) {  // a few tokens: logits, top-k and plan in one launch
+  const Path path = pick_path(ly, T, S);
+  const TcTiles tt = path_tiles(ly, T, path, S, path.merge);
+  if (route_plan_small_takes(dv, x, T)) {  // a few tokens: logits, top-k, plan and tiles in one launch
     PROF(c, PH_ROUTER);
-    launch_route_plan_small(L, dv, x, T, S.logits, S.ids, S.w, S.plan, nullptr, c->route_ticket);
+    launch_route_plan_small(L, dv, x, T, S.logits, S.ids, S.w, S.plan, nullptr, c->route_ticket, tt, c->dev_err, c->wait_ns);
   } else {
     { PROF(c, PH_ROUTER); launch_router(L, dv, x, T, S.logits); }
-    { PROF(c, PH_ROUTE); launch_route(L, dv, S.logits, T, S.ids, S.w); }
-    { PROF(c, PH_PLAN); launch_plan(L, dv, S.ids, T, S.plan, c->dev_err); }
+    { PROF(c, PH_ROUTE); launch_route_plan(L, dv, S.logits, T, S.ids, S.w, S.plan, S.seg, tt); }
   }
-  TRY(dev_experts(ly, x, T, S, S.w));
-  TRY(dev_shared(ly, x, T, S));
+  TRY(dev_experts(ly, x, T, S, S.w, false, path.tc || path.mx ? &tt : nullptr));
+  const float *shared_out = S.shared_out;
+  if (path.merge) {
+    shared_out = S.eo + (size_t)T * dv.desc.top_k * dv.desc.d;
+    TRY(shared_gate(ly, x, T, S));
+  } else {
+    TRY(dev_shared(ly, x, T, S));
+  }
   {
     PROF(c, PH_COMBINE);
-    launch_combine(L, dv, S.eo, S.plan.pair_pos, S.w, S.shared_out, S.shared_logit, T, y, accumulate);
+    launch_combine(L, dv, S.eo, S.plan.pair_pos, S.w, shared_out, S.shared_logit, T, y, accumulate);
   }
   CU(cudaGetLastError());
   return PM_OK;
@@ -1102,12 +1148,13 @@ static int32_t check_T(int32_t T) {
 // host-or-device input -> device pointer (staged in the workspace when host)
 template <typename T>
 static int32_t in_dev(pm_ctx *c, const T *p, size_t n, const T **out) {
-  if (is_device_ptr(p)) {
+  // (the kernels read 16 bytes at a time: a device buffer that starts elsewhere is copied as well)
+  if (is_device_ptr(p) && ((uintptr_t)p & 15) == 0) {
     *out = p;
     return PM_OK;
   }
   T *t = ws_take<T>(c, n);
-  CU(cudaMemcpyAsync(t, p, n * sizeof(T), cudaMemcpyHostToDevice, c->stream));
+  CU(cudaMemcpyAsync(t, p, n * sizeof(T), cudaMemcpyDefault, c->stream));
   *out = t;
   return PM_OK;
 }
@@ -1330,7 +1377,7 @@ extern "C" int32_t pm_experts(pm_layer *ly, const float *x, int32_t T, const uin
   LayerDev tmp = ly->dev;
   tmp.usage = nullptr;
   launch_plan(c->launch(), tmp, idd, T, S.plan, c->dev_err);
-  TRY(dev_experts(ly, xd, T, S, wd));
+  TRY(dev_experts(ly, xd, T, S, wd, false, nullptr));
   CU(cudaMemcpyAsync(pair_out, S.eo, P * D.d * 4, cudaMemcpyDefault, c->stream));
   CU(cudaStreamSynchronize(c->stream));
   return check_dev_err(c);
@@ -1366,7 +1413,7 @@ extern "C" int32_t pm_experts_rows(pm_layer *ly, const float *x, int32_t R, cons
   view.dev.desc = D;
   view.dev.usage = nullptr;
   { PROF(c, PH_PLAN); launch_plan(c->launch(), view.dev, idd, R, S.plan, c->dev_err); }
-  TRY(dev_experts(&view, xd, R, S, wd));
+  TRY(dev_experts(&view, xd, R, S, wd, false, nullptr));
   LayerDev cp = view.dev;
   cp.desc.weight_fold = PM_FOLD_BEFORE_DOWN;  // plain gather back to row order
   launch_combine(c->launch(), cp, S.eo, S.plan.pair_pos, wd, nullptr, nullptr, R, od, false);
@@ -2161,18 +2208,24 @@ extern "C" int32_t pm_moe_forward_ep(pm_ep *ep, pm_layer *ly, const float *x, in
 
   // ---- this rank's tokens: route, plan, counts ----
   TRY(ws_reserve(c, scratch_bytes(D, T > 0 ? T : 1) + al(P * row_bytes) + al(P * (nd + 1) * 4) + al(P * (nbs + 1) * 4) +
-                        al(P * 8) + 4096));
+                        al(P * 8) + al((size_t)T * d * 4) + 4096));
   Scratch S;
   scratch_carve(c, D, T > 0 ? T : 1, S);
   uint8_t *srows = ws_take<uint8_t>(c, P * row_bytes);
   float *sd = ws_take<float>(c, P * (size_t)(nd + 1));
   int32_t *sbs = ws_take<int32_t>(c, P * (size_t)(nbs + 1));
   uint32_t *smeta = ws_take<uint32_t>(c, P * 2);
-  if (T > 0 && T < PM_SMALL_ROUTE_TOKENS) {  // a few tokens: logits, top-k, (slots) and plan in one launch
+  const float *x_in = x;
+  if (T > 0 && ((uintptr_t)x & 15)) {  // (the kernels read 16 bytes at a time)
+    float *xa = ws_take<float>(c, (size_t)T * d);
+    CU(cudaMemcpyAsync(xa, x_in, (size_t)T * d * 4, cudaMemcpyDeviceToDevice, c->stream));
+    x = xa;
+  }
+  if (route_plan_small_takes(dv, x, T)) {  // a few tokens: logits, top-k, (slots) and plan in one launch
     auto st = ep->slots.find(ly);
     PROF(c, PH_ROUTER);
     launch_route_plan_small(L, dv, x, T, S.logits, S.ids, S.w, S.plan, st != ep->slots.end() ? st->second.dev : nullptr,
-                            c->route_ticket);
+                            c->route_ticket, TcTiles{}, c->dev_err, c->wait_ns);
   } else {
     if (T > 0) {
       { PROF(c, PH_ROUTER); launch_router(L, dv, x, T, S.logits); }
@@ -2289,7 +2342,7 @@ extern "C" int32_t pm_moe_forward_ep(pm_ep *ep, pm_layer *ly, const float *x, in
     view.dev.desc = D1;
     view.dev.usage = nullptr;
     { PROF(c, PH_PLAN); launch_plan(L, view.dev, reid, (int)R, RS.plan, c->dev_err); }
-    TRY(dev_experts(&view, q8 ? nullptr : (const float *)rrows, (int)R, RS, rw, q8));
+    TRY(dev_experts(&view, q8 ? nullptr : (const float *)rrows, (int)R, RS, rw, q8, nullptr));
     LayerDev cp = view.dev;
     cp.desc.weight_fold = PM_FOLD_BEFORE_DOWN;  // plain gather back to row order
     launch_combine(L, cp, RS.eo, RS.plan.pair_pos, rw, nullptr, nullptr, (int)R, orows, false);

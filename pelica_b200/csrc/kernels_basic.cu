@@ -384,79 +384,107 @@ __global__ void __launch_bounds__(256) k_router(const float *__restrict__ wr,
   }
 }
 
-// The same sums for many tokens: a warp owns EXP experts x TOK tokens (TOK * EXP accumulators a
-// lane), a CTA 8 * EXP experts x TOK tokens; the tokens' columns are staged in shared memory
-// 512 at a time. Lane L still runs, for every (token, expert), the fma chain over columns
-// L, L+32, ... in ascending order, so the result has the bits of k_router; the router
-// row is read once per TOK tokens instead of once per token.
-// 8 x 8 tiles have the fewest loads per fma (a 4096-token call on 256 experts is 2048 CTAs). While
-// such a grid does not even fill the SMs (512 tokens on 128 experts: 128 CTAs of 8 warps, every
-// column an L2 round trip that nothing hides) 4 x 4 tiles give four times the CTAs at a quarter of
-// the registers, several CTAs an SM, with UNROLL columns' router loads in flight together
-// (512 tokens on 128 experts: 45 -> 29 us a call).
-#define RT_CH 512
-template <int TOK, int EXP, int UNROLL>
-__global__ void __launch_bounds__(256) k_router_tile(const float *__restrict__ wr,
-                                                     const float *__restrict__ bias,
-                                                     const float *__restrict__ x, int T, int E, int d,
-                                                     float *logits) {
-  __shared__ float xs[TOK][RT_CH];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int t0 = blockIdx.y * TOK, e0 = blockIdx.x * (8 * EXP) + warp * EXP;
-  float acc[TOK][EXP];
+// The same sums for many tokens. A CTA of 8 warps owns 2 EW experts x 4 TW tokens, a warp EW x TW of them
+// (EW * TW accumulators a lane); 128 columns of its experts' and tokens' rows at a time come into shared memory
+// by cp.async, three stages. Lane L still runs, for every (token, expert), the fma chain over columns L,
+// L + 32, ... in ascending order, so the result has the bits of k_router.
+// 16 x 8 (128 fma for 24 shared-memory reads a column): bound by the FP32 pipe. 8 x 4 while tiles of the first size
+// would leave most SMs without one.
+// (before: rows from L2 straight into the fma, 8 x 8 tiles: 4096 tokens on 256 experts x 7168 916 us, the pipe's bound
+// 210 us; 64 tokens 75 us; 512 tokens on 128 experts x 2048 29 us)
+#define RT_CH 128
+#define RT_ST 3
+template <int EW, int TW> __global__ void __launch_bounds__(256, 1) k_router_tile(const float *__restrict__ wr,
+                                                                                 const float *__restrict__ bias,
+                                                                                 const float *__restrict__ x, int T, int E,
+                                                                                 int d, float *logits) {
+  constexpr int RE = 2 * EW, RT = 4 * TW, ROWS = RE + RT;  // rows of a stage: experts, then tokens
+  extern __shared__ __align__(16) float rs[];              // [RT_ST][ROWS][RT_CH]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int e0 = blockIdx.x * RE, t0 = blockIdx.y * RT;
+  const int we = (warp & 1) * EW, wt = (warp >> 1) * TW;
+  const int nch = (d + RT_CH - 1) / RT_CH;
+  auto load = [&](int ch) {  // a warp a row: 32 pieces of 16 bytes (rows past the end repeat the last one)
+    if (ch < nch) {
+      const int c = ch * RT_CH + 4 * lane;
+      float *dst = rs + (size_t)(ch % RT_ST) * ROWS * RT_CH + 4 * lane;
+      if (c < d)
 #pragma unroll
-  for (int t = 0; t < TOK; t++)
-#pragma unroll
-    for (int e = 0; e < EXP; e++) acc[t][e] = 0.0f;
-  for (int c0 = 0; c0 < d; c0 += RT_CH) {
-    const int n = min(RT_CH, d - c0);  // a multiple of 32 (d is)
-    __syncthreads();
-    for (int i = threadIdx.x; i < TOK * RT_CH; i += 256) {
-      const int t = i / RT_CH, c = i - t * RT_CH;
-      xs[t][c] = (t0 + t < T && c < n) ? x[(size_t)(t0 + t) * d + c0 + c] : 0.0f;
+        for (int r = warp; r < ROWS; r += 8) {
+          const float *src = r < RE ? wr + (size_t)min(e0 + r, E - 1) * d + c : x + (size_t)min(t0 + r - RE, T - 1) * d + c;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * RT_CH)), "l"(src) : "memory");
+        }
     }
-    __syncthreads();
-    if (e0 < E) {
-#pragma unroll UNROLL
-      for (int c = lane; c < n; c += 32) {
-        float w[EXP], xv[TOK];
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float acc[TW][EW];
 #pragma unroll
-        for (int e = 0; e < EXP; e++) w[e] = e0 + e < E ? __ldg(wr + (size_t)(e0 + e) * d + c0 + c) : 0.0f;
+  for (int t = 0; t < TW; t++)
 #pragma unroll
-        for (int t = 0; t < TOK; t++) xv[t] = xs[t][c];
+    for (int e = 0; e < EW; e++) acc[t][e] = 0.0f;
 #pragma unroll
-        for (int t = 0; t < TOK; t++)
+  for (int ch = 0; ch < RT_ST - 1; ch++) load(ch);
+  for (int ch = 0; ch < nch; ch++) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(RT_ST - 2) : "memory");
+    __syncthreads();  // chunk ch is here, and everybody is done with chunk ch - 1, whose stage the next load takes
+    load(ch + RT_ST - 1);
+    const float *S = rs + (size_t)(ch % RT_ST) * ROWS * RT_CH + lane;
+    const int n = min(RT_CH, d - ch * RT_CH) / 32;  // (d is a multiple of 32)
+    for (int s = 0; s < n; s++) {
+      float w[EW], xv[TW];
 #pragma unroll
-          for (int e = 0; e < EXP; e++) acc[t][e] = __fmaf_rn(w[e], xv[t], acc[t][e]);
-      }
+      for (int e = 0; e < EW; e++) w[e] = S[(we + e) * RT_CH + 32 * s];
+#pragma unroll
+      for (int t = 0; t < TW; t++) xv[t] = S[(RE + wt + t) * RT_CH + 32 * s];
+#pragma unroll
+      for (int t = 0; t < TW; t++)
+#pragma unroll
+        for (int e = 0; e < EW; e++) acc[t][e] = __fmaf_rn(w[e], xv[t], acc[t][e]);
     }
   }
-  if (e0 >= E) return;
+  // lane sums in pm_warp_sum_dot's order (xor 8, 16, 4, 2, 1), 32 of them at once: every step halves the sums a lane
+  // carries, 31 shuffles in place of 160; lane L ends with sum (bit 3, bit 4, bit 2, bit 1, bit 0 of L)
+  const int idx = ((lane >> 3) & 1) * 16 + ((lane >> 4) & 1) * 8 + (lane & 7);
 #pragma unroll
-  for (int t = 0; t < TOK; t++)
+  for (int b = 0; b < EW * TW / 32; b++) {
+    float v[32];
 #pragma unroll
-    for (int e = 0; e < EXP; e++) {
-      float s = pm_warp_sum_dot(acc[t][e]);
-      if (lane == 0 && t0 + t < T && e0 + e < E) {
-        if (bias) s = __fadd_rn(s, bias[e0 + e]);
-        logits[(size_t)(t0 + t) * E + e0 + e] = s;
+    for (int i = 0; i < 32; i++) v[i] = acc[(32 * b + i) / EW][(32 * b + i) % EW];
+    const int masks[5] = {8, 16, 4, 2, 1};
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+      const int half = 16 >> k;
+      const bool up = lane & masks[k];
+#pragma unroll
+      for (int i = 0; i < half; i++) {
+        const float keep = up ? v[i + half] : v[i], send = up ? v[i] : v[i + half];
+        v[i] = __fadd_rn(keep, __shfl_xor_sync(PM_FULL, send, masks[k]));
       }
     }
+    const int o = 32 * b + idx, t = t0 + wt + o / EW, e = e0 + we + o % EW;
+    if (t < T && e < E) logits[(size_t)t * E + e] = bias ? __fadd_rn(v[0], bias[e]) : v[0];
+  }
+}
+
+template <int EW, int TW>
+static void start_router_tile(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits) {
+  const int E = ly.desc.n_exp, d = ly.desc.d;
+  constexpr size_t smem = (size_t)RT_ST * (2 * EW + 4 * TW) * RT_CH * 4;
+  static bool set = false;  // (of every device: the attribute belongs to the function)
+  if (smem > 48 * 1024 && !set) {
+    cudaFuncSetAttribute(k_router_tile<EW, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    set = true;
+  }
+  const dim3 grid((E + 2 * EW - 1) / (2 * EW), (T + 4 * TW - 1) / (4 * TW));
+  KLAUNCH(L, (k_router_tile<EW, TW>), grid, 256, smem, ly.router, ly.logit_bias, x, T, E, d, logits);
 }
 
 void launch_router(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits) {
   if (T == 0) return;
   int E = ly.desc.n_exp, d = ly.desc.d;
-  if (T >= 8) {
-    dim3 grid((E + 63) / 64, (T + 7) / 8);
-    if ((int)(grid.x * grid.y) <= L.n_sm) {
-      dim3 g4((E + 31) / 32, (T + 3) / 4);
-      KLAUNCH(L, (k_router_tile<4, 4, 4>), g4, 256, 0, ly.router, ly.logit_bias, x, T, E, d, logits);
-    } else if ((int)(grid.x * grid.y) <= 2 * L.n_sm) {  // (2048 tokens on 32 experts: 1.62 -> 1.30 ms of a 24-layer step)
-      KLAUNCH(L, (k_router_tile<8, 8, 2>), grid, 256, 0, ly.router, ly.logit_bias, x, T, E, d, logits);
-    } else {  // (4096 tokens on 256 experts: two columns in flight measured 4 % slower)
-      KLAUNCH(L, (k_router_tile<8, 8, 1>), grid, 256, 0, ly.router, ly.logit_bias, x, T, E, d, logits);
-    }
+  if (T >= 8 && ((uintptr_t)x & 15) == 0) {
+    if ((long)((E + 31) / 32) * ((T + 31) / 32) >= L.n_sm) start_router_tile<16, 8>(L, ly, x, T, logits);
+    else start_router_tile<8, 4>(L, ly, x, T, logits);
     return;
   }
   dim3 grid((E + 7) / 8, T);
@@ -608,56 +636,250 @@ void launch_plan(const Launch &L, const LayerDev &ly, const uint32_t *ids, int T
   if (P > 0) KLAUNCH(L, k_plan_place, E, 256, 0, ids, P, K, pl);
 }
 
-// Router logits, top-k and the dispatch plan of a few tokens (T < 8) in ONE launch: the grid of
-// k_router computes the logits; the CTA that finishes last (a ticket counter; nobody waits for
-// anybody) routes every token, one warp each, and builds the plan in shared memory. Six launches of a
-// decode step become one; the values are those of k_router, k_route and k_plan_*.
+// ---------------------------------------------------------------------------
+// The same plan when the ids come from k_route's logits: the pairs are cut into segments of 32 tokens.
+// k_route_seg routes a segment (a warp a token) and counts its pairs by expert; k_plan_seg_scan turns the
+// [segments][E] counts into first positions (and writes the tile list of the tensor-core products);
+// k_plan_seg_place ranks the pairs of a segment. Three launches whose work grows with the pairs, where
+// k_plan_* takes four and has every expert's CTA walk all pairs (4096 tokens x 8 on 256 experts: 72 us).
+// ---------------------------------------------------------------------------
+#define PL_SEG 32 /* tokens of a segment = warps of its CTA */
+__global__ void __launch_bounds__(1024) k_route_seg(pm_layer_desc D, const float *__restrict__ logits,
+                                                   const float *__restrict__ sel_bias, int T, uint32_t *ids, float *wout,
+                                                   uint32_t *seg_cnt) {
+  extern __shared__ float rsm[];  // [32] x (E scores, E / 2 group scores, E / 2 bytes), then E counts
+  const int E = D.n_exp, K = D.top_k, lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const int per = E + E / 2 + (E / 2 + 3) / 4;
+  uint32_t *cnt = (uint32_t *)(rsm + PL_SEG * per);
+  for (int e = threadIdx.x; e < E; e += 1024) cnt[e] = 0;
+  __syncthreads();
+  const int t = blockIdx.x * PL_SEG + wi;
+  if (t < T) {
+    float *sv = rsm + wi * per;
+    pm_route_warp(D, logits + (size_t)t * E, sel_bias, lane, sv, sv + E, (unsigned char *)(sv + E + E / 2), ids + (size_t)t * K,
+                  wout + (size_t)t * K);
+    __syncwarp();
+    if (lane < K) atomicAdd(&cnt[ids[(size_t)t * K + lane]], 1u);  // (written by this warp above)
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += 1024) seg_cnt[(size_t)blockIdx.x * E + e] = cnt[e];
+}
+// exclusive scans over 512 values of one CTA of 512 threads: (a, b) -> sums of the earlier threads' values and the totals
+__device__ __forceinline__ void pm_scan2_512(uint32_t a, uint32_t b, uint32_t &ea, uint32_t &eb, uint32_t &ta, uint32_t &tb,
+                                             uint32_t (*sh)[16]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t x = a, y = b;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(PM_FULL, x, o), v = __shfl_up_sync(PM_FULL, y, o);
+    if (lane >= o) { x += u; y += v; }
+  }
+  if (lane == 31) { sh[0][warp] = x; sh[1][warp] = y; }
+  __syncthreads();
+  ea = x - a;
+  eb = y - b;
+  ta = tb = 0;
+#pragma unroll
+  for (int w = 0; w < 16; w++) {
+    if (w < warp) { ea += sh[0][w]; eb += sh[1][w]; }
+    ta += sh[0][w];
+    tb += sh[1][w];
+  }
+  __syncthreads();
+}
+// one CTA: counts of the segments -> the plan's active / offset / count / base, seg_cnt[s][e] -> first position of
+// segment s's pairs of expert e; and the tile list (k_tc_tiles' rules) when tt.tiles is given
+__global__ void __launch_bounds__(512) k_plan_seg_scan(PlanDev pl, int E, int T, int n_seg, uint32_t *seg_cnt, uint32_t *usage, TcTiles tt,
+                                                       int first_local, int n_local) {
+  __shared__ uint32_t sh[2][16];
+  const int e = threadIdx.x;
+  uint32_t c = 0;
+  if (e < E) {
+#pragma unroll 16
+    for (int s = 0; s < n_seg; s++) c += seg_cnt[(size_t)s * E + e];
+  }
+  uint32_t o, na, total, active;
+  pm_scan2_512(c, c > 0, o, na, total, active, sh);
+  if (e < E) {
+    pl.base[e] = o;
+    pl.cnt[e] = c;
+    if (c > 0) {
+      pl.active[na] = (uint32_t)e;
+      pl.offset[na] = o;
+      pl.count[na] = c;
+      if (usage) usage[e] += c;
+    }
+    if ((uint32_t)e >= active) {
+      pl.active[e] = 0;
+      pl.offset[e] = 0;
+      pl.count[e] = 0;
+    }
+    uint32_t run = o;
+#pragma unroll 16
+    for (int s = 0; s < n_seg; s++) {
+      const uint32_t v = seg_cnt[(size_t)s * E + e];
+      seg_cnt[(size_t)s * E + e] = run;
+      run += v;
+    }
+  }
+  if (e == 0) *pl.n_active = (int)active + (tt.shared ? 1 : 0);
+  if (tt.tiles) {
+    const uint32_t nt = (c + tt.ntok - 1) / tt.ntok, rp = (c + 15u) & ~15u;
+    uint32_t ft, r0, at, ar;
+    pm_scan2_512(nt, rp, ft, r0, at, ar, sh);
+    if (c > 0) {
+      tt.group_r0[na] = r0;
+      const int el = e - first_local;
+      for (uint32_t i = 0; i < nt && (int)(ft + i) < tt.max_tiles; i++)
+        tt.tiles[ft + i] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, o + i * tt.ntok,
+                                      min(c - i * tt.ntok, (uint32_t)tt.ntok), r0 + i * tt.ntok);
+    }
+    uint32_t st = 0;
+    if (tt.shared) {  // the shared expert as one more group: every token, pairs total .. total + T - 1
+      st = (T + tt.ntok - 1) / tt.ntok;
+      for (uint32_t i = e; i < st && (int)(at + i) < tt.max_tiles; i += 512)
+        tt.tiles[at + i] = make_uint4(TC_SHARED, total + i * tt.ntok, min((uint32_t)T - i * tt.ntok, (uint32_t)tt.ntok), ar + i * tt.ntok);
+      for (int i = e; i < T; i += 512) pl.pair_token[total + i] = (uint32_t)i;
+    }
+    if (e == 0) {
+      if (tt.shared) {
+        pl.offset[active] = total;
+        pl.count[active] = T;
+        tt.group_r0[active] = ar;
+      }
+      tt.n[0] = min((int)(at + st), tt.max_tiles);
+      tt.next[0] = tt.next[1] = 0;
+    }
+  }
+}
+// a CTA a segment: thread i = pair i of it; its rank among the segment's earlier pairs of the same expert
+__global__ void __launch_bounds__(512) k_plan_seg_place(const uint32_t *__restrict__ ids, int P, int K,
+                                                        const uint32_t *__restrict__ seg_pos, int E, PlanDev pl) {
+  __shared__ __align__(16) uint32_t s_id[512];
+  const int n = PL_SEG * K, p0 = blockIdx.x * n, i = threadIdx.x, g = p0 + i;
+  const bool on = i < n && g < P;
+  const uint32_t e = on ? ids[g] : 0xffffffffu;
+  s_id[i] = e;
+  __syncthreads();
+  if (!on) return;
+  uint32_t rank = 0;
+  for (int j = 0; j < (i & ~3); j += 4) {
+    const uint4 v = *(const uint4 *)(s_id + j);
+    rank += (v.x == e) + (v.y == e) + (v.z == e) + (v.w == e);
+  }
+  for (int j = i & ~3; j < i; j++) rank += s_id[j] == e;
+  const uint32_t p = seg_pos[(size_t)blockIdx.x * E + e] + rank;
+  pl.pair_pos[g] = p;
+  pl.pair_token[p] = (uint32_t)(g / K);
+  pl.pair_src[p] = (uint32_t)g;
+}
+
+size_t route_seg_words(int T, int E) { return (size_t)((T + PL_SEG - 1) / PL_SEG) * E; }
+void launch_route_plan(const Launch &L, const LayerDev &ly, const float *logits, int T, uint32_t *ids, float *w, PlanDev pl,
+                       uint32_t *seg, const TcTiles &tt) {
+  const int E = ly.desc.n_exp, K = ly.desc.top_k, nseg = (T + PL_SEG - 1) / PL_SEG;
+  const int smem = (PL_SEG * (E + E / 2 + (E / 2 + 3) / 4) + E) * 4;
+  static int smem_set = 48 * 1024;
+  if (smem > smem_set) {
+    cudaFuncSetAttribute(k_route_seg, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    smem_set = smem;
+  }
+  KLAUNCH(L, k_route_seg, nseg, 1024, smem, ly.desc, logits, ly.select_bias, T, ids, w, seg);
+  KLAUNCH(L, k_plan_seg_scan, 1, 512, 0, pl, E, T, nseg, seg, ly.usage, tt, ly.first_local, ly.n_local);
+  KLAUNCH(L, k_plan_seg_place, nseg, 512, 0, ids, T * K, K, seg, E, pl);
+}
+
+// Router logits, top-k and the dispatch plan of a few tokens (T < 8) in ONE launch: a CTA brings EPC experts' rows
+// and the tokens into shared memory by two bulk copies (a row is 8 to 28 KB: loads from registers kept 3 KB an SM
+// in flight, one token on 256 experts x 7168 46 us), a warp a (expert, token); the CTA that finishes last (a ticket
+// counter; nobody waits for anybody) routes every token, one warp each, and builds the plan and the tile list.
+// The values are those of k_router, k_route and k_plan_*.
 #define RS_TOK 8   /* tokens (= warps of the last CTA) */
 __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const float *__restrict__ wr,
                                                           const float *__restrict__ bias,
                                                           const float *__restrict__ sel_bias,
-                                                          const float *__restrict__ x, int T, float *logits,
+                                                          const float *__restrict__ x, int T, int epc, int tg, float *logits,
                                                           uint32_t *ids, float *wout, PlanDev pl, uint32_t *usage,
-                                                          const int32_t *__restrict__ slot_table, unsigned int *ticket) {
-  extern __shared__ float xs[];  // d floats (the token's row), reused by the last CTA
+                                                          const int32_t *__restrict__ slot_table, unsigned int *ticket,
+                                                          TcTiles tt, int first_local, int n_local, int *err,
+                                                          unsigned long long wait_ns) {
+  extern __shared__ __align__(16) float xs[];  // [epc][d] router rows, [tg][d] tokens; reused by the last CTA
+  __shared__ __align__(8) uint64_t s_bar;
   const int E = D.n_exp, d = D.d, K = D.top_k;
-  const int t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < d; i += 256) xs[i] = x[(size_t)t * d + i];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int e0 = blockIdx.x * epc, ne = min(epc, E - e0);
+  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_bar);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   __syncthreads();
-  {
-    const int e = blockIdx.x * 8 + warp;
-    if (e < E) {
-      const float *w = wr + (size_t)e * d;
+  auto bulk = [&](float *dst, const float *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+  };
+  uint32_t ph = 0;
+  for (int t0 = 0; t0 < T; t0 += tg, ph ^= 1) {
+    const int nt = min(tg, T - t0);
+    if (t0 > 0) __syncthreads();  // everybody is done with the tokens before
+    if (tid == 0) {
+      const uint32_t wb = t0 == 0 ? (uint32_t)(ne * d * 4) : 0u, xb = (uint32_t)(nt * d * 4);
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(wb + xb) : "memory");
+      if (wb) bulk(xs, wr + (size_t)e0 * d, wb);
+      bulk(xs + (size_t)epc * d, x + (size_t)t0 * d, xb);
+    }
+    {  // bounded: the copies' own time, a few us
+      unsigned long long s0 = 0;
+      for (;;) {
+        uint32_t ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok) : "r"(bar), "r"(ph) : "memory");
+        if (ok) break;
+        unsigned long long now;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+        if (s0 == 0) s0 = now;
+        if (now - s0 > wait_ns) {
+          atomicCAS(err, 0, 9);
+          break;
+        }
+      }
+    }
+    for (int i = warp; i < ne * nt; i += 8) {
+      const int el = i % ne, t = i / ne;
+      const float *w = xs + (size_t)el * d + lane, *xr = xs + (size_t)(epc + t) * d + lane;
       float acc = 0.0f;
-      for (int c = lane; c < d; c += 32) acc = __fmaf_rn(w[c], xs[c], acc);
+#pragma unroll 8
+      for (int c = 0; c < d; c += 32) acc = __fmaf_rn(w[c], xr[c], acc);
       float s = pm_warp_sum_dot(acc);
       if (lane == 0) {
-        if (bias) s = __fadd_rn(s, bias[e]);
-        logits[(size_t)t * E + e] = s;
+        if (bias) s = __fadd_rn(s, bias[e0 + el]);
+        logits[(size_t)(t0 + t) * E + e0 + el] = s;
       }
     }
   }
   __shared__ unsigned int s_last;
   __threadfence();  // this CTA's logits before its ticket
   __syncthreads();
-  if (tid == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x * gridDim.y - 1 ? 1u : 0u;
+  if (tid == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
   if (tid == 0) *ticket = 0;  // ready for the next launch (graph replays included)
 
   // ---- the last CTA: top-k per token (warp = token) ----
-  __shared__ float sm_lg[RS_TOK][PM_MAX_EXPERTS];
-  __shared__ float sm_sv[RS_TOK][PM_MAX_EXPERTS];
-  __shared__ float sm_gs[RS_TOK][PM_MAX_EXPERTS / 2];
-  __shared__ unsigned char sm_keep[RS_TOK][PM_MAX_EXPERTS / 2];
+  float *sm = xs;  // per token: E logits, E scores, E / 2 group scores, E / 2 bytes
+  const int per = 2 * E + E / 2 + (E / 2 + 3) / 4;
   __shared__ uint32_t s_ids[RS_TOK * PM_MAX_TOPK];
-  __shared__ uint32_t s_cnt[PM_MAX_EXPERTS], s_base[PM_MAX_EXPERTS], s_act[PM_MAX_EXPERTS];
+  __shared__ uint32_t s_cnt[PM_MAX_EXPERTS], s_base[PM_MAX_EXPERTS];
+  __shared__ uint32_t s_w[2][8];
   if (warp < T) {
-    for (int e = lane; e < E; e += 32) sm_lg[warp][e] = __ldcg(logits + (size_t)warp * E + e);
+    float *lg = sm + warp * per, *sv = lg + E;
+    for (int e = lane; e < E; e += 32) lg[e] = __ldcg(logits + (size_t)warp * E + e);
     __syncwarp();
-    pm_route_warp(D, sm_lg[warp], sel_bias, lane, sm_sv[warp], sm_gs[warp], sm_keep[warp], ids + (size_t)warp * K,
-                  wout + (size_t)warp * K);
+    pm_route_warp(D, lg, sel_bias, lane, sv, sv + E, (unsigned char *)(sv + E + E / 2), ids + (size_t)warp * K, wout + (size_t)warp * K);
     __syncwarp();
   }
   for (int e = tid; e < PM_MAX_EXPERTS; e += 256) s_cnt[e] = 0;
@@ -675,31 +897,74 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
     atomicAdd(&s_cnt[e], 1u);
   }
   __syncthreads();
-  if (tid == 0) {  // E <= 512 counts: one thread's pass is shorter than a scan's barriers
-    uint32_t o = 0, na = 0;
-    for (int e = 0; e < E; e++) {
-      const uint32_t c = s_cnt[e];
-      s_base[e] = o;
-      pl.base[e] = o;
-      pl.cnt[e] = c;
+  {  // thread = experts 2 tid, 2 tid + 1: exclusive scans of the counts and of the active experts
+    const uint32_t c0 = s_cnt[2 * tid], c1 = s_cnt[2 * tid + 1];
+    uint32_t o = c0 + c1, na = (c0 > 0) + (c1 > 0);
+    const uint32_t oi = o, ni = na;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+      const uint32_t u = __shfl_up_sync(PM_FULL, o, k), v = __shfl_up_sync(PM_FULL, na, k);
+      if (lane >= k) { o += u; na += v; }
+    }
+    if (lane == 31) { s_w[0][warp] = o; s_w[1][warp] = na; }
+    __syncthreads();
+    uint32_t active = 0;
+    o -= oi;
+    na -= ni;
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+      if (w < warp) { o += s_w[0][w]; na += s_w[1][w]; }
+      active += s_w[1][w];
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const int e = 2 * tid + k;
+      if (e < E) {
+        s_base[e] = o + (k ? c0 : 0);
+        pl.base[e] = o + (k ? c0 : 0);
+        pl.cnt[e] = k ? c1 : c0;
+        if ((uint32_t)e >= active) {
+          pl.active[e] = 0;
+          pl.offset[e] = 0;
+          pl.count[e] = 0;
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const int e = 2 * tid + k;
+      const uint32_t c = k ? c1 : c0;
       if (c) {
         pl.active[na] = (uint32_t)e;
         pl.offset[na] = o;
         pl.count[na] = c;
         if (usage && !slot_table) usage[e] += c;
+        if (tt.tiles) {  // (a group has fewer than 16 pairs: one tile each)
+          const int el = e - first_local;
+          tt.group_r0[na] = 16 * na;
+          tt.tiles[na] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, o, c, 16 * na);
+        }
         na++;
       }
       o += c;
     }
-    s_act[0] = na;
-    *pl.n_active = (int)na;
+    if (tid == 0) {
+      *pl.n_active = (int)active + (tt.shared ? 1 : 0);
+      if (tt.tiles) {
+        if (tt.shared) {  // the shared expert as one more group: every token, pairs P .. P + T - 1
+          pl.offset[active] = P;
+          pl.count[active] = T;
+          tt.group_r0[active] = 16 * active;
+          tt.tiles[active] = make_uint4(TC_SHARED, P, T, 16 * active);
+        }
+        tt.n[0] = (int)active + (tt.shared ? 1 : 0);
+        tt.next[0] = tt.next[1] = 0;
+      }
+    }
+    if (tt.shared && tid < T) pl.pair_token[P + tid] = (uint32_t)tid;
   }
   __syncthreads();
-  for (int e = (int)s_act[0] + tid; e < E; e += 256) {
-    pl.active[e] = 0;
-    pl.offset[e] = 0;
-    pl.count[e] = 0;
-  }
   if (tid < P) {  // stable: a pair goes behind the earlier pairs of its expert
     const uint32_t e = s_ids[tid];
     uint32_t before = 0;
@@ -711,28 +976,49 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
   }
 }
 
-// T < 8 tokens; ticket: a zeroed word of the context
+// whether launch_route_plan_small takes T tokens of this layer: a router row and a token's row have to fit shared memory
+bool route_plan_small_takes(const LayerDev &ly, const float *x, int T) {
+  return ((uintptr_t)x & 15) == 0 && T > 0 && T < PM_SMALL_ROUTE_TOKENS && (size_t)2 * ly.desc.d * 4 <= 200 * 1024;
+}
+// ticket: a zeroed word of the context
 void launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits, uint32_t *ids,
-                             float *w, PlanDev pl, const int32_t *slot_table, unsigned int *ticket) {
+                             float *w, PlanDev pl, const int32_t *slot_table, unsigned int *ticket, const TcTiles &tt, int *err,
+                             unsigned long long wait_ns) {
   const int E = ly.desc.n_exp, d = ly.desc.d;
-  dim3 grid((E + 7) / 8, T);
-  // (its static arrays take most of the 48 KB a kernel gets without asking; the attribute is raised on
-  // a layer's first call, which is never inside a stream capture)
+  const int most = (int)(200 * 1024 / ((size_t)d * 4));  // rows of d values that fit
+  int epc = (E + L.n_sm - 1) / L.n_sm;                   // about a CTA an SM
+  if (epc > most - 1) epc = most - 1;
+  int tg = most - epc < T ? most - epc : T;
+  const int per = 2 * E + E / 2 + (E / 2 + 3) / 4;       // the last CTA's scratch
+  int smem = (epc + tg) * d * 4;
+  if (T * per * 4 > smem) smem = T * per * 4;
   static int smem_set = 0;
-  if (d * 4 > smem_set) {
-    cudaFuncSetAttribute(k_route_plan_small, cudaFuncAttributeMaxDynamicSharedMemorySize, d * 4);
-    smem_set = d * 4;
+  if (smem > smem_set) {  // (raised on a layer's first call, which is never inside a stream capture)
+    cudaFuncSetAttribute(k_route_plan_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    smem_set = smem;
   }
-  KLAUNCH(L, k_route_plan_small, grid, 256, (size_t)d * 4, ly.desc, ly.router, ly.logit_bias, ly.select_bias, x, T, logits,
-          ids, w, pl, ly.usage, slot_table, ticket);
+  KLAUNCH(L, k_route_plan_small, (E + epc - 1) / epc, 256, smem, ly.desc, ly.router, ly.logit_bias, ly.select_bias, x, T, epc, tg,
+          logits, ids, w, pl, ly.usage, slot_table, ticket, tt, ly.first_local, ly.n_local, err, wait_ns);
 }
 
-__global__ void k_iota(uint32_t *p, uint32_t n) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = i;
+// the trivial plan of the shared expert: one group of all T tokens (and its tiles, when the tensor-core products serve it)
+__global__ void k_shared_groups(uint32_t *one, uint32_t *zero, uint32_t *count, uint32_t *token, uint32_t T, TcTiles tt) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < T) token[i] = i;
+  if (i == 0) {
+    *one = 1;
+    *zero = 0;
+    *count = T;
+    if (tt.tiles) {
+      tt.group_r0[0] = 0;
+      tt.n[0] = (int)((T + tt.ntok - 1) / tt.ntok);
+      tt.next[0] = tt.next[1] = 0;
+    }
+  }
+  if (tt.tiles && i * tt.ntok < T) tt.tiles[i] = make_uint4(TC_SHARED, i * tt.ntok, min(T - i * tt.ntok, (uint32_t)tt.ntok), i * tt.ntok);
 }
-void launch_iota(const Launch &L, uint32_t *p, uint32_t n) {
-  if (n) KLAUNCH(L, k_iota, (n + 255) / 256, 256, 0, p, n);
+void launch_shared_groups(const Launch &L, int *one, uint32_t *zero, uint32_t *count, uint32_t *token, int T, const TcTiles &tt) {
+  KLAUNCH(L, k_shared_groups, (T + 255) / 256, 256, 0, (uint32_t *)one, zero, count, token, (uint32_t)T, tt);
 }
 
 // ===========================================================================
@@ -1419,6 +1705,7 @@ void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int
 // ===========================================================================
 // combine (src/moe_kernels.rs:1798-1808): fixed k order, then the shared expert
 // ===========================================================================
+// (four columns a thread: 16-byte reads, all K of them in flight; 4096 tokens x 8 x 7168: 256 -> 190 us, 1.06 GB)
 __global__ void __launch_bounds__(256) k_combine(int d, int K, int in_combine,
                                                  const float *__restrict__ eo,
                                                  const uint32_t *__restrict__ pair_pos,
@@ -1426,24 +1713,36 @@ __global__ void __launch_bounds__(256) k_combine(int d, int K, int in_combine,
                                                  const float *__restrict__ shared_out,
                                                  const float *__restrict__ shared_logit, float *y,
                                                  int accumulate) {
-  int t = blockIdx.y;
-  int c = blockIdx.x * 256 + threadIdx.x;
+  const int t = blockIdx.y;
+  const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
   if (c >= d) return;
-  float s = 0.0f;
+  float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 8
   for (int k = 0; k < K; k++) {
     const uint32_t p = pair_pos[t * K + k];
-    float v = p == PM_PAIR_NONE ? 0.0f : eo[(size_t)p * d + c];  // a pair whose expert id was refused
-    if (in_combine) v = __fmul_rn(w[t * K + k], v);
-    s = __fadd_rn(s, v);
+    float4 v = p == PM_PAIR_NONE ? make_float4(0.0f, 0.0f, 0.0f, 0.0f)  // a pair whose expert id was refused
+                                 : __ldcs((const float4 *)(eo + (size_t)p * d + c));
+    if (in_combine) {
+      const float wk = w[t * K + k];
+      v = make_float4(__fmul_rn(wk, v.x), __fmul_rn(wk, v.y), __fmul_rn(wk, v.z), __fmul_rn(wk, v.w));
+    }
+    s = make_float4(__fadd_rn(s.x, v.x), __fadd_rn(s.y, v.y), __fadd_rn(s.z, v.z), __fadd_rn(s.w, v.w));
   }
   if (shared_out) {
-    float sv = shared_out[(size_t)t * d + c];
-    if (shared_logit)
-      sv = __fmul_rn(sv, __fdiv_rn(1.0f, __fadd_rn(1.0f, pm_exp(-shared_logit[t]))));
-    s = __fadd_rn(s, sv);
+    float4 v = *(const float4 *)(shared_out + (size_t)t * d + c);
+    if (shared_logit) {
+      const float f = __fdiv_rn(1.0f, __fadd_rn(1.0f, pm_exp(-shared_logit[t])));
+      v = make_float4(__fmul_rn(v.x, f), __fmul_rn(v.y, f), __fmul_rn(v.z, f), __fmul_rn(v.w, f));
+    }
+    s = make_float4(__fadd_rn(s.x, v.x), __fadd_rn(s.y, v.y), __fadd_rn(s.z, v.z), __fadd_rn(s.w, v.w));
   }
-  size_t o = (size_t)t * d + c;
-  y[o] = accumulate ? __fadd_rn(y[o], s) : s;
+  float *o = y + (size_t)t * d + c;  // (y is the caller's: 4-byte aligned)
+  if (accumulate) s = make_float4(__fadd_rn(o[0], s.x), __fadd_rn(o[1], s.y), __fadd_rn(o[2], s.z), __fadd_rn(o[3], s.w));
+  if (((uintptr_t)o & 15) == 0) {
+    *(float4 *)o = s;
+  } else {
+    o[0] = s.x; o[1] = s.y; o[2] = s.z; o[3] = s.w;
+  }
 }
 
 void launch_combine(const Launch &L, const LayerDev &ly, const float *eo, const uint32_t *pair_pos,
@@ -1451,7 +1750,7 @@ void launch_combine(const Launch &L, const LayerDev &ly, const float *eo, const 
                     float *y, bool accumulate) {
   if (T == 0) return;
   int d = ly.desc.d;
-  dim3 grid((d + 255) / 256, T);
+  dim3 grid((d + 1023) / 1024, T);
   KLAUNCH(L, k_combine, grid, 256, 0, d, ly.desc.top_k,
           (int)(ly.desc.weight_fold == PM_FOLD_IN_COMBINE), eo, pair_pos, w, shared_out,
           shared_logit, y, (int)accumulate);

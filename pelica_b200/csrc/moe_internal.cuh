@@ -135,40 +135,50 @@ void launch_route(const Launch &L, const LayerDev &ly, const float *logits, int 
                   float *w);
 // err: the context's error word (an expert id outside the layer is reported there, never used)
 void launch_plan(const Launch &L, const LayerDev &ly, const uint32_t *ids, int T, PlanDev plan, int *err);
-// router + top-k + plan of T < PM_SMALL_ROUTE_TOKENS tokens in one launch (ticket: a zeroed word the
+// router + top-k + plan (+ tile list) of T < PM_SMALL_ROUTE_TOKENS tokens in one launch (ticket: a zeroed word the
 // kernel leaves zeroed; slot_table: expert -> slot of an expert-parallel placement, or null)
 #define PM_SMALL_ROUTE_TOKENS 8
-void launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits, uint32_t *ids,
-                             float *w, PlanDev pl, const int32_t *slot_table, unsigned int *ticket);
-void launch_iota(const Launch &L, uint32_t *p, uint32_t n);
-void launch_gateup(const Launch &L, const LayerDev &ly, bool shared, Groups g, int n_pairs,
-                   const float *x, const int8_t *xq, const float *xd, const int32_t *xbsum,
-                   const float *w, float *h);
-void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int n_pairs,
-                 const float *h, const int8_t *hq, const float *hd, const int32_t *hbsum,
-                 float *eo);
-// tensor-core (tcgen05 int8) form of launch_gateup / launch_down for Q4_K / Q6_K x Q8x (prefill_tc.cu):
-// the token tiles of a grouping (one list serves both products), the activation rows regrouped by expert
-// in the products' layout (rec: tc_rec_bytes(n_pairs, max_groups, cols) bytes), the products.
-// src_row: row of the activations that holds pair p (null: row p itself)
+// the token tiles of a grouping for the tensor-core products (prefill_tc.cu)
 struct TcTiles {
   int *n;              // [1] tiles
   unsigned int *next;  // [2] item counters of the gate/up and the down launch (each list serves one of each)
   uint4 *tiles;        // (expert slot or ~0, first pair, pairs, first record row)
   uint32_t *group_r0;  // [512] first record row of a group
   int ntok;            // tokens of a full tile (128, or 64 where the groups are small)
+  int shared;          // the list holds the shared expert as one more group (pairs P .. P + T - 1)
   int max_tiles;
 };
+bool route_plan_small_takes(const LayerDev &ly, const float *x, int T);
+void launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits, uint32_t *ids,
+                             float *w, PlanDev pl, const int32_t *slot_table, unsigned int *ticket, const TcTiles &tt, int *err,
+                             unsigned long long wait_ns);
+// top-k, weights and plan of any number of tokens from their logits (seg: route_seg_words words of scratch)
+size_t route_seg_words(int T, int E);
+void launch_route_plan(const Launch &L, const LayerDev &ly, const float *logits, int T, uint32_t *ids, float *w, PlanDev pl,
+                       uint32_t *seg, const TcTiles &tt);
+void launch_shared_groups(const Launch &L, int *one, uint32_t *zero, uint32_t *count, uint32_t *token, int T, const TcTiles &tt);
+void launch_gateup(const Launch &L, const LayerDev &ly, bool shared, Groups g, int n_pairs,
+                   const float *x, const int8_t *xq, const float *xd, const int32_t *xbsum,
+                   const float *w, float *h);
+void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int n_pairs,
+                 const float *h, const int8_t *hq, const float *hd, const int32_t *hbsum,
+                 float *eo);
+#define TC_SHARED 0x40000000u  // expert slot of a tile of the shared expert
+// tensor-core (tcgen05 int8) form of launch_gateup / launch_down for Q4_K / Q6_K x Q8x (prefill_tc.cu):
+// the token tiles of a grouping (one list serves both products), the activation rows regrouped by expert
+// in the products' layout (rec: tc_rec_bytes(n_pairs, max_groups, cols) bytes), the products.
+// src_row: row of the activations that holds pair p (null: row p itself)
 size_t tc_tile_words(int n_pairs, int max_groups);
 // n_groups: groups that can have pairs (the experts this GPU holds)
-TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups);  // buf: tc_tile_words words, 16-byte aligned
+// shared_tokens: tokens of the shared expert's group in the same list (0: none)
+TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens);  // buf: tc_tile_words words, 16-byte aligned
 size_t tc_rec_bytes(int n_pairs, int max_groups, int cols);
-void launch_tc_tiles(const Launch &L, const LayerDev &ly, bool shared, Groups g, const TcTiles &t);
+void launch_tc_tiles(const Launch &L, const LayerDev &ly, Groups g, const TcTiles &t);
 void launch_tc_quant_rows(const Launch &L, Groups g, int n_pairs, const TcTiles &t, const uint32_t *src_row, int cols,
                           const float *x, uint8_t *rec);
 void launch_tc_rows(const Launch &L, Groups g, int n_pairs, const TcTiles &t, const uint32_t *src_row, int cols,
                     const int8_t *xq, const float *xd, const uint16_t *xbm, const int32_t *xs, uint8_t *rec);
-cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared, bool down, Groups g, int n_pairs, const TcTiles &t,
+cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared_only, bool down, const uint32_t *pair_src, const TcTiles &t,
                       const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns, int fault_block);
 // tensor-core (tcgen05 bf16) form for MXFP4 weights and f32 activations given as their bf16
 // (hi, lo) split (prefill_mx.cu); launch_split_bf16 makes the split: hi[n], lo[n] bf16

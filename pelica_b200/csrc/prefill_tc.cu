@@ -236,12 +236,14 @@ extern "C" __attribute__((visibility("default"))) int pm_debug_tc_trace(unsigned
 template <int V> struct PassC { static constexpr int value = V; };
 
 struct TcArgs {
-  CUtensorMap m0[2], m1[2];  // planes of the tile's matrices as [expert][row][bytes]: gate or down, up
+  CUtensorMap m0[2], m1[2];    // planes of the tile's matrices as [expert][row][bytes]: gate or down, up
+  CUtensorMap ms0[2], ms1[2];  // ... of the shared expert
   const uint4 *tiles;        // see k_tc_tiles
   const int *n_tiles;        // [1]
   unsigned int *next;        // [1] zero at launch: work items handed out so far (beyond two a CTA)
   const uint8_t *rec;        // the tokens' operand as records (TC_REC)
   const uint8_t *s0, *s1, *d0, *d1;  // Q6_K: the planes of the 16 sub-scales and of the f16 scales
+  const uint8_t *ss0, *ss1, *ds0, *ds1;  // ... of the shared expert
   size_t s0_stride, s1_stride, d0_stride, d1_stride;
   const float *bias0, *bias1;  // expert biases or null
   const float *wts;            // routing weights by pair source (gate/up with fold) or null
@@ -260,7 +262,7 @@ struct TcArgs {
 // The token tiles of a grouping: group a contributes ceil(count / ntok) tiles. tiles[i] = (expert slot, or
 // ~0 for an expert another rank holds; first pair; pairs; first record row). The records' rows keep a group's
 // pairs together and start every group on a multiple of 16 rows (group_r0). One CTA; groups <= 512.
-__global__ void __launch_bounds__(512) k_tc_tiles(Groups g, int shared, int first_local, int n_local, int *head,
+__global__ void __launch_bounds__(512) k_tc_tiles(Groups g, int first_local, int n_local, int *head,
                                                   uint4 *tiles, uint32_t *group_r0, int ntok, int max_tiles) {
   __shared__ uint32_t s_t[16], s_r[16];
   const int a = threadIdx.x, lane = a & 31, warp = a >> 5;
@@ -284,7 +286,7 @@ __global__ void __launch_bounds__(512) k_tc_tiles(Groups g, int shared, int firs
   const uint32_t first = bt + t - tc, r0 = br + r - rp;
   if (a < ng) {
     group_r0[a] = r0;
-    int el = shared ? 0 : (int)g.expert[a] - first_local;
+    int el = (int)g.expert[a] - first_local;
     if (el < 0 || el >= n_local) el = -1;
     const uint32_t off = g.offset[a];
     for (uint32_t i = 0; i < tc && (int)(first + i) < max_tiles; i++)
@@ -620,7 +622,9 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
         if ((int)Tc.x >= 0) {
           const uint32_t bytes = ((Tc.z + 15) >> 4) * (2u * TC_REC);
           const uint8_t *rec = A.rec + (size_t)(Tc.w >> 3) * nb * TC_REC;  // the tile's first record
-          const int el = (int)Tc.x;
+          const bool sh = Tc.x == TC_SHARED;
+          const int el = sh ? 0 : (int)Tc.x;
+          const CUtensorMap *m0 = sh ? A.ms0 : A.m0, *m1 = sh ? A.ms1 : A.m1;
           for (int b = 0; b < nb; b++) {
             // ---- the weights of block b -> the next raw area (a box past the matrix reads zeros) ----
             const uint32_t r = sRaw_a + sr * RAWB;
@@ -630,13 +634,13 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
             tc_mbar_expect(fr, (uint32_t)RAWB);
             // (a box costs the copy engine about 100 cycles + 3-4 a row: down tiles come as boxes of 128 rows)
             if (!Q6) {
-              tc_tma3(r, A.m0, b * 144, ra, el, fr);
-              if (!DOWN) tc_tma3(r + 64 * 144, A.m1, b * 144, ra, el, fr);
+              tc_tma3(r, m0, b * 144, ra, el, fr);
+              if (!DOWN) tc_tma3(r + 64 * 144, m1, b * 144, ra, el, fr);
             } else {
-              tc_tma3(r, A.m0, b * 128, ra, el, fr);
-              if (!DOWN) tc_tma3(r + 64 * 128, A.m1, b * 128, ra, el, fr);
-              tc_tma3(r + 16384, A.m0 + 1, b * 64, ra, el, fr);
-              if (!DOWN) tc_tma3(r + 16384 + 64 * 64, A.m1 + 1, b * 64, ra, el, fr);
+              tc_tma3(r, m0, b * 128, ra, el, fr);
+              if (!DOWN) tc_tma3(r + 64 * 128, m1, b * 128, ra, el, fr);
+              tc_tma3(r + 16384, m0 + 1, b * 64, ra, el, fr);
+              if (!DOWN) tc_tma3(r + 16384 + 64 * 64, m1 + 1, b * 64, ra, el, fr);
             }
             nr++;
             if (++sr == NS) { sr = 0; pr ^= 1; }
@@ -687,7 +691,8 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
     TcItem it;
     for (int k = 0; next_item(k, it); k++) {
       const uint4 T = it.t;
-      const int el = (int)T.x, nvalid = (int)T.z, npad = (nvalid + 15) & ~15, r0 = it.r0;
+      const bool sh = T.x == TC_SHARED;  // the shared expert: no biases, no routing weight
+      const int el = sh ? 0 : (int)T.x, nvalid = (int)T.z, npad = (nvalid + 15) & ~15, r0 = it.r0;
       if (el < 0) {  // an expert another rank holds: zeros (down) / nothing to do (gate/up)
         if (DOWN)
           for (int i = tid; i < nvalid * TC_M; i += S::NW) {
@@ -700,6 +705,7 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
       const int mrow = r0 + (second ? m - 64 : m);
       // (the item's code exists once per number of passes a block: with one loop for all the row sums moved
       // between registers at every join)
+      const float *bias0 = sh ? nullptr : A.bias0, *wts = sh ? nullptr : A.wts;
       auto run = [&](auto passes) {
         constexpr int NP = decltype(passes)::value, CH = S::CW / 2;
         // columns of the last pass that are this thread's (the others have all CW)
@@ -707,17 +713,18 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
         // gate/up: the routing weight of the columns this thread will activate (half of its own: see the epilogue),
         // pass p in lanes CH p ...
         float wreg = 1.0f;
-        if (!DOWN && A.wts && lane < NP * CH) {
+        if (!DOWN && wts && lane < NP * CH) {
           const int p = lane / CH, i = lane % CH, ew = p == NP - 1 ? ewl : S::CW;
           const int n = p * S::PN + part * ew + (second ? ew >> 1 : 0) + i;
-          if (i < (ew >> 1) && n < nvalid) wreg = A.wts[A.pair_src[T.y + n]];
+          if (i < (ew >> 1) && n < nvalid) wreg = wts[A.pair_src[T.y + n]];
         }
         const uint8_t *dptr = nullptr, *sptr = nullptr;  // Q6_K: the row's f16 scales and the thread's sub-scales, a block ahead
         uint32_t scw_n[QN], d_n = 0;
         if (Q6) {
           const size_t row = (size_t)min(mrow, rows - 1) * nb;
-          dptr = (second ? A.d1 + (size_t)el * A.d1_stride : A.d0 + (size_t)el * A.d0_stride) + row * 2;
-          sptr = (second ? A.s1 + (size_t)el * A.s1_stride : A.s0 + (size_t)el * A.s0_stride) + row * 16 + 4 * QN * part;
+          dptr = (second ? (sh ? A.ds1 : A.d1 + (size_t)el * A.d1_stride) : (sh ? A.ds0 : A.d0 + (size_t)el * A.d0_stride)) + row * 2;
+          sptr = (second ? (sh ? A.ss1 : A.s1 + (size_t)el * A.s1_stride) : (sh ? A.ss0 : A.s0 + (size_t)el * A.s0_stride)) + row * 16 +
+                 4 * QN * part;
 #pragma unroll
           for (int i = 0; i < QN; i++) scw_n[i] = __ldg((const uint32_t *)sptr + i);
           d_n = __ldg((const uint16_t *)dptr);
@@ -924,14 +931,14 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
         const bool dead = *(volatile int *)A.err != 0;
         if (DOWN) {
           if (!dead && mrow < rows) {
-            const float bd = A.bias0 ? A.bias0[(size_t)el * rows + mrow] : 0.0f;
+            const float bd = bias0 ? bias0[(size_t)el * rows + mrow] : 0.0f;
             float *o = A.out + (size_t)T.y * rows + mrow;
 #pragma unroll
             for (int i = 0; i < NP * CH; i++) {
               const int p = i / CH, c = 2 * (i % CH), ew = p == NP - 1 ? ewl : S::CW, n = p * S::PN + part * ew + c;
               float v0, v1;
               tc_unpack2(tot[i], v0, v1);
-              if (A.bias0) {
+              if (bias0) {
                 v0 = __fadd_rn(v0, bd);
                 v1 = __fadd_rn(v1, bd);
               }
@@ -943,8 +950,8 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
           // gate rows in tile rows 0..63, up rows in 64..127: a pass at a time the warps that hold the same
           // columns of both (w and w ^ 2) exchange their sums through shared memory; the gate warp activates
           // the first half of the columns, the up warp the second
-          const float bg = A.bias0 && mrow < rows ? A.bias0[(size_t)el * rows + mrow] : 0.0f;
-          const float bu = A.bias0 && mrow < rows ? A.bias1[(size_t)el * rows + mrow] : 0.0f;
+          const float bg = bias0 && mrow < rows ? bias0[(size_t)el * rows + mrow] : 0.0f;
+          const float bu = bias0 && mrow < rows ? A.bias1[(size_t)el * rows + mrow] : 0.0f;
           float *sx = sX + part * S::CW * TC_M;  // (the area of these warps, whatever the pass holds)
           const int mg = m & 63;
 #pragma unroll
@@ -966,12 +973,12 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
               const int c = h0 + i, n = p * S::PN + part * ew + c;
               float gv = sx[c * TC_M + mg], uv = sx[c * TC_M + 64 + mg];
               const float wt = __shfl_sync(PM_FULL, wreg, CH * p + i);
-              if (A.bias0) {
+              if (bias0) {
                 gv = __fadd_rn(gv, bg);
                 uv = __fadd_rn(uv, bu);
               }
               if (!dead && n < nvalid && mrow < rows)
-                A.out[(size_t)(T.y + n) * rows + mrow] = pm_act(A.act, A.act_limit, A.act_alpha, gv, uv, wt, A.wts != nullptr);
+                A.out[(size_t)(T.y + n) * rows + mrow] = pm_act(A.act, A.act_limit, A.act_alpha, gv, uv, wt, wts != nullptr);
             }
           }
           // (nobody writes the area again before every warp has stored operand A of the next item)
@@ -996,7 +1003,7 @@ static int tc_max_tiles(int n_pairs, int max_groups, int ntok = TcShape<2>::NTOK
   int groups = max_groups < n_pairs ? max_groups : n_pairs;
   return n_pairs / ntok + groups;
 }
-size_t tc_tile_words(int n_pairs, int max_groups) { return 4 + 4 * (size_t)tc_max_tiles(n_pairs, max_groups) + 512; }
+size_t tc_tile_words(int n_pairs, int max_groups) { return 4 + 4 * (size_t)(tc_max_tiles(n_pairs, max_groups) + 1) + 513; }
 // bytes of the records of n_pairs rows of `cols` values in at most max_groups groups (every group
 // starts on a multiple of 16 rows)
 size_t tc_rec_bytes(int n_pairs, int max_groups, int cols) {
@@ -1004,21 +1011,22 @@ size_t tc_rec_bytes(int n_pairs, int max_groups, int cols) {
   size_t rows = (size_t)n_pairs + 15 * groups + 16;
   return (rows / 8 + 1) * (size_t)(cols / 256) * TC_REC;
 }
-TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups) {
+TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens) {
   TcTiles t;
   // tiles of up to 64 tokens and the two-CTA shape while the groups hold up to 16 pairs on average (128 experts x 2048 x
   // 768, 32 pairs a group: 102 us in the one-CTA shape, 118 us in this one; 2 pairs: 1,049 -> 733 us of a 7168-wide layer)
   const int avg = n_pairs / (n_groups < n_pairs ? n_groups : n_pairs);
   t.ntok = avg <= 16 ? TcShape<2>::NTOK : TC_NMAX;
-  t.max_tiles = tc_max_tiles(n_pairs, max_groups, t.ntok);
+  t.shared = shared_tokens > 0;
+  t.max_tiles = tc_max_tiles(n_pairs, max_groups, t.ntok) + (shared_tokens + t.ntok - 1) / t.ntok;
   t.n = (int *)buf;
   t.next = (unsigned int *)buf + 1;
   t.tiles = (uint4 *)(buf + 4);
   t.group_r0 = buf + 4 + 4 * (size_t)t.max_tiles;
   return t;
 }
-void launch_tc_tiles(const Launch &L, const LayerDev &ly, bool shared, Groups g, const TcTiles &t) {
-  k_tc_tiles<<<1, 512, 0, L.stream>>>(g, (int)shared, ly.first_local, shared ? 1 : ly.n_local, t.n, t.tiles, t.group_r0, t.ntok, t.max_tiles);
+void launch_tc_tiles(const Launch &L, const LayerDev &ly, Groups g, const TcTiles &t) {
+  k_tc_tiles<<<1, 512, 0, L.stream>>>(g, ly.first_local, ly.n_local, t.n, t.tiles, t.group_r0, t.ntok, t.max_tiles);
   if (L.count) ++*L.count;
 }
 static dim3 rows_grid(Groups g, int n_pairs, int cols) {
@@ -1063,18 +1071,26 @@ template <int WT, bool DOWN> static cudaError_t tc_start_shape(const TcArgs &A, 
 
 // Tensor-core form of launch_gateup / launch_down for Q4_K or Q6_K weights and Q8x activations given as
 // the records of the grouping's rows.
-cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared, bool down, Groups g, int n_pairs, const TcTiles &t,
+// shared_only: the list holds the shared expert's tiles alone (its width may differ).
+cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared_only, bool down, const uint32_t *pair_src, const TcTiles &t,
                       const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns, int fault_block) {
-  if (n_pairs == 0) return cudaSuccess;
-  const WMat &W0 = down ? (shared ? ly.sdown : ly.down) : (shared ? ly.sgate : ly.gate), &W1 = shared ? ly.sup : ly.up;
+  if (t.max_tiles == 0) return cudaSuccess;
+  const WMat &W0 = down ? (shared_only ? ly.sdown : ly.down) : (shared_only ? ly.sgate : ly.gate), &W1 = ly.up;
+  const WMat &S0 = down ? ly.sdown : ly.sgate, &S1 = ly.sup;
   const LayerMaps &M = *ly.maps;
-  const WMaps &M0 = down ? (shared ? M.sdown : M.down) : (shared ? M.sgate : M.gate), &M1 = shared ? M.sup : M.up;
+  const WMaps &M0 = down ? M.down : M.gate, &MS0 = down ? M.sdown : M.sgate;
   const bool q6 = W0.type == PM_TYPE_Q6_K;
   TcArgs A;
   for (int i = 0; i < 2; i++) {
     A.m0[i] = M0.m[i];
-    A.m1[i] = M1.m[i];
+    A.m1[i] = M.up.m[i];
+    A.ms0[i] = MS0.m[i];
+    A.ms1[i] = M.sup.m[i];
   }
+  A.ss0 = S0.plane[2];
+  A.ss1 = S1.plane[2];
+  A.ds0 = S0.plane[3];
+  A.ds1 = S1.plane[3];
   A.tiles = t.tiles;
   A.n_tiles = t.n;
   A.next = t.next + (down ? 1 : 0);
@@ -1087,10 +1103,10 @@ cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared, bool dow
   A.d0_stride = W0.stride[3];
   A.d1 = W1.plane[3];
   A.d1_stride = W1.stride[3];
-  A.bias0 = shared ? nullptr : (down ? ly.bias_down : ly.bias_gate);
-  A.bias1 = shared || down ? nullptr : ly.bias_up;
-  A.wts = !down && !shared && ly.desc.weight_fold == PM_FOLD_BEFORE_DOWN ? wts : nullptr;
-  A.pair_src = g.pair_src;
+  A.bias0 = down ? ly.bias_down : ly.bias_gate;
+  A.bias1 = down ? nullptr : ly.bias_up;
+  A.wts = !down && ly.desc.weight_fold == PM_FOLD_BEFORE_DOWN ? wts : nullptr;
+  A.pair_src = pair_src;
   A.out = out;
   A.err = err;
   A.wait_ns = wait_ns;
