@@ -238,3 +238,13 @@ __device__ __forceinline__ void pm_q8_pack8(const float v[8], float id, uint32_t
   w0 = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
   w1 = __byte_perm(__byte_perm(b[4], b[5], 0x0040), __byte_perm(b[6], b[7], 0x0040), 0x5410);
 }
+
+// Programmatic dependent launch (pm_launch below): the next kernel of the stream may be set up - blocks
+// placed, barriers and tensor memory prepared - while this one runs, and waits here for everything before it
+// to be complete and visible. The first statement of a kernel that reads or writes global memory.
+__device__ __forceinline__ void pm_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pm_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pm_pdl() {
+  pm_pdl_trigger();
+  pm_pdl_wait();
+}

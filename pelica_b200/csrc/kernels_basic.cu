@@ -8,6 +8,7 @@
 #include "moe_internal.cuh"
 #include "route.cuh"
 
+#define PLAUNCH(L, kern, grid, block, smem, ...) pm_launch(L, kern, grid, block, smem, __VA_ARGS__)
 #define KLAUNCH(L, kern, grid, block, smem, ...)            \
   do {                                                      \
     kern<<<grid, block, smem, (L).stream>>>(__VA_ARGS__);   \
@@ -290,6 +291,7 @@ void launch_dequant(const Launch &L, int type, size_t n, const uint8_t *p0, cons
 __global__ void __launch_bounds__(256) k_quant_q8x(const float *__restrict__ x, size_t n_blocks,
                                                   int8_t *q, float *d, int32_t *bsum, uint16_t *bm,
                                                   int32_t *xs) {
+  pm_pdl();
   const size_t b = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (b >= n_blocks) return;
   const int lane = threadIdx.x & 31;
@@ -325,7 +327,7 @@ void launch_quant_q8x(const Launch &L, const float *x, size_t rows, int n, int8_
                       int32_t *bsum, uint16_t *bm, int32_t *xs) {
   size_t nb = rows * (size_t)(n / 256);
   if (nb == 0) return;
-  KLAUNCH(L, k_quant_q8x, (unsigned)((nb + 7) / 8), 256, 0, x, nb, q, d, bsum, bm, xs);
+  PLAUNCH(L, k_quant_q8x, (unsigned)((nb + 7) / 8), 256, 0, x, nb, q, d, bsum, bm, xs);
 }
 
 // `Q8::new` (src/q4x_cpu.rs:23-37): per 32 values amax, d = amax / 127, values rounded
@@ -333,6 +335,7 @@ void launch_quant_q8x(const Launch &L, const float *x, size_t rows, int n, int8_
 // f16_scale (PM_AQ_Q8_32_F16): the stored scale is rounded through f16, the values are not touched.
 __global__ void __launch_bounds__(256) k_quant_q8_32(const float *__restrict__ x, size_t n_blocks,
                                                     int8_t *q, float *d, int f16_scale) {
+  pm_pdl();
   size_t b = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (b >= n_blocks) return;
   int lane = threadIdx.x & 31;
@@ -355,7 +358,7 @@ __global__ void __launch_bounds__(256) k_quant_q8_32(const float *__restrict__ x
 void launch_quant_q8_32(const Launch &L, const float *x, size_t rows, int n, int8_t *q, float *d, bool f16_scale) {
   size_t nb = rows * (size_t)(n / 32);
   if (nb == 0) return;
-  KLAUNCH(L, k_quant_q8_32, (unsigned)((nb + 7) / 8), 256, 0, x, nb, q, d, f16_scale ? 1 : 0);
+  PLAUNCH(L, k_quant_q8_32, (unsigned)((nb + 7) / 8), 256, 0, x, nb, q, d, f16_scale ? 1 : 0);
 }
 
 // ===========================================================================
@@ -367,6 +370,7 @@ __global__ void __launch_bounds__(256) k_router(const float *__restrict__ wr,
                                                 const float *__restrict__ bias,
                                                 const float *__restrict__ x, int E, int d,
                                                 float *logits) {
+  pm_pdl();
   extern __shared__ float xs[];
   int t = blockIdx.y;
   for (int i = threadIdx.x; i < d; i += 256) xs[i] = x[(size_t)t * d + i];
@@ -398,6 +402,7 @@ template <int EW, int TW> __global__ void __launch_bounds__(256, 1) k_router_til
                                                                                  const float *__restrict__ bias,
                                                                                  const float *__restrict__ x, int T, int E,
                                                                                  int d, float *logits) {
+  pm_pdl();
   constexpr int RE = 2 * EW, RT = 4 * TW, ROWS = RE + RT;  // rows of a stage: experts, then tokens
   extern __shared__ __align__(16) float rs[];              // [RT_ST][ROWS][RT_CH]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -476,7 +481,7 @@ static void start_router_tile(const Launch &L, const LayerDev &ly, const float *
     set = true;
   }
   const dim3 grid((E + 2 * EW - 1) / (2 * EW), (T + 4 * TW - 1) / (4 * TW));
-  KLAUNCH(L, (k_router_tile<EW, TW>), grid, 256, smem, ly.router, ly.logit_bias, x, T, E, d, logits);
+  PLAUNCH(L, (k_router_tile<EW, TW>), grid, 256, smem, ly.router, ly.logit_bias, x, T, E, d, logits);
 }
 
 void launch_router(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits) {
@@ -491,12 +496,13 @@ void launch_router(const Launch &L, const LayerDev &ly, const float *x, int T, f
   // (x is staged in d * 4 bytes of dynamic shared memory: beyond 48 KB that needs the opt-in; the
   // layer descriptor is refused above PM_MAX_D, which fits)
   if ((size_t)d * 4 > 48 * 1024) cudaFuncSetAttribute(k_router, cudaFuncAttributeMaxDynamicSharedMemorySize, d * 4);
-  KLAUNCH(L, k_router, grid, 256, (size_t)d * 4, ly.router, ly.logit_bias, x, E, d, logits);
+  PLAUNCH(L, k_router, grid, 256, (size_t)d * 4, ly.router, ly.logit_bias, x, E, d, logits);
 }
 
 __global__ void __launch_bounds__(256) k_gate_logit(const float *__restrict__ wv,
                                                     const float *__restrict__ x, int T, int d,
                                                     float *out) {
+  pm_pdl();
   int lane = threadIdx.x & 31;
   int t = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (t >= T) return;
@@ -508,7 +514,7 @@ __global__ void __launch_bounds__(256) k_gate_logit(const float *__restrict__ wv
 void launch_shared_gate_logit(const Launch &L, const LayerDev &ly, const float *x, int T,
                               float *out) {
   if (T == 0) return;
-  KLAUNCH(L, k_gate_logit, (T + 7) / 8, 256, 0, ly.shared_gate_inp, x, T, ly.desc.d, out);
+  PLAUNCH(L, k_gate_logit, (T + 7) / 8, 256, 0, ly.shared_gate_inp, x, T, ly.desc.d, out);
 }
 
 // ===========================================================================
@@ -519,6 +525,7 @@ void launch_shared_gate_logit(const Launch &L, const LayerDev &ly, const float *
 __global__ void __launch_bounds__(128) k_route(pm_layer_desc D, const float *__restrict__ logits,
                                                const float *__restrict__ sel_bias, int T,
                                                uint32_t *ids, float *wout) {
+  pm_pdl();
   __shared__ float sm_sv[4][PM_MAX_EXPERTS];
   __shared__ float sm_gs[4][PM_MAX_EXPERTS / 2];
   __shared__ unsigned char sm_keep[4][PM_MAX_EXPERTS / 2];
@@ -532,7 +539,7 @@ __global__ void __launch_bounds__(128) k_route(pm_layer_desc D, const float *__r
 void launch_route(const Launch &L, const LayerDev &ly, const float *logits, int T, uint32_t *ids,
                   float *w) {
   if (T == 0) return;
-  KLAUNCH(L, k_route, (T + 3) / 4, 128, 0, ly.desc, logits, ly.select_bias, T, ids, w);
+  PLAUNCH(L, k_route, (T + 3) / 4, 128, 0, ly.desc, logits, ly.select_bias, T, ids, w);
 }
 
 // ===========================================================================
@@ -540,6 +547,7 @@ void launch_route(const Launch &L, const LayerDev &ly, const float *logits, int 
 // within an expert as src/ds4.rs:1461-1472)
 // ===========================================================================
 __global__ void k_plan_zero(uint32_t *cnt, int E) {
+  pm_pdl();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < E) cnt[i] = 0;
 }
@@ -549,6 +557,7 @@ __global__ void k_plan_zero(uint32_t *cnt, int E) {
 // is set so that the call reports PM_ERR_INVALID at its next synchronisation.
 __global__ void k_plan_count(const uint32_t *__restrict__ ids, int P, int E, uint32_t *cnt,
                              uint32_t *pair_pos, int *err) {
+  pm_pdl();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P) return;
   uint32_t e = ids[i];
@@ -561,6 +570,7 @@ __global__ void k_plan_count(const uint32_t *__restrict__ ids, int P, int E, uin
 }
 // single CTA of 512 threads: exclusive scans over the experts
 __global__ void __launch_bounds__(512) k_plan_scan(PlanDev pl, int E, uint32_t *usage) {
+  pm_pdl();
   __shared__ uint32_t s_c[PM_MAX_EXPERTS], s_a[PM_MAX_EXPERTS];
   int e = threadIdx.x;
   uint32_t c = e < E ? pl.cnt[e] : 0;
@@ -597,6 +607,7 @@ __global__ void __launch_bounds__(512) k_plan_scan(PlanDev pl, int E, uint32_t *
 // one CTA per expert walks all pairs in order: stable placement
 __global__ void __launch_bounds__(256) k_plan_place(const uint32_t *__restrict__ ids, int P, int K,
                                                     PlanDev pl) {
+  pm_pdl();
   __shared__ uint32_t wsum[8];
   uint32_t e = blockIdx.x;
   uint32_t total = pl.cnt[e];
@@ -630,10 +641,10 @@ __global__ void __launch_bounds__(256) k_plan_place(const uint32_t *__restrict__
 
 void launch_plan(const Launch &L, const LayerDev &ly, const uint32_t *ids, int T, PlanDev pl, int *err) {
   int E = ly.desc.n_exp, K = ly.desc.top_k, P = T * K;
-  KLAUNCH(L, k_plan_zero, (E + 255) / 256, 256, 0, pl.cnt, E);
-  if (P > 0) KLAUNCH(L, k_plan_count, (P + 255) / 256, 256, 0, ids, P, E, pl.cnt, pl.pair_pos, err);
-  KLAUNCH(L, k_plan_scan, 1, 512, 0, pl, E, ly.usage);
-  if (P > 0) KLAUNCH(L, k_plan_place, E, 256, 0, ids, P, K, pl);
+  PLAUNCH(L, k_plan_zero, (E + 255) / 256, 256, 0, pl.cnt, E);
+  if (P > 0) PLAUNCH(L, k_plan_count, (P + 255) / 256, 256, 0, ids, P, E, pl.cnt, pl.pair_pos, err);
+  PLAUNCH(L, k_plan_scan, 1, 512, 0, pl, E, ly.usage);
+  if (P > 0) PLAUNCH(L, k_plan_place, E, 256, 0, ids, P, K, pl);
 }
 
 // ---------------------------------------------------------------------------
@@ -647,6 +658,7 @@ void launch_plan(const Launch &L, const LayerDev &ly, const uint32_t *ids, int T
 __global__ void __launch_bounds__(1024) k_route_seg(pm_layer_desc D, const float *__restrict__ logits,
                                                    const float *__restrict__ sel_bias, int T, uint32_t *ids, float *wout,
                                                    uint32_t *seg_cnt) {
+  pm_pdl();
   extern __shared__ float rsm[];  // [32] x (E scores, E / 2 group scores, E / 2 bytes), then E counts
   const int E = D.n_exp, K = D.top_k, lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   const int per = E + E / 2 + (E / 2 + 3) / 4;
@@ -691,6 +703,7 @@ __device__ __forceinline__ void pm_scan2_512(uint32_t a, uint32_t b, uint32_t &e
 // segment s's pairs of expert e; and the tile list (k_tc_tiles' rules) when tt.tiles is given
 __global__ void __launch_bounds__(512) k_plan_seg_scan(PlanDev pl, int E, int T, int n_seg, uint32_t *seg_cnt, uint32_t *usage, TcTiles tt,
                                                        int first_local, int n_local) {
+  pm_pdl();
   __shared__ uint32_t sh[2][16];
   const int e = threadIdx.x;
   uint32_t c = 0;
@@ -728,7 +741,6 @@ __global__ void __launch_bounds__(512) k_plan_seg_scan(PlanDev pl, int E, int T,
     uint32_t ft, r0, at, ar;
     pm_scan2_512(nt, rp, ft, r0, at, ar, sh);
     if (c > 0) {
-      tt.group_r0[na] = r0;
       const int el = e - first_local;
       for (uint32_t i = 0; i < nt && (int)(ft + i) < tt.max_tiles; i++)
         tt.tiles[ft + i] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, o + i * tt.ntok,
@@ -745,7 +757,6 @@ __global__ void __launch_bounds__(512) k_plan_seg_scan(PlanDev pl, int E, int T,
       if (tt.shared) {
         pl.offset[active] = total;
         pl.count[active] = T;
-        tt.group_r0[active] = ar;
       }
       tt.n[0] = min((int)(at + st), tt.max_tiles);
       tt.next[0] = tt.next[1] = 0;
@@ -755,6 +766,7 @@ __global__ void __launch_bounds__(512) k_plan_seg_scan(PlanDev pl, int E, int T,
 // a CTA a segment: thread i = pair i of it; its rank among the segment's earlier pairs of the same expert
 __global__ void __launch_bounds__(512) k_plan_seg_place(const uint32_t *__restrict__ ids, int P, int K,
                                                         const uint32_t *__restrict__ seg_pos, int E, PlanDev pl) {
+  pm_pdl();
   __shared__ __align__(16) uint32_t s_id[512];
   const int n = PL_SEG * K, p0 = blockIdx.x * n, i = threadIdx.x, g = p0 + i;
   const bool on = i < n && g < P;
@@ -784,9 +796,9 @@ void launch_route_plan(const Launch &L, const LayerDev &ly, const float *logits,
     cudaFuncSetAttribute(k_route_seg, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     smem_set = smem;
   }
-  KLAUNCH(L, k_route_seg, nseg, 1024, smem, ly.desc, logits, ly.select_bias, T, ids, w, seg);
-  KLAUNCH(L, k_plan_seg_scan, 1, 512, 0, pl, E, T, nseg, seg, ly.usage, tt, ly.first_local, ly.n_local);
-  KLAUNCH(L, k_plan_seg_place, nseg, 512, 0, ids, T * K, K, seg, E, pl);
+  PLAUNCH(L, k_route_seg, nseg, 1024, smem, ly.desc, logits, ly.select_bias, T, ids, w, seg);
+  PLAUNCH(L, k_plan_seg_scan, 1, 512, 0, pl, E, T, nseg, seg, ly.usage, tt, ly.first_local, ly.n_local);
+  PLAUNCH(L, k_plan_seg_place, nseg, 512, 0, ids, T * K, K, seg, E, pl);
 }
 
 // Router logits, top-k and the dispatch plan of a few tokens (T < 8) in ONE launch: a CTA brings EPC experts' rows
@@ -803,6 +815,7 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
                                                           const int32_t *__restrict__ slot_table, unsigned int *ticket,
                                                           TcTiles tt, int first_local, int n_local, int *err,
                                                           unsigned long long wait_ns) {
+  pm_pdl_trigger();
   extern __shared__ __align__(16) float xs[];  // [epc][d] router rows, [tg][d] tokens; reused by the last CTA
   __shared__ __align__(8) uint64_t s_bar;
   const int E = D.n_exp, d = D.d, K = D.top_k;
@@ -827,9 +840,11 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
     if (tid == 0) {
       const uint32_t wb = t0 == 0 ? (uint32_t)(ne * d * 4) : 0u, xb = (uint32_t)(nt * d * 4);
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(wb + xb) : "memory");
-      if (wb) bulk(xs, wr + (size_t)e0 * d, wb);
+      if (wb) bulk(xs, wr + (size_t)e0 * d, wb);  // (the router's rows depend on nothing before this launch)
+      if (t0 == 0) pm_pdl_wait();
       bulk(xs + (size_t)epc * d, x + (size_t)t0 * d, xb);
     }
+    if (t0 == 0) pm_pdl_wait();
     {  // bounded: the copies' own time, a few us
       unsigned long long s0 = 0;
       for (;;) {
@@ -942,7 +957,6 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
         if (usage && !slot_table) usage[e] += c;
         if (tt.tiles) {  // (a group has fewer than 16 pairs: one tile each)
           const int el = e - first_local;
-          tt.group_r0[na] = 16 * na;
           tt.tiles[na] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, o, c, 16 * na);
         }
         na++;
@@ -955,7 +969,6 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
         if (tt.shared) {  // the shared expert as one more group: every token, pairs P .. P + T - 1
           pl.offset[active] = P;
           pl.count[active] = T;
-          tt.group_r0[active] = 16 * active;
           tt.tiles[active] = make_uint4(TC_SHARED, P, T, 16 * active);
         }
         tt.n[0] = (int)active + (tt.shared ? 1 : 0);
@@ -997,12 +1010,13 @@ void launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x
     cudaFuncSetAttribute(k_route_plan_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     smem_set = smem;
   }
-  KLAUNCH(L, k_route_plan_small, (E + epc - 1) / epc, 256, smem, ly.desc, ly.router, ly.logit_bias, ly.select_bias, x, T, epc, tg,
+  PLAUNCH(L, k_route_plan_small, (E + epc - 1) / epc, 256, smem, ly.desc, ly.router, ly.logit_bias, ly.select_bias, x, T, epc, tg,
           logits, ids, w, pl, ly.usage, slot_table, ticket, tt, ly.first_local, ly.n_local, err, wait_ns);
 }
 
 // the trivial plan of the shared expert: one group of all T tokens (and its tiles, when the tensor-core products serve it)
 __global__ void k_shared_groups(uint32_t *one, uint32_t *zero, uint32_t *count, uint32_t *token, uint32_t T, TcTiles tt) {
+  pm_pdl();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < T) token[i] = i;
   if (i == 0) {
@@ -1010,7 +1024,6 @@ __global__ void k_shared_groups(uint32_t *one, uint32_t *zero, uint32_t *count, 
     *zero = 0;
     *count = T;
     if (tt.tiles) {
-      tt.group_r0[0] = 0;
       tt.n[0] = (int)((T + tt.ntok - 1) / tt.ntok);
       tt.next[0] = tt.next[1] = 0;
     }
@@ -1018,7 +1031,7 @@ __global__ void k_shared_groups(uint32_t *one, uint32_t *zero, uint32_t *count, 
   if (tt.tiles && i * tt.ntok < T) tt.tiles[i] = make_uint4(TC_SHARED, i * tt.ntok, min(T - i * tt.ntok, (uint32_t)tt.ntok), i * tt.ntok);
 }
 void launch_shared_groups(const Launch &L, int *one, uint32_t *zero, uint32_t *count, uint32_t *token, int T, const TcTiles &tt) {
-  KLAUNCH(L, k_shared_groups, (T + 255) / 256, 256, 0, (uint32_t *)one, zero, count, token, (uint32_t)T, tt);
+  PLAUNCH(L, k_shared_groups, (T + 255) / 256, 256, 0, (uint32_t *)one, zero, count, token, (uint32_t)T, tt);
 }
 
 // ===========================================================================
@@ -1458,6 +1471,7 @@ __device__ __forceinline__ void rows_mx_f32(const uint8_t *const (&nib)[NR], con
 // consecutive h values (four rows an activation read); grid (ceil(ff / 16), groups)
 __global__ void __launch_bounds__(256) k_gateup_mx(LayerDev ly, Groups g, const float *__restrict__ x,
                                                    const float *__restrict__ wts, float *h) {
+  pm_pdl();
   int a = blockIdx.y;
   if (a >= *g.n_groups) return;
   const WMat &G = ly.gate, &U = ly.up;
@@ -1497,6 +1511,7 @@ __global__ void __launch_bounds__(256) k_gateup_mx(LayerDev ly, Groups g, const 
 // down for MXFP4 experts and f32 hidden vectors: a warp takes four consecutive output rows;
 // grid (ceil(d / 32), groups)
 __global__ void __launch_bounds__(256) k_down_mx(LayerDev ly, Groups g, const float *__restrict__ h, float *eo) {
+  pm_pdl();
   int a = blockIdx.y;
   if (a >= *g.n_groups) return;
   const WMat &Dn = ly.down;
@@ -1539,6 +1554,7 @@ __global__ void __launch_bounds__(256, 3) k_gateup(LayerDev ly, int shared, Grou
                                                 const float *__restrict__ xd,
                                                 const int32_t *__restrict__ xbsum,
                                                 const float *__restrict__ wts, float *h) {
+  pm_pdl();
   int a = blockIdx.y;
   if (a >= *g.n_groups) return;
   const WMat &G = shared ? ly.sgate : ly.gate;
@@ -1600,6 +1616,7 @@ __global__ void __launch_bounds__(256) k_down(LayerDev ly, int shared, Groups g,
                                               const int8_t *__restrict__ hq,
                                               const float *__restrict__ hd,
                                               const int32_t *__restrict__ hbsum, float *eo) {
+  pm_pdl();
   int a = blockIdx.y;
   if (a >= *g.n_groups) return;
   const WMat &Dn = shared ? ly.sdown : ly.down;
@@ -1640,6 +1657,7 @@ __global__ void __launch_bounds__(256) k_down(LayerDev ly, int shared, Groups g,
 __global__ void __launch_bounds__(256, 3) k_down_q4k2(LayerDev ly, int shared, Groups g, const int8_t *__restrict__ hq,
                                                       const float *__restrict__ hd, const int32_t *__restrict__ hbsum,
                                                       float *eo) {
+  pm_pdl();
   int a = blockIdx.y;
   if (a >= *g.n_groups) return;
   const WMat &Dn = shared ? ly.sdown : ly.down;
@@ -1677,11 +1695,11 @@ void launch_gateup(const Launch &L, const LayerDev &ly, bool shared, Groups g, i
   int ff = shared ? ly.sgate.rows : ly.gate.rows;
   if (!shared && ly.desc.act_quant == PM_AQ_F32 && ly.gate.type == PM_TYPE_MXFP4 && ly.up.type == PM_TYPE_MXFP4) {
     dim3 grid((ff + 15) / 16, min(g.max_groups, n_pairs));
-    KLAUNCH(L, k_gateup_mx, grid, 256, 0, ly, g, x, w, h);
+    PLAUNCH(L, k_gateup_mx, grid, 256, 0, ly, g, x, w, h);
     return;
   }
   dim3 grid((ff + 7) / 8, min(g.max_groups, n_pairs));
-  KLAUNCH(L, k_gateup, grid, 256, 0, ly, (int)shared, g, x, xq, xd, xbsum, w, h);
+  PLAUNCH(L, k_gateup, grid, 256, 0, ly, (int)shared, g, x, xq, xd, xbsum, w, h);
 }
 void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int n_pairs,
                  const float *h, const int8_t *hq, const float *hd, const int32_t *hbsum,
@@ -1690,16 +1708,16 @@ void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int
   int d = ly.desc.d;
   if (!shared && ly.desc.act_quant == PM_AQ_F32 && ly.down.type == PM_TYPE_MXFP4) {
     dim3 grid((d + 31) / 32, min(g.max_groups, n_pairs));
-    KLAUNCH(L, k_down_mx, grid, 256, 0, ly, g, h, eo);
+    PLAUNCH(L, k_down_mx, grid, 256, 0, ly, g, h, eo);
     return;
   }
   if (ly.desc.act_quant == PM_AQ_Q8X_256 && (shared ? ly.sdown : ly.down).type == PM_TYPE_Q4_K) {
     dim3 grid((d + 15) / 16, min(g.max_groups, n_pairs));
-    KLAUNCH(L, k_down_q4k2, grid, 256, 0, ly, (int)shared, g, hq, hd, hbsum, eo);
+    PLAUNCH(L, k_down_q4k2, grid, 256, 0, ly, (int)shared, g, hq, hd, hbsum, eo);
     return;
   }
   dim3 grid((d + 7) / 8, min(g.max_groups, n_pairs));
-  KLAUNCH(L, k_down, grid, 256, 0, ly, (int)shared, g, h, hq, hd, hbsum, eo);
+  PLAUNCH(L, k_down, grid, 256, 0, ly, (int)shared, g, h, hq, hd, hbsum, eo);
 }
 
 // ===========================================================================
@@ -1713,6 +1731,7 @@ __global__ void __launch_bounds__(256) k_combine(int d, int K, int in_combine,
                                                  const float *__restrict__ shared_out,
                                                  const float *__restrict__ shared_logit, float *y,
                                                  int accumulate) {
+  pm_pdl();
   const int t = blockIdx.y;
   const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
   if (c >= d) return;
@@ -1751,7 +1770,7 @@ void launch_combine(const Launch &L, const LayerDev &ly, const float *eo, const 
   if (T == 0) return;
   int d = ly.desc.d;
   dim3 grid((d + 1023) / 1024, T);
-  KLAUNCH(L, k_combine, grid, 256, 0, d, ly.desc.top_k,
+  PLAUNCH(L, k_combine, grid, 256, 0, d, ly.desc.top_k,
           (int)(ly.desc.weight_fold == PM_FOLD_IN_COMBINE), eo, pair_pos, w, shared_out,
           shared_logit, y, (int)accumulate);
 }
@@ -1759,6 +1778,7 @@ void launch_combine(const Launch &L, const LayerDev &ly, const float *eo, const 
 // x / rms(x), unit weight; the sum order is pm_rms_inv's (common.cuh)
 __global__ void __launch_bounds__(256) k_rmsnorm(const float *__restrict__ x, int T, int d,
                                                  float eps, float *out) {
+  pm_pdl();
   __shared__ float red8[8];
   int t = blockIdx.x;
   const float *xr = x + (size_t)t * d;
@@ -1767,7 +1787,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm(const float *__restrict__ x, in
 }
 void launch_rmsnorm(const Launch &L, const float *x, int T, int d, float eps, float *out) {
   if (T == 0) return;
-  KLAUNCH(L, k_rmsnorm, T, 256, 0, x, T, d, eps, out);
+  PLAUNCH(L, k_rmsnorm, T, 256, 0, x, T, d, eps, out);
 }
 
 // ===========================================================================

@@ -118,6 +118,25 @@ struct Launch {
   int n_sm = 148;  // SMs of the device
 };
 
+// Launch of a kernel that begins with pm_pdl(): it may start while the kernel before it in the stream is still
+// running (a layer of a small call is six to nine kernels of a few us each; started one by one they left 1-2 us
+// between any two).
+template <typename... P, typename... A>
+static inline cudaError_t pm_launch(const Launch &L, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = L.stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (L.count) ++*L.count;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 void launch_repack(const Launch &L, int type, const uint8_t *raw, size_t n_blocks, uint8_t *p0,
                    uint8_t *p1, uint8_t *p2, uint8_t *p3);
 void launch_unpack(const Launch &L, int type, uint8_t *raw, size_t n_blocks, const uint8_t *p0,
@@ -143,7 +162,6 @@ struct TcTiles {
   int *n;              // [1] tiles
   unsigned int *next;  // [2] item counters of the gate/up and the down launch (each list serves one of each)
   uint4 *tiles;        // (expert slot or ~0, first pair, pairs, first record row)
-  uint32_t *group_r0;  // [512] first record row of a group
   int ntok;            // tokens of a full tile (128, or 64 where the groups are small)
   int shared;          // the list holds the shared expert as one more group (pairs P .. P + T - 1)
   int max_tiles;
@@ -174,10 +192,10 @@ size_t tc_tile_words(int n_pairs, int max_groups);
 TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens);  // buf: tc_tile_words words, 16-byte aligned
 size_t tc_rec_bytes(int n_pairs, int max_groups, int cols);
 void launch_tc_tiles(const Launch &L, const LayerDev &ly, Groups g, const TcTiles &t);
-void launch_tc_quant_rows(const Launch &L, Groups g, int n_pairs, const TcTiles &t, const uint32_t *src_row, int cols,
-                          const float *x, uint8_t *rec);
-void launch_tc_rows(const Launch &L, Groups g, int n_pairs, const TcTiles &t, const uint32_t *src_row, int cols,
-                    const int8_t *xq, const float *xd, const uint16_t *xbm, const int32_t *xs, uint8_t *rec);
+void launch_tc_quant_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x,
+                          uint8_t *rec);
+void launch_tc_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const int8_t *xq,
+                    const float *xd, const uint16_t *xbm, const int32_t *xs, uint8_t *rec);
 cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared_only, bool down, const uint32_t *pair_src, const TcTiles &t,
                       const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns, int fault_block);
 // tensor-core (tcgen05 bf16) form for MXFP4 weights and f32 activations given as their bf16

@@ -101,6 +101,7 @@ __device__ __noinline__ bool mx_bar_wait(uint64_t *bar, uint32_t parity, int *er
 // x -> (hi, lo) bf16 with hi + lo = x up to 2^-17 relative
 __global__ void __launch_bounds__(256) k_split_bf16(const float *__restrict__ x, size_t n, __nv_bfloat16 *hi,
                                                     __nv_bfloat16 *lo) {
+  pm_pdl();
   size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
   const float v = x[i];
@@ -110,8 +111,7 @@ __global__ void __launch_bounds__(256) k_split_bf16(const float *__restrict__ x,
 }
 void launch_split_bf16(const Launch &L, const float *x, size_t n, void *hi, void *lo) {
   if (n == 0) return;
-  k_split_bf16<<<(unsigned)((n + 255) / 256), 256, 0, L.stream>>>(x, n, (__nv_bfloat16 *)hi, (__nv_bfloat16 *)lo);
-  if (L.count) ++*L.count;
+  pm_launch(L, k_split_bf16, (unsigned)((n + 255) / 256), 256, 0, x, n, (__nv_bfloat16 *)hi, (__nv_bfloat16 *)lo);
 }
 
 // Four E2M1 codes (one in the low nibble of each byte of c4) -> the four bf16 patterns of
@@ -158,6 +158,7 @@ struct MxArgs {
 };
 
 __global__ void __launch_bounds__(MX_NT, 1) k_tc_mx(const MxArgs A) {
+  pm_pdl();
   extern __shared__ __align__(128) uint8_t smem[];
   if ((int)blockIdx.y >= *A.n_tiles) return;
   const uint4 tile = A.tiles[blockIdx.y];
@@ -456,7 +457,6 @@ cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, Groups 
   A.tiles = t.tiles;
   const int row_tiles = down ? (W.rows + MX_M - 1) / MX_M : (W.rows + 63) / 64;
   dim3 grid(row_tiles, t.max_tiles);
-  k_tc_mx<<<grid, MX_NT, smem, L.stream>>>(A);
-  if (L.count) ++*L.count;
+  pm_launch(L, k_tc_mx, grid, MX_NT, smem, A);
   return cudaGetLastError();
 }

@@ -261,9 +261,10 @@ struct TcArgs {
 
 // The token tiles of a grouping: group a contributes ceil(count / ntok) tiles. tiles[i] = (expert slot, or
 // ~0 for an expert another rank holds; first pair; pairs; first record row). The records' rows keep a group's
-// pairs together and start every group on a multiple of 16 rows (group_r0). One CTA; groups <= 512.
+// pairs together and start every group on a multiple of 16 rows. One CTA; groups <= 512.
 __global__ void __launch_bounds__(512) k_tc_tiles(Groups g, int first_local, int n_local, int *head,
-                                                  uint4 *tiles, uint32_t *group_r0, int ntok, int max_tiles) {
+                                                  uint4 *tiles, int ntok, int max_tiles) {
+  pm_pdl();
   __shared__ uint32_t s_t[16], s_r[16];
   const int a = threadIdx.x, lane = a & 31, warp = a >> 5;
   const int ng = min(*g.n_groups, 512);
@@ -285,7 +286,6 @@ __global__ void __launch_bounds__(512) k_tc_tiles(Groups g, int first_local, int
   }
   const uint32_t first = bt + t - tc, r0 = br + r - rp;
   if (a < ng) {
-    group_r0[a] = r0;
     int el = (int)g.expert[a] - first_local;
     if (el < 0 || el >= n_local) el = -1;
     const uint32_t off = g.offset[a];
@@ -299,32 +299,27 @@ __global__ void __launch_bounds__(512) k_tc_tiles(Groups g, int first_local, int
   }
 }
 
-// the record of (local row group rgl of a group that starts at record row r0 and has nrg row groups, block b)
-// lt: log2 of the row groups of a full tile
-__device__ __forceinline__ uint8_t *tc_rec_ptr(uint8_t *rec, uint32_t r0, int rgl, int nrg, int b, int nb, int lt) {
-  const int t0 = rgl >> lt << lt, in = min(1 << lt, nrg - t0);  // the tile's first row group, its row groups
-  return rec + (((size_t)(r0 >> 3) + t0) * nb + (size_t)b * in + (rgl - t0)) * TC_REC;
-}
-
 // Rows of f32 values -> the records the products read: `Q8x::new` (src/ds4_cpu.rs:13-35) of every 256-value
-// block, one warp per (8 rows, block). Row i of group a is record row group_r0[a] + i and comes from row
-// src_row[offset[a] + i] of x (null: row offset[a] + i itself); rows past a group's count are zeros. A token
+// block, a CTA column a token tile, one warp per (8 rows, block). Row i of a tile comes from row src_row[first + i] of
+// x (null: row first + i itself), first = the tile's first pair; rows past the tile's count are zeros. A token
 // is read and quantised once per expert that serves it: a launch less for small calls, but four times the
 // bytes of a gather of quantised rows (4096 tokens x 8 experts x 7168 values: 280 us against 48 + 60), so large
 // calls quantise first (k_quant_q8x) and gather (k_tc_rows).
-__global__ void __launch_bounds__(256) k_tc_quant_rows(Groups g, const uint32_t *__restrict__ group_r0,
+__global__ void __launch_bounds__(256) k_tc_quant_rows(const int *__restrict__ n_tiles, const uint4 *__restrict__ tiles,
                                                        const uint32_t *__restrict__ src_row, int cols,
-                                                       const float *__restrict__ x, int lt, uint8_t *__restrict__ rec) {
+                                                       const float *__restrict__ x, uint8_t *__restrict__ rec) {
+  pm_pdl();
   __shared__ __align__(16) uint8_t s_rec[8][TC_REC];
-  const int a = blockIdx.y;
-  if (a >= *g.n_groups) return;
+  if ((int)blockIdx.y >= *n_tiles) return;
+  const uint4 T = tiles[blockIdx.y];
   const int nb = cols / 256;
-  const uint32_t off = g.offset[a], cnt = g.count[a], r0 = group_r0[a];
+  const uint32_t off = T.y, cnt = T.z;
   const int lane = threadIdx.x & 31;
   uint8_t *S = s_rec[threadIdx.x >> 5];
-  const int nrg = (int)((cnt + 15u) / 16u) * 2, units = nrg * nb;  // (row group, block) pairs of this group
+  const int nrg = (int)((cnt + 15u) / 16u) * 2, units = nrg * nb;  // (row group, block) pairs of this tile
+  uint8_t *rec0 = rec + (size_t)(T.w >> 3) * nb * TC_REC;
   for (int u = blockIdx.x * 8 + (threadIdx.x >> 5); u < units; u += gridDim.x * 8) {
-    const int rgl = u / nb, b = u - rgl * nb;
+    const int b = u / nrg, rgl = u - b * nrg;  // (the tile's records lie block by block)
     // lane = values 8 lane .. 8 lane + 7 of every row, as two words a row
     uint32_t q[8][2];
 #pragma unroll
@@ -383,7 +378,7 @@ __global__ void __launch_bounds__(256) k_tc_quant_rows(Groups g, const uint32_t 
       *(uint4 *)(S + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) = o;
     }
     __syncwarp();
-    uint4 *R = (uint4 *)tc_rec_ptr(rec, r0, rgl, nrg, b, nb, lt);
+    uint4 *R = (uint4 *)(rec0 + (size_t)u * TC_REC);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       const int p = 32 * k + lane, l = p >> 2;
@@ -396,20 +391,22 @@ __global__ void __launch_bounds__(256) k_tc_quant_rows(Groups g, const uint32_t 
 
 // The same records from rows that are quantised already (rows another rank sent): one warp per
 // (8 rows, block), xbm / xs as k_q8x_aux makes them.
-__global__ void __launch_bounds__(256) k_tc_rows(Groups g, const uint32_t *__restrict__ group_r0,
+__global__ void __launch_bounds__(256) k_tc_rows(const int *__restrict__ n_tiles, const uint4 *__restrict__ tiles,
                                                  const uint32_t *__restrict__ src_row, int cols,
                                                  const int8_t *__restrict__ xq, const float *__restrict__ xd,
                                                  const uint16_t *__restrict__ xbm, const int32_t *__restrict__ xs,
-                                                 int lt, uint8_t *__restrict__ rec) {
-  const int a = blockIdx.y;
-  if (a >= *g.n_groups) return;
+                                                 uint8_t *__restrict__ rec) {
+  pm_pdl();
+  if ((int)blockIdx.y >= *n_tiles) return;
+  const uint4 T = tiles[blockIdx.y];
   const int nb = cols / 256;
-  const uint32_t off = g.offset[a], cnt = g.count[a], r0 = group_r0[a];
+  const uint32_t off = T.y, cnt = T.z;
   const int lane = threadIdx.x & 31;
   const int nrg = (int)((cnt + 15u) / 16u) * 2, units = nrg * nb;
+  uint8_t *rec0 = rec + (size_t)(T.w >> 3) * nb * TC_REC;
   for (int u = blockIdx.x * 8 + (threadIdx.x >> 5); u < units; u += gridDim.x * 8) {
-    const int rgl = u / nb, b = u - rgl * nb;
-    uint8_t *R = tc_rec_ptr(rec, r0, rgl, nrg, b, nb, lt);
+    const int b = u / nrg, rgl = u - b * nrg;
+    uint8_t *R = rec0 + (size_t)u * TC_REC;
     {  // int8 values: lane = (row of the group, quarter of the block's 16 chunks)
       const int r8 = lane >> 2, q = lane & 3;
       const uint32_t i = (uint32_t)rgl * 8 + r8;
@@ -485,6 +482,7 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
   const int nb = A.cols / 256, rows = A.rows;
   const int tid = threadIdx.x, warp = __shfl_sync(PM_FULL, tid >> 5, 0), lane = tid & 31;
 
+  pm_pdl_trigger();
   if (warp == MW) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      tc_s32(tmem_slot)),
@@ -521,6 +519,7 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
   // (a warp reduction leaves its result in a uniform register: what is computed from it - descriptors, addresses,
   // the passes of a block - stays on the uniform datapath instead of being moved there product by product)
   const uint32_t tmem = __reduce_max_sync(PM_FULL, *tmem_slot);
+  pm_pdl_wait();  // (barriers and tensor memory were prepared under the kernel before)
   // the CTA's k-th item, as the issuing warp and the workers take it from the ring (false: no more)
   auto next_item = [&](int k, TcItem &it) -> bool {
     const int s = k & (TC_IT - 1);
@@ -1003,7 +1002,7 @@ static int tc_max_tiles(int n_pairs, int max_groups, int ntok = TcShape<2>::NTOK
   int groups = max_groups < n_pairs ? max_groups : n_pairs;
   return n_pairs / ntok + groups;
 }
-size_t tc_tile_words(int n_pairs, int max_groups) { return 4 + 4 * (size_t)(tc_max_tiles(n_pairs, max_groups) + 1) + 513; }
+size_t tc_tile_words(int n_pairs, int max_groups) { return 4 + 4 * (size_t)(tc_max_tiles(n_pairs, max_groups) + 1); }
 // bytes of the records of n_pairs rows of `cols` values in at most max_groups groups (every group
 // starts on a multiple of 16 rows)
 size_t tc_rec_bytes(int n_pairs, int max_groups, int cols) {
@@ -1022,31 +1021,26 @@ TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, in
   t.n = (int *)buf;
   t.next = (unsigned int *)buf + 1;
   t.tiles = (uint4 *)(buf + 4);
-  t.group_r0 = buf + 4 + 4 * (size_t)t.max_tiles;
   return t;
 }
 void launch_tc_tiles(const Launch &L, const LayerDev &ly, Groups g, const TcTiles &t) {
-  k_tc_tiles<<<1, 512, 0, L.stream>>>(g, ly.first_local, ly.n_local, t.n, t.tiles, t.group_r0, t.ntok, t.max_tiles);
-  if (L.count) ++*L.count;
+  pm_launch(L, k_tc_tiles, 1, 512, 0, g, ly.first_local, ly.n_local, t.n, t.tiles, t.ntok, t.max_tiles);
 }
-static dim3 rows_grid(Groups g, int n_pairs, int cols) {
-  const int groups = g.max_groups < n_pairs ? g.max_groups : n_pairs;
-  const long units = ((long)n_pairs / 8 + 2 * groups) * (cols / 256);  // (row group, block) records in all
-  long gx = (units / groups + 7) / 8;  // a warp writes about one record
-  return dim3((unsigned)(gx < 1 ? 1 : (gx > 256 ? 256 : gx)), (unsigned)groups);
+static dim3 rows_grid(int n_rows, const TcTiles &t, int cols) {
+  const long units = ((long)n_rows / 8 + 2 * t.max_tiles) * (cols / 256);  // (row group, block) records in all
+  long gx = (units / t.max_tiles + 7) / 8;  // a warp writes about one record
+  return dim3((unsigned)(gx < 1 ? 1 : gx), (unsigned)t.max_tiles);
 }
-void launch_tc_quant_rows(const Launch &L, Groups g, int n_pairs, const TcTiles &t, const uint32_t *src_row, int cols,
-                          const float *x, uint8_t *rec) {
-  k_tc_quant_rows<<<rows_grid(g, n_pairs, cols), 256, 0, L.stream>>>(g, t.group_r0, src_row, cols, x, t.ntok == TC_NMAX ? 4 : 3, rec);
-  if (L.count) ++*L.count;
+void launch_tc_quant_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x,
+                          uint8_t *rec) {
+  pm_launch(L, k_tc_quant_rows, rows_grid(n_rows, t, cols), 256, 0, t.n, t.tiles, src_row, cols, x, rec);
 }
-void launch_tc_rows(const Launch &L, Groups g, int n_pairs, const TcTiles &t, const uint32_t *src_row, int cols,
-                    const int8_t *xq, const float *xd, const uint16_t *xbm, const int32_t *xs, uint8_t *rec) {
-  k_tc_rows<<<rows_grid(g, n_pairs, cols), 256, 0, L.stream>>>(g, t.group_r0, src_row, cols, xq, xd, xbm, xs, t.ntok == TC_NMAX ? 4 : 3, rec);
-  if (L.count) ++*L.count;
+void launch_tc_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const int8_t *xq,
+                    const float *xd, const uint16_t *xbm, const int32_t *xs, uint8_t *rec) {
+  pm_launch(L, k_tc_rows, rows_grid(n_rows, t, cols), 256, 0, t.n, t.tiles, src_row, cols, xq, xd, xbm, xs, rec);
 }
 
-template <int WT, bool DOWN, int PARTS> static cudaError_t tc_start(const TcArgs &A, long items, int n_sm, cudaStream_t stream) {
+template <int WT, bool DOWN, int PARTS> static cudaError_t tc_start(const Launch &L, const TcArgs &A, long items) {
   using S = TcShape<PARTS>;
   constexpr bool Q6 = WT == PM_TYPE_Q6_K;
   constexpr int NS = TcStages<PARTS, Q6, DOWN>::raw, NSB = TcStages<PARTS, Q6, DOWN>::tok;
@@ -1061,12 +1055,11 @@ template <int WT, bool DOWN, int PARTS> static cudaError_t tc_start(const TcArgs
     if (e != cudaSuccess) return e;
     if (dev < 64) set[dev] = true;
   }
-  const long ctas = (long)S::CTAS * n_sm;
-  k_tc<WT, DOWN, PARTS><<<(unsigned)(items < ctas ? items : ctas), S::NT, smem, stream>>>(A);
-  return cudaGetLastError();
+  const long ctas = (long)S::CTAS * L.n_sm;
+  return pm_launch(L, k_tc<WT, DOWN, PARTS>, dim3((unsigned)(items < ctas ? items : ctas)), S::NT, smem, A);
 }
-template <int WT, bool DOWN> static cudaError_t tc_start_shape(const TcArgs &A, int ntok, long items, int n_sm, cudaStream_t stream) {
-  return ntok == TC_NMAX ? tc_start<WT, DOWN, 4>(A, items, n_sm, stream) : tc_start<WT, DOWN, 2>(A, items, n_sm, stream);
+template <int WT, bool DOWN> static cudaError_t tc_start_shape(const Launch &L, const TcArgs &A, int ntok, long items) {
+  return ntok == TC_NMAX ? tc_start<WT, DOWN, 4>(L, A, items) : tc_start<WT, DOWN, 2>(L, A, items);
 }
 
 // Tensor-core form of launch_gateup / launch_down for Q4_K or Q6_K weights and Q8x activations given as
@@ -1119,10 +1112,9 @@ cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared_only, boo
   A.act_limit = ly.desc.act_limit;
   A.act_alpha = ly.desc.act_alpha;
   const long items = (long)A.row_tiles * t.max_tiles;
-  cudaError_t e = q6 ? (down ? tc_start_shape<PM_TYPE_Q6_K, true>(A, t.ntok, items, L.n_sm, L.stream)
-                             : tc_start_shape<PM_TYPE_Q6_K, false>(A, t.ntok, items, L.n_sm, L.stream))
-                     : (down ? tc_start_shape<PM_TYPE_Q4_K, true>(A, t.ntok, items, L.n_sm, L.stream)
-                             : tc_start_shape<PM_TYPE_Q4_K, false>(A, t.ntok, items, L.n_sm, L.stream));
-  if (e == cudaSuccess && L.count) ++*L.count;
+  cudaError_t e = q6 ? (down ? tc_start_shape<PM_TYPE_Q6_K, true>(L, A, t.ntok, items)
+                             : tc_start_shape<PM_TYPE_Q6_K, false>(L, A, t.ntok, items))
+                     : (down ? tc_start_shape<PM_TYPE_Q4_K, true>(L, A, t.ntok, items)
+                             : tc_start_shape<PM_TYPE_Q4_K, false>(L, A, t.ntok, items));
   return e;
 }

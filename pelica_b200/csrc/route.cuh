@@ -82,6 +82,19 @@ __device__ __forceinline__ void pm_route_scores(const pm_layer_desc &D, const fl
       if (lane + 32 * i < E) ssv[lane + 32 * i] = sv[i];
     __syncwarp();
     const int G = D.n_group, gs = E / G;
+    if (gs == 32) {  // a group is one register of the warp: two reductions find its two largest scores
+#pragma unroll
+      for (int i = 0; i < NP; i++)
+        if (i < G) {
+          const uint32_t key = pm_fkey(sv[i]), m1 = __reduce_max_sync(PM_FULL, key);
+          const uint32_t top = __ballot_sync(PM_FULL, key == m1);
+          const uint32_t m2 = (top & (top - 1)) ? m1 : __reduce_max_sync(PM_FULL, key == m1 ? 0u : key);
+          if (lane == i) {
+            gsc[i] = __fadd_rn(pm_funkey(m1), pm_funkey(m2));
+            keep[i] = 0;
+          }
+        }
+    } else
     for (int g = lane; g < G; g += 32) {  // lane g scores groups g, g+32, ...
       int i1 = 0;
       float v1 = ssv[g * gs];
@@ -94,7 +107,17 @@ __device__ __forceinline__ void pm_route_scores(const pm_layer_desc &D, const fl
       keep[g] = 0;
     }
     __syncwarp();
-    if (lane == 0) {
+    if (G <= 32) {  // lane g ranks group g: kept when fewer than topk_group groups come before it
+      if (lane < G) {
+        const float mine = gsc[lane];
+        int before = 0;
+        for (int g = 0; g < G; g++) {
+          const float v = gsc[g];
+          before += v > mine || (v == mine && g < lane);
+        }
+        keep[lane] = before < D.topk_group;
+      }
+    } else if (lane == 0) {
       for (int r = 0; r < D.topk_group; r++) {
         int bg = -1;
         float bv = 0.0f;
