@@ -90,7 +90,7 @@ struct pm_ctx {
   int *dev_err = nullptr;   // error word of kernels with bounded waits
   unsigned int *route_ticket = nullptr;  // [1] zero between launches: the few-token routing kernel's last-CTA ticket
   // Tensor-core expert products from this many tokens (the reference's TC_MIN, src/moe.rs:35); 0 = never. Until the
-  // caller sets it, the exact integer products take fewer (see int_tc_min): they give the same bits either way.
+  // caller sets it, the products that lose nothing by it take fewer (see pick_path).
   int tc_min_tokens = 32;
   bool tc_min_set = false;
   int64_t launches = 0;
@@ -416,7 +416,7 @@ typedef CUresult (*pm_encode_tiled_t)(CUtensorMap *, CUtensorMapDataType, cuuint
                                       const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                       CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static int32_t wmat_maps(const WMat &W, int n_exp, int box_rows, WMaps &M) {
-  if (W.type != PM_TYPE_Q4_K && W.type != PM_TYPE_Q6_K) return PM_OK;
+  if (W.type != PM_TYPE_Q4_K && W.type != PM_TYPE_Q6_K && W.type != PM_TYPE_MXFP4) return PM_OK;
   static pm_encode_tiled_t enc = nullptr;
   if (!enc) {
     void *f = nullptr;
@@ -425,17 +425,20 @@ static int32_t wmat_maps(const WMat &W, int n_exp, int box_rows, WMaps &M) {
     if (q != cudaDriverEntryPointSuccess || !f) return fail(PM_ERR_CUDA, "cuTensorMapEncodeTiled is not there");
     enc = (pm_encode_tiled_t)f;
   }
-  const int nb = W.cols / 256, n = W.type == PM_TYPE_Q4_K ? 1 : 2;
-  const int block[2] = {W.type == PM_TYPE_Q4_K ? 144 : 128, 64};
-  // Q6_K: 128- and 64-byte rows swizzled so that the row-per-thread reads of the unpack have no bank conflicts
+  const bool mx = W.type == PM_TYPE_MXFP4, q4 = W.type == PM_TYPE_Q4_K;
+  const int nb = W.cols / 256, n = q4 ? 1 : 2;
+  // MXFP4: plane 0 alone, boxes of 256 values x 64 rows and x 128 rows (the last box of a row may reach past it)
+  const int block[2] = {q4 ? 144 : 128, mx ? 128 : 64};
+  // Q6_K and MXFP4: 128- and 64-byte rows swizzled so that the row-per-thread reads of the unpack have no bank conflicts
   // (a Q4_K row of 144 bytes has none as it is)
-  const CUtensorMapSwizzle sw[2] = {W.type == PM_TYPE_Q4_K ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
-                                    CU_TENSOR_MAP_SWIZZLE_64B};
+  const CUtensorMapSwizzle sw[2] = {q4 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                                    mx ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B};
   for (int p = 0; p < n; p++) {
-    const cuuint64_t row = (cuuint64_t)nb * block[p];
-    const cuuint64_t dims[3] = {row, (cuuint64_t)W.rows, (cuuint64_t)n_exp}, strides[2] = {row, (cuuint64_t)W.stride[p]};
-    const cuuint32_t box[3] = {(cuuint32_t)block[p], (cuuint32_t)box_rows, 1}, es[3] = {1, 1, 1};
-    const CUresult r = enc(&M.m[p], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, W.plane[p], dims, strides, box, es,
+    const int plane = mx ? 0 : p;
+    const cuuint64_t row = mx ? (cuuint64_t)W.cols / 2 : (cuuint64_t)nb * block[p];
+    const cuuint64_t dims[3] = {row, (cuuint64_t)W.rows, (cuuint64_t)n_exp}, strides[2] = {row, (cuuint64_t)W.stride[plane]};
+    const cuuint32_t box[3] = {(cuuint32_t)block[p], mx ? 64u << p : (cuuint32_t)box_rows, 1}, es[3] = {1, 1, 1};
+    const CUresult r = enc(&M.m[p], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, W.plane[plane], dims, strides, box, es,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, sw[p], CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(PM_ERR_CUDA, "cuTensorMapEncodeTiled: %d", (int)r);
@@ -830,10 +833,10 @@ struct Scratch {
   int8_t *xq; float *xd; int32_t *xbsum; uint16_t *xbm; int32_t *xs;
   float *h; int8_t *hq; float *hd; int32_t *hbsum; uint16_t *hbm; int32_t *hs;
   float *eo;
-  uint16_t *xhl, *hhl;  // MXFP4 tensor-core path: bf16 (hi, lo) split of x [2][T*d] and of h [2][P*ff]
+  int eo_parts;     // parts of eo [parts][P][d] to add up (MXFP4 products cut along K)
   uint32_t *tiles;  // tile list of the tensor-core kernels
   uint32_t *seg;    // per-segment counts of the plan
-  uint8_t *rec;     // activation rows regrouped into the int8 tensor-core kernel's records
+  uint8_t *rec;     // activation rows regrouped into the operand of the tensor-core kernels
   // shared expert
   int *one; uint32_t *zero_u, *tcount, *iota;
   float *sh; int8_t *shq; float *shd; int32_t *shbsum; uint16_t *shbm; int32_t *shs;
@@ -843,8 +846,14 @@ struct Scratch {
 // whether the shared expert can run as one more group of the routed experts' tensor-core launches
 static bool shared_merges(const pm_layer_desc &D) { return D.shared && D.shared_ff == D.ff && D.act_quant == PM_AQ_Q8X_256; }
 
-// the largest record buffer any tensor-core launch of a T-token call needs (Q8x activations only)
+// the layers k_tc_mx takes
+static bool mx_layer(const pm_layer_desc &D) {
+  return D.act_quant == PM_AQ_F32 && D.type_gate == PM_TYPE_MXFP4 && D.type_up == PM_TYPE_MXFP4 && D.type_down == PM_TYPE_MXFP4;
+}
+
+// the largest record buffer any tensor-core launch of a T-token call needs
 static size_t scratch_rec_bytes(const pm_layer_desc &D, int T) {
+  if (mx_layer(D)) return mx_rec_bytes(T * D.top_k, D.n_exp, std::max(D.d, D.ff));
   if (D.act_quant != PM_AQ_Q8X_256) return 0;
   const int m = shared_merges(D) ? 1 : 0, P = T * (D.top_k + m), E = D.n_exp + m;
   size_t r = std::max(tc_rec_bytes(P, E, D.d), tc_rec_bytes(P, E, D.ff));
@@ -861,8 +870,7 @@ static size_t scratch_bytes(const pm_layer_desc &D, int T) {
   b += al(T * d) + al(T * (d / 32 + 1) * 4) + al(T * (d / 256 + 1) * 4) + al(T * (d / 32) * 4) * 2;
   const size_t Pm = P + (shared_merges(D) ? T : 0);    // pairs with the shared expert's
   b += al(Pm * ff * 4) + al(P * ff) + al(P * (ff / 32 + 1) * 4) + al(P * (ff / 256 + 1) * 4) + al(P * (ff / 32) * 4) * 2;
-  b += al(Pm * d * 4);
-  if (D.act_quant == PM_AQ_F32 && D.type_gate == PM_TYPE_MXFP4) b += al(T * d * 4) + al(P * ff * 4);
+  b += al(Pm * d * 4 * (mx_layer(D) ? mx_splits(D, (int)P) : 1));
   b += al(tc_tile_words((int)P + T, (int)E + 1) * 4);
   b += al(scratch_rec_bytes(D, T));
   if (D.shared) {
@@ -900,12 +908,8 @@ static void scratch_carve(pm_ctx *c, const pm_layer_desc &D, int T, Scratch &S) 
   S.hbsum = ws_take<int32_t>(c, P * (ff / 32));
   S.hbm = ws_take<uint16_t>(c, P * (ff / 16));
   S.hs = ws_take<int32_t>(c, P * (ff / 256 + 1));
-  S.eo = ws_take<float>(c, Pm * d);
-  S.xhl = S.hhl = nullptr;
-  if (D.act_quant == PM_AQ_F32 && D.type_gate == PM_TYPE_MXFP4) {
-    S.xhl = ws_take<uint16_t>(c, 2 * T * d);
-    S.hhl = ws_take<uint16_t>(c, 2 * P * ff);
-  }
+  S.eo = ws_take<float>(c, Pm * d * (mx_layer(D) ? mx_splits(D, (int)P) : 1));
+  S.eo_parts = 1;
   S.tiles = ws_take<uint32_t>(c, tc_tile_words((int)P + T, (int)E + 1));
   S.seg = ws_take<uint32_t>(c, route_seg_words(T, D.n_exp));
   S.rec = ws_take<uint8_t>(c, scratch_rec_bytes(D, T));
@@ -947,7 +951,7 @@ struct Path {
   bool mx;         // bf16 tensor-core products for MXFP4 weights and f32 activations (tolerance parity, not bits)
   bool merge;      // the shared expert is one more group of the routed experts' launches
 };
-static Path pick_path(pm_layer *ly, int T, const Scratch &S) {
+static Path pick_path(pm_layer *ly, int T) {
   const pm_ctx *c = ly->ctx;
   const pm_layer_desc &D = ly->dev.desc;
   Path p;
@@ -957,8 +961,9 @@ static Path pick_path(pm_layer *ly, int T, const Scratch &S) {
   const int int_min = c->tc_min_set ? c->tc_min_tokens : (shared_merges(D) ? 1 : 2);
   p.tc = D.act_quant == PM_AQ_Q8X_256 && c->tc_min_tokens > 0 && T >= int_min;
   p.tc_gu = p.tc && D.type_gate == D.type_up;
-  p.mx = c->tc_min_tokens > 0 && T >= c->tc_min_tokens && D.act_quant == PM_AQ_F32 && D.type_gate == PM_TYPE_MXFP4 &&
-         D.type_up == PM_TYPE_MXFP4 && D.type_down == PM_TYPE_MXFP4 && S.xhl;
+  // (MXFP4: from two tokens up until the caller says otherwise; a layer of 32 experts, d = ff = 2880, row kernels against
+  // these: 1 token 60 : 66 us, 2 tokens 97 : 97, 4 tokens 162 : 130, 8 tokens 300 : 181)
+  p.mx = mx_layer(D) && c->tc_min_tokens > 0 && T >= (c->tc_min_set ? c->tc_min_tokens : 2);
   p.merge = p.tc_gu && shared_merges(D);
   return p;
 }
@@ -966,7 +971,7 @@ static TcTiles path_tiles(pm_layer *ly, int T, const Path &p, const Scratch &S, 
   const pm_layer_desc &D = ly->dev.desc;
   TcTiles t{};
   if (p.tc || p.mx)
-    t = tc_tiles_of(S.tiles, T * D.top_k, D.n_exp, p.mx ? 1 : std::min(D.n_exp, ly->dev.n_local), merge ? T : 0);
+    t = tc_tiles_of(S.tiles, T * D.top_k, D.n_exp, std::min(D.n_exp, ly->dev.n_local), merge ? T : 0, p.mx);
   return t;
 }
 
@@ -978,7 +983,7 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
   const LayerDev &dv = ly->dev;
   const pm_layer_desc &D = dv.desc;
   Launch L = c->launch();
-  const Path path = pick_path(ly, T, S);
+  const Path path = pick_path(ly, T);
   const bool tc = path.tc, tc_gu = path.tc_gu;
   Groups g = plan_groups(S.plan, D.n_exp);
   const int P = T * D.top_k;
@@ -993,22 +998,24 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
     launch_tc_tiles(L, dv, g, tt);
   }
   if (path.mx) {
-    const size_t nx = (size_t)T * D.d, nh = (size_t)P * D.ff;
+    // (few tokens: three pieces hold every bit of an f32; prompts: two, see prefill_mx.cu)
+    const int pieces = T < PM_MX_PROMPT ? 3 : 2;
+    S.eo_parts = made ? mx_splits(D, P) : 1;  // (the other callers take the pair outputs themselves)
     {
       PROF(c, PH_QUANT_X);
-      launch_split_bf16(L, x, nx, S.xhl, S.xhl + nx);
+      launch_mx_rows(L, P, tt, g.pair_token, D.d, x, pieces, S.rec);
     }
     {
       PROF(c, PH_GATEUP);
-      CU(launch_tc_mx(L, dv, false, g, P, tt, S.xhl, S.xhl + nx, w, S.h, c->dev_err, c->wait_ns));
+      CU(launch_tc_mx(L, dv, false, g.pair_src, tt, pieces, S.rec, w, S.h, 1, 0, c->dev_err, c->wait_ns));
     }
     {
       PROF(c, PH_QUANT_H);
-      launch_split_bf16(L, S.h, nh, S.hhl, S.hhl + nh);
+      launch_mx_rows(L, P, tt, nullptr, D.ff, S.h, pieces, S.rec);
     }
     {
       PROF(c, PH_DOWN);
-      CU(launch_tc_mx(L, dv, true, g, P, tt, S.hhl, S.hhl + nh, nullptr, S.eo, c->dev_err, c->wait_ns));
+      CU(launch_tc_mx(L, dv, true, g.pair_src, tt, pieces, S.rec, nullptr, S.eo, S.eo_parts, (size_t)P * D.d, c->dev_err, c->wait_ns));
     }
     c->path_count[PM_PATH_TENSOR] += 2;
     CU(cudaGetLastError());
@@ -1075,10 +1082,10 @@ static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
   if (!D.shared) return PM_OK;
   PROF(c, PH_SHARED);
   Launch L = c->launch();
-  const Path path = pick_path(ly, T, S);
+  const Path path = pick_path(ly, T);
   const bool use_tc = path.tc, tc_gu = path.tc_gu;
   TcTiles tt{};
-  if (use_tc) tt = tc_tiles_of(S.tiles, T, 1, 1, 0);
+  if (use_tc) tt = tc_tiles_of(S.tiles, T, 1, 1, 0, false);
   launch_shared_groups(L, S.one, S.zero_u, S.tcount, S.iota, T, tt);
   Groups g;
   g.n_groups = S.one;
@@ -1115,7 +1122,7 @@ static int32_t dev_forward(pm_layer *ly, const float *x, int T, float *y, bool a
   pm_ctx *c = ly->ctx;
   const LayerDev &dv = ly->dev;
   Launch L = c->launch();
-  const Path path = pick_path(ly, T, S);
+  const Path path = pick_path(ly, T);
   const TcTiles tt = path_tiles(ly, T, path, S, path.merge);
   if (route_plan_small_takes(dv, x, T)) {  // a few tokens: logits, top-k, plan and tiles in one launch
     PROF(c, PH_ROUTER);
@@ -1134,7 +1141,7 @@ static int32_t dev_forward(pm_layer *ly, const float *x, int T, float *y, bool a
   }
   {
     PROF(c, PH_COMBINE);
-    launch_combine(L, dv, S.eo, S.plan.pair_pos, S.w, shared_out, S.shared_logit, T, y, accumulate);
+    launch_combine(L, dv, S.eo, S.plan.pair_pos, S.w, shared_out, S.shared_logit, T, y, accumulate, S.eo_parts);
   }
   CU(cudaGetLastError());
   return PM_OK;

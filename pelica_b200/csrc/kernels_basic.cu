@@ -742,9 +742,10 @@ __global__ void __launch_bounds__(512) k_plan_seg_scan(PlanDev pl, int E, int T,
     pm_scan2_512(nt, rp, ft, r0, at, ar, sh);
     if (c > 0) {
       const int el = e - first_local;
+      const uint32_t each = tc_tile_tokens(c, nt, tt.ntok, tt.even);
       for (uint32_t i = 0; i < nt && (int)(ft + i) < tt.max_tiles; i++)
-        tt.tiles[ft + i] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, o + i * tt.ntok,
-                                      min(c - i * tt.ntok, (uint32_t)tt.ntok), r0 + i * tt.ntok);
+        tt.tiles[ft + i] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, o + i * each,
+                                      min(c - i * each, each), r0 + i * each);
     }
     uint32_t st = 0;
     if (tt.shared) {  // the shared expert as one more group: every token, pairs total .. total + T - 1
@@ -1730,7 +1731,7 @@ __global__ void __launch_bounds__(256) k_combine(int d, int K, int in_combine,
                                                  const float *__restrict__ w,
                                                  const float *__restrict__ shared_out,
                                                  const float *__restrict__ shared_logit, float *y,
-                                                 int accumulate) {
+                                                 int accumulate, int parts, size_t part_stride) {
   pm_pdl();
   const int t = blockIdx.y;
   const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
@@ -1741,6 +1742,11 @@ __global__ void __launch_bounds__(256) k_combine(int d, int K, int in_combine,
     const uint32_t p = pair_pos[t * K + k];
     float4 v = p == PM_PAIR_NONE ? make_float4(0.0f, 0.0f, 0.0f, 0.0f)  // a pair whose expert id was refused
                                  : __ldcs((const float4 *)(eo + (size_t)p * d + c));
+    for (int i = 1; i < parts; i++) {  // (products cut along K: the other parts of the sum)
+      if (p == PM_PAIR_NONE) break;
+      const float4 u = __ldcs((const float4 *)(eo + i * part_stride + (size_t)p * d + c));
+      v = make_float4(__fadd_rn(v.x, u.x), __fadd_rn(v.y, u.y), __fadd_rn(v.z, u.z), __fadd_rn(v.w, u.w));
+    }
     if (in_combine) {
       const float wk = w[t * K + k];
       v = make_float4(__fmul_rn(wk, v.x), __fmul_rn(wk, v.y), __fmul_rn(wk, v.z), __fmul_rn(wk, v.w));
@@ -1766,13 +1772,13 @@ __global__ void __launch_bounds__(256) k_combine(int d, int K, int in_combine,
 
 void launch_combine(const Launch &L, const LayerDev &ly, const float *eo, const uint32_t *pair_pos,
                     const float *w, const float *shared_out, const float *shared_logit, int T,
-                    float *y, bool accumulate) {
+                    float *y, bool accumulate, int parts) {
   if (T == 0) return;
   int d = ly.desc.d;
   dim3 grid((d + 1023) / 1024, T);
   PLAUNCH(L, k_combine, grid, 256, 0, d, ly.desc.top_k,
           (int)(ly.desc.weight_fold == PM_FOLD_IN_COMBINE), eo, pair_pos, w, shared_out,
-          shared_logit, y, (int)accumulate);
+          shared_logit, y, (int)accumulate, parts, (size_t)T * ly.desc.top_k * d);
 }
 
 // x / rms(x), unit weight; the sum order is pm_rms_inv's (common.cuh)

@@ -27,7 +27,7 @@ struct WMat {
 };
 
 // TMA descriptions of a family's planes as [expert][row][bytes of the row], boxes of 64 rows (gate, up) or 128 rows
-// (down) x one 256-value block (Q4_K: plane 0; Q6_K: ql, qh). Host memory of the layer: launchers copy them into parameters.
+// (down) x one 256-value block (Q4_K: plane 0; Q6_K: ql, qh; MXFP4: the nibbles, with 64 and with 128 rows). Host memory of the layer: launchers copy them into parameters.
 struct WMaps {
   CUtensorMap m[2];
 };
@@ -163,9 +163,15 @@ struct TcTiles {
   unsigned int *next;  // [2] item counters of the gate/up and the down launch (each list serves one of each)
   uint4 *tiles;        // (expert slot or ~0, first pair, pairs, first record row)
   int ntok;            // tokens of a full tile (128, or 64 where the groups are small)
+  int even;            // a group's tiles have the same number of tokens (of 16) instead of ntok and a remainder
   int shared;          // the list holds the shared expert as one more group (pairs P .. P + T - 1)
   int max_tiles;
 };
+// tokens of each of the n tiles that cnt pairs make. Even tiles for the bf16 products: a weight tile is decoded once a
+// token tile at a cost that a tile of a few tokens does not hide.
+__host__ __device__ inline uint32_t tc_tile_tokens(uint32_t cnt, uint32_t n, int ntok, int even) {
+  return even && n > 1 ? ((cnt + n - 1) / n + 15u) & ~15u : (uint32_t)ntok;
+}
 bool route_plan_small_takes(const LayerDev &ly, const float *x, int T);
 void launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits, uint32_t *ids,
                              float *w, PlanDev pl, const int32_t *slot_table, unsigned int *ticket, const TcTiles &tt, int *err,
@@ -181,6 +187,7 @@ void launch_gateup(const Launch &L, const LayerDev &ly, bool shared, Groups g, i
 void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int n_pairs,
                  const float *h, const int8_t *hq, const float *hd, const int32_t *hbsum,
                  float *eo);
+#define PM_MX_PROMPT 32  // tokens from which the bf16 products use two pieces of a value (below: three)
 #define TC_SHARED 0x40000000u  // expert slot of a tile of the shared expert
 // tensor-core (tcgen05 int8) form of launch_gateup / launch_down for Q4_K / Q6_K x Q8x (prefill_tc.cu):
 // the token tiles of a grouping (one list serves both products), the activation rows regrouped by expert
@@ -188,8 +195,8 @@ void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int
 // src_row: row of the activations that holds pair p (null: row p itself)
 size_t tc_tile_words(int n_pairs, int max_groups);
 // n_groups: groups that can have pairs (the experts this GPU holds)
-// shared_tokens: tokens of the shared expert's group in the same list (0: none)
-TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens);  // buf: tc_tile_words words, 16-byte aligned
+// shared_tokens: tokens of the shared expert's group in the same list (0: none); mx: for launch_tc_mx
+TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, bool mx);  // buf: tc_tile_words words, 16-byte aligned
 size_t tc_rec_bytes(int n_pairs, int max_groups, int cols);
 void launch_tc_tiles(const Launch &L, const LayerDev &ly, Groups g, const TcTiles &t);
 void launch_tc_quant_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x,
@@ -198,11 +205,16 @@ void launch_tc_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_
                     const float *xd, const uint16_t *xbm, const int32_t *xs, uint8_t *rec);
 cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared_only, bool down, const uint32_t *pair_src, const TcTiles &t,
                       const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns, int fault_block);
-// tensor-core (tcgen05 bf16) form for MXFP4 weights and f32 activations given as their bf16
-// (hi, lo) split (prefill_mx.cu); launch_split_bf16 makes the split: hi[n], lo[n] bf16
-void launch_split_bf16(const Launch &L, const float *x, size_t n, void *hi, void *lo);
-cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, Groups g, int n_pairs, const TcTiles &t,
-                         const void *xhi, const void *xlo, const float *wts, float *out, int *err,
+// tensor-core (tcgen05 bf16) form for MXFP4 weights and f32 activations (prefill_mx.cu). The rows are regrouped
+// by tile and split into 2 or 3 bf16 pieces a value (rec: mx_rec_bytes bytes); the down products may be cut along
+// K into mx_splits parts: part s goes to out + s * split_stride.
+size_t mx_rec_bytes(int n_pairs, int max_groups, int cols);
+int mx_small_tokens();
+int mx_splits(const pm_layer_desc &D, int n_pairs);
+void launch_mx_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x, int pieces,
+                    uint8_t *rec);
+cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t, int pieces,
+                         const uint8_t *rec, const float *wts, float *out, int splits, size_t split_stride, int *err,
                          unsigned long long wait_ns);
 // expert parallelism (kernels_basic.cu): per-rank pair counts, the wire records of a dispatch,
 // the received (expert, weight) records, the derived forms of received Q8x group sums
@@ -216,7 +228,7 @@ void launch_ep_unmeta(const Launch &L, int R, const uint32_t *meta, int first, i
 void launch_q8x_aux(const Launch &L, size_t n_blocks, const int32_t *bsum, uint16_t *bm, int32_t *xs);
 void launch_combine(const Launch &L, const LayerDev &ly, const float *eo, const uint32_t *pair_pos,
                     const float *w, const float *shared_out, const float *shared_logit, int T,
-                    float *y, bool accumulate);
+                    float *y, bool accumulate, int parts = 1);
 void launch_rmsnorm(const Launch &L, const float *x, int T, int d, float eps, float *out);
 void launch_shared_gate_logit(const Launch &L, const LayerDev &ly, const float *x, int T,
                               float *out);

@@ -1,462 +1,627 @@
-// prefill_mx.cu - grouped expert products for many tokens per expert on MXFP4 weights and
-// f32 activations (the gpt-oss path, src/oss_prefill.rs:237,548) on the 5th-gen tensor cores:
-// tcgen05.mma kind::f16 with bf16 operands, f32 accumulators in tensor memory.
+// prefill_mx.cu - grouped expert products on MXFP4 weights and f32 activations (the gpt-oss path,
+// src/oss_prefill.rs:237,548) on the 5th-gen tensor cores: tcgen05.mma kind::f16 with bf16 operands, operand A
+// and the f32 accumulators in tensor memory.
 //
 // MXFP4 weights are exact in bf16 (a one-bit mantissa times a power of two: the E2M1 code
 // doubled, times the halved E8M0 scale, src/oss_kernels.rs:41-55), the f32 activations are
-// not: each is split x = hi + lo into two bf16 values (lo = bf16(x - hi)) by a small kernel
-// before the products, and every K step runs twice, W * hi and W * lo, into the same
-// accumulator. Products of two bf16 values are exact in f32, so what differs from the f32
-// reference path (src/oss_batch.rs:774-789) is the 2^-17 relative residue of the split and
-// the summation order: parity is the layer tolerance (1e-3 relative + 1e-4 of the RMS), not bits.
+// not: each is split into bf16 pieces, x = x1 + x2 (+ x3), xi = bf16(what is left), and every K step runs once a
+// piece into the same accumulator. Products of two bf16 values are exact in f32. Three pieces hold all 24 bits of
+// an f32: calls of fewer than 32 tokens, which otherwise run on f32 multiply-adds, use them. Prompts use two:
+// what differs from the f32 reference path (src/oss_batch.rs:774-789) is then the 2^-17 relative residue and the
+// summation order; parity is the layer tolerance (1e-3 relative + 1e-4 of the RMS), not bits.
 //
-// One CTA = (128 weight rows of one active expert: 64 gate + 64 up, or 128 down rows) x
-// (up to 128 of its tokens): 16 worker warps and one warp that issues the products. K runs
-// in chunks of 64 values (two MXFP4 blocks) through a ring of MX_ST stages:
-//   workers: the chunk's activations (bf16, gathered through the token list) arrive by
-//            cp.async two chunks ahead; the chunk's weight nibbles and scale bytes arrive in
-//            registers one chunk ahead, are decoded to bf16 and stored as operand A in the
-//            canonical K-major layout ([8 K-chunks][128 rows][16 B]);
-//   issuer:  waits for the stage (named barrier), runs 4 K steps x (hi, lo) products and
-//            commits them to the stage's mbarrier, which the workers wait on before they
-//            refill that stage.
-// One accumulator for the whole K (the block scale lives in the bf16 weight), so there is no
-// per-block float step as in the exact integer kernels. Epilogue: bias + GLU (gate/up,
-// src/oss_prefill.rs:339) or bias (down; the routing weight is applied at combine,
-// src/oss_prefill.rs:342). Waits are time-bounded; tensor memory is freed on every path.
+// A persistent pipeline like the int8 kernel's (prefill_tc.cu): a producer thread brings the weights' nibbles in
+// by TMA (boxes of 256 K values) and the tokens' pieces by one bulk copy a chunk of 64 K values; the workers decode
+// a block of 32 codes a thread and store it to tensor memory, up to four chunks ahead of the products; work items
+// come from a counter. One accumulator for the whole K (the block scale lives in the bf16 weight).
+//  BIG (more than 16 pairs a group on average): a CTA an SM takes 256 weight rows (128 gate rows and the same 128
+//    rows of up, or 256 down rows) x 128 tokens. Both halves multiply one staging of the tokens' pieces, which
+//    halves what comes from L2: 31 bytes a cycle an SM; with 128 rows it would be the limit, 62. Gate and up sums of
+//    an output sit in the same thread. Bound by the tensor pipe (1,050 cycles a chunk; decoding takes about 500).
+//  else: two CTAs an SM of half the tensor memory, 128 rows (64 gate + 64 up, or 128 down) x 32 tokens. Bound by
+//    the weights' bytes and the decode. Down rows may be cut along K (launch_tc_mx), so that a few tokens fill the SMs.
 #include <cuda_bf16.h>
 
-#include "moe_internal.cuh"
+#include "tcgen.cuh"
 
-#define MX_NW 512
-#define MX_NT (MX_NW + 32)
 #define MX_M 128
-#define MX_NMAX 128
-#define MX_KC 64            /* K values per stage */
-#define MX_ST 4             /* stages */
-#define MX_TMEM_COLS 128
-#define MX_A_BYTES (8 * MX_M * 16)                 /* operand A of a stage */
-#define MX_B_BYTES (8 * (MX_NMAX + 1) * 16)        /* one of the two B operands of a stage (odd pitch) */
-#define MX_STAGE (MX_A_BYTES + 2 * MX_B_BYTES)
+#define MX_KC 64   /* K values of a chunk */
+#define MX_NA 4    /* chunks of operand A in tensor memory */
+#define MX_BOX (MX_M * 128)   /* nibbles of 128 rows x 256 K values */
 
-__device__ __forceinline__ uint32_t mx_s32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned long long mx_now() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-// shared-memory matrix descriptor, K-major, no swizzle: 8x16 B core matrices,
-// lbo = bytes between the two 16-byte K chunks of one product, sbo = bytes between 8-row groups
-__device__ __forceinline__ uint64_t mx_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((saddr >> 4) & 0x3fff) | ((uint64_t)((lbo >> 4) & 0x3fff) << 16) |
-         ((uint64_t)((sbo >> 4) & 0x3fff) << 32) | (1ull << 46);
-}
-__device__ __forceinline__ void mx_mma(uint32_t tmem_c, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_c),
-      "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// one lane of a converged warp: issuing under this predicate keeps the operands in uniform registers
-// (a product every 10-12 cycles; under "lane == 0" 48, which bound every tile of fewer than 96 tokens)
-__device__ __forceinline__ bool mx_elect() {
-  uint32_t p;
-  asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));
-  return p != 0;
-}
-__device__ __forceinline__ void mx_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mx_s32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void mx_ld8(uint32_t taddr, uint32_t r[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-}
-__device__ __forceinline__ void mx_cp16(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ bool mx_bar_test(uint64_t *bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(mx_s32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// false after the wait limit (or at once when an error is already recorded)
-__device__ __noinline__ bool mx_bar_wait(uint64_t *bar, uint32_t parity, int *err, unsigned long long wait_ns) {
-  unsigned long long t0 = mx_now();
-  for (uint32_t it = 0;; it++) {
-    if (mx_bar_test(bar, parity)) return true;
-    if ((it & 15) == 15 && (*(volatile int *)err != 0 || mx_now() - t0 > wait_ns)) break;
-  }
-  atomicCAS(err, 0, 8);
-  return false;
-}
-
-// x -> (hi, lo) bf16 with hi + lo = x up to 2^-17 relative
-__global__ void __launch_bounds__(256) k_split_bf16(const float *__restrict__ x, size_t n, __nv_bfloat16 *hi,
-                                                    __nv_bfloat16 *lo) {
-  pm_pdl();
-  size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
-  if (i >= n) return;
-  const float v = x[i];
-  const __nv_bfloat16 h = __float2bfloat16_rn(v);
-  hi[i] = h;
-  lo[i] = __float2bfloat16_rn(__fsub_rn(v, __bfloat162float(h)));
-}
-void launch_split_bf16(const Launch &L, const float *x, size_t n, void *hi, void *lo) {
-  if (n == 0) return;
-  pm_launch(L, k_split_bf16, (unsigned)((n + 255) / 256), 256, 0, x, n, (__nv_bfloat16 *)hi, (__nv_bfloat16 *)lo);
-}
-
-// Four E2M1 codes (one in the low nibble of each byte of c4) -> the four bf16 patterns of
-// code * 2^(e-128), as two words (codes 0,1 and 2,3), by byte-table look-ups (prmt): the low
-// and the high byte of the offset {0, 0, 128, 192, 256, 320, 384, 448}[m] that magnitude m adds to
-// the scale's own pattern `base2` ((e - 1) << 7 in both halves), the sign into bit 15, and a
-// mask that zeroes the lanes with m = 0.
-__device__ __forceinline__ void mx_decode4(uint32_t c4, uint32_t base2, uint32_t &w01, uint32_t &w23) {
-  const uint32_t m = c4 & 0x07070707u;
-  const uint32_t sel = (m & 0x7u) | ((m >> 4) & 0x70u) | ((m >> 8) & 0x700u) | ((m >> 12) & 0x7000u);
-  const uint32_t lo = __byte_perm(0xc0800000u, 0xc0804000u, sel);
-  const uint32_t hi = __byte_perm(0x00000000u, 0x01010101u, sel);
-  const uint32_t nz = __byte_perm(0xffffff00u, 0xffffffffu, sel);
-  const uint32_t hs = hi | ((c4 & 0x08080808u) << 4);
-  const uint32_t d01 = __byte_perm(lo, hs, 0x5140), d23 = __byte_perm(lo, hs, 0x7362);
-  w01 = (d01 + base2) & __byte_perm(nz, nz, 0x1100);
-  w23 = (d23 + base2) & __byte_perm(nz, nz, 0x3322);
-}
-
-// Compile with -DPM_MX_TRACE to stamp the phases of CTA (0, 0) with the SM clock:
-// [worker thread 0 | issuing thread][chunk][stamp]; read back with pm_debug_mx_trace.
-#ifdef PM_MX_TRACE
-__device__ unsigned long long g_mx_trace[2 * 64 * 8];
-#define MX_STAMP(who, kc, i)                                                                   \
-  if (blockIdx.x == 0 && blockIdx.y == 0 && (kc) < 64) g_mx_trace[(((who) * 64) + (kc)) * 8 + (i)] = clock64();
-extern "C" __attribute__((visibility("default"))) int pm_debug_mx_trace(unsigned long long *out) {
-  return (int)cudaMemcpyFromSymbol(out, g_mx_trace, sizeof(g_mx_trace));
-}
-#else
-#define MX_STAMP(who, kc, i)
-#endif
-
-struct MxArgs {
-  LayerDev ly;
-  int down;               // 0: gate+up with activation -> h; 1: down -> pair outputs
-  Groups g;
-  const __nv_bfloat16 *xhi, *xlo;  // gate/up: [T][cols] by token; down: [P][cols] by pair
-  const float *wts;       // routing weights [T*K] (gate/up with fold) or null
-  float *out;             // gate/up: h [P][ff]; down: eo [P][d]
-  int *err;
-  unsigned long long wait_ns;
-  const int *n_tiles;
-  const uint4 *tiles;
+template <bool BIG, int NPC> struct MxShape {
+  static constexpr int MT = BIG ? 2 : 1;                 // 128-row halves of a CTA
+  static constexpr int NW = BIG ? 512 : 256, NT = NW + 64;
+  static constexpr int CTAS = BIG ? 1 : 2;
+  static constexpr int NTOK = BIG ? 128 : 32;
+  static constexpr uint32_t COLS = BIG ? 512 : 256;      // tensor memory: accumulators, then MX_NA chunks of operand A
+  static constexpr uint32_t A0 = BIG ? 256 : 128, ACH = MT * MX_KC / 2;  // first column, columns a chunk
+  static constexpr int RAWB = MT * MX_BOX, NSR = 3;
+  static constexpr int BST = NTOK * MX_KC * 2 * NPC, NSB = 4;
+  static constexpr int XB = BIG ? 0 : NTOK * MX_M * 4;   // gate/up: exchange of the sums
+  static constexpr int NACC = BIG ? 1 : 2;               // accumulators of the first piece
 };
 
-__global__ void __launch_bounds__(MX_NT, 1) k_tc_mx(const MxArgs A) {
-  pm_pdl();
-  extern __shared__ __align__(128) uint8_t smem[];
-  if ((int)blockIdx.y >= *A.n_tiles) return;
-  const uint4 tile = A.tiles[blockIdx.y];
-  const LayerDev &ly = A.ly;
-  const WMat &W0 = A.down ? ly.down : ly.gate;
-  const WMat &W1 = ly.up;
-  const int cols = W0.cols, nb = cols / 32, rows = W0.rows;
-  const int nkc = (cols + MX_KC - 1) / MX_KC;  // K chunks (the last one may hold a single block)
-  const int el = (int)tile.x;
-  const uint32_t first = tile.y;  // first pair
-  const int nvalid = (int)tile.z;
-  const int npad = (nvalid + 15) & ~15;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const bool local = el >= 0 && el < ly.n_local;
-  const int rows_per_cta = A.down ? MX_M : MX_M / 2;
-  const int r0 = blockIdx.x * rows_per_cta;
-  if (!local) {  // an expert another rank holds: zeros (down) / nothing to do (gate/up)
-    if (A.down)
-      for (int i = tid; i < nvalid * MX_M; i += MX_NT) {
-        int n = i / MX_M, m = i % MX_M;
-        if (r0 + m < rows) A.out[(size_t)(first + n) * rows + r0 + m] = 0.0f;
-      }
-    return;
-  }
-  uint8_t *sStage = smem;                               // [MX_ST] x (A, B hi, B lo)
-  float *sS = (float *)smem;                            // (after the last chunk) gate/up exchange [128][129]
-  uint64_t *bar_empty = (uint64_t *)(smem + MX_ST * MX_STAGE);  // [MX_ST] products of a stage done
-  uint64_t *bar_done = bar_empty + MX_ST;
-  uint32_t *tmem_slot = (uint32_t *)(bar_done + 1);
+__device__ __forceinline__ void mx_mma_ta(uint32_t tmem_c, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(tmem_c),
+      "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 
-  if (warp == MX_NW / 32) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(mx_s32(tmem_slot)),
-                 "r"((uint32_t)MX_TMEM_COLS)
-                 : "memory");
+// A block: 16 bytes of E2M1 codes (value j in the low nibble of byte j, value j + 16 in the high one) and its E8M0
+// scale e -> 32 bf16. Two codes a word, 16 bits apart, in the order they lie in: word 4 j + i is nibbles i and i + 4
+// of the j-th word, the values (4 j, 4 j + 2), (16 + 4 j, 18 + 4 j), (4 j + 1, 4 j + 3), (17 + 4 j, 19 + 4 j) for
+// i = 0 .. 3 (k_mx_rows puts the tokens' values into the same order). The code's three magnitude bits at bits 8..6 of
+// a bf16 are the code times 2^-126 (its subnormal included), so one multiplication by 2^(e - 1) makes the value; four
+// ALU instructions and a multiplication a word, where look-ups of both bytes by prmt took ten (and the prmt, shifts
+// and logic, 64 lanes a cycle, were what the workers waited for: 2,070 -> 1,150 cycles a chunk).
+__device__ __forceinline__ uint32_t mx_mul2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ void mx_codes(const uint4 q, uint32_t scale2, uint32_t *w) {
+  const uint32_t v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    w[4 * j] = mx_mul2(((v[j] << 6) & 0x01c001c0u) | ((v[j] << 12) & 0x80008000u), scale2);
+    w[4 * j + 1] = mx_mul2(((v[j] << 2) & 0x01c001c0u) | ((v[j] << 8) & 0x80008000u), scale2);
+    w[4 * j + 2] = mx_mul2(((v[j] >> 2) & 0x01c001c0u) | ((v[j] << 4) & 0x80008000u), scale2);
+    w[4 * j + 3] = mx_mul2(((v[j] >> 6) & 0x01c001c0u) | (v[j] & 0x80008000u), scale2);
+  }
+}
+// scales outside 2 .. 128
+__device__ __forceinline__ void mx_codes_any(const uint4 q, uint32_t e, uint32_t *w) {
+  if (e >= 2u && e < 250u) {  // 2^(e - 1) in two steps: 2^127 is the largest power a bf16 holds
+    mx_codes(q, min(e + 126u, 254u) * 0x00800080u, w);
+    const uint32_t more2 = (e > 128u ? e - 1u : 127u) * 0x00800080u;
+#pragma unroll
+    for (int i = 0; i < 16; i++) w[i] = mx_mul2(w[i], more2);
+  } else {  // the scale's own subnormal branch (src/oss_kernels.rs:42-45) and scales near the top of the range: through f32
+    const uint32_t v[4] = {q.x, q.y, q.z, q.w};
+    const float s = pm_e8(e);
+    auto cv = [&](uint32_t c) { return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(s, pm_e2m1(c & 15u)))); };
+#pragma unroll
+    for (int i = 0; i < 16; i++) w[i] = cv(v[i >> 2] >> (4 * (i & 3))) | (cv(v[i >> 2] >> (4 * (i & 3) + 16)) << 16);
+  }
+}
+
+struct MxArgs {
+  CUtensorMap m0, m1;     // nibble planes of gate or down, of up
+  const uint8_t *s0, *s1; // their planes of scale bytes
+  size_t s0_stride, s1_stride;
+  const uint4 *tiles;
+  const int *n_tiles;
+  unsigned int *next;
+  const uint8_t *rec;     // the tokens' pieces (k_mx_rows)
+  const float *bias0, *bias1;
+  const float *wts;
+  const uint32_t *pair_src;
+  float *out;             // gate/up: h [P][ff]; down: eo [splits][P][d]
+  size_t split_stride;
+  int *err;
+  unsigned long long wait_ns;
+  int row_tiles, splits, split_chunks;
+  int cols, rows;
+  int act;
+  float act_limit, act_alpha;
+};
+
+// f32 rows -> the products' operand: per tile and chunk of 64 K values [piece][8 K groups][rows][8 bf16], rows padded
+// to 16 with zeros; a K group of 8 is values 4 j .. 4 j + 3 and 16 + 4 j .. of a block of 32, in the order the decoded
+// weights have. A thread a (row, K group): neighbouring lanes take neighbouring rows, whose 16 bytes are neighbours
+// in the operand.
+template <int NPC>
+__global__ void __launch_bounds__(256) k_mx_rows(const int *__restrict__ n_tiles, const uint4 *__restrict__ tiles,
+                                                 const uint32_t *__restrict__ src_row, int cols, const float *__restrict__ x,
+                                                 uint8_t *__restrict__ rec) {
+  pm_pdl();
+  if ((int)blockIdx.y >= *n_tiles) return;
+  const uint4 T = tiles[blockIdx.y];
+  const int npad = ((int)T.z + 15) & ~15, nch = (cols + MX_KC - 1) / MX_KC;
+  uint8_t *base = rec + (size_t)T.w * nch * (MX_KC * 2 * NPC);
+  for (int u = blockIdx.x * 256 + threadIdx.x; u < nch * 8 * npad; u += gridDim.x * 256) {
+    const int g = u / npad, r = u - g * npad;  // K group of 8 values, row of the tile
+    float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    if (r < (int)T.z && 8 * g < cols) {
+      const size_t row = src_row ? src_row[T.y + r] : T.y + r;
+      const float4 *src = (const float4 *)(x + row * cols + (g >> 2) * 32 + (g & 3) * 4);
+      const float4 a = __ldg(src), b = __ldg(src + 4);  // (the order of mx_decode_block)
+      v[0] = a.x; v[1] = a.z; v[2] = b.x; v[3] = b.z; v[4] = a.y; v[5] = a.w; v[6] = b.y; v[7] = b.w;
+    }
+    uint8_t *dst = base + (size_t)(g >> 3) * (npad * MX_KC * 2 * NPC) + ((g & 7) * npad + r) * 16;
+#pragma unroll
+    for (int p = 0; p < NPC; p++) {
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const __nv_bfloat16 a = __float2bfloat16_rn(v[2 * i]), b = __float2bfloat16_rn(v[2 * i + 1]);
+        v[2 * i] = __fsub_rn(v[2 * i], __bfloat162float(a));
+        v[2 * i + 1] = __fsub_rn(v[2 * i + 1], __bfloat162float(b));
+        w[i] = (uint32_t)__bfloat16_as_ushort(a) | ((uint32_t)__bfloat16_as_ushort(b) << 16);
+      }
+      *(uint4 *)(dst + (size_t)p * npad * MX_KC * 2) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+
+struct MxItem {
+  uint4 t;
+  int r0, c0, c1, split;  // first row, K chunks [c0, c1), which cut of K
+};
+#define MX_IT 4
+#define MX_END 0xfffffffeu
+
+template <bool DOWN, bool BIG, int NPC>
+__global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS) k_tc_mx(const __grid_constant__ MxArgs A) {
+  using S = MxShape<BIG, NPC>;
+  constexpr int MW = S::NW / 32, NSR = S::NSR, NSB = S::NSB, MT = S::MT;
+  constexpr int RPC = DOWN ? MT * MX_M : MT * MX_M / 2;  // matrix rows of an item
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t *sRaw = smem, *sB = sRaw + NSR * S::RAWB;
+  float *sX = (float *)(sB + NSB * S::BST);
+  MxItem *items = (MxItem *)((uint8_t *)sX + (DOWN ? 0 : S::XB));
+  uint64_t *full_raw = (uint64_t *)(items + MX_IT), *empty_raw = full_raw + NSR, *full_b = empty_raw + NSR, *empty_b = full_b + NSB;
+  uint64_t *a_ready = empty_b + NSB, *a_free = a_ready + MX_NA, *acc_full = a_free + MX_NA, *acc_free = acc_full + S::NACC;
+  uint64_t *it_full = acc_free + S::NACC, *it_empty = it_full + MX_IT;
+  uint32_t *tmem_slot = (uint32_t *)(it_empty + MX_IT);
+  const int nbk = A.cols / 32, rows = A.rows, nch = (A.cols + MX_KC - 1) / MX_KC;
+  const int tid = threadIdx.x, warp = __shfl_sync(PM_FULL, tid >> 5, 0), lane = tid & 31;
+
+  pm_pdl_trigger();
+  if (warp == MW) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_s32(tmem_slot)), "r"(S::COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
-    for (int i = 0; i <= MX_ST; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mx_s32(bar_empty + i)), "r"(1));
+    for (int i = 0; i < NSR; i++) {
+      tc_mbar_init(full_raw + i, 1);
+      tc_mbar_init(empty_raw + i, MW);
+    }
+    for (int i = 0; i < NSB; i++) {
+      tc_mbar_init(full_b + i, 1);
+      tc_mbar_init(empty_b + i, 1);  // the products' commit (nobody else reads the tokens' pieces)
+    }
+    for (int i = 0; i < MX_NA; i++) {
+      tc_mbar_init(a_ready + i, MW / 2);
+      tc_mbar_init(a_free + i, 1);
+    }
+    for (int i = 0; i < S::NACC; i++) {
+      tc_mbar_init(acc_full + i, 1);
+      tc_mbar_init(acc_free + i, MW);
+    }
+    for (int i = 0; i < MX_IT; i++) {
+      tc_mbar_init(it_full + i, 1);
+      tc_mbar_init(it_empty + i, 1 + MW);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
-  const uint32_t sStage_a = mx_s32(sStage);
-  const uint32_t bpitch = (uint32_t)(npad + 1) * 16u;
+  const uint32_t tmem = __reduce_max_sync(PM_FULL, *tmem_slot);
+  pm_pdl_wait();  // (barriers and tensor memory were prepared under the kernel before)
+  auto next_item = [&](int k, MxItem &it) -> bool {
+    const int s = k & (MX_IT - 1);
+    const bool ok = tc_wait(it_full + s, (uint32_t)((k / MX_IT) & 1), A.err, A.wait_ns);
+    it = items[s];
+    __syncwarp();
+    if (lane == 0) tc_mbar_arrive(it_empty + s);
+    return ok && it.t.x != MX_END;
+  };
 
-  if (warp == MX_NW / 32) {
+  if (warp == MW) {
     // ================= the issuing warp =================
-    // instruction descriptor: D f32, A and B bf16, both K-major, N = npad, M = 128
-    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(npad >> 3) << 17) | ((uint32_t)(MX_M >> 4) << 24);
-    const uint64_t da0 = mx_desc(sStage_a, MX_M * 16u, 128u);
-    const uint64_t dbh0 = mx_desc(sStage_a + MX_A_BYTES, bpitch, 128u);
-    for (int kc = 0; kc < nkc; kc++) {
-      const int s = kc % MX_ST;
-      // full[s]: named barrier 1 + s (workers arrive, this warp waits)
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + s), "n"(MX_NT) : "memory");
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (mx_elect()) {
-        MX_STAMP(1, kc, 0)
-        // (descriptors of stage s, step ks = those of stage 0, step 0 plus the byte offset >> 4 in
-        // the address field: shared memory addresses stay below 2^18)
-        const uint32_t so = (uint32_t)s * MX_STAGE;
-        const int ksteps = min(4, (cols - kc * MX_KC) / 16);  // (a trailing single block: 2 steps)
+    const uint32_t el = tc_elect() ? 1u : 0u;
+    const uint32_t sB_a = tc_s32(sB);
+    uint32_t st = 0, sb = 0, pb = 0, n_acc = 0;
+    MxItem it;
+    for (int k = 0; next_item(k, it); k++) {
+      if ((int)it.t.x < 0) continue;
+      const uint32_t npad = (__reduce_max_sync(PM_FULL, it.t.z) + 15u) & ~15u;
+      const int c0 = (int)__reduce_max_sync(PM_FULL, (uint32_t)it.c0), c1 = (int)__reduce_max_sync(PM_FULL, (uint32_t)it.c1);
+      // instruction descriptor: D f32, A and B bf16, both K-major, N = npad, M = 128
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((npad >> 3) << 17) | ((uint32_t)(MX_M >> 4) << 24);
+      // the accumulators of the item before have been read (n_acc: hand-overs of accumulators so far)
+      if (n_acc > 0) tc_wait(acc_free + (n_acc - 1) % S::NACC, ((n_acc - 1) / S::NACC) & 1, A.err, A.wait_ns);
+      uint32_t d_main = tmem, first = 0;  // first piece's accumulator; its first chunk
+      for (int c = c0; c < c1; c++) {
+        const uint32_t a = (uint32_t)(c - c0) & 3u;
+        if (!BIG && a == 0) {
+          const uint32_t set = n_acc & 1;
+          if (n_acc > 1) tc_wait(acc_free + set, ((n_acc >> 1) - 1) & 1, A.err, A.wait_ns);
+          d_main = tmem + set * 32u;
+          first = (uint32_t)(c - c0);
+        }
+        const uint64_t dB = tc_desc(sB_a + sb * S::BST, npad * 16u, 128u);
+        const int ksteps = min(4, (A.cols - c * MX_KC) / 16);  // (a trailing single block: 2 steps)
+        tc_wait(full_b + sb, pb, A.err, A.wait_ns);
+        tc_wait(a_ready + a, st & 1, A.err, A.wait_ns);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (el) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ks++) {
-          if (ks < ksteps) {
-            const uint64_t da = da0 + ((so + (uint32_t)(2 * ks) * (MX_M * 16u)) >> 4);
-            const uint64_t dbh = dbh0 + ((so + (uint32_t)(2 * ks) * bpitch) >> 4);
-            const uint64_t dbl = dbh + (MX_B_BYTES >> 4);
-            mx_mma(tmem, da, dbh, idesc, (kc > 0 || ks > 0) ? 1u : 0u);
-            mx_mma(tmem, da, dbl, idesc, 1u);
+          for (int h = 0; h < MT; h++)
+#pragma unroll
+            for (int ks = 0; ks < 4; ks++)
+              if (ks < ksteps) {
+#pragma unroll
+                for (int p = 0; p < NPC; p++) {  // (a piece is npad * 128 bytes, a K step two groups of npad * 16)
+                  const uint32_t at = tmem + S::A0 + a * S::ACH + h * (MX_KC / 2) + 8u * ks;
+                  const uint64_t db = dB + (uint64_t)(p * npad * 8 + ks * npad * 2);
+                  if (BIG) mx_mma_ta(tmem + h * 128u, at, db, idesc, (c > c0 || ks > 0 || p > 0) ? 1u : 0u);
+                  else if (p == 0) mx_mma_ta(d_main, at, db, idesc, (c - c0 > (int)first || ks > 0) ? 1u : 0u);
+                  else mx_mma_ta(tmem + 64u, at, db, idesc, (c > c0 || ks > 0 || p > 1) ? 1u : 0u);
+                }
+              }
+          tc_commit(a_free + a);
+          tc_commit(empty_b + sb);
+          if (c == c1 - 1 || (!BIG && a == 3)) tc_commit(acc_full + n_acc % S::NACC);
+        }
+        __syncwarp();
+        if (c == c1 - 1 || (!BIG && a == 3)) n_acc++;
+        if (a == 3) st++;
+        if (++sb == NSB) { sb = 0; pb ^= 1; }
+      }
+      // (a last group of fewer than four chunks: its other places in the ring go round empty)
+      for (uint32_t a = (uint32_t)(c1 - c0) & 3u; a != 0 && a < 4; a++) {
+        tc_wait(a_ready + a, st & 1, A.err, A.wait_ns);
+        if (el) tc_mbar_arrive(a_free + a);
+        if (a == 3) st++;
+      }
+    }
+  } else if (warp == MW + 1) {
+    // ================= the producer: one thread =================
+    if (tc_elect()) {
+      const uint32_t sRaw_a = tc_s32(sRaw), sB_a = tc_s32(sB);
+      const int per_tile = A.row_tiles * A.splits, n_items = *A.n_tiles * per_tile, G = (int)gridDim.x;
+      int cur = (int)blockIdx.x, nxt = cur + G;
+      uint4 Tc = make_uint4(MX_END, 0, 0, 0), Tn = Tc;
+      if (cur < n_items) Tc = __ldg(A.tiles + cur / per_tile);
+      uint32_t sr = 0, pr = 1, sb = 0, pb = 1, nr = 0, nbk_ = 0;
+      bool ok = true;
+      for (int k = 0; ok; k++) {
+        const int s = k & (MX_IT - 1);
+        if (k >= MX_IT && !tc_wait(it_empty + s, (uint32_t)((k / MX_IT - 1) & 1), A.err, A.wait_ns)) break;
+        const bool end = cur >= n_items;
+        const int in = cur % per_tile, rt = in / A.splits, sp = in - rt * A.splits;
+        const int r0 = rt * RPC, c0 = sp * A.split_chunks, c1 = min(nch, c0 + A.split_chunks);
+        MxItem it;
+        it.t = end ? make_uint4(MX_END, 0, 0, 0) : Tc;
+        it.r0 = r0;
+        it.c0 = c0;
+        it.c1 = c1;
+        it.split = sp;
+        items[s] = it;
+        tc_mbar_arrive(it_full + s);
+        if (end) break;
+        const int fut = 2 * G + (int)atomicAdd(A.next, 1u);  // (needed an item later)
+        if (nxt < n_items) Tn = __ldg(A.tiles + nxt / per_tile);
+        if ((int)Tc.x >= 0) {
+          const int el = (int)Tc.x;
+          const uint32_t bytes = ((Tc.z + 15) >> 4) * (16u * MX_KC * 2 * NPC);
+          const uint8_t *rec = A.rec + (size_t)Tc.w * nch * (MX_KC * 2 * NPC);
+          for (int c = c0; c < c1; c++) {
+            if (((c - c0) & 3) == 0) {  // nibbles of four chunks (a box past the matrix reads zeros; split_chunks is a multiple of 4)
+              const uint32_t r = sRaw_a + sr * S::RAWB;
+              if (nr >= NSR && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
+              tc_mbar_expect(full_raw + sr, (uint32_t)S::RAWB);
+              if (DOWN) {
+                tc_tma3(r, &A.m0, c * 32, r0, el, full_raw + sr);
+                if (BIG) tc_tma3(r + MX_BOX, &A.m0, c * 32, r0 + MX_M, el, full_raw + sr);
+              } else {  // (boxes of 128 rows, or of 64 in the small shape)
+                tc_tma3(r, &A.m0, c * 32, r0, el, full_raw + sr);
+                tc_tma3(r + (BIG ? MX_BOX : MX_BOX / 2), &A.m1, c * 32, r0, el, full_raw + sr);
+              }
+              nr++;
+              if (++sr == NSR) { sr = 0; pr ^= 1; }
+            }
+            if (nbk_ >= NSB && !tc_wait(empty_b + sb, pb, A.err, A.wait_ns)) { ok = false; break; }
+            tc_mbar_expect(full_b + sb, bytes);
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sB_a + sb * S::BST),
+                         "l"(rec + (size_t)c * bytes), "r"(bytes), "r"(tc_s32(full_b + sb))
+                         : "memory");
+            nbk_++;
+            if (++sb == NSB) { sb = 0; pb ^= 1; }
           }
         }
-        mx_commit(&bar_empty[s]);
-        if (kc == nkc - 1) mx_commit(bar_done);
-        MX_STAMP(1, kc, 1)
+        cur = nxt;
+        nxt = fut;
+        Tc = Tn;
       }
-      __syncwarp();
+      // the last copies have landed before the CTA gives up its shared memory
+      for (uint32_t i = 1; i <= NSR && i <= nr; i++) {
+        const uint32_t q = nr - i;
+        const unsigned long long t0 = tc_now();
+        while (!tc_bar_test(full_raw + q % NSR, (q / NSR) & 1) && tc_now() - t0 < A.wait_ns) {
+        }
+      }
+      for (uint32_t i = 1; i <= NSB && i <= nbk_; i++) {
+        const uint32_t q = nbk_ - i;
+        const unsigned long long t0 = tc_now();
+        while (!tc_bar_test(full_b + q % NSB, (q / NSB) & 1) && tc_now() - t0 < A.wait_ns) {
+        }
+      }
     }
+    __syncwarp();
   } else {
     // ================= the workers =================
-    // B: thread = (token t of the tile, K chunk c of 8 values): 2 x 16 B a stage (hi, lo);
-    // 128 tokens x 8 chunks = 1024 pieces, two a thread
-    int brow[2];
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-      const int t = (tid >> 3) + 64 * i;
-      brow[i] = t < nvalid ? (A.down ? (int)(first + t) : (int)A.g.pair_token[first + t]) : -1;
-    }
-    const int bc = tid & 7;
-    // (through registers: 16-byte cp.async moves about 21 bytes a cycle per SM, a chunk's 32 KB of
-    // activations would take three times as long as its products)
-    uint4 breg[4];
-    auto load_b = [&](int kc) {  // the tokens' chunk kc -> registers
-      const int k0 = kc * MX_KC + 8 * bc;
-      const bool on = kc < nkc && k0 < cols;
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        if (on && brow[i] >= 0) {
-          breg[2 * i] = __ldg((const uint4 *)(A.xhi + (size_t)brow[i] * cols + k0));
-          breg[2 * i + 1] = __ldg((const uint4 *)(A.xlo + (size_t)brow[i] * cols + k0));
-        }
-      }
-    };
-    auto store_b = [&](int kc) {  // registers -> chunk kc's stage
-      if (kc >= nkc) return;
-      uint8_t *sb = sStage + (size_t)(kc % MX_ST) * MX_STAGE + MX_A_BYTES;
-      if (kc * MX_KC + 8 * bc >= cols) return;
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        if (brow[i] < 0) continue;
-        const int t = (tid >> 3) + 64 * i;
-        uint8_t *dst = sb + (size_t)bc * bpitch + (size_t)t * 16;
-        *(uint4 *)dst = breg[2 * i];
-        *(uint4 *)(dst + MX_B_BYTES) = breg[2 * i + 1];
-      }
-    };
-    // padding tokens (and, in a trailing half chunk, the missing K): zero operands, once
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-      const int t = (tid >> 3) + 64 * i;
-      if (t >= nvalid && t < npad)
-        for (int st = 0; st < MX_ST; st++) {
-          uint8_t *sb = sStage + (size_t)st * MX_STAGE + MX_A_BYTES;
-          *(uint4 *)(sb + (size_t)bc * bpitch + (size_t)t * 16) = make_uint4(0, 0, 0, 0);
-          *(uint4 *)(sb + MX_B_BYTES + (size_t)bc * bpitch + (size_t)t * 16) = make_uint4(0, 0, 0, 0);
-        }
-    }
-    // A: thread = (row m of the tile, quarter q of the chunk): block b2 = q >> 1 of the chunk's
-    // two, bytes 8 h .. 8 h + 7 of its 16 (h = q & 1): values 8 h + i (low nibbles) -> K chunk
-    // 4 b2 + h, values 16 + 8 h + i (high nibbles) -> K chunk 4 b2 + 2 + h
-    const int m = tid & 127, q = tid >> 7, b2 = q >> 1, hh = q & 1;
-    const bool second = !A.down && m >= 64;  // the row belongs to the up matrix
-    const int grow = r0 + (second ? m - 64 : m);
-    const bool rvalid = grow < rows;
-    const WMat &W = second ? W1 : W0;
-    const uint8_t *nibp = W.plane[0] + (size_t)el * W.stride[0] + (size_t)(rvalid ? grow : 0) * nb * 16 + 8 * hh;
-    const uint8_t *sclp = W.plane[1] + (size_t)el * W.stride[1] + (size_t)(rvalid ? grow : 0) * nb;
-    uint2 raw = make_uint2(0, 0);
-    uint32_t rsc = 0;
-    auto load_a = [&](int kc) {  // chunk kc's bytes of this thread -> registers
-      const int blk = 2 * kc + b2;
-      if (kc < nkc && rvalid && blk < nb) {
-        raw = __ldg((const uint2 *)(nibp + (size_t)blk * 16));
-        rsc = __ldg(sclp + blk);
-      } else {
-        raw = make_uint2(0, 0);
-        rsc = 0;
-      }
-    };
-    auto store_a = [&](int kc, const uint2 raw, const uint32_t rsc) {  // (the bytes loaded one chunk earlier)
-      uint8_t *sa = sStage + (size_t)(kc % MX_ST) * MX_STAGE;
-      // (e < 2, the scale's own subnormal branch, src/oss_kernels.rs:42-45, and scales near the top of the range: decoded through f32)
-      uint32_t lo4[4], hi4[4];
-      if ((rsc >= 2u && rsc < 250u) || (raw.x | raw.y) == 0u) {
-        const uint32_t base2 = ((rsc - 1u) << 7) * 0x00010001u;
-        mx_decode4(raw.x, base2, lo4[0], lo4[1]);
-        mx_decode4(raw.y, base2, lo4[2], lo4[3]);
-        mx_decode4(raw.x >> 4, base2, hi4[0], hi4[1]);
-        mx_decode4(raw.y >> 4, base2, hi4[2], hi4[3]);
-      } else {
-        const float s = pm_e8(rsc);
-        const uint32_t w[2] = {raw.x, raw.y};
-#pragma unroll
-        for (int j = 0; j < 2; j++)
-#pragma unroll
-          for (int p = 0; p < 2; p++) {
-            const uint32_t b0 = (w[j] >> (16 * p)) & 0xffu, b1 = (w[j] >> (16 * p + 8)) & 0xffu;
-            auto cv = [&](uint32_t c) { return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(s, pm_e2m1(c)))); };
-            lo4[2 * j + p] = cv(b0 & 15u) | (cv(b1 & 15u) << 16);
-            hi4[2 * j + p] = cv(b0 >> 4) | (cv(b1 >> 4) << 16);
-          }
-      }
-      *(uint4 *)(sa + (size_t)(4 * b2 + hh) * (MX_M * 16) + (size_t)m * 16) = make_uint4(lo4[0], lo4[1], lo4[2], lo4[3]);
-      *(uint4 *)(sa + (size_t)(4 * b2 + 2 + hh) * (MX_M * 16) + (size_t)m * 16) = make_uint4(hi4[0], hi4[1], hi4[2], hi4[3]);
-    };
-
-    // chunk 0's activations directly, chunk 1's and the weight bytes of chunk 0 in registers
-    // (one chunk ahead: two chunks ahead, with twice the registers, measured slower)
-    load_b(0);
-    store_b(0);
-    load_b(1);
-    load_a(0);
-    bool dead = false;
-    for (int kc = 0; kc < nkc; kc++) {
-      const int s = kc % MX_ST;
-      if (tid == 0) { MX_STAMP(0, kc, 0) }
-      // chunk kc + 1's activations (in registers since the last round) go to the stage that held
-      // chunk kc + 1 - MX_ST: its products must be done
-      if (kc + 1 >= MX_ST && kc + 1 < nkc) {
-        const int kp = kc + 1 - MX_ST;  // (completion number kp / MX_ST of that stage's barrier)
-        if (!dead && !mx_bar_wait(&bar_empty[kp % MX_ST], (uint32_t)((kp / MX_ST) & 1), A.err, A.wait_ns)) dead = true;
-      }
-      if (tid == 0) { MX_STAMP(0, kc, 1) }
-      store_b(kc + 1);
-      load_b(kc + 2);
-      if (tid == 0) { MX_STAMP(0, kc, 2) }
-      // this chunk's own stage held chunk kc - MX_ST: waited for in the last round (as kc + 1 then).
-      // The next chunk's weight bytes are requested before this chunk's are decoded.
-      const uint2 raw_now = raw;
-      const uint32_t rsc_now = rsc;
-      load_a(kc + 1);
-      store_a(kc, raw_now, rsc_now);
-      if (tid == 0) { MX_STAMP(0, kc, 3) }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      asm volatile("bar.arrive %0, %1;" ::"r"(1 + s), "n"(MX_NT) : "memory");
-      if (tid == 0) { MX_STAMP(0, kc, 5) }
-    }
-    // ---- epilogue: all products done -> TMEM lane m, a quarter of the token columns ----
-    if (!mx_bar_test(bar_done, 0)) mx_bar_wait(bar_done, 0, A.err, A.wait_ns);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // decode: thread = (row m of a 128-row half, half h); the even chunks or the odd ones (two blocks of 32 codes each)
+    const int m = tid & 127, part = warp >> 2, h = BIG ? part >> 1 : 0, par = part & 1;
     const uint32_t tlane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-    const int part = tid >> 7;
-    const int ew = npad >> 2, ecol0 = part * ew;  // npad / 4 columns: a multiple of 4
-    float total[32];
-#pragma unroll
-    for (int c8 = 0; c8 < 32; c8 += 8) {
-      if (c8 < ew) {
-        uint32_t v[8];
-        // (ew is a multiple of 4: the second half of an 8-wide read may lie past this quarter; it is ignored below)
-        mx_ld8(tlane + (uint32_t)(ecol0 + c8), v);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-        for (int u = 0; u < 8; u++) total[c8 + u] = __uint_as_float(v[u]);
+    uint32_t st = 0, sr = 0, pr = 0, n_acc = 0;
+    MxItem it;
+    for (int k = 0; next_item(k, it); k++) {
+      const uint4 T = it.t;
+      const int el = (int)T.x, nvalid = (int)T.z, npad = (nvalid + 15) & ~15, r0 = it.r0;
+      float *out = A.out + (size_t)it.split * A.split_stride + (size_t)T.y * rows;
+      if (el < 0) {  // an expert another rank holds: zeros (down) / nothing to do (gate/up)
+        if (DOWN)
+          for (int i = tid; i < nvalid * RPC; i += S::NW) {
+            const int n = i / RPC, mm = i - n * RPC;
+            if (r0 + mm < rows) out[(size_t)n * rows + r0 + mm] = 0.0f;
+          }
+        continue;
       }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    asm volatile("bar.sync 6, %0;" ::"n"(MX_NW) : "memory");  // the stages are dead: their memory carries the exchange
-    const bool bad = *(volatile int *)A.err != 0;
-    if (A.down) {
-      if (!bad) {
-        const float bd = (ly.bias_down && rvalid) ? ly.bias_down[(size_t)el * rows + grow] : 0.0f;
+      // the matrix row this thread decodes: the up matrix holds half 1, or (small shape) rows 64 .. 127 of the tile
+      const bool up = !DOWN && (BIG ? h == 1 : m >= 64);
+      const int drow = DOWN ? r0 + h * MX_M + m : (BIG ? r0 + m : r0 + (m & 63));
+      // its scale bytes, eight blocks (four chunks) at a time: two aligned words hold them wherever the row starts
+      const uint8_t *sp = (up ? A.s1 + (size_t)el * A.s1_stride : A.s0 + (size_t)el * A.s0_stride) + (size_t)min(drow, rows - 1) * nbk;
+      auto scales = [&](int c) -> unsigned long long {
+        const uintptr_t p = (uintptr_t)(sp + 2 * c);
+        const unsigned long long *q = (const unsigned long long *)(p & ~(uintptr_t)7);
+        const int sh = 8 * (int)(p & 7);
+        const unsigned long long a = __ldg(q), b = __ldg(q + 1);
+        return sh ? (a >> sh) | (b << (64 - sh)) : a;
+      };
+      // small shape: the thread's columns of the products of the first piece, summed up here every 256 K values
+      const int ew = BIG ? 0 : npad >> 1, ec0 = par * ew;
+      float acc[16];
+      if (!BIG)
 #pragma unroll
-        for (int i = 0; i < 32; i++) {
-          const int n = ecol0 + i;
-          if (i < ew && n < nvalid && rvalid) {
-            float o = total[i];
-            if (ly.bias_down) o = __fadd_rn(o, bd);
-            A.out[(size_t)(first + n) * rows + grow] = o;
+        for (int u = 0; u < 16; u++) acc[u] = 0.0f;
+      auto fold = [&](bool last) {
+        const uint32_t set = n_acc & 1;
+        tc_wait(acc_full + set, (n_acc >> 1) & 1, A.err, A.wait_ns);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int c8 = 0; c8 < 16; c8 += 8)
+          if (c8 < ew) {
+            uint32_t v[8];
+            tc_ld8<0>(tlane + set * 32u + (uint32_t)(ec0 + c8), v);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int u = 0; u < 8; u++) acc[c8 + u] = __fadd_rn(acc[c8 + u], __uint_as_float(v[u]));
+            if (last) {
+              tc_ld8<64>(tlane + (uint32_t)(ec0 + c8), v);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+              for (int u = 0; u < 8; u++) acc[c8 + u] = __fadd_rn(acc[c8 + u], __uint_as_float(v[u]));
+            }
+          }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) tc_mbar_arrive(acc_free + set);
+        n_acc++;
+      };
+      unsigned long long sc_n = scales(it.c0);
+      for (int c4 = it.c0; c4 < it.c1; c4 += 4) {
+        const unsigned long long sc = sc_n;
+        if (c4 + 4 < it.c1) sc_n = scales(c4 + 4);
+        tc_wait(full_raw + sr, pr, A.err, A.wait_ns);
+        const uint8_t *raw = sRaw + sr * S::RAWB + h * MX_BOX + m * 128;
+        uint4 q[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++)  // (TMA swizzle: 16-byte piece i of a row sits at i ^ (row & 7))
+          q[j] = *(const uint4 *)(raw + (((4 * (j >> 1) + 2 * par + (j & 1)) ^ (m & 7)) << 4));
+#pragma unroll
+        for (int j = 0; j < 4; j++) asm volatile("" : "+r"(q[j].x), "+r"(q[j].y), "+r"(q[j].z), "+r"(q[j].w));
+        __syncwarp();
+        if (lane == 0) tc_mbar_arrive(empty_raw + sr);
+        if (++sr == NSR) { sr = 0; pr ^= 1; }
+        auto stored = [&](int a) {  // the stores to operand A's chunk a are done
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) tc_mbar_arrive(a_ready + a);
+        };
+        const uint32_t ew4[2] = {(uint32_t)sc >> (16 * par), (uint32_t)(sc >> 32) >> (16 * par)};
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          const int a = 2 * j + par;
+          const bool on = c4 + a < it.c1;
+          uint32_t w[32];
+          if (on) {
+            const uint32_t e0 = ew4[j] & 0xffu, e1 = (ew4[j] >> 8) & 0xffu;
+            if (__any_sync(PM_FULL, max(e0 - 2u, e1 - 2u) > 126u)) {
+              mx_codes_any(q[2 * j], e0, w);
+              mx_codes_any(q[2 * j + 1], e1, w + 16);
+            } else {
+              mx_codes(q[2 * j], (e0 + 126u) * 0x00800080u, w);
+              mx_codes(q[2 * j + 1], (e1 + 126u) * 0x00800080u, w + 16);
+            }
+          }
+          if (j > 0) stored(par);  // (the wait for a chunk's stores comes after the next one's decode)
+          tc_wait(a_free + a, (st & 1) ^ 1, A.err, A.wait_ns);
+          if (on) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            tc_st32(tlane + S::A0 + a * S::ACH + h * (MX_KC / 2), w);
           }
         }
+        stored(2 + par);
+        st++;
+        if (!BIG && c4 > it.c0) fold(false);  // (of the 256 K values before: these are still being multiplied)
       }
-    } else {
+      // ---- epilogue: TMEM lane m, the part's token columns ----
+      if (BIG) {
+        tc_wait(acc_full, n_acc & 1, A.err, A.wait_ns);
+        n_acc++;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      } else {
+        fold(true);
+      }
+      const bool dead = *(volatile int *)A.err != 0;
+      if (DOWN) {
+        const float bd = A.bias0 && it.split == 0 && drow < rows ? A.bias0[(size_t)el * rows + drow] : 0.0f;
+        const bool on = !dead && drow < rows, bias = A.bias0 && it.split == 0;
+        auto put = [&](int n, float o) {
+          if (bias) o = __fadd_rn(o, bd);
+          if (on && n < nvalid) out[(size_t)n * rows + drow] = o;
+        };
+        if constexpr (BIG) {
+          const int hw = npad >> 1, c0 = par * hw;  // half of the columns: a multiple of 8
+          for (int c8 = 0; c8 < hw; c8 += 8) {
+            uint32_t v[8];
+            tc_ld8<0>(tlane + h * 128u + (uint32_t)(c0 + c8), v);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int i = 0; i < 32; i++)
-        if (i < ew) sS[m * (MX_NMAX + 1) + ecol0 + i] = total[i];
-      asm volatile("bar.sync 6, %0;" ::"n"(MX_NW) : "memory");
-      const pm_layer_desc &D = ly.desc;
-      const bool fold = D.weight_fold == PM_FOLD_BEFORE_DOWN && A.wts;
-      const bool bias = ly.bias_gate != nullptr;
-      if (!bad)
-        for (int i = tid; i < nvalid * 64; i += MX_NW) {
-          const int j = i & 63, n = i >> 6;
-          if (r0 + j >= rows) continue;
-          float gv = sS[j * (MX_NMAX + 1) + n], uv = sS[(64 + j) * (MX_NMAX + 1) + n];
-          if (bias) {
-            gv = __fadd_rn(gv, ly.bias_gate[(size_t)el * rows + r0 + j]);
-            uv = __fadd_rn(uv, ly.bias_up[(size_t)el * rows + r0 + j]);
+            for (int u = 0; u < 8; u++) put(c0 + c8 + u, __uint_as_float(v[u]));
           }
-          const uint32_t p = first + n;
-          const float w = fold ? A.wts[A.g.pair_src[p]] : 1.0f;
-          A.out[(size_t)p * rows + r0 + j] = pm_act(D.act, D.act_limit, D.act_alpha, gv, uv, w, fold);
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) tc_mbar_arrive(acc_free);
+        } else {
+#pragma unroll
+          for (int u = 0; u < 16; u++)
+            if (u < ew) put(ec0 + u, acc[u]);
         }
+      } else {
+        const int hrow = BIG ? r0 + m : r0 + (m & 63);  // the h row this thread activates
+        const bool on = !dead && hrow < rows;
+        const float bg = A.bias0 && hrow < rows ? A.bias0[(size_t)el * rows + hrow] : 0.0f;
+        const float bu = A.bias0 && hrow < rows ? A.bias1[(size_t)el * rows + hrow] : 0.0f;
+        auto put = [&](int n, float gv, float uv) {
+          if (A.bias0) {
+            gv = __fadd_rn(gv, bg);
+            uv = __fadd_rn(uv, bu);
+          }
+          const float wt = A.wts ? A.wts[A.pair_src[T.y + n]] : 1.0f;
+          out[(size_t)n * rows + hrow] = pm_act(A.act, A.act_limit, A.act_alpha, gv, uv, wt, A.wts != nullptr);
+        };
+        if constexpr (BIG) {  // gate sums in columns 0 .., up sums in 128 ..: a quarter of the tokens a thread
+          const int qw = npad >> 2, c0 = part * qw;
+          for (int c4 = 0; c4 < qw; c4 += 4) {
+            uint32_t vg[4], vu[4];
+            tc_ld4<0>(tlane + (uint32_t)(c0 + c4), vg);
+            tc_ld4<128>(tlane + (uint32_t)(c0 + c4), vu);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+              if (on && c0 + c4 + u < nvalid) put(c0 + c4 + u, __uint_as_float(vg[u]), __uint_as_float(vu[u]));
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) tc_mbar_arrive(acc_free);
+        } else {  // gate rows in lanes 0..63, up rows in 64..127: the warps w and w ^ 2 exchange through shared memory
+          float *sx = sX + par * (S::NTOK / 2) * MX_M;
+#pragma unroll
+          for (int u = 0; u < 16; u++)
+            if (u < ew) sx[u * MX_M + m] = acc[u];
+          asm volatile("bar.sync %0, 64;" ::"r"(1 + 2 * par + (warp & 1)) : "memory");
+          const int f = up ? ew >> 1 : 0;
+#pragma unroll 2
+          for (int i = f; i < f + (ew >> 1); i++)
+            if (on && ec0 + i < nvalid) put(ec0 + i, sx[i * MX_M + (m & 63)], sx[i * MX_M + 64 + (m & 63)]);
+          // (nobody writes the area again before every warp has stored operand A of the next item's first chunk)
+        }
+      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == MX_NW / 32)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)MX_TMEM_COLS) : "memory");
+  if (warp == MW) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::COLS) : "memory");
 }
 
-// Tensor-core form of launch_gateup / launch_down for MXFP4 weights and f32 activations given
-// as their bf16 (hi, lo) split.
-cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, Groups g, int n_pairs, const TcTiles &t,
-                         const void *xhi, const void *xlo, const float *wts, float *out, int *err,
+// bytes of the pieces of n_pairs rows of `cols` values in at most max_groups groups, three pieces a value
+size_t mx_rec_bytes(int n_pairs, int max_groups, int cols) {
+  const size_t groups = (size_t)(max_groups < n_pairs ? max_groups : n_pairs);
+  return ((size_t)n_pairs + 15 * groups + 16) * ((cols + MX_KC - 1) / MX_KC) * (MX_KC * 2 * 3);
+}
+void launch_mx_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x, int pieces,
+                    uint8_t *rec) {
+  const long units = ((long)n_rows + 15 * t.max_tiles) * ((cols + 7) / 8);
+  const long gx = (units / t.max_tiles + 511) / 512;  // two units a thread
+  const dim3 grid((unsigned)(gx < 1 ? 1 : gx), (unsigned)t.max_tiles);
+  if (pieces == 3) pm_launch(L, k_mx_rows<3>, grid, 256, 0, t.n, t.tiles, src_row, cols, x, rec);
+  else pm_launch(L, k_mx_rows<2>, grid, 256, 0, t.n, t.tiles, src_row, cols, x, rec);
+}
+
+template <bool DOWN, bool BIG, int NPC> static cudaError_t mx_start(const Launch &L, const MxArgs &A, long items) {
+  using S = MxShape<BIG, NPC>;
+  constexpr size_t smem = (size_t)S::NSR * S::RAWB + (size_t)S::NSB * S::BST + (DOWN ? 0 : S::XB) + MX_IT * sizeof(MxItem) +
+                          (2 * S::NSR + 2 * S::NSB + 2 * MX_NA + 2 * S::NACC + 2 * MX_IT) * 8 + 16;
+  static_assert(smem <= (S::CTAS == 1 ? 232448 : 115712), "more than an SM's shared memory");
+  static bool set[64] = {};  // (one-time per device and kernel)
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !set[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(k_tc_mx<DOWN, BIG, NPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    if (dev < 64) set[dev] = true;
+  }
+  const long ctas = (long)S::CTAS * L.n_sm;
+  return pm_launch(L, k_tc_mx<DOWN, BIG, NPC>, dim3((unsigned)(items < ctas ? items : ctas)), S::NT, smem, A);
+}
+
+int mx_small_tokens() { return MxShape<false, 2>::NTOK; }
+// Cuts of K of the down products: a few tokens make ceil(d / 128) items an expert, each a chain of ff / 64 chunks;
+// while that leaves CTAs without work, K is cut in up to four (the combine step adds the parts in order).
+static int mx_split_chunks(int nch, int splits) { return ((nch + splits - 1) / splits + 3) & ~3; }  // whole boxes
+int mx_splits(const pm_layer_desc &D, int n_pairs) {
+  const int nch = (D.ff + MX_KC - 1) / MX_KC;
+  // (a pair is at most a tile of its own; two CTAs on each of 148 SMs)
+  const long items = (long)((D.d + MX_M - 1) / MX_M) * n_pairs;
+  long s = 296 / (items > 0 ? items : 1);
+  s = s > 4 ? 4 : s;
+  s = s > nch / 8 ? nch / 8 : s;  // at least eight chunks each
+  if (s <= 1) return 1;
+  const int sc = mx_split_chunks(nch, (int)s);
+  return (nch + sc - 1) / sc;  // (rounding up may leave fewer)
+}
+
+// Tensor-core form of launch_gateup / launch_down for MXFP4 weights and f32 activations given as the pieces of
+// the grouping's rows. splits: cuts of K (down only); split s goes to out + s * split_stride.
+cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t, int pieces,
+                         const uint8_t *rec, const float *wts, float *out, int splits, size_t split_stride, int *err,
                          unsigned long long wait_ns) {
-  if (n_pairs == 0) return cudaSuccess;
-  const WMat &W = down ? ly.down : ly.gate;
-  const size_t ex = (size_t)MX_M * (MX_NMAX + 1) * 4;
-  const size_t smem = ((size_t)MX_ST * MX_STAGE > ex ? (size_t)MX_ST * MX_STAGE : ex) + 8 * (MX_ST + 1) + 16;
-  cudaError_t e = cudaFuncSetAttribute((const void *)k_tc_mx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
+  if (t.max_tiles == 0) return cudaSuccess;
+  const bool big = t.ntok != MxShape<false, 2>::NTOK;
+  const WMat &W0 = down ? ly.down : ly.gate, &W1 = ly.up;
+  const WMaps &M0 = down ? ly.maps->down : ly.maps->gate, &M1 = ly.maps->up;
   MxArgs A;
-  A.ly = ly;
-  A.down = down;
-  A.g = g;
-  A.xhi = (const __nv_bfloat16 *)xhi;
-  A.xlo = (const __nv_bfloat16 *)xlo;
-  A.wts = wts;
+  const int box = !down && !big ? 0 : 1;  // boxes of 64 or 128 rows
+  A.m0 = M0.m[box];
+  A.m1 = M1.m[box];
+  A.s0 = W0.plane[1];
+  A.s0_stride = W0.stride[1];
+  A.s1 = W1.plane[1];
+  A.s1_stride = W1.stride[1];
+  A.tiles = t.tiles;
+  A.n_tiles = t.n;
+  A.next = t.next + (down ? 1 : 0);
+  A.rec = rec;
+  A.bias0 = down ? ly.bias_down : ly.bias_gate;
+  A.bias1 = down ? nullptr : ly.bias_up;
+  A.wts = !down && ly.desc.weight_fold == PM_FOLD_BEFORE_DOWN ? wts : nullptr;
+  A.pair_src = pair_src;
   A.out = out;
+  A.split_stride = split_stride;
   A.err = err;
   A.wait_ns = wait_ns;
-  A.n_tiles = t.n;
-  A.tiles = t.tiles;
-  const int row_tiles = down ? (W.rows + MX_M - 1) / MX_M : (W.rows + 63) / 64;
-  dim3 grid(row_tiles, t.max_tiles);
-  pm_launch(L, k_tc_mx, grid, MX_NT, smem, A);
-  return cudaGetLastError();
+  const int rpc = down ? (big ? 2 * MX_M : MX_M) : (big ? MX_M : MX_M / 2);
+  A.row_tiles = (W0.rows + rpc - 1) / rpc;
+  const int nch = (W0.cols + MX_KC - 1) / MX_KC;
+  A.split_chunks = mx_split_chunks(nch, splits);
+  A.splits = splits;
+  A.cols = W0.cols;
+  A.rows = W0.rows;
+  A.act = ly.desc.act;
+  A.act_limit = ly.desc.act_limit;
+  A.act_alpha = ly.desc.act_alpha;
+  const long items = (long)A.row_tiles * A.splits * t.max_tiles;
+  if (big) return down ? mx_start<true, true, 2>(L, A, items) : mx_start<false, true, 2>(L, A, items);
+  if (pieces == 3) return down ? mx_start<true, false, 3>(L, A, items) : mx_start<false, false, 3>(L, A, items);
+  return down ? mx_start<true, false, 2>(L, A, items) : mx_start<false, false, 2>(L, A, items);
 }

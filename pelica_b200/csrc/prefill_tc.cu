@@ -26,10 +26,9 @@
 // What bounds a block of 128 rows x 128 tokens: tensor pipe 2 x 17 products of N = 64 = 1,150 cycles;
 // CUDA cores about 350 (unpack) + 100 (operand store) + 2 x 450 (float terms: five rounded steps an
 // output, as f32x2 pairs, behind an integer add and a conversion).
-#include <cuda.h>  // CUtensorMap (encoded through the runtime's driver entry point)
 #include <cuda_fp16.h>
 
-#include "moe_internal.cuh"
+#include "tcgen.cuh"
 
 // The tokens' operand is read from records laid out for the products (k_tc_quant_rows writes them):
 // record (8 rows, block b) = [16 K chunks][8 rows][16 B] int8 activations, [2 K chunks][8 rows][8 f16]
@@ -69,152 +68,6 @@ template <int PARTS, bool Q6, bool DOWN> struct TcStages {
   static constexpr int tok = PARTS == 2 && Q6 && !DOWN ? 2 : 3;
 };
 
-__device__ __forceinline__ uint32_t tc_s32(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ unsigned long long tc_now() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-// shared-memory matrix descriptor, K-major, no swizzle: 8x16 B core matrices,
-// lbo = bytes between the two 16-byte K chunks of one MMA, sbo = bytes between
-// 8-row groups
-__device__ __forceinline__ uint64_t tc_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((saddr >> 4) & 0x3fff) | ((uint64_t)((lbo >> 4) & 0x3fff) << 16) |
-         ((uint64_t)((sbo >> 4) & 0x3fff) << 32) | (1ull << 46);
-}
-// D[tmem_c] (+)= A[tmem_a] * B[db]: A from tensor memory (row = lane, 32-bit column c =
-// K values 4c..4c+3), B from shared memory
-__device__ __forceinline__ void tc_mma_i8_ta(uint32_t tmem_c, uint32_t tmem_a, uint64_t db, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(tmem_c),
-      "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void tc_mma_f16(uint32_t tmem_c, uint64_t da, uint64_t db, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_c),
-      "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// One lane of a converged warp. The products are issued under this predicate and not under
-// "lane == 0": the compiler knows it to be one thread, keeps descriptors and addresses in uniform
-// registers and issues a product every 10-12 cycles; under a lane comparison every product first
-// moved its six operands across, 48 cycles whatever N is (measured: N = 16 50 -> 12, N = 64 50 -> 34,
-// N = 128 66 -> 66 cycles a K step).
-__device__ __forceinline__ bool tc_elect() {
-  uint32_t p;
-  asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));
-  return p != 0;
-}
-__device__ __forceinline__ void tc_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   tc_s32(bar))
-               : "memory");
-}
-// (OFF: a constant column offset on top of a warp-uniform address: the address stays in one uniform register)
-template <int OFF> __device__ __forceinline__ void tc_ld8(uint32_t taddr, uint32_t r[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8 + %9];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr), "n"(OFF));
-}
-template <int OFF> __device__ __forceinline__ void tc_ld4(uint32_t taddr, uint32_t r[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4 + %5];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(taddr), "n"(OFF));
-}
-__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t r[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-      "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ void tc_mbar_init(uint64_t *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_s32(bar)), "r"(count));
-}
-__device__ __forceinline__ void tc_mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_s32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_mbar_expect(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc_s32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool tc_bar_test(uint64_t *bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(tc_s32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool tc_bar_sleep(uint64_t *bar, uint32_t parity, uint32_t ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(tc_s32(bar)), "r"(parity), "r"(ns)
-      : "memory");
-  return ok != 0;
-}
-// A bounded wait on a phase of an mbarrier. False after the wait limit (or soon after an error is recorded):
-// the caller carries on with whatever the accumulators hold and the call reports the error. (All inline: a
-// call in the slow path makes the compiler keep the workers' registers out of its way everywhere.)
-__device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, int *err, unsigned long long wait_ns) {
-  if (tc_bar_test(bar, parity)) return true;
-  unsigned long long t0 = 0;
-  for (;;) {
-    // (sleeps in hardware for up to 2 us a turn: two waiting warps that polled took a fifth of the issue slots)
-    if (tc_bar_sleep(bar, parity, 2000u)) return true;
-    const unsigned long long t = tc_now();
-    if (t0 == 0) t0 = t;
-    if (*(volatile int *)err != 0 || t - t0 > wait_ns) break;
-  }
-  atomicCAS(err, 0, 7);
-  return false;
-}
-// Two f32 in one register pair. A product whose rounded value goes into an addition is written as
-// fma(a, b, -0) with a -0 that the compiler cannot see (a kernel parameter): it contracts a plain
-// mul.rn.f32x2 and the add.rn.f32x2 behind it into one fma, which has other bits than the reference's
-// separately rounded steps (adding -0 changes no product, signed zeros included).
-__device__ __forceinline__ uint64_t tc_pack2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void tc_unpack2(uint64_t v, float &a, float &b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ uint64_t tc_mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t tc_add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t tc_fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ void tc_tma3(uint32_t dst, const CUtensorMap *m, int x, int y, int z, uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-      "l"(m), "r"(x), "r"(y), "r"(z), "r"(tc_s32(bar))
-      : "memory");
-}
-
 // Compile with -DPM_TC_TRACE=1 (gate/up launches) or =2 (down launches) to stamp the phases of CTA 0's second
 // item with the SM clock: [worker thread 0 | thread 511 | issuing warp | producer][block][stamp], read back with
 // pm_debug_tc_trace.
@@ -231,9 +84,6 @@ extern "C" __attribute__((visibility("default"))) int pm_debug_tc_trace(unsigned
 #define TC_STAMP(who, b, i)
 #endif
 #define TC_STAMP_W(b, i) TC_STAMP(0, b, i) TC_STAMP(1, b, i)
-
-// a pass number as a type (the float terms of the two passes use registers of their own)
-template <int V> struct PassC { static constexpr int value = V; };
 
 struct TcArgs {
   CUtensorMap m0[2], m1[2];    // planes of the tile's matrices as [expert][row][bytes]: gate or down, up
@@ -263,7 +113,7 @@ struct TcArgs {
 // ~0 for an expert another rank holds; first pair; pairs; first record row). The records' rows keep a group's
 // pairs together and start every group on a multiple of 16 rows. One CTA; groups <= 512.
 __global__ void __launch_bounds__(512) k_tc_tiles(Groups g, int first_local, int n_local, int *head,
-                                                  uint4 *tiles, int ntok, int max_tiles) {
+                                                  uint4 *tiles, int ntok, int even, int max_tiles) {
   pm_pdl();
   __shared__ uint32_t s_t[16], s_r[16];
   const int a = threadIdx.x, lane = a & 31, warp = a >> 5;
@@ -289,8 +139,9 @@ __global__ void __launch_bounds__(512) k_tc_tiles(Groups g, int first_local, int
     int el = (int)g.expert[a] - first_local;
     if (el < 0 || el >= n_local) el = -1;
     const uint32_t off = g.offset[a];
+    const uint32_t nt = tc_tile_tokens(cnt, tc, ntok, even);
     for (uint32_t i = 0; i < tc && (int)(first + i) < max_tiles; i++)
-      tiles[first + i] = make_uint4((uint32_t)el, off + i * ntok, min(cnt - i * ntok, (uint32_t)ntok), r0 + i * ntok);
+      tiles[first + i] = make_uint4((uint32_t)el, off + i * nt, min(cnt - i * nt, nt), r0 + i * nt);
   }
   if (a == 0) {  // [0] tiles, [1], [2] the item counters of the two products
     head[0] = min((int)all, max_tiles);
@@ -998,7 +849,7 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)S::COLS) : "memory");
 }
 
-static int tc_max_tiles(int n_pairs, int max_groups, int ntok = TcShape<2>::NTOK) {  // (the default: of either shape)
+static int tc_max_tiles(int n_pairs, int max_groups, int ntok = 32) {  // (the default: of every shape)
   int groups = max_groups < n_pairs ? max_groups : n_pairs;
   return n_pairs / ntok + groups;
 }
@@ -1010,12 +861,13 @@ size_t tc_rec_bytes(int n_pairs, int max_groups, int cols) {
   size_t rows = (size_t)n_pairs + 15 * groups + 16;
   return (rows / 8 + 1) * (size_t)(cols / 256) * TC_REC;
 }
-TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens) {
+TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, bool mx) {
   TcTiles t;
   // tiles of up to 64 tokens and the two-CTA shape while the groups hold up to 16 pairs on average (128 experts x 2048 x
   // 768, 32 pairs a group: 102 us in the one-CTA shape, 118 us in this one; 2 pairs: 1,049 -> 733 us of a 7168-wide layer)
   const int avg = n_pairs / (n_groups < n_pairs ? n_groups : n_pairs);
-  t.ntok = avg <= 16 ? TcShape<2>::NTOK : TC_NMAX;
+  t.ntok = avg <= 16 ? (mx ? mx_small_tokens() : TcShape<2>::NTOK) : TC_NMAX;
+  t.even = mx;
   t.shared = shared_tokens > 0;
   t.max_tiles = tc_max_tiles(n_pairs, max_groups, t.ntok) + (shared_tokens + t.ntok - 1) / t.ntok;
   t.n = (int *)buf;
@@ -1024,7 +876,7 @@ TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, in
   return t;
 }
 void launch_tc_tiles(const Launch &L, const LayerDev &ly, Groups g, const TcTiles &t) {
-  pm_launch(L, k_tc_tiles, 1, 512, 0, g, ly.first_local, ly.n_local, t.n, t.tiles, t.ntok, t.max_tiles);
+  pm_launch(L, k_tc_tiles, 1, 512, 0, g, ly.first_local, ly.n_local, t.n, t.tiles, t.ntok, t.even, t.max_tiles);
 }
 static dim3 rows_grid(int n_rows, const TcTiles &t, int cols) {
   const long units = ((long)n_rows / 8 + 2 * t.max_tiles) * (cols / 256);  // (row group, block) records in all
