@@ -416,7 +416,7 @@ typedef CUresult (*pm_encode_tiled_t)(CUtensorMap *, CUtensorMapDataType, cuuint
                                       const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                       CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static int32_t wmat_maps(const WMat &W, int n_exp, int box_rows, WMaps &M) {
-  if (W.type != PM_TYPE_Q4_K && W.type != PM_TYPE_Q6_K && W.type != PM_TYPE_MXFP4) return PM_OK;
+  if (W.type != PM_TYPE_Q4_K && W.type != PM_TYPE_Q6_K && W.type != PM_TYPE_MXFP4 && !q32_weights(W.type)) return PM_OK;
   static pm_encode_tiled_t enc = nullptr;
   if (!enc) {
     void *f = nullptr;
@@ -425,17 +425,20 @@ static int32_t wmat_maps(const WMat &W, int n_exp, int box_rows, WMaps &M) {
     if (q != cudaDriverEntryPointSuccess || !f) return fail(PM_ERR_CUDA, "cuTensorMapEncodeTiled is not there");
     enc = (pm_encode_tiled_t)f;
   }
-  const bool mx = W.type == PM_TYPE_MXFP4, q4 = W.type == PM_TYPE_Q4_K;
+  const bool v32 = q32_weights(W.type), mx = W.type == PM_TYPE_MXFP4 || v32, q4 = W.type == PM_TYPE_Q4_K;
+  const bool nib64 = v32 && W.type != PM_TYPE_Q8_0;
   const int nb = W.cols / 256, n = q4 ? 1 : 2;
-  // MXFP4: plane 0 alone, boxes of 256 values x 64 rows and x 128 rows (the last box of a row may reach past it)
-  const int block[2] = {q4 ? 144 : 128, mx ? 128 : 64};
+  // MXFP4: plane 0 alone, boxes of 256 values x 64 rows and x 128 rows (the last box of a row may reach past it);
+  // Q8_0, IQ4_NL and IQ4_XS likewise with 128 values
+  const int block[2] = {q4 ? 144 : (nib64 ? 64 : 128), mx && !nib64 ? 128 : 64};
   // Q6_K and MXFP4: 128- and 64-byte rows swizzled so that the row-per-thread reads of the unpack have no bank conflicts
   // (a Q4_K row of 144 bytes has none as it is)
-  const CUtensorMapSwizzle sw[2] = {q4 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
-                                    mx ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B};
+  const CUtensorMapSwizzle sw[2] = {
+      q4 ? CU_TENSOR_MAP_SWIZZLE_NONE : (nib64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B),
+      mx && !nib64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B};
   for (int p = 0; p < n; p++) {
     const int plane = mx ? 0 : p;
-    const cuuint64_t row = mx ? (cuuint64_t)W.cols / 2 : (cuuint64_t)nb * block[p];
+    const cuuint64_t row = W.type == PM_TYPE_Q8_0 ? (cuuint64_t)W.cols : mx ? (cuuint64_t)W.cols / 2 : (cuuint64_t)nb * block[p];
     const cuuint64_t dims[3] = {row, (cuuint64_t)W.rows, (cuuint64_t)n_exp}, strides[2] = {row, (cuuint64_t)W.stride[plane]};
     const cuuint32_t box[3] = {(cuuint32_t)block[p], mx ? 64u << p : (cuuint32_t)box_rows, 1}, es[3] = {1, 1, 1};
     const CUresult r = enc(&M.m[p], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, W.plane[plane], dims, strides, box, es,
@@ -851,8 +854,15 @@ static bool mx_layer(const pm_layer_desc &D) {
   return D.act_quant == PM_AQ_F32 && D.type_gate == PM_TYPE_MXFP4 && D.type_up == PM_TYPE_MXFP4 && D.type_down == PM_TYPE_MXFP4;
 }
 
+// the layers k_tc_q32 takes
+static bool q32_layer(const pm_layer_desc &D) {
+  return (D.act_quant == PM_AQ_Q8_32 || D.act_quant == PM_AQ_Q8_32_F16) && D.type_gate == D.type_up && q32_weights(D.type_gate) &&
+         q32_weights(D.type_down);
+}
+
 // the largest record buffer any tensor-core launch of a T-token call needs
 static size_t scratch_rec_bytes(const pm_layer_desc &D, int T) {
+  if (q32_layer(D)) return q32_rec_bytes(T * D.top_k, D.n_exp, std::max(D.d, D.ff));
   if (mx_layer(D)) return mx_rec_bytes(T * D.top_k, D.n_exp, std::max(D.d, D.ff));
   if (D.act_quant != PM_AQ_Q8X_256) return 0;
   const int m = shared_merges(D) ? 1 : 0, P = T * (D.top_k + m), E = D.n_exp + m;
@@ -949,6 +959,7 @@ static Groups plan_groups(const PlanDev &pl, int E) {
 struct Path {
   bool tc, tc_gu;  // int8 tensor-core products (both; gate/up needs one type for the two matrices)
   bool mx;         // bf16 tensor-core products for MXFP4 weights and f32 activations (tolerance parity, not bits)
+  bool q32;        // int8 tensor-core products for 32-value activation blocks
   bool merge;      // the shared expert is one more group of the routed experts' launches
 };
 static Path pick_path(pm_layer *ly, int T) {
@@ -964,14 +975,16 @@ static Path pick_path(pm_layer *ly, int T) {
   // (MXFP4: from two tokens up until the caller says otherwise; a layer of 32 experts, d = ff = 2880, row kernels against
   // these: 1 token 60 : 66 us, 2 tokens 97 : 97, 4 tokens 162 : 130, 8 tokens 300 : 181)
   p.mx = mx_layer(D) && c->tc_min_tokens > 0 && T >= (c->tc_min_set ? c->tc_min_tokens : 2);
+  p.q32 = q32_layer(D) && c->tc_min_tokens > 0 && T >= int_min;
   p.merge = p.tc_gu && shared_merges(D);
   return p;
 }
 static TcTiles path_tiles(pm_layer *ly, int T, const Path &p, const Scratch &S, bool merge) {
   const pm_layer_desc &D = ly->dev.desc;
   TcTiles t{};
-  if (p.tc || p.mx)
-    t = tc_tiles_of(S.tiles, T * D.top_k, D.n_exp, std::min(D.n_exp, ly->dev.n_local), merge ? T : 0, p.mx);
+  if (p.tc || p.mx || p.q32)
+    t = tc_tiles_of(S.tiles, T * D.top_k, D.n_exp, std::min(D.n_exp, ly->dev.n_local), merge ? T : 0,
+                    p.mx ? TC_KIND_MX : (p.q32 ? TC_KIND_Q32 : TC_KIND_Q8X));
   return t;
 }
 
@@ -992,7 +1005,7 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
   TcTiles tt{};
   if (made) {
     tt = *made;
-  } else if (tc || path.mx) {
+  } else if (tc || path.mx || path.q32) {
     PROF(c, PH_PLAN);
     tt = path_tiles(ly, T, path, S, false);
     launch_tc_tiles(L, dv, g, tt);
@@ -1016,6 +1029,27 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
     {
       PROF(c, PH_DOWN);
       CU(launch_tc_mx(L, dv, true, g.pair_src, tt, pieces, S.rec, nullptr, S.eo, S.eo_parts, (size_t)P * D.d, c->dev_err, c->wait_ns));
+    }
+    c->path_count[PM_PATH_TENSOR] += 2;
+    CU(cudaGetLastError());
+    return PM_OK;
+  }
+  if (path.q32) {
+    {
+      PROF(c, PH_QUANT_X);
+      launch_q32_rows(L, P, tt, g.pair_token, D.d, x, D.type_gate, f16s, S.rec);
+    }
+    {
+      PROF(c, PH_GATEUP);
+      CU(launch_tc_q32(L, dv, false, g.pair_src, tt, S.rec, w, S.h, c->dev_err, c->wait_ns));
+    }
+    {
+      PROF(c, PH_QUANT_H);
+      launch_q32_rows(L, P, tt, nullptr, D.ff, S.h, D.type_down, f16s, S.rec);
+    }
+    {
+      PROF(c, PH_DOWN);
+      CU(launch_tc_q32(L, dv, true, g.pair_src, tt, S.rec, nullptr, S.eo, c->dev_err, c->wait_ns));
     }
     c->path_count[PM_PATH_TENSOR] += 2;
     CU(cudaGetLastError());
@@ -1085,7 +1119,7 @@ static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
   const Path path = pick_path(ly, T);
   const bool use_tc = path.tc, tc_gu = path.tc_gu;
   TcTiles tt{};
-  if (use_tc) tt = tc_tiles_of(S.tiles, T, 1, 1, 0, false);
+  if (use_tc) tt = tc_tiles_of(S.tiles, T, 1, 1, 0, TC_KIND_Q8X);
   launch_shared_groups(L, S.one, S.zero_u, S.tcount, S.iota, T, tt);
   Groups g;
   g.n_groups = S.one;
@@ -1131,7 +1165,7 @@ static int32_t dev_forward(pm_layer *ly, const float *x, int T, float *y, bool a
     { PROF(c, PH_ROUTER); launch_router(L, dv, x, T, S.logits); }
     { PROF(c, PH_ROUTE); launch_route_plan(L, dv, S.logits, T, S.ids, S.w, S.plan, S.seg, tt); }
   }
-  TRY(dev_experts(ly, x, T, S, S.w, false, path.tc || path.mx ? &tt : nullptr));
+  TRY(dev_experts(ly, x, T, S, S.w, false, path.tc || path.mx || path.q32 ? &tt : nullptr));
   const float *shared_out = S.shared_out;
   if (path.merge) {
     shared_out = S.eo + (size_t)T * dv.desc.top_k * dv.desc.d;

@@ -27,7 +27,8 @@ struct WMat {
 };
 
 // TMA descriptions of a family's planes as [expert][row][bytes of the row], boxes of 64 rows (gate, up) or 128 rows
-// (down) x one 256-value block (Q4_K: plane 0; Q6_K: ql, qh; MXFP4: the nibbles, with 64 and with 128 rows). Host memory of the layer: launchers copy them into parameters.
+// (down) x one 256-value block (Q4_K: plane 0; Q6_K: ql, qh; MXFP4: the nibbles, and Q8_0,
+// IQ4_NL, IQ4_XS: the values, with 64 and with 128 rows). Host memory of the layer: launchers copy them into parameters.
 struct WMaps {
   CUtensorMap m[2];
 };
@@ -195,8 +196,12 @@ void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int
 // src_row: row of the activations that holds pair p (null: row p itself)
 size_t tc_tile_words(int n_pairs, int max_groups);
 // n_groups: groups that can have pairs (the experts this GPU holds)
-// shared_tokens: tokens of the shared expert's group in the same list (0: none); mx: for launch_tc_mx
-TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, bool mx);  // buf: tc_tile_words words, 16-byte aligned
+// shared_tokens: tokens of the shared expert's group in the same list (0: none)
+// kind: of which products
+#define TC_KIND_Q8X 0
+#define TC_KIND_MX 1
+#define TC_KIND_Q32 2
+TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, int kind);  // buf: tc_tile_words words, 16-byte aligned
 size_t tc_rec_bytes(int n_pairs, int max_groups, int cols);
 void launch_tc_tiles(const Launch &L, const LayerDev &ly, Groups g, const TcTiles &t);
 void launch_tc_quant_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x,
@@ -216,6 +221,14 @@ void launch_mx_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_
 cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t, int pieces,
                          const uint8_t *rec, const float *wts, float *out, int splits, size_t split_stride, int *err,
                          unsigned long long wait_ns);
+// tensor-core (tcgen05 int8) form for Q8_0 / IQ4_NL / IQ4_XS weights and 32-value activation blocks (prefill_q32.cu)
+bool q32_weights(int type);
+int q32_tile_tokens();
+size_t q32_rec_bytes(int n_pairs, int max_groups, int cols);
+void launch_q32_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x, int weight_type,
+                     bool f16_scale, uint8_t *rec);
+cudaError_t launch_tc_q32(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
+                          const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns);
 // expert parallelism (kernels_basic.cu): per-rank pair counts, the wire records of a dispatch,
 // the received (expert, weight) records, the derived forms of received Q8x group sums
 void launch_ep_slots(const Launch &L, uint32_t *ids, int P, int E, const int32_t *table, uint32_t *usage);

@@ -861,13 +861,14 @@ size_t tc_rec_bytes(int n_pairs, int max_groups, int cols) {
   size_t rows = (size_t)n_pairs + 15 * groups + 16;
   return (rows / 8 + 1) * (size_t)(cols / 256) * TC_REC;
 }
-TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, bool mx) {
+TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, int kind) {
   TcTiles t;
   // tiles of up to 64 tokens and the two-CTA shape while the groups hold up to 16 pairs on average (128 experts x 2048 x
   // 768, 32 pairs a group: 102 us in the one-CTA shape, 118 us in this one; 2 pairs: 1,049 -> 733 us of a 7168-wide layer)
   const int avg = n_pairs / (n_groups < n_pairs ? n_groups : n_pairs);
-  t.ntok = avg <= 16 ? (mx ? mx_small_tokens() : TcShape<2>::NTOK) : TC_NMAX;
-  t.even = mx;
+  t.ntok = avg <= 16 ? (kind == TC_KIND_MX ? mx_small_tokens() : TcShape<2>::NTOK) : TC_NMAX;
+  if (kind == TC_KIND_Q32) t.ntok = q32_tile_tokens();
+  t.even = kind != TC_KIND_Q8X;
   t.shared = shared_tokens > 0;
   t.max_tiles = tc_max_tiles(n_pairs, max_groups, t.ntok) + (shared_tokens + t.ntok - 1) / t.ntok;
   t.n = (int *)buf;
