@@ -272,14 +272,15 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
   } else {
     // ================= the workers =================
     // expand: thread = (row m of the tile; blocks 2 part, 2 part + 1 of a stage); fold: row m, half `part` of the tokens
-    const int m = tid & 127, part = warp >> 2;
+    const int m = tid & 127, part = (int)__reduce_max_sync(PM_FULL, (unsigned)warp >> 2);
     const bool up = !DOWN && m >= 64;
-    const uint32_t tlane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    // (redux results live in uniform registers, as the addresses of tensor memory have to)
+    const uint32_t tlane = tmem + (__reduce_max_sync(PM_FULL, 32u * (warp & 3)) << 16);
     uint32_t st = 0, sr = 0, pr = 0, sb = 0, slot = 0, pf = 0;
     Q32Item it;
     for (int k = 0; next_item(k, it); k++) {
       const uint4 T = it.t;
-      const int el = (int)T.x, nvalid = (int)T.z, r0 = it.r0;
+      const int el = (int)T.x, nvalid = (int)__reduce_max_sync(PM_FULL, T.z), r0 = it.r0;
       const uint32_t npad = ((uint32_t)nvalid + 15u) & ~15u, G = group_of(npad);
       const int ew = (int)npad >> 1, e0 = part * ew;
       const int row = r0 + (DOWN ? m : (m & 63));
@@ -310,50 +311,61 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
       auto fold = [&](int s, unsigned long long sc) {
         const int nblk = min(Q32_KB, nb - s * Q32_KB);
         const uint8_t *xd = sB + sb * Q32_BST + npad * 32u + e0 * 4;
-#pragma unroll
-        for (int b = 0; b < Q32_KB; b++)
-          if (b < nblk) {
-            if ((b & (G - 1)) == 0) {
-              tc_wait(acc_full + slot, pf, A.err, A.wait_ns);
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            }
-            float dw;
-            if (XS) {  // d * (ls - 32) of sub-block ib (src/q4x_cpu.rs:102-117)
-              const int ib = 4 * (s & 1) + b;
-              const uint32_t lo = (uint32_t)sc, hi = (uint32_t)(sc >> 32);
-              const int ls = (int)((hi >> (4 * ib)) & 15) | (int)((((lo >> 16) >> (2 * ib)) & 3) << 4);
-              dw = __fmul_rn(pm_f16(lo), (float)(ls - 32));
-            } else {
-              dw = pm_f16((uint32_t)(sc >> (16 * b)));
-            }
-            const uint64_t dw2 = tc_pack2(dw, dw);
-            const uint32_t at = tlane + Q32_ACC + slot * 64u + (b & (G - 1)) * npad + (uint32_t)e0;
-#pragma unroll
-            for (int c = 0; c < Q32_N / 2; c += 16)
-              if (c < ew) {
-                uint32_t v[16];
-                tc_ld8<0>(at + c, v);
-                if (c + 8 < ew) tc_ld8<8>(at + c, v + 8);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int u = 0; u < 16; u += 4)
-                  if (u < 8 || c + 8 < ew) {
-                    const ulonglong2 x2 = *(const ulonglong2 *)(xd + (c + u) * 4);
-                    const uint64_t s0 = tc_pack2(__int2float_rn((int)v[u]), __int2float_rn((int)v[u + 1]));
-                    const uint64_t s1 = tc_pack2(__int2float_rn((int)v[u + 2]), __int2float_rn((int)v[u + 3]));
-                    uint64_t *ac = acc + (c + u) / 2;
-                    ac[0] = tc_add2(ac[0], tc_fma2(tc_mul2(dw2, x2.x), s0, A.neg_zero2));
-                    ac[1] = tc_add2(ac[1], tc_fma2(tc_mul2(dw2, x2.y), s1, A.neg_zero2));
-                  }
-              }
-            if ((b & (G - 1)) == G - 1 || b == nblk - 1) {
-              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-              __syncwarp();
-              if (lane == 0) tc_mbar_arrive(acc_free + slot);
-              if (++slot == Q32_NACC) { slot = 0; pf ^= 1; }
-            }
-            xd += npad * 36u;
+        uint32_t left = 0, at = 0;  // blocks left in the slot
+        // (not unrolled: with four copies the workers waited for instructions, not for the pipes)
+#pragma unroll 1
+        for (int b = 0; b < nblk; b++) {
+          if (left == 0) {
+            left = min(G, (uint32_t)(nblk - b));
+            tc_wait(acc_full + slot, pf, A.err, A.wait_ns);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            at = tlane + Q32_ACC + slot * 64u + (uint32_t)e0;
           }
+          float dw;
+          if (XS) {  // d * (ls - 32) of sub-block ib (src/q4x_cpu.rs:102-117)
+            const int ib = 4 * (s & 1) + b;
+            const uint32_t lo = (uint32_t)sc, hi = (uint32_t)(sc >> 32);
+            const int ls = (int)((hi >> (4 * ib)) & 15) | (int)((((lo >> 16) >> (2 * ib)) & 3) << 4);
+            dw = __fmul_rn(pm_f16(lo), (float)(ls - 32));
+          } else {
+            dw = pm_f16((uint32_t)(sc >> (16 * b)));
+          }
+          const uint64_t dw2 = tc_pack2(dw, dw);
+          auto half = [&](int c, auto n_) {  // columns c .. c + 7 (15)
+            constexpr int N = decltype(n_)::value;
+            uint32_t v[16];
+            tc_ld8<0>(at + c, v);
+            if (N > 8) tc_ld8<8>(at + c, v + 8);
+            ulonglong2 x2[N / 4];
+#pragma unroll
+            for (int u = 0; u < N / 4; u++) x2[u] = *(const ulonglong2 *)(xd + (c + 4 * u) * 4);
+#pragma unroll
+            for (int u = 0; u < N / 4; u++) {
+              x2[u].x = tc_mul2(dw2, x2[u].x);
+              x2[u].y = tc_mul2(dw2, x2[u].y);
+            }
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int u = 0; u < N; u += 4) {
+              const uint64_t s0 = tc_pack2(__int2float_rn((int)v[u]), __int2float_rn((int)v[u + 1]));
+              const uint64_t s1 = tc_pack2(__int2float_rn((int)v[u + 2]), __int2float_rn((int)v[u + 3]));
+              uint64_t *ac = acc + (c + u) / 2;
+              ac[0] = tc_add2(ac[0], tc_fma2(x2[u / 4].x, s0, A.neg_zero2));
+              ac[1] = tc_add2(ac[1], tc_fma2(x2[u / 4].y, s1, A.neg_zero2));
+            }
+          };
+          if (ew == 8) half(0, PassC<8>());
+          else half(0, PassC<16>());
+          if (ew > 16) half(16, PassC<16>());  // (24 columns: the last 8 are not used)
+          xd += npad * 36u;
+          at += npad;
+          if (--left == 0) {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc_mbar_arrive(acc_free + slot);
+            if (++slot == Q32_NACC) { slot = 0; pf ^= 1; }
+          }
+        }
         __syncwarp();
         if (lane == 0) tc_mbar_arrive(empty_b + sb);
         if (++sb == Q32_NSB) sb = 0;

@@ -103,13 +103,13 @@ __device__ __forceinline__ bool tc_bar_test(uint64_t *bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ bool tc_bar_sleep(uint64_t *bar, uint32_t parity, uint32_t ns) {
+__device__ __forceinline__ bool tc_bar_sleep(uint64_t *bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
       " selp.u32 %0, 1, 0, p;\n}\n"
       : "=r"(ok)
-      : "r"(tc_s32(bar)), "r"(parity), "r"(ns)
+      : "r"(tc_s32(bar)), "r"(parity)
       : "memory");
   return ok != 0;
 }
@@ -120,8 +120,8 @@ __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, int *err
   if (tc_bar_test(bar, parity)) return true;
   unsigned long long t0 = 0;
   for (;;) {
-    // (sleeps in hardware for up to 2 us a turn: two waiting warps that polled took a fifth of the issue slots)
-    if (tc_bar_sleep(bar, parity, 2000u)) return true;
+    // (sleeps in hardware for a while: two waiting warps that polled took a fifth of the issue slots)
+    if (tc_bar_sleep(bar, parity)) return true;
     const unsigned long long t = tc_now();
     if (t0 == 0) t0 = t;
     if (*(volatile int *)err != 0 || t - t0 > wait_ns) break;
