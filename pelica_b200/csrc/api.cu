@@ -863,7 +863,10 @@ static bool q32_layer(const pm_layer_desc &D) {
 // the largest record buffer any tensor-core launch of a T-token call needs
 static size_t scratch_rec_bytes(const pm_layer_desc &D, int T) {
   if (q32_layer(D)) return q32_rec_bytes(T * D.top_k, D.n_exp, std::max(D.d, D.ff));
-  if (mx_layer(D)) return mx_rec_bytes(T * D.top_k, D.n_exp, std::max(D.d, D.ff));
+  if (mx_layer(D)) {
+    const int P = T * D.top_k, cols = std::max(D.d, D.ff);
+    return std::max(mx_rec_bytes(P, D.n_exp, cols), mx8_rec_bytes(P, D.n_exp, cols));
+  }
   if (D.act_quant != PM_AQ_Q8X_256) return 0;
   const int m = shared_merges(D) ? 1 : 0, P = T * (D.top_k + m), E = D.n_exp + m;
   size_t r = std::max(tc_rec_bytes(P, E, D.d), tc_rec_bytes(P, E, D.ff));
@@ -972,9 +975,9 @@ static Path pick_path(pm_layer *ly, int T) {
   const int int_min = c->tc_min_set ? c->tc_min_tokens : (shared_merges(D) ? 1 : 2);
   p.tc = D.act_quant == PM_AQ_Q8X_256 && c->tc_min_tokens > 0 && T >= int_min;
   p.tc_gu = p.tc && D.type_gate == D.type_up;
-  // (MXFP4: from two tokens up until the caller says otherwise; a layer of 32 experts, d = ff = 2880, row kernels against
-  // these: 1 token 60 : 66 us, 2 tokens 97 : 97, 4 tokens 162 : 130, 8 tokens 300 : 181)
-  p.mx = mx_layer(D) && c->tc_min_tokens > 0 && T >= (c->tc_min_set ? c->tc_min_tokens : 2);
+  // (MXFP4: from one token up until the caller says otherwise; a layer of 32 experts, d = ff = 2880, row kernels against
+  // these: 1 token 60 : 55 us, 2 tokens 97 : 61, 4 tokens 162 : 79, 8 tokens 300 : 121)
+  p.mx = mx_layer(D) && c->tc_min_tokens > 0 && T >= (c->tc_min_set ? c->tc_min_tokens : 1);
   p.q32 = q32_layer(D) && c->tc_min_tokens > 0 && T >= int_min;
   p.merge = p.tc_gu && shared_merges(D);
   return p;
@@ -982,9 +985,10 @@ static Path pick_path(pm_layer *ly, int T) {
 static TcTiles path_tiles(pm_layer *ly, int T, const Path &p, const Scratch &S, bool merge) {
   const pm_layer_desc &D = ly->dev.desc;
   TcTiles t{};
+  const int groups = std::min(D.n_exp, ly->dev.n_local);
   if (p.tc || p.mx || p.q32)
-    t = tc_tiles_of(S.tiles, T * D.top_k, D.n_exp, std::min(D.n_exp, ly->dev.n_local), merge ? T : 0,
-                    p.mx ? TC_KIND_MX : (p.q32 ? TC_KIND_Q32 : TC_KIND_Q8X));
+    t = tc_tiles_of(S.tiles, T * D.top_k, D.n_exp, groups, merge ? T : 0,
+                    p.mx ? mx_tile_tokens(T, T * D.top_k, groups) : (p.q32 ? q32_tile_tokens() : 0));
   return t;
 }
 
@@ -1011,24 +1015,25 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
     launch_tc_tiles(L, dv, g, tt);
   }
   if (path.mx) {
-    // (few tokens: three pieces hold every bit of an f32; prompts: two, see prefill_mx.cu)
-    const int pieces = T < PM_MX_PROMPT ? 3 : 2;
-    S.eo_parts = made ? mx_splits(D, P) : 1;  // (the other callers take the pair outputs themselves)
+    const bool small = tt.ntok != 128;
+    S.eo_parts = made && small ? mx_splits(D, P) : 1;  // (the other callers take the pair outputs themselves)
     {
       PROF(c, PH_QUANT_X);
-      launch_mx_rows(L, P, tt, g.pair_token, D.d, x, pieces, S.rec);
+      (small ? launch_mx8_rows : launch_mx_rows)(L, P, tt, g.pair_token, D.d, x, S.rec);
     }
     {
       PROF(c, PH_GATEUP);
-      CU(launch_tc_mx(L, dv, false, g.pair_src, tt, pieces, S.rec, w, S.h, 1, 0, c->dev_err, c->wait_ns));
+      CU(small ? launch_tc_mx8(L, dv, false, g.pair_src, tt, S.rec, w, S.h, 1, 0, c->dev_err, c->wait_ns)
+               : launch_tc_mx(L, dv, false, g.pair_src, tt, S.rec, w, S.h, c->dev_err, c->wait_ns));
     }
     {
       PROF(c, PH_QUANT_H);
-      launch_mx_rows(L, P, tt, nullptr, D.ff, S.h, pieces, S.rec);
+      (small ? launch_mx8_rows : launch_mx_rows)(L, P, tt, nullptr, D.ff, S.h, S.rec);
     }
     {
       PROF(c, PH_DOWN);
-      CU(launch_tc_mx(L, dv, true, g.pair_src, tt, pieces, S.rec, nullptr, S.eo, S.eo_parts, (size_t)P * D.d, c->dev_err, c->wait_ns));
+      CU(small ? launch_tc_mx8(L, dv, true, g.pair_src, tt, S.rec, nullptr, S.eo, S.eo_parts, (size_t)P * D.d, c->dev_err, c->wait_ns)
+               : launch_tc_mx(L, dv, true, g.pair_src, tt, S.rec, nullptr, S.eo, c->dev_err, c->wait_ns));
     }
     c->path_count[PM_PATH_TENSOR] += 2;
     CU(cudaGetLastError());
@@ -1119,7 +1124,7 @@ static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
   const Path path = pick_path(ly, T);
   const bool use_tc = path.tc, tc_gu = path.tc_gu;
   TcTiles tt{};
-  if (use_tc) tt = tc_tiles_of(S.tiles, T, 1, 1, 0, TC_KIND_Q8X);
+  if (use_tc) tt = tc_tiles_of(S.tiles, T, 1, 1, 0, 0);
   launch_shared_groups(L, S.one, S.zero_u, S.tcount, S.iota, T, tt);
   Groups g;
   g.n_groups = S.one;

@@ -188,7 +188,7 @@ void launch_gateup(const Launch &L, const LayerDev &ly, bool shared, Groups g, i
 void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int n_pairs,
                  const float *h, const int8_t *hq, const float *hd, const int32_t *hbsum,
                  float *eo);
-#define PM_MX_PROMPT 32  // tokens from which the bf16 products use two pieces of a value (below: three)
+#define PM_MX_PROMPT 32  // tokens of a call from which the MXFP4 products need not hold every bit of an activation
 #define TC_SHARED 0x40000000u  // expert slot of a tile of the shared expert
 // tensor-core (tcgen05 int8) form of launch_gateup / launch_down for Q4_K / Q6_K x Q8x (prefill_tc.cu):
 // the token tiles of a grouping (one list serves both products), the activation rows regrouped by expert
@@ -197,11 +197,8 @@ void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int
 size_t tc_tile_words(int n_pairs, int max_groups);
 // n_groups: groups that can have pairs (the experts this GPU holds)
 // shared_tokens: tokens of the shared expert's group in the same list (0: none)
-// kind: of which products
-#define TC_KIND_Q8X 0
-#define TC_KIND_MX 1
-#define TC_KIND_Q32 2
-TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, int kind);  // buf: tc_tile_words words, 16-byte aligned
+// ntok: tokens of a full tile, 0 for launch_tc's own rule (anything else: even tiles)
+TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, int ntok);  // buf: tc_tile_words words, 16-byte aligned
 size_t tc_rec_bytes(int n_pairs, int max_groups, int cols);
 void launch_tc_tiles(const Launch &L, const LayerDev &ly, Groups g, const TcTiles &t);
 void launch_tc_quant_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x,
@@ -210,17 +207,21 @@ void launch_tc_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_
                     const float *xd, const uint16_t *xbm, const int32_t *xs, uint8_t *rec);
 cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared_only, bool down, const uint32_t *pair_src, const TcTiles &t,
                       const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns, int fault_block);
-// tensor-core (tcgen05 bf16) form for MXFP4 weights and f32 activations (prefill_mx.cu). The rows are regrouped
-// by tile and split into 2 or 3 bf16 pieces a value (rec: mx_rec_bytes bytes); the down products may be cut along
-// K into mx_splits parts: part s goes to out + s * split_stride.
+// tensor-core forms for MXFP4 weights and f32 activations: tiles of 128 tokens on bf16 pieces (prefill_mx.cu), smaller
+// ones (mx_tile_tokens) on block-scaled fp8 pieces (prefill_mx8.cu). The rows are regrouped by tile and split into their
+// pieces (rec: mx_rec_bytes / mx8_rec_bytes bytes); the down products of the second may be cut along K into mx_splits
+// parts: part s goes to out + s * split_stride.
 size_t mx_rec_bytes(int n_pairs, int max_groups, int cols);
-int mx_small_tokens();
+size_t mx8_rec_bytes(int n_pairs, int max_groups, int cols);
+int mx_tile_tokens(int T, int n_pairs, int n_groups);
 int mx_splits(const pm_layer_desc &D, int n_pairs);
-void launch_mx_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x, int pieces,
-                    uint8_t *rec);
-cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t, int pieces,
-                         const uint8_t *rec, const float *wts, float *out, int splits, size_t split_stride, int *err,
-                         unsigned long long wait_ns);
+void launch_mx_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x, uint8_t *rec);
+void launch_mx8_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x, uint8_t *rec);
+cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
+                         const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns);
+cudaError_t launch_tc_mx8(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
+                          const uint8_t *rec, const float *wts, float *out, int splits, size_t split_stride, int *err,
+                          unsigned long long wait_ns);
 // tensor-core (tcgen05 int8) form for Q8_0 / IQ4_NL / IQ4_XS weights and 32-value activation blocks (prefill_q32.cu)
 bool q32_weights(int type);
 int q32_tile_tokens();

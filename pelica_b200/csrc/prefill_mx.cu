@@ -4,22 +4,22 @@
 //
 // MXFP4 weights are exact in bf16 (a one-bit mantissa times a power of two: the E2M1 code
 // doubled, times the halved E8M0 scale, src/oss_kernels.rs:41-55), the f32 activations are
-// not: each is split into bf16 pieces, x = x1 + x2 (+ x3), xi = bf16(what is left), and every K step runs once a
-// piece into the same accumulator. Products of two bf16 values are exact in f32. Three pieces hold all 24 bits of
-// an f32: calls of fewer than 32 tokens, which otherwise run on f32 multiply-adds, use them. Prompts use two:
-// what differs from the f32 reference path (src/oss_batch.rs:774-789) is then the 2^-17 relative residue and the
-// summation order; parity is the layer tolerance (1e-3 relative + 1e-4 of the RMS), not bits.
+// not: each is split into bf16 pieces, x = x1 + x2, xi = bf16(what is left), and every K step runs once a
+// piece into the same accumulator. Products of two bf16 values are exact in f32: what differs from the f32 reference
+// path (src/oss_batch.rs:774-789) is the 2^-17 relative residue and the summation order; parity is the layer
+// tolerance (1e-3 relative + 1e-4 of the RMS), not bits. For prompts whose experts get many tokens; calls with fewer
+// tokens an expert run on prefill_mx8.cu.
 //
 // A persistent pipeline like the int8 kernel's (prefill_tc.cu): a producer thread brings the weights' nibbles in
 // by TMA (boxes of 256 K values) and the tokens' pieces by one bulk copy a chunk of 64 K values; the workers decode
 // a block of 32 codes a thread and store it to tensor memory, up to four chunks ahead of the products; work items
 // come from a counter. One accumulator for the whole K (the block scale lives in the bf16 weight).
-//  BIG (more than 16 pairs a group on average): a CTA an SM takes 256 weight rows (128 gate rows and the same 128
-//    rows of up, or 256 down rows) x 128 tokens. Both halves multiply one staging of the tokens' pieces, which
-//    halves what comes from L2: 31 bytes a cycle an SM; with 128 rows it would be the limit, 62. Gate and up sums of
-//    an output sit in the same thread. Bound by the tensor pipe (1,050 cycles a chunk; decoding takes about 500).
-//  else: two CTAs an SM of half the tensor memory, 128 rows (64 gate + 64 up, or 128 down) x 32 tokens. Bound by
-//    the weights' bytes and the decode. Down rows may be cut along K (launch_tc_mx), so that a few tokens fill the SMs.
+// A CTA takes 256 weight rows (128 gate rows and the same 128 rows of up, or 256 down rows) x 128 tokens. Both
+// halves multiply one staging of the tokens' pieces, which halves what comes from L2: 31 bytes a cycle an SM; with 128
+// rows it would be the limit, 62. Gate and up sums of an output sit in the same thread. Bound by the tensor pipe
+// (1,050 cycles a chunk, 60 % of the time at 2048 tokens, 32 experts, d = ff = 2880) and by what the workers' decode
+// adds where the two do not overlap: gate/up + down 2,110 -> 750 us against a kernel that staged decoded weights
+// in shared memory and took 128 rows.
 #include <cuda_bf16.h>
 
 #include "tcgen.cuh"
@@ -27,19 +27,17 @@
 #define MX_M 128
 #define MX_KC 64   /* K values of a chunk */
 #define MX_NA 4    /* chunks of operand A in tensor memory */
+#define NPC 2      /* bf16 pieces of an activation */
 #define MX_BOX (MX_M * 128)   /* nibbles of 128 rows x 256 K values */
 
-template <bool BIG, int NPC> struct MxShape {
-  static constexpr int MT = BIG ? 2 : 1;                 // 128-row halves of a CTA
-  static constexpr int NW = BIG ? 512 : 256, NT = NW + 64;
-  static constexpr int CTAS = BIG ? 1 : 2;
-  static constexpr int NTOK = BIG ? 128 : 32;
-  static constexpr uint32_t COLS = BIG ? 512 : 256;      // tensor memory: accumulators, then MX_NA chunks of operand A
-  static constexpr uint32_t A0 = BIG ? 256 : 128, ACH = MT * MX_KC / 2;  // first column, columns a chunk
+struct MxShape {
+  static constexpr int MT = 2;                 // 128-row halves of a CTA
+  static constexpr int NW = 512, NT = NW + 64;
+  static constexpr int NTOK = 128;
+  static constexpr uint32_t COLS = 512;        // tensor memory: accumulators, then MX_NA chunks of operand A
+  static constexpr uint32_t A0 = 256, ACH = MT * MX_KC / 2;  // first column, columns a chunk
   static constexpr int RAWB = MT * MX_BOX, NSR = 3;
   static constexpr int BST = NTOK * MX_KC * 2 * NPC, NSB = 4;
-  static constexpr int XB = BIG ? 0 : NTOK * MX_M * 4;   // gate/up: exchange of the sums
-  static constexpr int NACC = BIG ? 1 : 2;               // accumulators of the first piece
 };
 
 __device__ __forceinline__ void mx_mma_ta(uint32_t tmem_c, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
@@ -99,11 +97,10 @@ struct MxArgs {
   const float *bias0, *bias1;
   const float *wts;
   const uint32_t *pair_src;
-  float *out;             // gate/up: h [P][ff]; down: eo [splits][P][d]
-  size_t split_stride;
+  float *out;             // gate/up: h [P][ff]; down: eo [P][d]
   int *err;
   unsigned long long wait_ns;
-  int row_tiles, splits, split_chunks;
+  int row_tiles;
   int cols, rows;
   int act;
   float act_limit, act_alpha;
@@ -113,7 +110,6 @@ struct MxArgs {
 // to 16 with zeros; a K group of 8 is values 4 j .. 4 j + 3 and 16 + 4 j .. of a block of 32, in the order the decoded
 // weights have. A thread a (row, K group): neighbouring lanes take neighbouring rows, whose 16 bytes are neighbours
 // in the operand.
-template <int NPC>
 __global__ void __launch_bounds__(256) k_mx_rows(const int *__restrict__ n_tiles, const uint4 *__restrict__ tiles,
                                                  const uint32_t *__restrict__ src_row, int cols, const float *__restrict__ x,
                                                  uint8_t *__restrict__ rec) {
@@ -149,23 +145,23 @@ __global__ void __launch_bounds__(256) k_mx_rows(const int *__restrict__ n_tiles
 
 struct MxItem {
   uint4 t;
-  int r0, c0, c1, split;  // first row, K chunks [c0, c1), which cut of K
+  int r0;  // first row
+  int pad[3];
 };
 #define MX_IT 4
 #define MX_END 0xfffffffeu
 
-template <bool DOWN, bool BIG, int NPC>
-__global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS) k_tc_mx(const __grid_constant__ MxArgs A) {
-  using S = MxShape<BIG, NPC>;
+template <bool DOWN>
+__global__ void __launch_bounds__(MxShape::NT, 1) k_tc_mx(const __grid_constant__ MxArgs A) {
+  using S = MxShape;
   constexpr int MW = S::NW / 32, NSR = S::NSR, NSB = S::NSB, MT = S::MT;
-  constexpr int RPC = DOWN ? MT * MX_M : MT * MX_M / 2;  // matrix rows of an item
+  constexpr int RPC = DOWN ? MT * MX_M : MX_M;  // matrix rows of an item
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t *sRaw = smem, *sB = sRaw + NSR * S::RAWB;
-  float *sX = (float *)(sB + NSB * S::BST);
-  MxItem *items = (MxItem *)((uint8_t *)sX + (DOWN ? 0 : S::XB));
+  MxItem *items = (MxItem *)(sB + NSB * S::BST);
   uint64_t *full_raw = (uint64_t *)(items + MX_IT), *empty_raw = full_raw + NSR, *full_b = empty_raw + NSR, *empty_b = full_b + NSB;
-  uint64_t *a_ready = empty_b + NSB, *a_free = a_ready + MX_NA, *acc_full = a_free + MX_NA, *acc_free = acc_full + S::NACC;
-  uint64_t *it_full = acc_free + S::NACC, *it_empty = it_full + MX_IT;
+  uint64_t *a_ready = empty_b + NSB, *a_free = a_ready + MX_NA, *acc_full = a_free + MX_NA, *acc_free = acc_full + 1;
+  uint64_t *it_full = acc_free + 1, *it_empty = it_full + MX_IT;
   uint32_t *tmem_slot = (uint32_t *)(it_empty + MX_IT);
   const int nbk = A.cols / 32, rows = A.rows, nch = (A.cols + MX_KC - 1) / MX_KC;
   const int tid = threadIdx.x, warp = __shfl_sync(PM_FULL, tid >> 5, 0), lane = tid & 31;
@@ -188,10 +184,8 @@ __global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS
       tc_mbar_init(a_ready + i, MW / 2);
       tc_mbar_init(a_free + i, 1);
     }
-    for (int i = 0; i < S::NACC; i++) {
-      tc_mbar_init(acc_full + i, 1);
-      tc_mbar_init(acc_free + i, MW);
-    }
+    tc_mbar_init(acc_full, 1);
+    tc_mbar_init(acc_free, MW);
     for (int i = 0; i < MX_IT; i++) {
       tc_mbar_init(it_full + i, 1);
       tc_mbar_init(it_empty + i, 1 + MW);
@@ -221,20 +215,11 @@ __global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS
     for (int k = 0; next_item(k, it); k++) {
       if ((int)it.t.x < 0) continue;
       const uint32_t npad = (__reduce_max_sync(PM_FULL, it.t.z) + 15u) & ~15u;
-      const int c0 = (int)__reduce_max_sync(PM_FULL, (uint32_t)it.c0), c1 = (int)__reduce_max_sync(PM_FULL, (uint32_t)it.c1);
       // instruction descriptor: D f32, A and B bf16, both K-major, N = npad, M = 128
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((npad >> 3) << 17) | ((uint32_t)(MX_M >> 4) << 24);
-      // the accumulators of the item before have been read (n_acc: hand-overs of accumulators so far)
-      if (n_acc > 0) tc_wait(acc_free + (n_acc - 1) % S::NACC, ((n_acc - 1) / S::NACC) & 1, A.err, A.wait_ns);
-      uint32_t d_main = tmem, first = 0;  // first piece's accumulator; its first chunk
-      for (int c = c0; c < c1; c++) {
-        const uint32_t a = (uint32_t)(c - c0) & 3u;
-        if (!BIG && a == 0) {
-          const uint32_t set = n_acc & 1;
-          if (n_acc > 1) tc_wait(acc_free + set, ((n_acc >> 1) - 1) & 1, A.err, A.wait_ns);
-          d_main = tmem + set * 32u;
-          first = (uint32_t)(c - c0);
-        }
+      if (n_acc > 0) tc_wait(acc_free, (n_acc - 1) & 1, A.err, A.wait_ns);  // the item before has been read
+      for (int c = 0; c < nch; c++) {
+        const uint32_t a = (uint32_t)c & 3u;
         const uint64_t dB = tc_desc(sB_a + sb * S::BST, npad * 16u, 128u);
         const int ksteps = min(4, (A.cols - c * MX_KC) / 16);  // (a trailing single block: 2 steps)
         tc_wait(full_b + sb, pb, A.err, A.wait_ns);
@@ -250,22 +235,20 @@ __global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS
                 for (int p = 0; p < NPC; p++) {  // (a piece is npad * 128 bytes, a K step two groups of npad * 16)
                   const uint32_t at = tmem + S::A0 + a * S::ACH + h * (MX_KC / 2) + 8u * ks;
                   const uint64_t db = dB + (uint64_t)(p * npad * 8 + ks * npad * 2);
-                  if (BIG) mx_mma_ta(tmem + h * 128u, at, db, idesc, (c > c0 || ks > 0 || p > 0) ? 1u : 0u);
-                  else if (p == 0) mx_mma_ta(d_main, at, db, idesc, (c - c0 > (int)first || ks > 0) ? 1u : 0u);
-                  else mx_mma_ta(tmem + 64u, at, db, idesc, (c > c0 || ks > 0 || p > 1) ? 1u : 0u);
+                  mx_mma_ta(tmem + h * 128u, at, db, idesc, (c > 0 || ks > 0 || p > 0) ? 1u : 0u);
                 }
               }
           tc_commit(a_free + a);
           tc_commit(empty_b + sb);
-          if (c == c1 - 1 || (!BIG && a == 3)) tc_commit(acc_full + n_acc % S::NACC);
+          if (c == nch - 1) tc_commit(acc_full);
         }
         __syncwarp();
-        if (c == c1 - 1 || (!BIG && a == 3)) n_acc++;
         if (a == 3) st++;
         if (++sb == NSB) { sb = 0; pb ^= 1; }
       }
       // (a last group of fewer than four chunks: its other places in the ring go round empty)
-      for (uint32_t a = (uint32_t)(c1 - c0) & 3u; a != 0 && a < 4; a++) {
+      n_acc++;
+      for (uint32_t a = (uint32_t)nch & 3u; a != 0 && a < 4; a++) {
         tc_wait(a_ready + a, st & 1, A.err, A.wait_ns);
         if (el) tc_mbar_arrive(a_free + a);
         if (a == 3) st++;
@@ -275,44 +258,40 @@ __global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS
     // ================= the producer: one thread =================
     if (tc_elect()) {
       const uint32_t sRaw_a = tc_s32(sRaw), sB_a = tc_s32(sB);
-      const int per_tile = A.row_tiles * A.splits, n_items = *A.n_tiles * per_tile, G = (int)gridDim.x;
+      const int n_items = *A.n_tiles * A.row_tiles, G = (int)gridDim.x;
       int cur = (int)blockIdx.x, nxt = cur + G;
       uint4 Tc = make_uint4(MX_END, 0, 0, 0), Tn = Tc;
-      if (cur < n_items) Tc = __ldg(A.tiles + cur / per_tile);
+      if (cur < n_items) Tc = __ldg(A.tiles + cur / A.row_tiles);
       uint32_t sr = 0, pr = 1, sb = 0, pb = 1, nr = 0, nbk_ = 0;
       bool ok = true;
       for (int k = 0; ok; k++) {
         const int s = k & (MX_IT - 1);
         if (k >= MX_IT && !tc_wait(it_empty + s, (uint32_t)((k / MX_IT - 1) & 1), A.err, A.wait_ns)) break;
         const bool end = cur >= n_items;
-        const int in = cur % per_tile, rt = in / A.splits, sp = in - rt * A.splits;
-        const int r0 = rt * RPC, c0 = sp * A.split_chunks, c1 = min(nch, c0 + A.split_chunks);
+        const int r0 = (cur % A.row_tiles) * RPC;
         MxItem it;
         it.t = end ? make_uint4(MX_END, 0, 0, 0) : Tc;
         it.r0 = r0;
-        it.c0 = c0;
-        it.c1 = c1;
-        it.split = sp;
         items[s] = it;
         tc_mbar_arrive(it_full + s);
         if (end) break;
         const int fut = 2 * G + (int)atomicAdd(A.next, 1u);  // (needed an item later)
-        if (nxt < n_items) Tn = __ldg(A.tiles + nxt / per_tile);
+        if (nxt < n_items) Tn = __ldg(A.tiles + nxt / A.row_tiles);
         if ((int)Tc.x >= 0) {
           const int el = (int)Tc.x;
           const uint32_t bytes = ((Tc.z + 15) >> 4) * (16u * MX_KC * 2 * NPC);
           const uint8_t *rec = A.rec + (size_t)Tc.w * nch * (MX_KC * 2 * NPC);
-          for (int c = c0; c < c1; c++) {
-            if (((c - c0) & 3) == 0) {  // nibbles of four chunks (a box past the matrix reads zeros; split_chunks is a multiple of 4)
+          for (int c = 0; c < nch; c++) {
+            if ((c & 3) == 0) {  // nibbles of four chunks (a box past the matrix reads zeros)
               const uint32_t r = sRaw_a + sr * S::RAWB;
               if (nr >= NSR && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
               tc_mbar_expect(full_raw + sr, (uint32_t)S::RAWB);
               if (DOWN) {
                 tc_tma3(r, &A.m0, c * 32, r0, el, full_raw + sr);
-                if (BIG) tc_tma3(r + MX_BOX, &A.m0, c * 32, r0 + MX_M, el, full_raw + sr);
-              } else {  // (boxes of 128 rows, or of 64 in the small shape)
+                tc_tma3(r + MX_BOX, &A.m0, c * 32, r0 + MX_M, el, full_raw + sr);
+              } else {
                 tc_tma3(r, &A.m0, c * 32, r0, el, full_raw + sr);
-                tc_tma3(r + (BIG ? MX_BOX : MX_BOX / 2), &A.m1, c * 32, r0, el, full_raw + sr);
+                tc_tma3(r + MX_BOX, &A.m1, c * 32, r0, el, full_raw + sr);
               }
               nr++;
               if (++sr == NSR) { sr = 0; pr ^= 1; }
@@ -348,14 +327,14 @@ __global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS
   } else {
     // ================= the workers =================
     // decode: thread = (row m of a 128-row half, half h); the even chunks or the odd ones (two blocks of 32 codes each)
-    const int m = tid & 127, part = warp >> 2, h = BIG ? part >> 1 : 0, par = part & 1;
+    const int m = tid & 127, part = warp >> 2, h = part >> 1, par = part & 1;
     const uint32_t tlane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
     uint32_t st = 0, sr = 0, pr = 0, n_acc = 0;
     MxItem it;
     for (int k = 0; next_item(k, it); k++) {
       const uint4 T = it.t;
       const int el = (int)T.x, nvalid = (int)T.z, npad = (nvalid + 15) & ~15, r0 = it.r0;
-      float *out = A.out + (size_t)it.split * A.split_stride + (size_t)T.y * rows;
+      float *out = A.out + (size_t)T.y * rows;
       if (el < 0) {  // an expert another rank holds: zeros (down) / nothing to do (gate/up)
         if (DOWN)
           for (int i = tid; i < nvalid * RPC; i += S::NW) {
@@ -364,9 +343,8 @@ __global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS
           }
         continue;
       }
-      // the matrix row this thread decodes: the up matrix holds half 1, or (small shape) rows 64 .. 127 of the tile
-      const bool up = !DOWN && (BIG ? h == 1 : m >= 64);
-      const int drow = DOWN ? r0 + h * MX_M + m : (BIG ? r0 + m : r0 + (m & 63));
+      const bool up = !DOWN && h == 1;  // the up matrix is half 1
+      const int drow = DOWN ? r0 + h * MX_M + m : r0 + m;
       // its scale bytes, eight blocks (four chunks) at a time: two aligned words hold them wherever the row starts
       const uint8_t *sp = (up ? A.s1 + (size_t)el * A.s1_stride : A.s0 + (size_t)el * A.s0_stride) + (size_t)min(drow, rows - 1) * nbk;
       auto scales = [&](int c) -> unsigned long long {
@@ -376,40 +354,10 @@ __global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS
         const unsigned long long a = __ldg(q), b = __ldg(q + 1);
         return sh ? (a >> sh) | (b << (64 - sh)) : a;
       };
-      // small shape: the thread's columns of the products of the first piece, summed up here every 256 K values
-      const int ew = BIG ? 0 : npad >> 1, ec0 = par * ew;
-      float acc[16];
-      if (!BIG)
-#pragma unroll
-        for (int u = 0; u < 16; u++) acc[u] = 0.0f;
-      auto fold = [&](bool last) {
-        const uint32_t set = n_acc & 1;
-        tc_wait(acc_full + set, (n_acc >> 1) & 1, A.err, A.wait_ns);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-        for (int c8 = 0; c8 < 16; c8 += 8)
-          if (c8 < ew) {
-            uint32_t v[8];
-            tc_ld8<0>(tlane + set * 32u + (uint32_t)(ec0 + c8), v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int u = 0; u < 8; u++) acc[c8 + u] = __fadd_rn(acc[c8 + u], __uint_as_float(v[u]));
-            if (last) {
-              tc_ld8<64>(tlane + (uint32_t)(ec0 + c8), v);
-              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-              for (int u = 0; u < 8; u++) acc[c8 + u] = __fadd_rn(acc[c8 + u], __uint_as_float(v[u]));
-            }
-          }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) tc_mbar_arrive(acc_free + set);
-        n_acc++;
-      };
-      unsigned long long sc_n = scales(it.c0);
-      for (int c4 = it.c0; c4 < it.c1; c4 += 4) {
+      unsigned long long sc_n = scales(0);
+      for (int c4 = 0; c4 < nch; c4 += 4) {
         const unsigned long long sc = sc_n;
-        if (c4 + 4 < it.c1) sc_n = scales(c4 + 4);
+        if (c4 + 4 < nch) sc_n = scales(c4 + 4);
         tc_wait(full_raw + sr, pr, A.err, A.wait_ns);
         const uint8_t *raw = sRaw + sr * S::RAWB + h * MX_BOX + m * 128;
         uint4 q[4];
@@ -431,7 +379,7 @@ __global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS
 #pragma unroll
         for (int j = 0; j < 2; j++) {
           const int a = 2 * j + par;
-          const bool on = c4 + a < it.c1;
+          const bool on = c4 + a < nch;
           uint32_t w[32];
           if (on) {
             const uint32_t e0 = ew4[j] & 0xffu, e1 = (ew4[j] >> 8) & 0xffu;
@@ -452,25 +400,20 @@ __global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS
         }
         stored(2 + par);
         st++;
-        if (!BIG && c4 > it.c0) fold(false);  // (of the 256 K values before: these are still being multiplied)
       }
       // ---- epilogue: TMEM lane m, the part's token columns ----
-      if (BIG) {
-        tc_wait(acc_full, n_acc & 1, A.err, A.wait_ns);
-        n_acc++;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      } else {
-        fold(true);
-      }
+      tc_wait(acc_full, n_acc & 1, A.err, A.wait_ns);
+      n_acc++;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const bool dead = *(volatile int *)A.err != 0;
       if (DOWN) {
-        const float bd = A.bias0 && it.split == 0 && drow < rows ? A.bias0[(size_t)el * rows + drow] : 0.0f;
-        const bool on = !dead && drow < rows, bias = A.bias0 && it.split == 0;
+        const float bd = A.bias0 && drow < rows ? A.bias0[(size_t)el * rows + drow] : 0.0f;
+        const bool on = !dead && drow < rows, bias = A.bias0 != nullptr;
         auto put = [&](int n, float o) {
           if (bias) o = __fadd_rn(o, bd);
           if (on && n < nvalid) out[(size_t)n * rows + drow] = o;
         };
-        if constexpr (BIG) {
+        {
           const int hw = npad >> 1, c0 = par * hw;  // half of the columns: a multiple of 8
           for (int c8 = 0; c8 < hw; c8 += 8) {
             uint32_t v[8];
@@ -482,13 +425,9 @@ __global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0) tc_mbar_arrive(acc_free);
-        } else {
-#pragma unroll
-          for (int u = 0; u < 16; u++)
-            if (u < ew) put(ec0 + u, acc[u]);
         }
       } else {
-        const int hrow = BIG ? r0 + m : r0 + (m & 63);  // the h row this thread activates
+        const int hrow = r0 + m;  // the h row this thread activates
         const bool on = !dead && hrow < rows;
         const float bg = A.bias0 && hrow < rows ? A.bias0[(size_t)el * rows + hrow] : 0.0f;
         const float bu = A.bias0 && hrow < rows ? A.bias1[(size_t)el * rows + hrow] : 0.0f;
@@ -500,7 +439,7 @@ __global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS
           const float wt = A.wts ? A.wts[A.pair_src[T.y + n]] : 1.0f;
           out[(size_t)n * rows + hrow] = pm_act(A.act, A.act_limit, A.act_alpha, gv, uv, wt, A.wts != nullptr);
         };
-        if constexpr (BIG) {  // gate sums in columns 0 .., up sums in 128 ..: a quarter of the tokens a thread
+        {  // gate sums in columns 0 .., up sums in 128 ..: a quarter of the tokens a thread
           const int qw = npad >> 2, c0 = part * qw;
           for (int c4 = 0; c4 < qw; c4 += 4) {
             uint32_t vg[4], vu[4];
@@ -514,17 +453,6 @@ __global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0) tc_mbar_arrive(acc_free);
-        } else {  // gate rows in lanes 0..63, up rows in 64..127: the warps w and w ^ 2 exchange through shared memory
-          float *sx = sX + par * (S::NTOK / 2) * MX_M;
-#pragma unroll
-          for (int u = 0; u < 16; u++)
-            if (u < ew) sx[u * MX_M + m] = acc[u];
-          asm volatile("bar.sync %0, 64;" ::"r"(1 + 2 * par + (warp & 1)) : "memory");
-          const int f = up ? ew >> 1 : 0;
-#pragma unroll 2
-          for (int i = f; i < f + (ew >> 1); i++)
-            if (on && ec0 + i < nvalid) put(ec0 + i, sx[i * MX_M + (m & 63)], sx[i * MX_M + 64 + (m & 63)]);
-          // (nobody writes the area again before every warp has stored operand A of the next item's first chunk)
         }
       }
     }
@@ -534,66 +462,46 @@ __global__ void __launch_bounds__(MxShape<BIG, NPC>::NT, MxShape<BIG, NPC>::CTAS
   if (warp == MW) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::COLS) : "memory");
 }
 
-// bytes of the pieces of n_pairs rows of `cols` values in at most max_groups groups, three pieces a value
+// bytes of the pieces of n_pairs rows of `cols` values in at most max_groups groups
 size_t mx_rec_bytes(int n_pairs, int max_groups, int cols) {
   const size_t groups = (size_t)(max_groups < n_pairs ? max_groups : n_pairs);
-  return ((size_t)n_pairs + 15 * groups + 16) * ((cols + MX_KC - 1) / MX_KC) * (MX_KC * 2 * 3);
+  return ((size_t)n_pairs + 15 * groups + 16) * ((cols + MX_KC - 1) / MX_KC) * (MX_KC * 2 * NPC);
 }
-void launch_mx_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x, int pieces,
+void launch_mx_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x,
                     uint8_t *rec) {
   const long units = ((long)n_rows + 15 * t.max_tiles) * ((cols + 7) / 8);
   const long gx = (units / t.max_tiles + 511) / 512;  // two units a thread
   const dim3 grid((unsigned)(gx < 1 ? 1 : gx), (unsigned)t.max_tiles);
-  if (pieces == 3) pm_launch(L, k_mx_rows<3>, grid, 256, 0, t.n, t.tiles, src_row, cols, x, rec);
-  else pm_launch(L, k_mx_rows<2>, grid, 256, 0, t.n, t.tiles, src_row, cols, x, rec);
+  pm_launch(L, k_mx_rows, grid, 256, 0, t.n, t.tiles, src_row, cols, x, rec);
 }
 
-template <bool DOWN, bool BIG, int NPC> static cudaError_t mx_start(const Launch &L, const MxArgs &A, long items) {
-  using S = MxShape<BIG, NPC>;
-  constexpr size_t smem = (size_t)S::NSR * S::RAWB + (size_t)S::NSB * S::BST + (DOWN ? 0 : S::XB) + MX_IT * sizeof(MxItem) +
-                          (2 * S::NSR + 2 * S::NSB + 2 * MX_NA + 2 * S::NACC + 2 * MX_IT) * 8 + 16;
-  static_assert(smem <= (S::CTAS == 1 ? 232448 : 115712), "more than an SM's shared memory");
+template <bool DOWN> static cudaError_t mx_start(const Launch &L, const MxArgs &A, long items) {
+  using S = MxShape;
+  constexpr size_t smem = (size_t)S::NSR * S::RAWB + (size_t)S::NSB * S::BST + MX_IT * sizeof(MxItem) +
+                          (2 * S::NSR + 2 * S::NSB + 2 * MX_NA + 2 + 2 * MX_IT) * 8 + 16;
+  static_assert(smem <= 232448, "more than an SM's shared memory");
   static bool set[64] = {};  // (one-time per device and kernel)
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64 || !set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(k_tc_mx<DOWN, BIG, NPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_tc_mx<DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     if (dev < 64) set[dev] = true;
   }
-  const long ctas = (long)S::CTAS * L.n_sm;
-  return pm_launch(L, k_tc_mx<DOWN, BIG, NPC>, dim3((unsigned)(items < ctas ? items : ctas)), S::NT, smem, A);
-}
-
-int mx_small_tokens() { return MxShape<false, 2>::NTOK; }
-// Cuts of K of the down products: a few tokens make ceil(d / 128) items an expert, each a chain of ff / 64 chunks;
-// while that leaves CTAs without work, K is cut in up to four (the combine step adds the parts in order).
-static int mx_split_chunks(int nch, int splits) { return ((nch + splits - 1) / splits + 3) & ~3; }  // whole boxes
-int mx_splits(const pm_layer_desc &D, int n_pairs) {
-  const int nch = (D.ff + MX_KC - 1) / MX_KC;
-  // (a pair is at most a tile of its own; two CTAs on each of 148 SMs)
-  const long items = (long)((D.d + MX_M - 1) / MX_M) * n_pairs;
-  long s = 296 / (items > 0 ? items : 1);
-  s = s > 4 ? 4 : s;
-  s = s > nch / 8 ? nch / 8 : s;  // at least eight chunks each
-  if (s <= 1) return 1;
-  const int sc = mx_split_chunks(nch, (int)s);
-  return (nch + sc - 1) / sc;  // (rounding up may leave fewer)
+  const long ctas = L.n_sm;
+  return pm_launch(L, k_tc_mx<DOWN>, dim3((unsigned)(items < ctas ? items : ctas)), S::NT, smem, A);
 }
 
 // Tensor-core form of launch_gateup / launch_down for MXFP4 weights and f32 activations given as the pieces of
-// the grouping's rows. splits: cuts of K (down only); split s goes to out + s * split_stride.
-cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t, int pieces,
-                         const uint8_t *rec, const float *wts, float *out, int splits, size_t split_stride, int *err,
-                         unsigned long long wait_ns) {
+// the grouping's rows.
+cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
+                         const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns) {
   if (t.max_tiles == 0) return cudaSuccess;
-  const bool big = t.ntok != MxShape<false, 2>::NTOK;
   const WMat &W0 = down ? ly.down : ly.gate, &W1 = ly.up;
   const WMaps &M0 = down ? ly.maps->down : ly.maps->gate, &M1 = ly.maps->up;
   MxArgs A;
-  const int box = !down && !big ? 0 : 1;  // boxes of 64 or 128 rows
-  A.m0 = M0.m[box];
-  A.m1 = M1.m[box];
+    A.m0 = M0.m[1];  // boxes of 128 rows
+  A.m1 = M1.m[1];
   A.s0 = W0.plane[1];
   A.s0_stride = W0.stride[1];
   A.s1 = W1.plane[1];
@@ -607,21 +515,15 @@ cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const u
   A.wts = !down && ly.desc.weight_fold == PM_FOLD_BEFORE_DOWN ? wts : nullptr;
   A.pair_src = pair_src;
   A.out = out;
-  A.split_stride = split_stride;
   A.err = err;
   A.wait_ns = wait_ns;
-  const int rpc = down ? (big ? 2 * MX_M : MX_M) : (big ? MX_M : MX_M / 2);
+  const int rpc = down ? 2 * MX_M : MX_M;
   A.row_tiles = (W0.rows + rpc - 1) / rpc;
-  const int nch = (W0.cols + MX_KC - 1) / MX_KC;
-  A.split_chunks = mx_split_chunks(nch, splits);
-  A.splits = splits;
   A.cols = W0.cols;
   A.rows = W0.rows;
   A.act = ly.desc.act;
   A.act_limit = ly.desc.act_limit;
   A.act_alpha = ly.desc.act_alpha;
-  const long items = (long)A.row_tiles * A.splits * t.max_tiles;
-  if (big) return down ? mx_start<true, true, 2>(L, A, items) : mx_start<false, true, 2>(L, A, items);
-  if (pieces == 3) return down ? mx_start<true, false, 3>(L, A, items) : mx_start<false, false, 3>(L, A, items);
-  return down ? mx_start<true, false, 2>(L, A, items) : mx_start<false, false, 2>(L, A, items);
+  const long items = (long)A.row_tiles * t.max_tiles;
+  return down ? mx_start<true>(L, A, items) : mx_start<false>(L, A, items);
 }

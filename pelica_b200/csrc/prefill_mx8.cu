@@ -1,0 +1,542 @@
+// prefill_mx8.cu - grouped expert products on MXFP4 weights and f32 activations for small groups (a few tokens an
+// expert): tcgen05.mma kind::mxf8f6f4 with block scales. The tensor cores take the E2M1 codes and their E8M0
+// scales as they are stored (src/oss_kernels.rs:41-55: code * 2^(e - 127)), so nothing is decoded; a worker only
+// moves a row's nibbles from the packed box to the operand's layout.
+//
+// The activations are exact sums of E4M3 pieces with block scales of their own: x = x1 + x2 + ..., xi the
+// nearest E4M3 of what is left of x, in units of 2^(E - 7 - 5 (i - 1)), E the exponent of the block's largest value.
+// What a piece leaves is at most a 32nd of what it was given: 5 pieces hold all 24 bits of an f32 (calls of fewer than
+// PM_MX_PROMPT tokens), 4 leave 2^-19 (prompts; the two bf16 pieces of prefill_mx.cu leave 2^-17). The pieces of a
+// tile's tokens are columns of ONE product: N = pieces x tokens, a sum each, added up smallest first. With 5 pieces
+// the sums are folded into f32 registers every 256 K values (the tensor cores' own sums lose the low bits
+// of a long chain: 1e-5 of the RMS over 2,880 values against 1e-7).
+//
+// A persistent pipeline as in prefill_mx.cu; two CTAs an SM, 128 weight rows (64 of gate and 64 of up, or 128 of down) x
+// 16 tokens (5 pieces) or 32 (4). Rows of gate and up alternate in tensor memory, so the two sums of an output are
+// neighbouring lanes. Bound by the weights' bytes.
+#include <cuda_fp16.h>
+
+#include "tcgen.cuh"
+
+#define M8_M 128
+#define M8_KS 128     /* K values of a stage: four products of 32 */
+#define M8_RAW (M8_M * 128)   /* packed nibbles of 128 rows x 256 K values: two stages */
+#define M8_AST (M8_M * 128)   /* operand A of a stage: 16 codes = 8 bytes and 8 unused, rows of 128 bytes, swizzled */
+#define M8_NW 8
+#define M8_NT (32 * (M8_NW + 2))
+#define M8_NA 2
+#define M8_NSB 2
+#define M8_IT 4
+#define M8_END 0xfffffffeu
+
+template <int NP> struct M8Shape {
+  static constexpr int NTOK = NP == 5 ? 16 : 32;
+  static constexpr bool FOLD = NP == 5;
+  static constexpr int NSR = NP == 5 ? 3 : 2;
+  static constexpr int BST = NP * NTOK * M8_KS + 512;  // the pieces of a stage and their scales
+  static constexpr uint32_t SET = NP * 16;             // columns of a set of sums (folded: two sets)
+  static constexpr uint32_t SFA = 240, SFB = 244;      // columns of the scales
+  static constexpr int NACC = FOLD ? 2 : 1;
+};
+static_assert(2 * M8Shape<5>::SET <= M8Shape<5>::SFA && 4 * 32 <= M8Shape<4>::SFA, "sums and scales share 256 columns");
+
+struct M8Args {
+  CUtensorMap m0, m1;     // nibble planes of gate or down, of up (boxes of 64 rows; down: of 128)
+  const uint8_t *s0, *s1; // their planes of scale bytes
+  size_t s0_stride, s1_stride;
+  const uint4 *tiles;
+  const int *n_tiles;
+  unsigned int *next;
+  const uint8_t *rec;     // the tokens' pieces (k_mx8_rows)
+  const float *bias0, *bias1;
+  const float *wts;
+  const uint32_t *pair_src;
+  float *out;             // gate/up: h [P][ff]; down: eo [splits][P][d]
+  size_t split_stride;
+  int *err;
+  unsigned long long wait_ns;
+  int row_tiles, splits, split_stages;
+  int cols, rows;
+  int act;
+  float act_limit, act_alpha;
+};
+
+__device__ __forceinline__ void m8_mma(uint32_t tmem_c, uint64_t da, uint64_t db, uint32_t idesc, uint32_t sfa, uint32_t sfb,
+                                       uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], %1, %2, %3, [%4], [%5], p;\n\t}\n" ::"r"(tmem_c),
+      "l"(da), "l"(db), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
+      : "memory");
+}
+// 512 bytes of scales (row r, K block k at (r & 31) * 16 + (r >> 5) * 4 + k) -> four columns of every lane quarter
+__device__ __forceinline__ void m8_cp_scales(uint32_t tmem_c, uint64_t desc) {
+  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem_c), "l"(desc) : "memory");
+}
+__device__ __forceinline__ uint32_t m8_e4m3x2(float hi, float lo) {
+  uint16_t r;
+  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ float2 m8_from_e4m3x2(uint32_t v) {
+  uint32_t h;
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h) : "h"((uint16_t)v));
+  return __half22float2(*reinterpret_cast<const __half2 *>(&h));
+}
+__device__ __forceinline__ float m8_pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }  // -126 .. 127
+
+// f32 rows -> their pieces: per tile and stage [4 K blocks][2 groups of 16][pieces x rows][16], then the scales. A block's 32
+// values lie as the packed codes come apart: group 0 holds values 0, 16, 1, 17 .. 7, 23, group 1 the others. A thread
+// a (row, block).
+template <int NP>
+__global__ void __launch_bounds__(128) k_mx8_rows(const int *__restrict__ n_tiles, const uint4 *__restrict__ tiles,
+                                                  const uint32_t *__restrict__ src_row, int cols, const float *__restrict__ x,
+                                                  uint8_t *__restrict__ rec) {
+  pm_pdl();
+  if ((int)blockIdx.y >= *n_tiles) return;
+  const uint4 T = tiles[blockIdx.y];
+  const int npad = ((int)T.z + 15) & ~15, nst = (cols + M8_KS - 1) / M8_KS, nb = cols / 32, N = NP * npad;
+  uint8_t *base = rec + (size_t)(T.w >> 4) * nst * (2048 * NP + 512);
+  for (int u = blockIdx.x * 128 + threadIdx.x; u < nb * npad; u += gridDim.x * 128) {
+    const int b = u / npad, r = u - b * npad;
+    float v[32];
+    uint32_t top = 0;
+    const bool on = r < (int)T.z;
+    const size_t row = on ? (src_row ? src_row[T.y + r] : T.y + r) : 0;
+    const float4 *src = (const float4 *)(x + row * cols + 32 * b);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const float4 f = on ? __ldg(src + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
+    }
+#pragma unroll
+    for (int i = 0; i < 32; i++) top = max(top, __float_as_uint(v[i]) & 0x7fffffffu);
+    const int E = (int)(top >> 23) - 127;
+    uint8_t *dst = base + (size_t)(b >> 2) * (N * M8_KS + 512) + (size_t)(b & 3) * (N * 32);
+    uint8_t *sf = base + (size_t)(b >> 2) * (N * M8_KS + 512) + N * M8_KS + (b & 3);
+#pragma unroll
+    for (int p = 0; p < NP; p++) {
+      const int S = max(E - 7 - 5 * p, -126);
+      const float up = m8_pow2(-S), down = m8_pow2(S);
+      uint32_t w[8];
+#pragma unroll
+      for (int i = 0; i < 16; i++) {  // (16 times: values i and i + 16)
+        const uint32_t c = m8_e4m3x2(__fmul_rn(v[i + 16], up), __fmul_rn(v[i], up));
+        const float2 f = m8_from_e4m3x2(c);
+        v[i] = __fsub_rn(v[i], __fmul_rn(f.x, down));
+        v[i + 16] = __fsub_rn(v[i + 16], __fmul_rn(f.y, down));
+        if (i & 1) w[i >> 1] |= c << 16;
+        else w[i >> 1] = c;
+      }
+      if (top >= 0x7f800000u) {  // an infinity or a NaN in the block: NaN, as its bf16 pieces add up to
+#pragma unroll
+        for (int i = 0; i < 8; i++) w[i] = 0x7f7f7f7fu;
+      }
+      const int n = p * npad + r;
+      *(uint4 *)(dst + (size_t)n * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+      *(uint4 *)(dst + (size_t)(N + n) * 16) = make_uint4(w[4], w[5], w[6], w[7]);
+      sf[(n & 31) * 16 + (n >> 5) * 4] = (uint8_t)(S + 127);
+    }
+  }
+}
+
+struct M8Item {
+  uint4 t;
+  int r0, s0, s1, split;  // first row, stages [s0, s1), which cut of K
+};
+
+template <bool DOWN, int NP>
+__global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8Args A) {
+  using S = M8Shape<NP>;
+  constexpr int MW = M8_NW, NSR = S::NSR, NACC = S::NACC;
+  constexpr int RPC = DOWN ? M8_M : M8_M / 2;  // matrix rows of an item
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t *sRaw = smem, *sA = sRaw + NSR * M8_RAW, *sB = sA + M8_NA * M8_AST, *sSA = sB + M8_NSB * S::BST;
+  M8Item *items = (M8Item *)(sSA + M8_NA * 512);
+  uint64_t *full_raw = (uint64_t *)(items + M8_IT), *empty_raw = full_raw + NSR, *full_b = empty_raw + NSR;
+  uint64_t *empty_b = full_b + M8_NSB, *a_ready = empty_b + M8_NSB, *a_free = a_ready + M8_NA, *acc_full = a_free + M8_NA;
+  uint64_t *acc_free = acc_full + NACC, *it_full = acc_free + NACC, *it_empty = it_full + M8_IT;
+  uint32_t *tmem_slot = (uint32_t *)(it_empty + M8_IT);
+  const int nbk = A.cols / 32, rows = A.rows, nst = (A.cols + M8_KS - 1) / M8_KS;
+  const int tid = threadIdx.x, warp = __shfl_sync(PM_FULL, tid >> 5, 0), lane = tid & 31;
+
+  pm_pdl_trigger();
+  if (warp == MW) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_s32(tmem_slot)), "r"(256u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid == 0) {
+    for (int i = 0; i < NSR; i++) {
+      tc_mbar_init(full_raw + i, 1);
+      tc_mbar_init(empty_raw + i, MW);
+    }
+    for (int i = 0; i < M8_NSB; i++) {
+      tc_mbar_init(full_b + i, 1);
+      tc_mbar_init(empty_b + i, 1);
+    }
+    for (int i = 0; i < M8_NA; i++) {
+      tc_mbar_init(a_ready + i, MW);
+      tc_mbar_init(a_free + i, 1);
+    }
+    for (int i = 0; i < NACC; i++) {
+      tc_mbar_init(acc_full + i, 1);
+      tc_mbar_init(acc_free + i, MW);
+    }
+    for (int i = 0; i < M8_IT; i++) {
+      tc_mbar_init(it_full + i, 1);
+      tc_mbar_init(it_empty + i, 1 + MW);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = __reduce_max_sync(PM_FULL, *tmem_slot);
+  pm_pdl_wait();
+  auto next_item = [&](int k, M8Item &it) -> bool {
+    const int s = k & (M8_IT - 1);
+    const bool ok = tc_wait(it_full + s, (uint32_t)((k / M8_IT) & 1), A.err, A.wait_ns);
+    it = items[s];
+    __syncwarp();
+    if (lane == 0) tc_mbar_arrive(it_empty + s);
+    return ok && it.t.x != M8_END;
+  };
+
+  if (warp == MW) {
+    // ================= the issuing warp =================
+    const uint32_t el = tc_elect() ? 1u : 0u;
+    const uint32_t sA_a = tc_s32(sA), sB_a = tc_s32(sB), sSA_a = tc_s32(sSA);
+    uint32_t st = 0, sb = 0, pb = 0, set = 0, ps = 1;
+    M8Item it;
+    for (int k = 0; next_item(k, it); k++) {
+      if ((int)it.t.x < 0) continue;
+      const uint32_t npad = (__reduce_max_sync(PM_FULL, it.t.z) + 15u) & ~15u, N = NP * npad;
+      const int s0 = (int)__reduce_max_sync(PM_FULL, (uint32_t)it.s0), s1 = (int)__reduce_max_sync(PM_FULL, (uint32_t)it.s1);
+      // instruction descriptor: A E2M1 (5), B E4M3 (0), both K-major, UE8M0 scales, N, M = 128; bits 4..5 and 29..30: which
+      // byte of the scale columns
+      const uint32_t idesc = (5u << 7) | ((N >> 3) << 17) | (1u << 23) | (1u << 27);
+      for (int s = s0; s < s1; s++, st++) {
+        const uint32_t a = st & 1;
+        const bool first = S::FOLD ? ((s - s0) & 1) == 0 : s == s0;
+        const bool last = S::FOLD ? ((s - s0) & 1) == 1 || s == s1 - 1 : s == s1 - 1;
+        if (first) tc_wait(acc_free + set, ps, A.err, A.wait_ns);
+        tc_wait(full_b + sb, pb, A.err, A.wait_ns);
+        tc_wait(a_ready + a, (st >> 1) & 1, A.err, A.wait_ns);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // operand A: rows of 128 bytes, 128-byte swizzle (layout type 2), groups of 8 rows 1024 bytes apart
+        const uint64_t dA = (tc_desc(sA_a + a * M8_AST, 16u, 1024u)) | (2ull << 61);
+        const uint64_t dB = tc_desc(sB_a + sb * S::BST, N * 16u, 128u);
+        const int ksteps = min(4, (A.cols - s * M8_KS) / 32);
+        if (el) {
+          m8_cp_scales(tmem + S::SFA, tc_desc(sSA_a + a * 512u, 128u, 128u));
+          m8_cp_scales(tmem + S::SFB, tc_desc(sB_a + sb * S::BST + N * M8_KS, 128u, 128u));
+#pragma unroll
+          for (uint32_t ks = 0; ks < 4; ks++)
+            if ((int)ks < ksteps)
+              m8_mma(tmem + set * S::SET, dA + 2u * ks, dB + (uint64_t)(ks * N * 2u), idesc | (ks << 4) | (ks << 29), tmem + S::SFA,
+                     tmem + S::SFB, !first || ks > 0 ? 1u : 0u);
+          tc_commit(a_free + a);
+          tc_commit(empty_b + sb);
+          if (last) tc_commit(acc_full + set);
+        }
+        __syncwarp();
+        if (++sb == M8_NSB) { sb = 0; pb ^= 1; }
+        if (last && ++set == NACC) { set = 0; ps ^= 1; }
+      }
+    }
+  } else if (warp == MW + 1) {
+    // ================= the producer: one thread =================
+    if (tc_elect()) {
+      const uint32_t sRaw_a = tc_s32(sRaw), sB_a = tc_s32(sB);
+      const int per_tile = A.row_tiles * A.splits, n_items = *A.n_tiles * per_tile, G = (int)gridDim.x;
+      int cur = (int)blockIdx.x, nxt = cur + G;
+      uint4 Tc = make_uint4(M8_END, 0, 0, 0), Tn = Tc;
+      if (cur < n_items) Tc = __ldg(A.tiles + cur / per_tile);
+      uint32_t sr = 0, pr = 1, sb = 0, pb = 1, nr = 0, nB = 0;
+      bool ok = true;
+      for (int k = 0; ok; k++) {
+        const int s = k & (M8_IT - 1);
+        if (k >= M8_IT && !tc_wait(it_empty + s, (uint32_t)((k / M8_IT - 1) & 1), A.err, A.wait_ns)) break;
+        const bool end = cur >= n_items;
+        const int in = cur % per_tile, rt = in / A.splits, sp = in - rt * A.splits;
+        const int r0 = rt * RPC, s0 = sp * A.split_stages, s1 = min(nst, s0 + A.split_stages);
+        M8Item it;
+        it.t = end ? make_uint4(M8_END, 0, 0, 0) : Tc;
+        it.r0 = r0;
+        it.s0 = s0;
+        it.s1 = s1;
+        it.split = sp;
+        items[s] = it;
+        tc_mbar_arrive(it_full + s);
+        if (end) break;
+        const int fut = 2 * G + (int)atomicAdd(A.next, 1u);  // (needed an item later)
+        if (nxt < n_items) Tn = __ldg(A.tiles + nxt / per_tile);
+        if ((int)Tc.x >= 0) {
+          const int el = (int)Tc.x;
+          const uint32_t bytes = ((Tc.z + 15) >> 4) * (16u * M8_KS * NP) + 512u;
+          const uint8_t *rec = A.rec + (size_t)(Tc.w >> 4) * nst * (2048 * NP + 512);
+          for (int q = s0; q < s1; q++) {
+            if (((q - s0) & 1) == 0) {  // nibbles of two stages (a box past the matrix reads zeros; split_stages is even)
+              const uint32_t r = sRaw_a + sr * M8_RAW;
+              if (nr >= NSR && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
+              tc_mbar_expect(full_raw + sr, (uint32_t)M8_RAW);
+              tc_tma3(r, &A.m0, q * 64, r0, el, full_raw + sr);  // boxes of 128 rows (down) or 64
+              if (!DOWN) tc_tma3(r + M8_RAW / 2, &A.m1, q * 64, r0, el, full_raw + sr);
+              nr++;
+              if (++sr == NSR) { sr = 0; pr ^= 1; }
+            }
+            if (nB >= M8_NSB && !tc_wait(empty_b + sb, pb, A.err, A.wait_ns)) { ok = false; break; }
+            tc_mbar_expect(full_b + sb, bytes);
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sB_a + sb * S::BST),
+                         "l"(rec + (size_t)q * bytes), "r"(bytes), "r"(tc_s32(full_b + sb))
+                         : "memory");
+            nB++;
+            if (++sb == M8_NSB) { sb = 0; pb ^= 1; }
+          }
+        }
+        cur = nxt;
+        nxt = fut;
+        Tc = Tn;
+      }
+      // the last copies have landed before the CTA gives up its shared memory
+      for (uint32_t i = 1; i <= NSR && i <= nr; i++) {
+        const uint32_t q = nr - i;
+        const unsigned long long t0 = tc_now();
+        while (!tc_bar_test(full_raw + q % NSR, (q / NSR) & 1) && tc_now() - t0 < A.wait_ns) {
+        }
+      }
+      for (uint32_t i = 1; i <= M8_NSB && i <= nB; i++) {
+        const uint32_t q = nB - i;
+        const unsigned long long t0 = tc_now();
+        while (!tc_bar_test(full_b + q % M8_NSB, (q / M8_NSB) & 1) && tc_now() - t0 < A.wait_ns) {
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    // ================= the workers =================
+    // operand A: thread = (row m, half `part` of a stage's K values); sums: lane m, half `part` of the tokens. Row m of the
+    // tile: row m / 2 of gate (m even) or of up (odd); down: row m.
+    const int m = tid & 127;
+    const int part = (int)__reduce_max_sync(PM_FULL, (unsigned)warp >> 2);
+    const bool up = !DOWN && (m & 1);
+    const int mrow = DOWN ? m : m >> 1, rawr = DOWN ? m : (m >> 1) + 64 * (m & 1);
+    const uint32_t tlane = tmem + (__reduce_max_sync(PM_FULL, 32u * (warp & 3)) << 16);
+    uint32_t st = 0, sr = 0, pr = 0, set = 0, pf = 0;
+    M8Item it;
+    for (int k = 0; next_item(k, it); k++) {
+      const uint4 T = it.t;
+      const int el = (int)T.x, nvalid = (int)__reduce_max_sync(PM_FULL, T.z), r0 = it.r0;
+      const uint32_t npad = ((uint32_t)nvalid + 15u) & ~15u;
+      const int ew = (int)npad >> 1, e0 = part * ew, row = r0 + mrow;
+      if (el < 0) {  // an expert another rank holds: zeros (down) / nothing to do (gate/up)
+        if (DOWN)
+          for (int i = tid; i < nvalid * RPC; i += 32 * M8_NW) {
+            const int n = i / RPC, mm = i - n * RPC;
+            if (r0 + mm < rows) A.out[(size_t)it.split * A.split_stride + (size_t)(T.y + n) * rows + r0 + mm] = 0.0f;
+          }
+        continue;
+      }
+      // the row's scale bytes, eight blocks (two stages) at a time: two aligned words hold them wherever the row starts
+      const uint8_t *sp = (up ? A.s1 + (size_t)el * A.s1_stride : A.s0 + (size_t)el * A.s0_stride) + (size_t)min(row, rows - 1) * nbk;
+      auto scales = [&](int s) -> unsigned long long {
+        const uintptr_t p = (uintptr_t)(sp + 4 * s);
+        const unsigned long long *q = (const unsigned long long *)(p & ~(uintptr_t)7);
+        const int sh = 8 * (int)(p & 7);
+        const unsigned long long a = __ldg(q), b = __ldg(q + 1);
+        return sh ? (a >> sh) | (b << (64 - sh)) : a;
+      };
+      float acc[16];
+#pragma unroll
+      for (int u = 0; u < 16; u++) acc[u] = 0.0f;
+      auto fold = [&] {  // the pieces' sums of the thread's tokens, smallest piece first
+        tc_wait(acc_full + set, pf, A.err, A.wait_ns);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t at = tlane + set * S::SET + (uint32_t)e0;
+#pragma unroll
+        for (int c = 0; c < S::NTOK / 2; c += 8)
+          if (c < ew) {
+            uint32_t v[NP][8];
+#pragma unroll
+            for (int p = 0; p < NP; p++) tc_ld8<0>(at + (uint32_t)c + p * npad, v[p]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+              float t = __uint_as_float(v[NP - 1][u]);
+#pragma unroll
+              for (int p = NP - 2; p >= 0; p--) t = __fadd_rn(t, __uint_as_float(v[p][u]));
+              acc[c + u] = __fadd_rn(acc[c + u], t);
+            }
+          }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) tc_mbar_arrive(acc_free + set);
+        if (++set == NACC) { set = 0; pf ^= 1; }
+      };
+      unsigned long long sc_n = part == 0 ? scales(it.s0) : 0;
+#pragma unroll 1
+      for (int s2 = it.s0; s2 < it.s1; s2 += 2) {
+        const unsigned long long sc = sc_n;
+        if (part == 0 && s2 + 2 < it.s1) sc_n = scales(s2 + 2);
+        tc_wait(full_raw + sr, pr, A.err, A.wait_ns);
+        const uint8_t *raw = sRaw + sr * M8_RAW + rawr * 128;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          const bool on = s2 + j < it.s1;
+          uint4 q[2];
+          if (on)
+#pragma unroll
+            for (int i = 0; i < 2; i++)  // (TMA swizzle: 16-byte piece i of a row sits at i ^ (row & 7))
+              q[i] = *(const uint4 *)(raw + (((4 * j + 2 * part + i) ^ (rawr & 7)) << 4));
+          if (j == 1) {
+#pragma unroll
+            for (int i = 0; i < 2; i++) asm volatile("" : "+r"(q[i].x), "+r"(q[i].y), "+r"(q[i].z), "+r"(q[i].w));
+            __syncwarp();
+            if (lane == 0) tc_mbar_arrive(empty_raw + sr);
+            if (++sr == NSR) { sr = 0; pr ^= 1; }
+          }
+          if (on) {
+            const uint32_t a = st & 1;
+            if (st >= M8_NA) tc_wait(a_free + a, ((st >> 1) - 1) & 1, A.err, A.wait_ns);
+            uint8_t *dst = sA + a * M8_AST + m * 128;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {  // 32 codes: two groups of 16, the lower half of 16 bytes each
+              *(uint2 *)(dst + (((4 * part + 2 * i) ^ (m & 7)) << 4)) = make_uint2(q[i].x, q[i].y);
+              *(uint2 *)(dst + (((4 * part + 2 * i + 1) ^ (m & 7)) << 4)) = make_uint2(q[i].z, q[i].w);
+            }
+            if (part == 0) {  // (255, which the format reserves, counts as 254)
+              const uint32_t e4 = (uint32_t)(sc >> (32 * j));
+              *(uint32_t *)(sSA + a * 512 + (m & 31) * 16 + (m >> 5) * 4) = __vminu4(e4, 0xfefefefeu);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc_mbar_arrive(a_ready + a);
+            st++;
+          }
+        }
+        if (S::FOLD && s2 > it.s0) fold();  // (of the 256 K values before: these are still being multiplied)
+      }
+      fold();
+      // ---- epilogue ----
+      const bool on = row < rows && *(volatile int *)A.err == 0;
+      const bool bias = A.bias0 && it.split == 0;
+      const float b0 = bias && row < rows ? A.bias0[(size_t)el * rows + row] : 0.0f;
+      const float b1 = !DOWN && bias && row < rows ? A.bias1[(size_t)el * rows + row] : 0.0f;
+      float *out = A.out + (size_t)it.split * A.split_stride + (size_t)T.y * rows + row;
+#pragma unroll
+      for (int u = 0; u < S::NTOK / 2; u += 2)
+        if (u < ew) {
+          if constexpr (DOWN) {
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+              if (on && e0 + u + i < nvalid) out[(size_t)(e0 + u + i) * rows] = bias ? __fadd_rn(acc[u + i], b0) : acc[u + i];
+          } else {  // a gate lane activates token u, the up lane beside it token u + 1
+            const float other = __shfl_xor_sync(PM_FULL, up ? acc[u] : acc[u + 1], 1);
+            float gv = up ? other : acc[u], uv = up ? acc[u + 1] : other;
+            const int n = e0 + u + (up ? 1 : 0);
+            if (on && n < nvalid) {
+              if (bias) {
+                gv = __fadd_rn(gv, b0);
+                uv = __fadd_rn(uv, b1);
+              }
+              const float wt = A.wts ? A.wts[A.pair_src[T.y + n]] : 1.0f;
+              out[(size_t)n * rows] = pm_act(A.act, A.act_limit, A.act_alpha, gv, uv, wt, A.wts != nullptr);
+            }
+          }
+        }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == MW) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
+}
+
+size_t mx8_rec_bytes(int n_pairs, int max_groups, int cols) {
+  const size_t groups = (size_t)(max_groups < n_pairs ? max_groups : n_pairs);
+  return (((size_t)n_pairs + 15 * groups) / 16 + 1) * ((cols + M8_KS - 1) / M8_KS) * (2048 * 5 + 512);
+}
+void launch_mx8_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x, uint8_t *rec) {
+  const long units = ((long)n_rows + 15 * t.max_tiles) * (cols / 32);
+  const long gx = (units / t.max_tiles + 127) / 128;
+  const dim3 grid((unsigned)(gx < 1 ? 1 : gx), (unsigned)t.max_tiles);
+  if (t.ntok == M8Shape<5>::NTOK) pm_launch(L, k_mx8_rows<5>, grid, 128, 0, t.n, t.tiles, src_row, cols, x, rec);
+  else pm_launch(L, k_mx8_rows<4>, grid, 128, 0, t.n, t.tiles, src_row, cols, x, rec);
+}
+
+template <bool DOWN, int NP> static cudaError_t mx8_start(const Launch &L, const M8Args &A, long items) {
+  using S = M8Shape<NP>;
+  constexpr size_t smem = (size_t)S::NSR * M8_RAW + (size_t)M8_NA * M8_AST + (size_t)M8_NSB * S::BST + M8_NA * 512 + M8_IT * sizeof(M8Item) +
+                          (2 * S::NSR + 2 * M8_NSB + 2 * M8_NA + 2 * S::NACC + 2 * M8_IT) * 8 + 16;
+  static_assert(smem <= 115712, "two CTAs an SM");
+  static bool set[64] = {};  // (one-time per device and kernel)
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !set[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(k_tc_mx8<DOWN, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    if (dev < 64) set[dev] = true;
+  }
+  const long ctas = 2L * L.n_sm;
+  return pm_launch(L, k_tc_mx8<DOWN, NP>, dim3((unsigned)(items < ctas ? items : ctas)), M8_NT, smem, A);
+}
+
+// Tokens of a tile of a call of T tokens whose groups hold n_pairs / n_groups pairs on average; 128: prefill_mx.cu
+int mx_tile_tokens(int T, int n_pairs, int n_groups) {
+  if (T < PM_MX_PROMPT) return M8Shape<5>::NTOK;
+  return n_pairs / (n_groups < n_pairs ? n_groups : n_pairs) <= 48 ? M8Shape<4>::NTOK : 128;
+}
+
+// Cuts of K of the down products: a few tokens make ceil(d / 128) items an expert, each a chain of ff / 128 stages;
+// while that leaves CTAs without work, K is cut in up to four (the combine step adds the parts in order).
+static int mx8_split_stages(int nst, int splits) { return ((nst + splits - 1) / splits + 1) & ~1; }  // whole boxes
+int mx_splits(const pm_layer_desc &D, int n_pairs) {
+  const int nst = (D.ff + M8_KS - 1) / M8_KS;
+  // (a pair is at most a tile of its own; two CTAs on each of 148 SMs)
+  const long items = (long)((D.d + M8_M - 1) / M8_M) * n_pairs;
+  long s = 296 / (items > 0 ? items : 1);
+  s = s > 4 ? 4 : s;
+  s = s > nst / 4 ? nst / 4 : s;  // at least four stages each
+  if (s <= 1) return 1;
+  const int ss = mx8_split_stages(nst, (int)s);
+  return (nst + ss - 1) / ss;  // (rounding up may leave fewer)
+}
+
+// Tensor-core form of launch_gateup / launch_down for MXFP4 weights and f32 activations given as the pieces of
+// the grouping's rows. splits: cuts of K (down only); split s goes to out + s * split_stride.
+cudaError_t launch_tc_mx8(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
+                          const uint8_t *rec, const float *wts, float *out, int splits, size_t split_stride, int *err,
+                          unsigned long long wait_ns) {
+  if (t.max_tiles == 0) return cudaSuccess;
+  const WMat &W0 = down ? ly.down : ly.gate, &W1 = ly.up;
+  M8Args A;
+  A.m0 = (down ? ly.maps->down : ly.maps->gate).m[down ? 1 : 0];  // boxes of 128 or 64 rows
+  A.m1 = ly.maps->up.m[0];
+  A.s0 = W0.plane[1];
+  A.s0_stride = W0.stride[1];
+  A.s1 = W1.plane[1];
+  A.s1_stride = W1.stride[1];
+  A.tiles = t.tiles;
+  A.n_tiles = t.n;
+  A.next = t.next + (down ? 1 : 0);
+  A.rec = rec;
+  A.bias0 = down ? ly.bias_down : ly.bias_gate;
+  A.bias1 = down ? nullptr : ly.bias_up;
+  A.wts = !down && ly.desc.weight_fold == PM_FOLD_BEFORE_DOWN ? wts : nullptr;
+  A.pair_src = pair_src;
+  A.out = out;
+  A.split_stride = split_stride;
+  A.err = err;
+  A.wait_ns = wait_ns;
+  const int rpc = down ? M8_M : M8_M / 2, nst = (W0.cols + M8_KS - 1) / M8_KS;
+  A.row_tiles = (W0.rows + rpc - 1) / rpc;
+  A.split_stages = mx8_split_stages(nst, splits);
+  A.splits = splits;
+  A.cols = W0.cols;
+  A.rows = W0.rows;
+  A.act = ly.desc.act;
+  A.act_limit = ly.desc.act_limit;
+  A.act_alpha = ly.desc.act_alpha;
+  const long items = (long)A.row_tiles * A.splits * t.max_tiles;
+  if (t.ntok == M8Shape<5>::NTOK) return down ? mx8_start<true, 5>(L, A, items) : mx8_start<false, 5>(L, A, items);
+  return down ? mx8_start<true, 4>(L, A, items) : mx8_start<false, 4>(L, A, items);
+}

@@ -849,7 +849,7 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)S::COLS) : "memory");
 }
 
-static int tc_max_tiles(int n_pairs, int max_groups, int ntok = 32) {  // (the default: of every shape)
+static int tc_max_tiles(int n_pairs, int max_groups, int ntok = 16) {  // (the default: of every shape)
   int groups = max_groups < n_pairs ? max_groups : n_pairs;
   return n_pairs / ntok + groups;
 }
@@ -861,14 +861,13 @@ size_t tc_rec_bytes(int n_pairs, int max_groups, int cols) {
   size_t rows = (size_t)n_pairs + 15 * groups + 16;
   return (rows / 8 + 1) * (size_t)(cols / 256) * TC_REC;
 }
-TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, int kind) {
+TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, int ntok) {
   TcTiles t;
   // tiles of up to 64 tokens and the two-CTA shape while the groups hold up to 16 pairs on average (128 experts x 2048 x
   // 768, 32 pairs a group: 102 us in the one-CTA shape, 118 us in this one; 2 pairs: 1,049 -> 733 us of a 7168-wide layer)
   const int avg = n_pairs / (n_groups < n_pairs ? n_groups : n_pairs);
-  t.ntok = avg <= 16 ? (kind == TC_KIND_MX ? mx_small_tokens() : TcShape<2>::NTOK) : TC_NMAX;
-  if (kind == TC_KIND_Q32) t.ntok = q32_tile_tokens();
-  t.even = kind != TC_KIND_Q8X;
+  t.ntok = ntok ? ntok : (avg <= 16 ? TcShape<2>::NTOK : TC_NMAX);
+  t.even = ntok != 0;
   t.shared = shared_tokens > 0;
   t.max_tiles = tc_max_tiles(n_pairs, max_groups, t.ntok) + (shared_tokens + t.ntok - 1) / t.ntok;
   t.n = (int *)buf;

@@ -10,6 +10,14 @@ from tests.helpers import SMALL, bits_equal, make_pair, tol_ok
 pytestmark = [pytest.mark.gpu, pytest.mark.timeout(600)]
 
 
+@pytest.fixture(scope="module")
+def ctx():
+    """A context that nobody has given a threshold: the default choice of kernels."""
+    c = pb.Context(0)
+    yield c
+    c.close()
+
+
 @pytest.mark.parametrize("T", [2, 5, 33, 70, 300])
 @pytest.mark.parametrize("shape", ["c6", "c7", "c8", "c7-shard", "c6-f16"])
 def test_32_value_blocks(ctx, oracle, shape, T):
@@ -24,4 +32,25 @@ def test_32_value_blocks(ctx, oracle, shape, T):
     c1 = ctx.path_counts()
     assert c1["tensor"] - c0["tensor"] == 2 and c1["general"] == c0["general"]
     assert bits_equal(got, ol.forward(x))
+    gl.close()
+
+
+@pytest.mark.parametrize("T", [2, 5, 31, 32, 40, 150])
+@pytest.mark.parametrize("shape", ["c3", "c3-shard", "c3-wide"])
+def test_mxfp4(ctx, oracle, shape, T):
+    """MXFP4 weights and f32 activations: five or four fp8 pieces in tiles of 16 or 32 tokens, two bf16 pieces in tiles
+    of 128. ff = 160: a last stage of one block; the wide shape cuts the down products along K; calls of
+    fewer than 32 tokens keep f32 precision."""
+    cfg = {"c3-shard": SMALL["c3"].scaled(first_local_expert=2, n_exp_local=4),
+           "c3-wide": SMALL["c3"].scaled(d=288, ff=1120)}.get(shape) or SMALL[shape]
+    ol, gl, _ = make_pair(oracle, pb, ctx, cfg, 82)
+    x = synth.make_activations(T, cfg.d, 950 + T)
+    x[0, :32] *= 1e-12  # blocks of very different sizes, and one of zeros
+    x[1, 32:64] = 0.0
+    got = gl.forward(x)
+    want = ol.forward(x)
+    assert tol_ok(got, want), float(np.abs(got - want).max())
+    if T < 32:
+        rms = float(np.sqrt((want.astype(np.float64) ** 2).mean()))
+        assert float(np.abs(got - want).max()) < 4e-6 * rms
     gl.close()
