@@ -364,11 +364,6 @@ __global__ void __launch_bounds__(MxShape::NT, 1) k_tc_mx(const __grid_constant_
 #pragma unroll
         for (int j = 0; j < 4; j++)  // (TMA swizzle: 16-byte piece i of a row sits at i ^ (row & 7))
           q[j] = *(const uint4 *)(raw + (((4 * (j >> 1) + 2 * par + (j & 1)) ^ (m & 7)) << 4));
-#pragma unroll
-        for (int j = 0; j < 4; j++) asm volatile("" : "+r"(q[j].x), "+r"(q[j].y), "+r"(q[j].z), "+r"(q[j].w));
-        __syncwarp();
-        if (lane == 0) tc_mbar_arrive(empty_raw + sr);
-        if (++sr == NSR) { sr = 0; pr ^= 1; }
         auto stored = [&](int a) {  // the stores to operand A's chunk a are done
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -398,6 +393,9 @@ __global__ void __launch_bounds__(MxShape::NT, 1) k_tc_mx(const __grid_constant_
             tc_st32(tlane + S::A0 + a * S::ACH + h * (MX_KC / 2), w);
           }
         }
+        __syncwarp();  // (an arrival is not ordered behind loads whose registers nobody has read yet)
+        if (lane == 0) tc_mbar_arrive(empty_raw + sr);
+        if (++sr == NSR) { sr = 0; pr ^= 1; }
         stored(2 + par);
         st++;
       }

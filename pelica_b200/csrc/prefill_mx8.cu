@@ -23,9 +23,8 @@
 #define M8_RAW (M8_M * 128)   /* packed nibbles of 128 rows x 256 K values: two stages */
 #define M8_AST (M8_M * 128)   /* operand A of a stage: 16 codes = 8 bytes and 8 unused, rows of 128 bytes, swizzled */
 #define M8_NW 8
-#define M8_NT (32 * (M8_NW + 2))
-#define M8_NA 2
-#define M8_NSB 2
+#define M8_NT (32 * (M8_NW + 3))
+#define M8_NA 2     /* places of a stage: operand A, its scales, the tokens' pieces */
 #define M8_IT 4
 #define M8_END 0xfffffffeu
 
@@ -35,7 +34,9 @@ template <int NP> struct M8Shape {
   static constexpr int NSR = NP == 5 ? 3 : 2;
   static constexpr int BST = NP * NTOK * M8_KS + 512;  // the pieces of a stage and their scales
   static constexpr uint32_t SET = NP * 16;             // columns of a set of sums (folded: two sets)
-  static constexpr uint32_t SFA = 240, SFB = 244;      // columns of the scales
+  // columns of the scales, 8 on for the other place of a stage: nothing orders a copy of scales behind the products that
+  // read the ones before it but the commit that frees the place
+  static constexpr uint32_t SFA = 240, SFB = 244;
   static constexpr int NACC = FOLD ? 2 : 1;
 };
 static_assert(2 * M8Shape<5>::SET <= M8Shape<5>::SFA && 4 * 32 <= M8Shape<4>::SFA, "sums and scales share 256 columns");
@@ -151,10 +152,10 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
   constexpr int MW = M8_NW, NSR = S::NSR, NACC = S::NACC;
   constexpr int RPC = DOWN ? M8_M : M8_M / 2;  // matrix rows of an item
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t *sRaw = smem, *sA = sRaw + NSR * M8_RAW, *sB = sA + M8_NA * M8_AST, *sSA = sB + M8_NSB * S::BST;
+  uint8_t *sRaw = smem, *sA = sRaw + NSR * M8_RAW, *sB = sA + M8_NA * M8_AST, *sSA = sB + M8_NA * S::BST;
   M8Item *items = (M8Item *)(sSA + M8_NA * 512);
-  uint64_t *full_raw = (uint64_t *)(items + M8_IT), *empty_raw = full_raw + NSR, *full_b = empty_raw + NSR;
-  uint64_t *empty_b = full_b + M8_NSB, *a_ready = empty_b + M8_NSB, *a_free = a_ready + M8_NA, *acc_full = a_free + M8_NA;
+  uint64_t *full_raw = (uint64_t *)(items + M8_IT), *empty_raw = full_raw + NSR;
+  uint64_t *a_ready = empty_raw + NSR, *a_free = a_ready + M8_NA, *acc_full = a_free + M8_NA;
   uint64_t *acc_free = acc_full + NACC, *it_full = acc_free + NACC, *it_empty = it_full + M8_IT;
   uint32_t *tmem_slot = (uint32_t *)(it_empty + M8_IT);
   const int nbk = A.cols / 32, rows = A.rows, nst = (A.cols + M8_KS - 1) / M8_KS;
@@ -170,12 +171,8 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
       tc_mbar_init(full_raw + i, 1);
       tc_mbar_init(empty_raw + i, MW);
     }
-    for (int i = 0; i < M8_NSB; i++) {
-      tc_mbar_init(full_b + i, 1);
-      tc_mbar_init(empty_b + i, 1);
-    }
     for (int i = 0; i < M8_NA; i++) {
-      tc_mbar_init(a_ready + i, MW);
+      tc_mbar_init(a_ready + i, MW / 2 + 1);  // the workers of the stage; the pieces' copy
       tc_mbar_init(a_free + i, 1);
     }
     for (int i = 0; i < NACC; i++) {
@@ -184,7 +181,7 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
     }
     for (int i = 0; i < M8_IT; i++) {
       tc_mbar_init(it_full + i, 1);
-      tc_mbar_init(it_empty + i, 1 + MW);
+      tc_mbar_init(it_empty + i, 2 + MW);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -206,7 +203,7 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
     // ================= the issuing warp =================
     const uint32_t el = tc_elect() ? 1u : 0u;
     const uint32_t sA_a = tc_s32(sA), sB_a = tc_s32(sB), sSA_a = tc_s32(sSA);
-    uint32_t st = 0, sb = 0, pb = 0, set = 0, ps = 1;
+    uint32_t n_a[2] = {0, 0}, set = 0, ps = 1;
     M8Item it;
     for (int k = 0; next_item(k, it); k++) {
       if ((int)it.t.x < 0) continue;
@@ -215,44 +212,43 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
       // instruction descriptor: A E2M1 (5), B E4M3 (0), both K-major, UE8M0 scales, N, M = 128; bits 4..5 and 29..30: which
       // byte of the scale columns
       const uint32_t idesc = (5u << 7) | ((N >> 3) << 17) | (1u << 23) | (1u << 27);
-      for (int s = s0; s < s1; s++, st++) {
-        const uint32_t a = st & 1;
+      for (int s = s0; s < s1; s++) {
+        const uint32_t a = (uint32_t)(s - s0) & 1;
         const bool first = S::FOLD ? ((s - s0) & 1) == 0 : s == s0;
         const bool last = S::FOLD ? ((s - s0) & 1) == 1 || s == s1 - 1 : s == s1 - 1;
         if (first) tc_wait(acc_free + set, ps, A.err, A.wait_ns);
-        tc_wait(full_b + sb, pb, A.err, A.wait_ns);
-        tc_wait(a_ready + a, (st >> 1) & 1, A.err, A.wait_ns);
+        tc_wait(a_ready + a, (a ? n_a[1] : n_a[0]) & 1, A.err, A.wait_ns);
+        if (a) n_a[1]++;
+        else n_a[0]++;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // operand A: rows of 128 bytes, 128-byte swizzle (layout type 2), groups of 8 rows 1024 bytes apart
         const uint64_t dA = (tc_desc(sA_a + a * M8_AST, 16u, 1024u)) | (2ull << 61);
-        const uint64_t dB = tc_desc(sB_a + sb * S::BST, N * 16u, 128u);
+        const uint64_t dB = tc_desc(sB_a + a * S::BST, N * 16u, 128u);
         const int ksteps = min(4, (A.cols - s * M8_KS) / 32);
         if (el) {
-          m8_cp_scales(tmem + S::SFA, tc_desc(sSA_a + a * 512u, 128u, 128u));
-          m8_cp_scales(tmem + S::SFB, tc_desc(sB_a + sb * S::BST + N * M8_KS, 128u, 128u));
+          m8_cp_scales(tmem + S::SFA + 8u * a, tc_desc(sSA_a + a * 512u, 128u, 128u));
+          m8_cp_scales(tmem + S::SFB + 8u * a, tc_desc(sB_a + a * S::BST + N * M8_KS, 128u, 128u));
 #pragma unroll
           for (uint32_t ks = 0; ks < 4; ks++)
             if ((int)ks < ksteps)
-              m8_mma(tmem + set * S::SET, dA + 2u * ks, dB + (uint64_t)(ks * N * 2u), idesc | (ks << 4) | (ks << 29), tmem + S::SFA,
-                     tmem + S::SFB, !first || ks > 0 ? 1u : 0u);
+              m8_mma(tmem + set * S::SET, dA + 2u * ks, dB + (uint64_t)(ks * N * 2u), idesc | (ks << 4) | (ks << 29), tmem + S::SFA + 8u * a,
+                     tmem + S::SFB + 8u * a, !first || ks > 0 ? 1u : 0u);
           tc_commit(a_free + a);
-          tc_commit(empty_b + sb);
           if (last) tc_commit(acc_full + set);
         }
         __syncwarp();
-        if (++sb == M8_NSB) { sb = 0; pb ^= 1; }
         if (last && ++set == NACC) { set = 0; ps ^= 1; }
       }
     }
   } else if (warp == MW + 1) {
-    // ================= the producer: one thread =================
+    // ================= one thread: work items and the weights' boxes =================
     if (tc_elect()) {
-      const uint32_t sRaw_a = tc_s32(sRaw), sB_a = tc_s32(sB);
+      const uint32_t sRaw_a = tc_s32(sRaw);
       const int per_tile = A.row_tiles * A.splits, n_items = *A.n_tiles * per_tile, G = (int)gridDim.x;
       int cur = (int)blockIdx.x, nxt = cur + G;
       uint4 Tc = make_uint4(M8_END, 0, 0, 0), Tn = Tc;
       if (cur < n_items) Tc = __ldg(A.tiles + cur / per_tile);
-      uint32_t sr = 0, pr = 1, sb = 0, pb = 1, nr = 0, nB = 0;
+      uint32_t sr = 0, pr = 1, nr = 0;
       bool ok = true;
       for (int k = 0; ok; k++) {
         const int s = k & (M8_IT - 1);
@@ -271,29 +267,16 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
         if (end) break;
         const int fut = 2 * G + (int)atomicAdd(A.next, 1u);  // (needed an item later)
         if (nxt < n_items) Tn = __ldg(A.tiles + nxt / per_tile);
-        if ((int)Tc.x >= 0) {
-          const int el = (int)Tc.x;
-          const uint32_t bytes = ((Tc.z + 15) >> 4) * (16u * M8_KS * NP) + 512u;
-          const uint8_t *rec = A.rec + (size_t)(Tc.w >> 4) * nst * (2048 * NP + 512);
-          for (int q = s0; q < s1; q++) {
-            if (((q - s0) & 1) == 0) {  // nibbles of two stages (a box past the matrix reads zeros; split_stages is even)
-              const uint32_t r = sRaw_a + sr * M8_RAW;
-              if (nr >= NSR && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
-              tc_mbar_expect(full_raw + sr, (uint32_t)M8_RAW);
-              tc_tma3(r, &A.m0, q * 64, r0, el, full_raw + sr);  // boxes of 128 rows (down) or 64
-              if (!DOWN) tc_tma3(r + M8_RAW / 2, &A.m1, q * 64, r0, el, full_raw + sr);
-              nr++;
-              if (++sr == NSR) { sr = 0; pr ^= 1; }
-            }
-            if (nB >= M8_NSB && !tc_wait(empty_b + sb, pb, A.err, A.wait_ns)) { ok = false; break; }
-            tc_mbar_expect(full_b + sb, bytes);
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sB_a + sb * S::BST),
-                         "l"(rec + (size_t)q * bytes), "r"(bytes), "r"(tc_s32(full_b + sb))
-                         : "memory");
-            nB++;
-            if (++sb == M8_NSB) { sb = 0; pb ^= 1; }
+        if ((int)Tc.x >= 0)
+          for (int q = s0; q < s1; q += 2) {  // nibbles of two stages (a box past the matrix reads zeros; split_stages is even)
+            const uint32_t r = sRaw_a + sr * M8_RAW;
+            if (nr >= NSR && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
+            tc_mbar_expect(full_raw + sr, (uint32_t)M8_RAW);
+            tc_tma3(r, &A.m0, q * 64, r0, (int)Tc.x, full_raw + sr);  // boxes of 128 rows (down) or 64
+            if (!DOWN) tc_tma3(r + M8_RAW / 2, &A.m1, q * 64, r0, (int)Tc.x, full_raw + sr);
+            nr++;
+            if (++sr == NSR) { sr = 0; pr ^= 1; }
           }
-        }
         cur = nxt;
         nxt = fut;
         Tc = Tn;
@@ -305,18 +288,47 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
         while (!tc_bar_test(full_raw + q % NSR, (q / NSR) & 1) && tc_now() - t0 < A.wait_ns) {
         }
       }
-      for (uint32_t i = 1; i <= M8_NSB && i <= nB; i++) {
-        const uint32_t q = nB - i;
-        const unsigned long long t0 = tc_now();
-        while (!tc_bar_test(full_b + q % M8_NSB, (q / M8_NSB) & 1) && tc_now() - t0 < A.wait_ns) {
+    }
+    __syncwarp();
+  } else if (warp == MW + 2) {
+    // ================= the tokens' pieces (a warp of its own: in one loop with the boxes, whose ring is deeper, the
+    // boxes waited for the pieces' places) =================
+    const uint32_t sB_a = tc_s32(sB);
+    uint32_t n_a[2] = {0, 0};
+    bool ok = true;
+    M8Item it;
+    for (int k = 0; ok && next_item(k, it); k++) {
+      if ((int)it.t.x < 0) continue;
+      const uint32_t bytes = ((it.t.z + 15) >> 4) * (16u * M8_KS * NP) + 512u;
+      const uint8_t *rec = A.rec + (size_t)(it.t.w >> 4) * nst * (2048 * NP + 512);
+      for (int q = it.s0; q < it.s1; q++) {
+        const uint32_t a = (uint32_t)(q - it.s0) & 1;
+        ok = __all_sync(PM_FULL, tc_wait(a_free + a, ((a ? n_a[1] : n_a[0]) & 1) ^ 1, A.err, A.wait_ns));
+        if (!ok) break;
+        if (a) n_a[1]++;
+        else n_a[0]++;
+        if (lane == 0) {
+          tc_mbar_expect(a_ready + a, bytes);
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sB_a + a * S::BST),
+                       "l"(rec + (size_t)q * bytes), "r"(bytes), "r"(tc_s32(a_ready + a))
+                       : "memory");
         }
+        __syncwarp();
       }
     }
+    if (lane == 0)  // (as above)
+      for (int a = 0; a < 2; a++) {
+        const uint32_t n = a ? n_a[1] : n_a[0];
+        const unsigned long long t0 = tc_now();
+        while (n > 0 && !tc_bar_test(a_ready + a, (n - 1) & 1) && tc_now() - t0 < A.wait_ns) {
+        }
+      }
     __syncwarp();
   } else {
     // ================= the workers =================
-    // operand A: thread = (row m, half `part` of a stage's K values); sums: lane m, half `part` of the tokens. Row m of the
-    // tile: row m / 2 of gate (m even) or of up (odd); down: row m.
+    // operand A: thread = row m of the even stages (part 0) or the odd ones: a stage's chain of wait, copy and fence has
+    // the time of two; sums: lane m, half `part` of the tokens. Row m of the tile: row m / 2 of gate (m even) or
+    // of up (odd); down: row m.
     const int m = tid & 127;
     const int part = (int)__reduce_max_sync(PM_FULL, (unsigned)warp >> 2);
     const bool up = !DOWN && (m & 1);
@@ -373,47 +385,37 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
         if (lane == 0) tc_mbar_arrive(acc_free + set);
         if (++set == NACC) { set = 0; pf ^= 1; }
       };
-      unsigned long long sc_n = part == 0 ? scales(it.s0) : 0;
+      unsigned long long sc_n = scales(it.s0);
+      uint8_t *dst = sA + part * M8_AST + m * 128;
 #pragma unroll 1
       for (int s2 = it.s0; s2 < it.s1; s2 += 2) {
         const unsigned long long sc = sc_n;
-        if (part == 0 && s2 + 2 < it.s1) sc_n = scales(s2 + 2);
+        if (s2 + 2 < it.s1) sc_n = scales(s2 + 2);
         tc_wait(full_raw + sr, pr, A.err, A.wait_ns);
         const uint8_t *raw = sRaw + sr * M8_RAW + rawr * 128;
+        uint4 q[4];
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-          const bool on = s2 + j < it.s1;
-          uint4 q[2];
-          if (on)
+        for (int i = 0; i < 4; i++)  // (TMA swizzle: 16-byte piece i of a row sits at i ^ (row & 7))
+          q[i] = *(const uint4 *)(raw + (((4 * part + i) ^ (rawr & 7)) << 4));
+        if (s2 + part < it.s1) {
+          tc_wait(a_free + part, (st & 1) ^ 1, A.err, A.wait_ns);
+          st++;
 #pragma unroll
-            for (int i = 0; i < 2; i++)  // (TMA swizzle: 16-byte piece i of a row sits at i ^ (row & 7))
-              q[i] = *(const uint4 *)(raw + (((4 * j + 2 * part + i) ^ (rawr & 7)) << 4));
-          if (j == 1) {
-#pragma unroll
-            for (int i = 0; i < 2; i++) asm volatile("" : "+r"(q[i].x), "+r"(q[i].y), "+r"(q[i].z), "+r"(q[i].w));
-            __syncwarp();
-            if (lane == 0) tc_mbar_arrive(empty_raw + sr);
-            if (++sr == NSR) { sr = 0; pr ^= 1; }
+          for (int i = 0; i < 4; i++) {  // 32 codes: two groups of 16, the lower half of 16 bytes each
+            *(uint2 *)(dst + (((2 * i) ^ (m & 7)) << 4)) = make_uint2(q[i].x, q[i].y);
+            *(uint2 *)(dst + (((2 * i + 1) ^ (m & 7)) << 4)) = make_uint2(q[i].z, q[i].w);
           }
-          if (on) {
-            const uint32_t a = st & 1;
-            if (st >= M8_NA) tc_wait(a_free + a, ((st >> 1) - 1) & 1, A.err, A.wait_ns);
-            uint8_t *dst = sA + a * M8_AST + m * 128;
-#pragma unroll
-            for (int i = 0; i < 2; i++) {  // 32 codes: two groups of 16, the lower half of 16 bytes each
-              *(uint2 *)(dst + (((4 * part + 2 * i) ^ (m & 7)) << 4)) = make_uint2(q[i].x, q[i].y);
-              *(uint2 *)(dst + (((4 * part + 2 * i + 1) ^ (m & 7)) << 4)) = make_uint2(q[i].z, q[i].w);
-            }
-            if (part == 0) {  // (255, which the format reserves, counts as 254)
-              const uint32_t e4 = (uint32_t)(sc >> (32 * j));
-              *(uint32_t *)(sSA + a * 512 + (m & 31) * 16 + (m >> 5) * 4) = __vminu4(e4, 0xfefefefeu);
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) tc_mbar_arrive(a_ready + a);
-            st++;
-          }
+          // (255, which the format reserves, counts as 254)
+          *(uint32_t *)(sSA + part * 512 + (m & 31) * 16 + (m >> 5) * 4) = __vminu4((uint32_t)(sc >> (32 * part)), 0xfefefefeu);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) tc_mbar_arrive(a_ready + part);
         }
+        // (given back only now that every word of it has been stored: an arrival is not ordered behind loads whose
+        // registers nobody has read yet, and the next box then lands under them)
+        __syncwarp();
+        if (lane == 0) tc_mbar_arrive(empty_raw + sr);
+        if (++sr == NSR) { sr = 0; pr ^= 1; }
         if (S::FOLD && s2 > it.s0) fold();  // (of the 256 K values before: these are still being multiplied)
       }
       fold();
@@ -465,8 +467,8 @@ void launch_mx8_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32
 
 template <bool DOWN, int NP> static cudaError_t mx8_start(const Launch &L, const M8Args &A, long items) {
   using S = M8Shape<NP>;
-  constexpr size_t smem = (size_t)S::NSR * M8_RAW + (size_t)M8_NA * M8_AST + (size_t)M8_NSB * S::BST + M8_NA * 512 + M8_IT * sizeof(M8Item) +
-                          (2 * S::NSR + 2 * M8_NSB + 2 * M8_NA + 2 * S::NACC + 2 * M8_IT) * 8 + 16;
+  constexpr size_t smem = (size_t)S::NSR * M8_RAW + (size_t)M8_NA * M8_AST + (size_t)M8_NA * S::BST + M8_NA * 512 + M8_IT * sizeof(M8Item) +
+                          (2 * S::NSR + 2 * M8_NA + 2 * S::NACC + 2 * M8_IT) * 8 + 16;
   static_assert(smem <= 115712, "two CTAs an SM");
   static bool set[64] = {};  // (one-time per device and kernel)
   int dev = 0;
@@ -481,9 +483,11 @@ template <bool DOWN, int NP> static cudaError_t mx8_start(const Launch &L, const
 }
 
 // Tokens of a tile of a call of T tokens whose groups hold n_pairs / n_groups pairs on average; 128: prefill_mx.cu
+// (32 experts, d = ff = 2880, gate/up + down: 19 pairs a group 169 us here, 240 there; 37 pairs, two tiles a group here,
+// 275 : 251).
 int mx_tile_tokens(int T, int n_pairs, int n_groups) {
   if (T < PM_MX_PROMPT) return M8Shape<5>::NTOK;
-  return n_pairs / (n_groups < n_pairs ? n_groups : n_pairs) <= 48 ? M8Shape<4>::NTOK : 128;
+  return n_pairs / (n_groups < n_pairs ? n_groups : n_pairs) <= 24 ? M8Shape<4>::NTOK : 128;
 }
 
 // Cuts of K of the down products: a few tokens make ceil(d / 128) items an expert, each a chain of ff / 128 stages;

@@ -397,17 +397,15 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
             w[4 * j] = q.x; w[4 * j + 1] = q.y; w[4 * j + 2] = q.z; w[4 * j + 3] = q.w;
           }
         }
-#pragma unroll
-        for (int i = 0; i < 16; i++) asm volatile("" : "+r"(w[i]));
-        __syncwarp();
-        if (lane == 0) tc_mbar_arrive(empty_raw + sr);
-        if (++sr == Q32_NSR) { sr = 0; pr ^= 1; }
         const uint32_t a = st & 1;
         if (st >= 2) {
           tc_wait(a_free + a, ((st >> 1) - 1) & 1, A.err, A.wait_ns);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
         tc_st16(tlane + a * 32u + 16u * part, w);
+        __syncwarp();  // (an arrival is not ordered behind loads whose registers nobody has read yet)
+        if (lane == 0) tc_mbar_arrive(empty_raw + sr);
+        if (++sr == Q32_NSR) { sr = 0; pr ^= 1; }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();

@@ -745,11 +745,6 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
             // (computed before the wait: left alone the compiler moves the arithmetic behind it)
 #pragma unroll
             for (int j = 0; j < 16; j++) asm volatile("" : "+r"(ah[j]), "+r"(al[j]));
-            if (i == QN - 1) {
-              __syncwarp();
-              if (lane == 0) tc_mbar_arrive(empty_raw + sr);  // the whole warp has read the area
-              if (++sr == NS) { sr = 0; pr ^= 1; }
-            }
             TC_STAMP_W(b, 0)
             if (gb > 0) {
               tc_wait(a_free + q, (gb - 1) & 1, A.err, A.wait_ns);
@@ -758,6 +753,11 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
             TC_STAMP_W(b, 1)
             tc_st16(tlane + S::A_HI + 16u * q, ah);
             tc_st16(tlane + S::A_LO + 16u * q, al);
+            if (i == QN - 1) {  // the whole warp has read the area (its words are stored: an arrival is not ordered
+              __syncwarp();     // behind loads whose registers nobody has read yet)
+              if (lane == 0) tc_mbar_arrive(empty_raw + sr);
+              if (++sr == NS) { sr = 0; pr ^= 1; }
+            }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             if (!Q6) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the mins
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
