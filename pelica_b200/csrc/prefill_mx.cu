@@ -345,19 +345,13 @@ __global__ void __launch_bounds__(MxShape::NT, 1) k_tc_mx(const __grid_constant_
       }
       const bool up = !DOWN && h == 1;  // the up matrix is half 1
       const int drow = DOWN ? r0 + h * MX_M + m : r0 + m;
-      // its scale bytes, eight blocks (four chunks) at a time: two aligned words hold them wherever the row starts
+      // its scale bytes, eight blocks (four chunks) at a time
       const uint8_t *sp = (up ? A.s1 + (size_t)el * A.s1_stride : A.s0 + (size_t)el * A.s0_stride) + (size_t)min(drow, rows - 1) * nbk;
-      auto scales = [&](int c) -> unsigned long long {
-        const uintptr_t p = (uintptr_t)(sp + 2 * c);
-        const unsigned long long *q = (const unsigned long long *)(p & ~(uintptr_t)7);
-        const int sh = 8 * (int)(p & 7);
-        const unsigned long long a = __ldg(q), b = __ldg(q + 1);
-        return sh ? (a >> sh) | (b << (64 - sh)) : a;
-      };
-      unsigned long long sc_n = scales(0);
+      TcBytes8 sc_n;
+      sc_n.load(sp);
       for (int c4 = 0; c4 < nch; c4 += 4) {
-        const unsigned long long sc = sc_n;
-        if (c4 + 4 < nch) sc_n = scales(c4 + 4);
+        const unsigned long long sc = sc_n.get();
+        if (c4 + 4 < nch) sc_n.load(sp + 2 * (c4 + 4));
         tc_wait(full_raw + sr, pr, A.err, A.wait_ns);
         const uint8_t *raw = sRaw + sr * S::RAWB + h * MX_BOX + m * 128;
         uint4 q[4];

@@ -349,15 +349,8 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
           }
         continue;
       }
-      // the row's scale bytes, eight blocks (two stages) at a time: two aligned words hold them wherever the row starts
+      // the row's scale bytes, eight blocks (two stages) at a time
       const uint8_t *sp = (up ? A.s1 + (size_t)el * A.s1_stride : A.s0 + (size_t)el * A.s0_stride) + (size_t)min(row, rows - 1) * nbk;
-      auto scales = [&](int s) -> unsigned long long {
-        const uintptr_t p = (uintptr_t)(sp + 4 * s);
-        const unsigned long long *q = (const unsigned long long *)(p & ~(uintptr_t)7);
-        const int sh = 8 * (int)(p & 7);
-        const unsigned long long a = __ldg(q), b = __ldg(q + 1);
-        return sh ? (a >> sh) | (b << (64 - sh)) : a;
-      };
       float acc[16];
 #pragma unroll
       for (int u = 0; u < 16; u++) acc[u] = 0.0f;
@@ -385,12 +378,13 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
         if (lane == 0) tc_mbar_arrive(acc_free + set);
         if (++set == NACC) { set = 0; pf ^= 1; }
       };
-      unsigned long long sc_n = scales(it.s0);
+      TcBytes8 sc_n;
+      sc_n.load(sp + 4 * it.s0);
       uint8_t *dst = sA + part * M8_AST + m * 128;
 #pragma unroll 1
       for (int s2 = it.s0; s2 < it.s1; s2 += 2) {
-        const unsigned long long sc = sc_n;
-        if (s2 + 2 < it.s1) sc_n = scales(s2 + 2);
+        const unsigned long long sc = sc_n.get();
+        if (s2 + 2 < it.s1) sc_n.load(sp + 4 * (s2 + 2));
         tc_wait(full_raw + sr, pr, A.err, A.wait_ns);
         const uint8_t *raw = sRaw + sr * M8_RAW + rawr * 128;
         uint4 q[4];
@@ -487,7 +481,7 @@ template <bool DOWN, int NP> static cudaError_t mx8_start(const Launch &L, const
 // 275 : 251).
 int mx_tile_tokens(int T, int n_pairs, int n_groups) {
   if (T < PM_MX_PROMPT) return M8Shape<5>::NTOK;
-  return n_pairs / (n_groups < n_pairs ? n_groups : n_pairs) <= 24 ? M8Shape<4>::NTOK : 128;
+  return n_pairs / (n_groups < n_pairs ? n_groups : n_pairs) <= 28 ? M8Shape<4>::NTOK : 128;
 }
 
 // Cuts of K of the down products: a few tokens make ceil(d / 128) items an expert, each a chain of ff / 128 stages;

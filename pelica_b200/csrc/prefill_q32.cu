@@ -293,17 +293,14 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
           }
         continue;
       }
-      // the scales of a stage: four f16 (two aligned words hold them wherever the row starts), or the 8-byte header of
+      // the scales of a stage: four f16, or the 8-byte header of
       // the stage's 256-value block
       const uint8_t *sp = (up ? A.s1 + (size_t)el * A.s1_stride : A.s0 + (size_t)el * A.s0_stride) +
                           (size_t)min(row, rows - 1) * (XS ? nb : 2 * nb);
-      auto scales = [&](int s) -> unsigned long long {
-        if (XS) return __ldg((const unsigned long long *)(sp + (s >> 1) * 8));
-        const uintptr_t p = (uintptr_t)(sp + 8 * s);
-        const unsigned long long *q = (const unsigned long long *)(p & ~(uintptr_t)7);
-        const int sh = 8 * (int)(p & 7);
-        const unsigned long long a = __ldg(q), b = sh ? __ldg(q + 1) : 0;
-        return sh ? (a >> sh) | (b << (64 - sh)) : a;
+      TcBytes8 sc_n;
+      auto load_scales = [&](int s) {
+        if (XS) sc_n.a = __ldg((const unsigned long long *)(sp + (s >> 1) * 8));
+        else sc_n.load(sp + 8 * s);
       };
       uint64_t acc[Q32_N / 4];
 #pragma unroll
@@ -370,11 +367,12 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
         if (lane == 0) tc_mbar_arrive(empty_b + sb);
         if (++sb == Q32_NSB) sb = 0;
       };
-      unsigned long long sc_n = scales(0), sc = 0;
+      unsigned long long sc = 0;
+      load_scales(0);
       for (int s = 0; s < nst; s++, st++) {
         const unsigned long long sc_p = sc;
-        sc = sc_n;
-        if (s + 1 < nst) sc_n = scales(s + 1);
+        sc = XS ? sc_n.a : sc_n.get();
+        if (s + 1 < nst) load_scales(s + 1);
         tc_wait(full_raw + sr, pr, A.err, A.wait_ns);
         const uint8_t *raw = sRaw + sr * RAWB + m * RROW;
         uint32_t w[16];

@@ -156,6 +156,19 @@ __device__ __forceinline__ uint64_t tc_fma2(uint64_t a, uint64_t b, uint64_t c) 
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
+// eight bytes at any address as the two aligned words that hold them, put together only where they are used: shifted
+// right behind the loads they made the warp wait for memory there (650 of an iteration's 1,900 cycles)
+struct TcBytes8 {
+  unsigned long long a, b;
+  int sh;
+  __device__ __forceinline__ void load(const uint8_t *p) {
+    const unsigned long long *q = (const unsigned long long *)((uintptr_t)p & ~(uintptr_t)7);
+    sh = 8 * (int)((uintptr_t)p & 7);
+    a = __ldg(q);
+    b = __ldg(q + 1);
+  }
+  __device__ __forceinline__ unsigned long long get() const { return sh ? (a >> sh) | (b << (64 - sh)) : a; }
+};
 __device__ __forceinline__ void tc_tma3(uint32_t dst, const CUtensorMap *m, int x, int y, int z, uint64_t *bar) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
