@@ -526,13 +526,11 @@ __global__ void __launch_bounds__(128) k_route(pm_layer_desc D, const float *__r
                                                const float *__restrict__ sel_bias, int T,
                                                uint32_t *ids, float *wout) {
   pm_pdl();
-  __shared__ float sm_sv[4][PM_MAX_EXPERTS];
-  __shared__ float sm_gs[4][PM_MAX_EXPERTS / 2];
-  __shared__ unsigned char sm_keep[4][PM_MAX_EXPERTS / 2];
+  __shared__ float sm[4][2 * PM_MAX_EXPERTS + PM_MAX_EXPERTS / 2 + PM_MAX_EXPERTS / 8 + PM_MAX_TOPK];  // pm_route_scratch
   int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   int t = blockIdx.x * 4 + wi;
   if (t >= T) return;
-  pm_route_warp(D, logits + (size_t)t * D.n_exp, sel_bias, lane, sm_sv[wi], sm_gs[wi], sm_keep[wi],
+  pm_route_warp(D, logits + (size_t)t * D.n_exp, sel_bias, lane, sm[wi],
                 ids + (size_t)t * D.top_k, wout + (size_t)t * D.top_k);
 }
 
@@ -653,30 +651,10 @@ void launch_plan(const Launch &L, const LayerDev &ly, const uint32_t *ids, int T
 // [segments][E] counts into first positions (and writes the tile list of the tensor-core products);
 // k_plan_seg_place ranks the pairs of a segment. Three launches whose work grows with the pairs, where
 // k_plan_* takes four and has every expert's CTA walk all pairs (4096 tokens x 8 on 256 experts: 72 us).
+// One segment: its CTA does all three (the plan of 8 to 32 tokens).
 // ---------------------------------------------------------------------------
 #define PL_SEG 32 /* tokens of a segment = warps of its CTA */
-__global__ void __launch_bounds__(1024) k_route_seg(pm_layer_desc D, const float *__restrict__ logits,
-                                                   const float *__restrict__ sel_bias, int T, uint32_t *ids, float *wout,
-                                                   uint32_t *seg_cnt) {
-  pm_pdl();
-  extern __shared__ float rsm[];  // [32] x (E scores, E / 2 group scores, E / 2 bytes), then E counts
-  const int E = D.n_exp, K = D.top_k, lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-  const int per = E + E / 2 + (E / 2 + 3) / 4;
-  uint32_t *cnt = (uint32_t *)(rsm + PL_SEG * per);
-  for (int e = threadIdx.x; e < E; e += 1024) cnt[e] = 0;
-  __syncthreads();
-  const int t = blockIdx.x * PL_SEG + wi;
-  if (t < T) {
-    float *sv = rsm + wi * per;
-    pm_route_warp(D, logits + (size_t)t * E, sel_bias, lane, sv, sv + E, (unsigned char *)(sv + E + E / 2), ids + (size_t)t * K,
-                  wout + (size_t)t * K);
-    __syncwarp();
-    if (lane < K) atomicAdd(&cnt[ids[(size_t)t * K + lane]], 1u);  // (written by this warp above)
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < E; e += 1024) seg_cnt[(size_t)blockIdx.x * E + e] = cnt[e];
-}
-// exclusive scans over 512 values of one CTA of 512 threads: (a, b) -> sums of the earlier threads' values and the totals
+// exclusive scans over 512 values of a CTA's first 512 threads: (a, b) -> sums of the earlier threads' values and the totals
 __device__ __forceinline__ void pm_scan2_512(uint32_t a, uint32_t b, uint32_t &ea, uint32_t &eb, uint32_t &ta, uint32_t &tb,
                                              uint32_t (*sh)[16]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -686,7 +664,7 @@ __device__ __forceinline__ void pm_scan2_512(uint32_t a, uint32_t b, uint32_t &e
     const uint32_t u = __shfl_up_sync(PM_FULL, x, o), v = __shfl_up_sync(PM_FULL, y, o);
     if (lane >= o) { x += u; y += v; }
   }
-  if (lane == 31) { sh[0][warp] = x; sh[1][warp] = y; }
+  if (lane == 31 && warp < 16) { sh[0][warp] = x; sh[1][warp] = y; }
   __syncthreads();
   ea = x - a;
   eb = y - b;
@@ -699,18 +677,10 @@ __device__ __forceinline__ void pm_scan2_512(uint32_t a, uint32_t b, uint32_t &e
   }
   __syncthreads();
 }
-// one CTA: counts of the segments -> the plan's active / offset / count / base, seg_cnt[s][e] -> first position of
-// segment s's pairs of expert e; and the tile list (k_tc_tiles' rules) when tt.tiles is given
-__global__ void __launch_bounds__(512) k_plan_seg_scan(PlanDev pl, int E, int T, int n_seg, uint32_t *seg_cnt, uint32_t *usage, TcTiles tt,
-                                                       int first_local, int n_local) {
-  pm_pdl();
-  __shared__ uint32_t sh[2][16];
-  const int e = threadIdx.x;
-  uint32_t c = 0;
-  if (e < E) {
-#pragma unroll 16
-    for (int s = 0; s < n_seg; s++) c += seg_cnt[(size_t)s * E + e];
-  }
+// The plan's active / offset / count / base from the pairs c of expert e (thread e of a CTA), and the tile list
+// (k_tc_tiles' rules) when tt.tiles is given; returns the first position of e's pairs.
+__device__ __forceinline__ uint32_t pm_plan_scan(PlanDev pl, int e, uint32_t c, int E, int T, uint32_t *usage, const TcTiles &tt, int first_local,
+                                                 int n_local, uint32_t (*sh)[16]) {
   uint32_t o, na, total, active;
   pm_scan2_512(c, c > 0, o, na, total, active, sh);
   if (e < E) {
@@ -726,13 +696,6 @@ __global__ void __launch_bounds__(512) k_plan_seg_scan(PlanDev pl, int E, int T,
       pl.active[e] = 0;
       pl.offset[e] = 0;
       pl.count[e] = 0;
-    }
-    uint32_t run = o;
-#pragma unroll 16
-    for (int s = 0; s < n_seg; s++) {
-      const uint32_t v = seg_cnt[(size_t)s * E + e];
-      seg_cnt[(size_t)s * E + e] = run;
-      run += v;
     }
   }
   if (e == 0) *pl.n_active = (int)active + (tt.shared ? 1 : 0);
@@ -763,6 +726,74 @@ __global__ void __launch_bounds__(512) k_plan_seg_scan(PlanDev pl, int E, int T,
       tt.next[0] = tt.next[1] = 0;
     }
   }
+  return o;
+}
+// pair i of a segment (e: its expert, s_id: the segment's): its place behind the segment's earlier pairs of e
+__device__ __forceinline__ void pm_plan_place(PlanDev pl, const uint32_t *s_id, int i, int g, int K, uint32_t e, uint32_t first) {
+  uint32_t rank = 0;
+  for (int j = 0; j < (i & ~3); j += 4) {
+    const uint4 v = *(const uint4 *)(s_id + j);
+    rank += (v.x == e) + (v.y == e) + (v.z == e) + (v.w == e);
+  }
+  for (int j = i & ~3; j < i; j++) rank += s_id[j] == e;
+  const uint32_t p = first + rank;
+  pl.pair_pos[g] = p;
+  pl.pair_token[p] = (uint32_t)(g / K);
+  pl.pair_src[p] = (uint32_t)g;
+}
+__global__ void __launch_bounds__(1024) k_route_seg(pm_layer_desc D, const float *__restrict__ logits,
+                                                   const float *__restrict__ sel_bias, int T, uint32_t *ids, float *wout,
+                                                   uint32_t *seg_cnt, PlanDev pl, uint32_t *usage, TcTiles tt, int first_local, int n_local) {
+  pm_pdl();
+  extern __shared__ __align__(16) float rsm[];  // 512 experts of pairs, E counts, [32] x scratch
+  __shared__ uint32_t sh[2][16];
+  const int E = D.n_exp, K = D.top_k, lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  uint32_t *s_id = (uint32_t *)rsm, *cnt = s_id + 512;
+  float *sc = rsm + 512 + E + wi * pm_route_scratch(E);
+  for (int e = threadIdx.x; e < E; e += 1024) cnt[e] = 0;
+  __syncthreads();
+  const int t = blockIdx.x * PL_SEG + wi;
+  if (t < T) {
+    pm_route_warp(D, logits + (size_t)t * E, sel_bias, lane, sc, ids + (size_t)t * K, wout + (size_t)t * K);
+    __syncwarp();
+    if (lane < K) {
+      const uint32_t e = ids[(size_t)t * K + lane];  // (written by this warp above)
+      atomicAdd(&cnt[e], 1u);
+      s_id[wi * K + lane] = e;
+    }
+  }
+  __syncthreads();
+  if (gridDim.x > 1) {
+    for (int e = threadIdx.x; e < E; e += 1024) seg_cnt[(size_t)blockIdx.x * E + e] = cnt[e];
+    return;
+  }
+  const int i = threadIdx.x;
+  const uint32_t o = pm_plan_scan(pl, i, i < E ? cnt[i] : 0u, E, T, usage, tt, first_local, n_local, sh);
+  __syncthreads();
+  if (i < E) cnt[i] = o;
+  __syncthreads();
+  if (i < T * K) pm_plan_place(pl, s_id, i, i, K, s_id[i], cnt[s_id[i]]);
+}
+// one CTA: counts of the segments -> the plan, seg_cnt[s][e] -> first position of segment s's pairs of expert e
+__global__ void __launch_bounds__(512) k_plan_seg_scan(PlanDev pl, int E, int T, int n_seg, uint32_t *seg_cnt, uint32_t *usage, TcTiles tt,
+                                                       int first_local, int n_local) {
+  pm_pdl();
+  __shared__ uint32_t sh[2][16];
+  const int e = threadIdx.x;
+  uint32_t c = 0;
+  if (e < E) {
+#pragma unroll 16
+    for (int s = 0; s < n_seg; s++) c += seg_cnt[(size_t)s * E + e];
+  }
+  uint32_t run = pm_plan_scan(pl, e, c, E, T, usage, tt, first_local, n_local, sh);
+  if (e < E) {
+#pragma unroll 16
+    for (int s = 0; s < n_seg; s++) {
+      const uint32_t v = seg_cnt[(size_t)s * E + e];
+      seg_cnt[(size_t)s * E + e] = run;
+      run += v;
+    }
+  }
 }
 // a CTA a segment: thread i = pair i of it; its rank among the segment's earlier pairs of the same expert
 __global__ void __launch_bounds__(512) k_plan_seg_place(const uint32_t *__restrict__ ids, int P, int K,
@@ -774,30 +805,21 @@ __global__ void __launch_bounds__(512) k_plan_seg_place(const uint32_t *__restri
   const uint32_t e = on ? ids[g] : 0xffffffffu;
   s_id[i] = e;
   __syncthreads();
-  if (!on) return;
-  uint32_t rank = 0;
-  for (int j = 0; j < (i & ~3); j += 4) {
-    const uint4 v = *(const uint4 *)(s_id + j);
-    rank += (v.x == e) + (v.y == e) + (v.z == e) + (v.w == e);
-  }
-  for (int j = i & ~3; j < i; j++) rank += s_id[j] == e;
-  const uint32_t p = seg_pos[(size_t)blockIdx.x * E + e] + rank;
-  pl.pair_pos[g] = p;
-  pl.pair_token[p] = (uint32_t)(g / K);
-  pl.pair_src[p] = (uint32_t)g;
+  if (on) pm_plan_place(pl, s_id, i, g, K, e, seg_pos[(size_t)blockIdx.x * E + e]);
 }
 
 size_t route_seg_words(int T, int E) { return (size_t)((T + PL_SEG - 1) / PL_SEG) * E; }
 void launch_route_plan(const Launch &L, const LayerDev &ly, const float *logits, int T, uint32_t *ids, float *w, PlanDev pl,
                        uint32_t *seg, const TcTiles &tt) {
   const int E = ly.desc.n_exp, K = ly.desc.top_k, nseg = (T + PL_SEG - 1) / PL_SEG;
-  const int smem = (PL_SEG * (E + E / 2 + (E / 2 + 3) / 4) + E) * 4;
+  const int smem = (512 + E + PL_SEG * pm_route_scratch(E)) * 4;
   static int smem_set = 48 * 1024;
   if (smem > smem_set) {
     cudaFuncSetAttribute(k_route_seg, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     smem_set = smem;
   }
-  PLAUNCH(L, k_route_seg, nseg, 1024, smem, ly.desc, logits, ly.select_bias, T, ids, w, seg);
+  PLAUNCH(L, k_route_seg, nseg, 1024, smem, ly.desc, logits, ly.select_bias, T, ids, w, seg, pl, ly.usage, tt, ly.first_local, ly.n_local);
+  if (nseg == 1) return;
   PLAUNCH(L, k_plan_seg_scan, 1, 512, 0, pl, E, T, nseg, seg, ly.usage, tt, ly.first_local, ly.n_local);
   PLAUNCH(L, k_plan_seg_place, nseg, 512, 0, ids, T * K, K, seg, E, pl);
 }
@@ -805,7 +827,9 @@ void launch_route_plan(const Launch &L, const LayerDev &ly, const float *logits,
 // Router logits, top-k and the dispatch plan of a few tokens (T < 8) in ONE launch: a CTA brings EPC experts' rows
 // and the tokens into shared memory by two bulk copies (a row is 8 to 28 KB: loads from registers kept 3 KB an SM
 // in flight, one token on 256 experts x 7168 46 us), a warp a (expert, token); the CTA that finishes last (a ticket
-// counter; nobody waits for anybody) routes every token, one warp each, and builds the plan and the tile list.
+// counter; nobody waits for anybody) routes every token (scores by all threads, picks by a warp each) and builds the
+// plan and the tile list. That part runs once, cold: rolled loops, and the plan from comparisons of the few pairs with
+// each other in place of scans (one token on 256 experts in 8 groups: 20,300 cycles of it before).
 // The values are those of k_router, k_route and k_plan_*.
 #define RS_TOK 8   /* tokens (= warps of the last CTA) */
 __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const float *__restrict__ wr,
@@ -867,8 +891,16 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
       const int el = i % ne, t = i / ne;
       const float *w = xs + (size_t)el * d + lane, *xr = xs + (size_t)(epc + t) * d + lane;
       float acc = 0.0f;
-#pragma unroll 8
-      for (int c = 0; c < d; c += 32) acc = __fmaf_rn(w[c], xr[c], acc);
+#pragma unroll 1
+      for (int c = 0; c < (d & ~511); c += 512) {  // 16 columns a lane read at once: one latency for 16 steps of the chain
+        float a[16], b[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) { a[i] = w[c + 32 * i]; b[i] = xr[c + 32 * i]; }
+#pragma unroll
+        for (int i = 0; i < 16; i++) acc = __fmaf_rn(a[i], b[i], acc);
+      }
+#pragma unroll 1
+      for (int c = d & ~511; c < d; c += 32) acc = __fmaf_rn(w[c], xr[c], acc);
       float s = pm_warp_sum_dot(acc);
       if (lane == 0) {
         if (bias) s = __fadd_rn(s, bias[e0 + el]);
@@ -885,109 +917,128 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
   __threadfence();
   if (tid == 0) *ticket = 0;  // ready for the next launch (graph replays included)
 
-  // ---- the last CTA: top-k per token (warp = token) ----
-  float *sm = xs;  // per token: E logits, E scores, E / 2 group scores, E / 2 bytes
-  const int per = 2 * E + E / 2 + (E / 2 + 3) / 4;
+  // ---- the last CTA ----
+  const int per = E + pm_route_scratch(E);  // per token: logits, then its scratch
+  float *sm = xs;
   __shared__ uint32_t s_ids[RS_TOK * PM_MAX_TOPK];
-  __shared__ uint32_t s_cnt[PM_MAX_EXPERTS], s_base[PM_MAX_EXPERTS];
-  __shared__ uint32_t s_w[2][8];
-  if (warp < T) {
-    float *lg = sm + warp * per, *sv = lg + E;
-    for (int e = lane; e < E; e += 32) lg[e] = __ldcg(logits + (size_t)warp * E + e);
-    __syncwarp();
-    pm_route_warp(D, lg, sel_bias, lane, sv, sv + E, (unsigned char *)(sv + E + E / 2), ids + (size_t)warp * K, wout + (size_t)warp * K);
-    __syncwarp();
+  __shared__ unsigned char s_new[RS_TOK * PM_MAX_TOPK];  // 1: no earlier pair has this expert
+  __shared__ float s_red[RS_TOK];
+  const bool soft = D.gating == PM_GATE_SOFTMAX_ALL;
+  for (int t = 0; t < T; t++)
+    for (int e = tid; e < E; e += 256) sm[t * per + e] = __ldcg(logits + (size_t)t * E + e);
+  __syncthreads();
+  if (soft) {
+    if (warp < T) {
+      const float mx = pm_route_max(sm + warp * per, E, lane);
+      if (lane == 0) s_red[warp] = mx;
+    }
+    __syncthreads();
   }
-  for (int e = tid; e < PM_MAX_EXPERTS; e += 256) s_cnt[e] = 0;
+#pragma unroll 1
+  for (int t = 0; t < T; t++)
+#pragma unroll 1
+    for (int e = tid; e < E; e += 256) {
+      float *lg = sm + t * per;
+      const float p = pm_route_elem(D.gating, lg[e], soft ? s_red[t] : 0.0f);
+      lg[E + e] = p;
+      if (!soft) lg[2 * E + e] = sel_bias ? __fadd_rn(p, sel_bias[e]) : p;
+    }
+  __syncthreads();
+  if (soft) {
+    if (warp < T) {
+      const float sum = pm_route_sum(sm + warp * per + E, E, lane);
+      if (lane == 0) s_red[warp] = sum;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int t = 0; t < T; t++)
+#pragma unroll 1
+      for (int e = tid; e < E; e += 256) {
+        float *pr = sm + t * per + E;
+        const float p = __fdiv_rn(pr[e], s_red[t]);
+        pr[e] = p;
+        pr[E + e] = sel_bias ? __fadd_rn(p, sel_bias[e]) : p;
+      }
+    __syncthreads();
+  }
+  if (warp < T) {
+    float *pr = sm + warp * per + E;
+    pm_route_pick(D, pr, pr + E, pr + 2 * E, lane, ids + (size_t)warp * K, wout + (size_t)warp * K);
+  }
   __syncthreads();
   // ---- the plan of the P = T * K pairs (src/moe_kernels.rs:1083-1129 layout) ----
   const int P = T * K;
+  uint32_t mine = 0;
   if (tid < P) {
-    uint32_t e = ids[tid];  // written by this CTA's warps above
+    mine = ids[tid];  // written by this CTA's warps above
     if (slot_table) {  // a placement table: everything from here on names slots; use is counted by expert
-      if (usage) atomicAdd(&usage[e], 1u);
-      e = (uint32_t)slot_table[e];
-      ids[tid] = e;
+      if (usage) atomicAdd(&usage[mine], 1u);
+      mine = (uint32_t)slot_table[mine];
+      ids[tid] = mine;
     }
-    s_ids[tid] = e;
-    atomicAdd(&s_cnt[e], 1u);
+    s_ids[tid] = mine;
   }
   __syncthreads();
-  {  // thread = experts 2 tid, 2 tid + 1: exclusive scans of the counts and of the active experts
-    const uint32_t c0 = s_cnt[2 * tid], c1 = s_cnt[2 * tid + 1];
-    uint32_t o = c0 + c1, na = (c0 > 0) + (c1 > 0);
-    const uint32_t oi = o, ni = na;
-#pragma unroll
-    for (int k = 1; k < 32; k <<= 1) {
-      const uint32_t u = __shfl_up_sync(PM_FULL, o, k), v = __shfl_up_sync(PM_FULL, na, k);
-      if (lane >= k) { o += u; na += v; }
+  if (tid < P) {  // pairs by expert, an expert's pairs in their order
+    uint32_t less = 0, before = 0;
+#pragma unroll 4
+    for (int j = 0; j < P; j++) {
+      const uint32_t o = s_ids[j];
+      less += o < mine;
+      before += o == mine && j < tid;
     }
-    if (lane == 31) { s_w[0][warp] = o; s_w[1][warp] = na; }
-    __syncthreads();
-    uint32_t active = 0;
-    o -= oi;
-    na -= ni;
-#pragma unroll
-    for (int w = 0; w < 8; w++) {
-      if (w < warp) { o += s_w[0][w]; na += s_w[1][w]; }
-      active += s_w[1][w];
-    }
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const int e = 2 * tid + k;
-      if (e < E) {
-        s_base[e] = o + (k ? c0 : 0);
-        pl.base[e] = o + (k ? c0 : 0);
-        pl.cnt[e] = k ? c1 : c0;
-        if ((uint32_t)e >= active) {
-          pl.active[e] = 0;
-          pl.offset[e] = 0;
-          pl.count[e] = 0;
-        }
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const int e = 2 * tid + k;
-      const uint32_t c = k ? c1 : c0;
-      if (c) {
-        pl.active[na] = (uint32_t)e;
-        pl.offset[na] = o;
-        pl.count[na] = c;
-        if (usage && !slot_table) usage[e] += c;
-        if (tt.tiles) {  // (a group has fewer than 16 pairs: one tile each)
-          const int el = e - first_local;
-          tt.tiles[na] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, o, c, 16 * na);
-        }
-        na++;
-      }
-      o += c;
-    }
-    if (tid == 0) {
-      *pl.n_active = (int)active + (tt.shared ? 1 : 0);
-      if (tt.tiles) {
-        if (tt.shared) {  // the shared expert as one more group: every token, pairs P .. P + T - 1
-          pl.offset[active] = P;
-          pl.count[active] = T;
-          tt.tiles[active] = make_uint4(TC_SHARED, P, T, 16 * active);
-        }
-        tt.n[0] = (int)active + (tt.shared ? 1 : 0);
-        tt.next[0] = tt.next[1] = 0;
-      }
-    }
-    if (tt.shared && tid < T) pl.pair_token[P + tid] = (uint32_t)tid;
-  }
-  __syncthreads();
-  if (tid < P) {  // stable: a pair goes behind the earlier pairs of its expert
-    const uint32_t e = s_ids[tid];
-    uint32_t before = 0;
-    for (int j = 0; j < tid; j++) before += s_ids[j] == e;
-    const uint32_t p = s_base[e] + before;
+    s_new[tid] = before == 0;
+    const uint32_t p = less + before;
     pl.pair_pos[tid] = p;
     pl.pair_token[p] = (uint32_t)(tid / K);
     pl.pair_src[p] = (uint32_t)tid;
   }
+  __syncthreads();
+  uint32_t n_active = 0;
+#pragma unroll 1
+  for (int e = tid; e < E; e += 256) {
+    uint32_t less = 0, c = 0, na = 0, active = 0;
+#pragma unroll 4
+    for (int j = 0; j < P; j++) {
+      const uint32_t o = s_ids[j], nw = s_new[j];
+      less += o < (uint32_t)e;
+      c += o == (uint32_t)e;
+      na += o < (uint32_t)e ? nw : 0u;
+      active += nw;
+    }
+    pl.base[e] = less;
+    pl.cnt[e] = c;
+    if ((uint32_t)e >= active) {
+      pl.active[e] = 0;
+      pl.offset[e] = 0;
+      pl.count[e] = 0;
+    }
+    if (c) {
+      pl.active[na] = (uint32_t)e;
+      pl.offset[na] = less;
+      pl.count[na] = c;
+      if (usage && !slot_table) usage[e] += c;
+      if (tt.tiles) {  // (a group has fewer than 16 pairs: one tile each)
+        const int el = e - first_local;
+        tt.tiles[na] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, less, c, 16 * na);
+      }
+    }
+    n_active = active;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    *pl.n_active = (int)n_active + (tt.shared ? 1 : 0);
+    if (tt.tiles) {
+      if (tt.shared) {  // the shared expert as one more group: every token, pairs P .. P + T - 1
+        pl.offset[n_active] = P;
+        pl.count[n_active] = T;
+        tt.tiles[n_active] = make_uint4(TC_SHARED, P, T, 16 * n_active);
+      }
+      tt.n[0] = (int)n_active + (tt.shared ? 1 : 0);
+      tt.next[0] = tt.next[1] = 0;
+    }
+  }
+  if (tt.shared && tid < T) pl.pair_token[P + tid] = (uint32_t)tid;
 }
 
 // whether launch_route_plan_small takes T tokens of this layer: a router row and a token's row have to fit shared memory
@@ -1003,7 +1054,7 @@ void launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x
   int epc = (E + L.n_sm - 1) / L.n_sm;                   // about a CTA an SM
   if (epc > most - 1) epc = most - 1;
   int tg = most - epc < T ? most - epc : T;
-  const int per = 2 * E + E / 2 + (E / 2 + 3) / 4;       // the last CTA's scratch
+  const int per = E + pm_route_scratch(E);               // the last CTA's scratch
   int smem = (epc + tg) * d * 4;
   if (T * per * 4 > smem) smem = T * per * 4;
   static int smem_set = 0;

@@ -166,58 +166,126 @@ __device__ __forceinline__ float pm_route_weight(const pm_layer_desc &D, const f
   return x;
 }
 
-// The whole routing of one token by one warp; lane k < K writes ids_out[k], w_out[k].
-// sel_p: K floats of per-warp shared scratch.
-template <int NP>
-__device__ __forceinline__ void pm_route_warp_n(const pm_layer_desc &D, const float *lg,
-                                                const float *__restrict__ sel_bias, int lane,
-                                                float *ssv, float *gsc, unsigned char *keep,
-                                                uint32_t *ids_out, float *w_out) {
-  const int K = D.top_k;
-  float pr[NP];
-  uint32_t key[NP];
-  pm_route_scores<NP>(D, lg, sel_bias, lane, ssv, gsc, keep, pr, key);
-  float *sel_p = ssv;  // the group scratch is free again
-  __syncwarp();
-  // K rounds of (max, lowest index) (src/moe_kernels.rs:1053-1067), on ordered
-  // integer keys: one warp-wide max, then the first slot/lane that holds it
-  const uint32_t KNEG = pm_fkey(PM_NEG);
-  uint32_t my_e = 0;
+// The same routing with a token's scores in shared memory and every loop rolled. A kernel that routes a few tokens runs
+// each instruction once or a few times, cold: unrolled over registers (256 experts: 8 a lane, with the exponentials and
+// divisions of every gating) one token took 8.7 us of waiting for instructions.
+// Floats of scratch a token: scores, ranked scores, group scores, group marks, the picks' scores.
+__host__ __device__ inline int pm_route_scratch(int E) { return 2 * E + E / 2 + (E / 2 + 3) / 4 + PM_MAX_TOPK; }
+// elementwise part of the gating (mx: the largest logit, softmax over all experts only)
+__device__ __forceinline__ float pm_route_elem(int gating, float v, float mx) {
+  if (gating == PM_GATE_SOFTMAX_ALL) return pm_exp(__fsub_rn(v, mx));
+  if (gating == PM_GATE_SIGMOID) return __fdiv_rn(1.0f, __fadd_rn(1.0f, pm_exp(-v)));
+  if (gating == PM_GATE_SQRT_SOFTPLUS) return __fsqrt_rn(v > 20.0f ? v : pm_log1p(pm_exp(v)));
+  return v;
+}
+// one warp: the largest of E logits; the sum of E scores (lane L adds L, L + 32, ... in order, then the lanes)
+__device__ __forceinline__ float pm_route_max(const float *lg, int E, int lane) {
+  float mx = PM_NEG;
 #pragma unroll 1
-  for (int k = 0; k < K; k++) {
-    uint32_t lk = key[0];
-#pragma unroll
-    for (int i = 1; i < NP; i++) lk = max(lk, key[i]);
-    uint32_t m = __reduce_max_sync(PM_FULL, lk);
-    uint32_t e = 0;
-    float w = 0.0f;
-    bool found = false;
-#pragma unroll
-    for (int i = 0; i < NP; i++) {
-      uint32_t b = __ballot_sync(PM_FULL, key[i] == m);
-      if (!found && b != 0) {  // uniform across the warp
-        found = true;
-        int lw = __ffs((int)b) - 1;
-        e = (uint32_t)(32 * i + lw);
-        w = __shfl_sync(PM_FULL, pr[i], lw);
-        if (lane == lw) key[i] = KNEG;
+  for (int e = lane; e < E; e += 32) mx = fmaxf(mx, lg[e]);
+  return pm_funkey(__reduce_max_sync(PM_FULL, pm_fkey(mx)));
+}
+__device__ __forceinline__ float pm_route_sum(const float *pr, int E, int lane) {
+  float sum = 0.0f;
+#pragma unroll 1
+  for (int e = lane; e < E; e += 32) sum = __fadd_rn(sum, pr[e]);
+  return pm_warp_sum_16_1(sum);
+}
+// one warp: group mask, K picks and their weights from a token's scores pr[E] and ranked scores sv[E] (sv is used up);
+// rest: the scratch behind them. Lane k < K writes ids_out[k], w_out[k].
+__device__ __forceinline__ void pm_route_pick(const pm_layer_desc &D, const float *pr, float *sv, float *rest, int lane,
+                                              uint32_t *ids_out, float *w_out) {
+  const int E = D.n_exp, K = D.top_k;
+  float *gsc = rest, *sel_p = rest + E / 2 + (E / 2 + 3) / 4;
+  unsigned char *keep = (unsigned char *)(rest + E / 2);
+  if (D.n_group > 0) {  // the definition is pm_route_scores'
+    const int G = D.n_group, gs = E / G;
+    if (gs == 32) {
+#pragma unroll 1
+      for (int g = 0; g < G; g++) {
+        const uint32_t key = pm_fkey(sv[32 * g + lane]), m1 = __reduce_max_sync(PM_FULL, key);
+        const uint32_t top = __ballot_sync(PM_FULL, key == m1);
+        const uint32_t m2 = __reduce_max_sync(PM_FULL, key == m1 ? 0u : key);
+        if (lane == 0) gsc[g] = __fadd_rn(pm_funkey(m1), pm_funkey((top & (top - 1)) ? m1 : m2));
+      }
+    } else {
+#pragma unroll 1
+      for (int g = lane; g < G; g += 32) {
+        int i1 = 0;
+        float v1 = sv[g * gs], v2 = PM_NEG;
+        for (int i = 1; i < gs; i++)
+          if (sv[g * gs + i] > v1) { v1 = sv[g * gs + i]; i1 = i; }
+        for (int i = 0; i < gs; i++)
+          if (i != i1 && sv[g * gs + i] > v2) v2 = sv[g * gs + i];
+        gsc[g] = __fadd_rn(v1, v2);
       }
     }
-    if (lane == k) my_e = e;
-    if (lane == 0) sel_p[k] = w;
+    __syncwarp();
+#pragma unroll 1
+    for (int g = lane; g < G; g += 32) {  // kept when fewer than topk_group groups come before it
+      const float mine = gsc[g];
+      int before = 0;
+#pragma unroll 1
+      for (int j = 0; j < G; j++) {
+        const float v = gsc[j];
+        before += v > mine || (v == mine && j < g);
+      }
+      keep[g] = before < D.topk_group;
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int e = lane; e < E; e += 32)
+      if (!keep[gs == 32 ? e >> 5 : e / gs]) sv[e] = PM_NEG;
   }
+  // K rounds of (max, lowest index) (src/moe_kernels.rs:1053-1067) on ordered integer keys; a lane keeps the best of
+  // its own experts and looks for the next one only when it has lost it
+  uint32_t best = 0, at = 0xffffffffu, mine = 0;
+  auto look = [&] {
+    best = lane < E ? pm_fkey(sv[lane]) : 0u;
+    at = lane < E ? (uint32_t)lane : 0xffffffffu;
+#pragma unroll 4
+    for (int e = lane + 32; e < E; e += 32) {
+      const uint32_t k = pm_fkey(sv[e]);
+      if (k > best) {
+        best = k;
+        at = (uint32_t)e;
+      }
+    }
+  };
+  look();
+#pragma unroll 1
+  for (int k = 0; k < K; k++) {
+    const uint32_t m = __reduce_max_sync(PM_FULL, best);
+    const uint32_t e = __reduce_min_sync(PM_FULL, best == m ? at : 0xffffffffu);
+    if (lane == k) mine = e;
+    if (at == e) {
+      sv[e] = PM_NEG;
+      look();
+    }
+  }
+  if (lane < K) sel_p[lane] = pr[mine];
   __syncwarp();
   if (lane < K) {
-    ids_out[lane] = my_e;
+    ids_out[lane] = mine;
     w_out[lane] = pm_route_weight(D, sel_p, lane);
   }
 }
-
-__device__ __forceinline__ void pm_route_warp(const pm_layer_desc &D, const float *lg,
-                                              const float *__restrict__ sel_bias, int lane,
-                                              float *ssv, float *gsc, unsigned char *keep,
-                                              uint32_t *ids_out, float *w_out) {
-  if (D.n_exp <= 128) pm_route_warp_n<4>(D, lg, sel_bias, lane, ssv, gsc, keep, ids_out, w_out);
-  else if (D.n_exp <= 256) pm_route_warp_n<8>(D, lg, sel_bias, lane, ssv, gsc, keep, ids_out, w_out);
-  else pm_route_warp_n<16>(D, lg, sel_bias, lane, ssv, gsc, keep, ids_out, w_out);
+// the whole routing of one token by one warp; sc: pm_route_scratch(E) floats
+__device__ __forceinline__ void pm_route_warp(const pm_layer_desc &D, const float *lg, const float *__restrict__ sel_bias, int lane,
+                                              float *sc, uint32_t *ids_out, float *w_out) {
+  const int E = D.n_exp;
+  float *pr = sc, *sv = sc + E;
+  const bool soft = D.gating == PM_GATE_SOFTMAX_ALL;
+  const float mx = soft ? pm_route_max(lg, E, lane) : 0.0f;
+#pragma unroll 1
+  for (int e = lane; e < E; e += 32) pr[e] = pm_route_elem(D.gating, lg[e], mx);
+  const float sum = soft ? pm_route_sum(pr, E, lane) : 1.0f;
+#pragma unroll 1
+  for (int e = lane; e < E; e += 32) {
+    const float p = soft ? __fdiv_rn(pr[e], sum) : pr[e];
+    pr[e] = p;
+    sv[e] = sel_bias ? __fadd_rn(p, sel_bias[e]) : p;
+  }
+  __syncwarp();
+  pm_route_pick(D, pr, sv, sc + 2 * E, lane, ids_out, w_out);
 }
