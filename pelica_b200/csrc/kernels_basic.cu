@@ -647,6 +647,9 @@ void launch_plan(const Launch &L, const LayerDev &ly, const uint32_t *ids, int T
 
 // ---------------------------------------------------------------------------
 // The same plan when the ids come from k_route's logits: the pairs are cut into segments of 32 tokens.
+// The kernels that one CTA's latency decides run their code once for practice while they wait for the kernel before (on
+// zeros, into pm_plan_nowhere): executed once and cold, an instruction costs them some 30 cycles, all of it waiting
+// for the instruction (8 tokens on 128 experts: route 12,000 cycles, scan 10,700, place 2,200).
 // k_route_seg routes a segment (a warp a token) and counts its pairs by expert; k_plan_seg_scan turns the
 // [segments][E] counts into first positions (and writes the tile list of the tensor-core products);
 // k_plan_seg_place ranks the pairs of a segment. Three launches whose work grows with the pairs, where
@@ -654,6 +657,16 @@ void launch_plan(const Launch &L, const LayerDev &ly, const uint32_t *ids, int T
 // One segment: its CTA does all three (the plan of 8 to 32 tokens).
 // ---------------------------------------------------------------------------
 #define PL_SEG 32 /* tokens of a segment = warps of its CTA */
+// a plan whose arrays are all the same `words` of shared memory (at least max(E + 1, 512, 4 * tiles + 4) of them)
+__device__ __forceinline__ void pm_plan_nowhere(uint32_t *words, PlanDev &pl, TcTiles &tt) {
+  pl.n_active = (int *)words;
+  pl.active = pl.offset = pl.count = pl.base = pl.cnt = pl.pair_token = pl.pair_pos = pl.pair_src = words;
+  if (tt.tiles) {
+    tt.n = (int *)words;
+    tt.next = (unsigned int *)words;
+    tt.tiles = (uint4 *)words;
+  }
+}
 // exclusive scans over 512 values of a CTA's first 512 threads: (a, b) -> sums of the earlier threads' values and the totals
 __device__ __forceinline__ void pm_scan2_512(uint32_t a, uint32_t b, uint32_t &ea, uint32_t &eb, uint32_t &ta, uint32_t &tb,
                                              uint32_t (*sh)[16]) {
@@ -744,55 +757,93 @@ __device__ __forceinline__ void pm_plan_place(PlanDev pl, const uint32_t *s_id, 
 __global__ void __launch_bounds__(1024) k_route_seg(pm_layer_desc D, const float *__restrict__ logits,
                                                    const float *__restrict__ sel_bias, int T, uint32_t *ids, float *wout,
                                                    uint32_t *seg_cnt, PlanDev pl, uint32_t *usage, TcTiles tt, int first_local, int n_local) {
-  pm_pdl();
+  pm_pdl_trigger();
   extern __shared__ __align__(16) float rsm[];  // 512 experts of pairs, E counts, [32] x scratch
   __shared__ uint32_t sh[2][16];
-  const int E = D.n_exp, K = D.top_k, lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  __shared__ __align__(16) uint32_t nowhere[4 * 512 + 4];
+  const int E = D.n_exp, K = D.top_k, lane = threadIdx.x & 31, wi = threadIdx.x >> 5, i = threadIdx.x;
   uint32_t *s_id = (uint32_t *)rsm, *cnt = s_id + 512;
   float *sc = rsm + 512 + E + wi * pm_route_scratch(E);
-  for (int e = threadIdx.x; e < E; e += 1024) cnt[e] = 0;
-  __syncthreads();
-  const int t = blockIdx.x * PL_SEG + wi;
-  if (t < T) {
-    pm_route_warp(D, logits + (size_t)t * E, sel_bias, lane, sc, ids + (size_t)t * K, wout + (size_t)t * K);
-    __syncwarp();
-    if (lane < K) {
-      const uint32_t e = ids[(size_t)t * K + lane];  // (written by this warp above)
-      atomicAdd(&cnt[e], 1u);
-      s_id[wi * K + lane] = e;
+#pragma unroll 1
+  for (int practice = 1; practice >= 0; practice--) {
+    PlanDev p = pl;
+    TcTiles q = tt;
+    const int t = blockIdx.x * PL_SEG + wi;
+    const float *lg = logits + (size_t)t * E;
+    uint32_t *o_id = ids + (size_t)t * K;
+    float *o_w = wout + (size_t)t * K;
+    if (practice) {
+      pm_plan_nowhere(nowhere, p, q);
+      for (int e = i; e < 512; e += 1024) nowhere[e] = 0;
+      lg = (const float *)nowhere;
+      o_id = nowhere + 512;
+      o_w = (float *)nowhere + 512 + PM_MAX_TOPK;
+    } else {
+      pm_pdl_wait();
     }
+    for (int e = i; e < E; e += 1024) cnt[e] = 0;
+    __syncthreads();
+    const int lim = practice ? 1 : T;
+    if (practice ? wi == 0 : t < T) {
+      pm_route_warp(D, lg, sel_bias, lane, sc, o_id, o_w);
+      __syncwarp();
+      if (lane < K) {
+        const uint32_t e = o_id[lane];  // (written by this warp above)
+        atomicAdd(&cnt[e], 1u);
+        s_id[wi * K + lane] = e;
+      }
+    }
+    __syncthreads();
+    if (gridDim.x > 1) {
+      if (!practice)
+        for (int e = i; e < E; e += 1024) seg_cnt[(size_t)blockIdx.x * E + e] = cnt[e];
+      continue;
+    }
+    const uint32_t o = pm_plan_scan(p, i, i < E ? cnt[i] : 0u, E, lim, practice ? nullptr : usage, q, first_local, n_local, sh);
+    __syncthreads();
+    if (i < E) cnt[i] = o;
+    __syncthreads();
+    if (i < lim * K) pm_plan_place(p, s_id, i, i, K, s_id[i], cnt[s_id[i]]);
+    __syncthreads();
   }
-  __syncthreads();
-  if (gridDim.x > 1) {
-    for (int e = threadIdx.x; e < E; e += 1024) seg_cnt[(size_t)blockIdx.x * E + e] = cnt[e];
-    return;
-  }
-  const int i = threadIdx.x;
-  const uint32_t o = pm_plan_scan(pl, i, i < E ? cnt[i] : 0u, E, T, usage, tt, first_local, n_local, sh);
-  __syncthreads();
-  if (i < E) cnt[i] = o;
-  __syncthreads();
-  if (i < T * K) pm_plan_place(pl, s_id, i, i, K, s_id[i], cnt[s_id[i]]);
 }
 // one CTA: counts of the segments -> the plan, seg_cnt[s][e] -> first position of segment s's pairs of expert e
 __global__ void __launch_bounds__(512) k_plan_seg_scan(PlanDev pl, int E, int T, int n_seg, uint32_t *seg_cnt, uint32_t *usage, TcTiles tt,
                                                        int first_local, int n_local) {
-  pm_pdl();
+  pm_pdl_trigger();
   __shared__ uint32_t sh[2][16];
+  __shared__ __align__(16) uint32_t nowhere[4 * 512 + 4];
   const int e = threadIdx.x;
-  uint32_t c = 0;
-  if (e < E) {
-#pragma unroll 16
-    for (int s = 0; s < n_seg; s++) c += seg_cnt[(size_t)s * E + e];
-  }
-  uint32_t run = pm_plan_scan(pl, e, c, E, T, usage, tt, first_local, n_local, sh);
-  if (e < E) {
-#pragma unroll 16
-    for (int s = 0; s < n_seg; s++) {
-      const uint32_t v = seg_cnt[(size_t)s * E + e];
-      seg_cnt[(size_t)s * E + e] = run;
-      run += v;
+#pragma unroll 1
+  for (int practice = 1; practice >= 0; practice--) {
+    PlanDev p = pl;
+    TcTiles q = tt;
+    uint32_t *sc = seg_cnt;
+    int n = n_seg;
+    if (practice) {
+      pm_plan_nowhere(nowhere, p, q);
+      nowhere[e] = e < 8;
+      sc = nowhere;
+      n = 1;
+      __syncthreads();
+    } else {
+      pm_pdl_wait();
     }
+    uint32_t c = 0;
+    if (e < E) {
+#pragma unroll 8
+      for (int s = 0; s < n; s++) c += sc[(size_t)s * E + e];
+    }
+    uint32_t run = pm_plan_scan(p, e, c, E, practice ? 1 : T, practice ? nullptr : usage, q, first_local, n_local, sh);
+    if (e < E) {
+#pragma unroll 8
+      for (int s = 0; s < n; s++) {
+        const uint32_t v = sc[(size_t)s * E + e];
+        sc[(size_t)s * E + e] = run;
+        run += v;
+      }
+    }
+    __syncthreads();
   }
 }
 // a CTA a segment: thread i = pair i of it; its rank among the segment's earlier pairs of the same expert
@@ -813,7 +864,7 @@ void launch_route_plan(const Launch &L, const LayerDev &ly, const float *logits,
                        uint32_t *seg, const TcTiles &tt) {
   const int E = ly.desc.n_exp, K = ly.desc.top_k, nseg = (T + PL_SEG - 1) / PL_SEG;
   const int smem = (512 + E + PL_SEG * pm_route_scratch(E)) * 4;
-  static int smem_set = 48 * 1024;
+  static int smem_set = 32 * 1024;  // (and 8 KB of static shared memory)
   if (smem > smem_set) {
     cudaFuncSetAttribute(k_route_seg, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     smem_set = smem;
@@ -835,13 +886,13 @@ void launch_route_plan(const Launch &L, const LayerDev &ly, const float *logits,
 __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const float *__restrict__ wr,
                                                           const float *__restrict__ bias,
                                                           const float *__restrict__ sel_bias,
-                                                          const float *__restrict__ x, int T, int epc, int tg, float *logits,
-                                                          uint32_t *ids, float *wout, PlanDev pl, uint32_t *usage,
+                                                          const float *__restrict__ x, int n_tok, int epc, int tg, int practice_at, float *logits,
+                                                          uint32_t *ids_out, float *w_out, PlanDev plan, uint32_t *usage_out,
                                                           const int32_t *__restrict__ slot_table, unsigned int *ticket,
-                                                          TcTiles tt, int first_local, int n_local, int *err,
+                                                          TcTiles tiles, int first_local, int n_local, int *err,
                                                           unsigned long long wait_ns) {
   pm_pdl_trigger();
-  extern __shared__ __align__(16) float xs[];  // [epc][d] router rows, [tg][d] tokens; reused by the last CTA
+  extern __shared__ __align__(16) float xs[];  // [epc][d] router rows, [tg][d] tokens; reused by the last CTA; practice area
   __shared__ __align__(8) uint64_t s_bar;
   const int E = D.n_exp, d = D.d, K = D.top_k;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -858,187 +909,208 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
   };
-  uint32_t ph = 0;
-  for (int t0 = 0; t0 < T; t0 += tg, ph ^= 1) {
-    const int nt = min(tg, T - t0);
-    if (t0 > 0) __syncthreads();  // everybody is done with the tokens before
-    if (tid == 0) {
-      const uint32_t wb = t0 == 0 ? (uint32_t)(ne * d * 4) : 0u, xb = (uint32_t)(nt * d * 4);
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(wb + xb) : "memory");
-      if (wb) bulk(xs, wr + (size_t)e0 * d, wb);  // (the router's rows depend on nothing before this launch)
-      if (t0 == 0) pm_pdl_wait();
-      bulk(xs + (size_t)epc * d, x + (size_t)t0 * d, xb);
-    }
-    if (t0 == 0) pm_pdl_wait();
-    {  // bounded: the copies' own time, a few us
-      unsigned long long s0 = 0;
-      for (;;) {
-        uint32_t ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok) : "r"(bar), "r"(ph) : "memory");
-        if (ok) break;
-        unsigned long long now;
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
-        if (s0 == 0) s0 = now;
-        if (now - s0 > wait_ns) {
-          atomicCAS(err, 0, 9);
-          break;
-        }
-      }
-    }
-    for (int i = warp; i < ne * nt; i += 8) {
-      const int el = i % ne, t = i / ne;
-      const float *w = xs + (size_t)el * d + lane, *xr = xs + (size_t)(epc + t) * d + lane;
-      float acc = 0.0f;
-#pragma unroll 1
-      for (int c = 0; c < (d & ~511); c += 512) {  // 16 columns a lane read at once: one latency for 16 steps of the chain
-        float a[16], b[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++) { a[i] = w[c + 32 * i]; b[i] = xr[c + 32 * i]; }
-#pragma unroll
-        for (int i = 0; i < 16; i++) acc = __fmaf_rn(a[i], b[i], acc);
-      }
-#pragma unroll 1
-      for (int c = d & ~511; c < d; c += 32) acc = __fmaf_rn(w[c], xr[c], acc);
-      float s = pm_warp_sum_dot(acc);
-      if (lane == 0) {
-        if (bias) s = __fadd_rn(s, bias[e0 + el]);
-        logits[(size_t)(t0 + t) * E + e0 + el] = s;
-      }
-    }
-  }
-  __shared__ unsigned int s_last;
-  __threadfence();  // this CTA's logits before its ticket
-  __syncthreads();
-  if (tid == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  if (tid == 0) *ticket = 0;  // ready for the next launch (graph replays included)
-
-  // ---- the last CTA ----
-  const int per = E + pm_route_scratch(E);  // per token: logits, then its scratch
-  float *sm = xs;
   __shared__ uint32_t s_ids[RS_TOK * PM_MAX_TOPK];
   __shared__ unsigned char s_new[RS_TOK * PM_MAX_TOPK];  // 1: no earlier pair has this expert
   __shared__ float s_red[RS_TOK];
-  const bool soft = D.gating == PM_GATE_SOFTMAX_ALL;
-  for (int t = 0; t < T; t++)
-    for (int e = tid; e < E; e += 256) sm[t * per + e] = __ldcg(logits + (size_t)t * E + e);
-  __syncthreads();
-  if (soft) {
-    if (warp < T) {
-      const float mx = pm_route_max(sm + warp * per, E, lane);
-      if (lane == 0) s_red[warp] = mx;
-    }
-    __syncthreads();
+  __shared__ unsigned int s_last;
+  const uint32_t wb = (uint32_t)(ne * d * 4);
+  if (tid == 0) {  // (the router's rows depend on nothing before this launch)
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(wb) : "memory");
+    bulk(xs, wr + (size_t)e0 * d, wb);
   }
+  // the last CTA's part runs once for practice (see k_route_seg): any CTA may be the last
 #pragma unroll 1
-  for (int t = 0; t < T; t++)
+  for (int practice = 1; practice >= 0; practice--) {
+    if (!practice) {
+      uint32_t ph = 0;
+      for (int t0 = 0; t0 < n_tok; t0 += tg, ph ^= 1) {
+        const int nt = min(tg, n_tok - t0);
+        if (t0 > 0) __syncthreads();  // everybody is done with the tokens before
+        if (tid == 0) {
+          const uint32_t xb = (uint32_t)(nt * d * 4);
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(xb) : "memory");
+          if (t0 == 0) pm_pdl_wait();
+          bulk(xs + (size_t)epc * d, x + (size_t)t0 * d, xb);
+        }
+        if (t0 == 0) pm_pdl_wait();
+        {  // bounded: the copies' own time, a few us
+          unsigned long long s0 = 0;
+          for (;;) {
+            uint32_t ok;
+            asm volatile(
+                "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+                : "=r"(ok) : "r"(bar), "r"(ph) : "memory");
+            if (ok) break;
+            unsigned long long now;
+            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+            if (s0 == 0) s0 = now;
+            if (now - s0 > wait_ns) {
+              atomicCAS(err, 0, 9);
+              break;
+            }
+          }
+        }
+        for (int i = warp; i < ne * nt; i += 8) {
+          const int el = i % ne, t = i / ne;
+          const float *w = xs + (size_t)el * d + lane, *xr = xs + (size_t)(epc + t) * d + lane;
+          float acc = 0.0f;
 #pragma unroll 1
-    for (int e = tid; e < E; e += 256) {
-      float *lg = sm + t * per;
-      const float p = pm_route_elem(D.gating, lg[e], soft ? s_red[t] : 0.0f);
-      lg[E + e] = p;
-      if (!soft) lg[2 * E + e] = sel_bias ? __fadd_rn(p, sel_bias[e]) : p;
+          for (int c = 0; c < (d & ~511); c += 512) {  // 16 columns a lane read at once: one latency for 16 steps of the chain
+            float a[16], b[16];
+#pragma unroll
+            for (int i = 0; i < 16; i++) { a[i] = w[c + 32 * i]; b[i] = xr[c + 32 * i]; }
+#pragma unroll
+            for (int i = 0; i < 16; i++) acc = __fmaf_rn(a[i], b[i], acc);
+          }
+#pragma unroll 1
+          for (int c = d & ~511; c < d; c += 32) acc = __fmaf_rn(w[c], xr[c], acc);
+          float s = pm_warp_sum_dot(acc);
+          if (lane == 0) {
+            if (bias) s = __fadd_rn(s, bias[e0 + el]);
+            logits[(size_t)(t0 + t) * E + e0 + el] = s;
+          }
+        }
+      }
+      __threadfence();  // this CTA's logits before its ticket
+      __syncthreads();
+      if (tid == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
+      __syncthreads();
+      if (!s_last) return;
+      __threadfence();
+      if (tid == 0) *ticket = 0;  // ready for the next launch (graph replays included)
     }
-  __syncthreads();
-  if (soft) {
-    if (warp < T) {
-      const float sum = pm_route_sum(sm + warp * per + E, E, lane);
-      if (lane == 0) s_red[warp] = sum;
+    // ---- the last CTA ----
+    const int per = E + pm_route_scratch(E);  // per token: logits, then its scratch
+    float *sm = practice ? xs + practice_at : xs;
+    const int T = practice ? 1 : n_tok;
+    PlanDev pl = plan;
+    TcTiles tt = tiles;
+    uint32_t *ids = ids_out, *usage = practice ? nullptr : usage_out;
+    float *wout = w_out;
+    if (practice) {
+      uint32_t *nowhere = (uint32_t *)(sm + ((per + 3) & ~3));
+      pm_plan_nowhere(nowhere, pl, tt);
+      ids = nowhere + 512;
+      wout = (float *)nowhere + 512 + PM_MAX_TOPK;
     }
+    const bool soft = D.gating == PM_GATE_SOFTMAX_ALL;
+    for (int t = 0; t < T; t++)
+      for (int e = tid; e < E; e += 256) sm[t * per + e] = practice ? 0.0f : __ldcg(logits + (size_t)t * E + e);
     __syncthreads();
+    if (soft) {
+      if (warp < T) {
+        const float mx = pm_route_max(sm + warp * per, E, lane);
+        if (lane == 0) s_red[warp] = mx;
+      }
+      __syncthreads();
+    }
 #pragma unroll 1
     for (int t = 0; t < T; t++)
 #pragma unroll 1
       for (int e = tid; e < E; e += 256) {
-        float *pr = sm + t * per + E;
-        const float p = __fdiv_rn(pr[e], s_red[t]);
-        pr[e] = p;
-        pr[E + e] = sel_bias ? __fadd_rn(p, sel_bias[e]) : p;
+        float *lg = sm + t * per;
+        const float p = pm_route_elem(D.gating, lg[e], soft ? s_red[t] : 0.0f);
+        lg[E + e] = p;
+        if (!soft) lg[2 * E + e] = sel_bias ? __fadd_rn(p, sel_bias[e]) : p;
       }
     __syncthreads();
-  }
-  if (warp < T) {
-    float *pr = sm + warp * per + E;
-    pm_route_pick(D, pr, pr + E, pr + 2 * E, lane, ids + (size_t)warp * K, wout + (size_t)warp * K);
-  }
-  __syncthreads();
-  // ---- the plan of the P = T * K pairs (src/moe_kernels.rs:1083-1129 layout) ----
-  const int P = T * K;
-  uint32_t mine = 0;
-  if (tid < P) {
-    mine = ids[tid];  // written by this CTA's warps above
-    if (slot_table) {  // a placement table: everything from here on names slots; use is counted by expert
-      if (usage) atomicAdd(&usage[mine], 1u);
-      mine = (uint32_t)slot_table[mine];
-      ids[tid] = mine;
-    }
-    s_ids[tid] = mine;
-  }
-  __syncthreads();
-  if (tid < P) {  // pairs by expert, an expert's pairs in their order
-    uint32_t less = 0, before = 0;
-#pragma unroll 4
-    for (int j = 0; j < P; j++) {
-      const uint32_t o = s_ids[j];
-      less += o < mine;
-      before += o == mine && j < tid;
-    }
-    s_new[tid] = before == 0;
-    const uint32_t p = less + before;
-    pl.pair_pos[tid] = p;
-    pl.pair_token[p] = (uint32_t)(tid / K);
-    pl.pair_src[p] = (uint32_t)tid;
-  }
-  __syncthreads();
-  uint32_t n_active = 0;
+    if (soft) {
+      if (warp < T) {
+        const float sum = pm_route_sum(sm + warp * per + E, E, lane);
+        if (lane == 0) s_red[warp] = sum;
+      }
+      __syncthreads();
 #pragma unroll 1
-  for (int e = tid; e < E; e += 256) {
-    uint32_t less = 0, c = 0, na = 0, active = 0;
+      for (int t = 0; t < T; t++)
+#pragma unroll 1
+        for (int e = tid; e < E; e += 256) {
+          float *pr = sm + t * per + E;
+          const float p = __fdiv_rn(pr[e], s_red[t]);
+          pr[e] = p;
+          pr[E + e] = sel_bias ? __fadd_rn(p, sel_bias[e]) : p;
+        }
+      __syncthreads();
+    }
+    if (warp < T) {
+      float *pr = sm + warp * per + E;
+      pm_route_pick(D, pr, pr + E, pr + 2 * E, lane, ids + (size_t)warp * K, wout + (size_t)warp * K);
+    }
+    __syncthreads();
+    // ---- the plan of the P = T * K pairs (src/moe_kernels.rs:1083-1129 layout) ----
+    const int P = T * K;
+    uint32_t mine = 0;
+    if (tid < P) {
+      mine = ids[tid];  // written by this CTA's warps above
+      if (slot_table && !practice) {  // a placement table: everything from here on names slots; use is counted by expert
+        if (usage) atomicAdd(&usage[mine], 1u);
+        mine = (uint32_t)slot_table[mine];
+        ids[tid] = mine;
+      }
+      s_ids[tid] = mine;
+    }
+    __syncthreads();
+    if (tid < P) {  // pairs by expert, an expert's pairs in their order
+      uint32_t less = 0, before = 0;
 #pragma unroll 4
-    for (int j = 0; j < P; j++) {
-      const uint32_t o = s_ids[j], nw = s_new[j];
-      less += o < (uint32_t)e;
-      c += o == (uint32_t)e;
-      na += o < (uint32_t)e ? nw : 0u;
-      active += nw;
+      for (int j = 0; j < P; j++) {
+        const uint32_t o = s_ids[j];
+        less += o < mine;
+        before += o == mine && j < tid;
+      }
+      s_new[tid] = before == 0;
+      const uint32_t p = less + before;
+      pl.pair_pos[tid] = p;
+      pl.pair_token[p] = (uint32_t)(tid / K);
+      pl.pair_src[p] = (uint32_t)tid;
     }
-    pl.base[e] = less;
-    pl.cnt[e] = c;
-    if ((uint32_t)e >= active) {
-      pl.active[e] = 0;
-      pl.offset[e] = 0;
-      pl.count[e] = 0;
+    __syncthreads();
+    uint32_t n_active = 0;
+#pragma unroll 1
+    for (int e = tid; e < E; e += 256) {
+      uint32_t less = 0, c = 0, na = 0, active = 0;
+#pragma unroll 4
+      for (int j = 0; j < P; j++) {
+        const uint32_t o = s_ids[j], nw = s_new[j];
+        less += o < (uint32_t)e;
+        c += o == (uint32_t)e;
+        na += o < (uint32_t)e ? nw : 0u;
+        active += nw;
+      }
+      pl.base[e] = less;
+      pl.cnt[e] = c;
+      if ((uint32_t)e >= active) {
+        pl.active[e] = 0;
+        pl.offset[e] = 0;
+        pl.count[e] = 0;
+      }
+      if (c) {
+        pl.active[na] = (uint32_t)e;
+        pl.offset[na] = less;
+        pl.count[na] = c;
+        if (usage && !slot_table) usage[e] += c;
+        if (tt.tiles) {  // (a group has fewer than 16 pairs: one tile each)
+          const int el = e - first_local;
+          tt.tiles[na] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, less, c, 16 * na);
+        }
+      }
+      n_active = active;
     }
-    if (c) {
-      pl.active[na] = (uint32_t)e;
-      pl.offset[na] = less;
-      pl.count[na] = c;
-      if (usage && !slot_table) usage[e] += c;
-      if (tt.tiles) {  // (a group has fewer than 16 pairs: one tile each)
-        const int el = e - first_local;
-        tt.tiles[na] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, less, c, 16 * na);
+    __syncthreads();
+    if (tid == 0) {
+      *pl.n_active = (int)n_active + (tt.shared ? 1 : 0);
+      if (tt.tiles) {
+        if (tt.shared) {  // the shared expert as one more group: every token, pairs P .. P + T - 1
+          pl.offset[n_active] = P;
+          pl.count[n_active] = T;
+          tt.tiles[n_active] = make_uint4(TC_SHARED, P, T, 16 * n_active);
+        }
+        tt.n[0] = (int)n_active + (tt.shared ? 1 : 0);
+        tt.next[0] = tt.next[1] = 0;
       }
     }
-    n_active = active;
+    if (tt.shared && tid < T) pl.pair_token[P + tid] = (uint32_t)tid;
+    __syncthreads();
   }
-  __syncthreads();
-  if (tid == 0) {
-    *pl.n_active = (int)n_active + (tt.shared ? 1 : 0);
-    if (tt.tiles) {
-      if (tt.shared) {  // the shared expert as one more group: every token, pairs P .. P + T - 1
-        pl.offset[n_active] = P;
-        pl.count[n_active] = T;
-        tt.tiles[n_active] = make_uint4(TC_SHARED, P, T, 16 * n_active);
-      }
-      tt.n[0] = (int)n_active + (tt.shared ? 1 : 0);
-      tt.next[0] = tt.next[1] = 0;
-    }
-  }
-  if (tt.shared && tid < T) pl.pair_token[P + tid] = (uint32_t)tid;
 }
 
 // whether launch_route_plan_small takes T tokens of this layer: a router row and a token's row have to fit shared memory
@@ -1057,12 +1129,14 @@ void launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x
   const int per = E + pm_route_scratch(E);               // the last CTA's scratch
   int smem = (epc + tg) * d * 4;
   if (T * per * 4 > smem) smem = T * per * 4;
+  const int practice_at = (smem + 15) / 16 * 4;
+  smem = (practice_at + per + 512 + 2 * PM_MAX_TOPK + 4) * 4;
   static int smem_set = 0;
   if (smem > smem_set) {  // (raised on a layer's first call, which is never inside a stream capture)
     cudaFuncSetAttribute(k_route_plan_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     smem_set = smem;
   }
-  PLAUNCH(L, k_route_plan_small, (E + epc - 1) / epc, 256, smem, ly.desc, ly.router, ly.logit_bias, ly.select_bias, x, T, epc, tg,
+  PLAUNCH(L, k_route_plan_small, (E + epc - 1) / epc, 256, smem, ly.desc, ly.router, ly.logit_bias, ly.select_bias, x, T, epc, tg, practice_at,
           logits, ids, w, pl, ly.usage, slot_table, ticket, tt, ly.first_local, ly.n_local, err, wait_ns);
 }
 
