@@ -886,13 +886,13 @@ void launch_route_plan(const Launch &L, const LayerDev &ly, const float *logits,
 __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const float *__restrict__ wr,
                                                           const float *__restrict__ bias,
                                                           const float *__restrict__ sel_bias,
-                                                          const float *__restrict__ x, int n_tok, int epc, int tg, int practice_at, float *logits,
-                                                          uint32_t *ids_out, float *w_out, PlanDev plan, uint32_t *usage_out,
+                                                          const float *__restrict__ x, int T, int epc, int tg, float *logits,
+                                                          uint32_t *ids, float *wout, PlanDev pl, uint32_t *usage,
                                                           const int32_t *__restrict__ slot_table, unsigned int *ticket,
-                                                          TcTiles tiles, int first_local, int n_local, int *err,
+                                                          TcTiles tt, int first_local, int n_local, int *err,
                                                           unsigned long long wait_ns) {
   pm_pdl_trigger();
-  extern __shared__ __align__(16) float xs[];  // [epc][d] router rows, [tg][d] tokens; reused by the last CTA; practice area
+  extern __shared__ __align__(16) float xs[];  // [epc][d] router rows, [tg][d] tokens; reused by the last CTA
   __shared__ __align__(8) uint64_t s_bar;
   const int E = D.n_exp, d = D.d, K = D.top_k;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -918,199 +918,186 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
     asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(wb) : "memory");
     bulk(xs, wr + (size_t)e0 * d, wb);
   }
-  // the last CTA's part runs once for practice (see k_route_seg): any CTA may be the last
-#pragma unroll 1
-  for (int practice = 1; practice >= 0; practice--) {
-    if (!practice) {
-      uint32_t ph = 0;
-      for (int t0 = 0; t0 < n_tok; t0 += tg, ph ^= 1) {
-        const int nt = min(tg, n_tok - t0);
-        if (t0 > 0) __syncthreads();  // everybody is done with the tokens before
-        if (tid == 0) {
-          const uint32_t xb = (uint32_t)(nt * d * 4);
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(xb) : "memory");
-          if (t0 == 0) pm_pdl_wait();
-          bulk(xs + (size_t)epc * d, x + (size_t)t0 * d, xb);
-        }
-        if (t0 == 0) pm_pdl_wait();
-        {  // bounded: the copies' own time, a few us
-          unsigned long long s0 = 0;
-          for (;;) {
-            uint32_t ok;
-            asm volatile(
-                "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                : "=r"(ok) : "r"(bar), "r"(ph) : "memory");
-            if (ok) break;
-            unsigned long long now;
-            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
-            if (s0 == 0) s0 = now;
-            if (now - s0 > wait_ns) {
-              atomicCAS(err, 0, 9);
-              break;
-            }
-          }
-        }
-        for (int i = warp; i < ne * nt; i += 8) {
-          const int el = i % ne, t = i / ne;
-          const float *w = xs + (size_t)el * d + lane, *xr = xs + (size_t)(epc + t) * d + lane;
-          float acc = 0.0f;
-#pragma unroll 1
-          for (int c = 0; c < (d & ~511); c += 512) {  // 16 columns a lane read at once: one latency for 16 steps of the chain
-            float a[16], b[16];
-#pragma unroll
-            for (int i = 0; i < 16; i++) { a[i] = w[c + 32 * i]; b[i] = xr[c + 32 * i]; }
-#pragma unroll
-            for (int i = 0; i < 16; i++) acc = __fmaf_rn(a[i], b[i], acc);
-          }
-#pragma unroll 1
-          for (int c = d & ~511; c < d; c += 32) acc = __fmaf_rn(w[c], xr[c], acc);
-          float s = pm_warp_sum_dot(acc);
-          if (lane == 0) {
-            if (bias) s = __fadd_rn(s, bias[e0 + el]);
-            logits[(size_t)(t0 + t) * E + e0 + el] = s;
-          }
+  uint32_t ph = 0;
+  for (int t0 = 0; t0 < T; t0 += tg, ph ^= 1) {
+    const int nt = min(tg, T - t0);
+    if (t0 > 0) __syncthreads();  // everybody is done with the tokens before
+    if (tid == 0) {
+      const uint32_t xb = (uint32_t)(nt * d * 4);
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(xb) : "memory");
+      if (t0 == 0) pm_pdl_wait();
+      bulk(xs + (size_t)epc * d, x + (size_t)t0 * d, xb);
+    }
+    if (t0 == 0) pm_pdl_wait();
+    {  // bounded: the copies' own time, a few us
+      unsigned long long s0 = 0;
+      for (;;) {
+        uint32_t ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok) : "r"(bar), "r"(ph) : "memory");
+        if (ok) break;
+        unsigned long long now;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+        if (s0 == 0) s0 = now;
+        if (now - s0 > wait_ns) {
+          atomicCAS(err, 0, 9);
+          break;
         }
       }
-      __threadfence();  // this CTA's logits before its ticket
-      __syncthreads();
-      if (tid == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
-      __syncthreads();
-      if (!s_last) return;
-      __threadfence();
-      if (tid == 0) *ticket = 0;  // ready for the next launch (graph replays included)
     }
-    // ---- the last CTA ----
-    const int per = E + pm_route_scratch(E);  // per token: logits, then its scratch
-    float *sm = practice ? xs + practice_at : xs;
-    const int T = practice ? 1 : n_tok;
-    PlanDev pl = plan;
-    TcTiles tt = tiles;
-    uint32_t *ids = ids_out, *usage = practice ? nullptr : usage_out;
-    float *wout = w_out;
-    if (practice) {
-      uint32_t *nowhere = (uint32_t *)(sm + ((per + 3) & ~3));
-      pm_plan_nowhere(nowhere, pl, tt);
-      ids = nowhere + 512;
-      wout = (float *)nowhere + 512 + PM_MAX_TOPK;
+    for (int i = warp; i < ne * nt; i += 8) {
+      const int el = i % ne, t = i / ne;
+      const float *w = xs + (size_t)el * d + lane, *xr = xs + (size_t)(epc + t) * d + lane;
+      const uint32_t wa = (uint32_t)__cvta_generic_to_shared(w), xa = (uint32_t)__cvta_generic_to_shared(xr);
+      float acc = 0.0f;
+#pragma unroll 1
+      for (int c = 0; c < (d & ~511); c += 512) {  // 16 columns a lane read at once: one latency for 16 steps of the chain
+        float a[16], b[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {  // (volatile: otherwise the compiler reads two at a time to save registers)
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(a[i]) : "r"(wa + 4 * (c + 32 * i)));
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(b[i]) : "r"(xa + 4 * (c + 32 * i)));
+        }
+#pragma unroll
+        for (int i = 0; i < 16; i++) acc = __fmaf_rn(a[i], b[i], acc);
+      }
+#pragma unroll 1
+      for (int c = d & ~511; c < d; c += 32) acc = __fmaf_rn(w[c], xr[c], acc);
+      float s = pm_warp_sum_dot(acc);
+      if (lane == 0) {
+        if (bias) s = __fadd_rn(s, bias[e0 + el]);
+        logits[(size_t)(t0 + t) * E + e0 + el] = s;
+      }
     }
-    const bool soft = D.gating == PM_GATE_SOFTMAX_ALL;
-    for (int t = 0; t < T; t++)
-      for (int e = tid; e < E; e += 256) sm[t * per + e] = practice ? 0.0f : __ldcg(logits + (size_t)t * E + e);
+  }
+  __threadfence();  // this CTA's logits before its ticket
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (tid == 0) *ticket = 0;  // ready for the next launch (graph replays included)
+
+  // ---- the last CTA ----
+  const int per = E + pm_route_scratch(E);  // per token: logits, then its scratch
+  float *sm = xs;
+  const bool soft = D.gating == PM_GATE_SOFTMAX_ALL;
+  for (int t = 0; t < T; t++)
+    for (int e = tid; e < E; e += 256) sm[t * per + e] = __ldcg(logits + (size_t)t * E + e);
+  __syncthreads();
+  if (soft) {
+    if (warp < T) {
+      const float mx = pm_route_max(sm + warp * per, E, lane);
+      if (lane == 0) s_red[warp] = mx;
+    }
     __syncthreads();
-    if (soft) {
-      if (warp < T) {
-        const float mx = pm_route_max(sm + warp * per, E, lane);
-        if (lane == 0) s_red[warp] = mx;
-      }
-      __syncthreads();
+  }
+#pragma unroll 1
+  for (int t = 0; t < T; t++)
+#pragma unroll 1
+    for (int e = tid; e < E; e += 256) {
+      float *lg = sm + t * per;
+      const float p = pm_route_elem(D.gating, lg[e], soft ? s_red[t] : 0.0f);
+      lg[E + e] = p;
+      if (!soft) lg[2 * E + e] = sel_bias ? __fadd_rn(p, sel_bias[e]) : p;
     }
+  __syncthreads();
+  if (soft) {
+    if (warp < T) {
+      const float sum = pm_route_sum(sm + warp * per + E, E, lane);
+      if (lane == 0) s_red[warp] = sum;
+    }
+    __syncthreads();
 #pragma unroll 1
     for (int t = 0; t < T; t++)
 #pragma unroll 1
       for (int e = tid; e < E; e += 256) {
-        float *lg = sm + t * per;
-        const float p = pm_route_elem(D.gating, lg[e], soft ? s_red[t] : 0.0f);
-        lg[E + e] = p;
-        if (!soft) lg[2 * E + e] = sel_bias ? __fadd_rn(p, sel_bias[e]) : p;
+        float *pr = sm + t * per + E;
+        const float p = __fdiv_rn(pr[e], s_red[t]);
+        pr[e] = p;
+        pr[E + e] = sel_bias ? __fadd_rn(p, sel_bias[e]) : p;
       }
-    __syncthreads();
-    if (soft) {
-      if (warp < T) {
-        const float sum = pm_route_sum(sm + warp * per + E, E, lane);
-        if (lane == 0) s_red[warp] = sum;
-      }
-      __syncthreads();
-#pragma unroll 1
-      for (int t = 0; t < T; t++)
-#pragma unroll 1
-        for (int e = tid; e < E; e += 256) {
-          float *pr = sm + t * per + E;
-          const float p = __fdiv_rn(pr[e], s_red[t]);
-          pr[e] = p;
-          pr[E + e] = sel_bias ? __fadd_rn(p, sel_bias[e]) : p;
-        }
-      __syncthreads();
-    }
-    if (warp < T) {
-      float *pr = sm + warp * per + E;
-      pm_route_pick(D, pr, pr + E, pr + 2 * E, lane, ids + (size_t)warp * K, wout + (size_t)warp * K);
-    }
-    __syncthreads();
-    // ---- the plan of the P = T * K pairs (src/moe_kernels.rs:1083-1129 layout) ----
-    const int P = T * K;
-    uint32_t mine = 0;
-    if (tid < P) {
-      mine = ids[tid];  // written by this CTA's warps above
-      if (slot_table && !practice) {  // a placement table: everything from here on names slots; use is counted by expert
-        if (usage) atomicAdd(&usage[mine], 1u);
-        mine = (uint32_t)slot_table[mine];
-        ids[tid] = mine;
-      }
-      s_ids[tid] = mine;
-    }
-    __syncthreads();
-    if (tid < P) {  // pairs by expert, an expert's pairs in their order
-      uint32_t less = 0, before = 0;
-#pragma unroll 4
-      for (int j = 0; j < P; j++) {
-        const uint32_t o = s_ids[j];
-        less += o < mine;
-        before += o == mine && j < tid;
-      }
-      s_new[tid] = before == 0;
-      const uint32_t p = less + before;
-      pl.pair_pos[tid] = p;
-      pl.pair_token[p] = (uint32_t)(tid / K);
-      pl.pair_src[p] = (uint32_t)tid;
-    }
-    __syncthreads();
-    uint32_t n_active = 0;
-#pragma unroll 1
-    for (int e = tid; e < E; e += 256) {
-      uint32_t less = 0, c = 0, na = 0, active = 0;
-#pragma unroll 4
-      for (int j = 0; j < P; j++) {
-        const uint32_t o = s_ids[j], nw = s_new[j];
-        less += o < (uint32_t)e;
-        c += o == (uint32_t)e;
-        na += o < (uint32_t)e ? nw : 0u;
-        active += nw;
-      }
-      pl.base[e] = less;
-      pl.cnt[e] = c;
-      if ((uint32_t)e >= active) {
-        pl.active[e] = 0;
-        pl.offset[e] = 0;
-        pl.count[e] = 0;
-      }
-      if (c) {
-        pl.active[na] = (uint32_t)e;
-        pl.offset[na] = less;
-        pl.count[na] = c;
-        if (usage && !slot_table) usage[e] += c;
-        if (tt.tiles) {  // (a group has fewer than 16 pairs: one tile each)
-          const int el = e - first_local;
-          tt.tiles[na] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, less, c, 16 * na);
-        }
-      }
-      n_active = active;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      *pl.n_active = (int)n_active + (tt.shared ? 1 : 0);
-      if (tt.tiles) {
-        if (tt.shared) {  // the shared expert as one more group: every token, pairs P .. P + T - 1
-          pl.offset[n_active] = P;
-          pl.count[n_active] = T;
-          tt.tiles[n_active] = make_uint4(TC_SHARED, P, T, 16 * n_active);
-        }
-        tt.n[0] = (int)n_active + (tt.shared ? 1 : 0);
-        tt.next[0] = tt.next[1] = 0;
-      }
-    }
-    if (tt.shared && tid < T) pl.pair_token[P + tid] = (uint32_t)tid;
     __syncthreads();
   }
+  if (warp < T) {
+    float *pr = sm + warp * per + E;
+    pm_route_pick(D, pr, pr + E, pr + 2 * E, lane, ids + (size_t)warp * K, wout + (size_t)warp * K);
+  }
+  __syncthreads();
+  // ---- the plan of the P = T * K pairs (src/moe_kernels.rs:1083-1129 layout) ----
+  const int P = T * K;
+  uint32_t mine = 0;
+  if (tid < P) {
+    mine = ids[tid];  // written by this CTA's warps above
+    if (slot_table) {  // a placement table: everything from here on names slots; use is counted by expert
+      if (usage) atomicAdd(&usage[mine], 1u);
+      mine = (uint32_t)slot_table[mine];
+      ids[tid] = mine;
+    }
+    s_ids[tid] = mine;
+  }
+  __syncthreads();
+  if (tid < P) {  // pairs by expert, an expert's pairs in their order
+    uint32_t less = 0, before = 0;
+#pragma unroll 4
+    for (int j = 0; j < P; j++) {
+      const uint32_t o = s_ids[j];
+      less += o < mine;
+      before += o == mine && j < tid;
+    }
+    s_new[tid] = before == 0;
+    const uint32_t p = less + before;
+    pl.pair_pos[tid] = p;
+    pl.pair_token[p] = (uint32_t)(tid / K);
+    pl.pair_src[p] = (uint32_t)tid;
+  }
+  __syncthreads();
+  uint32_t n_active = 0;
+#pragma unroll 1
+  for (int e = tid; e < E; e += 256) {
+    uint32_t less = 0, c = 0, na = 0, active = 0;
+#pragma unroll 4
+    for (int j = 0; j < P; j++) {
+      const uint32_t o = s_ids[j], nw = s_new[j];
+      less += o < (uint32_t)e;
+      c += o == (uint32_t)e;
+      na += o < (uint32_t)e ? nw : 0u;
+      active += nw;
+    }
+    pl.base[e] = less;
+    pl.cnt[e] = c;
+    if ((uint32_t)e >= active) {
+      pl.active[e] = 0;
+      pl.offset[e] = 0;
+      pl.count[e] = 0;
+    }
+    if (c) {
+      pl.active[na] = (uint32_t)e;
+      pl.offset[na] = less;
+      pl.count[na] = c;
+      if (usage && !slot_table) usage[e] += c;
+      if (tt.tiles) {  // (a group has fewer than 16 pairs: one tile each)
+        const int el = e - first_local;
+        tt.tiles[na] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, less, c, 16 * na);
+      }
+    }
+    n_active = active;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    *pl.n_active = (int)n_active + (tt.shared ? 1 : 0);
+    if (tt.tiles) {
+      if (tt.shared) {  // the shared expert as one more group: every token, pairs P .. P + T - 1
+        pl.offset[n_active] = P;
+        pl.count[n_active] = T;
+        tt.tiles[n_active] = make_uint4(TC_SHARED, P, T, 16 * n_active);
+      }
+      tt.n[0] = (int)n_active + (tt.shared ? 1 : 0);
+      tt.next[0] = tt.next[1] = 0;
+    }
+  }
+  if (tt.shared && tid < T) pl.pair_token[P + tid] = (uint32_t)tid;
 }
 
 // whether launch_route_plan_small takes T tokens of this layer: a router row and a token's row have to fit shared memory
@@ -1129,14 +1116,12 @@ void launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x
   const int per = E + pm_route_scratch(E);               // the last CTA's scratch
   int smem = (epc + tg) * d * 4;
   if (T * per * 4 > smem) smem = T * per * 4;
-  const int practice_at = (smem + 15) / 16 * 4;
-  smem = (practice_at + per + 512 + 2 * PM_MAX_TOPK + 4) * 4;
   static int smem_set = 0;
   if (smem > smem_set) {  // (raised on a layer's first call, which is never inside a stream capture)
     cudaFuncSetAttribute(k_route_plan_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     smem_set = smem;
   }
-  PLAUNCH(L, k_route_plan_small, (E + epc - 1) / epc, 256, smem, ly.desc, ly.router, ly.logit_bias, ly.select_bias, x, T, epc, tg, practice_at,
+  PLAUNCH(L, k_route_plan_small, (E + epc - 1) / epc, 256, smem, ly.desc, ly.router, ly.logit_bias, ly.select_bias, x, T, epc, tg,
           logits, ids, w, pl, ly.usage, slot_table, ticket, tt, ly.first_local, ly.n_local, err, wait_ns);
 }
 
@@ -1850,14 +1835,18 @@ void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int
 // combine (src/moe_kernels.rs:1798-1808): fixed k order, then the shared expert
 // ===========================================================================
 // (four columns a thread: 16-byte reads, all K of them in flight; 4096 tokens x 8 x 7168: 256 -> 190 us, 1.06 GB)
+// PARTS: products cut along K, up to four parts a pair (read whole, a part more than once where there are fewer: the
+// reads of a pair are all in flight together; one token x 4 x 2880 in three parts 8.7 us of waiting for one after the other)
+template <bool PARTS>
 __global__ void __launch_bounds__(256) k_combine(int d, int K, int in_combine,
                                                  const float *__restrict__ eo,
                                                  const uint32_t *__restrict__ pair_pos,
                                                  const float *__restrict__ w,
                                                  const float *__restrict__ shared_out,
                                                  const float *__restrict__ shared_logit, float *y,
-                                                 int accumulate, int parts, size_t part_stride) {
-  pm_pdl();
+                                                 int accumulate, int parts, size_t part_stride, int early) {
+  if (early) pm_pdl_early();
+  else pm_pdl();
   const int t = blockIdx.y;
   const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
   if (c >= d) return;
@@ -1865,13 +1854,19 @@ __global__ void __launch_bounds__(256) k_combine(int d, int K, int in_combine,
 #pragma unroll 8
   for (int k = 0; k < K; k++) {
     const uint32_t p = pair_pos[t * K + k];
-    float4 v = p == PM_PAIR_NONE ? make_float4(0.0f, 0.0f, 0.0f, 0.0f)  // a pair whose expert id was refused
-                                 : __ldcs((const float4 *)(eo + (size_t)p * d + c));
-    for (int i = 1; i < parts; i++) {  // (products cut along K: the other parts of the sum)
-      if (p == PM_PAIR_NONE) break;
-      const float4 u = __ldcs((const float4 *)(eo + i * part_stride + (size_t)p * d + c));
-      v = make_float4(__fadd_rn(v.x, u.x), __fadd_rn(v.y, u.y), __fadd_rn(v.z, u.z), __fadd_rn(v.w, u.w));
+    // (a pair whose expert id was refused: row 0 read in its place, no branch between the reads)
+    const float *src = eo + (size_t)(p == PM_PAIR_NONE ? 0u : p) * d + c;
+    float4 v = __ldcs((const float4 *)src);
+    if (PARTS) {
+      float4 u[3];
+#pragma unroll
+      for (int i = 0; i < 3; i++) u[i] = __ldcs((const float4 *)(src + min(i + 1, parts - 1) * part_stride));
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+        if (i + 1 < parts)
+          v = make_float4(__fadd_rn(v.x, u[i].x), __fadd_rn(v.y, u[i].y), __fadd_rn(v.z, u[i].z), __fadd_rn(v.w, u[i].w));
     }
+    if (p == PM_PAIR_NONE) v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (in_combine) {
       const float wk = w[t * K + k];
       v = make_float4(__fmul_rn(wk, v.x), __fmul_rn(wk, v.y), __fmul_rn(wk, v.z), __fmul_rn(wk, v.w));
@@ -1901,9 +1896,17 @@ void launch_combine(const Launch &L, const LayerDev &ly, const float *eo, const 
   if (T == 0) return;
   int d = ly.desc.d;
   dim3 grid((d + 1023) / 1024, T);
-  PLAUNCH(L, k_combine, grid, 256, 0, d, ly.desc.top_k,
-          (int)(ly.desc.weight_fold == PM_FOLD_IN_COMBINE), eo, pair_pos, w, shared_out,
-          shared_logit, y, (int)accumulate, parts, (size_t)T * ly.desc.top_k * d);
+  // (a few tokens: the next layer's routing kernel fetches its rows meanwhile where they are a few us of HBM, 256 experts x
+  // 7168: 102 -> 97 us a layer)
+  const int early = T < PM_SMALL_ROUTE_TOKENS && (size_t)ly.desc.n_exp * d * 4 > (4u << 20);
+  if (parts > 1)
+    PLAUNCH(L, k_combine<true>, grid, 256, 0, d, ly.desc.top_k,
+            (int)(ly.desc.weight_fold == PM_FOLD_IN_COMBINE), eo, pair_pos, w, shared_out,
+            shared_logit, y, (int)accumulate, parts, (size_t)T * ly.desc.top_k * d, early);
+  else
+    PLAUNCH(L, k_combine<false>, grid, 256, 0, d, ly.desc.top_k,
+            (int)(ly.desc.weight_fold == PM_FOLD_IN_COMBINE), eo, pair_pos, w, shared_out,
+            shared_logit, y, (int)accumulate, parts, (size_t)T * ly.desc.top_k * d, early);
 }
 
 // x / rms(x), unit weight; the sum order is pm_rms_inv's (common.cuh)
