@@ -49,9 +49,9 @@ __device__ __forceinline__ void mx_mma_ta(uint32_t tmem_c, uint32_t tmem_a, uint
 }
 
 // A block: 16 bytes of E2M1 codes (value j in the low nibble of byte j, value j + 16 in the high one) and its E8M0
-// scale e -> 32 bf16. Two codes a word, 16 bits apart, in the order they lie in: word 4 j + i is nibbles i and i + 4
-// of the j-th word, the values (4 j, 4 j + 2), (16 + 4 j, 18 + 4 j), (4 j + 1, 4 j + 3), (17 + 4 j, 19 + 4 j) for
-// i = 0 .. 3 (k_mx_rows puts the tokens' values into the same order). The code's three magnitude bits at bits 8..6 of
+// scale e -> 32 bf16. Two codes a word, 16 bits apart as they lie: word 2 j holds nibbles 0 and 4 of the j-th word (values
+// 4 j, 4 j + 2), word 2 j + 1 nibbles 2 and 6 (4 j + 1, 4 j + 3), words 8 .. the same of the high nibbles (values 16 ..);
+// k_mx_rows puts the tokens' values into the same order. The code's three magnitude bits at bits 8..6 of
 // a bf16 are the code times 2^-126 (its subnormal included), so one multiplication by 2^(e - 1) makes the value; four
 // ALU instructions and a multiplication a word, where look-ups of both bytes by prmt took ten (and the prmt, shifts
 // and logic, 64 lanes a cycle, were what the workers waited for: 2,070 -> 1,150 cycles a chunk).
@@ -64,10 +64,10 @@ __device__ __forceinline__ void mx_codes(const uint4 q, uint32_t scale2, uint32_
   const uint32_t v[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
   for (int j = 0; j < 4; j++) {
-    w[4 * j] = mx_mul2(((v[j] << 6) & 0x01c001c0u) | ((v[j] << 12) & 0x80008000u), scale2);
-    w[4 * j + 1] = mx_mul2(((v[j] << 2) & 0x01c001c0u) | ((v[j] << 8) & 0x80008000u), scale2);
-    w[4 * j + 2] = mx_mul2(((v[j] >> 2) & 0x01c001c0u) | ((v[j] << 4) & 0x80008000u), scale2);
-    w[4 * j + 3] = mx_mul2(((v[j] >> 6) & 0x01c001c0u) | (v[j] & 0x80008000u), scale2);
+    w[2 * j] = mx_mul2(((v[j] << 6) & 0x01c001c0u) | ((v[j] << 12) & 0x80008000u), scale2);
+    w[8 + 2 * j] = mx_mul2(((v[j] << 2) & 0x01c001c0u) | ((v[j] << 8) & 0x80008000u), scale2);
+    w[2 * j + 1] = mx_mul2(((v[j] >> 2) & 0x01c001c0u) | ((v[j] << 4) & 0x80008000u), scale2);
+    w[8 + 2 * j + 1] = mx_mul2(((v[j] >> 6) & 0x01c001c0u) | (v[j] & 0x80008000u), scale2);
   }
 }
 // scales outside 2 .. 128
@@ -82,7 +82,10 @@ __device__ __forceinline__ void mx_codes_any(const uint4 q, uint32_t e, uint32_t
     const float s = pm_e8(e);
     auto cv = [&](uint32_t c) { return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(s, pm_e2m1(c & 15u)))); };
 #pragma unroll
-    for (int i = 0; i < 16; i++) w[i] = cv(v[i >> 2] >> (4 * (i & 3))) | (cv(v[i >> 2] >> (4 * (i & 3) + 16)) << 16);
+    for (int i = 0; i < 16; i++) {  // word i: nibbles n and n + 4 of word j
+      const int j = (i & 7) >> 1, n = 2 * (i & 1) + (i >> 3);
+      w[i] = cv(v[j] >> (4 * n)) | (cv(v[j] >> (4 * n + 16)) << 16);
+    }
   }
 }
 
@@ -107,9 +110,9 @@ struct MxArgs {
 };
 
 // f32 rows -> the products' operand: per tile and chunk of 64 K values [piece][8 K groups][rows][8 bf16], rows padded
-// to 16 with zeros; a K group of 8 is values 4 j .. 4 j + 3 and 16 + 4 j .. of a block of 32, in the order the decoded
-// weights have. A thread a (row, K group): neighbouring lanes take neighbouring rows, whose 16 bytes are neighbours
-// in the operand.
+// to 16 with zeros; the 8 values of a K group in the order the decoded weights have (0, 2, 1, 3, 4, 6, 5, 7). A thread a
+// (row, K group): neighbouring lanes take neighbouring rows, whose 16 bytes are neighbours in the operand (their
+// 32-byte reads are whole sectors).
 __global__ void __launch_bounds__(256) k_mx_rows(const int *__restrict__ n_tiles, const uint4 *__restrict__ tiles,
                                                  const uint32_t *__restrict__ src_row, int cols, const float *__restrict__ x,
                                                  uint8_t *__restrict__ rec) {
@@ -123,9 +126,9 @@ __global__ void __launch_bounds__(256) k_mx_rows(const int *__restrict__ n_tiles
     float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     if (r < (int)T.z && 8 * g < cols) {
       const size_t row = src_row ? src_row[T.y + r] : T.y + r;
-      const float4 *src = (const float4 *)(x + row * cols + (g >> 2) * 32 + (g & 3) * 4);
-      const float4 a = __ldg(src), b = __ldg(src + 4);  // (the order of mx_decode_block)
-      v[0] = a.x; v[1] = a.z; v[2] = b.x; v[3] = b.z; v[4] = a.y; v[5] = a.w; v[6] = b.y; v[7] = b.w;
+      const float4 *src = (const float4 *)(x + row * cols + 8 * g);
+      const float4 a = __ldg(src), b = __ldg(src + 1);  // (the order of mx_codes)
+      v[0] = a.x; v[1] = a.z; v[2] = a.y; v[3] = a.w; v[4] = b.x; v[5] = b.z; v[6] = b.y; v[7] = b.w;
     }
     uint8_t *dst = base + (size_t)(g >> 3) * (npad * MX_KC * 2 * NPC) + ((g & 7) * npad + r) * 16;
 #pragma unroll
