@@ -392,7 +392,9 @@ __global__ void __launch_bounds__(256) k_router(const float *__restrict__ wr,
 // (EW * TW accumulators a lane); 128 columns of its experts' and tokens' rows at a time come into shared memory
 // by cp.async, three stages. Lane L still runs, for every (token, expert), the fma chain over columns L,
 // L + 32, ... in ascending order, so the result has the bits of k_router.
-// 16 x 8 (128 fma for 24 shared-memory reads a column): bound by the FP32 pipe. 8 x 4 while tiles of the first size
+// 16 x 8, two experts an instruction (64 fma.f32x2 for 24 shared-memory reads a column: one fma an instruction took
+// every issue slot, two leave the reads half of them; the same roundings;
+// 4096 tokens on 256 experts x 7168 490 -> 437 us, and 8 x 4 loses by it, 18 -> 20 us): bound by the FP32 pipe. 8 x 4 while tiles of the first size
 // would leave most SMs without one.
 // (before: rows from L2 straight into the fma, 8 x 8 tiles: 4096 tokens on 256 experts x 7168 916 us, the pipe's bound
 // 210 us; 64 tokens 75 us; 512 tokens on 128 experts x 2048 29 us)
@@ -402,7 +404,8 @@ template <int EW, int TW> __global__ void __launch_bounds__(256, 1) k_router_til
                                                                                  const float *__restrict__ bias,
                                                                                  const float *__restrict__ x, int T, int E,
                                                                                  int d, float *logits) {
-  pm_pdl();
+  if (T <= 32) pm_pdl_early();  // (the one CTA of the routing kernel behind practises meanwhile)
+  else pm_pdl();
   constexpr int RE = 2 * EW, RT = 4 * TW, ROWS = RE + RT;  // rows of a stage: experts, then tokens
   extern __shared__ __align__(16) float rs[];              // [RT_ST][ROWS][RT_CH]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -422,11 +425,16 @@ template <int EW, int TW> __global__ void __launch_bounds__(256, 1) k_router_til
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  constexpr bool PAIRS = EW == 16;
   float acc[TW][EW];
+  uint64_t acc2[TW][EW / 2];  // PAIRS: experts 2 e, 2 e + 1
 #pragma unroll
-  for (int t = 0; t < TW; t++)
+  for (int t = 0; t < TW; t++) {
 #pragma unroll
     for (int e = 0; e < EW; e++) acc[t][e] = 0.0f;
+#pragma unroll
+    for (int e = 0; e < EW / 2; e++) acc2[t][e] = 0;
+  }
 #pragma unroll
   for (int ch = 0; ch < RT_ST - 1; ch++) load(ch);
   for (int ch = 0; ch < nch; ch++) {
@@ -436,16 +444,37 @@ template <int EW, int TW> __global__ void __launch_bounds__(256, 1) k_router_til
     const float *S = rs + (size_t)(ch % RT_ST) * ROWS * RT_CH + lane;
     const int n = min(RT_CH, d - ch * RT_CH) / 32;  // (d is a multiple of 32)
     for (int s = 0; s < n; s++) {
-      float w[EW], xv[TW];
+      float xv[TW];
+      if constexpr (PAIRS) {
+        uint64_t w2[EW / 2];
 #pragma unroll
-      for (int e = 0; e < EW; e++) w[e] = S[(we + e) * RT_CH + 32 * s];
+        for (int e = 0; e < EW / 2; e++) w2[e] = pm_pack2(S[(we + 2 * e) * RT_CH + 32 * s], S[(we + 2 * e + 1) * RT_CH + 32 * s]);
 #pragma unroll
-      for (int t = 0; t < TW; t++) xv[t] = S[(RE + wt + t) * RT_CH + 32 * s];
+        for (int t = 0; t < TW; t++) xv[t] = S[(RE + wt + t) * RT_CH + 32 * s];
 #pragma unroll
-      for (int t = 0; t < TW; t++)
+        for (int t = 0; t < TW; t++) {
+          const uint64_t x2 = pm_pack2(xv[t], xv[t]);
 #pragma unroll
-        for (int e = 0; e < EW; e++) acc[t][e] = __fmaf_rn(w[e], xv[t], acc[t][e]);
+          for (int e = 0; e < EW / 2; e++) acc2[t][e] = pm_fma2(w2[e], x2, acc2[t][e]);
+        }
+      } else {
+        float w[EW];
+#pragma unroll
+        for (int e = 0; e < EW; e++) w[e] = S[(we + e) * RT_CH + 32 * s];
+#pragma unroll
+        for (int t = 0; t < TW; t++) xv[t] = S[(RE + wt + t) * RT_CH + 32 * s];
+#pragma unroll
+        for (int t = 0; t < TW; t++)
+#pragma unroll
+          for (int e = 0; e < EW; e++) acc[t][e] = __fmaf_rn(w[e], xv[t], acc[t][e]);
+      }
     }
+  }
+  if constexpr (PAIRS) {
+#pragma unroll
+    for (int t = 0; t < TW; t++)
+#pragma unroll
+      for (int e = 0; e < EW / 2; e++) pm_unpack2(acc2[t][e], acc[t][2 * e], acc[t][2 * e + 1]);
   }
   // lane sums in pm_warp_sum_dot's order (xor 8, 16, 4, 2, 1), 32 of them at once: every step halves the sums a lane
   // carries, 31 shuffles in place of 160; lane L ends with sum (bit 3, bit 4, bit 2, bit 1, bit 0 of L)
@@ -765,7 +794,7 @@ __global__ void __launch_bounds__(1024) k_route_seg(pm_layer_desc D, const float
   uint32_t *s_id = (uint32_t *)rsm, *cnt = s_id + 512;
   float *sc = rsm + 512 + E + wi * pm_route_scratch(E);
 #pragma unroll 1
-  for (int practice = 1; practice >= 0; practice--) {
+  for (int practice = gridDim.x <= 4; practice >= 0; practice--) {  // (many CTAs: they would take the SMs from the router)
     PlanDev p = pl;
     TcTiles q = tt;
     const int t = blockIdx.x * PL_SEG + wi;

@@ -531,8 +531,10 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
     // 64 q .. 64 q + 63 = TMEM columns 16 q .. 16 q + 15 of each plane. The same thread adds row m's float terms
     // (TMEM lane m) for its part of a pass's token columns, so the row's (d, dmin) stay in registers.
     constexpr int QN = 4 / PARTS;  // quarters a thread
-    const int m = tid & 127, part = warp >> 2;
-    const uint32_t tlane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    // (redux results live in uniform registers, as the addresses of tensor memory have to: large tiles 1 to 2 % faster,
+    // and the small shape, which has other registers to spare, slower)
+    const int m = tid & 127, part = PARTS == 4 ? (int)__reduce_max_sync(PM_FULL, (unsigned)warp >> 2) : warp >> 2;
+    const uint32_t tlane = tmem + (PARTS == 4 ? __reduce_max_sync(PM_FULL, 32u * (warp & 3)) << 16 : (uint32_t)(32 * (warp & 3)) << 16);
     const float nz = __uint_as_float((uint32_t)A.neg_zero2);
     const uint64_t nz2 = tc_pack2(nz, nz);
     uint32_t gb = 0, gp = 0;  // blocks whose operand A this CTA has stored, passes whose float terms it has added
