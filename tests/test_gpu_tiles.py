@@ -54,3 +54,28 @@ def test_mxfp4(ctx, oracle, shape, T):
         rms = float(np.sqrt((want.astype(np.float64) ** 2).mean()))
         assert float(np.abs(got - want).max()) < 4e-6 * rms
     gl.close()
+
+
+@pytest.mark.parametrize("T", [1, 7, 8, 9, 32, 33, 70, 130, 260])
+@pytest.mark.parametrize("shape", ["c1", "c2", "c4", "c4-shard"])
+def test_q8x_blocks_and_plan(ctx, oracle, shape, T):
+    """Q4_K / Q6_K products in both shapes of the kernel (2 to 130 pairs a group: one to four passes, tiles that are
+    full and one over), the shared expert as a group of the same launches; routing and plan on either side of
+    8 tokens (one launch / a router of tiles) and of 32 (one segment / several): bits of the oracle."""
+    cfg = SMALL["c4"].scaled(first_local_expert=8, n_exp_local=16) if shape == "c4-shard" else SMALL[shape]
+    ol, gl, _ = make_pair(oracle, pb, ctx, cfg, 83)
+    x = synth.make_activations(T, cfg.d, 970 + T)
+    ids, w = gl.route(x)
+    ids_o, w_o = ol.route(x)
+    assert np.array_equal(ids, ids_o) and bits_equal(w, w_o)
+    assert bits_equal(gl.forward(x), ol.forward(x))
+    # rows that start 4 bytes off a 16-byte boundary take other loads, not other values
+    xd, yd = ctx.alloc(x.nbytes + 16), ctx.alloc(x.nbytes + 16)
+    xd.upload(np.concatenate([np.zeros(1, np.float32), x.ravel(), np.zeros(3, np.float32)]))
+    pb._check(gl.lib.pm_moe_forward(gl.h, xd.ptr + 4, T, yd.ptr + 4, 0))
+    ctx.sync()
+    got = yd.download(np.float32, (x.size + 4,))[1:1 + x.size].reshape(x.shape)
+    assert bits_equal(got, ol.forward(x))
+    xd.free()
+    yd.free()
+    gl.close()
