@@ -13,7 +13,10 @@
 //
 // A persistent pipeline as in prefill_mx.cu; two CTAs an SM, 128 weight rows (64 of gate and 64 of up, or 128 of down) x
 // 16 tokens (5 pieces) or 32 (4). Rows of gate and up alternate in tensor memory, so the two sums of an output are
-// neighbouring lanes. Bound by the weights' bytes.
+// neighbouring lanes. Bound by the
+// latency of a stage's steps (wait, copy, fence, products, fold: 900 cycles for 128 K values, two CTAs interleave): 31 tokens on
+// 32 experts, d = ff = 2880, 2.8 TB/s of weights; gate/up + down 223 us decoding to bf16, 149 here; 1 token 58 us on the row
+// kernels, 37 here.
 #include <cuda_fp16.h>
 
 #include "tcgen.cuh"
