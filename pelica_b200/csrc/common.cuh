@@ -252,6 +252,9 @@ __device__ __forceinline__ void pm_pdl() {
   pm_pdl_wait();
   pm_pdl_trigger();
 }
+// A small grid runs its body once for practice - on made-up values, storing nothing - while it waits for the kernel before:
+// an instruction that is executed once and cold costs some 30 cycles.
+#define PM_PRACTICE_CTAS 296
 // ... at once: for kernels in front of one that fetches its weights while it waits (k_route_plan_small)
 __device__ __forceinline__ void pm_pdl_early() {
   pm_pdl_trigger();

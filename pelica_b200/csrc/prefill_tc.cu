@@ -159,84 +159,92 @@ __global__ void __launch_bounds__(512) k_tc_tiles(Groups g, int first_local, int
 __global__ void __launch_bounds__(256) k_tc_quant_rows(const int *__restrict__ n_tiles, const uint4 *__restrict__ tiles,
                                                        const uint32_t *__restrict__ src_row, int cols,
                                                        const float *__restrict__ x, uint8_t *__restrict__ rec) {
-  pm_pdl();
   __shared__ __align__(16) uint8_t s_rec[8][TC_REC];
-  if ((int)blockIdx.y >= *n_tiles) return;
-  const uint4 T = tiles[blockIdx.y];
-  const int nb = cols / 256;
-  const uint32_t off = T.y, cnt = T.z;
-  const int lane = threadIdx.x & 31;
-  uint8_t *S = s_rec[threadIdx.x >> 5];
-  const int nrg = (int)((cnt + 15u) / 16u) * 2, units = nrg * nb;  // (row group, block) pairs of this tile
-  uint8_t *rec0 = rec + (size_t)(T.w >> 3) * nb * TC_REC;
-  for (int u = blockIdx.x * 8 + (threadIdx.x >> 5); u < units; u += gridDim.x * 8) {
-    const int b = u / nrg, rgl = u - b * nrg;  // (the tile's records lie block by block)
-    // lane = values 8 lane .. 8 lane + 7 of every row, as two words a row
-    uint32_t q[8][2];
+#pragma unroll 1
+  for (int practice = gridDim.x * gridDim.y <= PM_PRACTICE_CTAS; practice >= 0; practice--) {
+    uint4 T = make_uint4(0, 0, 0, 0);
+    if (!practice) {
+      pm_pdl();
+      if ((int)blockIdx.y >= *n_tiles) return;
+      T = tiles[blockIdx.y];
+    }
+    const int nb = cols / 256;
+    const uint32_t off = T.y, cnt = T.z;
+    const int lane = threadIdx.x & 31;
+    uint8_t *S = s_rec[threadIdx.x >> 5];
+    const int nrg = (int)((cnt + 15u) / 16u) * 2, units = practice ? 8 : nrg * nb;  // (row group, block) pairs of this tile
+    uint8_t *rec0 = rec + (size_t)(T.w >> 3) * nb * TC_REC;
+    for (int u = practice ? (int)(threadIdx.x >> 5) : (int)(blockIdx.x * 8 + (threadIdx.x >> 5)); u < units; u += gridDim.x * 8) {
+      const int b = u / max(nrg, 1), rgl = u - b * nrg;  // (the tile's records lie block by block)
+      // lane = values 8 lane .. 8 lane + 7 of every row, as two words a row
+      uint32_t q[8][2];
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      float v[4][8];
+      for (int h = 0; h < 2; h++) {
+        float v[4][8];
 #pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const uint32_t i = (uint32_t)(rgl * 8 + 4 * h + r);
-        if (i < cnt) {
-          const size_t row = src_row ? src_row[off + i] : off + i;
-          const float4 *src = (const float4 *)(x + row * cols + (size_t)b * 256 + 8 * lane);
-          const float4 p = __ldg(src), w = __ldg(src + 1);
-          v[r][0] = p.x; v[r][1] = p.y; v[r][2] = p.z; v[r][3] = p.w;
-          v[r][4] = w.x; v[r][5] = w.y; v[r][6] = w.z; v[r][7] = w.w;
-        } else {
+        for (int r = 0; r < 4; r++) {
+          const uint32_t i = (uint32_t)(rgl * 8 + 4 * h + r);
+          if (i < cnt) {
+            const size_t row = src_row ? src_row[off + i] : off + i;
+            const float4 *src = (const float4 *)(x + row * cols + (size_t)b * 256 + 8 * lane);
+            const float4 p = __ldg(src), w = __ldg(src + 1);
+            v[r][0] = p.x; v[r][1] = p.y; v[r][2] = p.z; v[r][3] = p.w;
+            v[r][4] = w.x; v[r][5] = w.y; v[r][6] = w.z; v[r][7] = w.w;
+          } else {
 #pragma unroll
-          for (int j = 0; j < 8; j++) v[r][j] = 0.0f;
+            for (int j = 0; j < 8; j++) v[r][j] = practice ? 1.0f : 0.0f;
+          }
+        }
+        float mx[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          float m = 0.0f;
+#pragma unroll
+          for (int j = 0; j < 8; j++) m = fmaxf(m, fabsf(v[r][j]));
+          mx[r] = __uint_as_float(__reduce_max_sync(PM_FULL, __float_as_uint(m)));  // (non-negative floats order like integers)
+        }
+        // lane r divides for row r
+        const float mine = lane == 0 ? mx[0] : (lane == 1 ? mx[1] : (lane == 2 ? mx[2] : mx[3]));
+        const float idv = mine != 0.0f ? __fdiv_rn(127.0f, mine) : 0.0f;
+        if (lane < 4) *(float *)(S + TC_REC_XD + (4 * h + lane) * 4) = mine != 0.0f ? __fdiv_rn(mine, 127.0f) : 0.0f;
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          const int r8 = 4 * h + r;
+          pm_q8_pack8(v[r], __shfl_sync(PM_FULL, idv, r), q[r8][0], q[r8][1]);
+          int s = __dp4a((int)q[r8][1], 0x01010101, __dp4a((int)q[r8][0], 0x01010101, 0));
+          s += __shfl_xor_sync(PM_FULL, s, 1);  // the sum of 32 values: lanes 4 j .. 4 j + 3 hold group j
+          s += __shfl_xor_sync(PM_FULL, s, 2);
+          if ((lane & 3) == 0) {  // s = 64 * (s >> 6) + (s & 63), both parts exact in f16
+            __half *bm = (__half *)(S + TC_REC_BM + r8 * 16) + (lane >> 2);
+            bm[0] = __int2half_rn((s >> 6) * 64);
+            bm[64] = __int2half_rn(s & 63);
+          }
+          const int tot = __reduce_add_sync(PM_FULL, s);  // (four times the block's sum)
+          if (lane == 0) *(int32_t *)(S + TC_REC_XS + r8 * 4) = -4128 * tot;
         }
       }
-      float mx[4];
+      // K chunk c = lane / 2 holds 16 bytes of each row: an even lane takes rows 0-3 whole, its odd neighbour
+      // rows 4-7 (64 consecutive bytes of the record each); to shared memory without bank conflicts
+      const bool odd = lane & 1;
 #pragma unroll
-      for (int r = 0; r < 4; r++) {
-        float m = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 8; j++) m = fmaxf(m, fabsf(v[r][j]));
-        mx[r] = __uint_as_float(__reduce_max_sync(PM_FULL, __float_as_uint(m)));  // (non-negative floats order like integers)
+      for (int i = 0; i < 4; i++) {
+        const uint32_t s0 = odd ? q[i][0] : q[4 + i][0], s1 = odd ? q[i][1] : q[4 + i][1];
+        const uint32_t t0 = __shfl_xor_sync(PM_FULL, s0, 1), t1 = __shfl_xor_sync(PM_FULL, s1, 1);
+        const uint4 o = odd ? make_uint4(t0, t1, q[4 + i][0], q[4 + i][1]) : make_uint4(q[i][0], q[i][1], t0, t1);
+        *(uint4 *)(S + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) = o;
       }
-      // lane r divides for row r
-      const float mine = lane == 0 ? mx[0] : (lane == 1 ? mx[1] : (lane == 2 ? mx[2] : mx[3]));
-      const float idv = mine != 0.0f ? __fdiv_rn(127.0f, mine) : 0.0f;
-      if (lane < 4) *(float *)(S + TC_REC_XD + (4 * h + lane) * 4) = mine != 0.0f ? __fdiv_rn(mine, 127.0f) : 0.0f;
+      __syncwarp();
+      uint4 *R = (uint4 *)(rec0 + (size_t)u * TC_REC);
+      if (!practice) {
 #pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const int r8 = 4 * h + r;
-        pm_q8_pack8(v[r], __shfl_sync(PM_FULL, idv, r), q[r8][0], q[r8][1]);
-        int s = __dp4a((int)q[r8][1], 0x01010101, __dp4a((int)q[r8][0], 0x01010101, 0));
-        s += __shfl_xor_sync(PM_FULL, s, 1);  // the sum of 32 values: lanes 4 j .. 4 j + 3 hold group j
-        s += __shfl_xor_sync(PM_FULL, s, 2);
-        if ((lane & 3) == 0) {  // s = 64 * (s >> 6) + (s & 63), both parts exact in f16
-          __half *bm = (__half *)(S + TC_REC_BM + r8 * 16) + (lane >> 2);
-          bm[0] = __int2half_rn((s >> 6) * 64);
-          bm[64] = __int2half_rn(s & 63);
+        for (int k = 0; k < 4; k++) {
+          const int p = 32 * k + lane, l = p >> 2;
+          R[p] = *(const uint4 *)(S + l * 64 + (((p & 3) ^ ((l >> 1) & 3)) << 4));
         }
-        const int tot = __reduce_add_sync(PM_FULL, s);  // (four times the block's sum)
-        if (lane == 0) *(int32_t *)(S + TC_REC_XS + r8 * 4) = -4128 * tot;
+        if (lane < (TC_REC - 2048) / 16 - 4) R[128 + lane] = *(const uint4 *)(S + 2048 + lane * 16);
       }
+      __syncwarp();
     }
-    // K chunk c = lane / 2 holds 16 bytes of each row: an even lane takes rows 0-3 whole, its odd neighbour
-    // rows 4-7 (64 consecutive bytes of the record each); to shared memory without bank conflicts
-    const bool odd = lane & 1;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const uint32_t s0 = odd ? q[i][0] : q[4 + i][0], s1 = odd ? q[i][1] : q[4 + i][1];
-      const uint32_t t0 = __shfl_xor_sync(PM_FULL, s0, 1), t1 = __shfl_xor_sync(PM_FULL, s1, 1);
-      const uint4 o = odd ? make_uint4(t0, t1, q[4 + i][0], q[4 + i][1]) : make_uint4(q[i][0], q[i][1], t0, t1);
-      *(uint4 *)(S + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) = o;
-    }
-    __syncwarp();
-    uint4 *R = (uint4 *)(rec0 + (size_t)u * TC_REC);
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int p = 32 * k + lane, l = p >> 2;
-      R[p] = *(const uint4 *)(S + l * 64 + (((p & 3) ^ ((l >> 1) & 3)) << 4));
-    }
-    if (lane < (TC_REC - 2048) / 16 - 4) R[128 + lane] = *(const uint4 *)(S + 2048 + lane * 16);
-    __syncwarp();
   }
 }
 
