@@ -35,9 +35,11 @@ static int32_t fail(int32_t code, const char *fmt, ...) {
 #define CU(call)                                                                       \
   do {                                                                                 \
     cudaError_t e_ = (call);                                                           \
-    if (e_ != cudaSuccess)                                                             \
+    if (e_ != cudaSuccess) {                                                           \
+      cudaGetLastError(); /* reported here: not once more by the next call */          \
       return fail(e_ == cudaErrorMemoryAllocation ? PM_ERR_OOM : PM_ERR_CUDA,          \
                   "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+    }                                                                                  \
   } while (0)
 #define TRY(call)            \
   do {                       \
@@ -1012,7 +1014,7 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
   } else if (tc || path.mx || path.q32) {
     PROF(c, PH_PLAN);
     tt = path_tiles(ly, T, path, S, false);
-    launch_tc_tiles(L, dv, g, tt);
+    CU(launch_tc_tiles(L, dv, g, tt));
   }
   if (path.mx) {
     const bool small = tt.ntok != 128;
@@ -1125,7 +1127,7 @@ static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
   const bool use_tc = path.tc, tc_gu = path.tc_gu;
   TcTiles tt{};
   if (use_tc) tt = tc_tiles_of(S.tiles, T, 1, 1, 0, 0);
-  launch_shared_groups(L, S.one, S.zero_u, S.tcount, S.iota, T, tt);
+  CU(launch_shared_groups(L, S.one, S.zero_u, S.tcount, S.iota, T, tt));
   Groups g;
   g.n_groups = S.one;
   g.expert = S.zero_u;
@@ -1165,10 +1167,10 @@ static int32_t dev_forward(pm_layer *ly, const float *x, int T, float *y, bool a
   const TcTiles tt = path_tiles(ly, T, path, S, path.merge);
   if (route_plan_small_takes(dv, x, T)) {  // a few tokens: logits, top-k, plan and tiles in one launch
     PROF(c, PH_ROUTER);
-    launch_route_plan_small(L, dv, x, T, S.logits, S.ids, S.w, S.plan, nullptr, c->route_ticket, tt, c->dev_err, c->wait_ns);
+    CU(launch_route_plan_small(L, dv, x, T, S.logits, S.ids, S.w, S.plan, nullptr, c->route_ticket, tt, c->dev_err, c->wait_ns));
   } else {
-    { PROF(c, PH_ROUTER); launch_router(L, dv, x, T, S.logits); }
-    { PROF(c, PH_ROUTE); launch_route_plan(L, dv, S.logits, T, S.ids, S.w, S.plan, S.seg, tt); }
+    { PROF(c, PH_ROUTER); CU(launch_router(L, dv, x, T, S.logits)); }
+    { PROF(c, PH_ROUTE); CU(launch_route_plan(L, dv, S.logits, T, S.ids, S.w, S.plan, S.seg, tt)); }
   }
   TRY(dev_experts(ly, x, T, S, S.w, false, path.tc || path.mx || path.q32 ? &tt : nullptr));
   const float *shared_out = S.shared_out;
@@ -1268,7 +1270,7 @@ extern "C" int32_t pm_router_logits(pm_layer *ly, const float *x, int32_t T, flo
   TRY(in_dev(c, x, n, &xd));
   OutBuf ob;
   float *ld = out_dev(c, logits, nl, ob);
-  launch_router(c->launch(), ly->dev, xd, T, ld);
+  CU(launch_router(c->launch(), ly->dev, xd, T, ld));
   CU(cudaGetLastError());
   return out_flush(c, &ob, 1);
 }
@@ -1288,7 +1290,7 @@ extern "C" int32_t pm_route_logits(pm_layer *ly, const float *logits, int32_t T,
   OutBuf ob[2];
   uint32_t *idd = out_dev(c, ids, P, ob[0]);
   float *wd = out_dev(c, w, P, ob[1]);
-  launch_route(c->launch(), ly->dev, ld, T, idd, wd);
+  CU(launch_route(c->launch(), ly->dev, ld, T, idd, wd));
   CU(cudaGetLastError());
   return out_flush(c, ob, 2);
 }
@@ -1308,8 +1310,8 @@ extern "C" int32_t pm_route(pm_layer *ly, const float *x, int32_t T, uint32_t *i
   OutBuf ob[2];
   uint32_t *idd = out_dev(c, ids, P, ob[0]);
   float *wd = out_dev(c, w, P, ob[1]);
-  { PROF(c, PH_ROUTER); launch_router(c->launch(), ly->dev, xd, T, ld); }
-  { PROF(c, PH_ROUTE); launch_route(c->launch(), ly->dev, ld, T, idd, wd); }
+  { PROF(c, PH_ROUTER); CU(launch_router(c->launch(), ly->dev, xd, T, ld)); }
+  { PROF(c, PH_ROUTE); CU(launch_route(c->launch(), ly->dev, ld, T, idd, wd)); }
   CU(cudaGetLastError());
   return out_flush(c, ob, 2);
 }
@@ -1345,8 +1347,8 @@ extern "C" int32_t pm_route_noalloc(pm_layer *ly, const float *x, int32_t T, uin
     g_noalloc_logits_dev[c->device] = p;
   }
   float *logits = g_noalloc_logits_dev[c->device];
-  launch_router(c->launch(), ly->dev, x, T, logits);
-  launch_route(c->launch(), ly->dev, logits, T, ids, w);
+  CU(launch_router(c->launch(), ly->dev, x, T, logits));
+  CU(launch_route(c->launch(), ly->dev, logits, T, ids, w));
   CU(cudaGetLastError());
   return PM_OK;
 }
@@ -1386,7 +1388,7 @@ extern "C" int32_t pm_plan(pm_layer *ly, const uint32_t *ids, int32_t T, pm_plan
   // the plan of a split call does not count towards usage[]
   LayerDev tmp = ly->dev;
   tmp.usage = nullptr;
-  launch_plan(c->launch(), tmp, idd, T, pl, c->dev_err);
+  CU(launch_plan(c->launch(), tmp, idd, T, pl, c->dev_err));
   CU(cudaGetLastError());
   cudaStream_t s = c->stream;
   CU(cudaMemcpyAsync(out->n_active, pl.n_active, 4, cudaMemcpyDefault, s));
@@ -1422,7 +1424,7 @@ extern "C" int32_t pm_experts(pm_layer *ly, const float *x, int32_t T, const uin
   scratch_carve(c, D, T, S);
   LayerDev tmp = ly->dev;
   tmp.usage = nullptr;
-  launch_plan(c->launch(), tmp, idd, T, S.plan, c->dev_err);
+  CU(launch_plan(c->launch(), tmp, idd, T, S.plan, c->dev_err));
   TRY(dev_experts(ly, xd, T, S, wd, false, nullptr));
   CU(cudaMemcpyAsync(pair_out, S.eo, P * D.d * 4, cudaMemcpyDefault, c->stream));
   CU(cudaStreamSynchronize(c->stream));
@@ -1458,7 +1460,7 @@ extern "C" int32_t pm_experts_rows(pm_layer *ly, const float *x, int32_t R, cons
   pm_layer view = *ly;
   view.dev.desc = D;
   view.dev.usage = nullptr;
-  { PROF(c, PH_PLAN); launch_plan(c->launch(), view.dev, idd, R, S.plan, c->dev_err); }
+  { PROF(c, PH_PLAN); CU(launch_plan(c->launch(), view.dev, idd, R, S.plan, c->dev_err)); }
   TRY(dev_experts(&view, xd, R, S, wd, false, nullptr));
   LayerDev cp = view.dev;
   cp.desc.weight_fold = PM_FOLD_BEFORE_DOWN;  // plain gather back to row order
@@ -1522,7 +1524,7 @@ extern "C" int32_t pm_combine(pm_layer *ly, const float *pair_out, const uint32_
   plan_carve(c, D.n_exp, P, pl);
   LayerDev tmp = ly->dev;
   tmp.usage = nullptr;
-  launch_plan(c->launch(), tmp, idd, T, pl, c->dev_err);
+  CU(launch_plan(c->launch(), tmp, idd, T, pl, c->dev_err));
   launch_combine(c->launch(), ly->dev, pod, pl.pair_pos, wd, sod, nullptr, T, yd, acc);
   CU(cudaGetLastError());
   return out_flush(c, &ob, 1);
@@ -2270,23 +2272,23 @@ extern "C" int32_t pm_moe_forward_ep(pm_ep *ep, pm_layer *ly, const float *x, in
   if (route_plan_small_takes(dv, x, T)) {  // a few tokens: logits, top-k, (slots) and plan in one launch
     auto st = ep->slots.find(ly);
     PROF(c, PH_ROUTER);
-    launch_route_plan_small(L, dv, x, T, S.logits, S.ids, S.w, S.plan, st != ep->slots.end() ? st->second.dev : nullptr,
-                            c->route_ticket, TcTiles{}, c->dev_err, c->wait_ns);
+    CU(launch_route_plan_small(L, dv, x, T, S.logits, S.ids, S.w, S.plan, st != ep->slots.end() ? st->second.dev : nullptr,
+                               c->route_ticket, TcTiles{}, c->dev_err, c->wait_ns));
   } else {
     if (T > 0) {
-      { PROF(c, PH_ROUTER); launch_router(L, dv, x, T, S.logits); }
-      { PROF(c, PH_ROUTE); launch_route(L, dv, S.logits, T, S.ids, S.w); }
+      { PROF(c, PH_ROUTER); CU(launch_router(L, dv, x, T, S.logits)); }
+      { PROF(c, PH_ROUTE); CU(launch_route(L, dv, S.logits, T, S.ids, S.w)); }
     }
     // with a placement table everything from here on names slots: the plan groups by slot, a pair goes
     // to the rank of its slot, the serving rank indexes its planes by slot
     auto st = ep->slots.find(ly);
     LayerDev dvp = dv;
     if (st != ep->slots.end()) {
-      launch_ep_slots(L, S.ids, (int)P, E, st->second.dev, dv.usage);
+      CU(launch_ep_slots(L, S.ids, (int)P, E, st->second.dev, dv.usage));
       dvp.usage = nullptr;  // counted by expert above
     }
     PROF(c, PH_PLAN);
-    launch_plan(L, dvp, S.ids, T, S.plan, c->dev_err);
+    CU(launch_plan(L, dvp, S.ids, T, S.plan, c->dev_err));
   }
   launch_ep_rank_counts(L, S.plan.cnt, E, W, ep->d_cnt);
   NC(g_nccl.AllGather(ep->d_cnt, ep->d_cnt + W, (size_t)W, PM_NCCL_INT32, ep->comm, c->stream));
@@ -2387,7 +2389,7 @@ extern "C" int32_t pm_moe_forward_ep(pm_ep *ep, pm_layer *ly, const float *x, in
     pm_layer view = *ly;
     view.dev.desc = D1;
     view.dev.usage = nullptr;
-    { PROF(c, PH_PLAN); launch_plan(L, view.dev, reid, (int)R, RS.plan, c->dev_err); }
+    { PROF(c, PH_PLAN); CU(launch_plan(L, view.dev, reid, (int)R, RS.plan, c->dev_err)); }
     TRY(dev_experts(&view, q8 ? nullptr : (const float *)rrows, (int)R, RS, rw, q8, nullptr));
     LayerDev cp = view.dev;
     cp.desc.weight_fold = PM_FOLD_BEFORE_DOWN;  // plain gather back to row order

@@ -872,9 +872,10 @@ static MegaKernel mega_kernel(const pm_layer_desc &D, bool trace) {
 }
 
 cudaError_t mega_prepare(const pm_layer_desc &D, size_t smem) {
-  cudaError_t e = cudaFuncSetAttribute((const void *)mega_kernel(D, false), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute((const void *)mega_kernel(D, true), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SmemOptIn opt[2][2];  // [down type][trace]
+  const int q6 = D.type_down == PM_TYPE_Q6_K ? 1 : 0;
+  const cudaError_t e = smem_optin(opt[q6][0], mega_kernel(D, false), smem);
+  return e != cudaSuccess ? e : smem_optin(opt[q6][1], mega_kernel(D, true), smem);
 }
 
 int mega_max_ctas_per_sm(const pm_layer_desc &D, size_t smem) {

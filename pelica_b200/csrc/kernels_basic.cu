@@ -501,31 +501,32 @@ template <int EW, int TW> __global__ void __launch_bounds__(256, 1) k_router_til
 }
 
 template <int EW, int TW>
-static void start_router_tile(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits) {
+static cudaError_t start_router_tile(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits) {
   const int E = ly.desc.n_exp, d = ly.desc.d;
   constexpr size_t smem = (size_t)RT_ST * (2 * EW + 4 * TW) * RT_CH * 4;
-  static bool set = false;  // (of every device: the attribute belongs to the function)
-  if (smem > 48 * 1024 && !set) {
-    cudaFuncSetAttribute(k_router_tile<EW, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    set = true;
-  }
+  static SmemOptIn opt;
+  const cudaError_t e = smem_optin(opt, k_router_tile<EW, TW>, smem);
+  if (e != cudaSuccess) return e;
   const dim3 grid((E + 2 * EW - 1) / (2 * EW), (T + 4 * TW - 1) / (4 * TW));
-  PLAUNCH(L, (k_router_tile<EW, TW>), grid, 256, smem, ly.router, ly.logit_bias, x, T, E, d, logits);
+  return PLAUNCH(L, (k_router_tile<EW, TW>), grid, 256, smem, ly.router, ly.logit_bias, x, T, E, d, logits);
 }
 
-void launch_router(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits) {
-  if (T == 0) return;
+cudaError_t launch_router(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits) {
+  if (T == 0) return cudaSuccess;
   int E = ly.desc.n_exp, d = ly.desc.d;
   if (T >= 8 && ((uintptr_t)x & 15) == 0) {
-    if ((long)((E + 31) / 32) * ((T + 31) / 32) >= L.n_sm) start_router_tile<16, 8>(L, ly, x, T, logits);
-    else start_router_tile<8, 4>(L, ly, x, T, logits);
-    return;
+    if ((long)((E + 31) / 32) * ((T + 31) / 32) >= L.n_sm) return start_router_tile<16, 8>(L, ly, x, T, logits);
+    return start_router_tile<8, 4>(L, ly, x, T, logits);
   }
   dim3 grid((E + 7) / 8, T);
   // (x is staged in d * 4 bytes of dynamic shared memory: beyond 48 KB that needs the opt-in; the
   // layer descriptor is refused above PM_MAX_D, which fits)
-  if ((size_t)d * 4 > 48 * 1024) cudaFuncSetAttribute(k_router, cudaFuncAttributeMaxDynamicSharedMemorySize, d * 4);
-  PLAUNCH(L, k_router, grid, 256, (size_t)d * 4, ly.router, ly.logit_bias, x, E, d, logits);
+  static SmemOptIn opt;
+  if ((size_t)d * 4 > 48 * 1024) {
+    const cudaError_t e = smem_optin(opt, k_router, (size_t)d * 4);
+    if (e != cudaSuccess) return e;
+  }
+  return PLAUNCH(L, k_router, grid, 256, (size_t)d * 4, ly.router, ly.logit_bias, x, E, d, logits);
 }
 
 __global__ void __launch_bounds__(256) k_gate_logit(const float *__restrict__ wv,
@@ -563,10 +564,10 @@ __global__ void __launch_bounds__(128) k_route(pm_layer_desc D, const float *__r
                 ids + (size_t)t * D.top_k, wout + (size_t)t * D.top_k);
 }
 
-void launch_route(const Launch &L, const LayerDev &ly, const float *logits, int T, uint32_t *ids,
-                  float *w) {
-  if (T == 0) return;
-  PLAUNCH(L, k_route, (T + 3) / 4, 128, 0, ly.desc, logits, ly.select_bias, T, ids, w);
+cudaError_t launch_route(const Launch &L, const LayerDev &ly, const float *logits, int T, uint32_t *ids,
+                         float *w) {
+  if (T == 0) return cudaSuccess;
+  return PLAUNCH(L, k_route, (T + 3) / 4, 128, 0, ly.desc, logits, ly.select_bias, T, ids, w);
 }
 
 // ===========================================================================
@@ -666,12 +667,13 @@ __global__ void __launch_bounds__(256) k_plan_place(const uint32_t *__restrict__
   }
 }
 
-void launch_plan(const Launch &L, const LayerDev &ly, const uint32_t *ids, int T, PlanDev pl, int *err) {
+cudaError_t launch_plan(const Launch &L, const LayerDev &ly, const uint32_t *ids, int T, PlanDev pl, int *err) {
   int E = ly.desc.n_exp, K = ly.desc.top_k, P = T * K;
-  PLAUNCH(L, k_plan_zero, (E + 255) / 256, 256, 0, pl.cnt, E);
-  if (P > 0) PLAUNCH(L, k_plan_count, (P + 255) / 256, 256, 0, ids, P, E, pl.cnt, pl.pair_pos, err);
-  PLAUNCH(L, k_plan_scan, 1, 512, 0, pl, E, ly.usage);
-  if (P > 0) PLAUNCH(L, k_plan_place, E, 256, 0, ids, P, K, pl);
+  cudaError_t e = PLAUNCH(L, k_plan_zero, (E + 255) / 256, 256, 0, pl.cnt, E);
+  if (e == cudaSuccess && P > 0) e = PLAUNCH(L, k_plan_count, (P + 255) / 256, 256, 0, ids, P, E, pl.cnt, pl.pair_pos, err);
+  if (e == cudaSuccess) e = PLAUNCH(L, k_plan_scan, 1, 512, 0, pl, E, ly.usage);
+  if (e == cudaSuccess && P > 0) e = PLAUNCH(L, k_plan_place, E, 256, 0, ids, P, K, pl);
+  return e;
 }
 
 // ---------------------------------------------------------------------------
@@ -889,19 +891,19 @@ __global__ void __launch_bounds__(512) k_plan_seg_place(const uint32_t *__restri
 }
 
 size_t route_seg_words(int T, int E) { return (size_t)((T + PL_SEG - 1) / PL_SEG) * E; }
-void launch_route_plan(const Launch &L, const LayerDev &ly, const float *logits, int T, uint32_t *ids, float *w, PlanDev pl,
-                       uint32_t *seg, const TcTiles &tt) {
+cudaError_t launch_route_plan(const Launch &L, const LayerDev &ly, const float *logits, int T, uint32_t *ids, float *w, PlanDev pl,
+                              uint32_t *seg, const TcTiles &tt) {
   const int E = ly.desc.n_exp, K = ly.desc.top_k, nseg = (T + PL_SEG - 1) / PL_SEG;
   const int smem = (512 + E + PL_SEG * pm_route_scratch(E)) * 4;
-  static int smem_set = 32 * 1024;  // (and 8 KB of static shared memory)
-  if (smem > smem_set) {
-    cudaFuncSetAttribute(k_route_seg, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    smem_set = smem;
-  }
-  PLAUNCH(L, k_route_seg, nseg, 1024, smem, ly.desc, logits, ly.select_bias, T, ids, w, seg, pl, ly.usage, tt, ly.first_local, ly.n_local);
-  if (nseg == 1) return;
-  PLAUNCH(L, k_plan_seg_scan, 1, 512, 0, pl, E, T, nseg, seg, ly.usage, tt, ly.first_local, ly.n_local);
-  PLAUNCH(L, k_plan_seg_place, nseg, 512, 0, ids, T * K, K, seg, E, pl);
+  static SmemOptIn opt;
+  cudaError_t e = cudaSuccess;
+  if (smem > 32 * 1024) e = smem_optin(opt, k_route_seg, smem);  // (8 KB of static shared memory besides)
+  if (e != cudaSuccess) return e;
+  e = PLAUNCH(L, k_route_seg, nseg, 1024, smem, ly.desc, logits, ly.select_bias, T, ids, w, seg, pl, ly.usage, tt, ly.first_local, ly.n_local);
+  if (nseg == 1 || e != cudaSuccess) return e;
+  e = PLAUNCH(L, k_plan_seg_scan, 1, 512, 0, pl, E, T, nseg, seg, ly.usage, tt, ly.first_local, ly.n_local);
+  if (e != cudaSuccess) return e;
+  return PLAUNCH(L, k_plan_seg_place, nseg, 512, 0, ids, T * K, K, seg, E, pl);
 }
 
 // Router logits, top-k and the dispatch plan of a few tokens (T < 8) in ONE launch: a CTA brings EPC experts' rows
@@ -1134,9 +1136,9 @@ bool route_plan_small_takes(const LayerDev &ly, const float *x, int T) {
   return ((uintptr_t)x & 15) == 0 && T > 0 && T < PM_SMALL_ROUTE_TOKENS && (size_t)2 * ly.desc.d * 4 <= 200 * 1024;
 }
 // ticket: a zeroed word of the context
-void launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits, uint32_t *ids,
-                             float *w, PlanDev pl, const int32_t *slot_table, unsigned int *ticket, const TcTiles &tt, int *err,
-                             unsigned long long wait_ns) {
+cudaError_t launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits, uint32_t *ids,
+                                    float *w, PlanDev pl, const int32_t *slot_table, unsigned int *ticket, const TcTiles &tt, int *err,
+                                    unsigned long long wait_ns) {
   const int E = ly.desc.n_exp, d = ly.desc.d;
   const int most = (int)(200 * 1024 / ((size_t)d * 4));  // rows of d values that fit
   int epc = (E + L.n_sm - 1) / L.n_sm;                   // about a CTA an SM
@@ -1145,12 +1147,10 @@ void launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x
   const int per = E + pm_route_scratch(E);               // the last CTA's scratch
   int smem = (epc + tg) * d * 4;
   if (T * per * 4 > smem) smem = T * per * 4;
-  static int smem_set = 0;
-  if (smem > smem_set) {  // (raised on a layer's first call, which is never inside a stream capture)
-    cudaFuncSetAttribute(k_route_plan_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    smem_set = smem;
-  }
-  PLAUNCH(L, k_route_plan_small, (E + epc - 1) / epc, 256, smem, ly.desc, ly.router, ly.logit_bias, ly.select_bias, x, T, epc, tg,
+  static SmemOptIn opt;
+  const cudaError_t e = smem_optin(opt, k_route_plan_small, smem);
+  if (e != cudaSuccess) return e;
+  return PLAUNCH(L, k_route_plan_small, (E + epc - 1) / epc, 256, smem, ly.desc, ly.router, ly.logit_bias, ly.select_bias, x, T, epc, tg,
           logits, ids, w, pl, ly.usage, slot_table, ticket, tt, ly.first_local, ly.n_local, err, wait_ns);
 }
 
@@ -1170,8 +1170,8 @@ __global__ void k_shared_groups(uint32_t *one, uint32_t *zero, uint32_t *count, 
   }
   if (tt.tiles && i * tt.ntok < T) tt.tiles[i] = make_uint4(TC_SHARED, i * tt.ntok, min(T - i * tt.ntok, (uint32_t)tt.ntok), i * tt.ntok);
 }
-void launch_shared_groups(const Launch &L, int *one, uint32_t *zero, uint32_t *count, uint32_t *token, int T, const TcTiles &tt) {
-  PLAUNCH(L, k_shared_groups, (T + 255) / 256, 256, 0, (uint32_t *)one, zero, count, token, (uint32_t)T, tt);
+cudaError_t launch_shared_groups(const Launch &L, int *one, uint32_t *zero, uint32_t *count, uint32_t *token, int T, const TcTiles &tt) {
+  return PLAUNCH(L, k_shared_groups, (T + 255) / 256, 256, 0, (uint32_t *)one, zero, count, token, (uint32_t)T, tt);
 }
 
 // ===========================================================================
@@ -2030,9 +2030,10 @@ __global__ void k_ep_slots(uint32_t *ids, int P, int E, const int32_t *__restric
   if (usage) atomicAdd(&usage[e], 1u);
   ids[i] = (uint32_t)table[e];
 }
-void launch_ep_slots(const Launch &L, uint32_t *ids, int P, int E, const int32_t *table, uint32_t *usage) {
-  if (P == 0) return;
+cudaError_t launch_ep_slots(const Launch &L, uint32_t *ids, int P, int E, const int32_t *table, uint32_t *usage) {
+  if (P == 0) return cudaSuccess;
   KLAUNCH(L, k_ep_slots, (P + 255) / 256, 256, 0, ids, P, E, table, usage);
+  return cudaPeekAtLastError();
 }
 
 // the two derived forms of the 8 group sums of a Q8x block that the tensor-core kernels read

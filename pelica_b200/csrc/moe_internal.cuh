@@ -4,6 +4,7 @@
 #include <cuda.h>  // CUtensorMap
 
 #include "common.cuh"
+#include "optin.h"
 
 // One expert tensor family ([n_local experts][rows][cols]) in its device layout.
 //  Q4_K : plane 0 = the GGUF blocks unchanged (144 B, 16-byte aligned rows)
@@ -138,6 +139,16 @@ static inline cudaError_t pm_launch(const Launch &L, void (*kern)(P...), dim3 gr
   return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
 
+// the current device's opt-in of `kern` to at least `bytes` of dynamic shared memory (a launch within the 48 KB every kernel
+// has needs none)
+template <typename... P> static inline cudaError_t smem_optin(SmemOptIn &o, void (*kern)(P...), size_t bytes) {
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  return (cudaError_t)o.raise(
+      dev, (int)bytes, [&](int b) { return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, b); });
+}
+
 void launch_repack(const Launch &L, int type, const uint8_t *raw, size_t n_blocks, uint8_t *p0,
                    uint8_t *p1, uint8_t *p2, uint8_t *p3);
 void launch_unpack(const Launch &L, int type, uint8_t *raw, size_t n_blocks, const uint8_t *p0,
@@ -150,11 +161,13 @@ void launch_dequant(const Launch &L, int type, size_t n_values, const uint8_t *p
 void launch_quant_q8x(const Launch &L, const float *x, size_t rows, int n, int8_t *q, float *d,
                       int32_t *bsum, uint16_t *bm = nullptr, int32_t *xs = nullptr);
 void launch_quant_q8_32(const Launch &L, const float *x, size_t rows, int n, int8_t *q, float *d, bool f16_scale);
-void launch_router(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits);
-void launch_route(const Launch &L, const LayerDev &ly, const float *logits, int T, uint32_t *ids,
+// The launches that route and plan return their status: what runs behind them takes positions and counts from their
+// results, so a call stops at the first that was refused.
+cudaError_t launch_router(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits);
+cudaError_t launch_route(const Launch &L, const LayerDev &ly, const float *logits, int T, uint32_t *ids,
                   float *w);
 // err: the context's error word (an expert id outside the layer is reported there, never used)
-void launch_plan(const Launch &L, const LayerDev &ly, const uint32_t *ids, int T, PlanDev plan, int *err);
+cudaError_t launch_plan(const Launch &L, const LayerDev &ly, const uint32_t *ids, int T, PlanDev plan, int *err);
 // router + top-k + plan (+ tile list) of T < PM_SMALL_ROUTE_TOKENS tokens in one launch (ticket: a zeroed word the
 // kernel leaves zeroed; slot_table: expert -> slot of an expert-parallel placement, or null)
 #define PM_SMALL_ROUTE_TOKENS 8
@@ -174,14 +187,14 @@ __host__ __device__ inline uint32_t tc_tile_tokens(uint32_t cnt, uint32_t n, int
   return even && n > 1 ? ((cnt + n - 1) / n + 15u) & ~15u : (uint32_t)ntok;
 }
 bool route_plan_small_takes(const LayerDev &ly, const float *x, int T);
-void launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits, uint32_t *ids,
-                             float *w, PlanDev pl, const int32_t *slot_table, unsigned int *ticket, const TcTiles &tt, int *err,
-                             unsigned long long wait_ns);
+cudaError_t launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits, uint32_t *ids,
+                                    float *w, PlanDev pl, const int32_t *slot_table, unsigned int *ticket, const TcTiles &tt, int *err,
+                                    unsigned long long wait_ns);
 // top-k, weights and plan of any number of tokens from their logits (seg: route_seg_words words of scratch)
 size_t route_seg_words(int T, int E);
-void launch_route_plan(const Launch &L, const LayerDev &ly, const float *logits, int T, uint32_t *ids, float *w, PlanDev pl,
-                       uint32_t *seg, const TcTiles &tt);
-void launch_shared_groups(const Launch &L, int *one, uint32_t *zero, uint32_t *count, uint32_t *token, int T, const TcTiles &tt);
+cudaError_t launch_route_plan(const Launch &L, const LayerDev &ly, const float *logits, int T, uint32_t *ids, float *w, PlanDev pl,
+                              uint32_t *seg, const TcTiles &tt);
+cudaError_t launch_shared_groups(const Launch &L, int *one, uint32_t *zero, uint32_t *count, uint32_t *token, int T, const TcTiles &tt);
 void launch_gateup(const Launch &L, const LayerDev &ly, bool shared, Groups g, int n_pairs,
                    const float *x, const int8_t *xq, const float *xd, const int32_t *xbsum,
                    const float *w, float *h);
@@ -200,7 +213,7 @@ size_t tc_tile_words(int n_pairs, int max_groups);
 // ntok: tokens of a full tile, 0 for launch_tc's own rule (anything else: even tiles)
 TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, int ntok);  // buf: tc_tile_words words, 16-byte aligned
 size_t tc_rec_bytes(int n_pairs, int max_groups, int cols);
-void launch_tc_tiles(const Launch &L, const LayerDev &ly, Groups g, const TcTiles &t);
+cudaError_t launch_tc_tiles(const Launch &L, const LayerDev &ly, Groups g, const TcTiles &t);
 void launch_tc_quant_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x,
                           uint8_t *rec);
 void launch_tc_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const int8_t *xq,
@@ -232,7 +245,7 @@ cudaError_t launch_tc_q32(const Launch &L, const LayerDev &ly, bool down, const 
                           const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns);
 // expert parallelism (kernels_basic.cu): per-rank pair counts, the wire records of a dispatch,
 // the received (expert, weight) records, the derived forms of received Q8x group sums
-void launch_ep_slots(const Launch &L, uint32_t *ids, int P, int E, const int32_t *table, uint32_t *usage);
+cudaError_t launch_ep_slots(const Launch &L, uint32_t *ids, int P, int E, const int32_t *table, uint32_t *usage);
 void launch_ep_rank_counts(const Launch &L, const uint32_t *cnt, int E, int W, int32_t *out);
 void launch_ep_pack(const Launch &L, int P, int row_bytes, int nd, int nbs, const void *rows, const float *xd,
                     const int32_t *xbs, const uint32_t *pair_token, const uint32_t *pair_src, const uint32_t *ids,

@@ -475,14 +475,9 @@ template <bool DOWN> static cudaError_t mx_start(const Launch &L, const MxArgs &
   constexpr size_t smem = (size_t)S::NSR * S::RAWB + (size_t)S::NSB * S::BST + MX_IT * sizeof(MxItem) +
                           (2 * S::NSR + 2 * S::NSB + 2 * MX_NA + 2 + 2 * MX_IT) * 8 + 16;
   static_assert(smem <= 232448, "more than an SM's shared memory");
-  static bool set[64] = {};  // (one-time per device and kernel)
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 64 || !set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(k_tc_mx<DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    if (dev < 64) set[dev] = true;
-  }
+  static SmemOptIn opt;
+  const cudaError_t e = smem_optin(opt, k_tc_mx<DOWN>, smem);
+  if (e != cudaSuccess) return e;
   const long ctas = L.n_sm;
   return pm_launch(L, k_tc_mx<DOWN>, dim3((unsigned)(items < ctas ? items : ctas)), S::NT, smem, A);
 }

@@ -476,14 +476,9 @@ template <bool DOWN, int NP> static cudaError_t mx8_start(const Launch &L, const
   constexpr size_t smem = (size_t)S::NSR * M8_RAW + (size_t)M8_NA * M8_AST + (size_t)M8_NA * S::BST + M8_NA * 512 + M8_IT * sizeof(M8Item) +
                           (2 * S::NSR + 2 * M8_NA + 2 * S::NACC + 2 * M8_IT) * 8 + 16;
   static_assert(smem <= 115712, "two CTAs an SM");
-  static bool set[64] = {};  // (one-time per device and kernel)
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 64 || !set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(k_tc_mx8<DOWN, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    if (dev < 64) set[dev] = true;
-  }
+  static SmemOptIn opt;
+  const cudaError_t e = smem_optin(opt, k_tc_mx8<DOWN, NP>, smem);
+  if (e != cudaSuccess) return e;
   const long ctas = 2L * L.n_sm;
   return pm_launch(L, k_tc_mx8<DOWN, NP>, dim3((unsigned)(items < ctas ? items : ctas)), M8_NT, smem, A);
 }

@@ -490,14 +490,9 @@ template <int WT, bool DOWN> static cudaError_t q32_start(const Launch &L, const
   constexpr size_t smem = (size_t)Q32_NSR * Q32Raw<WT>::BYTES + (size_t)Q32_NSB * Q32_BST + (DOWN ? 0 : Q32_N * Q32_M * 4) +
                           Q32_IT * sizeof(Q32Item) + (2 * Q32_NSR + 2 * Q32_NSB + 4 + 2 * Q32_NACC + 2 * Q32_IT) * 8 + 16;
   static_assert(smem <= 115712, "two CTAs an SM");
-  static bool set[64] = {};  // (one-time per device and kernel)
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 64 || !set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(k_tc_q32<WT, DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    if (dev < 64) set[dev] = true;
-  }
+  static SmemOptIn opt;
+  const cudaError_t e = smem_optin(opt, k_tc_q32<WT, DOWN>, smem);
+  if (e != cudaSuccess) return e;
   const long ctas = 2L * L.n_sm;
   return pm_launch(L, k_tc_q32<WT, DOWN>, dim3((unsigned)(items < ctas ? items : ctas)), Q32_NT, smem, A);
 }

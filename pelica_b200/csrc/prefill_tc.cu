@@ -885,8 +885,8 @@ TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, in
   t.tiles = (uint4 *)(buf + 4);
   return t;
 }
-void launch_tc_tiles(const Launch &L, const LayerDev &ly, Groups g, const TcTiles &t) {
-  pm_launch(L, k_tc_tiles, 1, 512, 0, g, ly.first_local, ly.n_local, t.n, t.tiles, t.ntok, t.even, t.max_tiles);
+cudaError_t launch_tc_tiles(const Launch &L, const LayerDev &ly, Groups g, const TcTiles &t) {
+  return pm_launch(L, k_tc_tiles, 1, 512, 0, g, ly.first_local, ly.n_local, t.n, t.tiles, t.ntok, t.even, t.max_tiles);
 }
 static dim3 rows_grid(int n_rows, const TcTiles &t, int cols) {
   const long units = ((long)n_rows / 8 + 2 * t.max_tiles) * (cols / 256);  // (row group, block) records in all
@@ -909,14 +909,9 @@ template <int WT, bool DOWN, int PARTS> static cudaError_t tc_start(const Launch
   constexpr size_t smem = (size_t)NS * (Q6 ? TC_RAW_Q6 : TC_RAW_Q4) + (size_t)NSB * S::BST + (Q6 ? 0 : 2 * 2 * TC_M * 16) +
                           (DOWN ? 0 : S::XB) + (2 * NS + 2 * NSB + 12 + 2 * TC_IT) * 8 + TC_IT * sizeof(TcItem) + 16;
   static_assert(smem <= (S::CTAS == 1 ? 232448 : 115712), "more than an SM's shared memory");
-  static bool set[64] = {};  // (one-time per device and kernel)
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 64 || !set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(k_tc<WT, DOWN, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    if (dev < 64) set[dev] = true;
-  }
+  static SmemOptIn opt;
+  const cudaError_t e = smem_optin(opt, k_tc<WT, DOWN, PARTS>, smem);
+  if (e != cudaSuccess) return e;
   const long ctas = (long)S::CTAS * L.n_sm;
   return pm_launch(L, k_tc<WT, DOWN, PARTS>, dim3((unsigned)(items < ctas ? items : ctas)), S::NT, smem, A);
 }
