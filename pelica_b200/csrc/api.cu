@@ -99,6 +99,9 @@ struct pm_ctx {
   int64_t path_count[PM_PATH_N] = {0, 0, 0, 0};  // launches per expert-product path (pelica_moe_diag.h)
   unsigned long long wait_ns = 2000000000ull;    // limit of every bounded device-side wait
   int tc_fault_block = -1;                       // test hook: the tensor-core kernel never completes this block
+  // Moves with every change of what picks a call's kernels or goes into their parameters (the three settings above): a
+  // stack's recorded graphs hold both.
+  uint64_t dispatch_gen = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // workspace: one region, carved per call
   uint8_t *ws = nullptr;
@@ -275,6 +278,7 @@ extern "C" int32_t pm_sync(pm_ctx *c) {
 }
 extern "C" int32_t pm_ctx_set_tensor_core_min_tokens(pm_ctx *c, int32_t min_tokens) {
   if (!c || min_tokens < 0) return fail(PM_ERR_INVALID, "pm_ctx_set_tensor_core_min_tokens");
+  if (!c->tc_min_set || c->tc_min_tokens != min_tokens) c->dispatch_gen++;
   c->tc_min_tokens = min_tokens;
   c->tc_min_set = true;
   return PM_OK;
@@ -289,6 +293,7 @@ extern "C" int32_t pm_ctx_path_counts(pm_ctx *c, int64_t *out) {
 }
 extern "C" int32_t pm_debug_set_wait_limit_ns(pm_ctx *c, uint64_t ns) {
   if (!c || ns == 0) return fail(PM_ERR_INVALID, "pm_debug_set_wait_limit_ns");
+  if (c->wait_ns != ns) c->dispatch_gen++;
   c->wait_ns = ns;
   return PM_OK;
 }
@@ -302,6 +307,7 @@ extern "C" int32_t pm_debug_device_free_bytes(pm_ctx *c, uint64_t *out) {
 }
 extern "C" int32_t pm_debug_tc_fault_block(pm_ctx *c, int32_t block) {
   if (!c) return fail(PM_ERR_INVALID, "pm_debug_tc_fault_block");
+  if (c->tc_fault_block != block) c->dispatch_gen++;
   c->tc_fault_block = block;
   return PM_OK;
 }
@@ -1635,6 +1641,7 @@ struct pm_stack {
   bool graph_off = false;
   bool fault_next = false;         // pm_debug_stack_fault_next_call
   std::vector<uint64_t> seen_gen;  // the layers' generation counters when their pointers were last snapshot
+  uint64_t seen_dispatch = 0;      // the context's dispatch_gen that the graphs were recorded under
 };
 
 // (re)writes the decode kernel's per-layer pointer table from the layers' current state
@@ -1876,6 +1883,11 @@ extern "C" int32_t pm_stack_forward(pm_stack *s, const float *x, int32_t T, floa
       cudaGetLastError();
       graphable = false;
     }
+  }
+  if (graphable && s->seen_dispatch != c->dispatch_gen) {
+    CU(cudaStreamSynchronize(c->stream));
+    stack_drop_graphs(s);
+    s->seen_dispatch = c->dispatch_gen;
   }
   if (graphable) {
     pm_stack::Graph *g = nullptr;

@@ -117,3 +117,45 @@ def test_shapes_outside_the_decode_kernel_use_the_general_path(ctx, oracle):
     assert tol_ok(got, want)
     st.close()
     gl.close()
+
+
+def test_recorded_loops_follow_the_context_settings(oracle):
+    """A threshold or a wait limit set after a token count was recorded holds for the next call: the recorded loop
+    of T = 8 is made anew, not replayed with the kernels (and limits) it was recorded with."""
+    c, r = pb.Context(0), pb.Context(0)
+    r.set_tensor_core_min_tokens(0)  # row kernels from the first call on
+    for name in ("c3", "c2"):
+        cfg = SMALL[name]
+        pairs = [make_pair(oracle, pb, c, cfg, 700 + l) for l in range(2)]
+        rows = [make_pair(oracle, pb, r, cfg, 700 + l)[1] for l in range(2)]
+        st, st_r = pb.Stack(c, [p[1] for p in pairs]), pb.Stack(r, rows)
+        x = synth.make_activations(8, cfg.d, 71)
+        want_rows = st_r.forward(x)
+        if name == "c3":
+            first = [st.forward(x) for _ in range(3)]  # plain, recorded, replayed
+            assert all(bits_equal(f, first[0]) for f in first)
+            assert not bits_equal(first[0], want_rows)  # f32 sums in another order
+            c.set_tensor_core_min_tokens(0)
+            for _ in range(3):
+                assert bits_equal(st.forward(x), want_rows)
+            c.set_tensor_core_min_tokens(1)
+            assert bits_equal(st.forward(x), first[0])
+        else:
+            for _ in range(3):
+                assert bits_equal(st.forward(x), want_rows)
+            c.set_wait_limit_ns(200_000)
+            c.tc_fault_block(1)  # the products of block 1 are never issued nor signalled
+            st.forward(x)
+            with pytest.raises(pb.PelicaError) as e:
+                c.sync()
+            assert e.value.code == -6
+            c.tc_fault_block(-1)
+            c.set_wait_limit_ns(2_000_000_000)
+            for _ in range(3):
+                assert bits_equal(st.forward(x), want_rows)
+        for s in (st, st_r):
+            s.close()
+        for g in [p[1] for p in pairs] + rows:
+            g.close()
+    c.close()
+    r.close()
