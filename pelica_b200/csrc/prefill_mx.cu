@@ -103,6 +103,7 @@ struct MxArgs {
   float *out;             // gate/up: h [P][ff]; down: eo [P][d]
   int *err;
   unsigned long long wait_ns;
+  uint32_t zero;  // 0 (see tc_mbar_arrive_used)
   int row_tiles;
   int cols, rows;
   int act;
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(MxShape::NT, 1) k_tc_mx(const __grid_constant_
     const bool ok = tc_wait(it_full + s, (uint32_t)((k / MX_IT) & 1), A.err, A.wait_ns);
     it = items[s];
     __syncwarp();
-    if (lane == 0) tc_mbar_arrive(it_empty + s);
+    if (lane == 0) tc_mbar_arrive_used(it_empty + s, it.t.x ^ (uint32_t)it.r0, A.zero);
     return ok && it.t.x != MX_END;
   };
 
@@ -507,6 +508,7 @@ cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const u
   A.out = out;
   A.err = err;
   A.wait_ns = wait_ns;
+  A.zero = 0;
   const int rpc = down ? 2 * MX_M : MX_M;
   A.row_tiles = (W0.rows + rpc - 1) / rpc;
   A.cols = W0.cols;

@@ -59,6 +59,7 @@ struct M8Args {
   size_t split_stride;
   int *err;
   unsigned long long wait_ns;
+  uint32_t zero;  // 0 (see tc_mbar_arrive_used)
   int row_tiles, splits, split_stages;
   int cols, rows;
   int act;
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
     const bool ok = tc_wait(it_full + s, (uint32_t)((k / M8_IT) & 1), A.err, A.wait_ns);
     it = items[s];
     __syncwarp();
-    if (lane == 0) tc_mbar_arrive(it_empty + s);
+    if (lane == 0) tc_mbar_arrive_used(it_empty + s, it.t.x ^ (uint32_t)it.r0, A.zero);
     return ok && it.t.x != M8_END;
   };
 
@@ -532,6 +533,7 @@ cudaError_t launch_tc_mx8(const Launch &L, const LayerDev &ly, bool down, const 
   A.split_stride = split_stride;
   A.err = err;
   A.wait_ns = wait_ns;
+  A.zero = 0;
   const int rpc = down ? M8_M : M8_M / 2, nst = (W0.cols + M8_KS - 1) / M8_KS;
   A.row_tiles = (W0.rows + rpc - 1) / rpc;
   A.split_stages = mx8_split_stages(nst, splits);

@@ -41,6 +41,7 @@ struct Q32Args {
   float *out;             // gate/up: h [P][ff]; down: eo [P][d]
   int *err;
   unsigned long long wait_ns;
+  uint32_t zero;  // 0 (see tc_mbar_arrive_used)
   uint64_t neg_zero2;     // (-0, -0): see tc_fma2
   int row_tiles;
   int cols, rows;
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
     const bool ok = tc_wait(it_full + s, (uint32_t)((k / Q32_IT) & 1), A.err, A.wait_ns);
     it = items[s];
     __syncwarp();
-    if (lane == 0) tc_mbar_arrive(it_empty + s);
+    if (lane == 0) tc_mbar_arrive_used(it_empty + s, it.t.x ^ (uint32_t)it.r0, A.zero);
     return ok && it.t.x != Q32_END;
   };
   // blocks whose sums share a slot of 64 columns: fewer barriers for small tiles
@@ -374,7 +375,10 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
           }
         }
         __syncwarp();
-        if (lane == 0) tc_mbar_arrive(empty_b + sb);
+        uint32_t used = 0;  // (every read of the scales - of four tokens - went into their sums)
+#pragma unroll
+        for (int i = 0; i < Q32_N / 4; i += 2) used ^= (uint32_t)acc[i];
+        if (lane == 0) tc_mbar_arrive_used(empty_b + sb, used, A.zero);
         if (++sb == Q32_NSB) sb = 0;
       };
       unsigned long long sc = 0;
@@ -520,6 +524,7 @@ cudaError_t launch_tc_q32(const Launch &L, const LayerDev &ly, bool down, const 
   A.out = out;
   A.err = err;
   A.wait_ns = wait_ns;
+  A.zero = 0;
   A.neg_zero2 = 0x8000000080000000ull;
   const int rpc = down ? Q32_M : Q32_M / 2;
   A.row_tiles = (W0.rows + rpc - 1) / rpc;

@@ -101,6 +101,7 @@ struct TcArgs {
   float *out;                  // gate/up: h [P][ff]; down: eo [P][d]
   int *err;
   unsigned long long wait_ns;  // limit of every wait on an mbarrier
+  uint32_t zero;  // 0 (see tc_mbar_arrive_used)
   uint64_t neg_zero2;          // (-0, -0): see tc_fma2
   int fault_block;             // test hook: no products are issued or signalled from this block on (-1 = off)
   int row_tiles;               // tiles of rows of the matrix (128 rows, or 64 gate + 64 up)
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
     it.t = items[s].t;
     it.r0 = items[s].r0;
     __syncwarp();
-    if (lane == 0) tc_mbar_arrive(it_empty + s);
+    if (lane == 0) tc_mbar_arrive_used(it_empty + s, it.t.x ^ (uint32_t)it.r0, A.zero);
     return ok && it.t.x != TC_END;
   };
 
@@ -656,8 +657,10 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
         for (int i = 0; i < NP * CH; i++) tot[i] = 0ull;
         // the float terms of the next pass (pass P of its block), in block order: TMEM lane m, the part's columns.
         // x.d of the block is visible once this thread has seen the tokens' barrier (long complete).
+        uint32_t used = 0;  // of every word that the folds of a block read from the tokens' area (tc_mbar_arrive_used)
         auto fold = [&](auto pass, float d, float dm) {
           constexpr int P = decltype(pass)::value;
+          if (P == 0) used = 0;
           constexpr bool LAST = P == NP - 1;
           const uint32_t set = gp & 1;
           const int ew = LAST ? ewl : S::CW, c0 = part * ew;
@@ -687,6 +690,7 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
             const ulonglong2 x4 = *(const ulonglong2 *)(rx + TC_REC_XD);
             int4 s4 = make_int4(0, 0, 0, 0);
             if (Q6) s4 = *(const int4 *)(rx + TC_REC_XS);
+            used ^= (uint32_t)x4.x ^ (uint32_t)s4.x;
             term2(v0[0], v0[1], v1[0], v1[1], v2[0], v2[1], x4.x, s4.x, s4.y, ta);
             term2(v0[2], v0[3], v1[2], v1[3], v2[2], v2[3], x4.y, s4.z, s4.w, tb);
           };
@@ -716,7 +720,7 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
           __syncwarp();
           if (lane == 0) {
             tc_mbar_arrive(acc_free + set);
-            if (LAST) tc_mbar_arrive(empty_b + sf);  // this warp has read the block's x.d
+            if (LAST) tc_mbar_arrive_used(empty_b + sf, used, A.zero);  // this warp has read the block's x.d
           }
           if (LAST)
             if (++sf == NSB) { sf = 0; pf ^= 1; }
@@ -960,6 +964,7 @@ cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared_only, boo
   A.out = out;
   A.err = err;
   A.wait_ns = wait_ns;
+  A.zero = 0;
   A.fault_block = fault_block;
   A.neg_zero2 = 0x8000000080000000ull;
   A.row_tiles = down ? (W0.rows + TC_M - 1) / TC_M : (W0.rows + 63) / 64;

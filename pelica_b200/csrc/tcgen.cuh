@@ -90,6 +90,16 @@ __device__ __forceinline__ void tc_mbar_init(uint64_t *bar, uint32_t count) {
 __device__ __forceinline__ void tc_mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_s32(bar)) : "memory");
 }
+// The arrival that hands a place of a ring back after words were read from it. `used` is made of every load's words
+// and goes into the address (times `zero`, which is 0 at run time and unknown to the compiler): the arrival cannot be
+// issued before the loads have returned, wherever the arithmetic on them is scheduled. (One lane's words stand for
+// the warp's where all lanes read the same address: one load instruction.)
+__device__ __forceinline__ void tc_mbar_arrive_used(uint64_t *bar, uint32_t used, uint32_t zero) {
+  asm volatile(
+      "{\n .reg .b32 a;\n and.b32 a, %1, %2;\n add.u32 a, a, %0;\n mbarrier.arrive.shared::cta.b64 _, [a];\n}\n" ::"r"(tc_s32(bar)),
+      "r"(used), "r"(zero)
+      : "memory");
+}
 __device__ __forceinline__ void tc_mbar_expect(uint64_t *bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc_s32(bar)), "r"(bytes) : "memory");
 }
