@@ -219,8 +219,8 @@ __device__ __forceinline__ int pm_warp_sum_i32(int v) {
 // `Q8x::new` / `Q8::new` rounding of eight values x * id (half away from zero, as f32::round, src/ds4_cpu.rs:25): the
 // low bytes of two words. id = 127 / (largest |x| of the block), so |x * id| rounds to at most 127. The common
 // case takes five float operations a value: adding 1.5 * 2^23 rounds to the nearest integer (ties to even) and
-// leaves it in the low byte; a value exactly between two integers - and a block so small that 127 / max is
-// infinite - takes the plain form instead.
+// leaves it in the low byte; a value exactly between two integers, a block so small that 127 / max is infinite, and a
+// product that is no number (a NaN, or an infinity times id = 0: -127, as fmaxf drops a NaN) take the plain form instead.
 __device__ __forceinline__ void pm_q8_pack8(const float v[8], float id, uint32_t &w0, uint32_t &w1) {
   const float M = 12582912.0f;
   uint32_t b[8];
@@ -228,7 +228,7 @@ __device__ __forceinline__ void pm_q8_pack8(const float v[8], float id, uint32_t
 #pragma unroll
   for (int j = 0; j < 8; j++) {
     const float f = __fmul_rn(v[j], id), m = __fadd_rn(f, M);
-    odd = odd || fabsf(__fsub_rn(f, __fsub_rn(m, M))) == 0.5f;
+    odd = odd || !(fabsf(__fsub_rn(f, __fsub_rn(m, M))) < 0.5f);
     b[j] = __float_as_uint(m);
   }
   if (odd) {

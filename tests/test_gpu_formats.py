@@ -87,6 +87,25 @@ def test_quant_act_32_bit_exact(ctx, oracle):
         assert bits_equal(d, od)
 
 
+def test_quant_act_of_what_is_no_number(ctx):
+    """A NaN is -127 in either quantiser (fmaxf drops it, the clamp gives the bound) and leaves its block's scale alone; an
+    infinity makes the scale infinite, itself -127 (inf * 0) and every other value of its block 0."""
+    x = np.random.default_rng(12).normal(0, 1, 3 * 256).astype(np.float32)
+    nan, inf = [5, 2 * 256 + 255], 256 + 40
+    x[nan] = 0.01  # (not the largest of their blocks)
+    clean = [ctx.quant_act(x), ctx.quant_act_32(x)]
+    x[nan] = [np.nan, -np.nan]
+    x[inf] = np.inf
+    for (q, d, *sums), (want_q, want_d, *_), n in zip([ctx.quant_act(x), ctx.quant_act_32(x)], clean, (256, 32)):
+        want_q[inf // n * n:(inf // n + 1) * n] = 0
+        want_q[nan + [inf]] = -127
+        want_d[inf // n] = np.inf
+        assert np.array_equal(q, want_q)
+        assert np.array_equal(d, want_d)
+        if sums:
+            assert np.array_equal(sums[0], want_q.astype(np.int32).reshape(-1, 32).sum(1))
+
+
 def test_quant_act_rejects_ragged(ctx):
     import pelica_b200 as pb
 
