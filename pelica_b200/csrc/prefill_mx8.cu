@@ -125,17 +125,21 @@ __global__ void __launch_bounds__(128) k_mx8_rows(const int *__restrict__ n_tile
       const int E = (int)(top >> 23) - 127;
       uint8_t *dst = base + (size_t)(b >> 2) * (N * M8_KS + 512) + (size_t)(b & 3) * (N * 32);
       uint8_t *sf = base + (size_t)(b >> 2) * (N * M8_KS + 512) + N * M8_KS + (b & 3);
+      // (what is left is kept in units of the next piece: exact, and in range also where x1, rounded up, is 2^128)
+      const float unit = m8_pow2(-max(E - 7, -126));
+#pragma unroll
+      for (int i = 0; i < 32; i++) v[i] = __fmul_rn(v[i], unit);
 #pragma unroll
       for (int p = 0; p < NP; p++) {
         const int S = max(E - 7 - 5 * p, -126);
-        const float up = m8_pow2(-S), down = m8_pow2(S);
+        const float next = m8_pow2(S - max(E - 12 - 5 * p, -126));  // 32, or less at the bottom of the range
         uint32_t w[8];
 #pragma unroll
         for (int i = 0; i < 16; i++) {  // (16 times: values i and i + 16)
-          const uint32_t c = m8_e4m3x2(__fmul_rn(v[i + 16], up), __fmul_rn(v[i], up));
+          const uint32_t c = m8_e4m3x2(v[i + 16], v[i]);
           const float2 f = m8_from_e4m3x2(c);
-          v[i] = __fsub_rn(v[i], __fmul_rn(f.x, down));
-          v[i + 16] = __fsub_rn(v[i + 16], __fmul_rn(f.y, down));
+          v[i] = __fmul_rn(__fsub_rn(v[i], f.x), next);
+          v[i + 16] = __fmul_rn(__fsub_rn(v[i + 16], f.y), next);
           if (i & 1) w[i >> 1] |= c << 16;
           else w[i >> 1] = c;
         }

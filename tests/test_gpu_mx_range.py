@@ -1,0 +1,76 @@
+"""MXFP4 products at the ends of the number range: the tensor-core kernels against the oracle and the row kernels, whichever
+of them the token count picks."""
+import numpy as np
+import pytest
+
+import pelica_b200 as pb
+from pelica_b200 import synth
+from tests.helpers import SMALL, tol_ok
+
+pytestmark = [pytest.mark.gpu, pytest.mark.timeout(600)]
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    """A context that nobody has given a threshold: the default choice of kernels."""
+    c = pb.Context(0)
+    yield c
+    c.close()
+
+
+@pytest.fixture(scope="module")
+def rows_ctx():
+    c = pb.Context(0)
+    c.set_tensor_core_min_tokens(0)
+    yield c
+    c.close()
+
+
+def codes(W, key, cfg):
+    """[expert][row][block][17] of a matrix: the scale byte, then 16 bytes of codes."""
+    rows, cols = (cfg.d, cfg.ff) if key == "down" else (cfg.ff, cfg.d)
+    return W[key].reshape(cfg.n_exp, rows, cols // 32, 17)
+
+
+def layers(oracle, ctx, rows_ctx, cfg, W):
+    return (oracle.Layer(oracle.LayerDesc(**cfg.desc_fields()), W), pb.MoeLayer(ctx, cfg).load(W),
+            pb.MoeLayer(rows_ctx, cfg).load(W))
+
+
+def picks(T, cfg):
+    """Expert ids spread evenly and weights that sum to one: the products without the router in front."""
+    ids = (np.arange(T)[:, None] + np.arange(cfg.top_k)[None, :] * (cfg.n_exp // cfg.top_k)) % cfg.n_exp
+    w = np.random.default_rng(T).uniform(0.5, 1.5, ids.shape).astype(np.float32)
+    return ids.astype(np.uint32), w / w.sum(1, keepdims=True)
+
+
+def agree(got, want):
+    """Infinities and NaN where the reference has them, the rest within the layer tolerance."""
+    fin = np.isfinite(want)
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(got[np.isinf(want)], want[np.isinf(want)])
+    assert tol_ok(got[fin], want[fin]), float(np.abs(got[fin] - want[fin]).max())
+
+
+@pytest.mark.parametrize("T", [1, 5, 40])
+def test_activations_that_round_up_past_the_largest_float(ctx, rows_ctx, oracle, T):
+    """|x| of 1.94 * 2^127 and more is 256 units of its first piece, 2^128: the pieces behind it still hold what is missing
+    (3 % without them). The column meets codes of 0.5 in gate (no overflow in the row kernels either) and 0 in up."""
+    cfg = SMALL["c3"].scaled(act_limit=3e38)
+    W = synth.make_weights(cfg, 91)
+    for key, code in (("gate", 1), ("up", 0)):
+        c = codes(W, key, cfg)
+        c[:, :, 2, 0] = 90                             # 2^-37: what comes out stays far from overflow
+        c[:, :, 2, 1] = (c[:, :, 2, 1] & 0xF0) | code  # value 0 of block 2: the low nibble
+    ol, gl, gr = layers(oracle, ctx, rows_ctx, cfg, W)
+    x = synth.make_activations(T, cfg.d, 92)
+    x[:, 64] = 3.4028234e38
+    x[0, 64] = 3.31e38
+    x[T // 2 + 1:, 64] *= -1
+    ids, w = picks(T, cfg)
+    want = ol.experts(x, ids, w)
+    assert np.isfinite(want).all() and np.abs(want).max() > 1e20
+    agree(gr.experts(x, ids, w), want)
+    agree(gl.experts(x, ids, w), want)
+    gl.close()
+    gr.close()
