@@ -233,8 +233,8 @@ void launch_mx8_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32
 cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
                          const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns);
 cudaError_t launch_tc_mx8(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
-                          const uint8_t *rec, const float *wts, float *out, int splits, size_t split_stride, int *err,
-                          unsigned long long wait_ns);
+                          const uint8_t *rec, const float *x, const uint32_t *src_row, const float *wts, float *out, int splits,
+                          size_t split_stride, int *err, unsigned long long wait_ns);
 // tensor-core (tcgen05 int8) form for Q8_0 / IQ4_NL / IQ4_XS weights and 32-value activation blocks (prefill_q32.cu)
 bool q32_weights(int type);
 int q32_tile_tokens();

@@ -19,7 +19,7 @@
 // kernels, 37 here.
 #include <cuda_fp16.h>
 
-#include "tcgen.cuh"
+#include "mxsum.cuh"
 
 #define M8_M 128
 #define M8_KS 128     /* K values of a stage: four products of 32 */
@@ -52,6 +52,10 @@ struct M8Args {
   const int *n_tiles;
   unsigned int *next;
   const uint8_t *rec;     // the tokens' pieces (k_mx8_rows)
+  const uint8_t *w0, *w1;       // the nibbles, the f32 rows and the row of each pair (null: its own), for mx_repair
+  size_t w0_stride, w1_stride;
+  const float *x;
+  const uint32_t *src_row;
   const float *bias0, *bias1;
   const float *wts;
   const uint32_t *pair_src;
@@ -143,7 +147,7 @@ __global__ void __launch_bounds__(128) k_mx8_rows(const int *__restrict__ n_tile
           if (i & 1) w[i >> 1] |= c << 16;
           else w[i >> 1] = c;
         }
-        if (top >= 0x7f800000u) {  // an infinity or a NaN in the block: NaN, as its bf16 pieces add up to
+        if (top >= 0x7f800000u) {  // an infinity or a NaN in the block: NaN (what it spoils is summed again, mxsum.cuh)
 #pragma unroll
           for (int i = 0; i < 8; i++) w[i] = 0x7f7f7f7fu;
         }
@@ -368,9 +372,9 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
       }
       // the row's scale bytes, eight blocks (two stages) at a time
       const uint8_t *sp = (up ? A.s1 + (size_t)el * A.s1_stride : A.s0 + (size_t)el * A.s0_stride) + (size_t)min(row, rows - 1) * nbk;
-      float acc[16];
+      float acc[S::NTOK / 2];
 #pragma unroll
-      for (int u = 0; u < 16; u++) acc[u] = 0.0f;
+      for (int u = 0; u < S::NTOK / 2; u++) acc[u] = 0.0f;
       auto fold = [&] {  // the pieces' sums of the thread's tokens, smallest piece first
         tc_wait(acc_full + set, pf, A.err, A.wait_ns);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -432,6 +436,14 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
       fold();
       // ---- epilogue ----
       const bool on = row < rows && *(volatile int *)A.err == 0;
+      mx_repair(
+          acc, [&](int u) { return row < rows && u < ew && e0 + u < nvalid; },
+          [&](int u) {
+            const uint32_t p = T.y + (uint32_t)(e0 + u);
+            return mx_sum_f32((up ? A.w1 + (size_t)el * A.w1_stride : A.w0 + (size_t)el * A.w0_stride) + (size_t)row * (A.cols / 2), sp,
+                              A.x + (size_t)(A.src_row ? A.src_row[p] : p) * A.cols, 4 * it.s0, min(4 * it.s1, nbk));
+          });
+      __syncwarp();
       const bool bias = A.bias0 && it.split == 0;
       const float b0 = bias && row < rows ? A.bias0[(size_t)el * rows + row] : 0.0f;
       const float b1 = !DOWN && bias && row < rows ? A.bias1[(size_t)el * rows + row] : 0.0f;
@@ -512,10 +524,11 @@ int mx_splits(const pm_layer_desc &D, int n_pairs) {
 }
 
 // Tensor-core form of launch_gateup / launch_down for MXFP4 weights and f32 activations given as the pieces of
-// the grouping's rows. splits: cuts of K (down only); split s goes to out + s * split_stride.
+// the grouping's rows. x, src_row: the rows the pieces were made of (as in launch_mx8_rows). splits: cuts of K (down only); split s
+// goes to out + s * split_stride.
 cudaError_t launch_tc_mx8(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
-                          const uint8_t *rec, const float *wts, float *out, int splits, size_t split_stride, int *err,
-                          unsigned long long wait_ns) {
+                          const uint8_t *rec, const float *x, const uint32_t *src_row, const float *wts, float *out, int splits,
+                          size_t split_stride, int *err, unsigned long long wait_ns) {
   if (t.max_tiles == 0) return cudaSuccess;
   const WMat &W0 = down ? ly.down : ly.gate, &W1 = ly.up;
   M8Args A;
@@ -529,6 +542,12 @@ cudaError_t launch_tc_mx8(const Launch &L, const LayerDev &ly, bool down, const 
   A.n_tiles = t.n;
   A.next = t.next + (down ? 1 : 0);
   A.rec = rec;
+  A.w0 = W0.plane[0];
+  A.w0_stride = W0.stride[0];
+  A.w1 = W1.plane[0];
+  A.w1_stride = W1.stride[0];
+  A.x = x;
+  A.src_row = src_row;
   A.bias0 = down ? ly.bias_down : ly.bias_gate;
   A.bias1 = down ? nullptr : ly.bias_up;
   A.wts = !down && ly.desc.weight_fold == PM_FOLD_BEFORE_DOWN ? wts : nullptr;

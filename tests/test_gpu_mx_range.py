@@ -74,3 +74,40 @@ def test_activations_that_round_up_past_the_largest_float(ctx, rows_ctx, oracle,
     agree(gl.experts(x, ids, w), want)
     gl.close()
     gr.close()
+
+
+@pytest.mark.parametrize("shape", ["c3", "c3-wide"])
+@pytest.mark.parametrize("T", [1, 5, 31, 40])
+def test_activations_that_are_no_finite_number(ctx, rows_ctx, oracle, T, shape):
+    """One infinity (or NaN) in a 32-value block spoils the sums that f32 arithmetic spoils and no others: inf where it meets a
+    weight, NaN where it meets a zero or its opposite. 0.03 of the codes of its column are zeros here, so most sums are
+    infinite and the clamp of the activation makes them finite again."""
+    cfg = SMALL["c3"] if shape == "c3" else SMALL["c3"].scaled(d=288, ff=1120)
+    W = synth.make_weights(cfg, 93)
+    rng = np.random.default_rng(94)
+    for key in ("gate", "up"):
+        c = codes(W, key, cfg)
+        low = np.where(rng.random(c.shape[:2]) < 0.03, 0, rng.integers(1, 8, c.shape[:2]) | 8 * rng.integers(0, 2, c.shape[:2]))
+        c[:, :, 1, 4] = (c[:, :, 1, 4] & 0xF0) | low  # value 3 of block 1: x[35]
+    ol, gl, gr = layers(oracle, ctx, rows_ctx, cfg, W)
+    x = synth.make_activations(T, cfg.d, 95)
+    x[0, 35] = np.inf
+    if T > 4:
+        x[2, 35] = -np.inf
+        x[2, 36] = np.inf
+        x[3, 35] = np.nan
+        x[T - 1, 35] = -np.inf
+    ids, w = picks(T, cfg)
+    with np.errstate(all="ignore"):
+        want = ol.experts(x, ids, w)
+        agree(gr.experts(x, ids, w), want)
+        agree(gl.experts(x, ids, w), want)
+        # the down products meet them in h
+        h_inf = cfg.scaled(act_limit=np.inf)
+        ol2, gl2, gr2 = layers(oracle, ctx, rows_ctx, h_inf, W)
+        want = ol2.experts(x, ids, w)
+        assert not np.isfinite(want).all()
+        agree(gr2.experts(x, ids, w), want)
+        agree(gl2.experts(x, ids, w), want)
+    for g in (gl, gr, gl2, gr2):
+        g.close()
