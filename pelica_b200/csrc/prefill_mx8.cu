@@ -420,8 +420,8 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
             *(uint2 *)(dst + (((2 * i) ^ (m & 7)) << 4)) = make_uint2(q[i].x, q[i].y);
             *(uint2 *)(dst + (((2 * i + 1) ^ (m & 7)) << 4)) = make_uint2(q[i].z, q[i].w);
           }
-          // (255, which the format reserves, counts as 254)
-          *(uint32_t *)(sSA + part * 512 + (m & 31) * 16 + (m >> 5) * 4) = __vminu4((uint32_t)(sc >> (32 * part)), 0xfefefefeu);
+          // (255 is a NaN to the tensor cores, 2^127 of the doubled codes elsewhere: mx_repair's)
+          *(uint32_t *)(sSA + part * 512 + (m & 31) * 16 + (m >> 5) * 4) = (uint32_t)(sc >> (32 * part));
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
           if (lane == 0) tc_mbar_arrive(a_ready + part);

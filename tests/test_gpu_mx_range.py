@@ -111,3 +111,30 @@ def test_activations_that_are_no_finite_number(ctx, rows_ctx, oracle, T, shape):
         agree(gl2.experts(x, ids, w), want)
     for g in (gl, gr, gl2, gr2):
         g.close()
+
+
+@pytest.mark.parametrize("e", [0, 1, 2, 129, 249, 250, 253, 254, 255])
+@pytest.mark.parametrize("T", [3, 40])
+def test_scale_bytes_of_the_whole_range(ctx, rows_ctx, oracle, T, e):
+    """A gate matrix whose blocks all have scale byte e, against activations that bring its sums back into range: fp8 products
+    (five and four pieces). 255 is 2^128 as in the row kernels: codes of 1 and more are
+    infinite, 0.5 is 2^127."""
+    cfg = SMALL["c3"].scaled(act_limit=1e30)
+    W = synth.make_weights(cfg, 96)
+    c = codes(W, "gate", cfg)
+    c[..., 0] = e
+    if e == 255:  # finite sums: codes of 0 and 0.5 only
+        c[..., 1:] &= 0x99
+    ol, gl, gr = layers(oracle, ctx, rows_ctx, cfg, W)
+    x = synth.make_activations(T, cfg.d, 97) * np.float32(2.0) ** int(np.clip(120 - e, -100, 60))
+    ids, w = picks(T, cfg)
+    want = ol.experts(x, ids, w)
+    assert np.isfinite(want).all() and want.any()
+    agree(gr.experts(x, ids, w), want)
+    got = gl.experts(x, ids, w)
+    agree(got, want)
+    if T < 32:
+        rms = float(np.sqrt((want.astype(np.float64) ** 2).mean()))
+        assert float(np.abs(got - want).max()) < 4e-6 * rms
+    gl.close()
+    gr.close()
