@@ -1032,7 +1032,7 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
     {
       PROF(c, PH_GATEUP);
       CU(small ? launch_tc_mx8(L, dv, false, g.pair_src, tt, S.rec, x, g.pair_token, w, S.h, 1, 0, c->dev_err, c->wait_ns)
-               : launch_tc_mx(L, dv, false, g.pair_src, tt, S.rec, w, S.h, c->dev_err, c->wait_ns));
+               : launch_tc_mx(L, dv, false, g.pair_src, tt, S.rec, x, g.pair_token, w, S.h, c->dev_err, c->wait_ns));
     }
     {
       PROF(c, PH_QUANT_H);
@@ -1042,7 +1042,7 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
       PROF(c, PH_DOWN);
       CU(small ? launch_tc_mx8(L, dv, true, g.pair_src, tt, S.rec, S.h, nullptr, nullptr, S.eo, S.eo_parts, (size_t)P * D.d, c->dev_err,
                                c->wait_ns)
-               : launch_tc_mx(L, dv, true, g.pair_src, tt, S.rec, nullptr, S.eo, c->dev_err, c->wait_ns));
+               : launch_tc_mx(L, dv, true, g.pair_src, tt, S.rec, S.h, nullptr, nullptr, S.eo, c->dev_err, c->wait_ns));
     }
     c->path_count[PM_PATH_TENSOR] += 2;
     CU(cudaGetLastError());

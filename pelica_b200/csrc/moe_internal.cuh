@@ -231,7 +231,7 @@ int mx_splits(const pm_layer_desc &D, int n_pairs);
 void launch_mx_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x, uint8_t *rec);
 void launch_mx8_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x, uint8_t *rec);
 cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
-                         const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns);
+                         const uint8_t *rec, const float *x, const uint32_t *src_row, const float *wts, float *out, int *err, unsigned long long wait_ns);
 cudaError_t launch_tc_mx8(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
                           const uint8_t *rec, const float *x, const uint32_t *src_row, const float *wts, float *out, int splits,
                           size_t split_stride, int *err, unsigned long long wait_ns);

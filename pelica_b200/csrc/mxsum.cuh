@@ -1,8 +1,9 @@
 // mxsum.cuh - sums of an MXFP4 row that the tensor-core products cannot make, once more in f32.
-// An activation that is no finite number has no pieces (its block's are NaN), scale byte 255 is no number, and a sum may leave a float's range piece by
-// piece where the f32 sum does not. Such a sum comes out as an infinity or a NaN: it is made again from the weights and
-// rows as stored, with the operations of the row kernels (kernels_basic.cu, rows_mx_f32). Rare: a thread's own loop over K;
-// where every sum is finite it costs an fma an output.
+// An activation that is no finite number has no pieces (its block's are NaN), scale byte 255 is no number, weights of 2^128
+// and more (scale bytes from 253 on) are no bf16, and a sum may leave a float's range piece by piece where the f32 sum
+// does not. Such a sum comes out as an infinity or a NaN: it is made again from the weights and rows as stored, with the
+// operations of the row kernels (kernels_basic.cu, rows_mx_f32). Rare: a thread's own loop over K; where every sum is
+// finite it costs an fma an output.
 #pragma once
 
 #include "tcgen.cuh"

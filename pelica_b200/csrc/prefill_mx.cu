@@ -22,7 +22,7 @@
 // in shared memory and took 128 rows.
 #include <cuda_bf16.h>
 
-#include "tcgen.cuh"
+#include "mxsum.cuh"
 
 #define MX_M 128
 #define MX_KC 64   /* K values of a chunk */
@@ -97,6 +97,10 @@ struct MxArgs {
   const int *n_tiles;
   unsigned int *next;
   const uint8_t *rec;     // the tokens' pieces (k_mx_rows)
+  const uint8_t *w0, *w1;       // the nibbles, the f32 rows and the row of each pair (null: its own), for mx_repair
+  size_t w0_stride, w1_stride;
+  const float *x;
+  const uint32_t *src_row;
   const float *bias0, *bias1;
   const float *wts;
   const uint32_t *pair_src;
@@ -402,6 +406,13 @@ __global__ void __launch_bounds__(MxShape::NT, 1) k_tc_mx(const __grid_constant_
       n_acc++;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const bool dead = *(volatile int *)A.err != 0;
+      // a sum once more in f32: matrix `second`, row r, token n of the tile
+      auto again = [&](bool second, int r, int n) {
+        const uint32_t p = T.y + (uint32_t)n;
+        return mx_sum_f32((second ? A.w1 + (size_t)el * A.w1_stride : A.w0 + (size_t)el * A.w0_stride) + (size_t)r * (A.cols / 2),
+                          (second ? A.s1 + (size_t)el * A.s1_stride : A.s0 + (size_t)el * A.s0_stride) + (size_t)r * nbk,
+                          A.x + (size_t)(A.src_row ? A.src_row[p] : p) * A.cols, 0, nbk);
+      };
       if (DOWN) {
         const float bd = A.bias0 && drow < rows ? A.bias0[(size_t)el * rows + drow] : 0.0f;
         const bool on = !dead && drow < rows, bias = A.bias0 != nullptr;
@@ -415,8 +426,13 @@ __global__ void __launch_bounds__(MxShape::NT, 1) k_tc_mx(const __grid_constant_
             uint32_t v[8];
             tc_ld8<0>(tlane + h * 128u + (uint32_t)(c0 + c8), v);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            float o[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) put(c0 + c8 + u, __uint_as_float(v[u]));
+            for (int u = 0; u < 8; u++) o[u] = __uint_as_float(v[u]);
+            mx_repair(o, [&](int u) { return on && c0 + c8 + u < nvalid; }, [&](int u) { return again(false, drow, c0 + c8 + u); });
+#pragma unroll
+            for (int u = 0; u < 8; u++) put(c0 + c8 + u, o[u]);
+            __syncwarp();
           }
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
@@ -442,9 +458,18 @@ __global__ void __launch_bounds__(MxShape::NT, 1) k_tc_mx(const __grid_constant_
             tc_ld4<0>(tlane + (uint32_t)(c0 + c4), vg);
             tc_ld4<128>(tlane + (uint32_t)(c0 + c4), vu);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            float o[8];  // gate, then up
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              o[u] = __uint_as_float(vg[u]);
+              o[4 + u] = __uint_as_float(vu[u]);
+            }
+            mx_repair(o, [&](int u) { return on && c0 + c4 + (u & 3) < nvalid; },
+                      [&](int u) { return again(u >= 4, hrow, c0 + c4 + (u & 3)); });
 #pragma unroll
             for (int u = 0; u < 4; u++)
-              if (on && c0 + c4 + u < nvalid) put(c0 + c4 + u, __uint_as_float(vg[u]), __uint_as_float(vu[u]));
+              if (on && c0 + c4 + u < nvalid) put(c0 + c4 + u, o[u], o[4 + u]);
+            __syncwarp();
           }
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
@@ -484,14 +509,14 @@ template <bool DOWN> static cudaError_t mx_start(const Launch &L, const MxArgs &
 }
 
 // Tensor-core form of launch_gateup / launch_down for MXFP4 weights and f32 activations given as the pieces of
-// the grouping's rows.
+// the grouping's rows. x, src_row: the rows the pieces were made of (as in launch_mx_rows).
 cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
-                         const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns) {
+                         const uint8_t *rec, const float *x, const uint32_t *src_row, const float *wts, float *out, int *err, unsigned long long wait_ns) {
   if (t.max_tiles == 0) return cudaSuccess;
   const WMat &W0 = down ? ly.down : ly.gate, &W1 = ly.up;
   const WMaps &M0 = down ? ly.maps->down : ly.maps->gate, &M1 = ly.maps->up;
   MxArgs A;
-    A.m0 = M0.m[1];  // boxes of 128 rows
+  A.m0 = M0.m[1];  // boxes of 128 rows
   A.m1 = M1.m[1];
   A.s0 = W0.plane[1];
   A.s0_stride = W0.stride[1];
@@ -501,6 +526,12 @@ cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const u
   A.n_tiles = t.n;
   A.next = t.next + (down ? 1 : 0);
   A.rec = rec;
+  A.w0 = W0.plane[0];
+  A.w0_stride = W0.stride[0];
+  A.w1 = W1.plane[0];
+  A.w1_stride = W1.stride[0];
+  A.x = x;
+  A.src_row = src_row;
   A.bias0 = down ? ly.bias_down : ly.bias_gate;
   A.bias1 = down ? nullptr : ly.bias_up;
   A.wts = !down && ly.desc.weight_fold == PM_FOLD_BEFORE_DOWN ? wts : nullptr;

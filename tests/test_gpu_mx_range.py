@@ -77,7 +77,7 @@ def test_activations_that_round_up_past_the_largest_float(ctx, rows_ctx, oracle,
 
 
 @pytest.mark.parametrize("shape", ["c3", "c3-wide"])
-@pytest.mark.parametrize("T", [1, 5, 31, 40])
+@pytest.mark.parametrize("T", [1, 5, 31, 40, 150])
 def test_activations_that_are_no_finite_number(ctx, rows_ctx, oracle, T, shape):
     """One infinity (or NaN) in a 32-value block spoils the sums that f32 arithmetic spoils and no others: inf where it meets a
     weight, NaN where it meets a zero or its opposite. 0.03 of the codes of its column are zeros here, so most sums are
@@ -114,10 +114,10 @@ def test_activations_that_are_no_finite_number(ctx, rows_ctx, oracle, T, shape):
 
 
 @pytest.mark.parametrize("e", [0, 1, 2, 129, 249, 250, 253, 254, 255])
-@pytest.mark.parametrize("T", [3, 40])
+@pytest.mark.parametrize("T", [3, 40, 150])
 def test_scale_bytes_of_the_whole_range(ctx, rows_ctx, oracle, T, e):
     """A gate matrix whose blocks all have scale byte e, against activations that bring its sums back into range: fp8 products
-    (five and four pieces). 255 is 2^128 as in the row kernels: codes of 1 and more are
+    (3 and 40 tokens: five and four pieces), bf16 products (150: a weight of 2^128 is none). 255 is 2^128 as in the row kernels: codes of 1 and more are
     infinite, 0.5 is 2^127."""
     cfg = SMALL["c3"].scaled(act_limit=1e30)
     W = synth.make_weights(cfg, 96)
