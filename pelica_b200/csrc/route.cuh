@@ -17,10 +17,66 @@ __device__ __forceinline__ float pm_funkey(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
-// lane L holds experts L, L+32, ... (NP per lane, NP*32 >= E); `lg` points at the
-// token's E logits (any address space); ssv[E], gsc[E/2], keep[E/2] are per-warp
-// scratch in shared memory (used for group-limited selection only). Lane k < K
-// writes ids_out[k], w_out[k].
+// Group-limited selection (this repository's definition): a group's score = the sum of its two largest biased scores, the
+// second no lower than PM_NEG; the best topk_group groups stay, ties -> lower group index. These two say it step by
+// step, for one thread; the warp-wide forms below give the same and leave what is no number (a NaN in a bias or a router
+// row) to them.
+__device__ __forceinline__ float pm_group_score(const float *sv, int gs) {
+  int i1 = 0;
+  float v1 = sv[0], v2 = PM_NEG;
+#pragma unroll 1
+  for (int i = 1; i < gs; i++)
+    if (sv[i] > v1) { v1 = sv[i]; i1 = i; }
+#pragma unroll 1
+  for (int i = 0; i < gs; i++)
+    if (i != i1 && sv[i] > v2) v2 = sv[i];
+  return __fadd_rn(v1, v2);
+}
+__device__ __forceinline__ void pm_group_keep(const float *gsc, int G, int topk_group, unsigned char *keep) {
+#pragma unroll 1
+  for (int g = 0; g < G; g++) keep[g] = 0;
+#pragma unroll 1
+  for (int r = 0; r < topk_group; r++) {
+    int bg = -1;
+    float bv = 0.0f;
+#pragma unroll 1
+    for (int g = 0; g < G; g++) {
+      if (keep[g]) continue;
+      const float v = gsc[g];
+      if (bg < 0 || v > bv) { bv = v; bg = g; }
+    }
+    keep[bg] = 1;
+  }
+}
+// the score of a group of 32 from its scores, one a lane (sv: the same in memory); all lanes get it
+__device__ __forceinline__ float pm_group_score32(float v, const float *sv) {
+  if (__any_sync(PM_FULL, v != v)) return pm_group_score(sv, 32);
+  const uint32_t key = pm_fkey(v), m1 = __reduce_max_sync(PM_FULL, key);
+  const uint32_t top = __ballot_sync(PM_FULL, key == m1);
+  const uint32_t m2 = __reduce_max_sync(PM_FULL, key == m1 && !(top & (top - 1)) ? 0u : key);
+  return __fadd_rn(pm_funkey(m1), fmaxf(pm_funkey(m2), PM_NEG));
+}
+// one warp: which of G groups stay
+__device__ __forceinline__ void pm_group_rank(const float *gsc, int G, int topk_group, int lane, unsigned char *keep) {
+  bool odd = false;
+#pragma unroll 1
+  for (int g = lane; g < G; g += 32) {  // kept when fewer than topk_group groups come before it
+    const float mine = gsc[g];
+    int before = 0;
+#pragma unroll 1
+    for (int j = 0; j < G; j++) {
+      const float v = gsc[j];
+      before += v > mine || (v == mine && j < g);
+    }
+    keep[g] = before < topk_group;
+    odd = odd || mine != mine;
+  }
+  if (__any_sync(PM_FULL, odd)) {
+    __syncwarp();
+    if (lane == 0) pm_group_keep(gsc, G, topk_group, keep);
+  }
+}
+
 // Scores of one token by one warp. lane L holds experts L, L+32, ... (NP per lane,
 // NP*32 >= E); `lg` points at the token's E logits (any address space); ssv[E],
 // gsc[E/2], keep[E/2] are per-warp scratch in shared memory (group-limited
@@ -73,9 +129,6 @@ __device__ __forceinline__ void pm_route_scores(const pm_layer_desc &D, const fl
     int e = lane + 32 * i;
     sv[i] = e < E ? (sel_bias ? __fadd_rn(pr[i], sel_bias[e]) : pr[i]) : PM_NEG;
   }
-  // group-limited selection (this repository's definition: group score = sum of
-  // the group's two largest biased scores; best topk_group groups stay, ties ->
-  // lower group index)
   if (D.n_group > 0) {
 #pragma unroll
     for (int i = 0; i < NP; i++)
@@ -86,49 +139,14 @@ __device__ __forceinline__ void pm_route_scores(const pm_layer_desc &D, const fl
 #pragma unroll
       for (int i = 0; i < NP; i++)
         if (i < G) {
-          const uint32_t key = pm_fkey(sv[i]), m1 = __reduce_max_sync(PM_FULL, key);
-          const uint32_t top = __ballot_sync(PM_FULL, key == m1);
-          const uint32_t m2 = (top & (top - 1)) ? m1 : __reduce_max_sync(PM_FULL, key == m1 ? 0u : key);
-          if (lane == i) {
-            gsc[i] = __fadd_rn(pm_funkey(m1), pm_funkey(m2));
-            keep[i] = 0;
-          }
+          const float s = pm_group_score32(sv[i], ssv + 32 * i);
+          if (lane == i) gsc[i] = s;
         }
-    } else
-    for (int g = lane; g < G; g += 32) {  // lane g scores groups g, g+32, ...
-      int i1 = 0;
-      float v1 = ssv[g * gs];
-      for (int i = 1; i < gs; i++)
-        if (ssv[g * gs + i] > v1) { v1 = ssv[g * gs + i]; i1 = i; }
-      float v2 = PM_NEG;
-      for (int i = 0; i < gs; i++)
-        if (i != i1 && ssv[g * gs + i] > v2) v2 = ssv[g * gs + i];
-      gsc[g] = __fadd_rn(v1, v2);
-      keep[g] = 0;
+    } else {
+      for (int g = lane; g < G; g += 32) gsc[g] = pm_group_score(ssv + g * gs, gs);  // lane g scores groups g, g+32, ...
     }
     __syncwarp();
-    if (G <= 32) {  // lane g ranks group g: kept when fewer than topk_group groups come before it
-      if (lane < G) {
-        const float mine = gsc[lane];
-        int before = 0;
-        for (int g = 0; g < G; g++) {
-          const float v = gsc[g];
-          before += v > mine || (v == mine && g < lane);
-        }
-        keep[lane] = before < D.topk_group;
-      }
-    } else if (lane == 0) {
-      for (int r = 0; r < D.topk_group; r++) {
-        int bg = -1;
-        float bv = 0.0f;
-        for (int g = 0; g < G; g++) {
-          if (keep[g]) continue;
-          float v = gsc[g];
-          if (bg < 0 || v > bv) { bv = v; bg = g; }
-        }
-        keep[bg] = 1;
-      }
-    }
+    pm_group_rank(gsc, G, D.topk_group, lane, keep);
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < NP; i++) {
@@ -198,40 +216,20 @@ __device__ __forceinline__ void pm_route_pick(const pm_layer_desc &D, const floa
   const int E = D.n_exp, K = D.top_k;
   float *gsc = rest, *sel_p = rest + E / 2 + (E / 2 + 3) / 4;
   unsigned char *keep = (unsigned char *)(rest + E / 2);
-  if (D.n_group > 0) {  // the definition is pm_route_scores'
+  if (D.n_group > 0) {
     const int G = D.n_group, gs = E / G;
     if (gs == 32) {
 #pragma unroll 1
       for (int g = 0; g < G; g++) {
-        const uint32_t key = pm_fkey(sv[32 * g + lane]), m1 = __reduce_max_sync(PM_FULL, key);
-        const uint32_t top = __ballot_sync(PM_FULL, key == m1);
-        const uint32_t m2 = __reduce_max_sync(PM_FULL, key == m1 ? 0u : key);
-        if (lane == 0) gsc[g] = __fadd_rn(pm_funkey(m1), pm_funkey((top & (top - 1)) ? m1 : m2));
+        const float s = pm_group_score32(sv[32 * g + lane], sv + 32 * g);
+        if (lane == 0) gsc[g] = s;
       }
     } else {
 #pragma unroll 1
-      for (int g = lane; g < G; g += 32) {
-        int i1 = 0;
-        float v1 = sv[g * gs], v2 = PM_NEG;
-        for (int i = 1; i < gs; i++)
-          if (sv[g * gs + i] > v1) { v1 = sv[g * gs + i]; i1 = i; }
-        for (int i = 0; i < gs; i++)
-          if (i != i1 && sv[g * gs + i] > v2) v2 = sv[g * gs + i];
-        gsc[g] = __fadd_rn(v1, v2);
-      }
+      for (int g = lane; g < G; g += 32) gsc[g] = pm_group_score(sv + g * gs, gs);
     }
     __syncwarp();
-#pragma unroll 1
-    for (int g = lane; g < G; g += 32) {  // kept when fewer than topk_group groups come before it
-      const float mine = gsc[g];
-      int before = 0;
-#pragma unroll 1
-      for (int j = 0; j < G; j++) {
-        const float v = gsc[j];
-        before += v > mine || (v == mine && j < g);
-      }
-      keep[g] = before < D.topk_group;
-    }
+    pm_group_rank(gsc, G, D.topk_group, lane, keep);
     __syncwarp();
 #pragma unroll 1
     for (int e = lane; e < E; e += 32)

@@ -150,3 +150,34 @@ def test_width_limit(ctx):
     with pytest.raises(pb.PelicaError) as e:
         pb.MoeLayer(ctx, synth.C2_QWEN3.scaled(n_exp=8, top_k=2, d=65536, ff=256))
     assert e.value.code == -7
+
+
+@pytest.mark.parametrize("mask", [-np.inf, np.nan])
+def test_groups_of_32_with_masked_experts(ctx, oracle, mask):
+    """Groups as wide as a warp are scored by two reductions. An expert masked by a bias of -inf leaves its group's
+    second score at -3e38 as in the other widths: a group with one live expert comes before a group with none. A NaN in
+    a group's biases counts for nothing, and for the whole group where it is the first. One token, a few, a tile, several segments; the decode kernel's form too."""
+    cfg = synth.C4_DSV3.scaled(n_exp=128, n_group=4, topk_group=2, top_k=8, d=512, ff=256, shared=0)
+    W = synth.make_weights(cfg, 45)
+    b = np.zeros(128, np.float32)
+    if np.isnan(mask):
+        b[:32], b[32:64], b[96:] = -0.5, 0.5, 0.75
+        b[5] = b[96] = mask    # neither group stays: a weak one, and the strongest
+    else:
+        b[32:] = mask          # groups 1 and 3: nobody
+        b[64 + 7] = 1e32       # group 2: one, whose score still shows beside -3e38
+    W["select_bias"] = b
+    ol = oracle.Layer(oracle.LayerDesc(**cfg.desc_fields()), W)
+    gl = pb.MoeLayer(ctx, cfg).load(W)
+    x = synth.make_activations(70, cfg.d, 46)
+    want, w_want = ol.route(x)
+    for T in (1, 5, 9, 70):
+        ids, w = gl.route(x[:T])
+        assert np.array_equal(ids, want[:T]) and bits_equal(w, w_want[:T])
+        assert bits_equal(gl.forward(x[:T]), ol.forward(x[:T]))
+    if not np.isnan(mask):
+        assert (want[:, 0] == 71).all()
+    st = pb.Stack(ctx, [gl, gl])
+    assert bits_equal(st.forward(x[:1]), oracle.stack_forward([ol, ol], 1e-6, x[:1]))
+    st.close()
+    gl.close()
