@@ -950,7 +950,22 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
     bulk(xs, wr + (size_t)e0 * d, wb);
   }
   uint32_t ph = 0;
-  for (int t0 = 0; t0 < T; t0 += tg, ph ^= 1) {
+  auto wait = [&](uint32_t phase, unsigned long long limit_ns) {  // bounded: the copies' own time, a few us
+    unsigned long long s0 = 0;
+    for (;;) {
+      uint32_t ok;
+      asm volatile(
+          "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+          : "=r"(ok) : "r"(bar), "r"(phase) : "memory");
+      if (ok) return true;
+      unsigned long long now;
+      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+      if (s0 == 0) s0 = now;
+      if (now - s0 > limit_ns) return false;
+    }
+  };
+  bool late = false;
+  for (int t0 = 0; t0 < T && !late; t0 += tg, ph ^= 1) {
     const int nt = min(tg, T - t0);
     if (t0 > 0) __syncthreads();  // everybody is done with the tokens before
     if (tid == 0) {
@@ -960,22 +975,17 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
       bulk(xs + (size_t)epc * d, x + (size_t)t0 * d, xb);
     }
     if (t0 == 0) pm_pdl_wait();
-    {  // bounded: the copies' own time, a few us
-      unsigned long long s0 = 0;
-      for (;;) {
-        uint32_t ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok) : "r"(bar), "r"(ph) : "memory");
-        if (ok) break;
-        unsigned long long now;
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
-        if (s0 == 0) s0 = now;
-        if (now - s0 > wait_ns) {
-          atomicCAS(err, 0, 9);
-          break;
-        }
+    // (given up by one thread is given up by all: nobody reads the areas, no further copy is started, and the one in flight
+    // has landed before the CTA goes on - its shared memory is the routing's next, or another CTA's)
+    late = __syncthreads_or(!wait(ph, wait_ns));
+    if (late) {
+      if (tid == 0) {
+        atomicCAS(err, 0, 9);
+        wait(ph, 100000000ull);
       }
+      __syncthreads();
+      for (int i = tid; i < ne * T; i += 256) logits[(size_t)(i / ne) * E + e0 + i % ne] = 0.0f;  // (the call reports the error)
+      break;
     }
     for (int i = warp; i < ne * nt; i += 8) {
       const int el = i % ne, t = i / ne;

@@ -320,15 +320,11 @@ __global__ void __launch_bounds__(MxShape::NT, 1) k_tc_mx(const __grid_constant_
       // the last copies have landed before the CTA gives up its shared memory
       for (uint32_t i = 1; i <= NSR && i <= nr; i++) {
         const uint32_t q = nr - i;
-        const unsigned long long t0 = tc_now();
-        while (!tc_bar_test(full_raw + q % NSR, (q / NSR) & 1) && tc_now() - t0 < A.wait_ns) {
-        }
+        tc_landed(full_raw + q % NSR, (q / NSR) & 1);
       }
       for (uint32_t i = 1; i <= NSB && i <= nbk_; i++) {
         const uint32_t q = nbk_ - i;
-        const unsigned long long t0 = tc_now();
-        while (!tc_bar_test(full_b + q % NSB, (q / NSB) & 1) && tc_now() - t0 < A.wait_ns) {
-        }
+        tc_landed(full_b + q % NSB, (q / NSB) & 1);
       }
     }
     __syncwarp();

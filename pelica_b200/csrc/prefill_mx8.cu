@@ -305,9 +305,7 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
       // the last copies have landed before the CTA gives up its shared memory
       for (uint32_t i = 1; i <= NSR && i <= nr; i++) {
         const uint32_t q = nr - i;
-        const unsigned long long t0 = tc_now();
-        while (!tc_bar_test(full_raw + q % NSR, (q / NSR) & 1) && tc_now() - t0 < A.wait_ns) {
-        }
+        tc_landed(full_raw + q % NSR, (q / NSR) & 1);
       }
     }
     __syncwarp();
@@ -340,9 +338,7 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
     if (lane == 0)  // (as above)
       for (int a = 0; a < 2; a++) {
         const uint32_t n = a ? n_a[1] : n_a[0];
-        const unsigned long long t0 = tc_now();
-        while (n > 0 && !tc_bar_test(a_ready + a, (n - 1) & 1) && tc_now() - t0 < A.wait_ns) {
-        }
+        if (n > 0) tc_landed(a_ready + a, (n - 1) & 1);
       }
     __syncwarp();
   } else {

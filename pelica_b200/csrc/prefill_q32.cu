@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
       int cur = (int)blockIdx.x, nxt = cur + G;
       uint4 Tc = make_uint4(Q32_END, 0, 0, 0), Tn = Tc;
       if (cur < n_items) Tc = __ldg(A.tiles + cur / A.row_tiles);
-      uint32_t sr = 0, pr = 1, sb = 0, pb = 1, nr = 0;
+      uint32_t sr = 0, pr = 1, sb = 0, pb = 1, nr = 0, ntk = 0;  // (copies issued per ring)
       bool ok = true;
       for (int k = 0; ok; k++) {
         const int s = k & (Q32_IT - 1);
@@ -249,18 +249,20 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
           const int el = (int)Tc.x;
           const uint32_t per_block = ((Tc.z + 15) >> 4) * (16u * 36u);
           const uint8_t *rec = A.rec + (size_t)Tc.w * nb * 36;
-          for (int q = 0; q < nst; q++, nr++) {
+          for (int q = 0; q < nst; q++) {
             if (nr >= Q32_NSR && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
             const uint32_t r = sRaw_a + sr * RAWB;
             tc_mbar_expect(full_raw + sr, (uint32_t)RAWB);  // (a box past the matrix reads zeros)
             tc_tma3(r, &A.m0, q * RROW, r0, el, full_raw + sr);  // boxes of 128 rows (down) or 64
             if (!DOWN) tc_tma3(r + RAWB / 2, &A.m1, q * RROW, r0, el, full_raw + sr);
-            if (nr >= Q32_NSB && !tc_wait(empty_b + sb, pb, A.err, A.wait_ns)) { ok = false; nr++; break; }
+            nr++;
+            if (ntk >= Q32_NSB && !tc_wait(empty_b + sb, pb, A.err, A.wait_ns)) { ok = false; break; }
             const uint32_t bytes = per_block * (uint32_t)min(Q32_KB, nb - q * Q32_KB);
             tc_mbar_expect(full_b + sb, bytes);
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sB_a + sb * Q32_BST),
                          "l"(rec + (size_t)q * (per_block * Q32_KB)), "r"(bytes), "r"(tc_s32(full_b + sb))
                          : "memory");
+            ntk++;
             if (++sr == Q32_NSR) { sr = 0; pr ^= 1; }
             if (++sb == Q32_NSB) { sb = 0; pb ^= 1; }
           }
@@ -270,14 +272,8 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
         Tc = Tn;
       }
       // the last copies have landed before the CTA gives up its shared memory
-      static_assert(Q32_NSR == Q32_NSB, "one count serves both rings");
-      for (uint32_t i = 1; i <= Q32_NSR && i <= nr; i++) {
-        const uint32_t q = nr - i;
-        const unsigned long long t0 = tc_now();
-        while (!(tc_bar_test(full_raw + q % Q32_NSR, (q / Q32_NSR) & 1) && (!ok || tc_bar_test(full_b + q % Q32_NSB, (q / Q32_NSB) & 1))) &&
-               tc_now() - t0 < A.wait_ns) {
-        }
-      }
+      for (uint32_t i = 1; i <= Q32_NSR && i <= nr; i++) tc_landed(full_raw + (nr - i) % Q32_NSR, ((nr - i) / Q32_NSR) & 1);
+      for (uint32_t i = 1; i <= Q32_NSB && i <= ntk; i++) tc_landed(full_b + (ntk - i) % Q32_NSB, ((ntk - i) / Q32_NSB) & 1);
     }
     __syncwarp();
   } else {

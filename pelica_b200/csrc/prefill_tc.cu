@@ -522,15 +522,11 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
       // the last copies have landed before the CTA gives up its shared memory
       for (uint32_t i = 1; i <= NS && i <= nr; i++) {
         const uint32_t g = nr - i;
-        const unsigned long long t0 = tc_now();
-        while (!tc_bar_test(full_raw + g % NS, (g / NS) & 1) && tc_now() - t0 < A.wait_ns) {
-        }
+        tc_landed(full_raw + g % NS, (g / NS) & 1);
       }
       for (uint32_t i = 1; i <= NSB && i <= nbk; i++) {
         const uint32_t g = nbk - i;
-        const unsigned long long t0 = tc_now();
-        while (!tc_bar_test(full_b + g % NSB, (g / NSB) & 1) && tc_now() - t0 < A.wait_ns) {
-        }
+        tc_landed(full_b + g % NSB, (g / NSB) & 1);
       }
     }
     __syncwarp();

@@ -139,6 +139,14 @@ __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, int *err
   atomicCAS(err, 0, 7);
   return false;
 }
+// A copy still in flight lands in whatever the SM's shared memory holds next: before a CTA ends - also when a wait ran
+// out and it gives up - its last copies are waited for, with a limit that is not the call's (a copy takes microseconds).
+#define TC_LANDED_NS 100000000ull
+__device__ __forceinline__ void tc_landed(uint64_t *bar, uint32_t parity) {
+  const unsigned long long t0 = tc_now();
+  while (!tc_bar_test(bar, parity) && tc_now() - t0 < TC_LANDED_NS) {
+  }
+}
 // Two f32 in one register pair. A product whose rounded value goes into an addition is written as
 // fma(a, b, -0) with a -0 that the compiler cannot see (a kernel parameter): it contracts a plain
 // mul.rn.f32x2 and the add.rn.f32x2 behind it into one fma, which has other bits than the reference's

@@ -31,3 +31,18 @@ def test_places_go_back_after_their_words_arrived(name):
 def test_the_arrival_depends_on_the_words():
     helper = source("tcgen.cuh").split("tc_mbar_arrive_used")[1].split("tc_mbar_expect")[0]
     assert re.search(r"and\.b32 a, %1, %2;.*add\.u32 a, a, %0;.*arrive[^;]*\[a\]", helper.replace("\n", " "))
+
+
+def test_copies_in_flight_are_waited_for():
+    """No CTA ends with a copy on its way into its shared memory, also where a wait ran out: every ring's last copies are
+    waited for, each ring by its own count, with a limit that a caller's short one does not shorten."""
+    rings = {"prefill_tc.cu": ("full_raw", "full_b"), "prefill_mx.cu": ("full_raw", "full_b"),
+             "prefill_mx8.cu": ("full_raw", "a_ready"), "prefill_q32.cu": ("full_raw", "full_b")}
+    for name, bars in rings.items():
+        text = source(name)
+        for bar in bars:
+            assert re.search(r"tc_landed\(%s \+" % bar, text), (name, bar)
+        assert "< A.wait_ns" not in text, name
+    assert "wait_ns" not in source("tcgen.cuh").split("TC_LANDED_NS")[1].split("tc_pack2")[0]
+    few = source("kernels_basic.cu").split("k_route_plan_small")[1].split("the last CTA")[0]
+    assert re.search(r"atomicCAS\(err, 0, 9\);\s*wait\(ph, \d+ull\);", few)
