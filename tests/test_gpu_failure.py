@@ -12,6 +12,14 @@ from tests.helpers import SMALL, bits_equal, make_pair
 pytestmark = [pytest.mark.gpu, pytest.mark.timeout(600)]
 
 
+@pytest.fixture(scope="module")
+def ctx():
+    """A context of this file's own: the threshold it sets stays set."""
+    c = pb.Context(0)
+    yield c
+    c.close()
+
+
 def test_decode_kernel_wait_runs_out_and_the_stack_falls_back(ctx, oracle):
     cfg = SMALL["c2"]
     ols, gls = [], []

@@ -10,6 +10,14 @@ from tests.helpers import SMALL, bits_equal, make_pair
 pytestmark = [pytest.mark.gpu, pytest.mark.timeout(600)]
 
 
+@pytest.fixture(scope="module")
+def ctx():
+    """A context of this file's own: the threshold it sets stays set."""
+    c = pb.Context(0)
+    yield c
+    c.close()
+
+
 @pytest.mark.parametrize("name", ["c1", "c2", "c4"])
 @pytest.mark.parametrize("T", [32, 77, 300])
 def test_tensor_core_path_matches_oracle_and_general(ctx, oracle, name, T):

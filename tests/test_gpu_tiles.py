@@ -35,19 +35,23 @@ def test_32_value_blocks(ctx, oracle, shape, T):
     gl.close()
 
 
-@pytest.mark.parametrize("T", [2, 5, 31, 32, 40, 150])
-@pytest.mark.parametrize("shape", ["c3", "c3-shard", "c3-wide"])
+@pytest.mark.parametrize("T", [1, 2, 5, 31, 32, 40, 150])
+@pytest.mark.parametrize("shape", ["c3", "c3-shard", "c3-wide", "c3-2048", "c3-2080"])
 def test_mxfp4(ctx, oracle, shape, T):
     """MXFP4 weights and f32 activations: five or four fp8 pieces in tiles of 16 or 32 tokens, two bf16 pieces in tiles
-    of 128. ff = 160: a last stage of one block; the wide shape cuts the down products along K; calls of
-    fewer than 32 tokens keep f32 precision."""
+    of 128. ff = 160: a last stage of one block; the wider shapes cut the down products of a few tokens along K, into two parts
+    (ff = 1120), four (2048: 16 stages) and three (2080: 17); calls of fewer than 32 tokens keep f32 precision."""
     cfg = {"c3-shard": SMALL["c3"].scaled(first_local_expert=2, n_exp_local=4),
-           "c3-wide": SMALL["c3"].scaled(d=288, ff=1120)}.get(shape) or SMALL[shape]
+           "c3-wide": SMALL["c3"].scaled(d=288, ff=1120), "c3-2048": SMALL["c3"].scaled(d=288, ff=2048),
+           "c3-2080": SMALL["c3"].scaled(d=288, ff=2080)}.get(shape) or SMALL[shape]
     ol, gl, _ = make_pair(oracle, pb, ctx, cfg, 82)
     x = synth.make_activations(T, cfg.d, 950 + T)
     x[0, :32] *= 1e-12  # blocks of very different sizes, and one of zeros
-    x[1, 32:64] = 0.0
+    x[T - 1, 32:64] = 0.0
+    c0 = ctx.path_counts()
     got = gl.forward(x)
+    c1 = ctx.path_counts()
+    assert c1["tensor"] - c0["tensor"] == 2 and c1["general"] == c0["general"]
     want = ol.forward(x)
     assert tol_ok(got, want), float(np.abs(got - want).max())
     if T < 32:
@@ -68,7 +72,13 @@ def test_q8x_blocks_and_plan(ctx, oracle, shape, T):
     ids, w = gl.route(x)
     ids_o, w_o = ol.route(x)
     assert np.array_equal(ids, ids_o) and bits_equal(w, w_o)
-    assert bits_equal(gl.forward(x), ol.forward(x))
+    c0 = ctx.path_counts()
+    got = gl.forward(x)
+    c1 = ctx.path_counts()
+    # one token takes the row kernels where no shared expert joins the launches
+    kind, other = ("general", "tensor") if T == 1 and not cfg.shared else ("tensor", "general")
+    assert c1[kind] - c0[kind] == 2 and c1[other] == c0[other]
+    assert bits_equal(got, ol.forward(x))
     # rows that start 4 bytes off a 16-byte boundary take other loads, not other values
     xd, yd = ctx.alloc(x.nbytes + 16), ctx.alloc(x.nbytes + 16)
     xd.upload(np.concatenate([np.zeros(1, np.float32), x.ravel(), np.zeros(3, np.float32)]))
