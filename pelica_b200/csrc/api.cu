@@ -873,7 +873,7 @@ static size_t scratch_rec_bytes(const pm_layer_desc &D, int T) {
   if (q32_layer(D)) return q32_rec_bytes(T * D.top_k, D.n_exp, std::max(D.d, D.ff));
   if (mx_layer(D)) {
     const int P = T * D.top_k, cols = std::max(D.d, D.ff);
-    return std::max(mx_rec_bytes(P, D.n_exp, cols), mx8_rec_bytes(P, D.n_exp, cols));
+    return std::max(mx_rec_bytes(P, D.n_exp, cols), mx8_rec_bytes(T, P, D.n_exp, cols));
   }
   if (D.act_quant != PM_AQ_Q8X_256) return 0;
   const int m = shared_merges(D) ? 1 : 0, P = T * (D.top_k + m), E = D.n_exp + m;

@@ -472,9 +472,10 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
   if (warp == MW) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
 }
 
-size_t mx8_rec_bytes(int n_pairs, int max_groups, int cols) {
-  const size_t groups = (size_t)(max_groups < n_pairs ? max_groups : n_pairs);
-  return (((size_t)n_pairs + 15 * groups) / 16 + 1) * ((cols + M8_KS - 1) / M8_KS) * (2048 * 5 + 512);
+// bytes of the pieces of a call of T tokens: n_pairs rows of `cols` values in at most max_groups groups
+size_t mx8_rec_bytes(int T, int n_pairs, int max_groups, int cols) {
+  const size_t groups = (size_t)(max_groups < n_pairs ? max_groups : n_pairs), pieces = T < PM_MX_PROMPT ? 5 : 4;
+  return (((size_t)n_pairs + 15 * groups) / 16 + 1) * ((cols + M8_KS - 1) / M8_KS) * (2048 * pieces + 512);
 }
 void launch_mx8_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x, uint8_t *rec) {
   const long units = ((long)n_rows + 15 * t.max_tiles) * (cols / 32);

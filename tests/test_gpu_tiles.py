@@ -89,3 +89,24 @@ def test_q8x_blocks_and_plan(ctx, oracle, shape, T):
     xd.free()
     yd.free()
     gl.close()
+
+
+def test_workspace_of_a_long_mxfp4_prompt():
+    """The pieces of a prompt take 4.25 bytes a value of workspace (four fp8 pieces and their scales; two bf16 pieces take
+    4): the five pieces of short calls are not kept room for."""
+    cfg, T = synth.C3_GPTOSS, 2048
+    c = pb.Context(0)
+    gl = pb.MoeLayer(c, cfg).fill_synthetic(5)
+    x, y = c.alloc(4 * T * cfg.d), c.alloc(4 * T * cfg.d)
+    before = c.device_free_bytes()
+    gl.forward_dev(x, T, y)
+    c.sync()
+    used = before - c.device_free_bytes()
+    P = T * cfg.top_k
+    # h f32 and its quantised forms (5.5 bytes), pair outputs, the tokens' quantised forms, the pieces of whole 128-value stages, room to stage x and y
+    need = P * cfg.ff * 5.5 + P * cfg.d * 4 + T * cfg.d * 2 + (P + 16 * cfg.n_exp) * 2944 * 4.25 + 2 * T * cfg.d * 4
+    assert used < 1.125 * need + (8 << 20), (used, need)  # (the workspace grows by an eighth more than asked for)
+    for b in (x, y):
+        b.free()
+    gl.close()
+    c.close()
