@@ -1883,9 +1883,8 @@ __global__ void __launch_bounds__(256) k_combine(int d, int K, int in_combine,
                                                  const float *__restrict__ w,
                                                  const float *__restrict__ shared_out,
                                                  const float *__restrict__ shared_logit, float *y,
-                                                 int accumulate, int parts, size_t part_stride, int early) {
-  if (early) pm_pdl_early();
-  else pm_pdl();
+                                                 int accumulate, int parts, size_t part_stride) {
+  pm_pdl();
   const int t = blockIdx.y;
   const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
   if (c >= d) return;
@@ -1935,17 +1934,14 @@ void launch_combine(const Launch &L, const LayerDev &ly, const float *eo, const 
   if (T == 0) return;
   int d = ly.desc.d;
   dim3 grid((d + 1023) / 1024, T);
-  // (a few tokens: the next layer's routing kernel fetches its rows meanwhile where they are a few us of HBM, 256 experts x
-  // 7168: 102 -> 97 us a layer)
-  const int early = T < PM_SMALL_ROUTE_TOKENS && (size_t)ly.desc.n_exp * d * 4 > (4u << 20);
   if (parts > 1)
     PLAUNCH(L, k_combine<true>, grid, 256, 0, d, ly.desc.top_k,
             (int)(ly.desc.weight_fold == PM_FOLD_IN_COMBINE), eo, pair_pos, w, shared_out,
-            shared_logit, y, (int)accumulate, parts, (size_t)T * ly.desc.top_k * d, early);
+            shared_logit, y, (int)accumulate, parts, (size_t)T * ly.desc.top_k * d);
   else
     PLAUNCH(L, k_combine<false>, grid, 256, 0, d, ly.desc.top_k,
             (int)(ly.desc.weight_fold == PM_FOLD_IN_COMBINE), eo, pair_pos, w, shared_out,
-            shared_logit, y, (int)accumulate, parts, (size_t)T * ly.desc.top_k * d, early);
+            shared_logit, y, (int)accumulate, parts, (size_t)T * ly.desc.top_k * d);
 }
 
 // x / rms(x), unit weight; the sum order is pm_rms_inv's (common.cuh)
