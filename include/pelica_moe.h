@@ -184,8 +184,9 @@ PM_API int32_t pm_ctx_destroy(pm_ctx *ctx);
 /* replaces: Pending::wait (src/ds4_gpu.rs:733) */
 PM_API int32_t pm_sync(pm_ctx *ctx);
 /* expert products run on the tensor cores when a call has at least this many tokens (the
- * reference's TC_MIN, src/moe.rs:35; 0 = never). Until it is set the library decides: from two
- * tokens, or one where that is faster. Integer layers (Q8x and 32-value activation blocks) give
+ * reference's TC_MIN, src/moe.rs:35; 0 = never). Until it is set the library decides: whole
+ * layers from two tokens, or one where that is faster; pm_experts and pm_experts_rows from 17
+ * pairs, pm_shared from 5 tokens; MXFP4 layers from one token. Integer layers (Q8x and 32-value activation blocks) give
  * the same bits on either path; MXFP4 layers stay within the layer tolerance. */
 PM_API int32_t pm_ctx_set_tensor_core_min_tokens(pm_ctx *ctx, int32_t min_tokens);
 /* the CUDA stream all work of this context is ordered on (cudaStream_t) */

@@ -973,21 +973,34 @@ struct Path {
   bool q32;        // int8 tensor-core products for 32-value activation blocks
   bool merge;      // the shared expert is one more group of the routed experts' launches
 };
-static Path pick_path(pm_layer *ly, int T) {
+// what a call does: the whole layer (pm_moe_forward, stacks: the plan's kernels make the tile list, the shared expert may
+// join the launches), the routed experts of a given plan, the shared expert alone
+enum PathCall { PATH_WHOLE, PATH_EXPERTS, PATH_SHARED };
+static Path pick_path(pm_layer *ly, int T, PathCall call) {
   const pm_ctx *c = ly->ctx;
   const pm_layer_desc &D = ly->dev.desc;
   Path p;
   // The integer products give the same bits on either path, so until the caller sets the threshold the faster one
-  // decides: two tokens up (one token, 8 experts x 2048 x 1024: 27 us on both; 8 tokens of a 7168-wide layer: 453 us
-  // on the row kernels, 323 us on the tensor cores), and one where the shared expert joins the launch.
-  const int int_min = c->tc_min_set ? c->tc_min_tokens : (shared_merges(D) ? 1 : 2);
-  p.tc = D.act_quant == PM_AQ_Q8X_256 && c->tc_min_tokens > 0 && T >= int_min;
+  // decides (us a call, row kernels : tensor cores):
+  //  whole layer: two tokens up (64 experts x 2048 x 1024, 1 / 2 / 3 / 4 / 8 tokens 29 : 36, 40 : 42, 52 : 54, 67 : 62, 109 : 73;
+  //    128 x 2048 x 768 31 : 35, 43 : 45, 58 : 50, 73 : 60, 135 : 95; 4-bit codebook layers of 32 x 2560 x 640 42 : 66, 63 : 68, 87 : 75,
+  //    111 : 77, 193 : 116), and one where the shared expert joins the launch (64 x 7168 x 2048 99 : 87);
+  //  experts of a given plan, which need the tile list in a launch of their own and may be one row an expert: more than
+  //    16 pairs (a row each, 8 / 16 / 24 rows: 64 x 2048 x 1024 28 : 37, 36 : 41, 48 : 50; 64 x 7168 x 2048 78 : 81, 130 : 127,
+  //    183 : 168; 32 x 2560 x 640 39 : 55, 63 : 66, 90 : 66; 8 an expert's token, 2 / 3 tokens 67 : 70, 79 : 80; 159 : 156, 213 : 196);
+  //  shared expert: more than 4 tokens (7168 x 2048, 1 / 4 / 5 / 8 tokens 19 : 47, 41 : 48, 49 : 48, 71 : 49; 2048 x 1024 16 : 27,
+  //    20 : 29, 22 : 30, 29 : 31, 12 tokens 39 : 31).
+  const bool int_tc = c->tc_min_set            ? T >= c->tc_min_tokens
+                      : call == PATH_WHOLE     ? T >= (shared_merges(D) ? 1 : 2)
+                      : call == PATH_EXPERTS   ? T * D.top_k > 16
+                                               : T > 4;
+  p.tc = D.act_quant == PM_AQ_Q8X_256 && c->tc_min_tokens > 0 && int_tc;
   p.tc_gu = p.tc && D.type_gate == D.type_up;
   // (MXFP4: from one token up until the caller says otherwise; a layer of 32 experts, d = ff = 2880, row kernels against
   // these: 1 token 60 : 55 us, 2 tokens 97 : 61, 4 tokens 162 : 79, 8 tokens 300 : 121)
   p.mx = mx_layer(D) && c->tc_min_tokens > 0 && T >= (c->tc_min_set ? c->tc_min_tokens : 1);
-  p.q32 = q32_layer(D) && c->tc_min_tokens > 0 && T >= int_min;
-  p.merge = p.tc_gu && shared_merges(D);
+  p.q32 = q32_layer(D) && c->tc_min_tokens > 0 && int_tc;
+  p.merge = call == PATH_WHOLE && p.tc_gu && shared_merges(D);
   return p;
 }
 static TcTiles path_tiles(pm_layer *ly, int T, const Path &p, const Scratch &S, bool merge) {
@@ -1008,7 +1021,7 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
   const LayerDev &dv = ly->dev;
   const pm_layer_desc &D = dv.desc;
   Launch L = c->launch();
-  const Path path = pick_path(ly, T);
+  const Path path = pick_path(ly, T, made ? PATH_WHOLE : PATH_EXPERTS);
   const bool tc = path.tc, tc_gu = path.tc_gu;
   Groups g = plan_groups(S.plan, D.n_exp);
   const int P = T * D.top_k;
@@ -1130,7 +1143,7 @@ static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
   if (!D.shared) return PM_OK;
   PROF(c, PH_SHARED);
   Launch L = c->launch();
-  const Path path = pick_path(ly, T);
+  const Path path = pick_path(ly, T, PATH_SHARED);
   const bool use_tc = path.tc, tc_gu = path.tc_gu;
   TcTiles tt{};
   if (use_tc) tt = tc_tiles_of(S.tiles, T, 1, 1, 0, 0);
@@ -1170,7 +1183,7 @@ static int32_t dev_forward(pm_layer *ly, const float *x, int T, float *y, bool a
   pm_ctx *c = ly->ctx;
   const LayerDev &dv = ly->dev;
   Launch L = c->launch();
-  const Path path = pick_path(ly, T);
+  const Path path = pick_path(ly, T, PATH_WHOLE);
   const TcTiles tt = path_tiles(ly, T, path, S, path.merge);
   if (route_plan_small_takes(dv, x, T)) {  // a few tokens: logits, top-k, plan and tiles in one launch
     PROF(c, PH_ROUTER);

@@ -110,3 +110,41 @@ def test_workspace_of_a_long_mxfp4_prompt():
         b.free()
     gl.close()
     c.close()
+
+
+@pytest.mark.parametrize("shape", ["c2", "c4", "c8"])
+def test_split_calls_choose_by_their_own_size(ctx, oracle, shape):
+    """Rows and plans served for somebody else, and the shared expert alone: up to 16 pairs (4 tokens of the one shared
+    expert) on the row kernels, more on the tensor cores; the same bits."""
+    cfg = SMALL[shape]
+    ol, gl, _ = make_pair(oracle, pb, ctx, cfg, 84)
+
+    def kinds(call):
+        c0 = ctx.path_counts()
+        got = call()
+        c1 = ctx.path_counts()
+        return got, c1["general"] - c0["general"], c1["tensor"] - c0["tensor"]
+
+    rng = np.random.default_rng(85)
+    for R in (1, 16, 17):
+        x = synth.make_activations(R, cfg.d, 980 + R)
+        eids, w = rng.integers(0, cfg.n_exp, R).astype(np.uint32), rng.uniform(0.5, 1.5, R).astype(np.float32)
+        got, row, tensor = kinds(lambda: gl.experts_rows(x, eids, w))
+        assert (row, tensor) == ((0, 2) if R > 16 else (2, 0))
+        for r in range(R):  # row r of a plan whose first pick is the row's expert
+            ids = np.array([[eids[r]] + [e for e in range(cfg.n_exp) if e != eids[r]][:cfg.top_k - 1]], np.uint32)
+            at = int(oracle.plan(ids, cfg.n_exp)["pair_pos"].ravel()[0])
+            assert bits_equal(got[r], ol.experts(x[r:r + 1], ids, np.full(ids.shape, w[r], np.float32))[at])
+    for T in (1, 2, 3, 9):
+        x = synth.make_activations(T, cfg.d, 990 + T)
+        ids, w = gl.route(x)
+        got, row, tensor = kinds(lambda: gl.experts(x, ids, w))
+        assert (row, tensor) == ((0, 2) if T * cfg.top_k > 16 else (2, 0))
+        assert bits_equal(got, ol.experts(x, ids, w))
+    if cfg.shared:
+        for T in (1, 4, 5):
+            x = synth.make_activations(T, cfg.d, 995 + T)
+            got = gl.shared(x)
+            ids, w = gl.route(x)
+            assert bits_equal(gl.combine(gl.experts(x, ids, w), ids, w, got), ol.forward(x))
+    gl.close()
