@@ -402,7 +402,8 @@ __global__ void __launch_bounds__(MxShape::NT, 1) k_tc_mx(const __grid_constant_
       n_acc++;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const bool dead = *(volatile int *)A.err != 0;
-      // a sum once more in f32: matrix `second`, row r, token n of the tile
+      // (The columns are read a second time where a sum was not finite: looked for eight columns at a time, the branch cost
+      // 2.5 % of a prompt.) A sum once more in f32: matrix `second`, row r, token n of the tile
       auto again = [&](bool second, int r, int n) {
         const uint32_t p = T.y + (uint32_t)n;
         return mx_sum_f32((second ? A.w1 + (size_t)el * A.w1_stride : A.w0 + (size_t)el * A.w0_stride) + (size_t)r * (A.cols / 2),
@@ -418,18 +419,27 @@ __global__ void __launch_bounds__(MxShape::NT, 1) k_tc_mx(const __grid_constant_
         };
         {
           const int hw = npad >> 1, c0 = par * hw;  // half of the columns: a multiple of 8
-          for (int c8 = 0; c8 < hw; c8 += 8) {
-            uint32_t v[8];
-            tc_ld8<0>(tlane + h * 128u + (uint32_t)(c0 + c8), v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            float o[8];
+          float poison = 0.0f;  // a NaN once a sum is not finite
+          auto columns = [&](bool repair) {
+            for (int c8 = 0; c8 < hw; c8 += 8) {
+              uint32_t v[8];
+              tc_ld8<0>(tlane + h * 128u + (uint32_t)(c0 + c8), v);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+              float o[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) o[u] = __uint_as_float(v[u]);
-            mx_repair(o, [&](int u) { return on && c0 + c8 + u < nvalid; }, [&](int u) { return again(false, drow, c0 + c8 + u); });
+              for (int u = 0; u < 8; u++) o[u] = __uint_as_float(v[u]);
+              if (repair)
+                mx_repair(o, [&](int u) { return on && c0 + c8 + u < nvalid; }, [&](int u) { return again(false, drow, c0 + c8 + u); });
 #pragma unroll
-            for (int u = 0; u < 8; u++) put(c0 + c8 + u, o[u]);
-            __syncwarp();
-          }
+              for (int u = 0; u < 8; u++) {
+                put(c0 + c8 + u, o[u]);
+                poison = __fmaf_rn(o[u], 0.0f, poison);
+              }
+              if (repair) __syncwarp();
+            }
+          };
+          columns(false);
+          if (__any_sync(PM_FULL, poison != 0.0f)) columns(true);
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0) tc_mbar_arrive(acc_free);
@@ -449,24 +459,32 @@ __global__ void __launch_bounds__(MxShape::NT, 1) k_tc_mx(const __grid_constant_
         };
         {  // gate sums in columns 0 .., up sums in 128 ..: a quarter of the tokens a thread
           const int qw = npad >> 2, c0 = part * qw;
-          for (int c4 = 0; c4 < qw; c4 += 4) {
-            uint32_t vg[4], vu[4];
-            tc_ld4<0>(tlane + (uint32_t)(c0 + c4), vg);
-            tc_ld4<128>(tlane + (uint32_t)(c0 + c4), vu);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            float o[8];  // gate, then up
+          float poison = 0.0f;
+          auto columns = [&](bool repair) {
+            for (int c4 = 0; c4 < qw; c4 += 4) {
+              uint32_t vg[4], vu[4];
+              tc_ld4<0>(tlane + (uint32_t)(c0 + c4), vg);
+              tc_ld4<128>(tlane + (uint32_t)(c0 + c4), vu);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+              float o[8];  // gate, then up
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-              o[u] = __uint_as_float(vg[u]);
-              o[4 + u] = __uint_as_float(vu[u]);
+              for (int u = 0; u < 4; u++) {
+                o[u] = __uint_as_float(vg[u]);
+                o[4 + u] = __uint_as_float(vu[u]);
+              }
+              if (repair)
+                mx_repair(o, [&](int u) { return on && c0 + c4 + (u & 3) < nvalid; },
+                          [&](int u) { return again(u >= 4, hrow, c0 + c4 + (u & 3)); });
+#pragma unroll
+              for (int u = 0; u < 4; u++) {
+                if (on && c0 + c4 + u < nvalid) put(c0 + c4 + u, o[u], o[4 + u]);
+                poison = __fmaf_rn(o[u], 0.0f, __fmaf_rn(o[4 + u], 0.0f, poison));
+              }
+              if (repair) __syncwarp();
             }
-            mx_repair(o, [&](int u) { return on && c0 + c4 + (u & 3) < nvalid; },
-                      [&](int u) { return again(u >= 4, hrow, c0 + c4 + (u & 3)); });
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-              if (on && c0 + c4 + u < nvalid) put(c0 + c4 + u, o[u], o[4 + u]);
-            __syncwarp();
-          }
+          };
+          columns(false);
+          if (__any_sync(PM_FULL, poison != 0.0f)) columns(true);
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0) tc_mbar_arrive(acc_free);
