@@ -996,8 +996,8 @@ static Path pick_path(pm_layer *ly, int T, PathCall call) {
                                                : T > 4;
   p.tc = D.act_quant == PM_AQ_Q8X_256 && c->tc_min_tokens > 0 && int_tc;
   p.tc_gu = p.tc && D.type_gate == D.type_up;
-  // (MXFP4: from one token up until the caller says otherwise; a layer of 32 experts, d = ff = 2880, row kernels against
-  // these: 1 token 60 : 55 us, 2 tokens 97 : 61, 4 tokens 162 : 79, 8 tokens 300 : 121)
+  // (MXFP4: from one token up until the caller says otherwise; a layer of 32 experts, d = ff = 2880, row kernels : these, 1 / 2 /
+  // 4 / 8 / 16 tokens 64 : 54 us, 102 : 78, 164 : 106, 289 : 141, 524 : 173)
   p.mx = mx_layer(D) && c->tc_min_tokens > 0 && T >= (c->tc_min_set ? c->tc_min_tokens : 1);
   p.q32 = q32_layer(D) && c->tc_min_tokens > 0 && int_tc;
   p.merge = call == PATH_WHOLE && p.tc_gu && shared_merges(D);
@@ -1087,7 +1087,10 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
   {
     PROF(c, PH_QUANT_X);
     if (tc_gu) {
-      // (many rows: quantise every token once and gather the quantised rows, see k_tc_quant_rows)
+      // Many rows: quantise every token once and gather the quantised rows, see k_tc_quant_rows. From 8 M values of all
+      // pairs on (a layer, this : quantised a pair: 128 experts x 2048 x 768, 512 / 1024 / 2048 tokens 247 : 250, 331 : 338, 525 : 540
+      // us; 64 x 2048 x 1024, 512 tokens 208 : 218; 32 x 7168 x 2048, 256 tokens 471 : 507); at 1 to 8 M the two are within
+      // 2 %, and a launch less is what a small call needs.
       const bool gather = prequant || (size_t)P * D.d > ((size_t)8 << 20);
       if (gather && !prequant) launch_quant_q8x(L, x, (size_t)T, D.d, S.xq, S.xd, S.xbsum, S.xbm, S.xs);
       if (gather) launch_tc_rows(L, Pr, tt, g.pair_token, D.d, S.xq, S.xd, S.xbm, S.xs, S.rec);

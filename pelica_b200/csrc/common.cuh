@@ -253,9 +253,9 @@ __device__ __forceinline__ void pm_pdl() {
   pm_pdl_trigger();
 }
 // A small grid runs its body once for practice - on made-up values, storing nothing - while it waits for the kernel before:
-// an instruction that is executed once and cold costs some 30 cycles.
+// an instruction that is executed once and cold costs some 30 cycles. Small: two CTAs an SM (148) at most, all of them resident.
 #define PM_PRACTICE_CTAS 296
-// ... at once: for kernels in front of one that fetches its weights while it waits (k_route_plan_small)
+// ... at once: for a kernel in front of one that practises while it waits (k_router_tile, k_route_seg)
 __device__ __forceinline__ void pm_pdl_early() {
   pm_pdl_trigger();
   pm_pdl_wait();

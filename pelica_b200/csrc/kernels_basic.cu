@@ -400,11 +400,15 @@ __global__ void __launch_bounds__(256) k_router(const float *__restrict__ wr,
 // 210 us; 64 tokens 75 us; 512 tokens on 128 experts x 2048 29 us)
 #define RT_CH 128
 #define RT_ST 3
+#define PL_SEG 32 /* tokens of a segment of the routing = warps of its CTA (k_route_seg) */
 template <int EW, int TW> __global__ void __launch_bounds__(256, 1) k_router_tile(const float *__restrict__ wr,
                                                                                  const float *__restrict__ bias,
                                                                                  const float *__restrict__ x, int T, int E,
                                                                                  int d, float *logits) {
-  if (T <= 32) pm_pdl_early();  // (the one CTA of the routing kernel behind practises meanwhile)
+  // One segment: the one CTA of the routing kernel behind practises meanwhile (384 experts x 2048, 12 / 16 / 32 tokens 124 /
+  // 142 / 212 us a layer, let in late 129 / 145 / 214; 64 to 256 experts the same either way). More segments: the same either
+  // way, or the CTAs behind take the SMs.
+  if (T <= PL_SEG) pm_pdl_early();
   else pm_pdl();
   constexpr int RE = 2 * EW, RT = 4 * TW, ROWS = RE + RT;  // rows of a stage: experts, then tokens
   extern __shared__ __align__(16) float rs[];              // [RT_ST][ROWS][RT_CH]
@@ -687,7 +691,6 @@ cudaError_t launch_plan(const Launch &L, const LayerDev &ly, const uint32_t *ids
 // k_plan_* takes four and has every expert's CTA walk all pairs (4096 tokens x 8 on 256 experts: 72 us).
 // One segment: its CTA does all three (the plan of 8 to 32 tokens).
 // ---------------------------------------------------------------------------
-#define PL_SEG 32 /* tokens of a segment = warps of its CTA */
 // a plan whose arrays are all the same `words` of shared memory (at least max(E + 1, 512, 4 * tiles + 4) of them)
 __device__ __forceinline__ void pm_plan_nowhere(uint32_t *words, PlanDev &pl, TcTiles &tt) {
   pl.n_active = (int *)words;

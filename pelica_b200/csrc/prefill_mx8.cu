@@ -5,8 +5,10 @@
 //
 // The activations are exact sums of E4M3 pieces with block scales of their own: x = x1 + x2 + ..., xi the
 // nearest E4M3 of what is left of x, in units of 2^(E - 7 - 5 (i - 1)), E the exponent of the block's largest value.
-// What a piece leaves is at most a 32nd of what it was given: 5 pieces hold all 24 bits of an f32 (calls of fewer than
-// PM_MX_PROMPT tokens), 4 leave 2^-19 (prompts; the two bf16 pieces of prefill_mx.cu leave 2^-17). The pieces of a
+// What a piece leaves is at most a 32nd of what it was given: 5 pieces hold all 24 bits of the values within 13 octaves of the
+// block's largest and leave 2^-37 of that of the smaller ones (calls of fewer than PM_MX_PROMPT tokens), 4 leave 2^-19 of
+// it (prompts; the two bf16 pieces of prefill_mx.cu leave 2^-17 of a value). No unit is below 2^-126: in blocks whose largest is
+// below 2^-99 the last pieces hold less, down to 2^-136. The pieces of a
 // tile's tokens are columns of ONE product: N = pieces x tokens, a sum each, added up smallest first. With 5 pieces
 // the sums are folded into f32 registers every 256 K values (the tensor cores' own sums lose the low bits
 // of a long chain: 1e-5 of the RMS over 2,880 values against 1e-7).
@@ -15,8 +17,8 @@
 // 16 tokens (5 pieces) or 32 (4). Rows of gate and up alternate in tensor memory, so the two sums of an output are
 // neighbouring lanes. Bound by the
 // latency of a stage's steps (wait, copy, fence, products, fold: 900 cycles for 128 K values, two CTAs interleave): 31 tokens on
-// 32 experts, d = ff = 2880, 2.8 TB/s of weights; gate/up + down 223 us decoding to bf16, 149 here; 1 token 58 us on the row
-// kernels, 37 here.
+// 32 experts, d = ff = 2880, 2.8 TB/s of weights; gate/up + down 223 us decoding to bf16, 149 here; 1 token, timed launch by
+// launch, 57 us on the row kernels, 43 here.
 #include <cuda_fp16.h>
 
 #include "mxsum.cuh"
@@ -497,9 +499,11 @@ template <bool DOWN, int NP> static cudaError_t mx8_start(const Launch &L, const
   return pm_launch(L, k_tc_mx8<DOWN, NP>, dim3((unsigned)(items < ctas ? items : ctas)), M8_NT, smem, A);
 }
 
-// Tokens of a tile of a call of T tokens whose groups hold n_pairs / n_groups pairs on average; 128: prefill_mx.cu
-// (32 experts, d = ff = 2880, gate/up + down: 19 pairs a group 169 us here, 240 there; 37 pairs, two tiles a group here,
-// 275 : 251).
+// Tokens of a tile of a call of T tokens whose groups hold n_pairs / n_groups pairs on average; 128: prefill_mx.cu. A
+// layer, us here : there at 8 / 20 / 28 / 32 / 36 / 48 pairs a group (above 32 two tiles a group here):
+//   32 experts x 2880 x 2880  182 : 257   212 : 271   244 : 280   259 : 284   297 : 287   336 : 302
+//   64 experts x 2048 x 1024  127 : 167   149 : 179   161 : 188   178 : 191   197 : 195   223 : 207
+//   16 experts x 4096 x 4096  211 : 267   241 : 281   287 : 292   310 : 293   328 : 299   377 : 312
 int mx_tile_tokens(int T, int n_pairs, int n_groups) {
   if (T < PM_MX_PROMPT) return M8Shape<5>::NTOK;
   return n_pairs / (n_groups < n_pairs ? n_groups : n_pairs) <= 28 ? M8Shape<4>::NTOK : 128;
@@ -510,7 +514,8 @@ int mx_tile_tokens(int T, int n_pairs, int n_groups) {
 static int mx8_split_stages(int nst, int splits) { return ((nst + splits - 1) / splits + 1) & ~1; }  // whole boxes
 int mx_splits(const pm_layer_desc &D, int n_pairs) {
   const int nst = (D.ff + M8_KS - 1) / M8_KS;
-  // (a pair is at most a tile of its own; two CTAs on each of 148 SMs)
+  // (a pair is at most a tile of its own; two CTAs on each of a B200's 148 SMs, also where the device offers fewer: the
+  // number of parts is part of how a sum rounds)
   const long items = (long)((D.d + M8_M - 1) / M8_M) * n_pairs;
   long s = 296 / (items > 0 ? items : 1);
   s = s > 4 ? 4 : s;

@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(512) k_tc_tiles(Groups g, int first_local, int
 // x (null: row first + i itself), first = the tile's first pair; rows past the tile's count are zeros. A token
 // is read and quantised once per expert that serves it: a launch less for small calls, but four times the
 // bytes of a gather of quantised rows (4096 tokens x 8 experts x 7168 values: 280 us against 48 + 60), so large
-// calls quantise first (k_quant_q8x) and gather (k_tc_rows).
+// calls quantise first (k_quant_q8x) and gather (k_tc_rows; the line and its figures: dev_experts).
 __global__ void __launch_bounds__(256) k_tc_quant_rows(const int *__restrict__ n_tiles, const uint4 *__restrict__ tiles,
                                                        const uint32_t *__restrict__ src_row, int cols,
                                                        const float *__restrict__ x, uint8_t *__restrict__ rec) {
@@ -873,8 +873,12 @@ size_t tc_rec_bytes(int n_pairs, int max_groups, int cols) {
 }
 TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, int ntok) {
   TcTiles t;
-  // tiles of up to 64 tokens and the two-CTA shape while the groups hold up to 16 pairs on average (128 experts x 2048 x
-  // 768, 32 pairs a group: 102 us in the one-CTA shape, 118 us in this one; 2 pairs: 1,049 -> 733 us of a 7168-wide layer)
+  // tiles of up to 64 tokens and the two-CTA shape while the groups hold up to 16 pairs on average. A layer, this shape :
+  // the one-CTA shape, us at 2 / 8 / 16 / 20 / 24 / 32 / 64 pairs a group:
+  //   128 experts x 2048 x 768   152 : 190   164 : 213   207 : 222   221 : 232   238 : 241   273 : 250   388 : 330
+  //    64 experts x 2048 x 1024  102 : 125   115 : 136   141 : 146   148 : 148   160 : 153   182 : 155   257 : 215
+  //    32 experts x 7168 x 2048  234 : 301   252 : 322   313 : 335   332 : 343   333 : 349   407 : 363   611 : 487
+  // (the line is below every crossing, 20 to 30 pairs: an average says little of the largest group)
   const int avg = n_pairs / (n_groups < n_pairs ? n_groups : n_pairs);
   t.ntok = ntok ? ntok : (avg <= 16 ? TcShape<2>::NTOK : TC_NMAX);
   t.even = ntok != 0;

@@ -1,7 +1,9 @@
 // route.cuh - one token's top-k experts and routing weights by one warp
 // (src/moe_kernels.rs:1019-1081, src/oss_kernels.rs:15-35, src/ds4.rs:1371-1426,
-// src/q4x.rs:2213-2231). Shared by the general kernel and the decode kernel so
-// both give the same bits.
+// src/q4x.rs:2213-2231). Two spellings of one definition, the same operations in the same
+// order: pm_route_scores keeps a token's experts in registers (the decode kernel, which ranks
+// them itself), pm_route_warp in shared memory with every loop rolled (all other kernels). The
+// group selection and the weights are one function for both.
 #pragma once
 
 #include "common.cuh"
@@ -77,7 +79,7 @@ __device__ __forceinline__ void pm_group_rank(const float *gsc, int G, int topk_
   }
 }
 
-// Scores of one token by one warp. lane L holds experts L, L+32, ... (NP per lane,
+// Scores of one token by one warp (decode kernel). Lane L holds experts L, L+32, ... (NP per lane,
 // NP*32 >= E); `lg` points at the token's E logits (any address space); ssv[E],
 // gsc[E/2], keep[E/2] are per-warp scratch in shared memory (group-limited
 // selection only). Out: pr[] = the score the weight is taken from, key[] = the
