@@ -1008,7 +1008,7 @@ static TcTiles path_tiles(pm_layer *ly, int T, const Path &p, const Scratch &S, 
   TcTiles t{};
   const int groups = std::min(D.n_exp, ly->dev.n_local);
   if (p.tc || p.mx || p.q32)
-    t = tc_tiles_of(S.tiles, T * D.top_k, D.n_exp, groups, merge ? T : 0,
+    t = tc_tiles_of(S.tiles, T * D.top_k, D.n_exp, groups, T, merge ? T : 0,
                     p.mx ? mx_tile_tokens(T, T * D.top_k, groups) : (p.q32 ? q32_tile_tokens() : 0));
   return t;
 }
@@ -1093,8 +1093,8 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
       // 2 %, and a launch less is what a small call needs.
       const bool gather = prequant || (size_t)P * D.d > ((size_t)8 << 20);
       if (gather && !prequant) launch_quant_q8x(L, x, (size_t)T, D.d, S.xq, S.xd, S.xbsum, S.xbm, S.xs);
-      if (gather) launch_tc_rows(L, Pr, tt, g.pair_token, D.d, S.xq, S.xd, S.xbm, S.xs, S.rec);
-      else launch_tc_quant_rows(L, Pr, tt, g.pair_token, D.d, x, S.rec);
+      if (gather) launch_tc_rows(L, D.type_gate, Pr, tt, g.pair_token, D.d, S.xq, S.xd, S.xbm, S.xs, S.rec);
+      else launch_tc_quant_rows(L, D.type_gate, Pr, tt, g.pair_token, D.d, x, S.rec);
     } else if (q8 && !prequant) {
       launch_quant_q8x(L, x, (size_t)T, D.d, S.xq, S.xd, S.xbsum);
     } else if (q32 && !prequant) {
@@ -1113,7 +1113,7 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
   }
   {
     PROF(c, PH_QUANT_H);
-    if (tc) launch_tc_quant_rows(L, Pr, tt, nullptr, D.ff, S.h, S.rec);
+    if (tc) launch_tc_quant_rows(L, D.type_down, Pr, tt, nullptr, D.ff, S.h, S.rec);
     else if (q8) launch_quant_q8x(L, S.h, (size_t)P, D.ff, S.hq, S.hd, S.hbsum);
     else if (q32) launch_quant_q8_32(L, S.h, (size_t)P, D.ff, S.hq, S.hd, f16s);
   }
@@ -1149,7 +1149,7 @@ static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
   const Path path = pick_path(ly, T, PATH_SHARED);
   const bool use_tc = path.tc, tc_gu = path.tc_gu;
   TcTiles tt{};
-  if (use_tc) tt = tc_tiles_of(S.tiles, T, 1, 1, 0, 0);
+  if (use_tc) tt = tc_tiles_of(S.tiles, T, 1, 1, T, 0, 0);
   CU(launch_shared_groups(L, S.one, S.zero_u, S.tcount, S.iota, T, tt));
   Groups g;
   g.n_groups = S.one;
@@ -1162,7 +1162,7 @@ static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
   const bool q8 = D.act_quant == PM_AQ_Q8X_256, f16s = D.act_quant == PM_AQ_Q8_32_F16;
   const bool q32 = D.act_quant == PM_AQ_Q8_32 || f16s;
   if (tc_gu) {
-    launch_tc_quant_rows(L, T, tt, nullptr, D.d, x, S.rec);
+    launch_tc_quant_rows(L, D.type_gate, T, tt, nullptr, D.d, x, S.rec);
     CU(launch_tc(L, dv, true, false, nullptr, tt, S.rec, nullptr, S.sh, c->dev_err, c->wait_ns, c->tc_fault_block));
   } else {
     if (q8) launch_quant_q8x(L, x, (size_t)T, D.d, S.xq, S.xd, S.xbsum);
@@ -1170,7 +1170,7 @@ static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
     launch_gateup(L, dv, true, g, T, x, S.xq, S.xd, S.xbsum, nullptr, S.sh);
   }
   if (use_tc) {
-    launch_tc_quant_rows(L, T, tt, nullptr, D.shared_ff, S.sh, S.rec);
+    launch_tc_quant_rows(L, D.type_down, T, tt, nullptr, D.shared_ff, S.sh, S.rec);
     CU(launch_tc(L, dv, true, true, nullptr, tt, S.rec, nullptr, S.shared_out, c->dev_err, c->wait_ns, c->tc_fault_block));
   } else {
     if (q8) launch_quant_q8x(L, S.sh, (size_t)T, D.shared_ff, S.shq, S.shd, S.shbsum);

@@ -747,7 +747,7 @@ __device__ __forceinline__ uint32_t pm_plan_scan(PlanDev pl, int e, uint32_t c, 
   }
   if (e == 0) *pl.n_active = (int)active + (tt.shared ? 1 : 0);
   if (tt.tiles) {
-    const uint32_t nt = (c + tt.ntok - 1) / tt.ntok, rp = (c + 15u) & ~15u;
+    const uint32_t nt = (c + tt.ntok - 1) / tt.ntok, rp = tc_group_rows(tt.ntok, c, nt);
     uint32_t ft, r0, at, ar;
     pm_scan2_512(nt, rp, ft, r0, at, ar, sh);
     if (c > 0) {
@@ -755,13 +755,14 @@ __device__ __forceinline__ uint32_t pm_plan_scan(PlanDev pl, int e, uint32_t c, 
       const uint32_t each = tc_tile_tokens(c, nt, tt.ntok, tt.even);
       for (uint32_t i = 0; i < nt && (int)(ft + i) < tt.max_tiles; i++)
         tt.tiles[ft + i] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, o + i * each,
-                                      min(c - i * each, each), r0 + i * each);
+                                      min(c - i * each, each), r0 + i * tc_tile_rows(tt.ntok, each));
     }
     uint32_t st = 0;
     if (tt.shared) {  // the shared expert as one more group: every token, pairs total .. total + T - 1
       st = (T + tt.ntok - 1) / tt.ntok;
       for (uint32_t i = e; i < st && (int)(at + i) < tt.max_tiles; i += 512)
-        tt.tiles[at + i] = make_uint4(TC_SHARED, total + i * tt.ntok, min((uint32_t)T - i * tt.ntok, (uint32_t)tt.ntok), ar + i * tt.ntok);
+        tt.tiles[at + i] = make_uint4(TC_SHARED, total + i * tt.ntok, min((uint32_t)T - i * tt.ntok, (uint32_t)tt.ntok),
+                                      ar + i * tc_tile_rows(tt.ntok, tt.ntok));
       for (int i = e; i < T; i += 512) pl.pair_token[total + i] = (uint32_t)i;
     }
     if (e == 0) {
@@ -1181,7 +1182,7 @@ __global__ void k_shared_groups(uint32_t *one, uint32_t *zero, uint32_t *count, 
       tt.next[0] = tt.next[1] = 0;
     }
   }
-  if (tt.tiles && i * tt.ntok < T) tt.tiles[i] = make_uint4(TC_SHARED, i * tt.ntok, min(T - i * tt.ntok, (uint32_t)tt.ntok), i * tt.ntok);
+  if (tt.tiles && i * tt.ntok < T) tt.tiles[i] = make_uint4(TC_SHARED, i * tt.ntok, min(T - i * tt.ntok, (uint32_t)tt.ntok), i * tc_tile_rows(tt.ntok, tt.ntok));
 }
 cudaError_t launch_shared_groups(const Launch &L, int *one, uint32_t *zero, uint32_t *count, uint32_t *token, int T, const TcTiles &tt) {
   return PLAUNCH(L, k_shared_groups, (T + 255) / 256, 256, 0, (uint32_t *)one, zero, count, token, (uint32_t)T, tt);

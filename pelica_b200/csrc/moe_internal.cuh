@@ -176,7 +176,7 @@ struct TcTiles {
   int *n;              // [1] tiles
   unsigned int *next;  // [2] item counters of the gate/up and the down launch (each list serves one of each)
   uint4 *tiles;        // (expert slot or ~0, first pair, pairs, first record row)
-  int ntok;            // tokens of a full tile (128, or 64 where the groups are small)
+  int ntok;            // tokens of a full tile (128; 64 where the groups are small, TC_FEW_TOKENS where they are a few pairs)
   int even;            // a group's tiles have the same number of tokens (of 16) instead of ntok and a remainder
   int shared;          // the list holds the shared expert as one more group (pairs P .. P + T - 1)
   int max_tiles;
@@ -188,6 +188,13 @@ __host__ __device__ inline uint32_t tc_tile_tokens(uint32_t cnt, uint32_t n, int
 }
 bool route_plan_small_takes(const LayerDev &ly, const float *x, int T);
 cudaError_t launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits, uint32_t *ids,
+#define TC_FEW_TOKENS 8  // tokens of a tile of prefill_few.cu
+// record rows from one tile of a group to the next, and of a group of cnt pairs in n tiles (every group starts on a multiple
+// of 16; a tile of few tokens has 16 rows of its own)
+__host__ __device__ inline uint32_t tc_tile_rows(int ntok, uint32_t tokens) { return ntok == TC_FEW_TOKENS ? 16u : tokens; }
+__host__ __device__ inline uint32_t tc_group_rows(int ntok, uint32_t cnt, uint32_t n) {
+  return ntok == TC_FEW_TOKENS ? 16u * n : (cnt + 15u) & ~15u;
+}
                                     float *w, PlanDev pl, const int32_t *slot_table, unsigned int *ticket, const TcTiles &tt, int *err,
                                     unsigned long long wait_ns);
 // top-k, weights and plan of any number of tokens from their logits (seg: route_seg_words words of scratch)
@@ -209,14 +216,15 @@ void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int
 // src_row: row of the activations that holds pair p (null: row p itself)
 size_t tc_tile_words(int n_pairs, int max_groups);
 // n_groups: groups that can have pairs (the experts this GPU holds)
-// shared_tokens: tokens of the shared expert's group in the same list (0: none)
+// tokens: of the call, the most a group can have; shared_tokens: of the shared expert's group in the same list (0: none)
 // ntok: tokens of a full tile, 0 for launch_tc's own rule (anything else: even tiles)
-TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, int ntok);  // buf: tc_tile_words words, 16-byte aligned
+TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int tokens, int shared_tokens, int ntok);  // buf: tc_tile_words words, 16-byte aligned
 size_t tc_rec_bytes(int n_pairs, int max_groups, int cols);
 cudaError_t launch_tc_tiles(const Launch &L, const LayerDev &ly, Groups g, const TcTiles &t);
-void launch_tc_quant_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x,
+// weight_type: of the matrix that the rows meet (it decides the records of tiles of few tokens)
+void launch_tc_quant_rows(const Launch &L, int weight_type, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x,
                           uint8_t *rec);
-void launch_tc_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const int8_t *xq,
+void launch_tc_rows(const Launch &L, int weight_type, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const int8_t *xq,
                     const float *xd, const uint16_t *xbm, const int32_t *xs, uint8_t *rec);
 cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared_only, bool down, const uint32_t *pair_src, const TcTiles &t,
                       const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns, int fault_block);

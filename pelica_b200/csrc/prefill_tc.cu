@@ -28,22 +28,8 @@
 // output, as f32x2 pairs, behind an integer add and a conversion).
 #include <cuda_fp16.h>
 
-#include "tcgen.cuh"
+#include "prefill_tc.cuh"
 
-// The tokens' operand is read from records laid out for the products (k_tc_quant_rows writes them):
-// record (8 rows, block b) = [16 K chunks][8 rows][16 B] int8 activations, [2 K chunks][8 rows][8 f16]
-// sub-block sums for the Q4_K mins product, [8] f32 x.d, [8] i32 offset term of Q6_K, padded to a
-// multiple of 128 bytes so that every 8 x 16 B core matrix sits in one 128-byte line of shared memory.
-// The records of a token tile lie block by block, so that a tile's operand of a block is ONE copy
-// (a copy costs its issuing warp about 70 cycles whatever its size).
-#define TC_REC 2432
-#define TC_REC_BM 2048
-#define TC_REC_XD 2304
-#define TC_REC_XS 2336
-#define TC_M 128
-#define TC_NMAX 128               /* tokens of the largest tile */
-#define TC_RAW_Q4 (TC_M * 144)                       /* bytes of a block's weights: as stored */
-#define TC_RAW_Q6 (TC_M * (128 + 64))                /* ql, qh (the scales and d come straight to the registers) */
 // The two shapes of the kernel. PARTS: worker threads a row.
 //  4 (tiles of up to 128 tokens): one CTA an SM of 16 worker warps, passes of 64 tokens.
 //  2 (tiles of up to 64 tokens): two CTAs an SM of 8 worker warps and half of the tensor memory each, passes of
@@ -85,31 +71,6 @@ extern "C" __attribute__((visibility("default"))) int pm_debug_tc_trace(unsigned
 #endif
 #define TC_STAMP_W(b, i) TC_STAMP(0, b, i) TC_STAMP(1, b, i)
 
-struct TcArgs {
-  CUtensorMap m0[2], m1[2];    // planes of the tile's matrices as [expert][row][bytes]: gate or down, up
-  CUtensorMap ms0[2], ms1[2];  // ... of the shared expert
-  const uint4 *tiles;        // see k_tc_tiles
-  const int *n_tiles;        // [1]
-  unsigned int *next;        // [1] zero at launch: work items handed out so far (beyond two a CTA)
-  const uint8_t *rec;        // the tokens' operand as records (TC_REC)
-  const uint8_t *s0, *s1, *d0, *d1;  // Q6_K: the planes of the 16 sub-scales and of the f16 scales
-  const uint8_t *ss0, *ss1, *ds0, *ds1;  // ... of the shared expert
-  size_t s0_stride, s1_stride, d0_stride, d1_stride;
-  const float *bias0, *bias1;  // expert biases or null
-  const float *wts;            // routing weights by pair source (gate/up with fold) or null
-  const uint32_t *pair_src;
-  float *out;                  // gate/up: h [P][ff]; down: eo [P][d]
-  int *err;
-  unsigned long long wait_ns;  // limit of every wait on an mbarrier
-  uint32_t zero;  // 0 (see tc_mbar_arrive_used)
-  uint64_t neg_zero2;          // (-0, -0): see tc_fma2
-  int fault_block;             // test hook: no products are issued or signalled from this block on (-1 = off)
-  int row_tiles;               // tiles of rows of the matrix (128 rows, or 64 gate + 64 up)
-  int cols, rows;
-  int act;
-  float act_limit, act_alpha;
-};
-
 // The token tiles of a grouping: group a contributes ceil(count / ntok) tiles. tiles[i] = (expert slot, or
 // ~0 for an expert another rank holds; first pair; pairs; first record row). The records' rows keep a group's
 // pairs together and start every group on a multiple of 16 rows. One CTA; groups <= 512.
@@ -120,7 +81,7 @@ __global__ void __launch_bounds__(512) k_tc_tiles(Groups g, int first_local, int
   const int a = threadIdx.x, lane = a & 31, warp = a >> 5;
   const int ng = min(*g.n_groups, 512);
   const uint32_t cnt = a < ng ? g.count[a] : 0;
-  const uint32_t tc = (cnt + ntok - 1) / ntok, rp = (cnt + 15u) & ~15u;
+  const uint32_t tc = (cnt + ntok - 1) / ntok, rp = tc_group_rows(ntok, cnt, tc);
   uint32_t t = tc, r = rp;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -142,7 +103,7 @@ __global__ void __launch_bounds__(512) k_tc_tiles(Groups g, int first_local, int
     const uint32_t off = g.offset[a];
     const uint32_t nt = tc_tile_tokens(cnt, tc, ntok, even);
     for (uint32_t i = 0; i < tc && (int)(first + i) < max_tiles; i++)
-      tiles[first + i] = make_uint4((uint32_t)el, off + i * nt, min(cnt - i * nt, nt), r0 + i * nt);
+      tiles[first + i] = make_uint4((uint32_t)el, off + i * nt, min(cnt - i * nt, nt), r0 + i * tc_tile_rows(ntok, nt));
   }
   if (a == 0) {  // [0] tiles, [1], [2] the item counters of the two products
     head[0] = min((int)all, max_tiles);
@@ -157,6 +118,9 @@ __global__ void __launch_bounds__(512) k_tc_tiles(Groups g, int first_local, int
 // is read and quantised once per expert that serves it: a launch less for small calls, but four times the
 // bytes of a gather of quantised rows (4096 tokens x 8 experts x 7168 values: 280 us against 48 + 60), so large
 // calls quantise first (k_quant_q8x) and gather (k_tc_rows; the line and its figures: dev_experts).
+// FEW: tiles of prefill_few.cu. 1: one record a block (its 8 rows serve all 16 columns); 2 (Q6_K): the rows twice, record g with
+// the sub-blocks of 16 whose number has the other parity than g as zeros. 0: two records every 16 rows.
+template <int FEW>
 __global__ void __launch_bounds__(256) k_tc_quant_rows(const int *__restrict__ n_tiles, const uint4 *__restrict__ tiles,
                                                        const uint32_t *__restrict__ src_row, int cols,
                                                        const float *__restrict__ x, uint8_t *__restrict__ rec) {
@@ -173,7 +137,7 @@ __global__ void __launch_bounds__(256) k_tc_quant_rows(const int *__restrict__ n
     const uint32_t off = T.y, cnt = T.z;
     const int lane = threadIdx.x & 31;
     uint8_t *S = s_rec[threadIdx.x >> 5];
-    const int nrg = (int)((cnt + 15u) / 16u) * 2, units = practice ? 8 : nrg * nb;  // (row group, block) pairs of this tile
+    const int nrg = FEW ? FEW : (int)((cnt + 15u) / 16u) * 2, units = practice ? 8 : nrg * nb;  // (row group, block) pairs of this tile
     uint8_t *rec0 = rec + (size_t)(T.w >> 3) * nb * TC_REC;
     for (int u = practice ? (int)(threadIdx.x >> 5) : (int)(blockIdx.x * 8 + (threadIdx.x >> 5)); u < units; u += gridDim.x * 8) {
       const int b = u / max(nrg, 1), rgl = u - b * nrg;  // (the tile's records lie block by block)
@@ -184,7 +148,7 @@ __global__ void __launch_bounds__(256) k_tc_quant_rows(const int *__restrict__ n
         float v[4][8];
 #pragma unroll
         for (int r = 0; r < 4; r++) {
-          const uint32_t i = (uint32_t)(rgl * 8 + 4 * h + r);
+          const uint32_t i = (uint32_t)((FEW ? 0 : rgl * 8) + 4 * h + r);
           if (i < cnt) {
             const size_t row = src_row ? src_row[off + i] : off + i;
             const float4 *src = (const float4 *)(x + row * cols + (size_t)b * 256 + 8 * lane);
@@ -231,7 +195,8 @@ __global__ void __launch_bounds__(256) k_tc_quant_rows(const int *__restrict__ n
       for (int i = 0; i < 4; i++) {
         const uint32_t s0 = odd ? q[i][0] : q[4 + i][0], s1 = odd ? q[i][1] : q[4 + i][1];
         const uint32_t t0 = __shfl_xor_sync(PM_FULL, s0, 1), t1 = __shfl_xor_sync(PM_FULL, s1, 1);
-        const uint4 o = odd ? make_uint4(t0, t1, q[4 + i][0], q[4 + i][1]) : make_uint4(q[i][0], q[i][1], t0, t1);
+        uint4 o = odd ? make_uint4(t0, t1, q[4 + i][0], q[4 + i][1]) : make_uint4(q[i][0], q[i][1], t0, t1);
+        if (FEW == 2 && ((lane >> 1) & 1) != rgl) o = make_uint4(0, 0, 0, 0);
         *(uint4 *)(S + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) = o;
       }
       __syncwarp();
@@ -251,6 +216,7 @@ __global__ void __launch_bounds__(256) k_tc_quant_rows(const int *__restrict__ n
 
 // The same records from rows that are quantised already (rows another rank sent): one warp per
 // (8 rows, block), xbm / xs as k_q8x_aux makes them.
+template <int FEW>
 __global__ void __launch_bounds__(256) k_tc_rows(const int *__restrict__ n_tiles, const uint4 *__restrict__ tiles,
                                                  const uint32_t *__restrict__ src_row, int cols,
                                                  const int8_t *__restrict__ xq, const float *__restrict__ xd,
@@ -262,26 +228,27 @@ __global__ void __launch_bounds__(256) k_tc_rows(const int *__restrict__ n_tiles
   const int nb = cols / 256;
   const uint32_t off = T.y, cnt = T.z;
   const int lane = threadIdx.x & 31;
-  const int nrg = (int)((cnt + 15u) / 16u) * 2, units = nrg * nb;
+  const int nrg = FEW ? FEW : (int)((cnt + 15u) / 16u) * 2, units = nrg * nb;
   uint8_t *rec0 = rec + (size_t)(T.w >> 3) * nb * TC_REC;
   for (int u = blockIdx.x * 8 + (threadIdx.x >> 5); u < units; u += gridDim.x * 8) {
     const int b = u / nrg, rgl = u - b * nrg;
     uint8_t *R = rec0 + (size_t)u * TC_REC;
     {  // int8 values: lane = (row of the group, quarter of the block's 16 chunks)
       const int r8 = lane >> 2, q = lane & 3;
-      const uint32_t i = (uint32_t)rgl * 8 + r8;
+      const uint32_t i = (uint32_t)(FEW ? 0 : rgl * 8) + r8;
       uint4 v[4] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
       if (i < cnt) {
         const size_t row = src_row ? src_row[off + i] : off + i;
         const uint4 *src = (const uint4 *)(xq + row * cols + (size_t)b * 256 + 64 * q);
 #pragma unroll
-        for (int c = 0; c < 4; c++) v[c] = __ldg(src + c);
+        for (int c = 0; c < 4; c++)
+          if (FEW != 2 || (c & 1) == rgl) v[c] = __ldg(src + c);
       }
 #pragma unroll
       for (int c = 0; c < 4; c++) *(uint4 *)(R + ((4 * q + c) * 8 + r8) * 16) = v[c];
     }
     const int r8 = lane < 16 ? lane >> 1 : (lane & 7);
-    const uint32_t i = (uint32_t)rgl * 8 + r8;
+    const uint32_t i = (uint32_t)(FEW ? 0 : rgl * 8) + r8;
     const size_t row = i < cnt ? (src_row ? (size_t)src_row[off + i] : (size_t)(off + i)) : 0;
     if (lane < 16) {  // the f16 form of the sub-block sums: lane = (row, K chunk of the mins product)
       const int k = lane & 1;
@@ -313,14 +280,6 @@ __global__ void __launch_bounds__(256) k_tc_rows(const int *__restrict__ n_tiles
 // a_ready[q]: quarter q of operand A of a block is in tensor memory (its four worker warps); a_free[q]: the last
 // products that read quarter q of operand A are complete; acc_full[s] / acc_free[s]: a pass's products
 // into set s are complete / have been read by every worker warp.
-struct TcItem {
-  uint4 t;   // the tile (k_tc_tiles); t.x = ~1: no more items
-  int r0;    // first row of the item's matrix rows
-  int pad[3];
-};
-#define TC_IT 4
-#define TC_END 0xfffffffeu
-
 template <int WT, bool DOWN, int PARTS>
 __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc(const __grid_constant__ TcArgs A) {
   constexpr bool Q6 = WT == PM_TYPE_Q6_K;
@@ -859,7 +818,8 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)S::COLS) : "memory");
 }
 
-static int tc_max_tiles(int n_pairs, int max_groups, int ntok = 16) {  // (the default: of every shape)
+#define TC_FEW_AVG 6
+static int tc_max_tiles(int n_pairs, int max_groups, int ntok = TC_FEW_TOKENS) {  // (the default: of every shape)
   int groups = max_groups < n_pairs ? max_groups : n_pairs;
   return n_pairs / ntok + groups;
 }
@@ -868,19 +828,28 @@ size_t tc_tile_words(int n_pairs, int max_groups) { return 4 + 4 * (size_t)(tc_m
 // starts on a multiple of 16 rows)
 size_t tc_rec_bytes(int n_pairs, int max_groups, int cols) {
   size_t groups = (size_t)(max_groups < n_pairs ? max_groups : n_pairs);
-  size_t rows = (size_t)n_pairs + 15 * groups + 16;
+  size_t few = (size_t)n_pairs < TC_FEW_AVG * groups + TC_FEW_TOKENS * groups ? (size_t)n_pairs : 0;  // (tiles of few tokens: 16 rows each)
+  size_t rows = (size_t)n_pairs + few + 16 * groups + 16;
   return (rows / 8 + 1) * (size_t)(cols / 256) * TC_REC;
 }
-TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int shared_tokens, int ntok) {
+TcTiles tc_tiles_of(uint32_t *buf, int n_pairs, int max_groups, int n_groups, int tokens, int shared_tokens, int ntok) {
   TcTiles t;
-  // tiles of up to 64 tokens and the two-CTA shape while the groups hold up to 16 pairs on average. A layer, this shape :
+  // Tiles of at most 8 tokens (prefill_few.cu) where no group can have more, and while the groups hold up to 6 pairs on average: a
+  // tile costs it 0.55 to 0.75 of one of k_tc's, and a group of more than 8 pairs makes two. A layer, there : here at 2 / 3 / 4 / 6 / 8
+  // pairs a group: 256 experts x 7168 x 2048 963 : 1270, 1065 : 1382, 1161 : 1435, 1380 : 1478, 1654 : 1543; at 2 / 4 / 6 / 8 / 10: 128
+  // experts x 2048 x 768, down Q6_K (four layers) 504 : 626, 531 : 632, 581 : 639, 653 : 681, 738 : 698; at 2 / 4 / 6 / 8 / 12: 64 x 2048 x
+  // 1024 80 : 95, 95 : 108, 100 : 112, 109 : 115, 134 : 126.
+  // Above that, tiles of up to 64 tokens and the two-CTA shape while the groups hold up to 16 pairs on average. A layer, this shape :
   // the one-CTA shape, us at 2 / 8 / 16 / 20 / 24 / 32 / 64 pairs a group:
   //   128 experts x 2048 x 768   152 : 190   164 : 213   207 : 222   221 : 232   238 : 241   273 : 250   388 : 330
   //    64 experts x 2048 x 1024  102 : 125   115 : 136   141 : 146   148 : 148   160 : 153   182 : 155   257 : 215
   //    32 experts x 7168 x 2048  234 : 301   252 : 322   313 : 335   332 : 343   333 : 349   407 : 363   611 : 487
   // (the line is below every crossing, 20 to 30 pairs: an average says little of the largest group)
   const int avg = n_pairs / (n_groups < n_pairs ? n_groups : n_pairs);
-  t.ntok = ntok ? ntok : (avg <= 16 ? TcShape<2>::NTOK : TC_NMAX);
+  t.ntok = ntok                                             ? ntok
+           : tokens <= TC_FEW_TOKENS || avg <= TC_FEW_AVG ? TC_FEW_TOKENS
+           : avg <= 16                                      ? TcShape<2>::NTOK
+                                                            : TC_NMAX;
   t.even = ntok != 0;
   t.shared = shared_tokens > 0;
   t.max_tiles = tc_max_tiles(n_pairs, max_groups, t.ntok) + (shared_tokens + t.ntok - 1) / t.ntok;
@@ -897,13 +866,20 @@ static dim3 rows_grid(int n_rows, const TcTiles &t, int cols) {
   long gx = (units / t.max_tiles + 7) / 8;  // a warp writes about one record
   return dim3((unsigned)(gx < 1 ? 1 : gx), (unsigned)t.max_tiles);
 }
-void launch_tc_quant_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x,
-                          uint8_t *rec) {
-  pm_launch(L, k_tc_quant_rows, rows_grid(n_rows, t, cols), 256, 0, t.n, t.tiles, src_row, cols, x, rec);
+static int few_records(const TcTiles &t, int weight_type) {
+  return t.ntok == TC_FEW_TOKENS ? (weight_type == PM_TYPE_Q6_K ? 2 : 1) : 0;
 }
-void launch_tc_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const int8_t *xq,
+void launch_tc_quant_rows(const Launch &L, int weight_type, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x,
+                          uint8_t *rec) {
+  const int few = few_records(t, weight_type);
+  pm_launch(L, few == 0 ? k_tc_quant_rows<0> : (few == 1 ? k_tc_quant_rows<1> : k_tc_quant_rows<2>), rows_grid(n_rows, t, cols), 256, 0, t.n,
+            t.tiles, src_row, cols, x, rec);
+}
+void launch_tc_rows(const Launch &L, int weight_type, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const int8_t *xq,
                     const float *xd, const uint16_t *xbm, const int32_t *xs, uint8_t *rec) {
-  pm_launch(L, k_tc_rows, rows_grid(n_rows, t, cols), 256, 0, t.n, t.tiles, src_row, cols, xq, xd, xbm, xs, rec);
+  const int few = few_records(t, weight_type);
+  pm_launch(L, few == 0 ? k_tc_rows<0> : (few == 1 ? k_tc_rows<1> : k_tc_rows<2>), rows_grid(n_rows, t, cols), 256, 0, t.n, t.tiles, src_row,
+            cols, xq, xd, xbm, xs, rec);
 }
 
 template <int WT, bool DOWN, int PARTS> static cudaError_t tc_start(const Launch &L, const TcArgs &A, long items) {
@@ -974,6 +950,7 @@ cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared_only, boo
   A.act_limit = ly.desc.act_limit;
   A.act_alpha = ly.desc.act_alpha;
   const long items = (long)A.row_tiles * t.max_tiles;
+  if (t.ntok == TC_FEW_TOKENS) return launch_tc_few(L, A, W0.type, down, items);
   cudaError_t e = q6 ? (down ? tc_start_shape<PM_TYPE_Q6_K, true>(L, A, t.ntok, items)
                              : tc_start_shape<PM_TYPE_Q6_K, false>(L, A, t.ntok, items))
                      : (down ? tc_start_shape<PM_TYPE_Q4_K, true>(L, A, t.ntok, items)

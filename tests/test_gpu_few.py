@@ -1,0 +1,75 @@
+"""Tiles of at most 8 tokens (prefill_few.cu): Q4_K and Q6_K products whose sub-block scales are applied to the sums of
+single product steps. Bits of the oracle at the edges of a tile (one column pair, one half, full, one over), for either
+type in either place, on codes and scales of the whole range."""
+import numpy as np
+import pytest
+
+import pelica_b200 as pb
+from pelica_b200 import synth
+from tests.helpers import SMALL, bits_equal
+
+pytestmark = [pytest.mark.gpu, pytest.mark.timeout(600)]
+
+Q4, Q6 = synth.Q4_K, synth.Q6_K
+TYPES = {"q4q4": (Q4, Q4), "q4q6": (Q4, Q6), "q6q4": (Q6, Q4), "q6q6": (Q6, Q6)}
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = pb.Context(0)
+    yield c
+    c.close()
+
+
+def random_blocks(w, ty, rng):
+    """Every code, sub-scale and min of the blocks at random, some blocks with all bits set; small f16 scales."""
+    b = w.reshape(-1, 144 if ty == Q4 else 210)
+    b[:] = rng.integers(0, 256, b.shape, dtype=np.uint8)
+    b[::7] = 255
+    d = np.array([1e-4, 3e-5], np.float16).view(np.uint8)
+    if ty == Q4:
+        b[:, :4] = d
+    else:
+        b[:, 208:] = d[:2]
+        b[1::9, 192:208] = 128  # sub-scales of -128
+
+
+def layer(oracle, ctx, types, seed, **change):
+    cfg = SMALL["c2"].scaled(n_exp=40, type_gate=types[0], type_up=types[0], type_down=types[1], **change)
+    W = synth.make_weights(cfg, seed)
+    rng = np.random.default_rng(seed)
+    for key, ty in (("gate", types[0]), ("up", types[0]), ("down", types[1])):
+        random_blocks(W[key], ty, rng)
+    return cfg, oracle.Layer(oracle.LayerDesc(**cfg.desc_fields()), W), pb.MoeLayer(ctx, cfg).load(W), rng
+
+
+@pytest.mark.parametrize("T", [2, 4, 5, 8])
+@pytest.mark.parametrize("types", sorted(TYPES))
+def test_whole_layers(ctx, oracle, types, T):
+    cfg, ol, gl, rng = layer(oracle, ctx, TYPES[types], 60 + T)
+    x = synth.make_activations(T, cfg.d, 61)
+    x[0] = rng.choice([-1.0, 1.0], cfg.d)  # every activation at the end of its range
+    c0 = ctx.path_counts()
+    got = gl.forward(x)
+    assert ctx.path_counts()["tensor"] - c0["tensor"] == 2
+    assert bits_equal(got, ol.forward(x))
+    gl.close()
+
+
+@pytest.mark.parametrize("most", [1, 3, 8, 9, 20])
+@pytest.mark.parametrize("shard", [False, True])
+@pytest.mark.parametrize("types", ["q4q4", "q6q6"])
+def test_groups_of_every_size(ctx, oracle, types, shard, most):
+    """A given plan: `most` tokens on one expert (above 8: several tiles), one to three on the others; a shard holds some."""
+    change = dict(first_local_expert=1, n_exp_local=30) if shard else {}
+    cfg, ol, gl, rng = layer(oracle, ctx, TYPES[types], 70 + most, **change)
+    T = 20
+    x = synth.make_activations(T, cfg.d, 71)
+    ids = np.stack([rng.choice(np.arange(4, cfg.n_exp), cfg.top_k, replace=False) for _ in range(T)]).astype(np.uint32)
+    ids[:most, 0] = 2
+    w = rng.uniform(0.5, 1.5, ids.shape).astype(np.float32)
+    c0 = ctx.path_counts()
+    got = gl.experts(x, ids, w)
+    assert ctx.path_counts()["tensor"] - c0["tensor"] == 2
+    assert bits_equal(got, ol.experts(x, ids, w))
+    gl.close()
