@@ -433,22 +433,37 @@ static int32_t wmat_maps(const WMat &W, int n_exp, int box_rows, WMaps &M) {
     if (q != cudaDriverEntryPointSuccess || !f) return fail(PM_ERR_CUDA, "cuTensorMapEncodeTiled is not there");
     enc = (pm_encode_tiled_t)f;
   }
-  const bool v32 = q32_weights(W.type), mx = W.type == PM_TYPE_MXFP4 || v32, q4 = W.type == PM_TYPE_Q4_K;
+  if (W.type == PM_TYPE_MXFP4) {
+    // [0]: 128 values, each 16 of them in a place of 16 bytes, swizzled (the form the block-scaled products read; the last box of a
+    // row may reach past it, into the next row's: those values are not multiplied); [1]: 256 values as stored, 128 rows
+    const cuuint64_t rb = mx_row_bytes(W.cols);
+    for (int p = 0; p < 2; p++) {
+      const cuuint64_t dims[3] = {p == 0 ? ((cuuint64_t)W.cols + 127) & ~(cuuint64_t)127 : (cuuint64_t)W.cols / 2, (cuuint64_t)W.rows,
+                                  (cuuint64_t)n_exp},
+                       strides[2] = {rb, (cuuint64_t)W.stride[0]};
+      const cuuint32_t box[3] = {128, p == 0 ? (cuuint32_t)box_rows : 128u, 1}, es[3] = {1, 1, 1};
+      const CUresult r = enc(&M.m[p], p == 0 ? CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, W.plane[0], dims,
+                             strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      if (r != CUDA_SUCCESS) return fail(PM_ERR_CUDA, "cuTensorMapEncodeTiled: %d", (int)r);
+    }
+    return PM_OK;
+  }
+  const bool v32 = q32_weights(W.type), q4 = W.type == PM_TYPE_Q4_K;
   const bool nib64 = v32 && W.type != PM_TYPE_Q8_0;
   const int nb = W.cols / 256, n = q4 ? 1 : 2;
-  // MXFP4: plane 0 alone, boxes of 256 values x 64 rows and x 128 rows (the last box of a row may reach past it);
-  // Q8_0, IQ4_NL and IQ4_XS likewise with 128 values
-  const int block[2] = {q4 ? 144 : (nib64 ? 64 : 128), mx && !nib64 ? 128 : 64};
-  // Q6_K and MXFP4: 128- and 64-byte rows swizzled so that the row-per-thread reads of the unpack have no bank conflicts
+  // Q8_0, IQ4_NL and IQ4_XS: plane 0 alone, boxes of 128 values x 64 rows and x 128 rows (the last box of a row may reach past it)
+  const int block[2] = {q4 ? 144 : (nib64 ? 64 : 128), v32 && !nib64 ? 128 : 64};
+  // 128- and 64-byte rows swizzled so that the row-per-thread reads of the unpack have no bank conflicts
   // (a Q4_K row of 144 bytes has none as it is)
   const CUtensorMapSwizzle sw[2] = {
       q4 ? CU_TENSOR_MAP_SWIZZLE_NONE : (nib64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B),
-      mx && !nib64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B};
+      v32 && !nib64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B};
   for (int p = 0; p < n; p++) {
-    const int plane = mx ? 0 : p;
-    const cuuint64_t row = W.type == PM_TYPE_Q8_0 ? (cuuint64_t)W.cols : mx ? (cuuint64_t)W.cols / 2 : (cuuint64_t)nb * block[p];
+    const int plane = v32 ? 0 : p;
+    const cuuint64_t row = W.type == PM_TYPE_Q8_0 ? (cuuint64_t)W.cols : v32 ? (cuuint64_t)W.cols / 2 : (cuuint64_t)nb * block[p];
     const cuuint64_t dims[3] = {row, (cuuint64_t)W.rows, (cuuint64_t)n_exp}, strides[2] = {row, (cuuint64_t)W.stride[plane]};
-    const cuuint32_t box[3] = {(cuuint32_t)block[p], mx ? 64u << p : (cuuint32_t)box_rows, 1}, es[3] = {1, 1, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)block[p], v32 ? 64u << p : (cuuint32_t)box_rows, 1}, es[3] = {1, 1, 1};
     const CUresult r = enc(&M.m[p], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, W.plane[plane], dims, strides, box, es,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, sw[p], CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -636,7 +651,7 @@ static int32_t upload_mat(pm_layer *ly, WMat &W, int el, const uint8_t *raw) {
   }
   uint8_t *p[4];
   for (int i = 0; i < 4; i++) p[i] = W.plane[i] ? W.plane[i] + (size_t)el * W.stride[i] : nullptr;
-  launch_repack(c->launch(), W.type, src, nb, p[0], p[1], p[2], p[3]);
+  launch_repack(c->launch(), W.type, W.cols, src, nb, p[0], p[1], p[2], p[3]);
   CU(cudaGetLastError());
   CU(cudaStreamSynchronize(c->stream));  // the staging buffer is reused by the next upload
   return PM_OK;
@@ -728,7 +743,7 @@ extern "C" int32_t pm_layer_get_expert(pm_layer *ly, int32_t e, int32_t which, u
   TRY(stage_reserve(c, bytes));
   const uint8_t *p[4];
   for (int i = 0; i < 4; i++) p[i] = W.plane[i] ? W.plane[i] + (size_t)el * W.stride[i] : nullptr;
-  launch_unpack(c->launch(), W.type, c->stage, nb, p[0], p[1], p[2], p[3]);
+  launch_unpack(c->launch(), W.type, W.cols, c->stage, nb, p[0], p[1], p[2], p[3]);
   CU(cudaGetLastError());
   CU(cudaMemcpyAsync(out, c->stage, bytes, cudaMemcpyDeviceToHost, c->stream));
   CU(cudaStreamSynchronize(c->stream));
@@ -765,7 +780,7 @@ static int32_t synth_mat(pm_layer *ly, WMat &W, int n_exp, uint64_t seed, float 
                         seed + 0x1000193ull * (uint64_t)e0, sigma);
     uint8_t *p[4];
     for (int i = 0; i < 4; i++) p[i] = W.plane[i] ? W.plane[i] + (size_t)e0 * W.stride[i] : nullptr;
-    launch_repack(c->launch(), W.type, c->stage, nb_per * n, p[0], p[1], p[2], p[3]);
+    launch_repack(c->launch(), W.type, W.cols, c->stage, nb_per * n, p[0], p[1], p[2], p[3]);
     CU(cudaGetLastError());
   }
   return PM_OK;
@@ -1574,7 +1589,7 @@ extern "C" int32_t pm_dequant(pm_ctx *c, int32_t type, const uint8_t *blocks, si
   for (int i = 0; i < 4; i++) p[i] = pb[i] ? ws_take<uint8_t>(c, pb[i]) : nullptr;
   OutBuf ob;
   float *od = out_dev(c, out, n_values, ob);
-  launch_repack(c->launch(), type, rd, nb, p[0], p[1], p[2], p[3]);
+  launch_repack(c->launch(), type, 0, rd, nb, p[0], p[1], p[2], p[3]);
   launch_dequant(c->launch(), type, n_values, p[0], p[1], p[2], p[3], od);
   CU(cudaGetLastError());
   return out_flush(c, &ob, 1);

@@ -47,20 +47,21 @@ __global__ void k_unpack_q6k(uint8_t *raw, size_t nb, const uint8_t *ql, const u
   else src = d + b * 2;
   *(uint16_t *)(raw + b * 210 + j) = *(const uint16_t *)src;
 }
-// byte-granular split: `head` bytes to plane h, the rest to plane r (or swapped)
+// byte-granular split: `head` bytes to plane h, the rest to plane r (or swapped); row_blocks > 0: every row_blocks
+// blocks of plane r take the room of row_blocks + 1
 __global__ void k_repack_split(const uint8_t *__restrict__ raw, size_t nb, int bb, int head,
-                               uint8_t *ph, uint8_t *pr, int back) {
+                               uint8_t *ph, uint8_t *pr, int back, int row_blocks = 0) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   size_t b = i / bb;
   int j = (int)(i % bb);
   if (b >= nb) return;
   uint8_t *rawm = const_cast<uint8_t *>(raw);
-  uint8_t *p = j < head ? ph + b * head + j : pr + b * (bb - head) + (j - head);
+  uint8_t *p = j < head ? ph + b * head + j : pr + (row_blocks ? b + b / row_blocks : b) * (bb - head) + (j - head);
   if (back) rawm[b * bb + j] = *p;
   else *p = raw[b * bb + j];
 }
 
-void launch_repack(const Launch &L, int type, const uint8_t *raw, size_t nb, uint8_t *p0,
+void launch_repack(const Launch &L, int type, int cols, const uint8_t *raw, size_t nb, uint8_t *p0,
                    uint8_t *p1, uint8_t *p2, uint8_t *p3) {
   if (nb == 0) return;
   switch (type) {
@@ -86,7 +87,8 @@ void launch_repack(const Launch &L, int type, const uint8_t *raw, size_t nb, uin
     }
     case PM_TYPE_MXFP4: {  // scale byte first in the raw block, nibbles after
       size_t n = nb * 17;
-      KLAUNCH(L, k_repack_split, (unsigned)((n + 255) / 256), 256, 0, raw, nb, 17, 1, p1, p0, 0);
+      KLAUNCH(L, k_repack_split, (unsigned)((n + 255) / 256), 256, 0, raw, nb, 17, 1, p1, p0, 0,
+              (cols / 32) & 1 ? cols / 32 : 0);
       break;
     }
     case PM_TYPE_Q8_0: {
@@ -106,7 +108,7 @@ void launch_repack(const Launch &L, int type, const uint8_t *raw, size_t nb, uin
     }
   }
 }
-void launch_unpack(const Launch &L, int type, uint8_t *raw, size_t nb, const uint8_t *p0,
+void launch_unpack(const Launch &L, int type, int cols, uint8_t *raw, size_t nb, const uint8_t *p0,
                    const uint8_t *p1, const uint8_t *p2, const uint8_t *p3) {
   if (nb == 0) return;
   switch (type) {
@@ -134,7 +136,7 @@ void launch_unpack(const Launch &L, int type, uint8_t *raw, size_t nb, const uin
     case PM_TYPE_MXFP4: {
       size_t n = nb * 17;
       KLAUNCH(L, k_repack_split, (unsigned)((n + 255) / 256), 256, 0, raw, nb, 17, 1,
-              const_cast<uint8_t *>(p1), const_cast<uint8_t *>(p0), 1);
+              const_cast<uint8_t *>(p1), const_cast<uint8_t *>(p0), 1, (cols / 32) & 1 ? cols / 32 : 0);
       break;
     }
     case PM_TYPE_Q8_0: {
@@ -1485,7 +1487,7 @@ __device__ __forceinline__ float row_f32(const WMat &W, int el, int r, const flo
   float acc = 0.0f;
   if (W.type == PM_TYPE_MXFP4) {
     int nb = W.cols / 32;
-    const uint8_t *nib = W.plane[0] + (size_t)el * W.stride[0] + (size_t)r * nb * 16;
+    const uint8_t *nib = W.plane[0] + (size_t)el * W.stride[0] + r * mx_row_bytes(W.cols);
     const uint8_t *scl = W.plane[1] + (size_t)el * W.stride[1] + (size_t)r * nb;
     // a lane takes whole blocks (16 bytes of codes, 32 activations): few, wide loads per row
     for (int b = lane; b < nb; b += 32) {
@@ -1642,8 +1644,8 @@ __global__ void __launch_bounds__(256) k_gateup_mx(LayerDev ly, Groups g, const 
   const bool bias = ly.bias_gate != nullptr;
   const uint8_t *gn = G.plane[0] + (size_t)el * G.stride[0], *gs = G.plane[1] + (size_t)el * G.stride[1];
   const uint8_t *un = U.plane[0] + (size_t)el * U.stride[0], *us = U.plane[1] + (size_t)el * U.stride[1];
-  const uint8_t *const nib[4] = {gn + (size_t)r * nb * 16, un + (size_t)r * nb * 16, gn + (size_t)r1 * nb * 16,
-                                 un + (size_t)r1 * nb * 16};
+  const size_t rb = mx_row_bytes(d);
+  const uint8_t *const nib[4] = {gn + r * rb, un + r * rb, gn + r1 * rb, un + r1 * rb};
   const uint8_t *const scl[4] = {gs + (size_t)r * nb, us + (size_t)r * nb, gs + (size_t)r1 * nb, us + (size_t)r1 * nb};
   for (uint32_t i = 0; i < cnt; i++) {
     const uint32_t p = off + i;
@@ -1682,8 +1684,8 @@ __global__ void __launch_bounds__(256) k_down_mx(LayerDev ly, Groups g, const fl
   }
   const uint8_t *dn = Dn.plane[0] + (size_t)el * Dn.stride[0], *ds = Dn.plane[1] + (size_t)el * Dn.stride[1];
   const int rr[4] = {r, min(r + 1, d - 1), min(r + 2, d - 1), min(r + 3, d - 1)};
-  const uint8_t *const nib[4] = {dn + (size_t)rr[0] * nb * 16, dn + (size_t)rr[1] * nb * 16, dn + (size_t)rr[2] * nb * 16,
-                                 dn + (size_t)rr[3] * nb * 16};
+  const size_t rb = mx_row_bytes(ff);
+  const uint8_t *const nib[4] = {dn + rr[0] * rb, dn + rr[1] * rb, dn + rr[2] * rb, dn + rr[3] * rb};
   const uint8_t *const scl[4] = {ds + (size_t)rr[0] * nb, ds + (size_t)rr[1] * nb, ds + (size_t)rr[2] * nb,
                                  ds + (size_t)rr[3] * nb};
   for (uint32_t i = 0; i < cnt; i++) {

@@ -11,7 +11,8 @@
 //  Q6_K : plane 0 = ql (128 B/block), 1 = qh (64 B), 2 = scales (16 B),
 //         3 = d (2 B): the block's four fields split into planes so every
 //         field is aligned; 210 B/block in total, as stored (no padding)
-//  MXFP4: plane 0 = E2M1 nibbles (16 B/block), 1 = E8M0 scale bytes (1 B/block)
+//  MXFP4: plane 0 = E2M1 nibbles (16 B/block, rows padded to an even number of blocks: the expanding tensor
+//         copies of prefill_mx8.cu take rows 32 bytes apart), 1 = E8M0 scale bytes (1 B/block)
 //         (the reference splits gpt-oss tensors the same way, src/oss.rs:241-253)
 //  Q8_0 : plane 0 = int8 values (32 B/block), 1 = f16 scales (2 B/block)
 //  IQ4_NL: plane 0 = codebook indices (16 B/block), 1 = f16 scales (2 B/block)
@@ -28,7 +29,8 @@ struct WMat {
 };
 
 // TMA descriptions of a family's planes as [expert][row][bytes of the row], boxes of 64 rows (gate, up) or 128 rows
-// (down) x one 256-value block (Q4_K: plane 0; Q6_K: ql, qh; MXFP4: the nibbles, and Q8_0,
+// (down) x one 256-value block (Q4_K: plane 0; Q6_K: ql, qh; MXFP4: the nibbles of
+// 128 values, each 16 in a place of 16 bytes, and of 256 values x 128 rows as stored; Q8_0,
 // IQ4_NL, IQ4_XS: the values, with 64 and with 128 rows). Host memory of the layer: launchers copy them into parameters.
 struct WMaps {
   CUtensorMap m[2];
@@ -76,6 +78,8 @@ struct PlanDev {
   uint32_t *pair_token, *pair_pos, *pair_src;  // [P]
 };
 
+// bytes of an MXFP4 row in plane 0
+__host__ __device__ inline size_t mx_row_bytes(int cols) { return ((size_t)(cols / 32) + 1) / 2 * 32; }
 // bytes of one expert's tensor in plane p
 static inline size_t wmat_plane_bytes(int type, int rows, int cols, int p) {
   size_t nb;
@@ -90,7 +94,7 @@ static inline size_t wmat_plane_bytes(int type, int rows, int cols, int p) {
     }
     case PM_TYPE_MXFP4:
       nb = (size_t)rows * (cols / 32);
-      return p == 0 ? nb * 16 : (p == 1 ? nb : 0);
+      return p == 0 ? rows * mx_row_bytes(cols) : (p == 1 ? nb : 0);
     case PM_TYPE_Q8_0:
       nb = (size_t)rows * (cols / 32);
       return p == 0 ? nb * 32 : (p == 1 ? nb * 2 : 0);
@@ -149,9 +153,10 @@ template <typename... P> static inline cudaError_t smem_optin(SmemOptIn &o, void
       dev, (int)bytes, [&](int b) { return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, b); });
 }
 
-void launch_repack(const Launch &L, int type, const uint8_t *raw, size_t n_blocks, uint8_t *p0,
+// cols: of the matrix's rows (0: blocks one after another, whatever row they are of)
+void launch_repack(const Launch &L, int type, int cols, const uint8_t *raw, size_t n_blocks, uint8_t *p0,
                    uint8_t *p1, uint8_t *p2, uint8_t *p3);
-void launch_unpack(const Launch &L, int type, uint8_t *raw, size_t n_blocks, const uint8_t *p0,
+void launch_unpack(const Launch &L, int type, int cols, uint8_t *raw, size_t n_blocks, const uint8_t *p0,
                    const uint8_t *p1, const uint8_t *p2, const uint8_t *p3);
 void launch_dequant(const Launch &L, int type, size_t n_values, const uint8_t *p0,
                     const uint8_t *p1, const uint8_t *p2, const uint8_t *p3, float *out);

@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(MxShape::NT, 1) k_tc_mx(const __grid_constant_
       // 2.5 % of a prompt.) A sum once more in f32: matrix `second`, row r, token n of the tile
       auto again = [&](bool second, int r, int n) {
         const uint32_t p = T.y + (uint32_t)n;
-        return mx_sum_f32((second ? A.w1 + (size_t)el * A.w1_stride : A.w0 + (size_t)el * A.w0_stride) + (size_t)r * (A.cols / 2),
+        return mx_sum_f32((second ? A.w1 + (size_t)el * A.w1_stride : A.w0 + (size_t)el * A.w0_stride) + r * mx_row_bytes(A.cols),
                           (second ? A.s1 + (size_t)el * A.s1_stride : A.s0 + (size_t)el * A.s0_stride) + (size_t)r * nbk,
                           A.x + (size_t)(A.src_row ? A.src_row[p] : p) * A.cols, 0, nbk);
       };

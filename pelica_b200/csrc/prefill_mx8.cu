@@ -1,7 +1,7 @@
 // prefill_mx8.cu - grouped expert products on MXFP4 weights and f32 activations for small groups (a few tokens an
 // expert): tcgen05.mma kind::mxf8f6f4 with block scales. The tensor cores take the E2M1 codes and their E8M0
-// scales as they are stored (src/oss_kernels.rs:41-55: code * 2^(e - 127)), so nothing is decoded; a worker only
-// moves a row's nibbles from the packed box to the operand's layout.
+// scales as they are stored (src/oss_kernels.rs:41-55: code * 2^(e - 127)), so nothing is decoded, and the weights' boxes are
+// expanding copies (16 codes of 4 bits into a place of 16 bytes: the tensor map's 16U4_ALIGN16B): they land as operand A.
 //
 // The activations are exact sums of E4M3 pieces with block scales of their own: x = x1 + x2 + ..., xi the
 // nearest E4M3 of what is left of x, in units of 2^(E - 7 - 5 (i - 1)), E the exponent of the block's largest value.
@@ -14,40 +14,39 @@
 // of a long chain: 1e-5 of the RMS over 2,880 values against 1e-7).
 //
 // A persistent pipeline as in prefill_mx.cu; two CTAs an SM, 128 weight rows (64 of gate and 64 of up, or 128 of down) x
-// 16 tokens (5 pieces) or 32 (4). Rows of gate and up alternate in tensor memory, so the two sums of an output are
-// neighbouring lanes. Bound by the
-// latency of a stage's steps (wait, copy, fence, products, fold: 900 cycles for 128 K values, two CTAs interleave): 31 tokens on
-// 32 experts, d = ff = 2880, 2.8 TB/s of weights; gate/up + down 223 us decoding to bf16, 149 here; 1 token, timed launch by
-// launch, 57 us on the row kernels, 43 here.
+// 16 tokens (5 pieces) or 32 (4), stages of 128 K values that four warps hand on: one thread issues every copy, one warp brings
+// the weights' scales, one issues the products, eight read the sums.
+// Bound by the weights' bytes and, above 8 tokens a tile, the products (two layers' figures in us a layer, before: workers moved the
+// codes from packed boxes to operand A, 900 cycles of latency a stage; 32 experts, d = ff = 2880): 1 token 53 -> 43, 8 tokens 144 -> 105,
+// 31 tokens 182 -> 133, 224 tokens 239 -> 178.
 #include <cuda_fp16.h>
 
 #include "mxsum.cuh"
 
 #define M8_M 128
 #define M8_KS 128     /* K values of a stage: four products of 32 */
-#define M8_RAW (M8_M * 128)   /* packed nibbles of 128 rows x 256 K values: two stages */
-#define M8_AST (M8_M * 128)   /* operand A of a stage: 16 codes = 8 bytes and 8 unused, rows of 128 bytes, swizzled */
+#define M8_AST (M8_M * 128)    /* operand A of a stage: 16 codes = 8 bytes and 8 unused, rows of 128 bytes, swizzled */
+#define M8_ABYTES (M8_M * 64)  /* ... the bytes of it that are copied */
 #define M8_NW 8
 #define M8_NT (32 * (M8_NW + 3))
-#define M8_NA 2     /* places of a stage: operand A, its scales, the tokens' pieces */
 #define M8_IT 4
 #define M8_END 0xfffffffeu
 
 template <int NP> struct M8Shape {
   static constexpr int NTOK = NP == 5 ? 16 : 32;
   static constexpr bool FOLD = NP == 5;
-  static constexpr int NSR = NP == 5 ? 3 : 2;
+  static constexpr int NSR = NP == 5 ? 4 : 3;          // stages: the weights with their scales, the tokens' pieces with theirs
   static constexpr int BST = NP * NTOK * M8_KS + 512;  // the pieces of a stage and their scales
-  static constexpr uint32_t SET = NP * 16;             // columns of a set of sums (folded: two sets)
-  // columns of the scales, 8 on for the other place of a stage: nothing orders a copy of scales behind the products that
+  static constexpr uint32_t SET = NP * NTOK;           // columns of a set of sums (folded: two sets)
+  // columns of the scales, a place a stage: nothing orders a copy of scales behind the products that
   // read the ones before it but the commit that frees the place
-  static constexpr uint32_t SFA = 240, SFB = 244;
+  static constexpr uint32_t SFA = 256 - 8 * NSR, SFB = 256 - 4 * NSR;
   static constexpr int NACC = FOLD ? 2 : 1;
 };
-static_assert(2 * M8Shape<5>::SET <= M8Shape<5>::SFA && 4 * 32 <= M8Shape<4>::SFA, "sums and scales share 256 columns");
+static_assert(2 * M8Shape<5>::SET <= M8Shape<5>::SFA && M8Shape<4>::SET <= M8Shape<4>::SFA, "sums and scales share 256 columns");
 
 struct M8Args {
-  CUtensorMap m0, m1;     // nibble planes of gate or down, of up (boxes of 64 rows; down: of 128)
+  CUtensorMap m0, m1;     // nibble planes of gate or down, of up (expanding boxes of 64 rows; down: of 128)
   const uint8_t *s0, *s1; // their planes of scale bytes
   size_t s0_stride, s1_stride;
   const uint4 *tiles;
@@ -111,7 +110,7 @@ __global__ void __launch_bounds__(128) k_mx8_rows(const int *__restrict__ n_tile
       if ((int)blockIdx.y >= *n_tiles) return;
       T = tiles[blockIdx.y];
     }
-    const int npad = practice ? 128 : ((int)T.z + 15) & ~15, nst = (cols + M8_KS - 1) / M8_KS, nb = practice ? 1 : cols / 32, N = NP * npad;
+    const int npad = practice ? 128 : ((int)T.z + 7) & ~7, nst = (cols + M8_KS - 1) / M8_KS, nb = practice ? 1 : cols / 32, N = NP * npad;
     uint8_t *base = rec + (size_t)(T.w >> 4) * nst * (2048 * NP + 512);
     for (int u = practice ? (int)threadIdx.x : (int)(blockIdx.x * 128 + threadIdx.x); u < nb * npad; u += gridDim.x * 128) {
       const int b = u / npad, r = u - b * npad;
@@ -174,11 +173,14 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
   using S = M8Shape<NP>;
   constexpr int MW = M8_NW, NSR = S::NSR, NACC = S::NACC;
   constexpr int RPC = DOWN ? M8_M : M8_M / 2;  // matrix rows of an item
+  constexpr int HX = S::NTOK / 4;              // gate/up: sums that a thread hands to its partner
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t *sRaw = smem, *sA = sRaw + NSR * M8_RAW, *sB = sA + M8_NA * M8_AST, *sSA = sB + M8_NA * S::BST;
-  M8Item *items = (M8Item *)(sSA + M8_NA * 512);
+  uint8_t *sA = smem, *sB = sA + NSR * M8_AST, *sSA = sB + NSR * S::BST;
+  float *sX = (float *)(sSA + NSR * 512);  // gate/up: [2 halves of the tokens][HX][128 rows]
+  M8Item *items = (M8Item *)((uint8_t *)sX + (DOWN ? 0 : 2 * HX * M8_M * 4));
+  // the rings: full_raw / empty_raw: operand A and its scales, a_ready / a_free: the activations' pieces
   uint64_t *full_raw = (uint64_t *)(items + M8_IT), *empty_raw = full_raw + NSR;
-  uint64_t *a_ready = empty_raw + NSR, *a_free = a_ready + M8_NA, *acc_full = a_free + M8_NA;
+  uint64_t *a_ready = empty_raw + NSR, *a_free = a_ready + NSR, *acc_full = a_free + NSR;
   uint64_t *acc_free = acc_full + NACC, *it_full = acc_free + NACC, *it_empty = it_full + M8_IT;
   uint32_t *tmem_slot = (uint32_t *)(it_empty + M8_IT);
   const int nbk = A.cols / 32, rows = A.rows, nst = (A.cols + M8_KS - 1) / M8_KS;
@@ -191,11 +193,9 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
   }
   if (tid == 0) {
     for (int i = 0; i < NSR; i++) {
-      tc_mbar_init(full_raw + i, 1);
-      tc_mbar_init(empty_raw + i, MW);
-    }
-    for (int i = 0; i < M8_NA; i++) {
-      tc_mbar_init(a_ready + i, MW / 2 + 1);  // the workers of the stage; the pieces' copy
+      tc_mbar_init(full_raw + i, 2);   // the box(es); the scales
+      tc_mbar_init(empty_raw + i, 1);  // the products' commits
+      tc_mbar_init(a_ready + i, 1);
       tc_mbar_init(a_free + i, 1);
     }
     for (int i = 0; i < NACC; i++) {
@@ -226,52 +226,52 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
     // ================= the issuing warp =================
     const uint32_t el = tc_elect() ? 1u : 0u;
     const uint32_t sA_a = tc_s32(sA), sB_a = tc_s32(sB), sSA_a = tc_s32(sSA);
-    uint32_t n_a[2] = {0, 0}, set = 0, ps = 1;
+    uint32_t st = 0, pf = 0, set = 0, ps = 1;  // the rings' place (they go round together) and its phase; the sums' set
     M8Item it;
     for (int k = 0; next_item(k, it); k++) {
       if ((int)it.t.x < 0) continue;
-      const uint32_t npad = (__reduce_max_sync(PM_FULL, it.t.z) + 15u) & ~15u, N = NP * npad;
+      const uint32_t npad = (__reduce_max_sync(PM_FULL, it.t.z) + 7u) & ~7u, N = NP * npad;
       const int s0 = (int)__reduce_max_sync(PM_FULL, (uint32_t)it.s0), s1 = (int)__reduce_max_sync(PM_FULL, (uint32_t)it.s1);
-      // instruction descriptor: A E2M1 (5), B E4M3 (0), both K-major, UE8M0 scales, N, M = 128; bits 4..5 and 29..30: which
-      // byte of the scale columns
-      const uint32_t idesc = (5u << 7) | ((N >> 3) << 17) | (1u << 23) | (1u << 27);
+      // instruction descriptor: A E2M1 (5), B E4M3 (0), both K-major, UE8M0 scales, N (of 16: 40 columns are followed by 8
+      // of whatever lies behind them, which nobody reads), M = 128; bits 4..5 and 29..30: which byte of the scale columns
+      const uint32_t idesc = (5u << 7) | (((N + 15u) >> 4) << 18) | (1u << 23) | (1u << 27);
       for (int s = s0; s < s1; s++) {
-        const uint32_t a = (uint32_t)(s - s0) & 1;
         const bool first = S::FOLD ? ((s - s0) & 1) == 0 : s == s0;
         const bool last = S::FOLD ? ((s - s0) & 1) == 1 || s == s1 - 1 : s == s1 - 1;
-        if (first) tc_wait(acc_free + set, ps, A.err, A.wait_ns);
-        tc_wait(a_ready + a, (a ? n_a[1] : n_a[0]) & 1, A.err, A.wait_ns);
-        if (a) n_a[1]++;
-        else n_a[0]++;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // operand A: rows of 128 bytes, 128-byte swizzle (layout type 2), groups of 8 rows 1024 bytes apart
-        const uint64_t dA = (tc_desc(sA_a + a * M8_AST, 16u, 1024u)) | (2ull << 61);
-        const uint64_t dB = tc_desc(sB_a + a * S::BST, N * 16u, 128u);
+        const uint64_t dA = (tc_desc(sA_a + st * M8_AST, 16u, 1024u)) | (2ull << 61);
+        const uint64_t dB = tc_desc(sB_a + st * S::BST, N * 16u, 128u);
         const int ksteps = min(4, (A.cols - s * M8_KS) / 32);
+        if (first) tc_wait(acc_free + set, ps, A.err, A.wait_ns);
+        tc_wait(a_ready + st, pf, A.err, A.wait_ns);
+        tc_wait(full_raw + st, pf, A.err, A.wait_ns);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (el) {
-          m8_cp_scales(tmem + S::SFA + 8u * a, tc_desc(sSA_a + a * 512u, 128u, 128u));
-          m8_cp_scales(tmem + S::SFB + 8u * a, tc_desc(sB_a + a * S::BST + N * M8_KS, 128u, 128u));
+          m8_cp_scales(tmem + S::SFA + 4u * st, tc_desc(sSA_a + st * 512u, 128u, 128u));
+          m8_cp_scales(tmem + S::SFB + 4u * st, tc_desc(sB_a + st * S::BST + N * M8_KS, 128u, 128u));
 #pragma unroll
           for (uint32_t ks = 0; ks < 4; ks++)
             if ((int)ks < ksteps)
-              m8_mma(tmem + set * S::SET, dA + 2u * ks, dB + (uint64_t)(ks * N * 2u), idesc | (ks << 4) | (ks << 29), tmem + S::SFA + 8u * a,
-                     tmem + S::SFB + 8u * a, !first || ks > 0 ? 1u : 0u);
-          tc_commit(a_free + a);
+              m8_mma(tmem + set * S::SET, dA + 2u * ks, dB + (uint64_t)(ks * N * 2u), idesc | (ks << 4) | (ks << 29), tmem + S::SFA + 4u * st,
+                     tmem + S::SFB + 4u * st, !first || ks > 0 ? 1u : 0u);
+          tc_commit(empty_raw + st);
+          tc_commit(a_free + st);
           if (last) tc_commit(acc_full + set);
         }
         __syncwarp();
+        if (++st == NSR) { st = 0; pf ^= 1; }
         if (last && ++set == NACC) { set = 0; ps ^= 1; }
       }
     }
   } else if (warp == MW + 1) {
-    // ================= one thread: work items and the weights' boxes =================
+    // ================= one thread: work items, the weights' boxes, the activations' pieces =================
     if (tc_elect()) {
-      const uint32_t sRaw_a = tc_s32(sRaw);
+      const uint32_t sA_a = tc_s32(sA), sB_a = tc_s32(sB);
       const int per_tile = A.row_tiles * A.splits, n_items = *A.n_tiles * per_tile, G = (int)gridDim.x;
       int cur = (int)blockIdx.x, nxt = cur + G;
       uint4 Tc = make_uint4(M8_END, 0, 0, 0), Tn = Tc;
       if (cur < n_items) Tc = __ldg(A.tiles + cur / per_tile);
-      uint32_t sr = 0, pr = 1, nr = 0;
+      uint32_t sr = 0, pr = 1, nr = 0, nb = 0;
       bool ok = true;
       for (int k = 0; ok; k++) {
         const int s = k & (M8_IT - 1);
@@ -290,76 +290,102 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
         if (end) break;
         const int fut = 2 * G + (int)atomicAdd(A.next, 1u);  // (needed an item later)
         if (nxt < n_items) Tn = __ldg(A.tiles + nxt / per_tile);
-        if ((int)Tc.x >= 0)
-          for (int q = s0; q < s1; q += 2) {  // nibbles of two stages (a box past the matrix reads zeros; split_stages is even)
-            const uint32_t r = sRaw_a + sr * M8_RAW;
+        if ((int)Tc.x >= 0) {
+          const uint32_t bytes = ((Tc.z + 7) >> 3) * (8u * M8_KS * NP) + 512u;
+          const uint8_t *rec = A.rec + (size_t)(Tc.w >> 4) * nst * (2048 * NP + 512);
+          for (int q = s0; q < s1; q++) {  // (a box past the matrix reads zeros)
             if (nr >= NSR && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
-            tc_mbar_expect(full_raw + sr, (uint32_t)M8_RAW);
-            tc_tma3(r, &A.m0, q * 64, r0, (int)Tc.x, full_raw + sr);  // boxes of 128 rows (down) or 64
-            if (!DOWN) tc_tma3(r + M8_RAW / 2, &A.m1, q * 64, r0, (int)Tc.x, full_raw + sr);
+            const uint32_t a = sA_a + sr * M8_AST;
+            tc_mbar_expect(full_raw + sr, (uint32_t)M8_ABYTES);  // (an expanding copy counts the bytes it has read)
+            tc_tma3(a, &A.m0, q * M8_KS, r0, (int)Tc.x, full_raw + sr);  // boxes of 128 rows (down) or 64
+            if (!DOWN) tc_tma3(a + M8_AST / 2, &A.m1, q * M8_KS, r0, (int)Tc.x, full_raw + sr);
             nr++;
+            if (nb >= NSR && !tc_wait(a_free + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
+            tc_mbar_expect(a_ready + sr, bytes);
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sB_a + sr * S::BST),
+                         "l"(rec + (size_t)q * bytes), "r"(bytes), "r"(tc_s32(a_ready + sr))
+                         : "memory");
+            nb++;
             if (++sr == NSR) { sr = 0; pr ^= 1; }
           }
+        }
         cur = nxt;
         nxt = fut;
         Tc = Tn;
       }
-      // the last copies have landed before the CTA gives up its shared memory
+      // the last copies have landed before the CTA gives up its shared memory (full_raw: also the scales' arrival, which
+      // comes when a wait has not run out; a copy takes microseconds, so the bounded wait covers it in any case)
       for (uint32_t i = 1; i <= NSR && i <= nr; i++) {
         const uint32_t q = nr - i;
         tc_landed(full_raw + q % NSR, (q / NSR) & 1);
       }
+      for (uint32_t i = 1; i <= NSR && i <= nb; i++) {
+        const uint32_t q = nb - i;
+        tc_landed(a_ready + q % NSR, (q / NSR) & 1);
+      }
     }
     __syncwarp();
   } else if (warp == MW + 2) {
-    // ================= the tokens' pieces (a warp of its own: in one loop with the boxes, whose ring is deeper, the
-    // boxes waited for the pieces' places) =================
-    const uint32_t sB_a = tc_s32(sB);
-    uint32_t n_a[2] = {0, 0};
+    // ================= the weights' scales: lane l brings those of the tile's rows l, l + 32, l + 64, l + 96 =================
+    // (gate/up: rows 0..63 are gate's, 64..127 up's). 512 bytes a stage: row r, K block k at (r & 31) * 16 + (r >> 5) * 4 + k.
+    uint32_t sr = 0, pr = 1, n = 0;
     bool ok = true;
     M8Item it;
     for (int k = 0; ok && next_item(k, it); k++) {
       if ((int)it.t.x < 0) continue;
-      const uint32_t bytes = ((it.t.z + 15) >> 4) * (16u * M8_KS * NP) + 512u;
-      const uint8_t *rec = A.rec + (size_t)(it.t.w >> 4) * nst * (2048 * NP + 512);
-      for (int q = it.s0; q < it.s1; q++) {
-        const uint32_t a = (uint32_t)(q - it.s0) & 1;
-        ok = __all_sync(PM_FULL, tc_wait(a_free + a, ((a ? n_a[1] : n_a[0]) & 1) ^ 1, A.err, A.wait_ns));
-        if (!ok) break;
-        if (a) n_a[1]++;
-        else n_a[0]++;
-        if (lane == 0) {
-          tc_mbar_expect(a_ready + a, bytes);
-          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sB_a + a * S::BST),
-                       "l"(rec + (size_t)q * bytes), "r"(bytes), "r"(tc_s32(a_ready + a))
-                       : "memory");
+      const size_t el = it.t.x;
+      const uint8_t *sp[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const bool up = !DOWN && i >= 2;
+        const int row = it.r0 + lane + 32 * (DOWN ? i : (i & 1));
+        sp[i] = (up ? A.s1 + el * A.s1_stride : A.s0 + el * A.s0_stride) + (size_t)min(row, rows - 1) * nbk;
+      }
+      TcBytes8 nx[2][4];  // eight blocks (two stages) at a time, two such ahead
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        nx[0][i].load(sp[i] + 4 * it.s0);
+        nx[1][i].load(sp[i] + 4 * min(it.s0 + 2, nst - 1));
+      }
+#pragma unroll 1
+      for (int s2 = it.s0; s2 < it.s1 && ok; s2 += 2) {
+        unsigned long long sc[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          sc[i] = nx[0][i].get();
+          nx[0][i] = nx[1][i];
+          if (s2 + 4 < it.s1) nx[1][i].load(sp[i] + 4 * (s2 + 4));
         }
-        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+          if (s2 + h < it.s1 && ok) {
+            if (n >= NSR) ok = __all_sync(PM_FULL, tc_wait(empty_raw + sr, pr, A.err, A.wait_ns));
+            if (!ok) break;
+            // (255 is a NaN to the tensor cores, 2^127 of the doubled codes elsewhere: mx_repair's)
+            *(uint4 *)(sSA + sr * 512 + lane * 16) =
+                make_uint4((uint32_t)(sc[0] >> (32 * h)), (uint32_t)(sc[1] >> (32 * h)), (uint32_t)(sc[2] >> (32 * h)), (uint32_t)(sc[3] >> (32 * h)));
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc_mbar_arrive(full_raw + sr);
+            n++;
+            if (++sr == NSR) { sr = 0; pr ^= 1; }
+          }
       }
     }
-    if (lane == 0)  // (as above)
-      for (int a = 0; a < 2; a++) {
-        const uint32_t n = a ? n_a[1] : n_a[0];
-        if (n > 0) tc_landed(a_ready + a, (n - 1) & 1);
-      }
-    __syncwarp();
   } else {
-    // ================= the workers =================
-    // operand A: thread = row m of the even stages (part 0) or the odd ones: a stage's chain of wait, copy and fence has
-    // the time of two; sums: lane m, half `part` of the tokens. Row m of the tile: row m / 2 of gate (m even) or
-    // of up (odd); down: row m.
+    // ================= the workers: lane m of the sums, half `part` of the tokens =================
+    // row m of the tile: gate's row m (m < 64) or up's row m - 64; down: row m
     const int m = tid & 127;
     const int part = (int)__reduce_max_sync(PM_FULL, (unsigned)warp >> 2);
-    const bool up = !DOWN && (m & 1);
-    const int mrow = DOWN ? m : m >> 1, rawr = DOWN ? m : (m >> 1) + 64 * (m & 1);
+    const bool up = !DOWN && m >= 64;
     const uint32_t tlane = tmem + (__reduce_max_sync(PM_FULL, 32u * (warp & 3)) << 16);
-    uint32_t st = 0, sr = 0, pr = 0, set = 0, pf = 0;
+    uint32_t set = 0, pf = 0;
     M8Item it;
     for (int k = 0; next_item(k, it); k++) {
       const uint4 T = it.t;
       const int el = (int)T.x, nvalid = (int)__reduce_max_sync(PM_FULL, T.z), r0 = it.r0;
-      const uint32_t npad = ((uint32_t)nvalid + 15u) & ~15u;
-      const int ew = (int)npad >> 1, e0 = part * ew, row = r0 + mrow;
+      const uint32_t npad = ((uint32_t)nvalid + 7u) & ~7u;
+      const int ew = (int)npad >> 1, e0 = part * ew, row = r0 + (DOWN ? m : (m & 63));
       if (el < 0) {  // an expert another rank holds: zeros (down) / nothing to do (gate/up)
         if (DOWN)
           for (int i = tid; i < nvalid * RPC; i += 32 * M8_NW) {
@@ -368,8 +394,6 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
           }
         continue;
       }
-      // the row's scale bytes, eight blocks (two stages) at a time
-      const uint8_t *sp = (up ? A.s1 + (size_t)el * A.s1_stride : A.s0 + (size_t)el * A.s0_stride) + (size_t)min(row, rows - 1) * nbk;
       float acc[S::NTOK / 2];
 #pragma unroll
       for (int u = 0; u < S::NTOK / 2; u++) acc[u] = 0.0f;
@@ -377,96 +401,82 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
         tc_wait(acc_full + set, pf, A.err, A.wait_ns);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t at = tlane + set * S::SET + (uint32_t)e0;
+        auto columns = [&](int c, auto width) {
+          constexpr int W = decltype(width)::value;
+          uint32_t v[NP][W];
 #pragma unroll
-        for (int c = 0; c < S::NTOK / 2; c += 8)
-          if (c < ew) {
-            uint32_t v[NP][8];
-#pragma unroll
-            for (int p = 0; p < NP; p++) tc_ld8<0>(at + (uint32_t)c + p * npad, v[p]);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-              float t = __uint_as_float(v[NP - 1][u]);
-#pragma unroll
-              for (int p = NP - 2; p >= 0; p--) t = __fadd_rn(t, __uint_as_float(v[p][u]));
-              acc[c + u] = __fadd_rn(acc[c + u], t);
-            }
+          for (int p = 0; p < NP; p++) {
+            if constexpr (W == 8) tc_ld8<0>(at + (uint32_t)c + p * npad, v[p]);
+            else tc_ld4<0>(at + (uint32_t)c + p * npad, v[p]);
           }
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int u = 0; u < W; u++) {
+            float t = __uint_as_float(v[NP - 1][u]);
+#pragma unroll
+            for (int p = NP - 2; p >= 0; p--) t = __fadd_rn(t, __uint_as_float(v[p][u]));
+            acc[c + u] = __fadd_rn(acc[c + u], t);
+          }
+        };
+#pragma unroll
+        for (int c = 0; c < S::NTOK / 2; c += 8) {
+          if (c + 8 <= ew) columns(c, PassC<8>());
+          else if (c < ew) columns(c, PassC<4>());
+        }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) tc_mbar_arrive(acc_free + set);
         if (++set == NACC) { set = 0; pf ^= 1; }
       };
-      TcBytes8 sc_n;
-      sc_n.load(sp + 4 * it.s0);
-      uint8_t *dst = sA + part * M8_AST + m * 128;
+      if (S::FOLD) {
 #pragma unroll 1
-      for (int s2 = it.s0; s2 < it.s1; s2 += 2) {
-        const unsigned long long sc = sc_n.get();
-        if (s2 + 2 < it.s1) sc_n.load(sp + 4 * (s2 + 2));
-        tc_wait(full_raw + sr, pr, A.err, A.wait_ns);
-        const uint8_t *raw = sRaw + sr * M8_RAW + rawr * 128;
-        uint4 q[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++)  // (TMA swizzle: 16-byte piece i of a row sits at i ^ (row & 7))
-          q[i] = *(const uint4 *)(raw + (((4 * part + i) ^ (rawr & 7)) << 4));
-        if (s2 + part < it.s1) {
-          tc_wait(a_free + part, (st & 1) ^ 1, A.err, A.wait_ns);
-          st++;
-#pragma unroll
-          for (int i = 0; i < 4; i++) {  // 32 codes: two groups of 16, the lower half of 16 bytes each
-            *(uint2 *)(dst + (((2 * i) ^ (m & 7)) << 4)) = make_uint2(q[i].x, q[i].y);
-            *(uint2 *)(dst + (((2 * i + 1) ^ (m & 7)) << 4)) = make_uint2(q[i].z, q[i].w);
-          }
-          // (255 is a NaN to the tensor cores, 2^127 of the doubled codes elsewhere: mx_repair's)
-          *(uint32_t *)(sSA + part * 512 + (m & 31) * 16 + (m >> 5) * 4) = (uint32_t)(sc >> (32 * part));
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) tc_mbar_arrive(a_ready + part);
-        }
-        // (given back only now that every word of it has been stored: an arrival is not ordered behind loads whose
-        // registers nobody has read yet, and the next box then lands under them)
-        __syncwarp();
-        if (lane == 0) tc_mbar_arrive(empty_raw + sr);
-        if (++sr == NSR) { sr = 0; pr ^= 1; }
-        if (S::FOLD && s2 > it.s0) fold();  // (of the 256 K values before: these are still being multiplied)
+        for (int s2 = it.s0; s2 < it.s1; s2 += 2) fold();
+      } else {
+        fold();
       }
-      fold();
       // ---- epilogue ----
       const bool on = row < rows && *(volatile int *)A.err == 0;
       mx_repair(
           acc, [&](int u) { return row < rows && u < ew && e0 + u < nvalid; },
           [&](int u) {
             const uint32_t p = T.y + (uint32_t)(e0 + u);
-            return mx_sum_f32((up ? A.w1 + (size_t)el * A.w1_stride : A.w0 + (size_t)el * A.w0_stride) + (size_t)row * (A.cols / 2), sp,
+            return mx_sum_f32((up ? A.w1 + (size_t)el * A.w1_stride : A.w0 + (size_t)el * A.w0_stride) + row * mx_row_bytes(A.cols),
+                              (up ? A.s1 + (size_t)el * A.s1_stride : A.s0 + (size_t)el * A.s0_stride) + (size_t)row * nbk,
                               A.x + (size_t)(A.src_row ? A.src_row[p] : p) * A.cols, 4 * it.s0, min(4 * it.s1, nbk));
           });
       __syncwarp();
       const bool bias = A.bias0 && it.split == 0;
       const float b0 = bias && row < rows ? A.bias0[(size_t)el * rows + row] : 0.0f;
-      const float b1 = !DOWN && bias && row < rows ? A.bias1[(size_t)el * rows + row] : 0.0f;
       float *out = A.out + (size_t)it.split * A.split_stride + (size_t)T.y * rows + row;
+      if constexpr (DOWN) {
 #pragma unroll
-      for (int u = 0; u < S::NTOK / 2; u += 2)
-        if (u < ew) {
-          if constexpr (DOWN) {
+        for (int u = 0; u < S::NTOK / 2; u++)
+          if (u < ew && on && e0 + u < nvalid) out[(size_t)(e0 + u) * rows] = bias ? __fadd_rn(acc[u], b0) : acc[u];
+      } else {
+        // the warps w and w ^ 2 hold gate's and up's sums of the same rows: a gate thread activates the even columns of its
+        // half of the tokens, the up thread the odd ones, each on the other's sum out of shared memory
+        const float b1 = bias && row < rows ? A.bias1[(size_t)el * rows + row] : 0.0f;
+        float *sx = sX + part * HX * M8_M;
 #pragma unroll
-            for (int i = 0; i < 2; i++)
-              if (on && e0 + u + i < nvalid) out[(size_t)(e0 + u + i) * rows] = bias ? __fadd_rn(acc[u + i], b0) : acc[u + i];
-          } else {  // a gate lane activates token u, the up lane beside it token u + 1
-            const float other = __shfl_xor_sync(PM_FULL, up ? acc[u] : acc[u + 1], 1);
-            float gv = up ? other : acc[u], uv = up ? acc[u + 1] : other;
-            const int n = e0 + u + (up ? 1 : 0);
-            if (on && n < nvalid) {
-              if (bias) {
-                gv = __fadd_rn(gv, b0);
-                uv = __fadd_rn(uv, b1);
-              }
-              const float wt = A.wts ? A.wts[A.pair_src[T.y + n]] : 1.0f;
-              out[(size_t)n * rows] = pm_act(A.act, A.act_limit, A.act_alpha, gv, uv, wt, A.wts != nullptr);
+        for (int i = 0; i < HX; i++)
+          if (2 * i < ew) sx[i * M8_M + m] = up ? acc[2 * i] : acc[2 * i + 1];
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + 2 * part + (warp & 1)) : "memory");
+#pragma unroll
+        for (int i = 0; i < HX; i++) {
+          const int n = e0 + 2 * i + (up ? 1 : 0);
+          if (2 * i < ew && n < nvalid) {
+            const float other = sx[i * M8_M + (m ^ 64)];
+            float gv = up ? other : acc[2 * i], uv = up ? acc[2 * i + 1] : other;
+            if (bias) {
+              gv = __fadd_rn(gv, b0);
+              uv = __fadd_rn(uv, b1);
             }
+            const float wt = A.wts ? A.wts[A.pair_src[T.y + n]] : 1.0f;
+            if (on) out[(size_t)n * rows] = pm_act(A.act, A.act_limit, A.act_alpha, gv, uv, wt, A.wts != nullptr);
           }
         }
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + 2 * part + (warp & 1)) : "memory");  // both have read before the next item's sums
+      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -489,8 +499,8 @@ void launch_mx8_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32
 
 template <bool DOWN, int NP> static cudaError_t mx8_start(const Launch &L, const M8Args &A, long items) {
   using S = M8Shape<NP>;
-  constexpr size_t smem = (size_t)S::NSR * M8_RAW + (size_t)M8_NA * M8_AST + (size_t)M8_NA * S::BST + M8_NA * 512 + M8_IT * sizeof(M8Item) +
-                          (2 * S::NSR + 2 * M8_NA + 2 * S::NACC + 2 * M8_IT) * 8 + 16;
+  constexpr size_t smem = (size_t)S::NSR * (M8_AST + S::BST + 512) + (DOWN ? 0 : 2 * (S::NTOK / 4) * M8_M * 4) + M8_IT * sizeof(M8Item) +
+                          (4 * S::NSR + 2 * S::NACC + 2 * M8_IT) * 8 + 16;
   static_assert(smem <= 115712, "two CTAs an SM");
   static SmemOptIn opt;
   const cudaError_t e = smem_optin(opt, k_tc_mx8<DOWN, NP>, smem);
@@ -499,14 +509,14 @@ template <bool DOWN, int NP> static cudaError_t mx8_start(const Launch &L, const
   return pm_launch(L, k_tc_mx8<DOWN, NP>, dim3((unsigned)(items < ctas ? items : ctas)), M8_NT, smem, A);
 }
 
-// Tokens of a tile of a call of T tokens whose groups hold n_pairs / n_groups pairs on average; 128: prefill_mx.cu. A
-// layer, us here : there at 8 / 20 / 28 / 32 / 36 / 48 pairs a group (above 32 two tiles a group here):
-//   32 experts x 2880 x 2880  182 : 257   212 : 271   244 : 280   259 : 284   297 : 287   336 : 302
-//   64 experts x 2048 x 1024  127 : 167   149 : 179   161 : 188   178 : 191   197 : 195   223 : 207
-//   16 experts x 4096 x 4096  211 : 267   241 : 281   287 : 292   310 : 293   328 : 299   377 : 312
+// Tokens of a tile of a call of T tokens whose groups hold n_pairs / n_groups pairs on average; 128: prefill_mx.cu. Four
+// layers of 32 experts x 2880 x 2880, us here : there at 32 / 37 / 44 / 50 / 64 / 87 pairs a group (above 32 two tiles a group here, above 64
+// three): 783 : 1169, 866 : 1195, 932 : 1223, 979 : 1256, 1184 : 1359, 1476 : 1526. (The sums here are also the more exact ones: 6e-7
+// of the RMS from 64 bits against 1.0e-5.)
+#define MX8_AVG 88
 int mx_tile_tokens(int T, int n_pairs, int n_groups) {
   if (T < PM_MX_PROMPT) return M8Shape<5>::NTOK;
-  return n_pairs / (n_groups < n_pairs ? n_groups : n_pairs) <= 28 ? M8Shape<4>::NTOK : 128;
+  return n_pairs / (n_groups < n_pairs ? n_groups : n_pairs) <= MX8_AVG ? M8Shape<4>::NTOK : 128;
 }
 
 // Cuts of K of the down products: a few tokens make ceil(d / 128) items an expert, each a chain of ff / 128 stages;
@@ -534,7 +544,7 @@ cudaError_t launch_tc_mx8(const Launch &L, const LayerDev &ly, bool down, const 
   if (t.max_tiles == 0) return cudaSuccess;
   const WMat &W0 = down ? ly.down : ly.gate, &W1 = ly.up;
   M8Args A;
-  A.m0 = (down ? ly.maps->down : ly.maps->gate).m[down ? 1 : 0];  // boxes of 128 or 64 rows
+  A.m0 = (down ? ly.maps->down : ly.maps->gate).m[0];  // boxes of 128 or 64 rows
   A.m1 = ly.maps->up.m[0];
   A.s0 = W0.plane[1];
   A.s0_stride = W0.stride[1];
