@@ -863,6 +863,7 @@ struct Scratch {
   uint32_t *tiles;  // tile list of the tensor-core kernels
   uint32_t *seg;    // per-segment counts of the plan
   uint8_t *rec;     // activation rows regrouped into the operand of the tensor-core kernels
+  uint8_t *rec_h;   // ... of h, where the gate/up products lay it out themselves
   // shared expert
   int *one; uint32_t *zero_u, *tcount, *iota;
   float *sh; int8_t *shq; float *shd; int32_t *shbsum; uint16_t *shbm; int32_t *shs;
@@ -897,6 +898,12 @@ static size_t scratch_rec_bytes(const pm_layer_desc &D, int T) {
   return r;
 }
 
+// ... of a second one, for the rows of h that the gate/up products lay out themselves
+static size_t scratch_rec_h_bytes(const pm_layer_desc &D, int T) {
+  const int P = T * D.top_k, groups = D.n_exp_local > 0 ? std::min(D.n_exp, D.n_exp_local) : D.n_exp;
+  return mx_layer(D) && mx_tile_tokens(T, P, groups) != 128 ? mx8_rec_bytes(T, P, D.n_exp, D.ff) : 0;
+}
+
 static size_t scratch_bytes(const pm_layer_desc &D, int T) {
   size_t P = (size_t)T * D.top_k, E = (size_t)D.n_exp, d = (size_t)D.d, ff = (size_t)D.ff;
   size_t b = 0;
@@ -908,7 +915,7 @@ static size_t scratch_bytes(const pm_layer_desc &D, int T) {
   b += al(Pm * ff * 4) + al(P * ff) + al(P * (ff / 32 + 1) * 4) + al(P * (ff / 256 + 1) * 4) + al(P * (ff / 32) * 4) * 2;
   b += al(Pm * d * 4 * (mx_layer(D) ? mx_splits(D, (int)P) : 1));
   b += al(tc_tile_words((int)P + T, (int)E + 1) * 4);
-  b += al(scratch_rec_bytes(D, T));
+  b += al(scratch_rec_bytes(D, T)) + al(scratch_rec_h_bytes(D, T));
   if (D.shared) {
     size_t sf = (size_t)D.shared_ff;
     b += al(4) + al(4) * 2 + al((size_t)T * 4);
@@ -949,6 +956,7 @@ static void scratch_carve(pm_ctx *c, const pm_layer_desc &D, int T, Scratch &S) 
   S.tiles = ws_take<uint32_t>(c, tc_tile_words((int)P + T, (int)E + 1));
   S.seg = ws_take<uint32_t>(c, route_seg_words(T, D.n_exp));
   S.rec = ws_take<uint8_t>(c, scratch_rec_bytes(D, T));
+  S.rec_h = ws_take<uint8_t>(c, scratch_rec_h_bytes(D, T));
   if (D.shared) {
     size_t sf = (size_t)D.shared_ff;
     S.one = ws_take<int>(c, 1);
@@ -1059,17 +1067,17 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
     }
     {
       PROF(c, PH_GATEUP);
-      CU(small ? launch_tc_mx8(L, dv, false, g.pair_src, tt, S.rec, x, g.pair_token, w, S.h, 1, 0, c->dev_err, c->wait_ns)
+      CU(small ? launch_tc_mx8(L, dv, false, g.pair_src, tt, S.rec, x, g.pair_token, w, S.h, S.rec_h, 1, 0, c->dev_err, c->wait_ns)
                : launch_tc_mx(L, dv, false, g.pair_src, tt, S.rec, x, g.pair_token, w, S.h, c->dev_err, c->wait_ns));
     }
-    {
+    if (!small) {
       PROF(c, PH_QUANT_H);
-      (small ? launch_mx8_rows : launch_mx_rows)(L, P, tt, nullptr, D.ff, S.h, S.rec);
+      launch_mx_rows(L, P, tt, nullptr, D.ff, S.h, S.rec);
     }
     {
       PROF(c, PH_DOWN);
-      CU(small ? launch_tc_mx8(L, dv, true, g.pair_src, tt, S.rec, S.h, nullptr, nullptr, S.eo, S.eo_parts, (size_t)P * D.d, c->dev_err,
-                               c->wait_ns)
+      CU(small ? launch_tc_mx8(L, dv, true, g.pair_src, tt, S.rec_h, S.h, nullptr, nullptr, S.eo, nullptr, S.eo_parts, (size_t)P * D.d,
+                               c->dev_err, c->wait_ns)
                : launch_tc_mx(L, dv, true, g.pair_src, tt, S.rec, S.h, nullptr, nullptr, S.eo, c->dev_err, c->wait_ns));
     }
     c->path_count[PM_PATH_TENSOR] += 2;

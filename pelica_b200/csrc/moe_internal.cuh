@@ -235,7 +235,7 @@ cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared_only, boo
                       const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns, int fault_block);
 // tensor-core forms for MXFP4 weights and f32 activations: tiles of 128 tokens on bf16 pieces (prefill_mx.cu), smaller
 // ones (mx_tile_tokens) on block-scaled fp8 pieces (prefill_mx8.cu). The rows are regrouped by tile and split into their
-// pieces (rec: mx_rec_bytes / mx8_rec_bytes bytes); the down products of the second may be cut along K into mx_splits
+// pieces (rec: mx_rec_bytes / mx8_rec_bytes bytes); the fp8 gate/up products write the pieces of h themselves (hrec). The down products of the second may be cut along K into mx_splits
 // parts: part s goes to out + s * split_stride.
 size_t mx_rec_bytes(int n_pairs, int max_groups, int cols);
 size_t mx8_rec_bytes(int T, int n_pairs, int max_groups, int cols);
@@ -246,7 +246,7 @@ void launch_mx8_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32
 cudaError_t launch_tc_mx(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
                          const uint8_t *rec, const float *x, const uint32_t *src_row, const float *wts, float *out, int *err, unsigned long long wait_ns);
 cudaError_t launch_tc_mx8(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
-                          const uint8_t *rec, const float *x, const uint32_t *src_row, const float *wts, float *out, int splits,
+                          const uint8_t *rec, const float *x, const uint32_t *src_row, const float *wts, float *out, uint8_t *hrec, int splits,
                           size_t split_stride, int *err, unsigned long long wait_ns);
 // tensor-core (tcgen05 int8) form for Q8_0 / IQ4_NL / IQ4_XS weights and 32-value activation blocks (prefill_q32.cu)
 bool q32_weights(int type);

@@ -61,6 +61,7 @@ struct M8Args {
   const float *wts;
   const uint32_t *pair_src;
   float *out;             // gate/up: h [P][ff]; down: eo [splits][P][d]
+  uint8_t *hrec;          // gate/up: the pieces of h, for the down products
   size_t split_stride;
   int *err;
   unsigned long long wait_ns;
@@ -435,6 +436,10 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
         fold();
       }
       // ---- epilogue ----
+      // (columns past the tile's tokens: of whatever their pieces' places hold)
+#pragma unroll
+      for (int u = 0; u < S::NTOK / 2; u++)
+        if (e0 + u >= nvalid) acc[u] = 0.0f;
       const bool on = row < rows && *(volatile int *)A.err == 0;
       mx_repair(
           acc, [&](int u) { return row < rows && u < ew && e0 + u < nvalid; },
@@ -472,7 +477,25 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
               uv = __fadd_rn(uv, b1);
             }
             const float wt = A.wts ? A.wts[A.pair_src[T.y + n]] : 1.0f;
-            if (on) out[(size_t)n * rows] = pm_act(A.act, A.act_limit, A.act_alpha, gv, uv, wt, A.wts != nullptr);
+            const float h = pm_act(A.act, A.act_limit, A.act_alpha, gv, uv, wt, A.wts != nullptr);
+            if (on) out[(size_t)n * rows] = h;
+            // the warp holds a block of 32 values of token n: its pieces (k_mx8_rows), as the down products read them
+            if (r0 + 32 * (warp & 1) < rows) {  // (rows: a multiple of 32)
+              const uint32_t top = __reduce_max_sync(PM_FULL, __float_as_uint(h) & 0x7fffffffu), N = NP * npad;
+              const int E = (int)(top >> 23) - 127, kb = (r0 >> 5) + (warp & 1), o = (lane & 15) * 2 + (lane >> 4);
+              uint8_t *stage = A.hrec + (size_t)(T.w >> 4) * ((rows + M8_KS - 1) / M8_KS) * (2048 * NP + 512) +
+                               (size_t)(kb >> 2) * (N * M8_KS + 512);
+              uint8_t *dst = stage + (kb & 3) * (N * 32) + (o >> 4) * (N * 16) + (o & 15) + n * 16, *sf = stage + N * M8_KS + (kb & 3);
+              float v = __fmul_rn(h, m8_pow2(-max(E - 7, -126)));
+#pragma unroll
+              for (int p = 0; p < NP; p++) {
+                const int S = max(E - 7 - 5 * p, -126);
+                const uint32_t c = m8_e4m3x2(0.0f, v), nn = (uint32_t)n + p * npad;
+                v = __fmul_rn(__fsub_rn(v, m8_from_e4m3x2(c).x), m8_pow2(S - max(E - 12 - 5 * p, -126)));
+                dst[p * npad * 16] = top >= 0x7f800000u ? 0x7f : (uint8_t)c;
+                if (lane == 0) sf[(nn & 31) * 16 + (nn >> 5) * 4] = (uint8_t)(S + 127);
+              }
+            }
           }
         }
         asm volatile("bar.sync %0, 64;" ::"r"(1 + 2 * part + (warp & 1)) : "memory");  // both have read before the next item's sums
@@ -539,11 +562,12 @@ int mx_splits(const pm_layer_desc &D, int n_pairs) {
 // the grouping's rows. x, src_row: the rows the pieces were made of (as in launch_mx8_rows). splits: cuts of K (down only); split s
 // goes to out + s * split_stride.
 cudaError_t launch_tc_mx8(const Launch &L, const LayerDev &ly, bool down, const uint32_t *pair_src, const TcTiles &t,
-                          const uint8_t *rec, const float *x, const uint32_t *src_row, const float *wts, float *out, int splits,
+                          const uint8_t *rec, const float *x, const uint32_t *src_row, const float *wts, float *out, uint8_t *hrec, int splits,
                           size_t split_stride, int *err, unsigned long long wait_ns) {
   if (t.max_tiles == 0) return cudaSuccess;
   const WMat &W0 = down ? ly.down : ly.gate, &W1 = ly.up;
   M8Args A;
+  A.hrec = hrec;
   A.m0 = (down ? ly.maps->down : ly.maps->gate).m[0];  // boxes of 128 or 64 rows
   A.m1 = ly.maps->up.m[0];
   A.s0 = W0.plane[1];
