@@ -449,7 +449,7 @@ template <int EW, int TW> __global__ void __launch_bounds__(256, 1) k_router_til
     load(ch + RT_ST - 1);
     const float *S = rs + (size_t)(ch % RT_ST) * ROWS * RT_CH + lane;
     const int n = min(RT_CH, d - ch * RT_CH) / 32;  // (d is a multiple of 32)
-    for (int s = 0; s < n; s++) {
+    auto step = [&](int s) {
       float xv[TW];
       if constexpr (PAIRS) {
         uint64_t w2[EW / 2];
@@ -474,6 +474,12 @@ template <int EW, int TW> __global__ void __launch_bounds__(256, 1) k_router_til
 #pragma unroll
           for (int e = 0; e < EW; e++) acc[t][e] = __fmaf_rn(w[e], xv[t], acc[t][e]);
       }
+    };
+    if (PAIRS && n == RT_CH / 32) {  // unrolled: the reads of a step are issued under the arithmetic of the one before
+#pragma unroll
+      for (int s = 0; s < RT_CH / 32; s++) step(s);
+    } else {
+      for (int s = 0; s < n; s++) step(s);
     }
   }
   if constexpr (PAIRS) {
