@@ -918,7 +918,7 @@ cudaError_t launch_route_plan(const Launch &L, const LayerDev &ly, const float *
   return PLAUNCH(L, k_plan_seg_place, nseg, 512, 0, ids, T * K, K, seg, E, pl);
 }
 
-// Router logits, top-k and the dispatch plan of a few tokens (T < 8) in ONE launch: a CTA brings EPC experts' rows
+// Router logits, top-k and the dispatch plan of a few tokens (T <= 8) in ONE launch: a CTA brings EPC experts' rows
 // and the tokens into shared memory by two bulk copies (a row is 8 to 28 KB: loads from registers kept 3 KB an SM
 // in flight, one token on 256 experts x 7168 46 us), a warp a (expert, token); the CTA that finishes last (a ticket
 // counter; nobody waits for anybody) routes every token (scores by all threads, picks by a warp each) and builds the
@@ -1130,7 +1130,7 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
       pl.offset[na] = less;
       pl.count[na] = c;
       if (usage && !slot_table) usage[e] += c;
-      if (tt.tiles) {  // (a group has fewer than 16 pairs: one tile each)
+      if (tt.tiles) {  // (a group has at most 8 pairs: one tile each)
         const int el = e - first_local;
         tt.tiles[na] = make_uint4(el < 0 || el >= n_local ? 0xffffffffu : (uint32_t)el, less, c, 16 * na);
       }
@@ -1155,7 +1155,7 @@ __global__ void __launch_bounds__(256) k_route_plan_small(pm_layer_desc D, const
 
 // whether launch_route_plan_small takes T tokens of this layer: a router row and a token's row have to fit shared memory
 bool route_plan_small_takes(const LayerDev &ly, const float *x, int T) {
-  return ((uintptr_t)x & 15) == 0 && T > 0 && T < PM_SMALL_ROUTE_TOKENS && (size_t)2 * ly.desc.d * 4 <= 200 * 1024;
+  return ((uintptr_t)x & 15) == 0 && T > 0 && T <= PM_SMALL_ROUTE_TOKENS && (size_t)2 * ly.desc.d * 4 <= 200 * 1024;
 }
 // ticket: a zeroed word of the context
 cudaError_t launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits, uint32_t *ids,

@@ -173,7 +173,7 @@ cudaError_t launch_route(const Launch &L, const LayerDev &ly, const float *logit
                   float *w);
 // err: the context's error word (an expert id outside the layer is reported there, never used)
 cudaError_t launch_plan(const Launch &L, const LayerDev &ly, const uint32_t *ids, int T, PlanDev plan, int *err);
-// router + top-k + plan (+ tile list) of T < PM_SMALL_ROUTE_TOKENS tokens in one launch (ticket: a zeroed word the
+// router + top-k + plan (+ tile list) of T <= PM_SMALL_ROUTE_TOKENS tokens in one launch (ticket: a zeroed word the
 // kernel leaves zeroed; slot_table: expert -> slot of an expert-parallel placement, or null)
 #define PM_SMALL_ROUTE_TOKENS 8
 // the token tiles of a grouping for the tensor-core products (prefill_tc.cu)
