@@ -1203,9 +1203,10 @@ static int32_t dev_shared(pm_layer *ly, const float *x, int T, Scratch &S) {
   return shared_gate(ly, x, T, S);
 }
 
-// the whole layer on device pointers (workspace already reserved and carved)
+// the whole layer on device pointers (workspace already reserved and carved); xn_next: where y goes normed, for the next
+// layer of a stack, or null (may be x itself)
 static int32_t dev_forward(pm_layer *ly, const float *x, int T, float *y, bool accumulate,
-                           Scratch &S) {
+                           Scratch &S, float *xn_next = nullptr, float eps = 0.0f) {
   pm_ctx *c = ly->ctx;
   const LayerDev &dv = ly->dev;
   Launch L = c->launch();
@@ -1228,7 +1229,7 @@ static int32_t dev_forward(pm_layer *ly, const float *x, int T, float *y, bool a
   }
   {
     PROF(c, PH_COMBINE);
-    launch_combine(L, dv, S.eo, S.plan.pair_pos, S.w, shared_out, S.shared_logit, T, y, accumulate, S.eo_parts);
+    CU(launch_combine(L, dv, S.eo, S.plan.pair_pos, S.w, shared_out, S.shared_logit, T, y, accumulate, S.eo_parts, xn_next, eps));
   }
   CU(cudaGetLastError());
   return PM_OK;
@@ -1945,12 +1946,13 @@ extern "C" int32_t pm_stack_forward(pm_stack *s, const float *x, int32_t T, floa
       bool ok = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
       int32_t rc = PM_OK;
       if (ok) {
+        size_t done = 0;
         for (pm_layer *ly : s->layers) {
           c->ws_off = mark;
           Scratch S;
           scratch_carve(c, ly->dev.desc, T, S);
-          launch_rmsnorm(c->launch(), q.gx, T, d, s->eps, xn);
-          rc = dev_forward(ly, xn, T, q.gx, true, S);
+          if (done == 0) launch_rmsnorm(c->launch(), q.gx, T, d, s->eps, xn);
+          rc = dev_forward(ly, xn, T, q.gx, true, S, ++done < s->layers.size() ? xn : nullptr, s->eps);
           if (rc != PM_OK) break;
         }
         ok = cudaStreamEndCapture(c->stream, &graph) == cudaSuccess && rc == PM_OK && graph;
@@ -1985,12 +1987,13 @@ extern "C" int32_t pm_stack_forward(pm_stack *s, const float *x, int32_t T, floa
   float *xn = ws_take<float>(c, n);
   if (xc != x) CU(cudaMemcpyAsync(xc, x, n * 4, cudaMemcpyDefault, c->stream));
   size_t mark = c->ws_off;
-  for (pm_layer *ly : s->layers) {
+  for (size_t i = 0; i < s->layers.size(); i++) {
+    pm_layer *ly = s->layers[i];
     c->ws_off = mark;
     Scratch S;
     scratch_carve(c, ly->dev.desc, T, S);
-    { PROF(c, PH_NORM); launch_rmsnorm(c->launch(), xc, T, d, s->eps, xn); }
-    TRY(dev_forward(ly, xn, T, xc, true, S));
+    if (i == 0) { PROF(c, PH_NORM); launch_rmsnorm(c->launch(), xc, T, d, s->eps, xn); }
+    TRY(dev_forward(ly, xn, T, xc, true, S, i + 1 < s->layers.size() ? xn : nullptr, s->eps));
   }
   if (xc != x_out) {
     CU(cudaMemcpyAsync(x_out, xc, n * 4, cudaMemcpyDeviceToHost, c->stream));

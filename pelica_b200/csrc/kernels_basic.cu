@@ -1888,72 +1888,112 @@ void launch_down(const Launch &L, const LayerDev &ly, bool shared, Groups g, int
 // (four columns a thread: 16-byte reads, all K of them in flight; 4096 tokens x 8 x 7168: 256 -> 190 us, 1.06 GB)
 // PARTS: products cut along K, up to four parts a pair (read whole, a part more than once where there are fewer: the
 // reads of a pair are all in flight together; one token x 4 x 2880 in three parts 8.7 us of waiting for one after the other)
-template <bool PARTS>
-__global__ void __launch_bounds__(256) k_combine(int d, int K, int in_combine,
-                                                 const float *__restrict__ eo,
-                                                 const uint32_t *__restrict__ pair_pos,
-                                                 const float *__restrict__ w,
-                                                 const float *__restrict__ shared_out,
-                                                 const float *__restrict__ shared_logit, float *y,
-                                                 int accumulate, int parts, size_t part_stride) {
-  pm_pdl();
-  const int t = blockIdx.y;
-  const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
-  if (c >= d) return;
+struct CombineArgs {
+  int d, K, in_combine, accumulate, parts;
+  size_t part_stride;
+  const float *eo;
+  const uint32_t *pair_pos;
+  const float *w, *shared_out, *shared_logit;
+  float *y;
+};
+// columns c .. c + 3 of token t: the picks in k order, the shared expert, (accumulate) the residual before them; written to y
+template <bool PARTS> __device__ __forceinline__ float4 pm_combine4(const CombineArgs &A, int t, int c) {
+  const int d = A.d, K = A.K;
+  const uint32_t *__restrict__ pair_pos = A.pair_pos + t * K;
+  const float *__restrict__ w = A.w + t * K, *__restrict__ eo = A.eo + c;
   float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 8
   for (int k = 0; k < K; k++) {
-    const uint32_t p = pair_pos[t * K + k];
+    const uint32_t p = __ldg(pair_pos + k);
     // (a pair whose expert id was refused: row 0 read in its place, no branch between the reads)
-    const float *src = eo + (size_t)(p == PM_PAIR_NONE ? 0u : p) * d + c;
+    const float *src = eo + (size_t)(p == PM_PAIR_NONE ? 0u : p) * d;
     float4 v = __ldcs((const float4 *)src);
     if (PARTS) {
       float4 u[3];
 #pragma unroll
-      for (int i = 0; i < 3; i++) u[i] = __ldcs((const float4 *)(src + min(i + 1, parts - 1) * part_stride));
+      for (int i = 0; i < 3; i++) u[i] = __ldcs((const float4 *)(src + min(i + 1, A.parts - 1) * A.part_stride));
 #pragma unroll
       for (int i = 0; i < 3; i++)
-        if (i + 1 < parts)
+        if (i + 1 < A.parts)
           v = make_float4(__fadd_rn(v.x, u[i].x), __fadd_rn(v.y, u[i].y), __fadd_rn(v.z, u[i].z), __fadd_rn(v.w, u[i].w));
     }
     if (p == PM_PAIR_NONE) v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (in_combine) {
-      const float wk = w[t * K + k];
+    if (A.in_combine) {
+      const float wk = __ldg(w + k);
       v = make_float4(__fmul_rn(wk, v.x), __fmul_rn(wk, v.y), __fmul_rn(wk, v.z), __fmul_rn(wk, v.w));
     }
     s = make_float4(__fadd_rn(s.x, v.x), __fadd_rn(s.y, v.y), __fadd_rn(s.z, v.z), __fadd_rn(s.w, v.w));
   }
-  if (shared_out) {
-    float4 v = *(const float4 *)(shared_out + (size_t)t * d + c);
-    if (shared_logit) {
-      const float f = __fdiv_rn(1.0f, __fadd_rn(1.0f, pm_exp(-shared_logit[t])));
+  if (A.shared_out) {
+    float4 v = *(const float4 *)(A.shared_out + (size_t)t * d + c);
+    if (A.shared_logit) {
+      const float f = __fdiv_rn(1.0f, __fadd_rn(1.0f, pm_exp(-A.shared_logit[t])));
       v = make_float4(__fmul_rn(v.x, f), __fmul_rn(v.y, f), __fmul_rn(v.z, f), __fmul_rn(v.w, f));
     }
     s = make_float4(__fadd_rn(s.x, v.x), __fadd_rn(s.y, v.y), __fadd_rn(s.z, v.z), __fadd_rn(s.w, v.w));
   }
-  float *o = y + (size_t)t * d + c;  // (y is the caller's: 4-byte aligned)
-  if (accumulate) s = make_float4(__fadd_rn(o[0], s.x), __fadd_rn(o[1], s.y), __fadd_rn(o[2], s.z), __fadd_rn(o[3], s.w));
+  float *o = A.y + (size_t)t * d + c;  // (y is the caller's: 4-byte aligned)
+  if (A.accumulate) s = make_float4(__fadd_rn(o[0], s.x), __fadd_rn(o[1], s.y), __fadd_rn(o[2], s.z), __fadd_rn(o[3], s.w));
   if (((uintptr_t)o & 15) == 0) {
     *(float4 *)o = s;
   } else {
     o[0] = s.x; o[1] = s.y; o[2] = s.z; o[3] = s.w;
   }
+  return s;
+}
+template <bool PARTS> __global__ void __launch_bounds__(256) k_combine(const CombineArgs A) {
+  pm_pdl();
+  const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
+  if (c < A.d) pm_combine4<PARTS>(A, blockIdx.y, c);
+}
+// The combine step of a stack's layer and the norm in front of the next one: a CTA a token, whose row stays in shared
+// memory between the two (k_combine's and k_rmsnorm's values).
+template <bool PARTS> __global__ void __launch_bounds__(1024) k_combine_norm(const CombineArgs A, float eps, float *__restrict__ xn) {
+  pm_pdl();
+  extern __shared__ __align__(16) float row[];
+  __shared__ float red8[8];
+  const int t = blockIdx.x;
+  for (int c = threadIdx.x * 4; c < A.d; c += blockDim.x * 4) *(float4 *)(row + c) = pm_combine4<PARTS>(A, t, c);
+  __syncthreads();
+  const float inv = pm_rms_inv(row, A.d, eps, red8);
+  for (int c = threadIdx.x * 4; c < A.d; c += blockDim.x * 4) {
+    const float4 v = *(const float4 *)(row + c);
+    *(float4 *)(xn + (size_t)t * A.d + c) = make_float4(__fmul_rn(v.x, inv), __fmul_rn(v.y, inv), __fmul_rn(v.z, inv), __fmul_rn(v.w, inv));
+  }
 }
 
-void launch_combine(const Launch &L, const LayerDev &ly, const float *eo, const uint32_t *pair_pos,
-                    const float *w, const float *shared_out, const float *shared_logit, int T,
-                    float *y, bool accumulate, int parts) {
-  if (T == 0) return;
-  int d = ly.desc.d;
-  dim3 grid((d + 1023) / 1024, T);
-  if (parts > 1)
-    PLAUNCH(L, k_combine<true>, grid, 256, 0, d, ly.desc.top_k,
-            (int)(ly.desc.weight_fold == PM_FOLD_IN_COMBINE), eo, pair_pos, w, shared_out,
-            shared_logit, y, (int)accumulate, parts, (size_t)T * ly.desc.top_k * d);
-  else
-    PLAUNCH(L, k_combine<false>, grid, 256, 0, d, ly.desc.top_k,
-            (int)(ly.desc.weight_fold == PM_FOLD_IN_COMBINE), eo, pair_pos, w, shared_out,
-            shared_logit, y, (int)accumulate, parts, (size_t)T * ly.desc.top_k * d);
+// xn: the next layer's normed rows (16-byte aligned), or null
+cudaError_t launch_combine(const Launch &L, const LayerDev &ly, const float *eo, const uint32_t *pair_pos,
+                           const float *w, const float *shared_out, const float *shared_logit, int T,
+                           float *y, bool accumulate, int parts, float *xn, float eps) {
+  if (T == 0) return cudaSuccess;
+  const int d = ly.desc.d;
+  CombineArgs A;
+  A.d = d;
+  A.K = ly.desc.top_k;
+  A.in_combine = ly.desc.weight_fold == PM_FOLD_IN_COMBINE;
+  A.accumulate = accumulate;
+  A.parts = parts;
+  A.part_stride = (size_t)T * ly.desc.top_k * d;
+  A.eo = eo;
+  A.pair_pos = pair_pos;
+  A.w = w;
+  A.shared_out = shared_out;
+  A.shared_logit = shared_logit;
+  A.y = y;
+  if (!xn) {
+    const dim3 grid((d + 1023) / 1024, T);
+    return parts > 1 ? PLAUNCH(L, k_combine<true>, grid, 256, 0, A) : PLAUNCH(L, k_combine<false>, grid, 256, 0, A);
+  }
+  int threads = (d / 4 + 31) & ~31;
+  threads = threads < 256 ? 256 : (threads > 1024 ? 1024 : threads);
+  static SmemOptIn opt[2];
+  const size_t smem = (size_t)d * 4;
+  if (smem > 48 * 1024 - 64) {
+    const cudaError_t e = parts > 1 ? smem_optin(opt[1], k_combine_norm<true>, smem) : smem_optin(opt[0], k_combine_norm<false>, smem);
+    if (e != cudaSuccess) return e;
+  }
+  return parts > 1 ? PLAUNCH(L, k_combine_norm<true>, T, threads, smem, A, eps, xn) : PLAUNCH(L, k_combine_norm<false>, T, threads, smem, A, eps, xn);
 }
 
 // x / rms(x), unit weight; the sum order is pm_rms_inv's (common.cuh)

@@ -188,11 +188,6 @@ struct TcTiles {
 };
 // tokens of each of the n tiles that cnt pairs make. Even tiles for the bf16 products: a weight tile is decoded once a
 // token tile at a cost that a tile of a few tokens does not hide.
-__host__ __device__ inline uint32_t tc_tile_tokens(uint32_t cnt, uint32_t n, int ntok, int even) {
-  return even && n > 1 ? ((cnt + n - 1) / n + 15u) & ~15u : (uint32_t)ntok;
-}
-bool route_plan_small_takes(const LayerDev &ly, const float *x, int T);
-cudaError_t launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits, uint32_t *ids,
 #define TC_FEW_TOKENS 8  // tokens of a tile of prefill_few.cu
 // record rows from one tile of a group to the next, and of a group of cnt pairs in n tiles (every group starts on a multiple
 // of 16; a tile of few tokens has 16 rows of its own)
@@ -200,6 +195,11 @@ __host__ __device__ inline uint32_t tc_tile_rows(int ntok, uint32_t tokens) { re
 __host__ __device__ inline uint32_t tc_group_rows(int ntok, uint32_t cnt, uint32_t n) {
   return ntok == TC_FEW_TOKENS ? 16u * n : (cnt + 15u) & ~15u;
 }
+__host__ __device__ inline uint32_t tc_tile_tokens(uint32_t cnt, uint32_t n, int ntok, int even) {
+  return even && n > 1 ? ((cnt + n - 1) / n + 15u) & ~15u : (uint32_t)ntok;
+}
+bool route_plan_small_takes(const LayerDev &ly, const float *x, int T);
+cudaError_t launch_route_plan_small(const Launch &L, const LayerDev &ly, const float *x, int T, float *logits, uint32_t *ids,
                                     float *w, PlanDev pl, const int32_t *slot_table, unsigned int *ticket, const TcTiles &tt, int *err,
                                     unsigned long long wait_ns);
 // top-k, weights and plan of any number of tokens from their logits (seg: route_seg_words words of scratch)
@@ -266,9 +266,10 @@ void launch_ep_pack(const Launch &L, int P, int row_bytes, int nd, int nbs, cons
 void launch_ep_unmeta(const Launch &L, int R, const uint32_t *meta, int first, int n_local, uint32_t *eids, float *w,
                       int *err);
 void launch_q8x_aux(const Launch &L, size_t n_blocks, const int32_t *bsum, uint16_t *bm, int32_t *xs);
-void launch_combine(const Launch &L, const LayerDev &ly, const float *eo, const uint32_t *pair_pos,
-                    const float *w, const float *shared_out, const float *shared_logit, int T,
-                    float *y, bool accumulate, int parts = 1);
+// xn: null, or where the rows go normed (the next layer of a stack)
+cudaError_t launch_combine(const Launch &L, const LayerDev &ly, const float *eo, const uint32_t *pair_pos,
+                           const float *w, const float *shared_out, const float *shared_logit, int T,
+                           float *y, bool accumulate, int parts = 1, float *xn = nullptr, float eps = 0.0f);
 void launch_rmsnorm(const Launch &L, const float *x, int T, int d, float eps, float *out);
 void launch_shared_gate_logit(const Launch &L, const LayerDev &ly, const float *x, int T,
                               float *out);
