@@ -8,10 +8,11 @@
 // weights in by TMA (boxes of 128 K values) and the tokens' blocks by bulk copies; eight worker warps expand
 // the weights into tensor memory and fold the sums of the stage before; two CTAs an SM.
 //
-// Bound by issue slots (63 to 70 % used): the folds' 2.5 instructions an integer sum on pipes that do 64 a cycle, and
-// at 16 tokens a tile the 560 instructions a warp spends on a stage of four blocks; the row kernels took 8 dp4a a sum
-// and read every weight once a token. 32 experts, 2560 x 640, top-8, gate/up + down: 33 tokens (IQ4_XS) 585 -> 99 us, 1024
-// tokens 18.5 ms -> 0.48 ms.
+// Bound by issue slots: the folds' 2.5 instructions an integer sum on pipes that do 64 a cycle, the expansion of the codes, and what
+// a block costs whatever its columns; so a tile of at most 16 (32) tokens reads the sums of four (two) blocks at once, and one of at
+// most 8 folds a quarter of the product's 16 columns. The row kernels took 8 dp4a a sum and read every weight once a token. 32 experts,
+// 2560 x 640, top-8, IQ4_XS, a layer of 4 / 33 / 200 / 600 tokens: 78 / 144 / 218 / 410 us folding block by block behind one loop for
+// every tile, 65 / 119 / 188 / 342 us here (gate/up + down on the row kernels: 33 tokens 585 us alone).
 #include "tcgen.cuh"
 
 #define Q32_M 128
@@ -288,8 +289,9 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
     for (int k = 0; next_item(k, it); k++) {
       const uint4 T = it.t;
       const int el = (int)T.x, nvalid = (int)__reduce_max_sync(PM_FULL, T.z), r0 = it.r0;
-      const uint32_t npad = ((uint32_t)nvalid + 15u) & ~15u, G = group_of(npad);
-      const int ew = (int)npad >> 1, e0 = part * ew;
+      const uint32_t npad = ((uint32_t)nvalid + 15u) & ~15u;
+      // columns this thread folds: half of the tokens (of a tile of at most 8: a quarter of the product's 16 columns)
+      const int ew = nvalid <= 8 ? 4 : (int)npad >> 1, e0 = part * ew;
       const int row = r0 + (DOWN ? m : (m & 63));
       float *out = A.out + (size_t)T.y * rows + row;
       if (el < 0) {  // an expert another rank holds: zeros (down) / nothing to do (gate/up)
@@ -312,19 +314,77 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
       uint64_t acc[Q32_N / 4];
 #pragma unroll
       for (int i = 0; i < Q32_N / 4; i++) acc[i] = 0;
+      // the sums of a stage for tiles of at most 16 and at most 32 tokens, W columns a thread: the blocks of a slot are read at once
+      auto fold_slots = [&](auto width, auto blocks, int s, unsigned long long sc) {
+        constexpr int W = decltype(width)::value, B = decltype(blocks)::value, NC = 64 / B;  // columns of a block
+        const int nblk = min(Q32_KB, nb - s * Q32_KB);
+        const uint8_t *xd = sB + sb * Q32_BST + NC * 32 + e0 * 4;
+        const float d = XS ? pm_f16((uint32_t)sc) : 0.0f;
+        // XS: the codes of the stage's four scales, low nibbles and two high bits; else four f16 scales
+        uint32_t low = (uint32_t)(sc >> 32) >> (16 * (s & 1)), high = (uint32_t)sc >> (16 + 8 * (s & 1));
+        uint32_t used = 0;
+#pragma unroll 1
+        for (int b0 = 0; b0 < nblk; b0 += B) {
+          tc_wait(acc_full + slot, pf, A.err, A.wait_ns);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t at = tlane + Q32_ACC + slot * 64u + (uint32_t)e0;
+          uint32_t v[B][W];
+#pragma unroll
+          for (int b = 0; b < B; b++) {  // (a block that is not there: whatever its columns hold)
+            if (W == 4) tc_ld4<0>(at + NC * b, v[b]);
+#pragma unroll
+            for (int u = 0; u < W / 8; u++) tc_ld8<0>(at + NC * b + 8 * u, v[b] + 8 * u);
+          }
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int b = 0; b < B; b++)
+            if (b0 + b < nblk) {
+              float dw;
+              if (XS) dw = __fmul_rn(d, (float)((int)(((low >> (4 * b)) & 15u) | (((high >> (2 * b)) & 3u) << 4)) - 32));
+              else dw = pm_f16((uint32_t)(sc >> (16 * b)));
+              const uint64_t dw2 = tc_pack2(dw, dw);
+#pragma unroll
+              for (int u = 0; u < W; u += 4) {
+                const ulonglong2 x2 = *(const ulonglong2 *)(xd + b * (NC * 36) + u * 4);
+                used ^= (uint32_t)x2.x;
+                const uint64_t s0 = tc_pack2(__int2float_rn((int)v[b][u]), __int2float_rn((int)v[b][u + 1]));
+                const uint64_t s1 = tc_pack2(__int2float_rn((int)v[b][u + 2]), __int2float_rn((int)v[b][u + 3]));
+                acc[u / 2] = tc_add2(acc[u / 2], tc_fma2(tc_mul2(dw2, x2.x), s0, A.neg_zero2));
+                acc[u / 2 + 1] = tc_add2(acc[u / 2 + 1], tc_fma2(tc_mul2(dw2, x2.y), s1, A.neg_zero2));
+              }
+            }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) tc_mbar_arrive(acc_free + slot);
+          if (++slot == Q32_NACC) { slot = 0; pf ^= 1; }
+          if (B < Q32_KB) {
+            xd += B * (NC * 36);
+            low >>= 4 * B;
+            high >>= 2 * B;
+            sc >>= 16 * (B & 3);
+          }
+        }
+        if (lane == 0) tc_mbar_arrive_used(empty_b + sb, used, A.zero);
+        if (++sb == Q32_NSB) sb = 0;
+      };
       auto fold = [&](int s, unsigned long long sc) {
+        if (npad == 16u) {
+          if (ew == 4) fold_slots(PassC<4>(), PassC<4>(), s, sc);
+          else fold_slots(PassC<8>(), PassC<4>(), s, sc);
+          return;
+        }
+        if (npad == 32u) {
+          fold_slots(PassC<16>(), PassC<2>(), s, sc);
+          return;
+        }
         const int nblk = min(Q32_KB, nb - s * Q32_KB);
         const uint8_t *xd = sB + sb * Q32_BST + npad * 32u + e0 * 4;
-        uint32_t left = 0, at = 0;  // blocks left in the slot
-        // (not unrolled: with four copies the workers waited for instructions, not for the pipes)
+        // (a slot a block; not unrolled: with four copies the workers waited for instructions, not for the pipes)
 #pragma unroll 1
         for (int b = 0; b < nblk; b++) {
-          if (left == 0) {
-            left = min(G, (uint32_t)(nblk - b));
-            tc_wait(acc_full + slot, pf, A.err, A.wait_ns);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            at = tlane + Q32_ACC + slot * 64u + (uint32_t)e0;
-          }
+          tc_wait(acc_full + slot, pf, A.err, A.wait_ns);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t at = tlane + Q32_ACC + slot * 64u + (uint32_t)e0;
           float dw;
           if (XS) {  // d * (ls - 32) of sub-block ib (src/q4x_cpu.rs:102-117)
             const int ib = 4 * (s & 1) + b;
@@ -335,11 +395,11 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
             dw = pm_f16((uint32_t)(sc >> (16 * b)));
           }
           const uint64_t dw2 = tc_pack2(dw, dw);
-          auto half = [&](int c, auto n_) {  // columns c .. c + 7 (15)
+          auto half = [&](int c, auto n_) {  // columns c .. c + 15
             constexpr int N = decltype(n_)::value;
             uint32_t v[16];
             tc_ld8<0>(at + c, v);
-            if (N > 8) tc_ld8<8>(at + c, v + 8);
+            tc_ld8<8>(at + c, v + 8);
             ulonglong2 x2[N / 4];
 #pragma unroll
             for (int u = 0; u < N / 4; u++) x2[u] = *(const ulonglong2 *)(xd + (c + 4 * u) * 4);
@@ -358,17 +418,13 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
               ac[1] = tc_add2(ac[1], tc_fma2(x2[u / 4].y, s1, A.neg_zero2));
             }
           };
-          if (ew == 8) half(0, PassC<8>());
-          else half(0, PassC<16>());
-          if (ew > 16) half(16, PassC<16>());  // (24 columns: the last 8 are not used)
+          half(0, PassC<16>());
+          half(16, PassC<16>());  // (24 columns: the last 8 are not used)
           xd += npad * 36u;
-          at += npad;
-          if (--left == 0) {
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) tc_mbar_arrive(acc_free + slot);
-            if (++slot == Q32_NACC) { slot = 0; pf ^= 1; }
-          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) tc_mbar_arrive(acc_free + slot);
+          if (++slot == Q32_NACC) { slot = 0; pf ^= 1; }
         }
         __syncwarp();
         uint32_t used = 0;  // (every read of the scales - of four tokens - went into their sums)

@@ -56,6 +56,26 @@ def test_whole_layers(ctx, oracle, types, T):
     gl.close()
 
 
+@pytest.mark.parametrize("most", [1, 7, 8, 9, 16, 17, 32, 33, 48, 49, 64, 65])
+@pytest.mark.parametrize("shape", ["c6", "c7", "c8"])
+def test_folds_of_32_value_blocks(ctx, oracle, shape, most):
+    """The same products' cousins on 32-value blocks (prefill_q32.cu): every width of a fold and a last stage of one block
+    (ff = 160), one expert with `most` tokens and others with a few."""
+    cfg = SMALL[shape].scaled(n_exp=32)
+    W = synth.make_weights(cfg, 90)
+    ol, gl = oracle.Layer(oracle.LayerDesc(**cfg.desc_fields()), W), pb.MoeLayer(ctx, cfg).load(W)
+    T, rng = max(most, 20), np.random.default_rng(90 + most)
+    x = synth.make_activations(T, cfg.d, 91)
+    ids = np.stack([rng.choice(np.arange(4, cfg.n_exp), cfg.top_k, replace=False) for _ in range(T)]).astype(np.uint32)
+    ids[:most, 0] = 2
+    w = rng.uniform(0.5, 1.5, ids.shape).astype(np.float32)
+    c0 = ctx.path_counts()
+    got = gl.experts(x, ids, w)
+    assert ctx.path_counts()["tensor"] - c0["tensor"] == 2
+    assert bits_equal(got, ol.experts(x, ids, w))
+    gl.close()
+
+
 @pytest.mark.parametrize("most", [1, 3, 8, 9, 20])
 @pytest.mark.parametrize("shard", [False, True])
 @pytest.mark.parametrize("types", ["q4q4", "q6q6"])
