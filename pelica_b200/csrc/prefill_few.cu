@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(FW_NT, 2) k_tc_few(const __grid_constant__ TcA
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = __reduce_max_sync(PM_FULL, *tmem_slot);
-  pm_pdl_wait();
+  if (warp != MW + 1) pm_pdl_wait();  // (the producer's weights do not wait: see there)
   auto next_item = [&](int k, TcItem &it) -> bool {
     const int s = k & (TC_IT - 1);
     const bool ok = tc_wait(it_full + s, (uint32_t)((k / TC_IT) & 1), A.err, A.wait_ns);
@@ -149,13 +149,37 @@ __global__ void __launch_bounds__(FW_NT, 2) k_tc_few(const __grid_constant__ TcA
     // ================= the producer: one thread =================
     if (tc_elect()) {
       const uint32_t sRaw_a = tc_s32(sRaw), sB_a = tc_s32(sB);
-      const int n_items = *A.n_tiles * A.row_tiles, G = (int)gridDim.x;
+      const int G = (int)gridDim.x;
       int cur = (int)blockIdx.x, nxt = cur + G;
-      uint4 Tc = make_uint4(TC_END, 0, 0, 0), Tn = Tc;
-      if (cur < n_items) Tc = __ldg(A.tiles + cur / A.row_tiles);
+      uint4 Tc = __ldcg(A.tiles + cur / A.row_tiles), Tn = make_uint4(TC_END, 0, 0, 0);  // (the list has room for every item of the grid)
+      const int n_items = __ldcg(A.n_tiles) * A.row_tiles;
       uint32_t sr = 0, pr = 1, sb = 0, pb = 1;  // stages and the phases of their empty barriers (1: the first round does not wait)
       uint32_t nr = 0, nbk = 0;                 // copies issued per ring (for the end)
       bool ok = true;
+      auto weights = [&](const uint4 &T, int ra, int b) {  // block b of the item's rows -> the next stage
+        const bool sh = T.x == TC_SHARED;
+        const int el = sh ? 0 : (int)T.x;
+        const CUtensorMap *m0 = sh ? A.ms0 : A.m0, *m1 = sh ? A.ms1 : A.m1;
+        const uint32_t r = sRaw_a + sr * S::RAWB;
+        uint64_t *fr = full_raw + sr;
+        tc_mbar_expect(fr, (uint32_t)S::RAWB);  // (a box past the matrix reads zeros)
+        if (!Q6) {
+          tc_tma3(r, m0, b * 144, ra, el, fr);
+          if (!DOWN) tc_tma3(r + 64 * 144, m1, b * 144, ra, el, fr);
+        } else {
+          tc_tma3(r, m0, b * 128, ra, el, fr);
+          if (!DOWN) tc_tma3(r + 64 * 128, m1, b * 128, ra, el, fr);
+          tc_tma3(r + 16384, m0 + 1, b * 64, ra, el, fr);
+          if (!DOWN) tc_tma3(r + 16384 + 64 * 64, m1 + 1, b * 64, ra, el, fr);
+        }
+        nr++;
+        if (++sr == NS) { sr = 0; pr ^= 1; }
+      };
+      // The first item's weights, under the launch before this one, which makes the tokens' records (TC_EARLY_WEIGHTS)
+      int early = 0;
+      if (cur < n_items && (int)Tc.x >= 0)
+        for (; early < min(NS, nb); early++) weights(Tc, (cur % A.row_tiles) * (DOWN ? TC_M : TC_M / 2), early);
+      pm_pdl_wait();
       for (int k = 0; ok; k++) {
         const int s = k & (TC_IT - 1);
         if (k >= TC_IT && !tc_wait(it_empty + s, (uint32_t)((k / TC_IT - 1) & 1), A.err, A.wait_ns)) break;
@@ -166,28 +190,16 @@ __global__ void __launch_bounds__(FW_NT, 2) k_tc_few(const __grid_constant__ TcA
         tc_mbar_arrive(it_full + s);
         if (end) break;
         const int fut = 2 * G + (int)atomicAdd(A.next, 1u);  // (needed an item later)
-        if (nxt < n_items) Tn = __ldg(A.tiles + nxt / A.row_tiles);
+        if (nxt < n_items) Tn = __ldcg(A.tiles + nxt / A.row_tiles);
         if ((int)Tc.x >= 0) {
           const uint8_t *rec = A.rec + (size_t)(Tc.w >> 3) * nb * TC_REC;  // the tile's first record
-          const bool sh = Tc.x == TC_SHARED;
-          const int el = sh ? 0 : (int)Tc.x;
-          const CUtensorMap *m0 = sh ? A.ms0 : A.m0, *m1 = sh ? A.ms1 : A.m1;
           for (int b = 0; b < nb; b++) {
-            const uint32_t r = sRaw_a + sr * S::RAWB;
-            uint64_t *fr = full_raw + sr;
-            if (nr >= NS && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
-            tc_mbar_expect(fr, (uint32_t)S::RAWB);  // (a box past the matrix reads zeros)
-            if (!Q6) {
-              tc_tma3(r, m0, b * 144, ra, el, fr);
-              if (!DOWN) tc_tma3(r + 64 * 144, m1, b * 144, ra, el, fr);
+            if (early > 0) {
+              early--;
             } else {
-              tc_tma3(r, m0, b * 128, ra, el, fr);
-              if (!DOWN) tc_tma3(r + 64 * 128, m1, b * 128, ra, el, fr);
-              tc_tma3(r + 16384, m0 + 1, b * 64, ra, el, fr);
-              if (!DOWN) tc_tma3(r + 16384 + 64 * 64, m1 + 1, b * 64, ra, el, fr);
+              if (nr >= NS && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
+              weights(Tc, ra, b);
             }
-            nr++;
-            if (++sr == NS) { sr = 0; pr ^= 1; }
             if (nbk >= NSB && !tc_wait(empty_b + sb, pb, A.err, A.wait_ns)) { ok = false; break; }
             tc_mbar_expect(full_b + sb, (uint32_t)S::BST);
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(

@@ -122,8 +122,8 @@ __global__ void __launch_bounds__(256) k_mx_rows(const int *__restrict__ n_tiles
                                                  const uint32_t *__restrict__ src_row, int cols, const float *__restrict__ x,
                                                  uint8_t *__restrict__ rec) {
   pm_pdl();
+  const uint4 T = tiles[blockIdx.y];  // (read beside the count: the list has room for every row of the grid)
   if ((int)blockIdx.y >= *n_tiles) return;
-  const uint4 T = tiles[blockIdx.y];
   const int npad = ((int)T.z + 15) & ~15, nch = (cols + MX_KC - 1) / MX_KC;
   uint8_t *base = rec + (size_t)T.w * nch * (MX_KC * 2 * NPC);
   for (int u = blockIdx.x * 256 + threadIdx.x; u < nch * 8 * npad; u += gridDim.x * 256) {

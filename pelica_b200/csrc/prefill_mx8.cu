@@ -108,8 +108,8 @@ __global__ void __launch_bounds__(128) k_mx8_rows(const int *__restrict__ n_tile
     uint4 T = make_uint4(0, 0, 0, 0);
     if (!practice) {
       pm_pdl();
+      T = tiles[blockIdx.y];  // (read beside the count: the list has room for every row of the grid)
       if ((int)blockIdx.y >= *n_tiles) return;
-      T = tiles[blockIdx.y];
     }
     const int npad = practice ? 128 : ((int)T.z + 7) & ~7, nst = (cols + M8_KS - 1) / M8_KS, nb = practice ? 1 : cols / 32, N = NP * npad;
     uint8_t *base = rec + (size_t)(T.w >> 4) * nst * (2048 * NP + 512);
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = __reduce_max_sync(PM_FULL, *tmem_slot);
-  pm_pdl_wait();
+  if (DOWN || warp != MW + 1) pm_pdl_wait();  // (gate/up: the producer waits later)
   auto next_item = [&](int k, M8Item &it) -> bool {
     const int s = k & (M8_IT - 1);
     const bool ok = tc_wait(it_full + s, (uint32_t)((k / M8_IT) & 1), A.err, A.wait_ns);
@@ -268,12 +268,27 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
     // ================= one thread: work items, the weights' boxes, the activations' pieces =================
     if (tc_elect()) {
       const uint32_t sA_a = tc_s32(sA), sB_a = tc_s32(sB);
-      const int per_tile = A.row_tiles * A.splits, n_items = *A.n_tiles * per_tile, G = (int)gridDim.x;
+      const int per_tile = A.row_tiles * A.splits, G = (int)gridDim.x;
       int cur = (int)blockIdx.x, nxt = cur + G;
-      uint4 Tc = make_uint4(M8_END, 0, 0, 0), Tn = Tc;
-      if (cur < n_items) Tc = __ldg(A.tiles + cur / per_tile);
+      uint4 Tc = __ldcg(A.tiles + cur / per_tile), Tn = make_uint4(M8_END, 0, 0, 0);  // (the list has room for every item of the grid)
+      const int n_items = __ldcg(A.n_tiles) * per_tile;
       uint32_t sr = 0, pr = 1, nr = 0, nb = 0;
       bool ok = true;
+      auto weights = [&](int el, int r0, int q) {  // stage q of the item's rows (a box past the matrix reads zeros)
+        const uint32_t s = nr % NSR, a = sA_a + s * M8_AST;
+        tc_mbar_expect(full_raw + s, (uint32_t)M8_ABYTES);  // (an expanding copy counts the bytes it has read)
+        tc_tma3(a, &A.m0, q * M8_KS, r0, el, full_raw + s);  // boxes of 128 rows (down) or 64
+        if (!DOWN) tc_tma3(a + M8_AST / 2, &A.m1, q * M8_KS, r0, el, full_raw + s);
+        nr++;
+      };
+      // gate/up: the first item's weights, under the launch before this one (TC_EARLY_WEIGHTS, prefill_tc.cuh; down follows gate/up, which
+      // lets it in before the plan need be there)
+      int early = 0;
+      if (!DOWN) {
+        if (cur < n_items && (int)Tc.x >= 0)
+          for (; early < min(NSR, nst); early++) weights((int)Tc.x, (cur % per_tile) * RPC, early);
+        pm_pdl_wait();
+      }
       for (int k = 0; ok; k++) {
         const int s = k & (M8_IT - 1);
         if (k >= M8_IT && !tc_wait(it_empty + s, (uint32_t)((k / M8_IT - 1) & 1), A.err, A.wait_ns)) break;
@@ -290,17 +305,17 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
         tc_mbar_arrive(it_full + s);
         if (end) break;
         const int fut = 2 * G + (int)atomicAdd(A.next, 1u);  // (needed an item later)
-        if (nxt < n_items) Tn = __ldg(A.tiles + nxt / per_tile);
+        if (nxt < n_items) Tn = __ldcg(A.tiles + nxt / per_tile);
         if ((int)Tc.x >= 0) {
           const uint32_t bytes = ((Tc.z + 7) >> 3) * (8u * M8_KS * NP) + 512u;
           const uint8_t *rec = A.rec + (size_t)(Tc.w >> 4) * nst * (2048 * NP + 512);
           for (int q = s0; q < s1; q++) {  // (a box past the matrix reads zeros)
-            if (nr >= NSR && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
-            const uint32_t a = sA_a + sr * M8_AST;
-            tc_mbar_expect(full_raw + sr, (uint32_t)M8_ABYTES);  // (an expanding copy counts the bytes it has read)
-            tc_tma3(a, &A.m0, q * M8_KS, r0, (int)Tc.x, full_raw + sr);  // boxes of 128 rows (down) or 64
-            if (!DOWN) tc_tma3(a + M8_AST / 2, &A.m1, q * M8_KS, r0, (int)Tc.x, full_raw + sr);
-            nr++;
+            if (early > 0) {
+              early--;
+            } else {
+              if (nr >= NSR && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
+              weights((int)Tc.x, r0, q);
+            }
             if (nb >= NSR && !tc_wait(a_free + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
             tc_mbar_expect(a_ready + sr, bytes);
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sB_a + sr * S::BST),

@@ -62,8 +62,8 @@ __global__ void __launch_bounds__(128) k_q32_rows(const int *__restrict__ n_tile
     uint4 T = make_uint4(0, 0, 0, 0);
     if (!practice) {
       pm_pdl();
+      T = tiles[blockIdx.y];  // (read beside the count: the list has room for every row of the grid)
       if ((int)blockIdx.y >= *n_tiles) return;
-      T = tiles[blockIdx.y];
     }
     const int npad = practice ? 128 : ((int)T.z + 15) & ~15, nb = practice ? 1 : cols / 32;
     uint8_t *base = rec + (size_t)T.w * nb * 36;
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = __reduce_max_sync(PM_FULL, *tmem_slot);
-  pm_pdl_wait();
+  if (warp != MW + 1) pm_pdl_wait();  // (the producer waits later)
   auto next_item = [&](int k, Q32Item &it) -> bool {
     const int s = k & (Q32_IT - 1);
     const bool ok = tc_wait(it_full + s, (uint32_t)((k / Q32_IT) & 1), A.err, A.wait_ns);
@@ -227,12 +227,25 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
     // ================= the producer: one thread =================
     if (tc_elect()) {
       const uint32_t sRaw_a = tc_s32(sRaw), sB_a = tc_s32(sB);
-      const int n_items = *A.n_tiles * A.row_tiles, G = (int)gridDim.x;
+      const int G = (int)gridDim.x;
       int cur = (int)blockIdx.x, nxt = cur + G;
-      uint4 Tc = make_uint4(Q32_END, 0, 0, 0), Tn = Tc;
-      if (cur < n_items) Tc = __ldg(A.tiles + cur / A.row_tiles);
+      uint4 Tc = __ldcg(A.tiles + cur / A.row_tiles), Tn = make_uint4(Q32_END, 0, 0, 0);  // (the list has room for every item of the grid)
+      const int n_items = __ldcg(A.n_tiles) * A.row_tiles;
       uint32_t sr = 0, pr = 1, sb = 0, pb = 1, nr = 0, ntk = 0;  // (copies issued per ring)
       bool ok = true;
+      auto weights = [&](int el, int r0, int q) {  // stage q of the item's rows (a box past the matrix reads zeros)
+        const uint32_t r = sRaw_a + sr * RAWB;
+        tc_mbar_expect(full_raw + sr, (uint32_t)RAWB);
+        tc_tma3(r, &A.m0, q * RROW, r0, el, full_raw + sr);  // boxes of 128 rows (down) or 64
+        if (!DOWN) tc_tma3(r + RAWB / 2, &A.m1, q * RROW, r0, el, full_raw + sr);
+        nr++;
+        if (++sr == Q32_NSR) { sr = 0; pr ^= 1; }
+      };
+      // the first item's weights, under the launch before this one (TC_EARLY_WEIGHTS, prefill_tc.cuh)
+      int early = 0;
+      if (cur < n_items && (int)Tc.x >= 0)
+        for (; early < min(Q32_NSR, nst); early++) weights((int)Tc.x, (cur % A.row_tiles) * RPC, early);
+      pm_pdl_wait();
       for (int k = 0; ok; k++) {
         const int s = k & (Q32_IT - 1);
         if (k >= Q32_IT && !tc_wait(it_empty + s, (uint32_t)((k / Q32_IT - 1) & 1), A.err, A.wait_ns)) break;
@@ -245,18 +258,18 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
         tc_mbar_arrive(it_full + s);
         if (end) break;
         const int fut = 2 * G + (int)atomicAdd(A.next, 1u);  // (needed an item later)
-        if (nxt < n_items) Tn = __ldg(A.tiles + nxt / A.row_tiles);
+        if (nxt < n_items) Tn = __ldcg(A.tiles + nxt / A.row_tiles);
         if ((int)Tc.x >= 0) {
           const int el = (int)Tc.x;
           const uint32_t per_block = ((Tc.z + 15) >> 4) * (16u * 36u);
           const uint8_t *rec = A.rec + (size_t)Tc.w * nb * 36;
           for (int q = 0; q < nst; q++) {
-            if (nr >= Q32_NSR && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
-            const uint32_t r = sRaw_a + sr * RAWB;
-            tc_mbar_expect(full_raw + sr, (uint32_t)RAWB);  // (a box past the matrix reads zeros)
-            tc_tma3(r, &A.m0, q * RROW, r0, el, full_raw + sr);  // boxes of 128 rows (down) or 64
-            if (!DOWN) tc_tma3(r + RAWB / 2, &A.m1, q * RROW, r0, el, full_raw + sr);
-            nr++;
+            if (early > 0) {
+              early--;
+            } else {
+              if (nr >= Q32_NSR && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
+              weights(el, r0, q);
+            }
             if (ntk >= Q32_NSB && !tc_wait(empty_b + sb, pb, A.err, A.wait_ns)) { ok = false; break; }
             const uint32_t bytes = per_block * (uint32_t)min(Q32_KB, nb - q * Q32_KB);
             tc_mbar_expect(full_b + sb, bytes);
@@ -264,7 +277,6 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
                          "l"(rec + (size_t)q * (per_block * Q32_KB)), "r"(bytes), "r"(tc_s32(full_b + sb))
                          : "memory");
             ntk++;
-            if (++sr == Q32_NSR) { sr = 0; pr ^= 1; }
             if (++sb == Q32_NSB) { sb = 0; pb ^= 1; }
           }
         }

@@ -130,8 +130,8 @@ __global__ void __launch_bounds__(256) k_tc_quant_rows(const int *__restrict__ n
     uint4 T = make_uint4(0, 0, 0, 0);
     if (!practice) {
       pm_pdl();
+      T = tiles[blockIdx.y];  // (read beside the count: the list has room for every row of the grid)
       if ((int)blockIdx.y >= *n_tiles) return;
-      T = tiles[blockIdx.y];
     }
     const int nb = cols / 256;
     const uint32_t off = T.y, cnt = T.z;
@@ -223,8 +223,8 @@ __global__ void __launch_bounds__(256) k_tc_rows(const int *__restrict__ n_tiles
                                                  const uint16_t *__restrict__ xbm, const int32_t *__restrict__ xs,
                                                  uint8_t *__restrict__ rec) {
   pm_pdl();
+  const uint4 T = tiles[blockIdx.y];  // (read beside the count: the list has room for every row of the grid)
   if ((int)blockIdx.y >= *n_tiles) return;
-  const uint4 T = tiles[blockIdx.y];
   const int nb = cols / 256;
   const uint32_t off = T.y, cnt = T.z;
   const int lane = threadIdx.x & 31;
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
   // (a warp reduction leaves its result in a uniform register: what is computed from it - descriptors, addresses,
   // the passes of a block - stays on the uniform datapath instead of being moved there product by product)
   const uint32_t tmem = __reduce_max_sync(PM_FULL, *tmem_slot);
-  pm_pdl_wait();  // (barriers and tensor memory were prepared under the kernel before)
+  if (warp != MW + 1) pm_pdl_wait();  // (barriers and tensor memory were prepared under the kernel before; the producer waits later)
   // the CTA's k-th item, as the issuing warp and the workers take it from the ring (false: no more)
   auto next_item = [&](int k, TcItem &it) -> bool {
     const int s = k & (TC_IT - 1);
@@ -418,13 +418,38 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
     // ================= the producer: one thread =================
     if (tc_elect()) {
       const uint32_t sRaw_a = tc_s32(sRaw), sB_a = tc_s32(sB);
-      const int n_items = *A.n_tiles * A.row_tiles, G = (int)gridDim.x;
+      const int G = (int)gridDim.x;
       int cur = (int)blockIdx.x, nxt = cur + G;
-      uint4 Tc = make_uint4(TC_END, 0, 0, 0), Tn = Tc;
-      if (cur < n_items) Tc = __ldg(A.tiles + cur / A.row_tiles);
+      uint4 Tc = __ldcg(A.tiles + cur / A.row_tiles), Tn = make_uint4(TC_END, 0, 0, 0);  // (the list has room for every item of the grid)
+      const int n_items = __ldcg(A.n_tiles) * A.row_tiles;
       uint32_t sr = 0, pr = 1, sb = 0, pb = 1;  // stages and the phases of their empty barriers (1: the first round does not wait)
       uint32_t nr = 0, nbk = 0;                 // copies issued per ring (for the end)
       bool ok = true;
+      auto weights = [&](const uint4 &T, int ra, int b) {  // block b of the item's rows -> the next raw area (a box past the matrix reads zeros)
+        const bool sh = T.x == TC_SHARED;
+        const int el = sh ? 0 : (int)T.x;
+        const CUtensorMap *m0 = sh ? A.ms0 : A.m0, *m1 = sh ? A.ms1 : A.m1;
+        const uint32_t r = sRaw_a + sr * RAWB;
+        uint64_t *fr = full_raw + sr;
+        tc_mbar_expect(fr, (uint32_t)RAWB);
+        // (a box costs the copy engine about 100 cycles + 3-4 a row: down tiles come as boxes of 128 rows)
+        if (!Q6) {
+          tc_tma3(r, m0, b * 144, ra, el, fr);
+          if (!DOWN) tc_tma3(r + 64 * 144, m1, b * 144, ra, el, fr);
+        } else {
+          tc_tma3(r, m0, b * 128, ra, el, fr);
+          if (!DOWN) tc_tma3(r + 64 * 128, m1, b * 128, ra, el, fr);
+          tc_tma3(r + 16384, m0 + 1, b * 64, ra, el, fr);
+          if (!DOWN) tc_tma3(r + 16384 + 64 * 64, m1 + 1, b * 64, ra, el, fr);
+        }
+        nr++;
+        if (++sr == NS) { sr = 0; pr ^= 1; }
+      };
+      // the first item's weights, under the launch before this one (TC_EARLY_WEIGHTS)
+      int early = 0;
+      if (cur < n_items && (int)Tc.x >= 0)
+        for (; early < min(NS, nb); early++) weights(Tc, (cur % A.row_tiles) * (DOWN ? TC_M : TC_M / 2), early);
+      pm_pdl_wait();
       for (int k = 0; ok; k++) {
         const int s = k & (TC_IT - 1);
         if (k >= TC_IT && !tc_wait(it_empty + s, (uint32_t)((k / TC_IT - 1) & 1), A.err, A.wait_ns)) break;
@@ -436,32 +461,19 @@ __global__ void __launch_bounds__(TcShape<PARTS>::NT, TcShape<PARTS>::CTAS) k_tc
         if (end) break;
         // the item after next, and the next one's tile: asked for now, needed an item later
         const int fut = 2 * G + (int)atomicAdd(A.next, 1u);
-        if (nxt < n_items) Tn = __ldg(A.tiles + nxt / A.row_tiles);
+        if (nxt < n_items) Tn = __ldcg(A.tiles + nxt / A.row_tiles);
         if ((int)Tc.x >= 0) {
           const uint32_t bytes = ((Tc.z + 15) >> 4) * (2u * TC_REC);
           const uint8_t *rec = A.rec + (size_t)(Tc.w >> 3) * nb * TC_REC;  // the tile's first record
-          const bool sh = Tc.x == TC_SHARED;
-          const int el = sh ? 0 : (int)Tc.x;
-          const CUtensorMap *m0 = sh ? A.ms0 : A.m0, *m1 = sh ? A.ms1 : A.m1;
           for (int b = 0; b < nb; b++) {
-            // ---- the weights of block b -> the next raw area (a box past the matrix reads zeros) ----
-            const uint32_t r = sRaw_a + sr * RAWB;
-            uint64_t *fr = full_raw + sr;
-            if (nr >= NS && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
-            TC_STAMP(3, b, 0)
-            tc_mbar_expect(fr, (uint32_t)RAWB);
-            // (a box costs the copy engine about 100 cycles + 3-4 a row: down tiles come as boxes of 128 rows)
-            if (!Q6) {
-              tc_tma3(r, m0, b * 144, ra, el, fr);
-              if (!DOWN) tc_tma3(r + 64 * 144, m1, b * 144, ra, el, fr);
+            // ---- the weights of block b ----
+            if (early > 0) {
+              early--;
             } else {
-              tc_tma3(r, m0, b * 128, ra, el, fr);
-              if (!DOWN) tc_tma3(r + 64 * 128, m1, b * 128, ra, el, fr);
-              tc_tma3(r + 16384, m0 + 1, b * 64, ra, el, fr);
-              if (!DOWN) tc_tma3(r + 16384 + 64 * 64, m1 + 1, b * 64, ra, el, fr);
+              if (nr >= NS && !tc_wait(empty_raw + sr, pr, A.err, A.wait_ns)) { ok = false; break; }
+              TC_STAMP(3, b, 0)
+              weights(Tc, ra, b);
             }
-            nr++;
-            if (++sr == NS) { sr = 0; pr ^= 1; }
             // ---- the tokens' records of block b -> their area ----
             if (nbk >= NSB && !tc_wait(empty_b + sb, pb, A.err, A.wait_ns)) { ok = false; break; }
             TC_STAMP(3, b, 1)
