@@ -187,7 +187,8 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
   const int nbk = A.cols / 32, rows = A.rows, nst = (A.cols + M8_KS - 1) / M8_KS;
   const int tid = threadIdx.x, warp = __shfl_sync(PM_FULL, tid >> 5, 0), lane = tid & 31;
 
-  pm_pdl_trigger();
+  // (gate/up lets the down products in only after its own wait: they read the tile list before theirs)
+  if (DOWN) pm_pdl_trigger();
   if (warp == MW) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_s32(tmem_slot)), "r"(256u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -213,7 +214,10 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = __reduce_max_sync(PM_FULL, *tmem_slot);
-  if (DOWN || warp != MW + 1) pm_pdl_wait();  // (gate/up: the producer waits later)
+  if (warp != MW + 1) {  // (the producer waits later)
+    pm_pdl_wait();
+    if (!DOWN) pm_pdl_trigger();
+  }
   auto next_item = [&](int k, M8Item &it) -> bool {
     const int s = k & (M8_IT - 1);
     const bool ok = tc_wait(it_full + s, (uint32_t)((k / M8_IT) & 1), A.err, A.wait_ns);
@@ -281,14 +285,13 @@ __global__ void __launch_bounds__(M8_NT, 2) k_tc_mx8(const __grid_constant__ M8A
         if (!DOWN) tc_tma3(a + M8_AST / 2, &A.m1, q * M8_KS, r0, el, full_raw + s);
         nr++;
       };
-      // gate/up: the first item's weights, under the launch before this one (TC_EARLY_WEIGHTS, prefill_tc.cuh; down follows gate/up, which
-      // lets it in before the plan need be there)
+      // the first item's weights, under the launch before this one (TC_EARLY_WEIGHTS, prefill_tc.cuh)
       int early = 0;
-      if (!DOWN) {
-        if (cur < n_items && (int)Tc.x >= 0)
-          for (; early < min(NSR, nst); early++) weights((int)Tc.x, (cur % per_tile) * RPC, early);
-        pm_pdl_wait();
+      if (cur < n_items && (int)Tc.x >= 0) {
+        const int in = cur % per_tile, rt = in / A.splits, s0 = (in - rt * A.splits) * A.split_stages;
+        for (; early < min(NSR, min(nst - s0, A.split_stages)); early++) weights((int)Tc.x, rt * RPC, s0 + early);
       }
+      pm_pdl_wait();
       for (int k = 0; ok; k++) {
         const int s = k & (M8_IT - 1);
         if (k >= M8_IT && !tc_wait(it_empty + s, (uint32_t)((k / M8_IT - 1) & 1), A.err, A.wait_ns)) break;

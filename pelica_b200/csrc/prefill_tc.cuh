@@ -44,8 +44,8 @@ struct TcArgs {
 };
 
 // TC_EARLY_WEIGHTS. The product kernels let their producer thread begin before griddepcontrol.wait: it reads the tile list and fills the
-// weights' ring. Allowed because the launch before each of them is a k_*_rows kernel, which lets the next one in only after
-// its own wait: the plan, and all else before that launch, is complete by then, and the weights are nobody's output. (Read
+// weights' ring. Allowed because the launch before each of them - a k_*_rows kernel, or k_tc_mx8's gate/up before its down - lets the
+// next one in only after its own wait: the plan, and all else before that launch, is complete by then, and the weights are nobody's output. (Read
 // past L1: __ldcg.) The tokens' operand and every write come after the wait.
 // (48 layers of 128 experts x 2048 x 768, 8 tokens 3,475 -> 3,326 us; 256 x 7168 x 2048, 1 token 72.4 -> 69.1 us; 64 x 2048 x 1024, 64 tokens
 // 174.5 -> 169.9 us; prompts within 1 %.)
