@@ -1005,12 +1005,12 @@ static Path pick_path(pm_layer *ly, int T, PathCall call) {
   Path p;
   // The integer products give the same bits on either path, so until the caller sets the threshold the faster one
   // decides (us a call, row kernels : tensor cores):
-  //  whole layer: two tokens up (64 experts x 2048 x 1024, 1 / 2 / 3 / 4 / 8 tokens 29 : 36, 40 : 42, 52 : 54, 67 : 62, 109 : 73;
-  //    128 x 2048 x 768 31 : 35, 43 : 45, 58 : 50, 73 : 60, 135 : 95; 4-bit codebook layers of 32 x 2560 x 640 42 : 66, 63 : 68, 87 : 75,
-  //    111 : 77, 193 : 116), and one where the shared expert joins the launch (64 x 7168 x 2048 99 : 87);
+  //  whole layer: two tokens up (64 experts x 2048 x 1024, 1 / 2 / 3 / 4 / 8 tokens 30 : 35, 42 : 34, 51 : 39, 63 : 45, 106 : 61;
+  //    128 x 2048 x 768 31 : 31, 43 : 36, 57 : 39, 73 : 46, 130 : 66; 4-bit codebook layers of 32 x 2560 x 640 43 : 53, 64 : 55, 86 : 60,
+  //    109 : 61, 187 : 70), and one where the shared expert joins the launch (64 x 7168 x 2048 101 : 67);
   //  experts of a given plan, which need the tile list in a launch of their own and may be one row an expert: more than
-  //    16 pairs (a row each, 8 / 16 / 24 rows: 64 x 2048 x 1024 28 : 37, 36 : 41, 48 : 50; 64 x 7168 x 2048 78 : 81, 130 : 127,
-  //    183 : 168; 32 x 2560 x 640 39 : 55, 63 : 66, 90 : 66; 8 an expert's token, 2 / 3 tokens 67 : 70, 79 : 80; 159 : 156, 213 : 196);
+  //    16 pairs (a row each, 8 / 16 / 24 rows: 64 x 2048 x 1024 27 : 31, 37 : 33, 48 : 39; 128 x 2048 x 768 27 : 30, 40 : 35, 53 : 38; 64 x 7168 x 2048
+  //    77 : 62, 132 : 92, 181 : 120; 32 x 2560 x 640 41 : 53, 62 : 55, 83 : 55: the kernels cross between 8 and 16, wide layers below);
   //  shared expert: more than 4 tokens (7168 x 2048, 1 / 4 / 5 / 8 tokens 19 : 47, 41 : 48, 49 : 48, 71 : 49; 2048 x 1024 16 : 27,
   //    20 : 29, 22 : 30, 29 : 31, 12 tokens 39 : 31).
   const bool int_tc = c->tc_min_set            ? T >= c->tc_min_tokens
