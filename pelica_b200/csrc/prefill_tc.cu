@@ -141,9 +141,11 @@ __global__ void __launch_bounds__(256) k_tc_quant_rows(const int *__restrict__ n
     uint8_t *rec0 = rec + (size_t)(T.w >> 3) * nb * TC_REC;
     for (int u = practice ? (int)(threadIdx.x >> 5) : (int)(blockIdx.x * 8 + (threadIdx.x >> 5)); u < units; u += gridDim.x * 8) {
       const int b = u / max(nrg, 1), rgl = u - b * nrg;  // (the tile's records lie block by block)
-      // lane = values 8 lane .. 8 lane + 7 of every row, as two words a row
-      uint32_t q[8][2];
-#pragma unroll
+      // lane = values 8 lane .. 8 lane + 7 of every row = half of K chunk lane / 2; row r of chunk c waits in shared memory in place
+      // r ^ (c & 7) of the chunk's eight (no bank conflicts). Two times four rows through the same code: executed once a warp it is
+      // fetched cold, so half as much of it counts (8 tokens through 48 layers of 128 experts 3,147 -> 3,120 us; prompts the same).
+      const int ch = lane >> 1;
+#pragma unroll 1
       for (int h = 0; h < 2; h++) {
         float v[4][8];
 #pragma unroll
@@ -175,8 +177,9 @@ __global__ void __launch_bounds__(256) k_tc_quant_rows(const int *__restrict__ n
 #pragma unroll
         for (int r = 0; r < 4; r++) {
           const int r8 = 4 * h + r;
-          pm_q8_pack8(v[r], __shfl_sync(PM_FULL, idv, r), q[r8][0], q[r8][1]);
-          int s = __dp4a((int)q[r8][1], 0x01010101, __dp4a((int)q[r8][0], 0x01010101, 0));
+          uint32_t w0, w1;
+          pm_q8_pack8(v[r], __shfl_sync(PM_FULL, idv, r), w0, w1);
+          int s = __dp4a((int)w1, 0x01010101, __dp4a((int)w0, 0x01010101, 0));
           s += __shfl_xor_sync(PM_FULL, s, 1);  // the sum of 32 values: lanes 4 j .. 4 j + 3 hold group j
           s += __shfl_xor_sync(PM_FULL, s, 2);
           if ((lane & 3) == 0) {  // s = 64 * (s >> 6) + (s & 63), both parts exact in f16
@@ -186,26 +189,17 @@ __global__ void __launch_bounds__(256) k_tc_quant_rows(const int *__restrict__ n
           }
           const int tot = __reduce_add_sync(PM_FULL, s);  // (four times the block's sum)
           if (lane == 0) *(int32_t *)(S + TC_REC_XS + r8 * 4) = -4128 * tot;
+          if (FEW == 2 && (ch & 1) != rgl) w0 = w1 = 0u;
+          *(uint2 *)(S + ch * 128 + ((r8 ^ (ch & 7)) << 4) + ((lane & 1) << 3)) = make_uint2(w0, w1);
         }
-      }
-      // K chunk c = lane / 2 holds 16 bytes of each row: an even lane takes rows 0-3 whole, its odd neighbour
-      // rows 4-7 (64 consecutive bytes of the record each); to shared memory without bank conflicts
-      const bool odd = lane & 1;
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const uint32_t s0 = odd ? q[i][0] : q[4 + i][0], s1 = odd ? q[i][1] : q[4 + i][1];
-        const uint32_t t0 = __shfl_xor_sync(PM_FULL, s0, 1), t1 = __shfl_xor_sync(PM_FULL, s1, 1);
-        uint4 o = odd ? make_uint4(t0, t1, q[4 + i][0], q[4 + i][1]) : make_uint4(q[i][0], q[i][1], t0, t1);
-        if (FEW == 2 && ((lane >> 1) & 1) != rgl) o = make_uint4(0, 0, 0, 0);
-        *(uint4 *)(S + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) = o;
       }
       __syncwarp();
       uint4 *R = (uint4 *)(rec0 + (size_t)u * TC_REC);
       if (!practice) {
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-          const int p = 32 * k + lane, l = p >> 2;
-          R[p] = *(const uint4 *)(S + l * 64 + (((p & 3) ^ ((l >> 1) & 3)) << 4));
+          const int p = 32 * k + lane, c = p >> 3;
+          R[p] = *(const uint4 *)(S + c * 128 + (((p & 7) ^ (c & 7)) << 4));
         }
         if (lane < (TC_REC - 2048) / 16 - 4) R[128 + lane] = *(const uint4 *)(S + 2048 + lane * 16);
       }
