@@ -1,6 +1,6 @@
 """MXFP4 products of small groups at the edges of their tiles: groups that fill one, two .. places of 8 tokens, one over,
-and more than one tile, with five and with four pieces; rows of an odd number of blocks; a shard. Also the calls whose
-pieces are made by token beside the routing (up to 8 tokens)."""
+and more than one tile, with five and with four pieces; rows of an odd number of blocks; a shard. Also whole calls on both
+sides of the 8 tokens that one launch routes."""
 import numpy as np
 import pytest
 
@@ -39,9 +39,8 @@ def test_groups_of_every_size(ctx, oracle, shape, T, most):
 
 @pytest.mark.parametrize("T", [3, 7, 8, 9])
 @pytest.mark.parametrize("shape", ["c1", "c3", "c3-odd", "c4", "c4-q6", "c3-shard"])
-def test_by_token_and_by_pair_agree(ctx, oracle, shape, T):
-    """Up to 8 tokens the gate/up products read the rows in token order, more in the order of the pairs: a token's output is
-    the oracle's either way, also where one is no finite number."""
+def test_calls_around_the_one_launch_routing(ctx, oracle, shape, T):
+    """Up to 8 tokens one launch routes and plans the call, above that two or more: the output is the oracle's either way."""
     cfg = {"c3-odd": SMALL["c3"].scaled(d=288, ff=224), "c4-q6": SMALL["c4"].scaled(type_gate=synth.Q6_K, type_up=synth.Q6_K),
            "c3-shard": SMALL["c3"].scaled(first_local_expert=2, n_exp_local=4)}.get(shape) or SMALL[shape]
     ol, gl, _ = make_pair(oracle, pb, ctx, cfg, 88)
