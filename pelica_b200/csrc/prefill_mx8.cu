@@ -16,9 +16,9 @@
 // A persistent pipeline as in prefill_mx.cu; two CTAs an SM, 128 weight rows (64 of gate and 64 of up, or 128 of down) x
 // 16 tokens (5 pieces) or 32 (4), stages of 128 K values that four warps hand on: one thread issues every copy, one warp brings
 // the weights' scales, one issues the products, eight read the sums.
-// Bound by the weights' bytes and, above 8 tokens a tile, the products (two layers' figures in us a layer, before: workers moved the
-// codes from packed boxes to operand A, 900 cycles of latency a stage; 32 experts, d = ff = 2880): 1 token 53 -> 43, 8 tokens 144 -> 105,
-// 31 tokens 182 -> 133, 224 tokens 239 -> 178.
+// Bound by the weights' bytes and, above 8 tokens a tile, the products (whole layers of 32 experts, d = ff = 2880, us a layer, before: workers moved the codes
+// from packed boxes to operand A, 900 cycles of latency a stage, and a launch between the products split h): 1 token 53 -> 37.5, 8 tokens
+// 144 -> 90, 31 tokens 183 -> 126, 224 tokens 239 -> 176.
 #include <cuda_fp16.h>
 
 #include "mxsum.cuh"
