@@ -57,6 +57,10 @@ PM_API int32_t pm_debug_stack_fault_next_call(pm_stack *stack);
  * `block` on (and never signal them): the workers' wait runs out. -1 = off */
 PM_API int32_t pm_debug_tc_fault_block(pm_ctx *ctx, int32_t block);
 
+/* the rule that picks the MXFP4 kernel of a call (no device is touched): tokens of a tile of the block-scaled
+ * fp8 products (16 or 32), or 128 for the bf16 products; 0 for arguments below 1 */
+PM_API int32_t pm_debug_mx_tile_tokens(int32_t tokens, int32_t pairs, int32_t groups, int32_t ff);
+
 /* free device memory as the CUDA runtime reports it (a test checks that a call that must
  * not allocate leaves it unchanged) */
 PM_API int32_t pm_debug_device_free_bytes(pm_ctx *ctx, uint64_t *out);

@@ -132,6 +132,7 @@ ABI_DIAG = {
     "pm_debug_set_wait_limit_ns": (C.c_int32, [_VP, C.c_uint64]),
     "pm_debug_stack_fault_next_call": (C.c_int32, [_VP]),
     "pm_debug_tc_fault_block": (C.c_int32, [_VP, C.c_int32]),
+    "pm_debug_mx_tile_tokens": (C.c_int32, [C.c_int32] * 4),
     "pm_debug_device_free_bytes": (C.c_int32, [_VP, C.POINTER(C.c_uint64)]),
 }
 PATHS = ("general", "tensor", "decode", "multi")

@@ -305,6 +305,9 @@ extern "C" int32_t pm_debug_device_free_bytes(pm_ctx *c, uint64_t *out) {
   *out = (uint64_t)fr;
   return PM_OK;
 }
+extern "C" int32_t pm_debug_mx_tile_tokens(int32_t tokens, int32_t pairs, int32_t groups, int32_t ff) {
+  return tokens < 1 || pairs < 1 || groups < 1 || ff < 1 ? 0 : mx_tile_tokens(tokens, pairs, groups, ff);
+}
 extern "C" int32_t pm_debug_tc_fault_block(pm_ctx *c, int32_t block) {
   if (!c) return fail(PM_ERR_INVALID, "pm_debug_tc_fault_block");
   if (c->tc_fault_block != block) c->dispatch_gen++;
@@ -901,7 +904,7 @@ static size_t scratch_rec_bytes(const pm_layer_desc &D, int T) {
 // ... of a second one, for the rows of h that the gate/up products lay out themselves
 static size_t scratch_rec_h_bytes(const pm_layer_desc &D, int T) {
   const int P = T * D.top_k, groups = D.n_exp_local > 0 ? std::min(D.n_exp, D.n_exp_local) : D.n_exp;
-  return mx_layer(D) && mx_tile_tokens(T, P, groups) != 128 ? mx8_rec_bytes(T, P, D.n_exp, D.ff) : 0;
+  return mx_layer(D) && mx_tile_tokens(T, P, groups, D.ff) != 128 ? mx8_rec_bytes(T, P, D.n_exp, D.ff) : 0;
 }
 
 static size_t scratch_bytes(const pm_layer_desc &D, int T) {
@@ -1032,7 +1035,7 @@ static TcTiles path_tiles(pm_layer *ly, int T, const Path &p, const Scratch &S, 
   const int groups = std::min(D.n_exp, ly->dev.n_local);
   if (p.tc || p.mx || p.q32)
     t = tc_tiles_of(S.tiles, T * D.top_k, D.n_exp, groups, T, merge ? T : 0,
-                    p.mx ? mx_tile_tokens(T, T * D.top_k, groups) : (p.q32 ? q32_tile_tokens() : 0));
+                    p.mx ? mx_tile_tokens(T, T * D.top_k, groups, D.ff) : (p.q32 ? q32_tile_tokens() : 0));
   return t;
 }
 

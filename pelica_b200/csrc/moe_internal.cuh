@@ -239,7 +239,7 @@ cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared_only, boo
 // parts: part s goes to out + s * split_stride.
 size_t mx_rec_bytes(int n_pairs, int max_groups, int cols);
 size_t mx8_rec_bytes(int T, int n_pairs, int max_groups, int cols);
-int mx_tile_tokens(int T, int n_pairs, int n_groups);
+int mx_tile_tokens(int T, int n_pairs, int n_groups, int ff);
 int mx_splits(const pm_layer_desc &D, int n_pairs);
 void launch_mx_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x, uint8_t *rec);
 void launch_mx8_rows(const Launch &L, int n_rows, const TcTiles &t, const uint32_t *src_row, int cols, const float *x, uint8_t *rec);

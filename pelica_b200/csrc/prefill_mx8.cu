@@ -550,14 +550,28 @@ template <bool DOWN, int NP> static cudaError_t mx8_start(const Launch &L, const
   return pm_launch(L, k_tc_mx8<DOWN, NP>, dim3((unsigned)(items < ctas ? items : ctas)), M8_NT, smem, A);
 }
 
-// Tokens of a tile of a call of T tokens whose groups hold n_pairs / n_groups pairs on average; 128: prefill_mx.cu. Four
-// layers of 32 experts x 2880 x 2880, us here : there at 32 / 37 / 44 / 50 / 64 / 87 pairs a group (above 32 two tiles a group here, above 64
-// three): 783 : 1169, 866 : 1195, 932 : 1223, 979 : 1256, 1184 : 1359, 1476 : 1526. (The sums here are also the more exact ones: 6e-7
-// of the RMS from 64 bits against 1.0e-5.)
-#define MX8_AVG 88
-int mx_tile_tokens(int T, int n_pairs, int n_groups) {
+// Tokens of a tile of a call of T tokens whose n_groups groups hold n_pairs / n_groups pairs on average; 128: prefill_mx.cu. Here a group makes
+// a tile every 32 pairs, there mostly one. us a call of one layer, here : there, at 48 / 56 / 60 / 64 / 72 / 88 pairs a group (median of three runs):
+//   24 experts x 2880 x 2880  198 : 232   209 : 246   241 : 250   258 : 255   288 : 259   314 : 287
+//   32 experts x 2880 x 2880  257 : 305   266 : 305   299 : 312   332 : 326   373 : 346   402 : 384
+//   32 experts x 4096 x 1536  199 : 256   219 : 274   239 : 279   267 : 280   297 : 291   336 : 310
+//   64 experts x 2048 x 1024  166 : 201   175 : 211   185 : 216   205 : 218   233 : 227   261 : 258
+//  128 experts x 2880 x 2880  882 : 1035  980 : 1068  1193 : 1133 1197 : 1233 1328 : 1203 1601 : 1417
+// (two layers of 32 x 2880 x 2880 at 80 pairs 785 : 722, at 96 928 : 793; 16 x 4096 x 4096 at 65 / 80 pairs 340 : 317, 378 : 339; 32 x 1024 x 512 at
+// 56 / 64 / 80 59 : 63, 68 : 64, 74 : 72; these kernels run into the power limit, a time repeats within 10 %): the line is at 64, two tiles a group.
+// Up to 88 where the tiles of 128 tokens would leave a sixth of the SMs without work (their gate/up items: 128 rows each, waves of one item an SM):
+//    4 experts x 2880 x 2880 (62 % of a wave)           74 : 99 at 64, 76 : 102 at 72, 78 : 108 at 88
+//    8 experts x 2880 x 2880 (62 % of two)             106 : 143, 112 : 147, 122 : 159
+//    8 experts x 2048 x 1024 (43 % of one)              62 : 75, 63 : 75, 66 : 80
+//   16 experts x 2880 x 2880 (83 % of three)           181 : 210, 192 : 221, 225 : 242
+// and not above (86 % and more: 8 x 4096 x 4096 209 : 204 at 88; 32 x 1024 x 512 76 : 72 at 87).
+// (Sums from four fp8 pieces are 6e-7 of the RMS from 64 bits, from two bf16 pieces 1.0e-5.)
+int mx_tile_tokens(int T, int n_pairs, int n_groups, int ff) {
   if (T < PM_MX_PROMPT) return M8Shape<5>::NTOK;
-  return n_pairs / (n_groups < n_pairs ? n_groups : n_pairs) <= MX8_AVG ? M8Shape<4>::NTOK : 128;
+  const int groups = n_groups < n_pairs ? n_groups : n_pairs, avg = n_pairs / groups;
+  const long places = 148, items = (long)groups * ((ff + M8_M - 1) / M8_M), waves = (items + places - 1) / places;
+  const bool idle = 6 * items < 5 * waves * places;
+  return avg <= 64 || (idle && avg <= 88) ? M8Shape<4>::NTOK : 128;
 }
 
 // Cuts of K of the down products: a few tokens make ceil(d / 128) items an expert, each a chain of ff / 128 stages;
