@@ -1011,14 +1011,17 @@ static Path pick_path(pm_layer *ly, int T, PathCall call) {
   //  whole layer: two tokens up (64 experts x 2048 x 1024, 1 / 2 / 3 / 4 / 8 tokens 30 : 35, 42 : 34, 51 : 39, 63 : 45, 106 : 61;
   //    128 x 2048 x 768 31 : 31, 43 : 36, 57 : 39, 73 : 46, 130 : 66; 4-bit codebook layers of 32 x 2560 x 640 43 : 53, 64 : 55, 86 : 60,
   //    109 : 61, 187 : 70), and one where the shared expert joins the launch (64 x 7168 x 2048 101 : 67);
-  //  experts of a given plan, which need the tile list in a launch of their own and may be one row an expert: more than
-  //    16 pairs (a row each, 8 / 16 / 24 rows: 64 x 2048 x 1024 27 : 31, 37 : 33, 48 : 39; 128 x 2048 x 768 27 : 30, 40 : 35, 53 : 38; 64 x 7168 x 2048
-  //    77 : 62, 132 : 92, 181 : 120; 32 x 2560 x 640 41 : 53, 62 : 55, 83 : 55: the kernels cross between 8 and 16, wide layers below);
+  //  experts of a given plan, which need the tile list in a launch of their own and may be one row an expert: more than 16 pairs, or from 48 K
+  //    pairs x (d + ff) on - a row kernel's time goes with the bytes of its pairs, the tensor cores' hardly. Last call below : first above the line,
+  //    a row each: 64 x 7168 x 2048 5 rows 56 : 53, 6 63 : 57, 8 76 : 61, 16 131 : 91; 64 x 5120 x 1536 7 51 : 40, 8 52 : 47; 64 x 4096 x 1536 8 44 : 41, 9 47 : 42;
+  //    64 x 3072 x 1024 11 39 : 36, 12 41 : 36; 64 x 2048 x 1024 15 36 : 33, 16 37 : 34; 64 x 2048 x 4096 7 47 : 40, 8 54 : 47; 64 x 7168 x 512
+  //    6 34 : 39, 7 46 : 41; Q8_0 32 x 5120 x 1280 7 92 : 69, 8 90 : 81, 32 x 2560 x 640 15 50 : 45, 16 50 : 45; and 64 x 1024 x 512, below
+  //    it up to the 17th, 16 25 : 27 (some shapes cross two to four pairs earlier: the line is where none loses);
   //  shared expert: more than 4 tokens (7168 x 2048, 1 / 4 / 5 / 8 tokens 19 : 47, 41 : 48, 49 : 48, 71 : 49; 2048 x 1024 16 : 27,
   //    20 : 29, 22 : 30, 29 : 31, 12 tokens 39 : 31).
   const bool int_tc = c->tc_min_set            ? T >= c->tc_min_tokens
                       : call == PATH_WHOLE     ? T >= (shared_merges(D) ? 1 : 2)
-                      : call == PATH_EXPERTS   ? T * D.top_k > 16
+                      : call == PATH_EXPERTS   ? T * D.top_k > 16 || T * D.top_k * (D.d + D.ff) >= 48 * 1024
                                                : T > 4;
   p.tc = D.act_quant == PM_AQ_Q8X_256 && c->tc_min_tokens > 0 && int_tc;
   p.tc_gu = p.tc && D.type_gate == D.type_up;

@@ -148,3 +148,28 @@ def test_split_calls_choose_by_their_own_size(ctx, oracle, shape):
             ids, w = gl.route(x)
             assert bits_equal(gl.combine(gl.experts(x, ids, w), ids, w, got), ol.forward(x))
     gl.close()
+
+
+@pytest.mark.parametrize("shape", ["q4q6", "q8_0"])
+def test_split_calls_of_wide_layers(ctx, oracle, shape):
+    """Up to 16 pairs the width decides: from 48 K pairs x (d + ff) on (here 8 pairs) rows and plans take the tensor cores; the same bits."""
+    cfg = {"q4q6": SMALL["c2"], "q8_0": SMALL["c6"]}[shape].scaled(d=6144, ff=256, n_exp=6, top_k=2)
+    ol, gl, _ = make_pair(oracle, pb, ctx, cfg, 86)
+    rng = np.random.default_rng(87)
+    for T, tensor in ((1, 0), (3, 0), (4, 2), (8, 2)):
+        x = synth.make_activations(T, cfg.d, 940 + T)
+        ids, w = gl.route(x)
+        c0 = ctx.path_counts()
+        got = gl.experts(x, ids, w)
+        assert ctx.path_counts()["tensor"] - c0["tensor"] == tensor
+        assert bits_equal(got, ol.experts(x, ids, w))
+        x = synth.make_activations(2 * T, cfg.d, 945 + T)
+        eids, w = rng.integers(0, cfg.n_exp, 2 * T).astype(np.uint32), rng.uniform(0.5, 1.5, 2 * T).astype(np.float32)
+        c0 = ctx.path_counts()
+        got = gl.experts_rows(x, eids, w)
+        assert ctx.path_counts()["tensor"] - c0["tensor"] == tensor
+        for r in range(2 * T):
+            ids = np.array([[eids[r], (eids[r] + 1) % cfg.n_exp]], np.uint32)
+            at = int(oracle.plan(ids, cfg.n_exp)["pair_pos"].ravel()[0])
+            assert bits_equal(got[r], ol.experts(x[r:r + 1], ids, np.full(ids.shape, w[r], np.float32))[at])
+    gl.close()
