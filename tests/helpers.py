@@ -85,3 +85,9 @@ def device_pair(po, pb, ctx, cfg, seed):
     W = gl.get_weights(dense=False)
     ol = po.Layer(po.LayerDesc(**cfg.desc_fields()), W)
     return ol, gl
+
+
+def mx_tile(pb, cfg, T):
+    """Which MXFP4 kernel T tokens of a layer take: 16 or 32 tokens a tile (five or four fp8 pieces) or 128 (bf16 pieces)."""
+    groups = min(cfg.n_exp, cfg.n_exp_local) if cfg.n_exp_local > 0 else cfg.n_exp
+    return pb.load_library().pm_debug_mx_tile_tokens(T, T * cfg.top_k, groups, cfg.ff)

@@ -13,7 +13,7 @@ import pytest
 
 import pelica_b200 as pb
 from pelica_b200 import synth
-from tests.helpers import bits_equal, device_pair, tol_ok
+from tests.helpers import bits_equal, device_pair, mx_tile, tol_ok
 
 pytestmark = [pytest.mark.gpu, pytest.mark.timeout(1200)]
 
@@ -40,13 +40,14 @@ def test_c4_full_width_layer(ctx, oracle, T):
     gl.close()
 
 
-@pytest.mark.parametrize("T", [1, 2, 8, 31, 150, 300])
-def test_c3_full_width_layer(ctx, oracle, T):
+@pytest.mark.parametrize("T,tile", [(1, 16), (2, 16), (8, 16), (31, 16), (150, 32), (300, 32), (800, 128)])
+def test_c3_full_width_layer(ctx, oracle, T, tile):
     """d = ff = 2880, 32 experts, top-4 with softmax over the picks, router bias, expert
     biases, the gpt-oss GLU; f32 activations: tolerance 1e-3 relative + 1e-4 of the RMS. 90 MXFP4 blocks a row: 23 stages of
-    the block-scaled products (five pieces below 32 tokens, one token's down products in three parts along K; four pieces at 150),
-    45 chunks of the bf16 ones (300)."""
+    the block-scaled products (five pieces below 32 tokens, one token's down products in three parts along K; four pieces at 150
+    and 300), 45 chunks of the bf16 ones (800: the outputs of a sample of tokens)."""
     cfg = synth.C3_GPTOSS
+    assert mx_tile(pb, cfg, T) == tile
     ol, gl = device_pair(oracle, pb, ctx, cfg, 4300)
     x = synth.make_activations(T, cfg.d, 4400 + T)
     ids, w = gl.route(x)
@@ -56,10 +57,12 @@ def test_c3_full_width_layer(ctx, oracle, T):
     got = gl.forward(x)
     after = ctx.path_counts()
     assert after["tensor"] - before["tensor"] == 2 and after["general"] == before["general"]
-    want = ol.forward(x)
+    pick = np.arange(T) if T <= 300 else np.sort(np.random.default_rng(T).choice(T, 120, replace=False))
+    got, want = got[pick], ol.forward(x[pick])
     assert tol_ok(got, want), float(np.abs(got - want).max())
-    if T < 32:  # as close as the f32 sums in another order (the row kernels: 2e-7 of the RMS a sum)
-        rms = float(np.sqrt((want.astype(np.float64) ** 2).mean()))
+    rms = float(np.sqrt((want.astype(np.float64) ** 2).mean()))
+    if tile < 128:  # below 32 tokens as close as the f32 sums in another order (the row kernels: 2e-7 of the RMS a sum); four pieces hold a value to
+        # 2^-19 of its block's largest (6e-7 of the RMS of an output)
         assert float(np.abs(got - want).max()) < 1e-5 * rms
     gl.close()
 

@@ -1,11 +1,11 @@
-"""MXFP4 products at the ends of the number range: the tensor-core kernels against the oracle and the row kernels, whichever
-of them the token count picks."""
+"""MXFP4 products at the ends of the number range: each of the tensor-core kernels (five and four fp8 pieces, two bf16 pieces)
+against the oracle and the row kernels."""
 import numpy as np
 import pytest
 
 import pelica_b200 as pb
 from pelica_b200 import synth
-from tests.helpers import SMALL, tol_ok
+from tests.helpers import SMALL, mx_tile, tol_ok
 
 pytestmark = [pytest.mark.gpu, pytest.mark.timeout(600)]
 
@@ -24,6 +24,10 @@ def rows_ctx():
     c.set_tensor_core_min_tokens(0)
     yield c
     c.close()
+
+
+# tokens -> tokens of a tile of the kernel that a call of 8 experts, 4 a token, takes
+TILES = {1: 16, 3: 16, 5: 16, 31: 16, 40: 32, 150: 32, 200: 128}
 
 
 def codes(W, key, cfg):
@@ -52,11 +56,12 @@ def agree(got, want):
     assert tol_ok(got[fin], want[fin]), float(np.abs(got[fin] - want[fin]).max())
 
 
-@pytest.mark.parametrize("T", [1, 5, 40])
+@pytest.mark.parametrize("T", [1, 5, 40, 200])
 def test_activations_that_round_up_past_the_largest_float(ctx, rows_ctx, oracle, T):
     """|x| of 1.94 * 2^127 and more is 256 units of its first piece, 2^128: the pieces behind it still hold what is missing
     (3 % without them). The column meets codes of 0.5 in gate (no overflow in the row kernels either) and 0 in up."""
     cfg = SMALL["c3"].scaled(act_limit=3e38)
+    assert mx_tile(pb, cfg, T) == TILES[T]
     W = synth.make_weights(cfg, 91)
     for key, code in (("gate", 1), ("up", 0)):
         c = codes(W, key, cfg)
@@ -77,12 +82,13 @@ def test_activations_that_round_up_past_the_largest_float(ctx, rows_ctx, oracle,
 
 
 @pytest.mark.parametrize("shape", ["c3", "c3-wide"])
-@pytest.mark.parametrize("T", [1, 5, 31, 40, 150])
+@pytest.mark.parametrize("T", [1, 5, 31, 40, 150, 200])
 def test_activations_that_are_no_finite_number(ctx, rows_ctx, oracle, T, shape):
     """One infinity (or NaN) in a 32-value block spoils the sums that f32 arithmetic spoils and no others: inf where it meets a
     weight, NaN where it meets a zero or its opposite. 0.03 of the codes of its column are zeros here, so most sums are
     infinite and the clamp of the activation makes them finite again."""
     cfg = SMALL["c3"] if shape == "c3" else SMALL["c3"].scaled(d=288, ff=1120)
+    assert mx_tile(pb, cfg, T) == TILES[T]
     W = synth.make_weights(cfg, 93)
     rng = np.random.default_rng(94)
     for key in ("gate", "up"):
@@ -114,12 +120,13 @@ def test_activations_that_are_no_finite_number(ctx, rows_ctx, oracle, T, shape):
 
 
 @pytest.mark.parametrize("e", [0, 1, 2, 129, 249, 250, 253, 254, 255])
-@pytest.mark.parametrize("T", [3, 40, 150])
+@pytest.mark.parametrize("T", [3, 40, 150, 200])
 def test_scale_bytes_of_the_whole_range(ctx, rows_ctx, oracle, T, e):
     """A gate matrix whose blocks all have scale byte e, against activations that bring its sums back into range: fp8 products
-    (3 and 40 tokens: five and four pieces), bf16 products (150: a weight of 2^128 is none). 255 is 2^128 as in the row kernels: codes of 1 and more are
-    infinite, 0.5 is 2^127."""
-    cfg = SMALL["c3"].scaled(act_limit=1e30)
+    (3 tokens: five pieces, 40 and 150: four), bf16 products (200: a weight of 2^128 is none; an odd number of blocks a row). 255 is 2^128 as in
+    the row kernels: codes of 1 and more are infinite, 0.5 is 2^127."""
+    cfg = SMALL["c3"].scaled(act_limit=1e30, d=288 if T == 200 else 320)
+    assert mx_tile(pb, cfg, T) == TILES[T]
     W = synth.make_weights(cfg, 96)
     c = codes(W, "gate", cfg)
     c[..., 0] = e
