@@ -6,7 +6,7 @@ import pytest
 
 import pelica_b200 as pb
 from pelica_b200 import synth
-from tests.helpers import SMALL, bits_equal
+from tests.helpers import SMALL, bits_equal, device_pair, make_pair
 
 pytestmark = [pytest.mark.gpu, pytest.mark.timeout(600)]
 
@@ -93,3 +93,53 @@ def test_groups_of_every_size(ctx, oracle, types, shard, most):
     assert ctx.path_counts()["tensor"] - c0["tensor"] == 2
     assert bits_equal(got, ol.experts(x, ids, w))
     gl.close()
+
+
+@pytest.mark.parametrize("T", [8, 24])
+@pytest.mark.parametrize("types", ["q4q6", "q6q4", "q6q6"])
+def test_rings_go_round(ctx, oracle, types, T):
+    """Rows of six and five blocks (more than any ring has stages) and more items than CTAs: about 28 experts x 20 tiles of gate and up rows,
+    12 of down rows on two CTAs an SM, so a CTA takes a second item and its rings go round within an item and across two."""
+    gu, down = TYPES[types]
+    cfg = SMALL["c2"].scaled(d=1536, ff=1280, n_exp=32, type_gate=gu, type_up=gu, type_down=down)
+    ol, gl = device_pair(oracle, pb, ctx, cfg, 95)
+    x = synth.make_activations(T, cfg.d, 96 + T)
+    used = len(np.unique(gl.route(x)[0]))
+    assert used * (cfg.d // 128) > 2 * 148 and T * cfg.top_k // cfg.n_exp <= 6
+    c0 = ctx.path_counts()
+    got = gl.forward(x)
+    assert ctx.path_counts()["tensor"] - c0["tensor"] == 2
+    assert bits_equal(got, ol.forward(x))
+    gl.close()
+
+
+@pytest.mark.parametrize("T", [3, 9, 20])
+def test_received_rows_of_q6k_layers(ctx, oracle, T):
+    """Rows that arrive quantised (the expert-parallel call, a world of one) against Q6_K gate and up matrices: the record comes twice, each with
+    every other sub-block zero (24 to 160 rows on 24 experts)."""
+    cfg = SMALL["c2"].scaled(type_gate=Q6, type_up=Q6)
+    ol, gl, _ = make_pair(oracle, pb, ctx, cfg, 97)
+    x = synth.make_activations(T, cfg.d, 98 + T)
+    ep = pb.ExpertParallel(ctx, pb.ep_unique_id(), 0, 1)
+    c0 = ctx.path_counts()
+    got = ep.forward(gl, x)
+    assert ctx.path_counts()["tensor"] - c0["tensor"] == 2
+    assert bits_equal(got, ol.forward(x))
+    ep.close()
+    gl.close()
+
+
+@pytest.mark.parametrize("T", [1, 3, 40])
+@pytest.mark.parametrize("d", [4096, 4352, 12544])
+def test_wide_stacks(ctx, oracle, d, T):
+    """The combine step that norms the rows for the next layer: one round of its 1,024 threads (4096 columns), a second one, and
+    rows that need more than 48 KB of shared memory (12,544)."""
+    cfg = SMALL["c2"].scaled(d=d, ff=256, n_exp=6, top_k=2)
+    pairs = [device_pair(oracle, pb, ctx, cfg, 100 + l) for l in range(3)]
+    st = pb.Stack(ctx, [p[1] for p in pairs], eps=1e-6)
+    st.set_mode(True)  # (one token: not the decode kernel)
+    x = np.random.default_rng(d + T).normal(0, 1, (T, d)).astype(np.float32)
+    assert bits_equal(st.forward(x), oracle.stack_forward([p[0] for p in pairs], 1e-6, x))
+    st.close()
+    for p in pairs:
+        p[1].close()

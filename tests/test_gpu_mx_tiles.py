@@ -6,7 +6,7 @@ import pytest
 
 import pelica_b200 as pb
 from pelica_b200 import synth
-from tests.helpers import SMALL, make_pair, tol_ok
+from tests.helpers import SMALL, device_pair, make_pair, tol_ok
 
 pytestmark = [pytest.mark.gpu, pytest.mark.timeout(600)]
 
@@ -52,3 +52,19 @@ def test_calls_around_the_one_launch_routing(ctx, oracle, shape, T):
     else:
         assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
     gl.close()
+
+
+@pytest.mark.parametrize("d", [4096, 4608, 12544])
+def test_wide_stacks_of_parts(ctx, oracle, d):
+    """One token through a stack: down products cut along K, whose parts the combine step adds before it norms the row for the next
+    layer (one and two rounds of its threads, and more than 48 KB of shared memory)."""
+    cfg = SMALL["c3"].scaled(d=d, ff=1120 if d < 8192 else 2080, n_exp=4, top_k=1)
+    pairs = [device_pair(oracle, pb, ctx, cfg, 110 + l) for l in range(3)]
+    st = pb.Stack(ctx, [p[1] for p in pairs], eps=1e-6)
+    x = np.random.default_rng(d).normal(0, 1, (1, d)).astype(np.float32)
+    got, want = st.forward(x), oracle.stack_forward([p[0] for p in pairs], 1e-6, x)
+    assert tol_ok(got, want), float(np.abs(got - want).max())
+    assert float(np.abs(got - want).max()) < 4e-6 * float(np.sqrt((want.astype(np.float64) ** 2).mean()))
+    st.close()
+    for p in pairs:
+        p[1].close()
