@@ -186,8 +186,6 @@ struct TcTiles {
   int shared;          // the list holds the shared expert as one more group (pairs P .. P + T - 1)
   int max_tiles;
 };
-// tokens of each of the n tiles that cnt pairs make. Even tiles for the bf16 products: a weight tile is decoded once a
-// token tile at a cost that a tile of a few tokens does not hide.
 #define TC_FEW_TOKENS 8  // tokens of a tile of prefill_few.cu
 // record rows from one tile of a group to the next, and of a group of cnt pairs in n tiles (every group starts on a multiple
 // of 16; a tile of few tokens has 16 rows of its own)
@@ -195,6 +193,8 @@ __host__ __device__ inline uint32_t tc_tile_rows(int ntok, uint32_t tokens) { re
 __host__ __device__ inline uint32_t tc_group_rows(int ntok, uint32_t cnt, uint32_t n) {
   return ntok == TC_FEW_TOKENS ? 16u * n : (cnt + 15u) & ~15u;
 }
+// tokens of each of the n tiles that cnt pairs make. Even tiles for the bf16 products: a weight tile is decoded once a
+// token tile at a cost that a tile of a few tokens does not hide.
 __host__ __device__ inline uint32_t tc_tile_tokens(uint32_t cnt, uint32_t n, int ntok, int even) {
   return even && n > 1 ? ((cnt + n - 1) / n + 15u) & ~15u : (uint32_t)ntok;
 }
@@ -235,8 +235,8 @@ cudaError_t launch_tc(const Launch &L, const LayerDev &ly, bool shared_only, boo
                       const uint8_t *rec, const float *wts, float *out, int *err, unsigned long long wait_ns, int fault_block);
 // tensor-core forms for MXFP4 weights and f32 activations: tiles of 128 tokens on bf16 pieces (prefill_mx.cu), smaller
 // ones (mx_tile_tokens) on block-scaled fp8 pieces (prefill_mx8.cu). The rows are regrouped by tile and split into their
-// pieces (rec: mx_rec_bytes / mx8_rec_bytes bytes); the fp8 gate/up products write the pieces of h themselves (hrec). The down products of the second may be cut along K into mx_splits
-// parts: part s goes to out + s * split_stride.
+// pieces (rec: mx_rec_bytes / mx8_rec_bytes bytes); the fp8 gate/up products write the pieces of h themselves (hrec). The down
+// products of the second may be cut along K into mx_splits parts: part s goes to out + s * split_stride.
 size_t mx_rec_bytes(int n_pairs, int max_groups, int cols);
 size_t mx8_rec_bytes(int T, int n_pairs, int max_groups, int cols);
 int mx_tile_tokens(int T, int n_pairs, int n_groups, int ff);

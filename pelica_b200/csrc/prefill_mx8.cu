@@ -96,7 +96,7 @@ __device__ __forceinline__ float2 m8_from_e4m3x2(uint32_t v) {
 }
 __device__ __forceinline__ float m8_pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }  // -126 .. 127
 
-// f32 rows -> their pieces: per tile and stage [4 K blocks][2 groups of 16][pieces x rows][16], then the scales. A block's 32
+// the tokens' f32 rows (of pair p: row src_row[p]) -> their pieces: per tile and stage [4 K blocks][2 groups of 16][pieces x rows][16], then the scales. A block's 32
 // values lie as the packed codes come apart: group 0 holds values 0, 16, 1, 17 .. 7, 23, group 1 the others. A thread
 // a (row, block).
 template <int NP>
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(128) k_mx8_rows(const int *__restrict__ n_tile
       float v[32];
       uint32_t top = 0;
       const bool on = r < (int)T.z;
-      const size_t row = on ? (src_row ? src_row[T.y + r] : T.y + r) : 0;
+      const size_t row = on ? src_row[T.y + r] : 0;
       const float4 *src = (const float4 *)(x + row * cols + 32 * b);
 #pragma unroll
       for (int i = 0; i < 8; i++) {

@@ -115,6 +115,10 @@ __device__ __forceinline__ void q32_codes(uint32_t q, uint32_t &w0, uint32_t &w1
   w1 = __byte_perm(__byte_perm(0xbfad9881u, 0xf6eaddcfu, s >> 16), __byte_perm(0x26190d01u, 0x71594535u, s >> 16), p >> 16);
 }
 
+// blocks whose sums share a slot of 64 columns, of a tile of npad columns: fewer barriers for small tiles (the issuing warp fills the slots,
+// the workers read them)
+__host__ __device__ constexpr uint32_t q32_slot_blocks(uint32_t npad) { return npad <= 16 ? 4u : (npad <= 32 ? 2u : 1u); }
+
 struct Q32Item {
   uint4 t;
   int r0;
@@ -184,8 +188,6 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
     if (lane == 0) tc_mbar_arrive_used(it_empty + s, it.t.x ^ (uint32_t)it.r0, A.zero);
     return ok && it.t.x != Q32_END;
   };
-  // blocks whose sums share a slot of 64 columns: fewer barriers for small tiles
-  auto group_of = [](uint32_t npad) -> uint32_t { return npad <= 16 ? 4u : (npad <= 32 ? 2u : 1u); };
 
   if (warp == MW) {
     // ================= the issuing warp =================
@@ -195,7 +197,7 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
     Q32Item it;
     for (int k = 0; next_item(k, it); k++) {
       if ((int)it.t.x < 0) continue;
-      const uint32_t npad = (__reduce_max_sync(PM_FULL, it.t.z) + 15u) & ~15u, G = group_of(npad);
+      const uint32_t npad = (__reduce_max_sync(PM_FULL, it.t.z) + 15u) & ~15u, G = q32_slot_blocks(npad);
       // instruction descriptor: D s32, A and B s8, both K-major, N = npad, M = 128
       const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((npad >> 3) << 17) | ((uint32_t)(Q32_M >> 4) << 24);
       for (int s = 0; s < nst; s++, st++) {
@@ -381,14 +383,15 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
       };
       auto fold = [&](int s, unsigned long long sc) {
         if (npad == 16u) {
-          if (ew == 4) fold_slots(PassC<4>(), PassC<4>(), s, sc);
-          else fold_slots(PassC<8>(), PassC<4>(), s, sc);
+          if (ew == 4) fold_slots(PassC<4>(), PassC<(int)q32_slot_blocks(16)>(), s, sc);
+          else fold_slots(PassC<8>(), PassC<(int)q32_slot_blocks(16)>(), s, sc);
           return;
         }
         if (npad == 32u) {
-          fold_slots(PassC<16>(), PassC<2>(), s, sc);
+          fold_slots(PassC<16>(), PassC<(int)q32_slot_blocks(32)>(), s, sc);
           return;
         }
+        static_assert(q32_slot_blocks(48) == 1 && q32_slot_blocks(Q32_N) == 1, "one block a slot from here on");
         const int nblk = min(Q32_KB, nb - s * Q32_KB);
         const uint8_t *xd = sB + sb * Q32_BST + npad * 32u + e0 * 4;
         // (a slot a block; not unrolled: with four copies the workers waited for instructions, not for the pipes)
@@ -407,22 +410,21 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
             dw = pm_f16((uint32_t)(sc >> (16 * b)));
           }
           const uint64_t dw2 = tc_pack2(dw, dw);
-          auto half = [&](int c, auto n_) {  // columns c .. c + 15
-            constexpr int N = decltype(n_)::value;
+          auto half = [&](int c) {  // columns c .. c + 15
             uint32_t v[16];
             tc_ld8<0>(at + c, v);
             tc_ld8<8>(at + c, v + 8);
-            ulonglong2 x2[N / 4];
+            ulonglong2 x2[4];
 #pragma unroll
-            for (int u = 0; u < N / 4; u++) x2[u] = *(const ulonglong2 *)(xd + (c + 4 * u) * 4);
+            for (int u = 0; u < 4; u++) x2[u] = *(const ulonglong2 *)(xd + (c + 4 * u) * 4);
 #pragma unroll
-            for (int u = 0; u < N / 4; u++) {
+            for (int u = 0; u < 4; u++) {
               x2[u].x = tc_mul2(dw2, x2[u].x);
               x2[u].y = tc_mul2(dw2, x2[u].y);
             }
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int u = 0; u < N; u += 4) {
+            for (int u = 0; u < 16; u += 4) {
               const uint64_t s0 = tc_pack2(__int2float_rn((int)v[u]), __int2float_rn((int)v[u + 1]));
               const uint64_t s1 = tc_pack2(__int2float_rn((int)v[u + 2]), __int2float_rn((int)v[u + 3]));
               uint64_t *ac = acc + (c + u) / 2;
@@ -430,8 +432,8 @@ __global__ void __launch_bounds__(Q32_NT, 2) k_tc_q32(const __grid_constant__ Q3
               ac[1] = tc_add2(ac[1], tc_fma2(x2[u / 4].y, s1, A.neg_zero2));
             }
           };
-          half(0, PassC<16>());
-          half(16, PassC<16>());  // (24 columns: the last 8 are not used)
+          half(0);
+          half(16);  // (24 columns: the last 8 are not used)
           xd += npad * 36u;
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
