@@ -1008,17 +1008,18 @@ static Path pick_path(pm_layer *ly, int T, PathCall call) {
   Path p;
   // The integer products give the same bits on either path, so until the caller sets the threshold the faster one
   // decides (us a call, row kernels : tensor cores):
-  //  whole layer: two tokens up (64 experts x 2048 x 1024, 1 / 2 / 3 / 4 / 8 tokens 30 : 35, 42 : 34, 51 : 39, 63 : 45, 106 : 61;
-  //    128 x 2048 x 768 31 : 31, 43 : 36, 57 : 39, 73 : 46, 130 : 66; 4-bit codebook layers of 32 x 2560 x 640 43 : 53, 64 : 55, 86 : 60,
-  //    109 : 61, 187 : 70), and one where the shared expert joins the launch (64 x 7168 x 2048 101 : 67);
+  //  whole layer: two tokens up (64 experts x 2048 x 1024, 1 / 2 / 3 / 4 / 8 tokens 30 : 30, 41 : 34, 54 : 40, 62 : 42, 107 : 62;
+  //    128 x 2048 x 768 32 : 31, 43 : 36, 60 : 40, 69 : 43, 132 : 70; 4-bit codebook layers of 32 x 2560 x 640 43 : 54, 64 : 60, 90 : 60,
+  //    107 : 61, 193 : 67; Q8_0 38 : 43, 56 : 50, 80 : 51, 89 : 51, 157 : 59), and one where the shared expert joins the launch (64 x 7168 x 2048
+  //    101 : 67);
   //  experts of a given plan, which need the tile list in a launch of their own and may be one row an expert: more than 16 pairs, or from 48 K
   //    pairs x (d + ff) on - a row kernel's time goes with the bytes of its pairs, the tensor cores' hardly. Last call below : first above the line,
   //    a row each: 64 x 7168 x 2048 5 rows 56 : 53, 6 63 : 57, 8 76 : 61, 16 131 : 91; 64 x 5120 x 1536 7 51 : 40, 8 52 : 47; 64 x 4096 x 1536 8 44 : 41, 9 47 : 42;
   //    64 x 3072 x 1024 11 39 : 36, 12 41 : 36; 64 x 2048 x 1024 15 36 : 33, 16 37 : 34; 64 x 2048 x 4096 7 47 : 40, 8 54 : 47; 64 x 7168 x 512
   //    6 34 : 39, 7 46 : 41; Q8_0 32 x 5120 x 1280 7 92 : 69, 8 90 : 81, 32 x 2560 x 640 15 50 : 45, 16 50 : 45; and 64 x 1024 x 512, below
   //    it up to the 17th, 16 25 : 27 (some shapes cross two to four pairs earlier: the line is where none loses);
-  //  shared expert: more than 4 tokens (7168 x 2048, 1 / 4 / 5 / 8 tokens 19 : 47, 41 : 48, 49 : 48, 71 : 49; 2048 x 1024 16 : 27,
-  //    20 : 29, 22 : 30, 29 : 31, 12 tokens 39 : 31).
+  //  shared expert: more than 4 tokens (7168 x 2048, 1 / 3 / 4 / 5 / 8 tokens 21 : 35, 36 : 37, 43 : 38, 51 : 41, 73 : 42; 4096 x 1536 17 : 28,
+  //    25 : 30, 29 : 30, 33 : 33, 44 : 34; 2048 x 1024 17 : 23, 19 : 25, 21 : 25, 23 : 26, 30 : 27: the widths cross between 4 and 7).
   const bool int_tc = c->tc_min_set            ? T >= c->tc_min_tokens
                       : call == PATH_WHOLE     ? T >= (shared_merges(D) ? 1 : 2)
                       : call == PATH_EXPERTS   ? T * D.top_k > 16 || T * D.top_k * (D.d + D.ff) >= 48 * 1024
@@ -1026,7 +1027,7 @@ static Path pick_path(pm_layer *ly, int T, PathCall call) {
   p.tc = D.act_quant == PM_AQ_Q8X_256 && c->tc_min_tokens > 0 && int_tc;
   p.tc_gu = p.tc && D.type_gate == D.type_up;
   // (MXFP4: from one token up until the caller says otherwise; a layer of 32 experts, d = ff = 2880, row kernels : these, 1 / 2 /
-  // 4 / 8 / 16 tokens 64 : 54 us, 102 : 78, 164 : 106, 289 : 141, 524 : 173)
+  // 3 / 4 / 8 tokens 54 : 33 us, 94 : 47, 124 : 53, 162 : 61, 272 : 84; rows of a given plan, 1 / 2 / 4 / 16 29 : 32, 41 : 33, 51 : 37, 150 : 55)
   p.mx = mx_layer(D) && c->tc_min_tokens > 0 && T >= (c->tc_min_set ? c->tc_min_tokens : 1);
   p.q32 = q32_layer(D) && c->tc_min_tokens > 0 && int_tc;
   p.merge = call == PATH_WHOLE && p.tc_gu && shared_merges(D);
@@ -1117,9 +1118,9 @@ static int32_t dev_experts(pm_layer *ly, const float *x, int T, Scratch &S, cons
     PROF(c, PH_QUANT_X);
     if (tc_gu) {
       // Many rows: quantise every token once and gather the quantised rows, see k_tc_quant_rows. From 8 M values of all
-      // pairs on (a layer, this : quantised a pair: 128 experts x 2048 x 768, 512 / 1024 / 2048 tokens 247 : 250, 331 : 338, 525 : 540
-      // us; 64 x 2048 x 1024, 512 tokens 208 : 218; 32 x 7168 x 2048, 256 tokens 471 : 507); at 1 to 8 M the two are within
-      // 2 %, and a launch less is what a small call needs.
+      // pairs on (a layer, this : quantised a pair: 128 experts x 2048 x 768, 512 / 1024 / 2048 tokens 238 : 241, 321 : 328, 510 : 521
+      // us; 64 x 2048 x 1024, 512 / 2048 tokens 203 : 209, 527 : 538; 256 x 7168 x 2048, 512 tokens 2,025 : 2,044); at 1 to 8 M it is up to 2 %
+      // ahead (64 x 2048 x 1024, 64 / 256 tokens 108 : 110, 145 : 146; 64 x 4096 x 1536, 64 / 128 210 : 210, 258 : 258) for a launch more.
       const bool gather = prequant || (size_t)P * D.d > ((size_t)8 << 20);
       if (gather && !prequant) launch_quant_q8x(L, x, (size_t)T, D.d, S.xq, S.xd, S.xbsum, S.xbm, S.xs);
       if (gather) launch_tc_rows(L, D.type_gate, Pr, tt, g.pair_token, D.d, S.xq, S.xd, S.xbm, S.xs, S.rec);
