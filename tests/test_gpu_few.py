@@ -139,7 +139,9 @@ def test_wide_stacks(ctx, oracle, d, T):
     st = pb.Stack(ctx, [p[1] for p in pairs], eps=1e-6)
     st.set_mode(True)  # (one token: not the decode kernel)
     x = np.random.default_rng(d + T).normal(0, 1, (T, d)).astype(np.float32)
-    assert bits_equal(st.forward(x), oracle.stack_forward([p[0] for p in pairs], 1e-6, x))
+    want = oracle.stack_forward([p[0] for p in pairs], 1e-6, x)
+    for _ in range(3 if T <= 16 else 1):  # launch by launch, recorded, replayed
+        assert bits_equal(st.forward(x), want)
     st.close()
     for p in pairs:
         p[1].close()
